@@ -24,6 +24,7 @@ attn_simt_kernel(const T* __restrict__ q, long long q_rs, long long q_hs, const 
                  const T* __restrict__ v, long long kv_bs, long long kv_rs, long long kv_hs,
                  T* __restrict__ out, long long o_rs, long long o_hs, int n_keys, int n_keys_pad,
                  const int32_t* __restrict__ offsets, int l_max, float scale, int* status) {
+    pdl_begin();
     extern __shared__ float smem[];
     float* Qs = smem;                       // [AQ][AD]
     float* KV = Qs + AQ * AD;               // [AKC][AD + 1]
@@ -127,13 +128,13 @@ int attention_cuda_cores(const AttnArgs& p, cudaStream_t st) {
     if (p.dtype == VTP_F32) {
         e = cudaFuncSetAttribute(attn_simt_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e == cudaSuccess)
-            attn_simt_kernel<float><<<grid, 128, smem, st>>>(
+            launch_kernel(attn_simt_kernel<float>, false, 1, dim3(grid), dim3(128), smem, st, 
                 (const float*)p.q, p.q_rs, p.q_hs, (const float*)p.k, (const float*)p.v, p.kv_bs, p.kv_rs,
                 p.kv_hs, (float*)p.out, p.o_rs, p.o_hs, p.n_keys, n_pad, p.offsets, p.l_max, p.scale, device_status_ptr());
     } else {
         e = cudaFuncSetAttribute(attn_simt_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e == cudaSuccess)
-            attn_simt_kernel<bf16><<<grid, 128, smem, st>>>(
+            launch_kernel(attn_simt_kernel<bf16>, false, 1, dim3(grid), dim3(128), smem, st, 
                 (const bf16*)p.q, p.q_rs, p.q_hs, (const bf16*)p.k, (const bf16*)p.v, p.kv_bs, p.kv_rs,
                 p.kv_hs, (bf16*)p.out, p.o_rs, p.o_hs, p.n_keys, n_pad, p.offsets, p.l_max, p.scale, device_status_ptr());
     }

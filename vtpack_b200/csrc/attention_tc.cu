@@ -124,8 +124,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     }
     // Nothing above depends on the kernel in front of this one on the stream; the packed-row
     // offsets, q, k and v below do.
-    griddep_launch();
-    griddep_wait();
+    pdl_begin();
     // tile_prefix[b] = number of 128-query tiles of the images in front of b.  All threads fetch the
     // per-image tile counts at once (one global-load latency), then warp 0 scans them in shared memory.
     // (the offsets come from the caller: a count outside [0, max_q] is clamped, so the item list
@@ -483,7 +482,7 @@ int attention_tcgen05(const AttnArgs& p, cudaStream_t st) {
     }
     const long long worst = (long long)p.B * ceil_div(p.max_q, QT) * p.heads;
     const int grid = (int)(worst < 2ll * sm_count() ? worst : 2ll * sm_count());
-    const cudaError_t le = launch_pdl(attn_tc_kernel, dim3(grid), dim3(192), (size_t)smem, st, tq, tk, tv,
+    const cudaError_t le = launch_kernel(attn_tc_kernel, worst <= sm_count(), 1, dim3(grid), dim3(192), (size_t)smem, st, tq, tk, tv,
                                       (const bf16*)p.k, (const bf16*)p.v, p.q_hs, p.kv_bs, p.kv_rs, p.kv_hs, (bf16*)p.out,
                                       p.o_rs, p.o_hs, p.B, p.heads, p.n_keys, KC, n_chunks, p.offsets, p.l_max, p.max_q,
                                       p.scale * 1.4426950408889634f, device_status_ptr());

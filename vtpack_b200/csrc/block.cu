@@ -14,6 +14,9 @@ namespace vtp {
 int token_im2col(const void* x, int dtype, int B, int H, int W, int C, int sr, void* cols, cudaStream_t st,
                  const float2* stats = nullptr, const float* lnw = nullptr, const float* lnb = nullptr);  // patch_embed.cu
 
+int patch_im2col(const void* images, int image_dtype, int B, int S, int P, int dtype, void* cols, int ld,
+                 const void* cls_token, const void* pos_embed, int C, void* x, int32_t* counts, cudaStream_t st);   // patch_embed.cu
+
 struct Carver {
     char* base;
     long long off = 0;
@@ -58,7 +61,7 @@ static BlockScratch carve_block(const vtp_dge_shape& s, void* ws) {
     b.stats_x[0] = (float2*)c.take(rows * 8);
     b.stats_x[1] = (float2*)c.take(rows * 8);
     b.stats_q = (float2*)c.take(rows * 8);
-    b.stats_acc = (float2*)c.take(rows * 8 * STAT_SLOTS);
+    b.stats_acc = (float2*)c.take(rows * 8 * linear_stat_slots_max(s.C));
     b.comp = c.take(rows * s.C * e);
     b.xn = c.take(rows * s.C * e);
     b.qn = c.take(rows * s.C * e);
@@ -109,11 +112,6 @@ struct StageMarks {
     }
 };
 
-__global__ void fill_i32_kernel(int32_t* p, int n, int v) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = v;
-}
-
 static bool has_folded_weights(const vtp_block_weights& w) {
     return w.q_wf && w.q_s && w.q_c && w.kv_wf && w.kv_s && w.kv_c && w.fc1_wf && w.fc1_s && w.fc1_c;
 }
@@ -143,6 +141,8 @@ static bool block_folds(const vtp_dge_shape& s, const vtp_block_weights& w) {
 // the block that follows, whose gate and statistics this block's unpool can produce.
 struct BlockChain {
     bool have_gate = false;
+    bool counts_started = false;         // not chained: an earlier kernel set this block's counts to num_extra
+    int32_t* counts_next = nullptr;      // where the next block's counts go (null: scratch)
     int parity = 0;
     const vtp_block_weights* next = nullptr;
     const float* image_bias = nullptr;   // fp32 [B, n_splits] added to this and the next block's router logits
@@ -185,7 +185,8 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
     const bool fold_fc1 = fold_q && s.C > 128;
     const int par = chain.parity & 1;
     int32_t* idx = b.idx[par];
-    int32_t* counts = b.counts[par];
+    int32_t* counts = counts_out ? counts_out : b.counts[par];      // worked out in place: no copy afterwards
+    int32_t* counts_next = chain.counts_next ? chain.counts_next : b.counts[par ^ 1];
     float2* stats_x = b.stats_x[par];
     bool stats_x_ready = false;
     // chained: gate decisions, per-image counts and token statistics came from the previous
@@ -198,33 +199,34 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
         stats_x_ready = true;
         rc = VTP_OK;
     } else if (forced_logits) {
-        rc = vtp_gate_argmax(forced_logits, s.B * Hr * Wr, s.n_splits, idx, st);
+        rc = by_region ? count_queries(forced_logits, idx, sp, s.B, Hr * Wr, s.num_extra, counts, st)
+                       : vtp_gate_argmax(forced_logits, s.B * Hr * Wr, s.n_splits, idx, st);
     } else if (by_region) {
         RegionGateArgs ga;
         ga.g = g; ga.x = x_in; ga.gw = w.gate_w; ga.gb = w.gate_b; ga.S = s.n_splits; ga.logits_out = b.logits[par];
         ga.idx_out = idx; ga.eps = s.eps; ga.image_bias = chain.image_bias;
         if (fold_q) { ga.stats_x = stats_x; stats_x_ready = true; }
+        ga.sp = sp;
+        if (chain.counts_started) ga.counts = counts;
         rc = region_gate(ga, s.dtype, st);
     } else {
         rc = vtp_router_gate(x_in, s.dtype, s.B, s.H, s.W, C, s.num_extra, s.region, w.gate_w, w.gate_b,
                              s.n_splits, b.logits[par], idx, st);
     }
     if (rc || (rc = marks.mark(1))) return rc;
-    if (!chained)
-        rc = index_to_patch(idx, 0, sp, s.B, Hr, Wr, s.region, s.num_extra, counts, b.offsets,
-                            by_region ? nullptr : b.patches, nullptr, b.region_first, st);
+    // the region-parallel pool derives the packed rows from the counts; only the patch-list path needs the list
+    if (!by_region)
+        rc = index_to_patch(idx, 0, sp, s.B, Hr, Wr, s.region, s.num_extra, counts, b.offsets, b.patches, nullptr,
+                            nullptr, st);
+    else if (!chained && !forced_logits && !chain.counts_started)
+        rc = count_queries(nullptr, idx, sp, s.B, Hr * Wr, s.num_extra, counts, st);
     if (rc || (rc = marks.mark(2))) return rc;
-    if (counts_out) {
-        const cudaError_t e = cudaMemcpyAsync(counts_out, counts, (size_t)s.B * 4, cudaMemcpyDeviceToDevice, st);
-        if (e != cudaSuccess) return fail((int)e, "block: counts copy: %s", cudaGetErrorString(e));
-    }
     if (by_region) {
         RegionPoolArgs pa;
         pa.g = g; pa.sp = sp; pa.x = x_in; pa.idx = idx; pa.comp = b.comp; pa.eps = s.eps;
-        pa.region_first = chained ? nullptr : b.region_first;
-        pa.offsets = b.offsets; pa.counts = counts; pa.offsets_out = b.offsets; pa.region_first_out = b.region_first;
+        pa.counts = counts; pa.offsets_out = b.offsets; pa.region_first_out = b.region_first;
         const bool will_chain = fold_q && chain.next && block_folds(s, *chain.next);
-        pa.counts_next = (chained && will_chain) ? b.counts[par ^ 1] : nullptr;
+        pa.counts_next = will_chain ? counts_next : nullptr;
         if (fold_q) {
             pa.stats_x = stats_x; pa.stats_q = b.stats_q;
             pa.stats_x_ready = stats_x_ready;
@@ -297,7 +299,7 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
     l1.y = b.hid; l1.ldy = s.hidden; l1.dtype = s.dtype; l1.m_max = rows; l1.m_dev = L_dev; l1.N = s.hidden; l1.K = C;
     l1.flags = kflag | VTP_FLAG_GELU;
     if (fold_fc1) { l1.ln_mode = 2; l1.ln_stats = b.stats_acc; l1.ln_s = w.fc1_s; l1.ln_dim = C; l1.ln_eps = s.eps;
-                l1.ln_slots = linear_stat_slots(C); }
+                l1.ln_slots = linear_stat_slots(C, rows); }
     if ((rc = linear(l1, st)) || (rc = marks.mark(9))) return rc;
 
     LinearArgs l2;   // q2 = q1 + hid W2^T + b   (into the q-projection buffer, dead by now)
@@ -315,13 +317,8 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
             ua.next.stats_x = b.stats_x[par ^ 1]; ua.next.eps = s.eps;
             ua.next.gw = chain.next->gate_w; ua.next.gb = chain.next->gate_b; ua.next.S = s.n_splits;
             ua.next.logits = b.logits[par ^ 1]; ua.next.idx = b.idx[par ^ 1];
-            ua.next.counts = b.counts[par ^ 1];
+            ua.next.counts = counts_next;
             ua.next.image_bias = chain.image_bias;
-            if (!chained) {
-                // this block's pool did not reset the next block's counts: start them at the extra tokens
-                fill_i32_kernel<<<ceil_div(s.B, 256), 256, 0, st>>>(b.counts[par ^ 1], s.B, s.num_extra);
-                if ((rc = check_launch("counts reset"))) return rc;
-            }
         }
         rc = region_unpool(ua, s.dtype, st);
     } else {
@@ -333,6 +330,7 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
 }
 
 __global__ void dense_offsets_kernel(int32_t* offsets, int B, int N) {
+    pdl_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i <= B) offsets[i] = i * N;
 }
@@ -345,7 +343,7 @@ static int dense_block_forward(const vtp_dge_shape& s, const vtp_block_weights& 
     const unsigned kflag = s.flags & VTP_FLAG_CUDA_CORES;
     BlockScratch b = carve_block(s, ws);
     int rc;
-    dense_offsets_kernel<<<ceil_div(s.B + 1, 128), 128, 0, st>>>(b.offsets, s.B, N);
+    launch_chain(dense_offsets_kernel, dim3(ceil_div(s.B + 1, 128)), dim3(128), 0, st, b.offsets, s.B, N);
     if ((rc = check_launch("dense offsets"))) return rc;
     rc = vtp_layernorm(x_in, s.dtype, rows, nullptr, C, C, w.norm1_w, w.norm1_b, s.eps, b.xn, st);
     if (rc) return rc;
@@ -440,6 +438,7 @@ extern "C" int vtp_dge_blocks_forward(const vtp_dge_shape* s, const vtp_block_we
         chain.have_gate = chained;
         chain.parity = i & 1;
         chain.next = (i + 1 < n_blocks) ? &w[i + 1] : nullptr;
+        chain.counts_next = (counts_out && chain.next) ? counts_out + (size_t)(i + 1) * s->B : nullptr;
         if (int rc = block_forward(*s, w[i], i == 0 ? x_in : x_out, x_out, nullptr,
                                    counts_out ? counts_out + (size_t)i * s->B : nullptr, workspace, st, StageMarks(),
                                    chain))
@@ -502,8 +501,10 @@ extern "C" int vtp_deit_dge_forward_ex(const vtp_dge_shape* s, const vtp_model_w
     const int HW = s->H * s->W, N = HW + 1, C = s->C;
     const int KP = 3 * m->patch * m->patch;
     const long long e = (long long)elem_size(s->dtype);
-    int rc = vtp_patch_im2col(images, m->image_dtype, s->B, m->img_size, m->patch, s->dtype, ms.cols, m->cls_token,
-                              m->pos_embed, C, ms.x, st);
+    const BlockScratch bs = carve_block(*s, ms.block_ws);
+    // (the kernel that writes the cls rows also starts the first block's query counts)
+    int rc = patch_im2col(images, m->image_dtype, s->B, m->img_size, m->patch, s->dtype, ms.cols, 3 * m->patch * m->patch,
+                          m->cls_token, m->pos_embed, C, ms.x, counts_out ? counts_out : bs.counts[0], st);
     if (rc) return rc;
     LinearArgs pe;   // token (b, 1+t) = cols(b,t) Wp^T + bias + pos_embed[1+t]
     pe.a = ms.cols; pe.lda = KP; pe.w = m->patch_w; pe.bias = m->patch_b; pe.res = m->pos_embed; pe.ldr = C;
@@ -512,13 +513,14 @@ extern "C" int vtp_deit_dge_forward_ex(const vtp_dge_shape* s, const vtp_model_w
     pe.out_grp = HW; pe.out_skip = 1; pe.res_mod = HW; pe.res_off = 1;
     if ((rc = linear(pe, st))) return rc;
     bool chained = false;      // block i-1's unpool prepared block i's gate
-    const BlockScratch bs = carve_block(*s, ms.block_ws);
     const long long R = (long long)(s->H / s->region) * (s->W / s->region);
     for (int i = 0; i < m->depth; ++i) {
         BlockChain chain;
         chain.have_gate = chained;
         chain.parity = i & 1;
         chain.next = (i + 1 < m->depth) ? &blocks[i + 1] : nullptr;
+        chain.counts_next = (counts_out && chain.next) ? counts_out + (size_t)(i + 1) * s->B : nullptr;
+        chain.counts_started = i == 0;
         chain.image_bias = opt ? opt->gate_image_bias : nullptr;
         if (opt && opt->tokens_trace) {
             const size_t nb = (size_t)s->B * N * C * e;

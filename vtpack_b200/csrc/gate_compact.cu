@@ -17,6 +17,7 @@ router_gate_kernel(const T* __restrict__ x, int n_regions, int Hr, int Wr, int W
                    int num_extra, int region, const float* __restrict__ gw,
                    const float* __restrict__ gb, int S, float* __restrict__ logits_out,
                    int32_t* __restrict__ idx_out) {
+    pdl_begin();
     constexpr int VN = Vec<T>::N;
     const int lane = threadIdx.x & 31;
     const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -80,6 +81,7 @@ router_gate_kernel(const T* __restrict__ x, int n_regions, int Hr, int Wr, int W
 
 __global__ void gate_argmax_kernel(const float* __restrict__ logits, int rows, int S,
                                    int32_t* __restrict__ idx_out) {
+    pdl_begin();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= rows) return;
     float best = logits[(size_t)r * S];
@@ -95,6 +97,7 @@ __global__ void gate_argmax_kernel(const float* __restrict__ logits, int rows, i
 template <typename I>
 __global__ void count_kernel(const I* __restrict__ idx, int B, int R, Splits sp, int num_extra,
                              int32_t* __restrict__ counts) {
+    pdl_begin();
     const int lane = threadIdx.x & 31;
     const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (b >= B) return;
@@ -102,6 +105,35 @@ __global__ void count_kernel(const I* __restrict__ idx, int B, int R, Splits sp,
     for (int r = lane; r < R; r += 32) {
         int k = (int)idx[(size_t)b * R + r];
         k = min(max(k, 0), sp.n - 1);
+        c += sp.v[k] * sp.v[k];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    if (lane == 0) counts[b] = c + num_extra;
+}
+
+// The same for a block forward, which needs no patch list: counts only, after the argmax of given logits if any.
+__global__ void __launch_bounds__(128)
+argmax_count_kernel(const float* __restrict__ logits, int32_t* __restrict__ idx, int B, int R, Splits sp, int num_extra,
+                    int32_t* __restrict__ counts) {
+    pdl_begin();
+    const int lane = threadIdx.x & 31;
+    const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (b >= B) return;
+    int c = 0;
+    for (int r = lane; r < R; r += 32) {
+        const size_t rid = (size_t)b * R + r;
+        int k;
+        if (logits) {
+            const float* p = logits + rid * sp.n;
+            float best = p[0];
+            k = 0;
+            for (int s = 1; s < sp.n; ++s)
+                if (p[s] > best) { best = p[s]; k = s; }
+            idx[rid] = k;
+        } else {
+            k = min(max(idx[rid], 0), sp.n - 1);
+        }
         c += sp.v[k] * sp.v[k];
     }
 #pragma unroll
@@ -118,6 +150,7 @@ write_patches_kernel(const I* __restrict__ idx, int B, int Hr, int Wr, Splits sp
                      int num_extra, const int32_t* __restrict__ counts,
                      int32_t* __restrict__ offsets, int32_t* __restrict__ patches,
                      int64_t* __restrict__ patches64, int32_t* __restrict__ region_first) {
+    pdl_begin();
     extern __shared__ int s_start[];   // [R + 1] first row of each region within the image
     __shared__ int s_warp[4];
     __shared__ int s_base;
@@ -200,7 +233,7 @@ static int launch_router(const void* x, int B, int H, int W, int C, int num_extr
     const int grid = ceil_div(n_regions, 4);
     const T* xp = static_cast<const T*>(x);
 #define VTP_LAUNCH_ROUTER(M)                                                                   \
-    router_gate_kernel<T, M><<<grid, 128, 0, st>>>(xp, n_regions, Hr, Wr, W, N, C, num_extra,  \
+    launch_chain(router_gate_kernel<T, M>, dim3(grid), dim3(128), 0, st, xp, n_regions, Hr, Wr, W, N, C, num_extra,  \
                                                    region, gw, gb, S, logits, idx)
     if (maxch <= 1) VTP_LAUNCH_ROUTER(1);
     else if (maxch == 2) VTP_LAUNCH_ROUTER(2);
@@ -242,7 +275,7 @@ extern "C" int vtp_gate_argmax(const float* logits, int rows, int n_splits, int3
     VTP_REQUIRE(logits && grain_idx, VTP_ERR_NULL, "gate argmax: null pointer");
     VTP_REQUIRE(rows >= 0 && n_splits >= 1, VTP_ERR_SHAPE, "gate argmax: bad shape");
     if (rows == 0) return VTP_OK;
-    gate_argmax_kernel<<<ceil_div(rows, 128), 128, 0, static_cast<cudaStream_t>(stream)>>>(
+    launch_chain(gate_argmax_kernel, dim3(ceil_div(rows, 128)), dim3(128), 0, static_cast<cudaStream_t>(stream), 
         logits, rows, n_splits, grain_idx);
     return check_launch("gate_argmax");
 }
@@ -255,16 +288,22 @@ int index_to_patch(const void* indices, int idx_is_i64, const Splits& sp, int B,
     const size_t smem = (size_t)(R + 1) * sizeof(int);
     if (idx_is_i64) {
         const int64_t* ip = static_cast<const int64_t*>(indices);
-        count_kernel<int64_t><<<ceil_div(B, 4), 128, 0, st>>>(ip, B, R, sp, num_extra, counts);
-        write_patches_kernel<int64_t><<<B, 128, smem, st>>>(ip, B, Hr, Wr, sp, region, num_extra, counts, offsets,
+        launch_chain(count_kernel<int64_t>, dim3(ceil_div(B, 4)), dim3(128), 0, st, ip, B, R, sp, num_extra, counts);
+        launch_chain(write_patches_kernel<int64_t>, dim3(B), dim3(128), smem, st, ip, B, Hr, Wr, sp, region, num_extra, counts, offsets,
                                                             patches, patches64, region_first);
     } else {
         const int32_t* ip = static_cast<const int32_t*>(indices);
-        count_kernel<int32_t><<<ceil_div(B, 4), 128, 0, st>>>(ip, B, R, sp, num_extra, counts);
-        write_patches_kernel<int32_t><<<B, 128, smem, st>>>(ip, B, Hr, Wr, sp, region, num_extra, counts, offsets,
+        launch_chain(count_kernel<int32_t>, dim3(ceil_div(B, 4)), dim3(128), 0, st, ip, B, R, sp, num_extra, counts);
+        launch_chain(write_patches_kernel<int32_t>, dim3(B), dim3(128), smem, st, ip, B, Hr, Wr, sp, region, num_extra, counts, offsets,
                                                             patches, patches64, region_first);
     }
     return check_launch("index_to_patch");
+}
+
+int count_queries(const float* logits, int32_t* idx, const Splits& sp, int B, int R, int num_extra, int32_t* counts,
+                  cudaStream_t st) {
+    launch_chain(argmax_count_kernel, dim3(ceil_div(B, 4)), dim3(128), 0, st, logits, idx, B, R, sp, num_extra, counts);
+    return check_launch("count_queries");
 }
 
 int make_splits(Splits* sp, const int* splits, int n_splits, int region) {

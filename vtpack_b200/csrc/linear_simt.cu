@@ -15,6 +15,7 @@ linear_simt_kernel(const T* __restrict__ a, long long lda, const T* __restrict__
                    const float* __restrict__ bias, const T* __restrict__ res, long long ldr,
                    OutT* __restrict__ y, long long ldy, int m_max, const int32_t* __restrict__ m_dev,
                    int N, int K, unsigned flags, RowMap rm) {
+    pdl_begin();
     __shared__ float As[SBK][SBM + 4];
     __shared__ float Bs[SBK][SBN + 4];
     int M = m_max;
@@ -85,15 +86,15 @@ int linear_cuda_cores(const LinearArgs& p, cudaStream_t st) {
     const dim3 grid(ceil_div(p.N, SBN), ceil_div(p.m_max, SBM));
     const RowMap rm{p.out_grp, p.out_skip, p.res_mod, p.res_off};
     if (p.dtype == VTP_F32) {
-        linear_simt_kernel<float, float><<<grid, 256, 0, st>>>(
+        launch_kernel(linear_simt_kernel<float, float>, false, 1, dim3(grid), dim3(256), 0, st, 
             (const float*)p.a, p.lda, (const float*)p.w, p.bias, (const float*)p.res, p.ldr,
             (float*)p.y, p.ldy, p.m_max, p.m_dev, p.N, p.K, p.flags, rm);
     } else if (p.flags & VTP_FLAG_OUT_F32) {
-        linear_simt_kernel<bf16, float><<<grid, 256, 0, st>>>(
+        launch_kernel(linear_simt_kernel<bf16, float>, false, 1, dim3(grid), dim3(256), 0, st, 
             (const bf16*)p.a, p.lda, (const bf16*)p.w, p.bias, (const bf16*)p.res, p.ldr,
             (float*)p.y, p.ldy, p.m_max, p.m_dev, p.N, p.K, p.flags, rm);
     } else {
-        linear_simt_kernel<bf16, bf16><<<grid, 256, 0, st>>>(
+        launch_kernel(linear_simt_kernel<bf16, bf16>, false, 1, dim3(grid), dim3(256), 0, st, 
             (const bf16*)p.a, p.lda, (const bf16*)p.w, p.bias, (const bf16*)p.res, p.ldr,
             (bf16*)p.y, p.ldy, p.m_max, p.m_dev, p.N, p.K, p.flags, rm);
     }

@@ -50,6 +50,7 @@ __device__ __forceinline__ void store4(bf16* p, const float* f) {
 template <typename I, typename T, typename IDX>
 __global__ void __launch_bounds__(256)
 im2col4_kernel(const I* __restrict__ img, long long total4, int S, int P, T* __restrict__ cols, int ld) {
+    pdl_begin();
     const int G = S / P;
     const int KP = 3 * P * P;
     const IDX uS = (IDX)S, plane = (IDX)S * (IDX)S;
@@ -77,6 +78,7 @@ im2col4_kernel(const I* __restrict__ img, long long total4, int S, int P, T* __r
 template <typename I, typename T>
 __global__ void __launch_bounds__(256)
 im2col_p4_kernel(const I* __restrict__ img, int S, T* __restrict__ cols, int ld) {
+    pdl_begin();
     constexpr int P = 4, KP = 48, VT = 16 / (int)sizeof(T);     // VT: elements of a 16-byte store
     extern __shared__ __align__(16) unsigned char tile_raw[];
     T* tile = reinterpret_cast<T*>(tile_raw);
@@ -104,13 +106,26 @@ im2col_p4_kernel(const I* __restrict__ img, int S, T* __restrict__ cols, int ld)
     }
 }
 
+// What the extra CTAs of the 8-pixel kernel write: x[b, 0, :] = cls token + its position row, and (optional) the
+// number of queries image b starts with in the first block, its cls token.
+template <typename T>
+struct ClsRows { const T* token; const T* pos; int C; long long row_stride; T* x; int32_t* counts; };
+
 template <typename I, typename T>
 __global__ void __launch_bounds__(256)
-im2col_kernel(const I* __restrict__ img, long long total8, int S, int P, T* __restrict__ cols) {
+im2col_kernel(const I* __restrict__ img, long long total8, int S, int P, T* __restrict__ cols, int n_move, ClsRows<T> cls) {
+    pdl_begin();
+    if ((int)blockIdx.x >= n_move) {                     // one CTA per image behind the pixel movers: its cls row
+        const int b = blockIdx.x - n_move;
+        for (int c = threadIdx.x; c < cls.C; c += blockDim.x)
+            cls.x[(size_t)b * cls.row_stride + c] = from_f32<T>(to_f32(cls.token[c]) + to_f32(cls.pos[c]));
+        if (threadIdx.x == 0 && cls.counts) cls.counts[b] = 1;
+        return;
+    }
     const int G = S / P;
     const int KP = 3 * P * P;
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total8;
-         e += (long long)gridDim.x * blockDim.x) {
+         e += (long long)n_move * blockDim.x) {
         const long long pix = e * 8;
         const int ix = (int)(pix % S);
         const int iy = (int)((pix / S) % S);
@@ -131,14 +146,6 @@ im2col_kernel(const I* __restrict__ img, long long total8, int S, int P, T* __re
     }
 }
 
-template <typename T>
-__global__ void cls_row_kernel(const T* __restrict__ cls, const T* __restrict__ pos, int C, long long row_stride,
-                               T* __restrict__ x) {
-    const int b = blockIdx.x;
-    for (int c = threadIdx.x; c < C; c += blockDim.x)
-        x[(size_t)b * row_stride + c] = from_f32<T>(to_f32(cls[c]) + to_f32(pos[c]));
-}
-
 // Rows of the stride-sr reduction convolution of a PVT block as a GEMM operand: row (b, oy, ox) is
 // the sr x sr window of tokens, column (dy, dx, c).  A window row (fixed dy) is sr consecutive
 // tokens = sr*C contiguous elements on both sides; one thread moves 16 bytes.
@@ -147,6 +154,7 @@ template <typename T, typename IDX>
 __global__ void __launch_bounds__(256)
 token_im2col_kernel(const T* __restrict__ x, long long total_vec, int H, int W, int C, int sr, T* __restrict__ cols,
                     const float2* __restrict__ stats, const float* __restrict__ lnw, const float* __restrict__ lnb) {
+    pdl_begin();
     // stats != null: the rows gathered are LayerNorm(x), normalised on the way from each token's (mean, rstd)
     // (IDX: unsigned when the vector count fits 32 bits, see im2col4_kernel)
     constexpr int VN = Vec<T>::N;
@@ -192,14 +200,18 @@ int token_im2col(const void* x, int dtype, int B, int H, int W, int C, int sr, v
     const int grid = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
     const bool small = total < (1ll << 31);
     if (dtype == VTP_BF16) {
-        if (small) token_im2col_kernel<bf16, unsigned><<<grid, 256, 0, st>>>((const bf16*)x, total, H, W, C, sr, (bf16*)cols, stats, lnw, lnb);
-        else token_im2col_kernel<bf16, long long><<<grid, 256, 0, st>>>((const bf16*)x, total, H, W, C, sr, (bf16*)cols, stats, lnw, lnb);
+        if (small) launch_chain(token_im2col_kernel<bf16, unsigned>, dim3(grid), dim3(256), 0, st, (const bf16*)x, total, H, W, C, sr, (bf16*)cols, stats, lnw, lnb);
+        else launch_chain(token_im2col_kernel<bf16, long long>, dim3(grid), dim3(256), 0, st, (const bf16*)x, total, H, W, C, sr, (bf16*)cols, stats, lnw, lnb);
     } else {
-        if (small) token_im2col_kernel<float, unsigned><<<grid, 256, 0, st>>>((const float*)x, total, H, W, C, sr, (float*)cols, stats, lnw, lnb);
-        else token_im2col_kernel<float, long long><<<grid, 256, 0, st>>>((const float*)x, total, H, W, C, sr, (float*)cols, stats, lnw, lnb);
+        if (small) launch_chain(token_im2col_kernel<float, unsigned>, dim3(grid), dim3(256), 0, st, (const float*)x, total, H, W, C, sr, (float*)cols, stats, lnw, lnb);
+        else launch_chain(token_im2col_kernel<float, long long>, dim3(grid), dim3(256), 0, st, (const float*)x, total, H, W, C, sr, (float*)cols, stats, lnw, lnb);
     }
     return check_launch("spatial reduction im2col");
 }
+
+// patch_im2col below: images -> GEMM rows, and when x is given the cls rows and the first block's query counts.
+int patch_im2col(const void* images, int image_dtype, int B, int S, int P, int dtype, void* cols, int ld,
+                 const void* cls_token, const void* pos_embed, int C, void* x, int32_t* counts, cudaStream_t st);
 
 // out[orow(r)] = x[r % x_mod] + addend[r % a_mod + a_off], orow(r) = (r / out_grp) * out_stride + out_off + r % out_grp:
 // the position-embedding add of a token stage, and (x_mod = a_mod = out_grp = 1) the cls rows put in front of it.
@@ -207,6 +219,7 @@ template <typename T, typename IDX>
 __global__ void __launch_bounds__(256)
 add_rows_kernel(const T* __restrict__ x, int x_mod, const T* __restrict__ addend, int a_mod, int a_off,
                 T* __restrict__ out, int out_grp, int out_stride, int out_off, long long total_vec, int C) {
+    pdl_begin();
     // (IDX: unsigned when the vector count fits 32 bits, see im2col4_kernel)
     constexpr int VN = Vec<T>::N;
     const int cv = C / VN;
@@ -255,7 +268,7 @@ extern "C" int vtp_add_rows(const void* x, int x_mod, const void* addend, int a_
     const int grid = (int)((total + 255) / 256 < (long long)sm_count() * 16 ? (total + 255) / 256 : (long long)sm_count() * 16);
     const bool small = total < (1ll << 31);
 #define VTP_ADD_ROWS(T, IDX)                                                                                  \
-    add_rows_kernel<T, IDX><<<grid, 256, 0, st>>>((const T*)x, x_mod, (const T*)addend, a_mod, a_off, (T*)out, \
+    launch_chain(add_rows_kernel<T, IDX>, dim3(grid), dim3(256), 0, st, (const T*)x, x_mod, (const T*)addend, a_mod, a_off, (T*)out, \
                                                   out_grp, out_stride, out_off, total, C)
     if (dtype == VTP_BF16) { if (small) VTP_ADD_ROWS(bf16, unsigned); else VTP_ADD_ROWS(bf16, long long); }
     else { if (small) VTP_ADD_ROWS(float, unsigned); else VTP_ADD_ROWS(float, long long); }
@@ -263,12 +276,10 @@ extern "C" int vtp_add_rows(const void* x, int x_mod, const void* addend, int a_
     return check_launch("add rows");
 }
 
-static int patch_im2col(const void* images, int image_dtype, int B, int S, int P, int dtype, void* cols, int ld,
-                        const void* cls_token, const void* pos_embed, int C, void* x, void* stream);
-
 extern "C" int vtp_patch_im2col(const void* images, int image_dtype, int B, int S, int P, int dtype, void* cols,
                                 const void* cls_token, const void* pos_embed, int C, void* x, void* stream) {
-    return patch_im2col(images, image_dtype, B, S, P, dtype, cols, 3 * P * P, cls_token, pos_embed, C, x, stream);
+    return patch_im2col(images, image_dtype, B, S, P, dtype, cols, 3 * P * P, cls_token, pos_embed, C, x, nullptr,
+                        static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int vtp_patch_im2col_padded(const void* images, int image_dtype, int B, int S, int P, int dtype, void* cols,
@@ -278,18 +289,20 @@ extern "C" int vtp_patch_im2col_padded(const void* images, int image_dtype, int 
     VTP_REQUIRE(ld_cols >= 3 * P * P && ld_cols % 8 == 0, VTP_ERR_SHAPE,
                 "im2col (padded rows): row pitch %d for %d columns (a multiple of 8, at least the columns)", ld_cols,
                 3 * P * P);
-    return patch_im2col(images, image_dtype, B, S, P, dtype, cols, ld_cols, nullptr, nullptr, 0, nullptr, stream);
+    return patch_im2col(images, image_dtype, B, S, P, dtype, cols, ld_cols, nullptr, nullptr, 0, nullptr, nullptr,
+                        static_cast<cudaStream_t>(stream));
 }
 
-static int patch_im2col(const void* images, int image_dtype, int B, int S, int P, int dtype, void* cols, int ld,
-                        const void* cls_token, const void* pos_embed, int C, void* x, void* stream) {
+namespace vtp {
+
+int patch_im2col(const void* images, int image_dtype, int B, int S, int P, int dtype, void* cols, int ld,
+                 const void* cls_token, const void* pos_embed, int C, void* x, int32_t* counts, cudaStream_t st) {
     VTP_REQUIRE(images && cols, VTP_ERR_NULL, "im2col: null pointer");
     VTP_REQUIRE(dtype == VTP_F32 || dtype == VTP_BF16, VTP_ERR_DTYPE, "im2col: dtype %d", dtype);
     VTP_REQUIRE(image_dtype == VTP_F32 || image_dtype == VTP_BF16, VTP_ERR_DTYPE, "im2col: image dtype %d", image_dtype);
     VTP_REQUIRE(B > 0 && S > 0 && P > 0 && S % P == 0 && P % 4 == 0, VTP_ERR_SHAPE,
                 "im2col: image %d / patch %d (patch must be a multiple of 4)", S, P);
     VTP_REQUIRE(aligned16(images) && aligned16(cols), VTP_ERR_ALIGN, "im2col: unaligned pointer");
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (P % 8 != 0) {
         VTP_REQUIRE(!x, VTP_ERR_UNSUPPORTED, "im2col: the cls row is written for patches that are multiples of 8 only");
         const long long total4 = (long long)B * 3 * S * S / 4;
@@ -299,56 +312,49 @@ static int patch_im2col(const void* images, int image_dtype, int B, int S, int P
         if (P == 4 && ld % (16 / (int)elem_size(dtype)) == 0 && p4_smem <= 48 * 1024) {
             const int grid = B * (S / 4);
             if (image_dtype == VTP_F32 && dtype == VTP_F32)
-                im2col_p4_kernel<float, float><<<grid, 256, p4_smem, st>>>((const float*)images, S, (float*)cols, ld);
+                launch_chain(im2col_p4_kernel<float, float>, dim3(grid), dim3(256), p4_smem, st, (const float*)images, S, (float*)cols, ld);
             else if (image_dtype == VTP_F32)
-                im2col_p4_kernel<float, bf16><<<grid, 256, p4_smem, st>>>((const float*)images, S, (bf16*)cols, ld);
+                launch_chain(im2col_p4_kernel<float, bf16>, dim3(grid), dim3(256), p4_smem, st, (const float*)images, S, (bf16*)cols, ld);
             else if (dtype == VTP_F32)
-                im2col_p4_kernel<bf16, float><<<grid, 256, p4_smem, st>>>((const bf16*)images, S, (float*)cols, ld);
+                launch_chain(im2col_p4_kernel<bf16, float>, dim3(grid), dim3(256), p4_smem, st, (const bf16*)images, S, (float*)cols, ld);
             else
-                im2col_p4_kernel<bf16, bf16><<<grid, 256, p4_smem, st>>>((const bf16*)images, S, (bf16*)cols, ld);
+                launch_chain(im2col_p4_kernel<bf16, bf16>, dim3(grid), dim3(256), p4_smem, st, (const bf16*)images, S, (bf16*)cols, ld);
             return check_launch("im2col");
         }
         // 32-bit indices when the pixel count and the padded output both fit
         const bool small = (long long)B * 3 * S * S < (1ll << 31) && (long long)B * (S / P) * (S / P) * ld < (1ll << 31);
-#define VTP_IM2COL4(I, T, ARGS)                                                              \
+#define VTP_IM2COL4(I, T, ...)                                                              \
     do {                                                                                     \
-        if (small) im2col4_kernel<I, T, unsigned><<<g4, 256, 0, st>>> ARGS;                   \
-        else im2col4_kernel<I, T, long long><<<g4, 256, 0, st>>> ARGS;                        \
+        if (small) launch_chain(im2col4_kernel<I, T, unsigned>, dim3(g4), dim3(256), 0, st, __VA_ARGS__);   \
+        else launch_chain(im2col4_kernel<I, T, long long>, dim3(g4), dim3(256), 0, st, __VA_ARGS__);        \
     } while (0)
         if (image_dtype == VTP_F32 && dtype == VTP_F32)
-            VTP_IM2COL4(float, float, ((const float*)images, total4, S, P, (float*)cols, ld));
+            VTP_IM2COL4(float, float, (const float*)images, total4, S, P, (float*)cols, ld);
         else if (image_dtype == VTP_F32)
-            VTP_IM2COL4(float, bf16, ((const float*)images, total4, S, P, (bf16*)cols, ld));
+            VTP_IM2COL4(float, bf16, (const float*)images, total4, S, P, (bf16*)cols, ld);
         else if (dtype == VTP_F32)
-            VTP_IM2COL4(bf16, float, ((const bf16*)images, total4, S, P, (float*)cols, ld));
+            VTP_IM2COL4(bf16, float, (const bf16*)images, total4, S, P, (float*)cols, ld);
         else
-            VTP_IM2COL4(bf16, bf16, ((const bf16*)images, total4, S, P, (bf16*)cols, ld));
+            VTP_IM2COL4(bf16, bf16, (const bf16*)images, total4, S, P, (bf16*)cols, ld);
 #undef VTP_IM2COL4
         return check_launch("im2col");
     }
     const long long total8 = (long long)B * 3 * S * S / 8;
     const int grid = (int)((total8 + 255) / 256 < (long long)sm_count() * 16 ? (total8 + 255) / 256
                                                                              : (long long)sm_count() * 16);
-    if (image_dtype == VTP_F32 && dtype == VTP_F32)
-        im2col_kernel<float, float><<<grid, 256, 0, st>>>((const float*)images, total8, S, P, (float*)cols);
-    else if (image_dtype == VTP_F32)
-        im2col_kernel<float, bf16><<<grid, 256, 0, st>>>((const float*)images, total8, S, P, (bf16*)cols);
-    else if (dtype == VTP_F32)
-        im2col_kernel<bf16, float><<<grid, 256, 0, st>>>((const bf16*)images, total8, S, P, (float*)cols);
-    else
-        im2col_kernel<bf16, bf16><<<grid, 256, 0, st>>>((const bf16*)images, total8, S, P, (bf16*)cols);
-    if (int rc = check_launch("im2col")) return rc;
-    if (x) {
-        VTP_REQUIRE(cls_token && pos_embed && C > 0, VTP_ERR_NULL, "im2col: cls row needs cls_token and pos_embed");
-        const int G = S / P;
-        const long long row_stride = (long long)(G * G + 1) * C;
-        if (dtype == VTP_F32)
-            cls_row_kernel<float><<<B, 128, 0, st>>>((const float*)cls_token, (const float*)pos_embed, C,
-                                                     row_stride, (float*)x);
-        else
-            cls_row_kernel<bf16><<<B, 128, 0, st>>>((const bf16*)cls_token, (const bf16*)pos_embed, C, row_stride,
-                                                    (bf16*)x);
-        return check_launch("cls row");
-    }
-    return VTP_OK;
+    VTP_REQUIRE(!x || (cls_token && pos_embed && C > 0), VTP_ERR_NULL, "im2col: cls row needs cls_token and pos_embed");
+    const int G = S / P;
+    const long long row_stride = (long long)(G * G + 1) * C;
+    const int blocks = grid + (x ? B : 0);
+#define VTP_IM2COL8(I, T)                                                                                          \
+    launch_chain(im2col_kernel<I, T>, dim3(blocks), dim3(256), 0, st, (const I*)images, total8, S, P, (T*)cols, grid, \
+               ClsRows<T>{(const T*)cls_token, (const T*)pos_embed, C, row_stride, (T*)x, counts})
+    if (image_dtype == VTP_F32 && dtype == VTP_F32) VTP_IM2COL8(float, float);
+    else if (image_dtype == VTP_F32) VTP_IM2COL8(float, bf16);
+    else if (dtype == VTP_F32) VTP_IM2COL8(bf16, float);
+    else VTP_IM2COL8(bf16, bf16);
+#undef VTP_IM2COL8
+    return check_launch("im2col");
 }
+
+}  // namespace vtp

@@ -103,6 +103,7 @@ pool_kernel(const T* __restrict__ x, int B, int N, int C, int W, int num_extra,
             const int4* __restrict__ patches, const int32_t* __restrict__ n_dev, int n_max,
             T* __restrict__ comp, const float* __restrict__ lnw, const float* __restrict__ lnb,
             float eps, T* __restrict__ xn, T* __restrict__ qn, int mean, int* status) {
+    pdl_begin();
     constexpr int VN = Vec<T>::N;
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -191,6 +192,7 @@ __global__ void __launch_bounds__(256)
 unpool_kernel(const T* __restrict__ q, const T* __restrict__ comp, int B, int N, int C, int W,
               int num_extra, const int4* __restrict__ patches, const int32_t* __restrict__ n_dev,
               int n_max, const T* ref, T* out, int inv_area, int* status) {
+    pdl_begin();
     constexpr int VN = Vec<T>::N;
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -284,6 +286,7 @@ __global__ void __launch_bounds__(256)
 pool_any_c_kernel(const T* __restrict__ x, int B, int N, int C, int W, int num_extra,
                   const int4* __restrict__ patches, const int32_t* __restrict__ n_dev, int n_max,
                   T* __restrict__ comp, int mean, int* status) {
+    pdl_begin();
     int L = n_max;
     if (n_dev) L = min(__ldg(n_dev), n_max);
     const long long total = (long long)L * C;
@@ -312,6 +315,7 @@ __global__ void __launch_bounds__(256)
 unpool_any_c_kernel(const T* __restrict__ q, const T* __restrict__ comp, int B, int N, int C, int W, int num_extra,
                     const int4* __restrict__ patches, const int32_t* __restrict__ n_dev, int n_max,
                     const T* ref, T* out, int inv_area, int* status) {
+    pdl_begin();
     int L = n_max;
     if (n_dev) L = min(__ldg(n_dev), n_max);
     const long long total = (long long)L * C;
@@ -358,6 +362,7 @@ __global__ void __launch_bounds__(256)
 layernorm_kernel(const T* __restrict__ x, int rows_max, const int32_t* __restrict__ rows_dev, int C,
                  long long in_stride, const float* __restrict__ lnw, const float* __restrict__ lnb,
                  float eps, T* __restrict__ y, RowAdd add) {
+    pdl_begin();
     constexpr int VN = Vec<T>::N;
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -399,6 +404,7 @@ __global__ void __launch_bounds__(256)
 layernorm_narrow_kernel(const T* __restrict__ x, int rows_max, const int32_t* __restrict__ rows_dev, int C,
                         long long in_stride, const float* __restrict__ lnw, const float* __restrict__ lnb,
                         float eps, T* __restrict__ y, RowAdd add) {
+    pdl_begin();
     constexpr int VN = Vec<T>::N, RPW = 32 / G;
     const int lane = threadIdx.x & 31, sub = lane % G, grp = lane / G;
     const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -472,7 +478,7 @@ static int launch_pool(const void* x, int B, int N, int C, int W, int num_extra,
                        const float* lnb, float eps, void* xn, void* qn, int mean, cudaStream_t st) {
     if (C % Vec<T>::N != 0) {
         if (lnw) return fail(VTP_ERR_SHAPE, "pool: fused LayerNorm needs C=%d in whole 16-byte chunks", C);
-        pool_any_c_kernel<T><<<elem_grid((long long)n_max * C), 256, 0, st>>>(
+        launch_chain(pool_any_c_kernel<T>, dim3(elem_grid((long long)n_max * C)), dim3(256), 0, st, 
             (const T*)x, B, N, C, W, num_extra, (const int4*)patches, n_dev, n_max, (T*)comp, mean, device_status_ptr());
         return check_launch("pool");
     }
@@ -482,11 +488,11 @@ static int launch_pool(const void* x, int B, int N, int C, int W, int num_extra,
 #define VTP_POOL(M)                                                                                  \
     do {                                                                                             \
         if (ln)                                                                                      \
-            pool_kernel<T, M, true><<<grid, 256, 0, st>>>(                                           \
+            launch_chain(pool_kernel<T, M, true>, dim3(grid), dim3(256), 0, st,                                            \
                 (const T*)x, B, N, C, W, num_extra, (const int4*)patches, n_dev, n_max, (T*)comp, lnw,  \
                 lnb, eps, (T*)xn, (T*)qn, mean, device_status_ptr());                                \
         else                                                                                         \
-            pool_kernel<T, M, false><<<grid, 256, 0, st>>>(                                          \
+            launch_chain(pool_kernel<T, M, false>, dim3(grid), dim3(256), 0, st,                                           \
                 (const T*)x, B, N, C, W, num_extra, (const int4*)patches, n_dev, n_max, (T*)comp,    \
                 nullptr, nullptr, eps, nullptr, nullptr, mean, device_status_ptr());                 \
     } while (0)
@@ -505,7 +511,7 @@ static int launch_unpool(const void* q, const void* comp, int B, int N, int C, i
                          const int32_t* patches, const int32_t* n_dev, int n_max, const void* ref,
                          void* out, int inv_area, cudaStream_t st) {
     if (C % Vec<T>::N != 0) {
-        unpool_any_c_kernel<T><<<elem_grid((long long)n_max * C), 256, 0, st>>>(
+        launch_chain(unpool_any_c_kernel<T>, dim3(elem_grid((long long)n_max * C)), dim3(256), 0, st, 
             (const T*)q, (const T*)comp, B, N, C, W, num_extra, (const int4*)patches, n_dev, n_max, (const T*)ref,
             (T*)out, inv_area, device_status_ptr());
         return check_launch("unpool_add");
@@ -513,7 +519,7 @@ static int launch_unpool(const void* q, const void* comp, int B, int N, int C, i
     const int maxch = ceil_div(C / Vec<T>::N, 32);
     const int grid = row_grid(n_max);
 #define VTP_UNPOOL(M)                                                                           \
-    unpool_kernel<T, M><<<grid, 256, 0, st>>>((const T*)q, (const T*)comp, B, N, C, W, num_extra,  \
+    launch_chain(unpool_kernel<T, M>, dim3(grid), dim3(256), 0, st, (const T*)q, (const T*)comp, B, N, C, W, num_extra,  \
                                               (const int4*)patches, n_dev, n_max, (const T*)ref,      \
                                               (T*)out, inv_area, device_status_ptr())
     if (maxch <= 1) VTP_UNPOOL(1);
@@ -535,14 +541,14 @@ static int launch_ln(const void* x, int rows_max, const int32_t* rows_dev, int C
         const int rpw = nchunks <= 8 ? 4 : 2;
         const int g = row_grid(ceil_div(rows_max, rpw));
         if (nchunks <= 8)
-            layernorm_narrow_kernel<T, 8><<<g, 256, 0, st>>>((const T*)x, rows_max, rows_dev, C, stride, w, b, eps, (T*)y, add);
+            launch_chain(layernorm_narrow_kernel<T, 8>, dim3(g), dim3(256), 0, st, (const T*)x, rows_max, rows_dev, C, stride, w, b, eps, (T*)y, add);
         else
-            layernorm_narrow_kernel<T, 16><<<g, 256, 0, st>>>((const T*)x, rows_max, rows_dev, C, stride, w, b, eps, (T*)y, add);
+            launch_chain(layernorm_narrow_kernel<T, 16>, dim3(g), dim3(256), 0, st, (const T*)x, rows_max, rows_dev, C, stride, w, b, eps, (T*)y, add);
         return check_launch("layernorm");
     }
     const int grid = row_grid(rows_max);
 #define VTP_LN(M)                                                                                 \
-    layernorm_kernel<T, M><<<grid, 256, 0, st>>>((const T*)x, rows_max, rows_dev, C, stride, w, b, \
+    launch_chain(layernorm_kernel<T, M>, dim3(grid), dim3(256), 0, st, (const T*)x, rows_max, rows_dev, C, stride, w, b, \
                                                  eps, (T*)y, add)
     if (maxch <= 1) VTP_LN(1);
     else if (maxch == 2) VTP_LN(2);

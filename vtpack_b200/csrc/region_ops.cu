@@ -212,6 +212,7 @@ pool_region_kernel(const T* __restrict__ x, RegionGeom g, const int32_t* __restr
                    float2* __restrict__ stats_acc, int write_stats_x, const float* __restrict__ lnw,
                    const float* __restrict__ lnb, float eps, T* __restrict__ xn, T* __restrict__ qn, int sum_only,
                    int* status) {
+    pdl_begin();
     constexpr bool STATS = MODE == POOL_STATS, EXPLICIT_LN = MODE == POOL_LN;
     using L = Lay<T, G, CPL>;
     constexpr int VN = L::VN, GROUPS = L::GROUPS, TPG = L::TPG;
@@ -434,6 +435,7 @@ __global__ void __launch_bounds__(128, (Lay<T, G, CPL>::TPG * CPL <= 1) ? 16 : (
 unpool_region_kernel(const T* __restrict__ q, const T* __restrict__ comp, const T* ref, T* out, RegionGeom g,
                      const int32_t* __restrict__ idx, const int32_t* __restrict__ region_first,
                      const int32_t* __restrict__ offsets, Splits sp, NextBlock nx) {
+    pdl_begin();
     using L = Lay<T, G, CPL>;
     constexpr int VN = L::VN, GROUPS = L::GROUPS, TPG = L::TPG;
     extern __shared__ float part[];          // [4 grid rows][2 halves][C] row sums of the output (next gate)
@@ -547,7 +549,8 @@ __global__ void __launch_bounds__(128)
 gate_region_kernel(const T* __restrict__ x, RegionGeom g, const float* __restrict__ gw,
                    const float* __restrict__ gb, int S, float* __restrict__ logits_out,
                    int32_t* __restrict__ idx_out, float2* __restrict__ stats_x, float eps,
-                   const float* __restrict__ image_bias) {
+                   const float* __restrict__ image_bias, int32_t* __restrict__ counts, Splits sp) {
+    pdl_begin();
     using L = Lay<T, G, CPL>;
     constexpr int VN = L::VN, GROUPS = L::GROUPS, TPG = L::TPG;
     extern __shared__ float part[];          // [4][2][C]
@@ -591,9 +594,7 @@ gate_region_kernel(const T* __restrict__ x, RegionGeom g, const float* __restric
     }
     publish_partials<T, G, CPL>(part, acc, w, grp, sub, g.C);
     if (w != 0 || grp != 0) return;
-    Splits none;
-    none.n = 1; none.v[0] = 0;
-    gate_from_partials<T, G, CPL>(part, g.C, sub, gw, gb, S, logits_out, idx_out, rid, nullptr, none,
+    gate_from_partials<T, G, CPL>(part, g.C, sub, gw, gb, S, logits_out, idx_out, rid, counts ? counts + b : nullptr, sp,
                                   image_bias ? image_bias + (size_t)b * S : nullptr);
 }
 
@@ -614,16 +615,16 @@ static void launch_pool_t(const RegionPoolArgs& a, cudaStream_t st) {
     const int grid = a.g.B * R + ceil_div(a.g.B * a.g.num_extra, RG * (32 / G));
     const size_t smem = (size_t)8 * a.g.C * sizeof(float);
     if (a.stats_q)
-        pool_region_kernel<T, G, CPL, POOL_STATS><<<grid, 128, smem, st>>>(
+        launch_chain(pool_region_kernel<T, G, CPL, POOL_STATS>, dim3(grid), dim3(128), smem, st, 
             (const T*)a.x, a.g, a.idx, a.region_first, a.offsets, a.counts, a.offsets_out, a.region_first_out,
             a.counts_next, a.sp, (T*)a.comp, a.stats_x, a.stats_q, a.stats_acc, a.stats_x_ready ? 0 : 1, nullptr,
             nullptr, a.eps, nullptr, nullptr, 0, nullptr);
     else if (a.xn && a.qn)
-        pool_region_kernel<T, G, CPL, POOL_LN><<<grid, 128, smem, st>>>(
+        launch_chain(pool_region_kernel<T, G, CPL, POOL_LN>, dim3(grid), dim3(128), smem, st, 
             (const T*)a.x, a.g, a.idx, a.region_first, a.offsets, a.counts, a.offsets_out, a.region_first_out,
             a.counts_next, a.sp, (T*)a.comp, nullptr, nullptr, nullptr, 0, a.lnw, a.lnb, a.eps, (T*)a.xn, (T*)a.qn, 0, nullptr);
     else
-        pool_region_kernel<T, G, CPL, POOL_PLAIN><<<grid, 128, smem, st>>>(
+        launch_chain(pool_region_kernel<T, G, CPL, POOL_PLAIN>, dim3(grid), dim3(128), smem, st, 
             (const T*)a.x, a.g, a.idx, a.region_first, a.offsets, a.counts, a.offsets_out, a.region_first_out,
             a.counts_next, a.sp, (T*)a.comp, nullptr, nullptr, nullptr, 0, nullptr, nullptr, a.eps, nullptr, nullptr,
             a.sum_only ? 1 : 0, device_status_ptr());
@@ -633,7 +634,7 @@ template <typename T, int G, int CPL>
 static void launch_unpool_t(const RegionUnpoolArgs& a, cudaStream_t st) {
     const int R = a.g.Hr * a.g.Wr;
     const int grid = a.g.B * R + ceil_div(a.g.B * a.g.num_extra, RG * (32 / G));
-    unpool_region_kernel<T, G, CPL><<<grid, 128, (size_t)8 * a.g.C * sizeof(float), st>>>(
+    launch_chain(unpool_region_kernel<T, G, CPL>, dim3(grid), dim3(128), (size_t)8 * a.g.C * sizeof(float), st, 
         (const T*)a.q, (const T*)a.comp, (const T*)a.ref, (T*)a.out, a.g, a.idx, a.region_first, a.offsets, a.sp, a.next);
 }
 
@@ -641,8 +642,8 @@ template <typename T, int G, int CPL>
 static void launch_gate_t(const RegionGateArgs& a, cudaStream_t st) {
     const int R = a.g.Hr * a.g.Wr;
     const int grid = a.g.B * R + (a.stats_x ? ceil_div(a.g.B * a.g.num_extra, RG * (32 / G)) : 0);
-    gate_region_kernel<T, G, CPL><<<grid, 128, (size_t)8 * a.g.C * sizeof(float), st>>>(
-        (const T*)a.x, a.g, a.gw, a.gb, a.S, a.logits_out, a.idx_out, a.stats_x, a.eps, a.image_bias);
+    launch_chain(gate_region_kernel<T, G, CPL>, dim3(grid), dim3(128), (size_t)8 * a.g.C * sizeof(float), st, 
+        (const T*)a.x, a.g, a.gw, a.gb, a.S, a.logits_out, a.idx_out, a.stats_x, a.eps, a.image_bias, a.counts, a.sp);
 }
 
 #define VTP_DISPATCH_LAYOUT(FN, T, ARGS, ST)                                    \

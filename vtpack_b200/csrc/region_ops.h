@@ -63,6 +63,8 @@ struct RegionGateArgs {
     float* logits_out = nullptr; int32_t* idx_out = nullptr;
     float2* stats_x = nullptr; float eps = 1e-6f;     // optional: also the token rows' (mean, rstd)
     const float* image_bias = nullptr;                // [B, S] added to the logits of every region of image b, or null
+    // optional: per-image query counts, started at num_extra by an earlier kernel; every region adds its own
+    int32_t* counts = nullptr; Splits sp;
 };
 
 bool region_ops_supported(const RegionGeom& g, int dtype);
@@ -74,6 +76,11 @@ int region_gate(const RegionGateArgs& a, int dtype, cudaStream_t st);
 int index_to_patch(const void* indices, int idx_is_i64, const Splits& sp, int B, int Hr, int Wr, int region,
                    int num_extra, int32_t* counts, int32_t* offsets, int32_t* patches, int64_t* patches64,
                    int32_t* region_first, cudaStream_t st);
+
+// Per-image query counts of the grain indices `idx` [B, R]; with `logits` [B, R, n_splits] the indices are their
+// argmax (lowest index wins) and are written.  One warp per image.
+int count_queries(const float* logits, int32_t* idx, const Splits& sp, int B, int R, int num_extra, int32_t* counts,
+                  cudaStream_t st);
 
 int make_splits(Splits* sp, const int* splits, int n_splits, int region);
 

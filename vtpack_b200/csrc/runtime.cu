@@ -47,12 +47,6 @@ int sm_count() {
     return cached[dev];
 }
 
-bool pdl_enabled() {
-    static int cached = -1;
-    if (cached < 0) cached = getenv("VTP_PDL") ? 1 : 0;
-    return cached == 1;
-}
-
 __device__ int g_status_word = 0;
 
 int* device_status_ptr() {
