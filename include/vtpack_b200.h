@@ -468,6 +468,22 @@ int vtp_deit_dge_forward_ex(const vtp_dge_shape* s, const vtp_model_weights* m,
                             int32_t* counts_out, const vtp_forward_options* opt, void* workspace,
                             long long workspace_bytes, void* stream);
 
+/*
+ * One or more parts of the same forward, in order (FRONT, TRUNK, HEAD may come from separate calls with the
+ * same workspace and nothing else of this library using it in between).  TRUNK takes every address from the
+ * workspace, the weights and counts_out only, so a host can capture it into a CUDA graph once and replay it for
+ * images and logits at any address: FRONT (the one kernel that reads the images) and HEAD (the one that writes
+ * the logits) stay ordinary launches.  `images` is only needed by FRONT, `logits` only by HEAD; counts_out must be
+ * the same for FRONT and TRUNK.
+ */
+#define VTP_PART_FRONT 1u
+#define VTP_PART_TRUNK 2u
+#define VTP_PART_HEAD 4u
+int vtp_deit_dge_forward_part(const vtp_dge_shape* s, const vtp_model_weights* m,
+                              const vtp_block_weights* blocks, const void* images, float* logits,
+                              int32_t* counts_out, const vtp_forward_options* opt, unsigned parts,
+                              void* workspace, long long workspace_bytes, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -433,3 +433,52 @@ def test_pvt_model_other_input_size_and_pyramid(golden_dir):
         assert list(v.shape) == g[f"{k}_shape"].tolist(), k
         assert rel_err(v[:, :, ::8, ::8], torch.from_numpy(g[f"{k}_sub"])) < 1e-4, k
         assert abs(float(v.double().sum()) - float(g[f"{k}_sum"])) < 1e-4 * float(v.double().abs().sum()), k
+
+
+@pytest.mark.parametrize("kind", ["deit", "pvt"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_repeated_forwards_replay_one_capture(kind, dtype):
+    """The second forward of a shape captures the launches between the image kernel and the head, later ones replay
+    them: images and logits at other addresses, two batch sizes in turn, a larger batch that replaces the scratch
+    buffer and changed weights give bit for bit what a first (launch by launch) forward gives."""
+    from vtpack_b200 import _lib, synthetic
+    from vtpack_b200.models.dge.pvt_dge import pvt_dge_s124_tiny_256
+
+    def make(seed):
+        if kind == "deit":
+            m = synthetic.build_model("tiny", DEV, dtype, depth=2, seed=seed)
+        else:
+            m = pvt_dge_s124_tiny_256()
+            m.load_state_dict(O.make_pvt_state_dict(O.PVT_CONFIGS["tiny"], seed=seed), strict=True)
+            m = m.eval().to(device=DEV, dtype=dtype)
+        return m
+
+    def first(seed, img):                                    # a model that has never run before
+        m = make(seed)
+        return m(img), [c.clone() for c in m.last_counts]
+
+    def same(m, ref, img):
+        out = m(img)
+        assert torch.equal(out, ref[0])
+        assert all(torch.equal(a, b) for a, b in zip(m.last_counts, ref[1]))
+        return out
+
+    m = make(0)
+    imgs = {b: [O.make_images(b, 256, seed=b + k).to(DEV) for k in range(2)] for b in (1, 3)}
+    refs = {b: [first(0, i) for i in v] for b, v in imgs.items()}
+    kept = None
+    for _ in range(3):
+        for b in imgs:
+            for k in range(2):
+                out = same(m, refs[b][k], imgs[b][k].clone())
+                kept = out if kept is None else kept         # an earlier result is not overwritten
+    assert torch.equal(kept, refs[1][0][0])
+    big = O.make_images(40, 256, seed=9).to(DEV)
+    m(big)                                                   # may replace the scratch buffers
+    for _ in range(3):
+        same(m, refs[3][0], imgs[3][0])
+    m.load_state_dict(make(5).state_dict())
+    ref5 = first(5, imgs[3][1])
+    for _ in range(3):
+        same(m, ref5, imgs[3][1])
+    assert _lib.device_status() == 0

@@ -11,6 +11,7 @@ LIB_PATH = os.path.join(HERE, "libvtpack_b200.so")
 
 VTP_F32, VTP_BF16 = 0, 1
 FLAG_GELU, FLAG_OUT_F32, FLAG_CUDA_CORES = 1, 2, 4
+PART_FRONT, PART_TRUNK, PART_HEAD = 1, 2, 4
 # return codes (include/vtpack_b200.h) and the index-guard bit of the device status word
 ERR_NULL, ERR_SHAPE, ERR_DTYPE, ERR_ALIGN, ERR_UNSUPPORTED, ERR_DRIVER = -1, -2, -3, -4, -5, -6
 STATUS_BAD_INDEX = 64
@@ -110,6 +111,9 @@ PROTOTYPES = {
     "vtp_deit_dge_forward_ex": (c_int, [C.POINTER(DgeShape), C.POINTER(ModelWeights), C.POINTER(BlockWeights),
                                         c_void_p, c_void_p, c_void_p, C.POINTER(ForwardOptions), c_void_p, c_ll,
                                         c_void_p]),
+    "vtp_deit_dge_forward_part": (c_int, [C.POINTER(DgeShape), C.POINTER(ModelWeights), C.POINTER(BlockWeights),
+                                          c_void_p, c_void_p, c_void_p, C.POINTER(ForwardOptions), c_uint, c_void_p,
+                                          c_ll, c_void_p]),
 }
 
 _lib = None

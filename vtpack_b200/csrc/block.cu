@@ -399,6 +399,51 @@ static ModelScratch carve_model(const vtp_dge_shape& s, const vtp_model_weights&
     return r;
 }
 
+// Patch embedding Linear, blocks and final LayerNorm: everything between the im2col and the head.
+static int deit_trunk(const vtp_dge_shape& s, const vtp_model_weights& m, const vtp_block_weights* blocks,
+                      int32_t* counts_out, const vtp_forward_options* opt, const ModelScratch& ms, const BlockScratch& bs,
+                      cudaStream_t st) {
+    const int HW = s.H * s.W, N = HW + 1, C = s.C;
+    const int KP = 3 * m.patch * m.patch;
+    const long long e = (long long)elem_size(s.dtype);
+    int rc;
+    LinearArgs pe;   // token (b, 1+t) = cols(b,t) Wp^T + bias + pos_embed[1+t]
+    pe.a = ms.cols; pe.lda = KP; pe.w = m.patch_w; pe.bias = m.patch_b; pe.res = m.pos_embed; pe.ldr = C;
+    pe.y = ms.x; pe.ldy = C; pe.dtype = s.dtype; pe.m_max = s.B * HW; pe.N = C; pe.K = KP;
+    pe.flags = s.flags & VTP_FLAG_CUDA_CORES;
+    pe.out_grp = HW; pe.out_skip = 1; pe.res_mod = HW; pe.res_off = 1;
+    if ((rc = linear(pe, st))) return rc;
+    bool chained = false;      // block i-1's unpool prepared block i's gate
+    const long long R = (long long)(s.H / s.region) * (s.W / s.region);
+    for (int i = 0; i < m.depth; ++i) {
+        BlockChain chain;
+        chain.have_gate = chained;
+        chain.parity = i & 1;
+        chain.next = (i + 1 < m.depth) ? &blocks[i + 1] : nullptr;
+        chain.counts_next = (counts_out && chain.next) ? counts_out + (size_t)(i + 1) * s.B : nullptr;
+        chain.counts_started = i == 0;
+        chain.image_bias = opt ? opt->gate_image_bias : nullptr;
+        if (opt && opt->tokens_trace) {
+            const size_t nb = (size_t)s.B * N * C * e;
+            const cudaError_t ce = cudaMemcpyAsync(static_cast<char*>(opt->tokens_trace) + (size_t)i * nb, ms.x, nb,
+                                                   cudaMemcpyDeviceToDevice, st);
+            if (ce != cudaSuccess) return fail((int)ce, "model: tokens trace copy: %s", cudaGetErrorString(ce));
+        }
+        rc = block_forward(s, blocks[i], ms.x, ms.x, nullptr, counts_out ? counts_out + (size_t)i * s.B : nullptr,
+                           ms.block_ws, st, StageMarks(), chain);
+        if (rc) return rc;
+        if (opt && opt->grain_trace) {
+            // the block's grain indices stay in its slot of the scratch (its unpool writes the other slot)
+            const size_t nb = (size_t)s.B * R * sizeof(int32_t);
+            const cudaError_t ce = cudaMemcpyAsync(opt->grain_trace + (size_t)i * s.B * R, bs.idx[i & 1], nb,
+                                                   cudaMemcpyDeviceToDevice, st);
+            if (ce != cudaSuccess) return fail((int)ce, "model: grain trace copy: %s", cudaGetErrorString(ce));
+        }
+        chained = chain.next && block_folds(s, blocks[i]) && block_folds(s, *chain.next);
+    }
+    return vtp_layernorm(ms.x, s.dtype, s.B, nullptr, C, (long long)N * C, m.norm_w, m.norm_b, s.eps, ms.cls_n, st);
+}
+
 }  // namespace vtp
 
 using namespace vtp;
@@ -487,8 +532,18 @@ extern "C" int vtp_deit_dge_forward_ex(const vtp_dge_shape* s, const vtp_model_w
                                        const vtp_block_weights* blocks, const void* images, float* logits,
                                        int32_t* counts_out, const vtp_forward_options* opt, void* workspace,
                                        long long workspace_bytes, void* stream) {
+    return vtp_deit_dge_forward_part(s, m, blocks, images, logits, counts_out, opt,
+                                     VTP_PART_FRONT | VTP_PART_TRUNK | VTP_PART_HEAD, workspace, workspace_bytes, stream);
+}
+
+extern "C" int vtp_deit_dge_forward_part(const vtp_dge_shape* s, const vtp_model_weights* m,
+                                         const vtp_block_weights* blocks, const void* images, float* logits,
+                                         int32_t* counts_out, const vtp_forward_options* opt, unsigned parts,
+                                         void* workspace, long long workspace_bytes, void* stream) {
     if (int rc = check_shape(s)) return rc;
-    VTP_REQUIRE(m && blocks && images && logits && workspace, VTP_ERR_NULL, "model: null pointer");
+    VTP_REQUIRE(m && blocks && workspace, VTP_ERR_NULL, "model: null pointer");
+    VTP_REQUIRE(parts != 0 && (parts & ~7u) == 0, VTP_ERR_SHAPE, "model: parts %u", parts);
+    VTP_REQUIRE((images || !(parts & VTP_PART_FRONT)) && (logits || !(parts & VTP_PART_HEAD)), VTP_ERR_NULL, "model: null pointer");
     VTP_REQUIRE(m->depth > 0 && m->patch > 0 && m->num_classes > 0, VTP_ERR_SHAPE, "model: bad shape");
     VTP_REQUIRE(m->img_size == s->H * m->patch && s->H == s->W && s->num_extra == 1, VTP_ERR_SHAPE,
                 "model: image %d does not match a %dx%d grid of %d-pixel patches with one cls token",
@@ -498,50 +553,19 @@ extern "C" int vtp_deit_dge_forward_ex(const vtp_dge_shape* s, const vtp_model_w
     VTP_REQUIRE(workspace_bytes >= ms.bytes, VTP_ERR_SHAPE, "model: workspace of %lld bytes, %lld needed",
                 workspace_bytes, ms.bytes);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int HW = s->H * s->W, N = HW + 1, C = s->C;
-    const int KP = 3 * m->patch * m->patch;
-    const long long e = (long long)elem_size(s->dtype);
+    const int C = s->C, KP = 3 * m->patch * m->patch;
     const BlockScratch bs = carve_block(*s, ms.block_ws);
-    // (the kernel that writes the cls rows also starts the first block's query counts)
-    int rc = patch_im2col(images, m->image_dtype, s->B, m->img_size, m->patch, s->dtype, ms.cols, 3 * m->patch * m->patch,
-                          m->cls_token, m->pos_embed, C, ms.x, counts_out ? counts_out : bs.counts[0], st);
-    if (rc) return rc;
-    LinearArgs pe;   // token (b, 1+t) = cols(b,t) Wp^T + bias + pos_embed[1+t]
-    pe.a = ms.cols; pe.lda = KP; pe.w = m->patch_w; pe.bias = m->patch_b; pe.res = m->pos_embed; pe.ldr = C;
-    pe.y = ms.x; pe.ldy = C; pe.dtype = s->dtype; pe.m_max = s->B * HW; pe.N = C; pe.K = KP;
-    pe.flags = s->flags & VTP_FLAG_CUDA_CORES;
-    pe.out_grp = HW; pe.out_skip = 1; pe.res_mod = HW; pe.res_off = 1;
-    if ((rc = linear(pe, st))) return rc;
-    bool chained = false;      // block i-1's unpool prepared block i's gate
-    const long long R = (long long)(s->H / s->region) * (s->W / s->region);
-    for (int i = 0; i < m->depth; ++i) {
-        BlockChain chain;
-        chain.have_gate = chained;
-        chain.parity = i & 1;
-        chain.next = (i + 1 < m->depth) ? &blocks[i + 1] : nullptr;
-        chain.counts_next = (counts_out && chain.next) ? counts_out + (size_t)(i + 1) * s->B : nullptr;
-        chain.counts_started = i == 0;
-        chain.image_bias = opt ? opt->gate_image_bias : nullptr;
-        if (opt && opt->tokens_trace) {
-            const size_t nb = (size_t)s->B * N * C * e;
-            const cudaError_t ce = cudaMemcpyAsync(static_cast<char*>(opt->tokens_trace) + (size_t)i * nb, ms.x, nb,
-                                                   cudaMemcpyDeviceToDevice, st);
-            if (ce != cudaSuccess) return fail((int)ce, "model: tokens trace copy: %s", cudaGetErrorString(ce));
-        }
-        rc = block_forward(*s, blocks[i], ms.x, ms.x, nullptr, counts_out ? counts_out + (size_t)i * s->B : nullptr,
-                           ms.block_ws, st, StageMarks(), chain);
+    int rc = VTP_OK;
+    if (parts & VTP_PART_FRONT) {
+        // (the kernel that writes the cls rows also starts the first block's query counts)
+        rc = patch_im2col(images, m->image_dtype, s->B, m->img_size, m->patch, s->dtype, ms.cols, KP, m->cls_token,
+                          m->pos_embed, C, ms.x, counts_out ? counts_out : bs.counts[0], st);
         if (rc) return rc;
-        if (opt && opt->grain_trace) {
-            // the block's grain indices stay in its slot of the scratch (its unpool writes the other slot)
-            const size_t nb = (size_t)s->B * R * sizeof(int32_t);
-            const cudaError_t ce = cudaMemcpyAsync(opt->grain_trace + (size_t)i * s->B * R, bs.idx[i & 1], nb,
-                                                   cudaMemcpyDeviceToDevice, st);
-            if (ce != cudaSuccess) return fail((int)ce, "model: grain trace copy: %s", cudaGetErrorString(ce));
-        }
-        chained = chain.next && block_folds(*s, blocks[i]) && block_folds(*s, *chain.next);
     }
-    rc = vtp_layernorm(ms.x, s->dtype, s->B, nullptr, C, (long long)N * C, m->norm_w, m->norm_b, s->eps, ms.cls_n, st);
-    if (rc) return rc;
+    if (parts & VTP_PART_TRUNK) {
+        if ((rc = deit_trunk(*s, *m, blocks, counts_out, opt, ms, bs, st))) return rc;
+    }
+    if (!(parts & VTP_PART_HEAD)) return VTP_OK;
     LinearArgs hd;
     hd.a = ms.cls_n; hd.lda = C; hd.w = m->head_w; hd.bias = m->head_b; hd.y = logits; hd.ldy = m->num_classes;
     hd.dtype = s->dtype; hd.m_max = s->B; hd.N = m->num_classes; hd.K = C;

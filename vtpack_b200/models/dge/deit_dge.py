@@ -21,7 +21,8 @@ import torch.nn as nn
 
 from ... import _lib
 from ...layers import DynamicGrainedEncoder, batched_sparse_attention, batched_sparse_gemm
-from ...runtime import dtype_code, ptr, require_cuda, scratch, scratch_generation, stream_ptr
+from ...runtime import (LaunchPlans, ParamWatch, capture_launches, dtype_code, ptr, require_cuda, scratch,
+                        scratch_generation, stream_ptr)
 
 __all__ = [
     "deit_dge_s124_tiny_patch16_256", "deit_dge_s124_small_patch16_256",
@@ -164,10 +165,17 @@ class _WeightPack:
         self.key = None
         self.tensors = None
         self.struct = None
+        self.watch = None
+
+    def __reduce__(self):                     # addresses mean nothing to a copy of the module
+        return (_WeightPack, ())
 
 
 def _param_key(mod: nn.Module, dtype):
-    return (dtype, getattr(mod, "fold_layernorm", None), getattr(mod, "fold_q_fc1", None)) + tuple((p.data_ptr(), p._version, p.dtype) for p in mod.parameters())
+    pk = mod._pack
+    if pk.watch is None:
+        pk.watch = ParamWatch(mod)
+    return (dtype, getattr(mod, "fold_layernorm", None), getattr(mod, "fold_q_fc1", None), pk.watch.generation())
 
 
 def _pack_block(blk, dtype) -> _lib.BlockWeights:
@@ -366,6 +374,7 @@ class VisionTransformer(nn.Module):
         self.flags = 0
         self.fold_layernorm = True
         self._pack = _WeightPack()
+        self._plans = LaunchPlans()
         self._graphs = {}
         self.last_counts = None
         # eval-mode options of the fused forward (vtp_forward_options):
@@ -425,6 +434,7 @@ class VisionTransformer(nn.Module):
                 blocks[i] = _pack_block(blk, dtype)
             pk.key, pk.tensors, pk.struct = key, t, (m, blocks)
             self._graphs.clear()        # captured graphs hold the addresses of the previous pack
+            self._plans.clear()
         return pk.struct
 
     def forward_graph(self, x, logits_out):
@@ -439,6 +449,9 @@ class VisionTransformer(nn.Module):
         differentiable op-by-op sequence in the parameters' dtype."""
         if self.training:
             return self._forward_train(x)
+        return self._forward_eval(x, logits_out)
+
+    def _forward_eval(self, x, logits_out=None, use_plans=True):
         require_cuda(x)
         if x.dtype not in (torch.float32, torch.bfloat16):
             x = x.float()
@@ -456,7 +469,6 @@ class VisionTransformer(nn.Module):
         ws = scratch(x.device, nbytes)
         logits = logits_out if logits_out is not None else torch.empty(
             B, self.num_classes, dtype=torch.float32, device=x.device)
-        counts = torch.empty(self.depth, B, dtype=torch.int32, device=x.device)
         opt = _lib.ForwardOptions()
         if self.gate_image_bias is not None:
             bias = self.gate_image_bias
@@ -464,26 +476,53 @@ class VisionTransformer(nn.Module):
                     or tuple(bias.shape) != (B, len(self.split_sizes))):
                 raise ValueError("gate_image_bias must be a contiguous fp32 CUDA tensor [B, n_splits]")
             opt.gate_image_bias = bias.data_ptr()
-        if self.trace:
-            if self.trace != "grains":
-                self.last_tokens = torch.empty(self.depth, B, G * G + 1, self.embed_dim, dtype=dtype,
+
+        def launch(parts, counts, stream):
+            _lib.check(lib.vtp_deit_dge_forward_part(
+                ctypes.byref(s), ctypes.byref(m), blocks, ptr(x), ptr(logits), ptr(counts), ctypes.byref(opt), parts,
+                ptr(ws), nbytes, stream))
+
+        stream = stream_ptr(x.device)
+        plan = None
+        if use_plans and not self.trace:
+            plan = self._plans.get((B, opt.gate_image_bias, int(self.flags)),
+                                   lambda p: p.scratch_gen == scratch_generation(x.device),
+                                   lambda: self._capture_trunk(launch, ws, B, x.device))
+        if plan is not None:
+            # the one kernel that reads the images and the one that writes the logits are ordinary launches; what
+            # lies between them takes its addresses from the workspace and the weights and is replayed
+            launch(_lib.PART_FRONT, plan.counts, stream)
+            plan.graph.replay()
+            launch(_lib.PART_HEAD, plan.counts, stream)
+            counts = plan.counts.clone()
+        else:
+            counts = torch.empty(self.depth, B, dtype=torch.int32, device=x.device)
+            if self.trace:
+                if self.trace != "grains":
+                    self.last_tokens = torch.empty(self.depth, B, G * G + 1, self.embed_dim, dtype=dtype,
+                                                   device=x.device)
+                self.last_grains = torch.empty(self.depth, B, (G // max(self.split_sizes)) ** 2, dtype=torch.int32,
                                                device=x.device)
-            self.last_grains = torch.empty(self.depth, B, (G // max(self.split_sizes)) ** 2, dtype=torch.int32,
-                                           device=x.device)
-            opt.grain_trace = self.last_grains.data_ptr()
-            if self.trace != "grains":
-                opt.tokens_trace = self.last_tokens.data_ptr()
-        _lib.check(lib.vtp_deit_dge_forward_ex(ctypes.byref(s), ctypes.byref(m), blocks, ptr(x), ptr(logits),
-                                               ptr(counts), ctypes.byref(opt), ptr(ws), nbytes,
-                                               stream_ptr(x.device)))
+                opt.grain_trace = self.last_grains.data_ptr()
+                if self.trace != "grains":
+                    opt.tokens_trace = self.last_tokens.data_ptr()
+            launch(_lib.PART_FRONT | _lib.PART_TRUNK | _lib.PART_HEAD, counts, stream)
         self.last_counts = counts
         # what get_complexity() of each block's encoder needs (dge.py:40-59): shapes only, and the
         # per-image query counts, which stay on the device
         tokens = torch.empty(0, device=x.device).expand(B, G * G + 1, 0)
-        for i, blk in enumerate(self.blocks):
-            blk.dge.states.update({"batches_device": counts[i], "input": tokens, "gate": None, "size": (G, G),
+        for blk, blk_counts in zip(self.blocks, counts.unbind(0)):
+            blk.dge.states.update({"batches_device": blk_counts, "input": tokens, "gate": None, "size": (G, G),
                                    "num_extra_tokens": 1})
         return logits
+
+    def _capture_trunk(self, launch, ws, B, device):
+        counts = torch.empty(self.depth, B, dtype=torch.int32, device=device)
+        graph = capture_launches(device, lambda stream: launch(_lib.PART_TRUNK, counts, stream))
+        keep = (ws, counts, self.gate_image_bias, self._pack.tensors, [blk._pack.tensors for blk in self.blocks])
+        plan = _CapturedForward(graph, keep, scratch_generation(device))
+        plan.counts = counts
+        return plan
 
     def _forward_train(self, x):
         """``deit_dge.py:267-299`` with ``self.training`` (cls token, no distillation token)."""
@@ -538,12 +577,12 @@ def _graph_forward(model, x, logits_out):
         side.wait_stream(cur)
         with torch.cuda.stream(side):          # warm-up outside capture: scratch, attributes, weight packs
             for _ in range(2):
-                model.forward(x, logits_out)
+                model._forward_eval(x, logits_out, use_plans=False)
         cur.wait_stream(side)
         torch.cuda.synchronize(x.device)
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
-            model.forward(x, logits_out)
+            model._forward_eval(x, logits_out, use_plans=False)
         keep = (x, logits_out, bias, model._pack.tensors, [blk._pack.tensors for blk in model.blocks],
                 scratch(x.device, 1), model.last_counts, model.last_tokens, model.last_grains)
         g = _CapturedForward(graph, keep, scratch_generation(x.device))

@@ -18,8 +18,9 @@ import torch.nn as nn
 
 from ... import _lib
 from ...layers import DynamicGrainedEncoder, batched_sparse_attention, batched_sparse_gemm
-from ...runtime import dtype_code, ptr, require_cuda, scratch, scratch_generation, stream_ptr
-from .deit_dge import DropPath, Mlp, _WeightPack, _pack_block, _shape_struct
+from ...runtime import (LaunchPlans, ParamWatch, capture_launches, dtype_code, ptr, require_cuda, scratch,
+                        scratch_generation, stream_ptr)
+from .deit_dge import DropPath, Mlp, _CapturedForward, _WeightPack, _pack_block, _shape_struct
 
 __all__ = ["Mlp", "Attention", "Block", "PatchEmbed", "PyramidVisionTransformer",
            "pvt_dge_s124_tiny_256", "pvt_dge_s124_small_256", "pvt_dge_s124_medium_256", "pvt_dge_s124_large_256"]
@@ -155,8 +156,22 @@ def stage_forward(blocks, x, H, W):
     require_cuda(x)
     x = x.contiguous()
     B, N, C = x.shape
+    out = torch.empty_like(x)
+    counts = torch.empty(len(blocks), B, dtype=torch.int32, device=x.device)
+    _launch_stage(blocks, x.dtype, B, N, H, W, ptr(x), ptr(out), ptr(counts), x.device, stream_ptr(x.device))
+    for i, blk in enumerate(blocks):
+        # (the input of a block after the first is overwritten in place; the complexity accounting only takes
+        # its shape, which the stage's output buffer has too)
+        blk.dge.states.update({"batches_device": counts[i], "input": x if i == 0 else out, "gate": None,
+                               "size": (H, W), "num_extra_tokens": N - H * W})
+    return out
+
+
+def _launch_stage(blocks, dtype, B, N, H, W, x_ptr, out_ptr, counts_ptr, device, stream):
+    """The launches of a stage's blocks: tokens at ``x_ptr`` [B, N, C] -> ``out_ptr`` (which may be ``x_ptr``), per-image
+    query counts of every block at ``counts_ptr`` int32 [blocks, B]."""
     b0 = blocks[0]
-    s = _shape_struct(x.dtype, B, H, W, N - H * W, C, b0.attn.num_heads, b0.mlp.fc1.out_features,
+    s = _shape_struct(dtype, B, H, W, N - H * W, b0.dim, b0.attn.num_heads, b0.mlp.fc1.out_features,
                       b0.split_sizes, b0.norm1.eps, b0.flags, b0.attn.scale)
     if b0.attn.sr_ratio > 1:
         s.sr_ratio = b0.attn.sr_ratio
@@ -164,24 +179,16 @@ def stage_forward(blocks, x, H, W):
     for blk in blocks[1:]:
         same = (blk.attn.num_heads == b0.attn.num_heads and blk.mlp.fc1.out_features == b0.mlp.fc1.out_features
                 and blk.split_sizes == b0.split_sizes and blk.norm1.eps == b0.norm1.eps and blk.flags == b0.flags
-                and blk.attn.scale == b0.attn.scale and blk.attn.sr_ratio == b0.attn.sr_ratio)
+                and blk.attn.scale == b0.attn.scale and blk.attn.sr_ratio == b0.attn.sr_ratio and blk.dim == b0.dim)
         if not same:
             raise ValueError("stage_forward: the blocks of a stage must share one shape")
-    packs = (_lib.BlockWeights * len(blocks))(*[_pack_block(blk, x.dtype) for blk in blocks])
+    packs = (_lib.BlockWeights * len(blocks))(*[_pack_block(blk, dtype) for blk in blocks])
     lib = _lib.lib()
     nbytes = lib.vtp_block_workspace_bytes(ctypes.byref(s))
     _lib.check(0 if nbytes >= 0 else int(nbytes))
-    ws = scratch(x.device, nbytes)
-    out = torch.empty_like(x)
-    counts = torch.empty(len(blocks), B, dtype=torch.int32, device=x.device)
-    _lib.check(lib.vtp_dge_blocks_forward(ctypes.byref(s), packs, len(blocks), ptr(x), ptr(out), ptr(counts), ptr(ws),
-                                          nbytes, stream_ptr(x.device)))
-    for i, blk in enumerate(blocks):
-        # (the input of a block after the first is overwritten in place; the complexity accounting only takes
-        # its shape, which the stage's output buffer has too)
-        blk.dge.states.update({"batches_device": counts[i], "input": x if i == 0 else out, "gate": None,
-                               "size": (H, W), "num_extra_tokens": N - H * W})
-    return out
+    ws = scratch(device, nbytes)
+    _lib.check(lib.vtp_dge_blocks_forward(ctypes.byref(s), packs, len(blocks), x_ptr, out_ptr, counts_ptr, ptr(ws),
+                                          nbytes, stream))
 
 
 class PatchEmbed(nn.Module):
@@ -209,24 +216,11 @@ class PatchEmbed(nn.Module):
         return comp
 
 
-def _matmul_rows(cols, weight, bias, flags=0, out_dtype=None):
-    """cols [M, K] x weight [N, K]^T + bias through vtp_linear."""
-    M, K = cols.shape
-    N = weight.shape[0]
-    y = torch.empty(M, N, dtype=out_dtype or cols.dtype, device=cols.device)
-    b = None if bias is None else bias.detach().float().contiguous()
-    _lib.check(_lib.lib().vtp_linear(ptr(cols), K, ptr(weight), ptr(b), None, 0, ptr(y), N, dtype_code(cols.dtype), M,
-                                     None, N, K, flags, stream_ptr(cols.device)))
-    return y
-
-
-def _norm_rows(x, rows, C, row_stride, ln, eps=None, wb=None):
-    y = torch.empty(rows, C, dtype=x.dtype, device=x.device)
-    # both fp32 copies must be alive together: a temporary freed between the two would hand its memory to the other
-    w, b = wb if wb is not None else (ln.weight.detach().float().contiguous(), ln.bias.detach().float().contiguous())
-    _lib.check(_lib.lib().vtp_layernorm(ptr(x), dtype_code(x.dtype), rows, None, C, row_stride, ptr(w), ptr(b),
-                                        float(ln.eps if eps is None else eps), ptr(y), stream_ptr(x.device)))
-    return y
+def _launch_linear(cols, weight, bias, out, rows, flags, stream):
+    """out [rows, N] = cols [rows, K] x weight [N, K]^T + bias through vtp_linear; cols and out are addresses."""
+    N, K = weight.shape
+    _lib.check(_lib.lib().vtp_linear(cols, K, ptr(weight), ptr(bias), None, 0, out, N, dtype_code(weight.dtype), rows,
+                                     None, N, K, flags, stream))
 
 
 class PyramidVisionTransformer(nn.Module):
@@ -277,6 +271,9 @@ class PyramidVisionTransformer(nn.Module):
             elif isinstance(m, DynamicGrainedEncoder):
                 m.router.init_parameters()
         self.last_counts = None
+        self._pack = _WeightPack()
+        self._plans = LaunchPlans(4)
+        self._graph = None
 
     def _const(self, name, sources, make, extra=()):
         """A tensor derived from parameters only (a weight matrix in GEMM layout and dtype, fp32 copies of bias and
@@ -299,23 +296,22 @@ class PyramidVisionTransformer(nn.Module):
         has changed, when the per-device scratch buffer has been replaced, or for another input buffer."""
         if self.training:
             raise RuntimeError("forward_graph is an eval-mode path")
-        key = (x.data_ptr(), tuple(x.shape), x.dtype,
-               tuple((p.data_ptr(), p._version) for p in self.parameters()))
-        g = getattr(self, "_graph", None)
-        if g is None or g["key"] != key or g["scratch_gen"] != scratch_generation(x.device):
+        key = (x.data_ptr(), tuple(x.shape), x.dtype, self._param_generation())
+        g = self._graph
+        if g is None or g["key"] != key or g["scratch_gen"] != self._scratch_gen(x.device):
             cur = torch.cuda.current_stream(x.device)
             side = torch.cuda.Stream(x.device)
             side.wait_stream(cur)
             with torch.cuda.stream(side):          # warm-up outside capture: scratch, attributes, weight packs
                 for _ in range(2):
-                    self.forward(x)
+                    self._forward_eval(x, use_plans=False)
             cur.wait_stream(side)
             torch.cuda.synchronize(x.device)
             graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(graph):
-                out = self.forward(x)
+                out = self._forward_eval(x, use_plans=False)
             g = {"key": key, "graph": graph, "out": out, "counts": self.last_counts, "x": x,
-                 "scratch": scratch(x.device, 1), "scratch_gen": scratch_generation(x.device)}
+                 "keep": self._keep(x.device), "scratch_gen": self._scratch_gen(x.device)}
             self._graph = g
         g["graph"].replay()
         self.last_counts = g["counts"]
@@ -367,87 +363,185 @@ class PyramidVisionTransformer(nn.Module):
         regions and reduction windows.  In training mode: the differentiable op-by-op sequence."""
         if self.training:
             return self._forward_train(x)
+        return self._forward_eval(x)
+
+    def _param_generation(self):
+        if self._pack.watch is None:
+            self._pack.watch = ParamWatch(self)
+        return self._pack.watch.generation()
+
+    def _scratch_gen(self, device):
+        return scratch_generation(device), scratch_generation(device, "pvt")
+
+    def _keep(self, device):
+        """What a captured forward holds the addresses of."""
+        packs = [blk._pack.tensors for i in range(self.num_stages) for blk in getattr(self, f"block{i + 1}")]
+        return (scratch(device, 1), scratch(device, 1, "pvt"), dict(self.__dict__.get("_consts", {})), packs)
+
+    def _grids(self, S):
+        """Token grid side of every stage for S x S images."""
+        P = self.patch_embed1.patch_size[0]
+        if S % P:
+            raise ValueError(f"input size {S} is not a multiple of the patch size {P}")
+        sides = [S // P]
+        for i in range(1, self.num_stages):
+            sides.append(sides[-1] // getattr(self, f"patch_embed{i + 1}").patch_size[0])
+        return sides
+
+    def _forward_eval(self, x, use_plans=True):
+        """The stages' launches with every intermediate in per-device scratch buffers: cols (im2col rows of a stage's
+        embedding), y (its Linear), tokens (its rows, in place through the blocks).  Between the first kernel,
+        which reads the images, and the last, which writes the logits, no address depends on the call."""
         require_cuda(x)
         if x.dtype not in (torch.float32, torch.bfloat16):
             x = x.float()
         x = x.contiguous()
         B, _, S, _ = x.shape
-        dtype = self.cls_token.dtype
-        lib, st = _lib.lib(), stream_ptr(x.device)
-        counts, outputs = [], {}
-        tokens, H, W = None, 0, 0
-        for i in range(self.num_stages):
-            pe = getattr(self, f"patch_embed{i + 1}")
-            pos_full = getattr(self, f"pos_embed{i + 1}").detach()
-            C = self.embed_dims[i]
-            P = pe.patch_size[0]
-            if i == 0:
-                if S % P:
-                    raise ValueError(f"input size {S} is not a multiple of the patch size {P}")
-                H = W = S // P
-                KP = 3 * P * P
-                padded = dtype == torch.bfloat16 and P % 8 != 0 and KP % 64 != 0
-                ld = (KP + 63) // 64 * 64 if padded else KP
-                wm = self._const(f"wm{i}", (pe.proj.weight,), lambda: torch.nn.functional.pad(
-                    pe.proj.weight.detach().reshape(C, -1).to(dtype), (0, ld - KP)).contiguous(), (dtype, ld))
-                if padded:
-                    # 48 columns: pad the reduction to a whole 64-element block (zero columns in the rows and in
-                    # the weight), which takes the GEMM from the CUDA-core kernel to the tensor-core one
-                    cols = torch.empty(B * H * W, ld, dtype=dtype, device=x.device)
-                    _lib.check(lib.vtp_patch_im2col_padded(ptr(x), dtype_code(x.dtype), B, S, P, dtype_code(dtype),
-                                                           ptr(cols), ld, st))
-                else:
-                    cols = torch.empty(B * H * W, KP, dtype=dtype, device=x.device)
-                    _lib.check(lib.vtp_patch_im2col(ptr(x), dtype_code(x.dtype), B, S, P, dtype_code(dtype), ptr(cols),
-                                                    None, None, C, None, st))
+        dev, dtype = x.device, self.cls_token.dtype
+        sides = self._grids(S)
+        e = x.new_empty(0, dtype=dtype).element_size()
+        P = self.patch_embed1.patch_size[0]
+        KP = 3 * P * P
+        # 48 columns: pad the reduction to a whole 64-element block (zero columns in the rows and in
+        # the weight), which takes the GEMM from the CUDA-core kernel to the tensor-core one
+        padded = dtype == torch.bfloat16 and P % 8 != 0 and KP % 64 != 0
+        ld = (KP + 63) // 64 * 64 if padded else KP
+        cols_n, rows_n = B * sides[0] ** 2 * ld, 0
+        for i, side in enumerate(sides):
+            rows_n = max(rows_n, B * (side * side + 1) * self.embed_dims[i])
+            if i > 0:
+                cols_n = max(cols_n, B * sides[i - 1] ** 2 * self.embed_dims[i - 1])
+        up = lambda n: (n * e + 255) // 256 * 256      # noqa: E731
+        arena = scratch(dev, up(cols_n) + 2 * up(rows_n), "pvt")
+        cols = arena.data_ptr()
+        y = cols + up(cols_n)
+        tokens = y + up(rows_n)
+        lib, stream = _lib.lib(), stream_ptr(dev)
+
+        def front():
+            if padded:
+                _lib.check(lib.vtp_patch_im2col_padded(ptr(x), dtype_code(x.dtype), B, S, P, dtype_code(dtype), cols, ld,
+                                                       stream))
             else:
-                cols = torch.empty(B * (H // P) * (W // P), P * P * tokens.shape[-1], dtype=dtype, device=x.device)
-                _lib.check(lib.vtp_token_im2col(ptr(tokens), dtype_code(dtype), B, H, W, tokens.shape[-1], P, ptr(cols), st))
-                H, W = H // P, W // P
-                wm = self._const(f"wm{i}", (pe.proj.weight,), lambda: pe.proj.weight.detach().permute(0, 2, 3, 1)
-                                 .reshape(C, -1).to(dtype).contiguous(), (dtype,))
-            bias = self._const(f"eb{i}", (pe.proj.bias,), lambda: pe.proj.bias.detach().float().contiguous())
-            wb = self._const(f"en{i}", (pe.norm.weight, pe.norm.bias), lambda: (
-                pe.norm.weight.detach().float().contiguous(), pe.norm.bias.detach().float().contiguous()))
-            y = _matmul_rows(cols, wm, bias)
-            HW = H * W
-            last = i == self.num_stages - 1
-            # the stage's position rows ([cls row;] grid rows), resized when the grid is not the trained one
-            def make_pos(pos_full=pos_full, pe=pe, H=H, W=W, last=last):
-                if last:
-                    pos = torch.cat((pos_full[:, 0:1], self._stage_pos_embed(pos_full[:, 1:], pe, H, W)), dim=1)
-                else:
-                    pos = self._stage_pos_embed(pos_full, pe, H, W)
-                return pos[0].to(dtype).contiguous()
-            pos = self._const(f"pos{i}", (getattr(self, f"pos_embed{i + 1}"),), make_pos, (dtype, H, W))
-            tokens = torch.empty(B, HW + (1 if last else 0), C, dtype=dtype, device=x.device)
-            # tokens = norm(proj(x)) + pos_embed in one pass (written behind the cls slot in the last stage)
-            _lib.check(lib.vtp_layernorm_add_rows(ptr(y), dtype_code(dtype), B * HW, C, C, ptr(wb[0]), ptr(wb[1]),
-                                                  float(pe.norm.eps), ptr(pos), HW, 1 if last else 0, ptr(tokens), HW,
-                                                  HW + (1 if last else 0), 1 if last else 0, st))
-            if last:
-                cls = self._const("cls", (self.cls_token,), lambda: self.cls_token.detach().reshape(1, C).contiguous())
-                _lib.check(lib.vtp_add_rows(ptr(cls), 1, ptr(pos), 1, 0, ptr(tokens), 1, HW + 1, 0, dtype_code(dtype),
-                                            B, C, st))
-            stage = getattr(self, f"block{i + 1}")
-            tokens = stage_forward(stage, tokens, H, W)
-            counts.extend(blk.dge.states["batches_device"] for blk in stage)
-            if self.num_classes == 0:
-                grid_rows = tokens[:, 1:] if last else tokens
-                outputs[f"res{i + 2}"] = grid_rows.reshape(B, H, W, C).permute(0, 3, 1, 2).contiguous()
-        self.last_counts = counts
+                _lib.check(lib.vtp_patch_im2col(ptr(x), dtype_code(x.dtype), B, S, P, dtype_code(dtype), cols, None, None,
+                                                self.embed_dims[0], None, stream))
+
         if self.num_classes == 0:
+            counts = torch.empty(sum(self.depths), B, dtype=torch.int32, device=dev)
+            outputs = {}
+            front()
+            self._trunk(B, sides, dtype, self._trunk_consts(sides, dtype, ld), cols, y, tokens, counts, dev, stream, outputs,
+                        arena)
+            self._set_states(B, sides, counts)
             return outputs
-        N = tokens.shape[1]
-        C = tokens.shape[2]
-        wb = self._const("norm", (self.norm.weight, self.norm.bias), lambda: (
-            self.norm.weight.detach().float().contiguous(), self.norm.bias.detach().float().contiguous()))
-        cls_n = _norm_rows(tokens, B, C, N * C, self.norm, wb=wb)
+        plan = None
+        if use_plans:
+            plan = self._plans.get((B, S, dtype, self._param_generation()),
+                                   lambda p: p.scratch_gen == self._scratch_gen(dev),
+                                   lambda: self._capture_trunk(B, sides, ld, dtype, cols, y, tokens, dev))
+        front()
+        if plan is not None:
+            plan.graph.replay()
+            counts = plan.counts.clone()
+        else:
+            counts = torch.empty(sum(self.depths), B, dtype=torch.int32, device=dev)
+            self._trunk(B, sides, dtype, self._trunk_consts(sides, dtype, ld), cols, y, tokens, counts, dev, stream)
         head_w = self._const("head_w", (self.head.weight,), lambda: self.head.weight.detach().to(dtype).contiguous(), (dtype,))
         head_b = self._const("head_b", (self.head.bias,), lambda: self.head.bias.detach().float().contiguous())
-        logits = _matmul_rows(cls_n, head_w, head_b, flags=_lib.FLAG_OUT_F32, out_dtype=torch.float32)
-        self.last_counts = counts
+        logits = torch.empty(B, self.num_classes, dtype=torch.float32, device=dev)
+        _launch_linear(y, head_w, head_b, ptr(logits), B, _lib.FLAG_OUT_F32, stream)      # y: the normed cls rows
+        self._set_states(B, sides, counts)
         return logits
+
+    def _capture_trunk(self, B, sides, ld, dtype, cols, y, tokens, dev):
+        counts = torch.empty(sum(self.depths), B, dtype=torch.int32, device=dev)
+        consts = self._trunk_consts(sides, dtype, ld)
+        graph = capture_launches(dev, lambda stream: self._trunk(B, sides, dtype, consts, cols, y, tokens, counts, dev, stream))
+        plan = _CapturedForward(graph, (consts,) + self._keep(dev), self._scratch_gen(dev))
+        plan.counts = counts
+        return plan
+
+    def _set_states(self, B, sides, counts):
+        self.last_counts = list(counts.unbind(0))
+        k = 0
+        for i, side in enumerate(sides):
+            extra = 1 if i == self.num_stages - 1 else 0
+            # shapes only, for the complexity accounting
+            shape = counts.new_empty(0).expand(B, side * side + extra, 0)
+            for blk in getattr(self, f"block{i + 1}"):
+                blk.dge.states.update({"batches_device": self.last_counts[k], "input": shape, "gate": None,
+                                       "size": (side, side), "num_extra_tokens": extra})
+                k += 1
+
+    def _stage_consts(self, i, side, dtype, ld):
+        """What the launches of stage i need besides the blocks' weights: the embedding's matrix and bias, its LayerNorm
+        vectors, the position rows and (last stage) the cls row."""
+        pe = getattr(self, f"patch_embed{i + 1}")
+        pos_full = getattr(self, f"pos_embed{i + 1}").detach()
+        C, P = self.embed_dims[i], pe.patch_size[0]
+        last = i == self.num_stages - 1
+        if i == 0:
+            wm = self._const(f"wm{i}", (pe.proj.weight,), lambda: torch.nn.functional.pad(
+                pe.proj.weight.detach().reshape(C, -1).to(dtype), (0, ld - 3 * P * P)).contiguous(), (dtype, ld))
+        else:
+            wm = self._const(f"wm{i}", (pe.proj.weight,), lambda: pe.proj.weight.detach().permute(0, 2, 3, 1)
+                             .reshape(C, -1).to(dtype).contiguous(), (dtype,))
+        bias = self._const(f"eb{i}", (pe.proj.bias,), lambda: pe.proj.bias.detach().float().contiguous())
+        wb = self._const(f"en{i}", (pe.norm.weight, pe.norm.bias), lambda: (
+            pe.norm.weight.detach().float().contiguous(), pe.norm.bias.detach().float().contiguous()))
+
+        # the stage's position rows ([cls row;] grid rows), resized when the grid is not the trained one
+        def make_pos():
+            if last:
+                pos = torch.cat((pos_full[:, 0:1], self._stage_pos_embed(pos_full[:, 1:], pe, side, side)), dim=1)
+            else:
+                pos = self._stage_pos_embed(pos_full, pe, side, side)
+            return pos[0].to(dtype).contiguous()
+        pos = self._const(f"pos{i}", (getattr(self, f"pos_embed{i + 1}"),), make_pos, (dtype, side))
+        cls = self._const("cls", (self.cls_token,), lambda: self.cls_token.detach().reshape(1, C).contiguous()) if last else None
+        return wm, bias, wb, pos, cls
+
+    def _trunk_consts(self, sides, dtype, ld):
+        """Every tensor the trunk's launches take the address of: made (or found) before anything is captured."""
+        consts = [self._stage_consts(i, side, dtype, ld) for i, side in enumerate(sides)]
+        norm = None
+        if self.num_classes > 0:
+            norm = self._const("norm", (self.norm.weight, self.norm.bias), lambda: (
+                self.norm.weight.detach().float().contiguous(), self.norm.bias.detach().float().contiguous()))
+        for i in range(self.num_stages):
+            for blk in getattr(self, f"block{i + 1}"):
+                _pack_block(blk, dtype)
+        return consts, norm
+
+    def _trunk(self, B, sides, dtype, trunk_consts, cols, y, tokens, counts, dev, st, outputs=None, arena=None):
+        """Everything between the im2col of the images and the head: ``cols`` -> the normed cls rows in ``y``, or
+        with ``outputs`` the stage maps cut out of ``tokens`` (which lies in ``arena``)."""
+        lib, code = _lib.lib(), dtype_code(dtype)
+        consts, norm = trunk_consts
+        first = 0
+        for i, (side, (wm, bias, wb, pos, cls)) in enumerate(zip(sides, consts)):
+            pe = getattr(self, f"patch_embed{i + 1}")
+            C, HW = self.embed_dims[i], side * side
+            N = HW + (0 if cls is None else 1)
+            if i > 0:
+                _lib.check(lib.vtp_token_im2col(tokens, code, B, sides[i - 1], sides[i - 1], self.embed_dims[i - 1],
+                                                pe.patch_size[0], cols, st))
+            _launch_linear(cols, wm, bias, y, B * HW, 0, st)
+            # tokens = norm(proj(x)) + pos_embed in one pass (written behind the cls slot in the last stage)
+            _lib.check(lib.vtp_layernorm_add_rows(y, code, B * HW, C, C, ptr(wb[0]), ptr(wb[1]), float(pe.norm.eps), ptr(pos),
+                                                  HW, N - HW, tokens, HW, N, N - HW, st))
+            if cls is not None:
+                _lib.check(lib.vtp_add_rows(ptr(cls), 1, ptr(pos), 1, 0, tokens, 1, N, 0, code, B, C, st))
+            stage = list(getattr(self, f"block{i + 1}"))
+            _launch_stage(stage, dtype, B, N, side, side, tokens, tokens, counts[first:].data_ptr(), dev, st)
+            first += len(stage)
+            if outputs is not None:
+                at = tokens - arena.data_ptr()
+                rows = arena[at:at + B * N * C * wm.element_size()].view(dtype).view(B, N, C)
+                outputs[f"res{i + 2}"] = rows[:, N - HW:].reshape(B, side, side, C).permute(0, 3, 1, 2).contiguous()
+        if outputs is None:
+            _lib.check(lib.vtp_layernorm(tokens, code, B, None, C, N * C, ptr(norm[0]), ptr(norm[1]), float(self.norm.eps), y,
+                                         st))
 
 
 def _pvt(depths, **kwargs):
