@@ -456,3 +456,40 @@ def test_gelu_epilogue_error_on_a_dense_sweep(vl):
     assert bool((err <= bound).all()), float((err / bound).max())
     sp = got[n_fin::K][:5]
     assert sp[0] >= 65000 and sp[1] == 0 and torch.isnan(sp[2]) and sp[3] >= 65000 and sp[4] == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 64, 4), (127, 64, 64), (128, 65, 68), (129, 200, 100), (300, 10, 384), (130, 384, 768),
+                                   (1500, 384, 1536), (40, 192, 832), (2600, 1000, 192), (20000, 256, 320)])
+@pytest.mark.parametrize("gelu,res,positive", [(False, False, False), (True, True, False), (False, True, True)])
+def test_linear_fp32_split_terms_are_as_accurate_as_fmaf_chains(vl, M, N, K, gelu, res, positive):
+    """The fp32 Linear on tensor cores (three bf16 terms per operand) against float64: tile edges in every direction,
+    reductions split over two and four CTAs of a cluster, both tile widths, positive operands (where a biased rounding
+    would add up).  Bound: every product is exact to 2^-23 of |a||w| (the three terms left out), a k-block's sum
+    is rounded a few times to 2^-24 of itself and the k-blocks are added with one rounding each, so the error of an
+    output is below (4 + K / 64) 2^-23 sum |a||w|; and over the whole result it is no larger than that of the
+    CUDA-core kernel's fmaf chain (plus half an ulp for the rounding of y that both share)."""
+    from vtpack_b200 import _lib
+    from vtpack_b200.runtime import ptr, stream_ptr
+    g = torch.Generator(DEV).manual_seed(M + N + K)
+    x = torch.randn(M, K, device=DEV, generator=g)
+    w = torch.randn(N, K, device=DEV, generator=g) * 0.1
+    if positive:
+        x, w = x.abs() + 0.5, w.abs()
+    b = torch.randn(N, device=DEV, generator=g)
+    r = torch.randn(M, N, device=DEV, generator=g) if res else None
+    z = x.double() @ w.double().t() + b.double()
+    ref = torch.nn.functional.gelu(z) if gelu else z
+    ref = ref + r.double() if res else ref
+
+    def run(flags):
+        y = torch.full((M, N), float("nan"), device=DEV)
+        _lib.check(_lib.lib().vtp_linear(ptr(x), K, ptr(w), ptr(b), ptr(r), N, ptr(y), N, 0, M, None, N, K,
+                                         flags | (_lib.FLAG_GELU if gelu else 0), stream_ptr(x.device)))
+        return y.double()
+
+    mag = x.abs().double() @ w.abs().double().t() + b.abs().double() + (r.abs().double() if res else 0.0)
+    got, chain = run(0), run(_lib.FLAG_CUDA_CORES)
+    assert bool(((got - ref).abs() <= 1.2 * (4 + K / 64) * 2.0 ** -23 * mag).all())      # GELU's slope is at most 1.13
+    e = [float((t - ref).norm() / ref.norm()) for t in (got, chain)]
+    assert e[0] <= e[1] + 2.0 ** -24
+    assert _lib.device_status() == 0

@@ -128,12 +128,18 @@ static RegionGeom region_geom(const vtp_dge_shape& s) {
 }
 
 // Whether a block of this shape runs with norm1 folded into q and norm2 into fc1 (bf16 tensor-core path,
-// region-parallel token movers, prepared weights).  A block without a spatial reduction folds kv too.  Only
-// such blocks hand the next block its gate decisions and token statistics from their unpool.
+// region-parallel token movers, prepared weights).  A block without a spatial reduction folds kv too.
 static bool block_folds(const vtp_dge_shape& s, const vtp_block_weights& w) {
     if (!region_ops_supported(region_geom(s), s.dtype) || s.dtype != VTP_BF16 || (s.flags & VTP_FLAG_CUDA_CORES))
         return false;
     return s.sr_ratio > 1 ? has_folded_q_fc1(w) : has_folded_weights(w);
+}
+
+// Whether a block can hand the next one its gate decisions (and, where both fold, the token statistics) from its
+// unpool.  The sums behind a decision are the stand-alone gate's, in the same order, on the values it would read.
+static bool block_chains(const vtp_dge_shape& s, const vtp_block_weights& w, const vtp_block_weights& next) {
+    if (!region_ops_supported(region_geom(s), s.dtype)) return false;
+    return block_folds(s, w) == block_folds(s, next);
 }
 
 // Position of a block inside a model forward: whether the previous block's unpool already
@@ -191,12 +197,12 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
     bool stats_x_ready = false;
     // chained: gate decisions, per-image counts and token statistics came from the previous
     // block's unpool; the pool kernel then also derives the row offsets itself
-    const bool chained = chain.have_gate && fold_q && !forced_logits;
+    const bool chained = chain.have_gate && by_region && !forced_logits;
     VTP_REQUIRE(!chain.image_bias || by_region, VTP_ERR_UNSUPPORTED,
                 "block: a per-image gate bias needs the region-parallel gate (4x4-token regions)");
 
     if (chained) {
-        stats_x_ready = true;
+        stats_x_ready = fold_q;
         rc = VTP_OK;
     } else if (forced_logits) {
         rc = by_region ? count_queries(forced_logits, idx, sp, s.B, Hr * Wr, s.num_extra, counts, st)
@@ -225,7 +231,7 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
         RegionPoolArgs pa;
         pa.g = g; pa.sp = sp; pa.x = x_in; pa.idx = idx; pa.comp = b.comp; pa.eps = s.eps;
         pa.counts = counts; pa.offsets_out = b.offsets; pa.region_first_out = b.region_first;
-        const bool will_chain = fold_q && chain.next && block_folds(s, *chain.next);
+        const bool will_chain = chain.next && block_chains(s, w, *chain.next);
         pa.counts_next = will_chain ? counts_next : nullptr;
         if (fold_q) {
             pa.stats_x = stats_x; pa.stats_q = b.stats_q;
@@ -311,10 +317,11 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
         RegionUnpoolArgs ua;
         ua.g = g; ua.sp = sp; ua.q = b.qp; ua.comp = b.comp; ua.ref = x_in; ua.out = x_out; ua.idx = idx;
         ua.region_first = b.region_first; ua.offsets = b.offsets;
-        if (fold_q && chain.next && block_folds(s, *chain.next)) {
+        if (chain.next && block_chains(s, w, *chain.next)) {
             // the rows being written are the next block's input: leave its LayerNorm statistics and
             // its router gate's decisions in the other scratch slot
-            ua.next.stats_x = b.stats_x[par ^ 1]; ua.next.eps = s.eps;
+            if (fold_q) ua.next.stats_x = b.stats_x[par ^ 1];
+            ua.next.eps = s.eps;
             ua.next.gw = chain.next->gate_w; ua.next.gb = chain.next->gate_b; ua.next.S = s.n_splits;
             ua.next.logits = b.logits[par ^ 1]; ua.next.idx = b.idx[par ^ 1];
             ua.next.counts = counts_next;
@@ -439,7 +446,7 @@ static int deit_trunk(const vtp_dge_shape& s, const vtp_model_weights& m, const 
                                                    cudaMemcpyDeviceToDevice, st);
             if (ce != cudaSuccess) return fail((int)ce, "model: grain trace copy: %s", cudaGetErrorString(ce));
         }
-        chained = chain.next && block_folds(s, blocks[i]) && block_folds(s, *chain.next);
+        chained = chain.next && block_chains(s, blocks[i], *chain.next);
     }
     return vtp_layernorm(ms.x, s.dtype, s.B, nullptr, C, (long long)N * C, m.norm_w, m.norm_b, s.eps, ms.cls_n, st);
 }
@@ -488,7 +495,7 @@ extern "C" int vtp_dge_blocks_forward(const vtp_dge_shape* s, const vtp_block_we
                                    counts_out ? counts_out + (size_t)i * s->B : nullptr, workspace, st, StageMarks(),
                                    chain))
             return rc;
-        chained = chain.next && block_folds(*s, w[i]) && block_folds(*s, *chain.next);
+        chained = chain.next && block_chains(*s, w[i], *chain.next);
     }
     return VTP_OK;
 }

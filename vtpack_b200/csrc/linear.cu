@@ -23,6 +23,8 @@ int linear(const LinearArgs& p, cudaStream_t st) {
     const bool tc_shape = (p.K % 64 == 0 && p.N % 8 == 0 && p.lda % 8 == 0 && p.ldy % 8 == 0 &&
                            (!p.res || p.ldr % 8 == 0)) || p.ln_mode != 0 || p.emit_stats;
     if (p.dtype == VTP_BF16 && !(p.flags & VTP_FLAG_CUDA_CORES) && tc_shape) return linear_tcgen05(p, st);
+    // fp32: tensor cores on split operands; the CUDA-core kernel where rows do not allow 16-byte loads, and on request
+    if (!(p.flags & VTP_FLAG_CUDA_CORES) && linear_f32_tc_supported(p)) return linear_f32_tcgen05(p, st);
     VTP_REQUIRE(p.ln_mode == 0 && !p.emit_stats, VTP_ERR_UNSUPPORTED,
                 "linear (CUDA cores): folded LayerNorm is a feature of the tcgen05 kernel");
     return linear_cuda_cores(p, st);

@@ -44,6 +44,8 @@ struct LnFold { const float2* stats; const float* s; int mode, dim; float eps; f
 int linear_validate(const LinearArgs& p);
 int linear_cuda_cores(const LinearArgs& p, cudaStream_t st);   // fp32 or bf16 inputs, CUDA cores
 int linear_tcgen05(const LinearArgs& p, cudaStream_t st);      // bf16 inputs, tcgen05 + TMA
+bool linear_f32_tc_supported(const LinearArgs& p);
+int linear_f32_tcgen05(const LinearArgs& p, cudaStream_t st);  // fp32 inputs as three bf16 terms each, tcgen05
 int linear(const LinearArgs& p, cudaStream_t st);              // picks by dtype / flags
 bool linear_pair_supported(const LinearArgs& a, const LinearArgs& b);
 int linear_tcgen05_pair(const LinearArgs& a, const LinearArgs& b, cudaStream_t st);   // two problems, one launch

@@ -527,6 +527,8 @@ unpool_region_kernel(const T* __restrict__ q, const T* __restrict__ comp, const 
         if (nx.stats_x) {
             const float2 st = mean_rstd(row_sums<T, G, CPL>(o), g.C, nx.eps);
             if (sub == 0) nx.stats_x[tok0 + j] = st;
+        }
+        if (nx.gw) {
 #pragma unroll
             for (int ch = 0; ch < CPL; ++ch)
 #pragma unroll
