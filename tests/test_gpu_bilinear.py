@@ -62,6 +62,32 @@ def test_bilinear_attention_shapes(op, mode, B, H, W, C, G, P):
     assert rel_err(got16[1].float(), refs16[1]) < 6e-2          # sums of bf16 atomics
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("mode", ["point", "channel"])
+@pytest.mark.parametrize("C,shift", [(8, 0), (32, 0), (48, 0), (72, 0), (128, 0), (192, 0), (48, 2), (20, 0), (48, 1)])
+def test_bilinear_attention_channel_layouts(op, dtype, mode, C, shift):
+    """Every lane layout (4 to 32 lanes per query with 16-byte vectors, whole or part-filled; channel pairs; single
+    channels), an instance count that leaves groups of the last warp idle, and operands that start `shift` elements
+    behind a 16-byte boundary.  fp32 bound: sums of at most 4 P + log2(C) terms, 2^-24 each; bf16 bounds as above."""
+    B, H, W, G, P = 3, 5, 6, 11, 5
+    inp, grid, weight, grad_out = BO.make_bilinear_inputs(B, H, W, C, G, P, seed=C + shift, mode=mode)
+
+    def place(t):                              # a contiguous operand at the given offset
+        buf = torch.zeros(t.numel() + shift, dtype=dtype, device=DEV)
+        buf[shift:] = t.to(DEV, dtype).flatten()
+        return buf[shift:].view(t.shape).requires_grad_(True)
+
+    a, gr, w, go = map(place, (inp, grid, weight, grad_out))
+    y = op(a, gr, w, mode)
+    got = (y.detach(),) + torch.autograd.grad(y, (a, gr, w), go.detach())
+    r = [t.to(dtype).double() for t in (inp, grid, weight, grad_out)]
+    want = (getattr(BO, f"bilinear_attention_{mode}wise_forward")(*r[:3]),) + \
+        getattr(BO, f"bilinear_attention_{mode}wise_backward")(r[3], *r[:3])
+    bounds = (2e-5,) * 4 if dtype == torch.float32 else (2e-2, 6e-2, 2e-2, 2e-2)
+    for name, t, ref, bound in zip(("out", "grad_input", "grad_grid", "grad_weight"), got, want, bounds):
+        assert rel_err(t.float(), ref) < bound, name
+
+
 def test_bilinear_attention_points_outside_and_non_finite(op):
     """Points far outside the map, at infinity or NaN read zero and leave zero gradients; nothing is
     dereferenced out of bounds."""

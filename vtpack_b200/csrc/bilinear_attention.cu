@@ -6,20 +6,24 @@
 // Replaces bilinear_attention_{pointwise,channelwise}_{forward,backward}
 // (vtpack/layers/csrc/bilinear_attention/bilinear_attention.cu:88-132, :134-232, :234-268, :270-362).
 //
-// The reference runs one thread per (b, g) that walks the channels serially, so neighbouring
-// threads read addresses C elements apart.  Here one warp owns a (b, g) instance and its lanes walk
-// the channels: every corner read, every atomic of the input gradient and every output row is a
-// run of consecutive addresses; with an even C a lane takes two neighbouring channels, which halves
-// the loads and (packed float2 / bf16x2 atomics) the atomic traffic of the input gradient.  All four
-// kernels are bound by those gathers (4 corner rows per point), not by arithmetic.
+// The reference runs one thread per (b, g) that walks the channels serially, so neighbouring threads read addresses
+// C elements apart.  Here a group of LG lanes owns a (b, g) instance and each lane a 16-byte vector of its channels
+// (8 bf16 / 4 fp32): 4 instances per warp at C = 64 in bf16.  A point's corner arithmetic and the reductions over
+// the channels are then paid once per 16 bytes instead of once per channel pair, and the input gradient leaves as
+// one vector red per corner.
+// Measured on 32 maps of 64 x 64 x 64, 9 points, bf16, point mode: forward + backward 525 -> 245 us (now 71 + 163
+// us) against a warp per instance with a channel pair per lane.  Bound: the issue slots (76 % busy) and, in the
+// backward, the SM's request port to L2 (69 %: 4 x 128 bytes of reds per point); DRAM 5 %.  Tried and not kept, same
+// inputs: contiguous query ranges per SM for the L1 (71 -> 76 / 163 -> 157 us), packed f32x2 arithmetic (70 / 163 us),
+// a point's corners worked out by one lane and handed round by shuffles (78 / 159 us), no reds at all 136 us.
 #include <initializer_list>
 
 #include "common.cuh"
 
 namespace vtp {
 
-constexpr int BA_WARPS = 8;           // instances per 256-thread block
-constexpr int BA_MAXCH = 8;           // channel-mode backward keeps C / 32 weight gradients per lane
+constexpr int BA_WARPS = 8;           // warps per block
+constexpr int BA_MAXCH = 8;           // widest C of the backward / 32: a lane keeps its weight gradients in registers
 
 struct Corner {
     int x0, y0;
@@ -49,8 +53,31 @@ __device__ __forceinline__ float sane(float v, int extent) {
     return (v > -4.f && v < (float)extent + 4.f) ? v : -4.f;
 }
 
-// V consecutive channels per lane (2 when C is even: half the loads and half the atomics)
-template <typename T, int V> struct Pack;
+// V consecutive channels per lane: 16 bytes, or one pair / one channel where the rows are not made of 16-byte vectors
+template <typename T, int V> struct Pack {
+    static_assert(V == Vec<T>::N, "");
+    static __device__ __forceinline__ void load(const T* p, float (&f)[V]) {
+        Vec<T> v;
+        v.load(p);
+        v.to_float(f);
+    }
+    static __device__ __forceinline__ void store(T* p, const float (&f)[V]) {
+        Vec<T> v;
+        v.from_float(f);
+        v.store(p);
+    }
+    static __device__ __forceinline__ void atomic_add(T* p, const float (&f)[V]) {
+        Vec<T> v;
+        v.from_float(f);
+        const uint4 r = *reinterpret_cast<const uint4*>(&v.raw);
+        if constexpr (sizeof(T) == 4)
+            asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(f[0]), "f"(f[1]),
+                         "f"(f[2]), "f"(f[3]));
+        else
+            asm volatile("red.relaxed.gpu.global.add.noftz.v4.bf16x2 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(r.x),
+                         "r"(r.y), "r"(r.z), "r"(r.w));
+    }
+};
 template <> struct Pack<float, 1> {
     static __device__ __forceinline__ void load(const float* p, float (&f)[1]) { f[0] = *p; }
     static __device__ __forceinline__ void store(float* p, const float (&f)[1]) { *p = f[0]; }
@@ -121,45 +148,69 @@ __device__ __forceinline__ void scatter(T* __restrict__ gimg, const Corner& k, i
 #undef VTP_BA_SCATTER
 }
 
+// sum over the LG lanes of a group
+template <int LG> __device__ __forceinline__ float group_sum(float v) {
+#pragma unroll
+    for (int o = LG / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// a point's coordinates; one load where the caller checked that pairs are aligned
+template <bool VEC> __device__ __forceinline__ float2 point_xy(const float* p) {
+    if constexpr (VEC) return *reinterpret_cast<const float2*>(p);
+    else return make_float2(p[0], p[1]);
+}
+template <bool VEC> __device__ __forceinline__ float2 point_xy(const bf16* p) {
+    if constexpr (VEC) return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+    else return make_float2(__bfloat162float(p[0]), __bfloat162float(p[1]));
+}
+
 // ---------------------------------------------------------------------------- forward
-template <typename T, bool POINT, int V>
+template <typename T, bool POINT, int V, int LG>
 __global__ void __launch_bounds__(BA_WARPS * 32)
 bilinear_attention_fwd_kernel(const T* __restrict__ input, const T* __restrict__ grid, const T* __restrict__ weight,
                               T* __restrict__ out, int B, int H, int W, int C, int G, int P,
                               const long long* __restrict__ batch_of) {
     // batch_of == null: B * G instances, G per image; else G packed instances, instance i reads image batch_of[i]
-    const int lane = threadIdx.x & 31;
+    constexpr int PW = 32 / LG;                          // instances per warp
+    constexpr bool VEC = V == Vec<T>::N;
+    const int lane = threadIdx.x & 31, gl = lane % LG, sub = lane / LG;
     const long long n_inst = batch_of ? (long long)G : (long long)B * G;
-    for (long long inst = (long long)blockIdx.x * BA_WARPS + (threadIdx.x >> 5); inst < n_inst;
-         inst += (long long)gridDim.x * BA_WARPS) {
+    for (long long first = ((long long)blockIdx.x * BA_WARPS + (threadIdx.x >> 5)) * PW; first < n_inst;
+         first += (long long)gridDim.x * BA_WARPS * PW) {
+        const bool own = first + sub < n_inst;           // a group past the end goes along for the shuffles
+        const long long inst = own ? first + sub : first;
         long long b = batch_of ? batch_of[inst] : inst / G;
-        const bool image_ok = b >= 0 && b < B;          // an instance naming no image reads zeros
+        const bool image_ok = b >= 0 && b < B;           // an instance naming no image reads zeros
         if (!image_ok) b = 0;
         const int Hb = image_ok ? H : 0;                 // no pixel is in bounds
         const T* img = input + (size_t)b * H * W * C;
         const T* pts = grid + (size_t)inst * P * 2;
         if (POINT) {
             const T* wt = weight + (size_t)inst * P;
-            for (int c = lane * V; c < C; c += 32 * V) {
+            for (int c = gl * V; c < C; c += LG * V) {
                 float acc[V];
 #pragma unroll
                 for (int v = 0; v < V; ++v) acc[v] = 0.f;
+#pragma unroll 3
                 for (int p = 0; p < P; ++p) {
-                    const Corner k = corners_of(sane(to_f32(pts[2 * p]), W), sane(to_f32(pts[2 * p + 1]), H), Hb, W);
+                    const float2 xy = point_xy<VEC>(pts + 2 * p);
+                    const Corner k = corners_of(sane(xy.x, W), sane(xy.y, H), Hb, W);
                     Taps<T, V> t;
                     t.load(img, k, W, C, c);
                     const float wp = to_f32(wt[p]);
 #pragma unroll
                     for (int v = 0; v < V; ++v) acc[v] = fmaf(t.value(k, v), wp, acc[v]);
                 }
-                Pack<T, V>::store(out + (size_t)inst * C + c, acc);
+                if (own) Pack<T, V>::store(out + (size_t)inst * C + c, acc);
             }
         } else {
             const T* wt = weight + (size_t)inst * C;
             for (int p = 0; p < P; ++p) {
-                const Corner k = corners_of(sane(to_f32(pts[2 * p]), W), sane(to_f32(pts[2 * p + 1]), H), Hb, W);
+                const float2 xy = point_xy<VEC>(pts + 2 * p);
+                const Corner k = corners_of(sane(xy.x, W), sane(xy.y, H), Hb, W);
                 float acc = 0.f;
-                for (int c = lane * V; c < C; c += 32 * V) {
+                for (int c = gl * V; c < C; c += LG * V) {
                     Taps<T, V> t;
                     t.load(img, k, W, C, c);
                     float wc[V];
@@ -167,8 +218,8 @@ bilinear_attention_fwd_kernel(const T* __restrict__ input, const T* __restrict__
 #pragma unroll
                     for (int v = 0; v < V; ++v) acc = fmaf(t.value(k, v), wc[v], acc);
                 }
-                acc = warp_sum(acc);
-                if (lane == 0) out[(size_t)inst * P + p] = from_f32<T>(acc);
+                acc = group_sum<LG>(acc);
+                if (gl == 0 && own) out[(size_t)inst * P + p] = from_f32<T>(acc);
             }
         }
     }
@@ -176,16 +227,21 @@ bilinear_attention_fwd_kernel(const T* __restrict__ input, const T* __restrict__
 
 // --------------------------------------------------------------------------- backward
 // grad_input must be zero on entry (the host wrapper clears it on the same stream).
-template <typename T, bool POINT, int V>
+template <typename T, bool POINT, int V, int LG>
 __global__ void __launch_bounds__(BA_WARPS * 32)
 bilinear_attention_bwd_kernel(const T* __restrict__ grad_out, const T* __restrict__ input, const T* __restrict__ grid,
                               const T* __restrict__ weight, T* __restrict__ grad_input, T* __restrict__ grad_grid,
                               T* __restrict__ grad_weight, int B, int H, int W, int C, int G, int P) {
-    constexpr int J = BA_MAXCH / V;                        // channel groups per lane
-    const int lane = threadIdx.x & 31;
+    constexpr int J = LG == 32 && BA_MAXCH > V ? BA_MAXCH / V : 1;   // channel groups per lane
+    constexpr int PW = 32 / LG;                                      // instances per warp
+    constexpr bool VEC = V == Vec<T>::N;
+    const int lane = threadIdx.x & 31, gl = lane % LG, sub = lane / LG;
     const long long n_inst = (long long)B * G;
-    for (long long inst = (long long)blockIdx.x * BA_WARPS + (threadIdx.x >> 5); inst < n_inst;
-         inst += (long long)gridDim.x * BA_WARPS) {
+    for (long long first = ((long long)blockIdx.x * BA_WARPS + (threadIdx.x >> 5)) * PW; first < n_inst;
+         first += (long long)gridDim.x * BA_WARPS * PW) {
+        const bool own = first + sub < n_inst;           // a group past the end goes along for the shuffles
+        const long long inst = own ? first + sub : first;
+        const int Hb = own ? H : 0;                      // and touches no pixel
         const int b = (int)(inst / G);
         const T* img = input + (size_t)b * H * W * C;
         T* gimg = grad_input + (size_t)b * H * W * C;
@@ -195,26 +251,27 @@ bilinear_attention_bwd_kernel(const T* __restrict__ grad_out, const T* __restric
         float up[J][V], gw_c[J][V];
 #pragma unroll
         for (int j = 0; j < J; ++j) {
-            const int c = (lane + 32 * j) * V;
+            const int c = (gl + LG * j) * V;
 #pragma unroll
             for (int v = 0; v < V; ++v) up[j][v] = gw_c[j][v] = 0.f;
             if (c < C) Pack<T, V>::load((POINT ? grad_out : weight) + (size_t)inst * C + c, up[j]);
         }
         for (int p = 0; p < P; ++p) {
-            const Corner k = corners_of(sane(to_f32(pts[2 * p]), W), sane(to_f32(pts[2 * p + 1]), H), H, W);
+            const float2 xy = point_xy<VEC>(pts + 2 * p);
+            const Corner k = corners_of(sane(xy.x, W), sane(xy.y, H), Hb, W);
             // scale turning up[] into g = d(loss) / d(sample(b, p, c))
             const float sc = POINT ? to_f32(weight[(size_t)inst * P + p]) : to_f32(grad_out[(size_t)inst * P + p]);
             float gix = 0.f, giy = 0.f, giw = 0.f;
 #pragma unroll
             for (int j = 0; j < J; ++j) {
-                const int c = (lane + 32 * j) * V;
+                const int c = (gl + LG * j) * V;
                 if (c < C) {
                     float g[V];
 #pragma unroll
                     for (int v = 0; v < V; ++v) g[v] = up[j][v] * sc;
-                    scatter<T, V>(gimg, k, W, C, c, g);
                     Taps<T, V> t;
                     t.load(img, k, W, C, c);
+                    scatter<T, V>(gimg, k, W, C, c, g);
 #pragma unroll
                     for (int v = 0; v < V; ++v) {
                         // d(sample)/dx and d(sample)/dy of the bilinear form
@@ -225,27 +282,27 @@ bilinear_attention_bwd_kernel(const T* __restrict__ grad_out, const T* __restric
                     }
                 }
             }
-            gix = warp_sum(gix);
-            giy = warp_sum(giy);
-            if (POINT) giw = warp_sum(giw);
-            if (lane == 0) {
+            gix = group_sum<LG>(gix);
+            giy = group_sum<LG>(giy);
+            if (POINT) giw = group_sum<LG>(giw);
+            if (gl == 0 && own) {
                 grad_grid[((size_t)inst * P + p) * 2] = from_f32<T>(gix);
                 grad_grid[((size_t)inst * P + p) * 2 + 1] = from_f32<T>(giy);
                 if (POINT) grad_weight[(size_t)inst * P + p] = from_f32<T>(giw);
             }
         }
-        if (!POINT) {
+        if (!POINT && own) {
 #pragma unroll
             for (int j = 0; j < J; ++j) {
-                const int c = (lane + 32 * j) * V;
+                const int c = (gl + LG * j) * V;
                 if (c < C) Pack<T, V>::store(grad_weight + (size_t)inst * C + c, gw_c[j]);
             }
         }
     }
 }
 
-static int ba_grid(long long instances) {
-    const long long want = (instances + BA_WARPS - 1) / BA_WARPS;
+static int ba_grid(long long instances, int per_warp) {
+    const long long want = (instances + BA_WARPS * per_warp - 1) / (BA_WARPS * per_warp);
     const long long cap = (long long)sm_count() * 16;
     return (int)(want < 1 ? 1 : (want < cap ? want : cap));
 }
@@ -257,14 +314,33 @@ static int ba_check(const char* what, int dtype, int mode, int B, int H, int W, 
     return VTP_OK;
 }
 
-// channel pairs need an even C and every channel-indexed pointer aligned to a pair
-static bool ba_pairs(int dtype, int C, std::initializer_list<const void*> ptrs) {
-    if (C % 2) return false;
-    const uintptr_t mask = 2 * elem_size(dtype) - 1;
-    for (const void* p : ptrs)
-        if (reinterpret_cast<uintptr_t>(p) & mask) return false;
-    return true;
+struct BaLayout {
+    int v, lanes;          // channels per lane, lanes per instance
+};
+
+// 16-byte vectors where every row of channels is made of them (C a multiple of 8 bf16 / 4 fp32, channel-indexed
+// pointers on 16-byte boundaries, points on pair boundaries), as few lanes per instance as hold C; else pairs of
+// channels (even C, pair-aligned pointers) or single channels, with a warp per instance.
+static BaLayout ba_layout(int dtype, int C, const void* grid, std::initializer_list<const void*> ptrs) {
+    const size_t e = elem_size(dtype);
+    uintptr_t low = 0;
+    for (const void* p : ptrs) low |= reinterpret_cast<uintptr_t>(p);
+    const int v = (int)(16 / e);
+    if (C % v == 0 && low % 16 == 0 && reinterpret_cast<uintptr_t>(grid) % (2 * e) == 0)
+        return {v, C <= 4 * v ? 4 : C <= 8 * v ? 8 : C <= 16 * v ? 16 : 32};
+    return {C % 2 == 0 && low % (2 * e) == 0 ? 2 : 1, 32};
 }
+
+// calls F<T, V, LG>() of the layout
+#define VTP_BA_DISPATCH(T, NV, F)                                          \
+    do {                                                                   \
+        if (lay.v == NV && lay.lanes == 4) F(T, NV, 4);                    \
+        else if (lay.v == NV && lay.lanes == 8) F(T, NV, 8);               \
+        else if (lay.v == NV && lay.lanes == 16) F(T, NV, 16);             \
+        else if (lay.v == NV) F(T, NV, 32);                                \
+        else if (lay.v == 2) F(T, 2, 32);                                  \
+        else F(T, 1, 32);                                                  \
+    } while (0)
 
 }  // namespace vtp
 
@@ -275,19 +351,13 @@ static int ba_forward(const void* input, const void* grid, const void* weight, v
     VTP_REQUIRE(input && grid && weight && out, VTP_ERR_NULL, "bilinear_attention: null pointer");
     if (int rc = ba_check("bilinear_attention", dtype, mode, B, H, W, C, G, P)) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int blocks = ba_grid(batch_of ? (long long)G : (long long)B * G);
-    const bool pairs = ba_pairs(dtype, C, {input, weight, out});
-#define VTP_BA_FWD(T, PT)                                                                                    \
-    do {                                                                                                     \
-        if (pairs)                                                                                           \
-            bilinear_attention_fwd_kernel<T, PT, 2><<<blocks, BA_WARPS * 32, 0, st>>>(                       \
-                (const T*)input, (const T*)grid, (const T*)weight, (T*)out, B, H, W, C, G, P, batch_of);     \
-        else                                                                                                 \
-            bilinear_attention_fwd_kernel<T, PT, 1><<<blocks, BA_WARPS * 32, 0, st>>>(                       \
-                (const T*)input, (const T*)grid, (const T*)weight, (T*)out, B, H, W, C, G, P, batch_of);     \
-    } while (0)
-    if (dtype == VTP_F32) { if (mode == 0) VTP_BA_FWD(float, true); else VTP_BA_FWD(float, false); }
-    else { if (mode == 0) VTP_BA_FWD(bf16, true); else VTP_BA_FWD(bf16, false); }
+    const BaLayout lay = ba_layout(dtype, C, grid, {input, mode == 0 ? out : weight});
+    const int blocks = ba_grid(batch_of ? (long long)G : (long long)B * G, 32 / lay.lanes);
+#define VTP_BA_FWD(T, V, LG)                                                                                 \
+    (mode == 0 ? bilinear_attention_fwd_kernel<T, true, V, LG> : bilinear_attention_fwd_kernel<T, false, V, LG>) \
+        <<<blocks, BA_WARPS * 32, 0, st>>>((const T*)input, (const T*)grid, (const T*)weight, (T*)out, B, H, W, C, G, P, batch_of)
+    if (dtype == VTP_F32) VTP_BA_DISPATCH(float, 4, VTP_BA_FWD);
+    else VTP_BA_DISPATCH(bf16, 8, VTP_BA_FWD);
 #undef VTP_BA_FWD
     return check_launch("bilinear_attention_forward");
 }
@@ -317,21 +387,15 @@ extern "C" int vtp_bilinear_attention_backward(const void* grad_out, const void*
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     cudaError_t e = cudaMemsetAsync(grad_input, 0, (size_t)B * H * W * C * elem_size(dtype), st);
     if (e != cudaSuccess) return fail((int)e, "bilinear_attention_backward: clearing grad_input: %s", cudaGetErrorString(e));
-    const int blocks = ba_grid((long long)B * G);
-    const bool pairs = ba_pairs(dtype, C, {grad_out, input, weight, grad_input, grad_weight});
-#define VTP_BA_BWD(T, PT)                                                                                    \
-    do {                                                                                                     \
-        if (pairs)                                                                                           \
-            bilinear_attention_bwd_kernel<T, PT, 2><<<blocks, BA_WARPS * 32, 0, st>>>(                       \
-                (const T*)grad_out, (const T*)input, (const T*)grid, (const T*)weight, (T*)grad_input,       \
-                (T*)grad_grid, (T*)grad_weight, B, H, W, C, G, P);                                           \
-        else                                                                                                 \
-            bilinear_attention_bwd_kernel<T, PT, 1><<<blocks, BA_WARPS * 32, 0, st>>>(                       \
-                (const T*)grad_out, (const T*)input, (const T*)grid, (const T*)weight, (T*)grad_input,       \
-                (T*)grad_grid, (T*)grad_weight, B, H, W, C, G, P);                                           \
-    } while (0)
-    if (dtype == VTP_F32) { if (mode == 0) VTP_BA_BWD(float, true); else VTP_BA_BWD(float, false); }
-    else { if (mode == 0) VTP_BA_BWD(bf16, true); else VTP_BA_BWD(bf16, false); }
+    const BaLayout lay = mode == 0 ? ba_layout(dtype, C, grid, {input, grad_input, grad_out})
+                                   : ba_layout(dtype, C, grid, {input, grad_input, weight, grad_weight});
+    const int blocks = ba_grid((long long)B * G, 32 / lay.lanes);
+#define VTP_BA_BWD(T, V, LG)                                                                                 \
+    (mode == 0 ? bilinear_attention_bwd_kernel<T, true, V, LG> : bilinear_attention_bwd_kernel<T, false, V, LG>) \
+        <<<blocks, BA_WARPS * 32, 0, st>>>((const T*)grad_out, (const T*)input, (const T*)grid, (const T*)weight, \
+                                           (T*)grad_input, (T*)grad_grid, (T*)grad_weight, B, H, W, C, G, P)
+    if (dtype == VTP_F32) VTP_BA_DISPATCH(float, 4, VTP_BA_BWD);
+    else VTP_BA_DISPATCH(bf16, 8, VTP_BA_BWD);
 #undef VTP_BA_BWD
     return check_launch("bilinear_attention_backward");
 }
