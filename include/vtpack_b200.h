@@ -87,6 +87,13 @@ int vtp_index_to_patch(const void* indices, int idx_is_i64, const int* splits, i
                        int B, int Hr, int Wr, int region, int num_extra, int32_t* counts,
                        int32_t* offsets, int32_t* patches, int64_t* patches64, void* stream);
 
+/* The same, and what vtp_unpool_grad_regions reads instead of the list: idx32 int32 [B,Hr,Wr], the grain indices, and
+ * region_first int32 [B,Hr,Wr], the packed row of each region's first patch (either may be null). */
+int vtp_index_to_patch_regions(const void* indices, int idx_is_i64, const int* splits, int n_splits, int B, int Hr,
+                               int Wr, int region, int num_extra, int32_t* counts, int32_t* offsets,
+                               int32_t* patches, int64_t* patches64, int32_t* idx32, int32_t* region_first,
+                               void* stream);
+
 /*
  * vtp_router_gate + vtp_index_to_patch in one call that needs no scratch from the caller.
  * It has no counterpart in the reference.  It exists for hosts that can hand over input and
@@ -193,6 +200,13 @@ int vtp_batched_sparse_gemm(const void* a, const void* b, void* out, int dtype, 
                             const int32_t* a_offsets, const int32_t* b_offsets, int max_a_len,
                             int max_b_len, int a_transposed, int b_transposed, long long out_rows,
                             int out_cols, void* stream);
+
+/* The same product with the images' row counts in HOST arrays (a_lengths, b_lengths: n_images entries each, read
+ * before the call returns): the offsets travel with the launch, nothing is copied to the device.  1 to 512 images. */
+int vtp_batched_sparse_gemm_lengths(const void* a, const void* b, void* out, int dtype, int heads, int n_images,
+                                    long long a_rows, int a_cols, long long b_rows, int b_cols,
+                                    const long long* a_lengths, const long long* b_lengths, int a_transposed,
+                                    int b_transposed, long long out_rows, int out_cols, void* stream);
 
 /*
  * Bilinear-sampling attention of the deformable PVT (vtpack/models/standard/dpvt.py:92-115).

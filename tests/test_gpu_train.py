@@ -428,3 +428,45 @@ def test_training_pvt_model_matches_reference(golden_dir):
         F.gumbel_softmax = real
     assert [tuple(feats[f"res{i}"].shape) for i in (2, 3, 4, 5)] == [(2, 64, 64, 64), (2, 128, 32, 32),
                                                                        (2, 320, 16, 16), (2, 512, 8, 8)]
+
+
+def _ragged_case(B, dtype, seed):
+    g = torch.Generator().manual_seed(seed)
+    la = torch.randint(0, 9, (B,), generator=g)
+    la[0] = 7
+    lb = la.new_full([B], 5)
+    a = torch.randn(2, int(la.sum()), 16, generator=g).to(dtype)
+    b = torch.randn(2, int(lb.sum()), 16, generator=g).to(dtype)
+    return a, b, la, lb
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 8e-3)])
+@pytest.mark.parametrize("B", [1, 512, 513])
+def test_ragged_product_image_counts(layers, dtype, tol, B):
+    """Offsets that travel with the launch (up to 512 images) and offsets in device memory (more): the product and
+    both gradients, empty images among them; changing the caller's lengths after the forward changes nothing."""
+    a, b, la, lb = _ragged_case(B, dtype, B)
+    ref_a, ref_b = a.double().requires_grad_(True), b.double().requires_grad_(True)
+    ref = O.batched_sparse_gemm_forward(ref_a, ref_b, la, lb, False, True)
+    go = torch.randn(ref.shape, generator=torch.Generator().manual_seed(3)).to(dtype)
+    want = torch.autograd.grad(ref, (ref_a, ref_b), go.double())
+    x, y = a.to(DEV).requires_grad_(True), b.to(DEV).requires_grad_(True)
+    out = layers.batched_sparse_gemm(x, y, la, lb, False, True)
+    la.zero_()
+    got = torch.autograd.grad(out, (x, y), go.to(DEV))
+    for t, r in zip((out,) + got, (ref,) + want):
+        assert rel_err(t.float(), r) < tol
+
+
+@pytest.mark.parametrize("dt", [torch.int32, torch.int64])
+@pytest.mark.parametrize("extra,splits", [(0, [4, 2, 1]), (1, [4, 2, 1]), (2, [2, 1])])
+def test_region_rows_of_patch_list(layers, dt, extra, splits):
+    """The per-region first rows that come with a patch list, against their prefix-sum definition."""
+    B, Hr, Wr = 5, 3, 7
+    idx = torch.randint(0, len(splits), (B, Hr, Wr), generator=torch.Generator().manual_seed(extra), dtype=dt)
+    patches, lengths = layers.grained_sample_index_to_patch(idx.to(DEV), torch.tensor(splits), max(splits), extra)
+    idx32, first = patches._vtp_regions[:2]
+    per = torch.tensor(splits)[idx.reshape(B, -1).long()] ** 2
+    start = torch.cumsum(lengths, 0) - lengths
+    want = start[:, None] + extra + torch.cumsum(per, 1) - per
+    assert torch.equal(first.cpu().long(), want) and torch.equal(idx32.cpu().long(), idx.reshape(B, -1).long())

@@ -55,6 +55,9 @@ PROTOTYPES = {
     "vtp_gate_argmax": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p]),
     "vtp_index_to_patch": (c_int, [c_void_p, c_int, C.POINTER(c_int), c_int, c_int, c_int, c_int, c_int,
                                    c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "vtp_index_to_patch_regions": (c_int, [c_void_p, c_int, C.POINTER(c_int), c_int, c_int, c_int, c_int, c_int,
+                                           c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                           c_void_p]),
     "vtp_gate_compact_static": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
                                         c_void_p, C.POINTER(c_int), c_int, c_void_p, c_void_p, c_void_p]),
     "vtp_pool": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
@@ -71,6 +74,8 @@ PROTOTYPES = {
     "vtp_batched_sparse_gemm": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_int, c_ll,
                                         c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_ll, c_int,
                                         c_void_p]),
+    "vtp_batched_sparse_gemm_lengths": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_int, c_ll,
+                                                c_int, c_void_p, c_void_p, c_int, c_int, c_ll, c_int, c_void_p]),
     "vtp_bilinear_attention_forward": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                                c_int, c_int, c_int, c_int, c_void_p]),
     "vtp_sparse_bilinear_attention_forward": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,

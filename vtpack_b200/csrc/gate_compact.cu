@@ -149,7 +149,8 @@ __global__ void __launch_bounds__(128)
 write_patches_kernel(const I* __restrict__ idx, int B, int Hr, int Wr, Splits sp, int region,
                      int num_extra, const int32_t* __restrict__ counts,
                      int32_t* __restrict__ offsets, int32_t* __restrict__ patches,
-                     int64_t* __restrict__ patches64, int32_t* __restrict__ region_first) {
+                     int64_t* __restrict__ patches64, int32_t* __restrict__ region_first,
+                     int32_t* __restrict__ idx32) {
     pdl_begin();
     extern __shared__ int s_start[];   // [R + 1] first row of each region within the image
     __shared__ int s_warp[4];
@@ -186,6 +187,8 @@ write_patches_kernel(const I* __restrict__ idx, int B, int Hr, int Wr, Splits sp
     const int base = s_base;
     if (region_first)
         for (int r = tid; r < R; r += blockDim.x) region_first[(size_t)b * R + r] = base + s_start[r];
+    if (idx32)
+        for (int r = tid; r < R; r += blockDim.x) idx32[(size_t)b * R + r] = (int32_t)idx[(size_t)b * R + r];
 
     for (int e = tid; e < num_extra && patches; e += blockDim.x) {
         const int row = base + e;
@@ -283,19 +286,19 @@ extern "C" int vtp_gate_argmax(const float* logits, int rows, int n_splits, int3
 namespace vtp {
 int index_to_patch(const void* indices, int idx_is_i64, const Splits& sp, int B, int Hr, int Wr, int region,
                    int num_extra, int32_t* counts, int32_t* offsets, int32_t* patches, int64_t* patches64,
-                   int32_t* region_first, cudaStream_t st) {
+                   int32_t* region_first, cudaStream_t st, int32_t* idx32) {
     const int R = Hr * Wr;
     const size_t smem = (size_t)(R + 1) * sizeof(int);
     if (idx_is_i64) {
         const int64_t* ip = static_cast<const int64_t*>(indices);
         launch_chain(count_kernel<int64_t>, dim3(ceil_div(B, 4)), dim3(128), 0, st, ip, B, R, sp, num_extra, counts);
         launch_chain(write_patches_kernel<int64_t>, dim3(B), dim3(128), smem, st, ip, B, Hr, Wr, sp, region, num_extra, counts, offsets,
-                                                            patches, patches64, region_first);
+                                                            patches, patches64, region_first, idx32);
     } else {
         const int32_t* ip = static_cast<const int32_t*>(indices);
         launch_chain(count_kernel<int32_t>, dim3(ceil_div(B, 4)), dim3(128), 0, st, ip, B, R, sp, num_extra, counts);
         launch_chain(write_patches_kernel<int32_t>, dim3(B), dim3(128), smem, st, ip, B, Hr, Wr, sp, region, num_extra, counts, offsets,
-                                                            patches, patches64, region_first);
+                                                            patches, patches64, region_first, idx32);
     }
     return check_launch("index_to_patch");
 }
@@ -319,9 +322,10 @@ int make_splits(Splits* sp, const int* splits, int n_splits, int region) {
 }
 }  // namespace vtp
 
-extern "C" int vtp_index_to_patch(const void* indices, int idx_is_i64, const int* splits, int n_splits, int B,
-                                  int Hr, int Wr, int region, int num_extra, int32_t* counts, int32_t* offsets,
-                                  int32_t* patches, int64_t* patches64, void* stream) {
+extern "C" int vtp_index_to_patch_regions(const void* indices, int idx_is_i64, const int* splits, int n_splits, int B,
+                                          int Hr, int Wr, int region, int num_extra, int32_t* counts,
+                                          int32_t* offsets, int32_t* patches, int64_t* patches64, int32_t* idx32,
+                                          int32_t* region_first, void* stream) {
     VTP_REQUIRE(indices && splits && counts && offsets && patches, VTP_ERR_NULL, "index_to_patch: null pointer");
     VTP_REQUIRE(B > 0 && Hr > 0 && Wr > 0 && region > 0 && num_extra >= 0, VTP_ERR_SHAPE,
                 "index_to_patch: bad shape");
@@ -331,5 +335,12 @@ extern "C" int vtp_index_to_patch(const void* indices, int idx_is_i64, const int
     VTP_REQUIRE(aligned16(patches) && (!patches64 || aligned16(patches64)), VTP_ERR_ALIGN,
                 "index_to_patch: unaligned patch buffer");
     return index_to_patch(indices, idx_is_i64, sp, B, Hr, Wr, region, num_extra, counts, offsets, patches,
-                          patches64, nullptr, static_cast<cudaStream_t>(stream));
+                          patches64, region_first, static_cast<cudaStream_t>(stream), idx32);
+}
+
+extern "C" int vtp_index_to_patch(const void* indices, int idx_is_i64, const int* splits, int n_splits, int B,
+                                  int Hr, int Wr, int region, int num_extra, int32_t* counts, int32_t* offsets,
+                                  int32_t* patches, int64_t* patches64, void* stream) {
+    return vtp_index_to_patch_regions(indices, idx_is_i64, splits, n_splits, B, Hr, Wr, region, num_extra, counts,
+                                      offsets, patches, patches64, nullptr, nullptr, stream);
 }

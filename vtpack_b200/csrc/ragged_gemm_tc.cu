@@ -21,6 +21,7 @@
 // 150-196: one library bmm per image and a concatenation) and serves its backward products
 // (vtpack/layers/sparse_ops.py:30-55).
 #include "common.cuh"
+#include "ragged_gemm.h"
 #include "runtime.h"
 #include "sm100.cuh"
 
@@ -57,7 +58,6 @@ struct RaggedTcArgs {
     const bf16* a; const bf16* b; bf16* out;
     long long a_rows, b_rows, out_rows;
     int a_cols, b_cols, out_cols;
-    const int32_t* a_off; const int32_t* b_off;
     int ta, tb, tiles_n, absorb_tail;
     int heads;
 };
@@ -187,7 +187,7 @@ __device__ __forceinline__ uint64_t ragged_desc(uint32_t saddr) {
 // that hold a slice's loads in flight: the common products need far fewer than the general case.
 template <bool A_HI, int RT_BSUB>
 __global__ void __launch_bounds__(RT_THREADS, 2)
-ragged_gemm_tc_kernel(RaggedTcArgs g, int* status) {
+ragged_gemm_tc_kernel(RaggedTcArgs g, const __grid_constant__ RaggedOffsets off, int* status) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sa = base;                                   // two A slices
@@ -206,8 +206,8 @@ ragged_gemm_tc_kernel(RaggedTcArgs g, int* status) {
     float* tail_part = reinterpret_cast<float*>(base + 2 * (RT_A_BYTES + RT_B_BYTES) - RT_M * RT_TAIL * 4);
 
     const int img = blockIdx.y, head = blockIdx.z;
-    const int a0 = g.a_off[img], la = g.a_off[img + 1] - a0;
-    const int b0 = g.b_off[img], lb = g.b_off[img + 1] - b0;
+    const int a0 = off.a_at(img), la = off.a_at(img + 1) - a0;
+    const int b0 = off.b_at(img), lb = off.b_at(img + 1) - b0;
     const int M = g.ta ? g.a_cols : la;
     const int Ka = g.ta ? la : g.a_cols;
     const int Kb = g.tb ? g.b_cols : lb;
@@ -537,7 +537,7 @@ ragged_gemm_tc_kernel(RaggedTcArgs g, int* status) {
 }
 
 int ragged_gemm_tcgen05(const void* a, const void* b, void* out, int heads, int n_images, long long a_rows,
-                        int a_cols, long long b_rows, int b_cols, const int32_t* a_off, const int32_t* b_off,
+                        int a_cols, long long b_rows, int b_cols, const RaggedOffsets& off,
                         int max_m, int max_n, int ta, int tb, long long out_rows, int out_cols, cudaStream_t st) {
     VTP_REQUIRE(aligned16(a) && aligned16(b), VTP_ERR_ALIGN,
                 "batched_sparse_gemm (tcgen05): the operand arrays must start on a 16-byte boundary");
@@ -545,7 +545,7 @@ int ragged_gemm_tcgen05(const void* a, const void* b, void* out, int heads, int 
     g.a = static_cast<const bf16*>(a); g.b = static_cast<const bf16*>(b); g.out = static_cast<bf16*>(out);
     g.a_rows = a_rows; g.b_rows = b_rows; g.out_rows = out_rows;
     g.a_cols = a_cols; g.b_cols = b_cols; g.out_cols = out_cols;
-    g.a_off = a_off; g.b_off = b_off; g.ta = ta; g.tb = tb; g.heads = heads;
+    g.ta = ta; g.tb = tb; g.heads = heads;
     g.tiles_n = ceil_div(max_n, RT_N);
     // a few columns beyond the last full tile stay with that tile (CUDA-core dot products from the staged
     // slices; needs both operands' rows along the reduction axis)
@@ -560,7 +560,7 @@ int ragged_gemm_tcgen05(const void* a, const void* b, void* out, int heads, int 
     auto launch = [&](auto kern) -> int {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_SMEM);
         if (e != cudaSuccess) return fail((int)e, "batched_sparse_gemm (tcgen05): shared memory: %s", cudaGetErrorString(e));
-        kern<<<grid, RT_THREADS, RT_SMEM, st>>>(g, device_status_ptr());
+        kern<<<grid, RT_THREADS, RT_SMEM, st>>>(g, off, device_status_ptr());
         return VTP_OK;
     };
     int rc;

@@ -75,7 +75,7 @@ int region_gate(const RegionGateArgs& a, int dtype, cudaStream_t st);
 // Patch list + per-region first rows (internal form of vtp_index_to_patch).
 int index_to_patch(const void* indices, int idx_is_i64, const Splits& sp, int B, int Hr, int Wr, int region,
                    int num_extra, int32_t* counts, int32_t* offsets, int32_t* patches, int64_t* patches64,
-                   int32_t* region_first, cudaStream_t st);
+                   int32_t* region_first, cudaStream_t st, int32_t* idx32 = nullptr);
 
 // Per-image query counts of the grain indices `idx` [B, R]; with `logits` [B, R, n_splits] the indices are their
 // argmax (lowest index wins) and are written.  One warp per image.

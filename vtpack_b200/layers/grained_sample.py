@@ -42,22 +42,20 @@ def grained_sample_index_to_patch(indices, split_sizes, region_size, num_extra_t
     p32 = torch.empty(l_max, 4, dtype=torch.int32, device=dev)
     p64 = torch.empty(l_max, 4, dtype=torch.int64, device=dev)
     arr = (ctypes.c_int * len(splits))(*splits)
-    _lib.check(_lib.lib().vtp_index_to_patch(
+    # what the region-parallel gradient kernel needs instead of the list: the grain index of every region and
+    # the packed row of its first patch (the image's first row + its extra tokens + the patches of the regions
+    # in front of it)
+    idx32, first = torch.empty(2, B, Hr * Wr, dtype=torch.int32, device=dev)
+    _lib.check(_lib.lib().vtp_index_to_patch_regions(
         ptr(indices), 1 if is64 else 0, arr, len(splits), B, Hr, Wr, int(region_size),
-        int(num_extra_tokens), ptr(counts), ptr(offsets), ptr(p32), ptr(p64), stream_ptr(dev)))
+        int(num_extra_tokens), ptr(counts), ptr(offsets), ptr(p32), ptr(p64), ptr(idx32), ptr(first),
+        stream_ptr(dev)))
     batch_lengths = counts.to("cpu", torch.int64)
     L = int(batch_lengths.sum())
     patches = p64[:L]
     patches._vtp_i32 = p32[:L]
     patches._vtp_offsets = offsets
-    # what the region-parallel gradient kernel needs instead of the list: the grain index of every region and
-    # the packed row of its first patch (the image's first row + its extra tokens + the patches of the regions
-    # in front of it)
-    per_side = torch.tensor(splits, dtype=torch.int32, device=dev)[indices.reshape(B, -1).clamp(0, len(splits) - 1)]
-    per_region = per_side * per_side
-    first = offsets[:B, None] + int(num_extra_tokens) + torch.cumsum(per_region, 1, dtype=torch.int32) - per_region
-    patches._vtp_regions = (indices.reshape(B, -1).to(torch.int32).contiguous(), first.to(torch.int32).contiguous(),
-                            splits, int(region_size), Hr, Wr, int(num_extra_tokens))
+    patches._vtp_regions = (idx32, first, splits, int(region_size), Hr, Wr, int(num_extra_tokens))
     return patches, batch_lengths
 
 

@@ -38,32 +38,45 @@ def batched_sparse_attention(q, k, v, q_lengths, scale, flags: int = 0):
     return out.permute(1, 0, 2)
 
 
-def _offsets(lengths, device):
-    lengths = lengths.to("cpu", torch.int64)
-    off = torch.zeros(lengths.numel() + 1, dtype=torch.int32)
-    off[1:] = torch.cumsum(lengths, 0)
-    return off.to(device, non_blocking=True), int(off[-1]), int(lengths.max()) if lengths.numel() else 0
+class _Lengths:
+    """The per-image row counts of an operand, read once for the forward and the backward products."""
+
+    def __init__(self, lengths):
+        self.host = lengths.to("cpu", torch.int64).contiguous().clone()
+        values = self.host.tolist()
+        self.n, self.total = len(values), sum(values)
+        self.max, self.min = (max(values), min(values)) if values else (0, 0)
+
+    def offsets(self, device):
+        off = torch.zeros(self.n + 1, dtype=torch.int32)
+        off[1:] = torch.cumsum(self.host, 0)
+        return off.to(device, non_blocking=True)
 
 
-def _ragged_gemm(a, b, a_lengths, b_lengths, ta, tb):
-    """One launch of ``vtp_batched_sparse_gemm``: a [H,La,ka], b [H,Lb,kb] -> the per-image products
+_INLINE_IMAGES = 512            # the library passes the offsets of up to this many images with the launch
+
+
+def _ragged_gemm(a, b, la, lb, ta, tb):
+    """One launch of the ragged product: a [H,La,ka], b [H,Lb,kb] -> the per-image products
     stacked along dim 1 (``batched_sparse_gemm.cu:150-196``)."""
     require_cuda(a, b)
     a, b = a.contiguous(), b.contiguous()
-    H, B = a.shape[0], a_lengths.numel()
-    a_off, a_total, a_max = _offsets(a_lengths, a.device)
-    b_off, b_total, b_max = _offsets(b_lengths, a.device)
-    assert a_total <= a.shape[1] and b_total <= b.shape[1], "lengths exceed the rows of the operands"
+    H, B = a.shape[0], la.n
+    assert la.total <= a.shape[1] and lb.total <= b.shape[1], "lengths exceed the rows of the operands"
     if tb:
-        assert b.shape[1] % B == 0 and int(b_lengths.min()) == b_max, \
+        assert b.shape[1] % B == 0 and lb.min == lb.max, \
             "a transposed b needs the same number of rows in every image"
-    out_rows = B * a.shape[2] if ta else a_total
-    out_cols = b_max if tb else b.shape[2]
+    out_rows = B * a.shape[2] if ta else la.total
+    out_cols = lb.max if tb else b.shape[2]
     out = torch.empty(H, out_rows, out_cols, dtype=a.dtype, device=a.device)
-    _lib.check(_lib.lib().vtp_batched_sparse_gemm(
-        ptr(a), ptr(b), ptr(out), dtype_code(a.dtype), H, B, a.shape[1], a.shape[2], b.shape[1], b.shape[2],
-        ptr(a_off), ptr(b_off), a_max, b_max, int(bool(ta)), int(bool(tb)), out_rows, out_cols,
-        stream_ptr(a.device)))
+    lib = _lib.lib()
+    head = (ptr(a), ptr(b), ptr(out), dtype_code(a.dtype), H, B, a.shape[1], a.shape[2], b.shape[1], b.shape[2])
+    tail = (int(bool(ta)), int(bool(tb)), out_rows, out_cols, stream_ptr(a.device))
+    if 0 < B <= _INLINE_IMAGES and la.min >= 0 and lb.min >= 0 and lb.n == B:
+        _lib.check(lib.vtp_batched_sparse_gemm_lengths(*head, ptr(la.host), ptr(lb.host), *tail))
+    else:
+        a_off, b_off = la.offsets(a.device), lb.offsets(a.device)
+        _lib.check(lib.vtp_batched_sparse_gemm(*head, ptr(a_off), ptr(b_off), la.max, lb.max, *tail))
     return out
 
 
@@ -75,9 +88,11 @@ class _BatchedSparseGEMM(Function):
     def forward(ctx, a, b, a_lengths, b_lengths, is_a_transposed, is_b_transposed):
         a, b = a.contiguous(), b.contiguous()
         ctx.ta, ctx.tb = bool(is_a_transposed), bool(is_b_transposed)
-        ctx.lengths = (a_lengths, b_lengths)
+        la = _Lengths(a_lengths)
+        lb = la if b_lengths is a_lengths else _Lengths(b_lengths)
+        ctx.lengths = (la, lb)
         ctx.save_for_backward(a, b)
-        return _ragged_gemm(a, b, a_lengths, b_lengths, ctx.ta, ctx.tb)
+        return _ragged_gemm(a, b, la, lb, ctx.ta, ctx.tb)
 
     @staticmethod
     @once_differentiable
