@@ -493,3 +493,37 @@ def test_linear_fp32_split_terms_are_as_accurate_as_fmaf_chains(vl, M, N, K, gel
     e = [float((t - ref).norm() / ref.norm()) for t in (got, chain)]
     assert e[0] <= e[1] + 2.0 ** -24
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(70, 100, 64), (300, 384, 384), (130, 384, 768), (20000, 256, 320)])
+def test_linear_fp32_non_finite_operands(vl, M, N, K):
+    """Infinities, NaN and values whose first bf16 term rounds up to infinity, in rows of both operands (whole
+    reductions, ones split over two and four CTAs, both tile widths): infinite, NaN and finite results where the
+    fmaf chain of the CUDA-core kernel has them, other rows untouched."""
+    from vtpack_b200 import _lib
+    from vtpack_b200.runtime import ptr, stream_ptr
+    g = torch.Generator(DEV).manual_seed(K)
+    x = torch.randn(M, K, device=DEV, generator=g)
+    w = torch.randn(N, K, device=DEV, generator=g) * 0.1
+    inf = float("inf")
+    x[1, 3], x[5, K - 1], x[33, 0], x[M - 1, 7] = inf, -inf, float("nan"), 3.4e38
+    x[40, 1], x[40, 2] = inf, -inf
+    x[41] = 0.0
+    x[41, 2], x[42, 0] = inf, 1e30
+    w[2, 3], w[N - 1, 5] = 0.0, inf
+    w[4, 7] = 1e-3
+
+    def run(flags):
+        y = torch.full((M, N), 7.0, device=DEV)
+        _lib.check(_lib.lib().vtp_linear(ptr(x), K, ptr(w), None, None, 0, ptr(y), N, 0, M, None, N, K, flags,
+                                         stream_ptr(x.device)))
+        return y
+
+    got, chain = run(0), run(_lib.FLAG_CUDA_CORES)
+    assert torch.equal(got.isnan(), chain.isnan()) and torch.equal(got.isposinf(), chain.isposinf())
+    assert torch.equal(got.isneginf(), chain.isneginf()) and bool(chain.isposinf().any())
+    ok = chain.isfinite()
+    mag = (x.abs().double().nan_to_num(0, 0, 0) @ w.abs().double().nan_to_num(0, 0, 0).t())[ok]
+    # a chain of K roundings on one side, the split's bound (see above) on the other
+    assert bool(((got.double() - chain.double())[ok].abs() <= (K + 4) * 2.0 ** -23 * mag).all())
+    assert _lib.device_status() == 0

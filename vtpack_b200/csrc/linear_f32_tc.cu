@@ -26,7 +26,10 @@
 //   eight warps  add finished accumulators to their registers (one row x BN / 2 columns per thread); after the last
 //                k-block bias / GELU / residual and 128-byte stores through a per-warp shared-memory transpose
 //
-// Non-finite inputs give NaN (inf - inf in the split).
+// An infinite or NaN operand (and a finite one within 2^-9 of the largest fp32 number, whose first term rounds up to
+// inf) turns every sum it enters into NaN through its second term, inf - inf.  Sums that come out non-finite are
+// therefore worked out again as a plain fmaf chain over the fp32 operands (redo_nonfinite): results are infinite, NaN
+// or finite where that chain's are.  The check is one fmaf per output.
 //
 // Replaces nn.Linear q/kv/proj/fc1/fc2/head, nn.GELU and the residual adds of
 // vtpack/models/dge/deit_dge.py:38-44,72-74,96,127-128 when the model runs in fp32.
@@ -93,6 +96,39 @@ __device__ __forceinline__ void split8(const float4& x0, const float4& x1, uint4
     }
 #pragma unroll
     for (int p = 0; p < 3; ++p) t[p] = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+}
+
+// acc: NC columns n0.. of row m0 + lane.  Rows with a sum that is not finite are worked out again, a row at a time, a
+// lane per column (K and lda are multiples of four floats, see linear_f32_tc_supported).
+template <int NC>
+__device__ __forceinline__ void redo_nonfinite(float (&acc)[NC], const F32Args& g, int M, int m0, int n0, int lane) {
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < NC; ++i) t = fmaf(acc[i], 0.f, t);              // inf * 0 and NaN * 0 are NaN
+    unsigned bad = __ballot_sync(0xffffffffu, t != t && m0 + lane < M);
+    while (bad) {
+        const int r = __ffs(bad) - 1;
+        bad &= bad - 1;
+        const float4* a = reinterpret_cast<const float4*>(g.a + (size_t)(m0 + r) * g.lda);
+#pragma unroll
+        for (int c0 = 0; c0 < NC; c0 += 32) {
+            const int n = n0 + c0 + lane;
+            float s = 0.f;
+            if (c0 + lane < NC && n < g.N) {
+                const float4* w = reinterpret_cast<const float4*>(g.w + (size_t)n * g.K);
+#pragma unroll 1
+                for (int k = 0; k < g.K / 4; ++k) {
+                    const float4 x = __ldg(a + k), y = __ldg(w + k);
+                    s = fmaf(x.x, y.x, s); s = fmaf(x.y, y.y, s); s = fmaf(x.z, y.z, s); s = fmaf(x.w, y.w, s);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 32 && c0 + i < NC; ++i) {
+                const float v = __shfl_sync(0xffffffffu, s, i);
+                if (lane == r) acc[c0 + i] = v;
+            }
+        }
+    }
 }
 
 // SPLIT: CTAs of a cluster that share a tile's reduction (1: none).
@@ -321,6 +357,7 @@ linear_f32_tc_kernel(const F32Args g, int* status) {
                     for (int d = 0; d < SPLIT; ++d)
                         if (d != rank) mbar_arrive_release_cluster(mapa_u32(smem_u32(part_free), d));
                 }
+                redo_nonfinite<SC>(own, g, M, m0, n0 + rank * SC, lane);
                 const int m = m0 + lane;
                 if (m >= M) continue;
                 float* y = g.y + map_out_row(g.rm, m) * g.ldy;
@@ -348,6 +385,7 @@ linear_f32_tc_kernel(const F32Args g, int* status) {
                 }
                 continue;
             }
+            redo_nonfinite<CW>(acc, g, M, m0, n0, lane);
             // 32 columns at a time through the warp's transpose buffer (rows of eight 16-byte chunks, XOR-swizzled):
             // a lane then holds four columns of a row and eight lanes a whole 128-byte line
 #pragma unroll
