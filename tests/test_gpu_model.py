@@ -482,3 +482,45 @@ def test_repeated_forwards_replay_one_capture(kind, dtype):
     for _ in range(3):
         same(m, ref5, imgs[3][1])
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("kind", ["deit", "pvt"])
+def test_replayed_forward_follows_settings_and_streams(kind):
+    """What the launches take by value (softmax scale, LayerNorm epsilon) may change between calls of a model whose
+    launches have been captured, and the calls may come from different streams."""
+    from vtpack_b200 import synthetic
+    from vtpack_b200.models.dge.pvt_dge import pvt_dge_s124_tiny_256
+
+    def make():
+        if kind == "deit":
+            return synthetic.build_model("tiny", DEV, torch.bfloat16, depth=2, seed=0)
+        m = pvt_dge_s124_tiny_256()
+        m.load_state_dict(O.make_pvt_state_dict(O.PVT_CONFIGS["tiny"], seed=0), strict=True)
+        return m.eval().to(device=DEV, dtype=torch.bfloat16)
+
+    def scale(m):
+        for blk in (m.blocks if kind == "deit" else m.block1):
+            blk.attn.scale *= 4.0
+
+    def eps(m):
+        m.norm.eps = 0.1
+
+    img = O.make_images(2, 256, seed=3).to(DEV)
+    m, changes = make(), []
+    for change in (None, scale, eps):
+        if change is not None:
+            change(m)
+            changes.append(change)
+        fresh = make()
+        for c in changes:
+            c(fresh)
+        want = fresh(img)
+        for _ in range(3):
+            assert torch.equal(m(img), want)
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            got = m(img)
+        torch.cuda.current_stream().wait_stream(side)
+        assert torch.equal(got, want)
+    assert not torch.equal(make()(img), want)

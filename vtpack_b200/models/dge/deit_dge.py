@@ -485,16 +485,14 @@ class VisionTransformer(nn.Module):
         stream = stream_ptr(x.device)
         plan = None
         if use_plans and not self.trace:
-            plan = self._plans.get((B, opt.gate_image_bias, int(self.flags)),
+            plan = self._plans.get((bytes(s), opt.gate_image_bias),       # all that the trunk takes by value
                                    lambda p: p.scratch_gen == scratch_generation(x.device),
                                    lambda: self._capture_trunk(launch, ws, B, x.device))
         if plan is not None:
             # the one kernel that reads the images and the one that writes the logits are ordinary launches; what
             # lies between them takes its addresses from the workspace and the weights and is replayed
             launch(_lib.PART_FRONT, plan.counts, stream)
-            plan.graph.replay()
-            launch(_lib.PART_HEAD, plan.counts, stream)
-            counts = plan.counts.clone()
+            counts = plan.replay(x.device, lambda: launch(_lib.PART_HEAD, plan.counts, stream))
         else:
             counts = torch.empty(self.depth, B, dtype=torch.int32, device=x.device)
             if self.trace:
@@ -520,9 +518,7 @@ class VisionTransformer(nn.Module):
         counts = torch.empty(self.depth, B, dtype=torch.int32, device=device)
         graph = capture_launches(device, lambda stream: launch(_lib.PART_TRUNK, counts, stream))
         keep = (ws, counts, self.gate_image_bias, self._pack.tensors, [blk._pack.tensors for blk in self.blocks])
-        plan = _CapturedForward(graph, keep, scratch_generation(device))
-        plan.counts = counts
-        return plan
+        return _CapturedTrunk(graph, keep, scratch_generation(device), counts)
 
     def _forward_train(self, x):
         """``deit_dge.py:267-299`` with ``self.training`` (cls token, no distillation token)."""
@@ -554,6 +550,25 @@ class _CapturedForward:
 
     def __init__(self, graph, keep, scratch_gen):
         self.graph, self.keep, self.scratch_gen = graph, keep, scratch_gen
+
+
+class _CapturedTrunk(_CapturedForward):
+    """A captured trunk and the query counts its launches leave behind."""
+
+    def __init__(self, graph, keep, scratch_gen, counts):
+        super().__init__(graph, keep, scratch_gen)
+        self.counts = counts
+        self.stream = torch.cuda.current_stream(counts.device)        # the stream the counts were allocated on
+
+    def replay(self, device, then=None):
+        """Replays the launches, runs `then`, and returns a copy of the counts."""
+        cur = torch.cuda.current_stream(device)
+        if cur != self.stream:
+            self.counts.record_stream(cur)        # the plan may be dropped while this stream still works on it
+        self.graph.replay()
+        if then is not None:
+            then()
+        return self.counts.clone()
 
 
 def _graph_forward(model, x, logits_out):

@@ -20,7 +20,7 @@ from ... import _lib
 from ...layers import DynamicGrainedEncoder, batched_sparse_attention, batched_sparse_gemm
 from ...runtime import (LaunchPlans, ParamWatch, capture_launches, dtype_code, ptr, require_cuda, scratch,
                         scratch_generation, stream_ptr)
-from .deit_dge import DropPath, Mlp, _CapturedForward, _WeightPack, _pack_block, _shape_struct
+from .deit_dge import DropPath, Mlp, _CapturedTrunk, _WeightPack, _pack_block, _shape_struct
 
 __all__ = ["Mlp", "Attention", "Block", "PatchEmbed", "PyramidVisionTransformer",
            "pvt_dge_s124_tiny_256", "pvt_dge_s124_small_256", "pvt_dge_s124_medium_256", "pvt_dge_s124_large_256"]
@@ -370,6 +370,20 @@ class PyramidVisionTransformer(nn.Module):
             self._pack.watch = ParamWatch(self)
         return self._pack.watch.generation()
 
+    def _launch_config(self):
+        """What the blocks' launches take by value besides shapes: it may be changed between calls."""
+        config = []
+        for i in range(self.num_stages):
+            config.append(getattr(self, f"patch_embed{i + 1}").norm.eps)
+            for blk in getattr(self, f"block{i + 1}"):
+                att = blk.attn
+                config += [blk.flags, blk.fold_layernorm, blk.fold_q_fc1, blk.norm1.eps, att.scale, att.num_heads,
+                           att.sr_ratio, tuple(blk.split_sizes)]
+                if att.sr_ratio > 1:
+                    config.append(att.norm.eps)
+        config.append(getattr(self.norm, "eps", None))
+        return tuple(config)
+
     def _scratch_gen(self, device):
         return scratch_generation(device), scratch_generation(device, "pvt")
 
@@ -436,13 +450,12 @@ class PyramidVisionTransformer(nn.Module):
             return outputs
         plan = None
         if use_plans:
-            plan = self._plans.get((B, S, dtype, self._param_generation()),
+            plan = self._plans.get((B, S, dtype, self._param_generation(), self._launch_config()),
                                    lambda p: p.scratch_gen == self._scratch_gen(dev),
                                    lambda: self._capture_trunk(B, sides, ld, dtype, cols, y, tokens, dev))
         front()
         if plan is not None:
-            plan.graph.replay()
-            counts = plan.counts.clone()
+            counts = plan.replay(dev)
         else:
             counts = torch.empty(sum(self.depths), B, dtype=torch.int32, device=dev)
             self._trunk(B, sides, dtype, self._trunk_consts(sides, dtype, ld), cols, y, tokens, counts, dev, stream)
@@ -457,9 +470,7 @@ class PyramidVisionTransformer(nn.Module):
         counts = torch.empty(sum(self.depths), B, dtype=torch.int32, device=dev)
         consts = self._trunk_consts(sides, dtype, ld)
         graph = capture_launches(dev, lambda stream: self._trunk(B, sides, dtype, consts, cols, y, tokens, counts, dev, stream))
-        plan = _CapturedForward(graph, (consts,) + self._keep(dev), self._scratch_gen(dev))
-        plan.counts = counts
-        return plan
+        return _CapturedTrunk(graph, (consts,) + self._keep(dev), self._scratch_gen(dev), counts)
 
     def _set_states(self, B, sides, counts):
         self.last_counts = list(counts.unbind(0))
