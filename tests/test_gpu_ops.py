@@ -227,6 +227,24 @@ def test_attention_bf16_tensor_cores(vl, B, N, h, lens):
     assert rel_err(got2.float(), ref2) < 1e-2
 
 
+@pytest.mark.parametrize("N", [16, 17, 31, 260, 271, 527])
+@pytest.mark.parametrize("far", [False, True])
+def test_attention_bf16_tail_keys(vl, N, far):
+    """0 to 15 keys behind the tensor-core part, which start the online softmax: against float32; with `far`, a last key
+    whose scores are -inf (weight zero, whatever comes first).  Bound as above."""
+    _, layers = vl
+    g = torch.Generator().manual_seed(N)
+    lens = [5, 130]
+    q = torch.randn(2, sum(lens), 64, generator=g).bfloat16()
+    k, v = (torch.randn(2, 2, N, 64, generator=g).bfloat16() for _ in range(2))
+    if far:
+        q = q.abs() + 0.5
+        k[:, :, -1] = -3e38
+    ref = O.batched_sparse_attention_forward(q.float(), k.float(), v.float(), torch.tensor(lens), 64 ** -0.5)
+    got = layers.batched_sparse_attention(q.to(DEV), k.to(DEV), v.to(DEV), torch.tensor(lens), 64 ** -0.5)
+    assert torch.isfinite(ref).all() and rel_err(got.float(), ref) < 8e-3
+
+
 def test_attention_strided_views(vl):
     """q / k / v as permuted views of Linear outputs, as the model passes them."""
     _, layers = vl

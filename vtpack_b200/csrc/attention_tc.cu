@@ -14,8 +14,8 @@
 //   O_c = P V_c        tcgen05.mma with A = P from TMEM and B = V chunk as an MN-major operand
 //                      straight from the TMA image of the [keys, d] rows; accumulator in TMEM
 //                      columns [128, 192)
-//   O  = O*alpha + O_c in registers of the softmax threads (online-softmax rescale), then the
-//                      tail keys, the 1/rowsum and the bf16 store.
+//   O  = O*alpha + O_c in registers of the softmax threads (online-softmax rescale, started by the
+//                      tail keys), then the 1/rowsum and the bf16 store.
 // Warp 0 lane 0 issues TMA (Q is double-buffered so the next item's Q and K stream in during
 // the current softmax), warp 1 lane 0 issues MMA, warps 2-5 do softmax and output.
 // q, k, v are read in place from the Linear outputs through strided tensor maps.
@@ -117,6 +117,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         mbar_init(o_full, 1); mbar_init(o_free, QT);
         *abort_flag = 0;
         fence_barrier_init();
+        prefetch_tmap(&tmap_q);
+        prefetch_tmap(&tmap_k);
+        prefetch_tmap(&tmap_v);
     }
     if (warp == 0) {
         tmem_alloc(tmem_slot, ATT_TMEM_COLS);
@@ -169,9 +172,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     if (warp == 0) {
         if (lane == 0) {
             // ------------------------------------------------------------ TMA producer
-            prefetch_tmap(&tmap_q);
-            prefetch_tmap(&tmap_k);
-            prefetch_tmap(&tmap_v);
             const uint32_t kv_bytes = (uint32_t)KC * HD * 2;
             int li = 0, g = 0;
             bool ok = true;
@@ -266,6 +266,45 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
             float o[HD];
 #pragma unroll
             for (int i = 0; i < HD; ++i) o[i] = 0.f;
+            const uint8_t* qrow = base + SM_Q + qb * (QT * HD * 2) + r * 128;
+            if (tail > 0 && live) {
+                // ---- the last n_keys % 16 keys on CUDA cores, one online-softmax step per key.  They come first: their
+                // rows arrived with Q, and the scores of the chunk are still being loaded and multiplied (behind the
+                // chunk this step took 1500 of the 17 k cycles of a lone item: DeiT-Ti, one image, 527 -> 515 us).
+                const uint8_t* tb = base + SM_TAIL + qb * (2 * TAIL_ROWS * HD * 2);
+                for (int t = 0; t < tail; ++t) {
+                    const uint4* krow = reinterpret_cast<const uint4*>(tb + t * (HD * 2));
+                    const uint4* vrow = reinterpret_cast<const uint4*>(tb + (TAIL_ROWS + t) * (HD * 2));
+                    float d4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int ch = 0; ch < HD / 8; ++ch) {
+                        Vec<bf16> qv, kv;
+                        float qf[8], kf[8];
+                        qv.raw = *reinterpret_cast<const uint4*>(qrow + ((ch ^ (r & 7)) << 4));
+                        kv.raw = krow[ch];
+                        qv.to_float(qf);
+                        kv.to_float(kf);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) d4[i & 3] = fmaf(qf[i], kf[i], d4[i & 3]);
+                    }
+                    const float sdot = (d4[0] + d4[1]) + (d4[2] + d4[3]);
+                    const float m_new = fmaxf(m, sdot);
+                    const float m_at = m_new == -INFINITY ? 0.f : m_new;      // (a score of -inf has weight zero)
+                    const float alpha = fast_exp2((m - m_at) * scale_log2e);
+                    const float p = fast_exp2((sdot - m_at) * scale_log2e);
+                    l = l * alpha + p;
+                    m = m_new;
+#pragma unroll
+                    for (int ch = 0; ch < HD / 8; ++ch) {
+                        Vec<bf16> vv;
+                        float vf[8];
+                        vv.raw = vrow[ch];
+                        vv.to_float(vf);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) o[8 * ch + i] = fmaf(o[8 * ch + i], alpha, p * vf[i]);
+                    }
+                }
+            }
             for (int c = 0; c < n_chunks && ok; ++c, ++g) {
                 const uint32_t ph = g & 1;
                 ok = mbar_wait(s_full, ph, abort_flag, status, STATUS_ATTN_SOFTMAX);
@@ -306,7 +345,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
                 }
                 const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
                 const float m_new = fmaxf(m, mx);
-                const float alpha = fast_exp2((m - m_new) * scale_log2e);       // 0 on the first chunk
+                const float alpha = fast_exp2((m - m_new) * scale_log2e);       // 0 while m is -inf
                 const float mb = m_new * scale_log2e;
                 float ls4[4] = {0.f, 0.f, 0.f, 0.f};
                 for (int blk = 0; blk < nblk; ++blk) {
@@ -360,41 +399,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
             if (!live) {
                 mbar_arrive(&q_free[qb]);
                 continue;
-            }
-            const uint8_t* qrow = base + SM_Q + qb * (QT * HD * 2) + r * 128;
-            if (tail > 0) {
-                // ---- the last n_keys % 16 keys on CUDA cores, one online-softmax step per key
-                const uint8_t* tb = base + SM_TAIL + qb * (2 * TAIL_ROWS * HD * 2);
-                for (int t = 0; t < tail; ++t) {
-                    const uint4* krow = reinterpret_cast<const uint4*>(tb + t * (HD * 2));
-                    const uint4* vrow = reinterpret_cast<const uint4*>(tb + (TAIL_ROWS + t) * (HD * 2));
-                    float sdot = 0.f;
-#pragma unroll
-                    for (int ch = 0; ch < HD / 8; ++ch) {
-                        Vec<bf16> qv, kv;
-                        float qf[8], kf[8];
-                        qv.raw = *reinterpret_cast<const uint4*>(qrow + ((ch ^ (r & 7)) << 4));
-                        kv.raw = krow[ch];
-                        qv.to_float(qf);
-                        kv.to_float(kf);
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) sdot = fmaf(qf[i], kf[i], sdot);
-                    }
-                    const float m_new = fmaxf(m, sdot);
-                    const float alpha = fast_exp2((m - m_new) * scale_log2e);
-                    const float p = fast_exp2((sdot - m_new) * scale_log2e);
-                    l = l * alpha + p;
-                    m = m_new;
-#pragma unroll
-                    for (int ch = 0; ch < HD / 8; ++ch) {
-                        Vec<bf16> vv;
-                        float vf[8];
-                        vv.raw = vrow[ch];
-                        vv.to_float(vf);
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) o[8 * ch + i] = fmaf(o[8 * ch + i], alpha, p * vf[i]);
-                    }
-                }
             }
             // ---- normalise, then out through the warp's own 32 rows of the Q tile (no longer needed) so that
             // eight lanes write one full 128-byte line of a row instead of every lane a piece of its own row
