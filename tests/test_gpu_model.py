@@ -524,3 +524,33 @@ def test_replayed_forward_follows_settings_and_streams(kind):
         torch.cuda.current_stream().wait_stream(side)
         assert torch.equal(got, want)
     assert not torch.equal(make()(img), want)
+
+
+@pytest.mark.parametrize("kind", ["deit", "pvt"])
+def test_forward_with_swapped_in_weights_updated_in_place(kind):
+    """Weights handed over by functional_call and updated in place between calls (a moving average): every forward, the
+    replayed ones among them, uses their current values."""
+    from torch.func import functional_call
+
+    from vtpack_b200 import synthetic
+    from vtpack_b200.models.dge.pvt_dge import pvt_dge_s124_tiny_256
+
+    def make():
+        if kind == "deit":
+            return synthetic.build_model("tiny", DEV, torch.bfloat16, depth=2, seed=0)
+        m = pvt_dge_s124_tiny_256()
+        m.load_state_dict(O.make_pvt_state_dict(O.PVT_CONFIGS["tiny"], seed=0), strict=True)
+        return m.eval().to(device=DEV, dtype=torch.bfloat16)
+
+    img = O.make_images(2, 256, seed=3).to(DEV)
+    m, fresh = make(), make()
+    ema = {k: v.detach().clone() for k, v in m.named_parameters()}
+    for step in range(3):
+        if step:
+            for t in ema.values():
+                if t.is_floating_point():
+                    t.mul_(0.9)
+        fresh.load_state_dict(ema, strict=False)
+        want = fresh._forward_eval(img, use_plans=False)
+        for _ in range(3):
+            assert torch.equal(functional_call(m, ema, (img,)), want)

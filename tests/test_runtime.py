@@ -1,0 +1,39 @@
+"""CPU tests of the host-side plumbing: what makes a model pack its weights again and drop its captured launches."""
+import torch
+from torch.func import functional_call
+
+from vtpack_b200.models.dge import deit_dge
+from vtpack_b200.models.dge.deit_dge import _param_key
+
+
+def _tiny():
+    return deit_dge.VisionTransformer(img_size=64, patch_size=16, embed_dim=64, depth=2, num_heads=1, num_classes=10,
+                                      split_sizes=[4, 2, 1])
+
+
+class _Keyed(torch.nn.Module):
+    """A model whose forward returns the key of its weight pack."""
+
+    def __init__(self, model):
+        super().__init__()
+        self.model = model
+
+    def forward(self):
+        return _param_key(self.model, torch.bfloat16)
+
+
+def test_weight_key_follows_tensors_in_the_parameters_place():
+    """functional_call puts plain tensors where the parameters are: an in-place update of one between two calls (a moving
+    average) makes another key, the same tensors untouched the same key."""
+    m = _Keyed(_tiny())
+    ema = {k: v.detach().clone() for k, v in m.named_parameters()}
+    keys = [functional_call(m, ema, ())]
+    assert functional_call(m, ema, ()) == keys[0]
+    for name in ("model.head.weight", "model.blocks.1.attn.q.bias", "model.cls_token"):
+        ema[name].mul_(0.5)
+        keys.append(functional_call(m, ema, ()))
+    keys.append(m())                                         # the module's own parameters again
+    assert len(set(keys)) == len(keys)
+    with torch.no_grad():
+        m.model.head.weight.add_(1.0)
+    assert m() not in keys

@@ -75,7 +75,8 @@ _version_of = attrgetter("_version")
 class ParamWatch:
     """Tells whether a module's parameters are still the ones seen before, without walking the module tree: a
     snapshot of every owner's parameters and submodules is compared by identity, then versions and addresses.
-    ``generation()`` returns a number that changes with any replacement, in-place update or move of a parameter
+    ``generation()`` returns a number that changes with any replacement, in-place update or move of a parameter,
+    plain tensors in a parameter's place (``torch.func.functional_call`` puts them there) among them
     (48 us for a 12-block model where building a key from ``module.parameters()`` takes 320 us)."""
 
     def __init__(self, module):
@@ -93,7 +94,7 @@ class ParamWatch:
             self._owners = [d for d in dicts for _ in d]
             self._names = [n for d in dicts for n in d]
             self._kept = [v for d in dicts for v in d.values()]
-            self._params = [v for v in self._kept if isinstance(v, torch.nn.Parameter)]
+            self._params = [v for v in self._kept if isinstance(v, torch.Tensor)]
             self._state = None
         state = (list(map(_version_of, self._params)), list(map(torch.Tensor.data_ptr, self._params)))
         if state != self._state:
