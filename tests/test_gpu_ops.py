@@ -1,5 +1,6 @@
 """GPU parity of the individual ops, called through the C ABI, against the CPU oracle."""
 import ctypes
+import math
 
 import pytest
 import torch
@@ -243,6 +244,39 @@ def test_attention_bf16_tail_keys(vl, N, far):
     ref = O.batched_sparse_attention_forward(q.float(), k.float(), v.float(), torch.tensor(lens), 64 ** -0.5)
     got = layers.batched_sparse_attention(q.to(DEV), k.to(DEV), v.to(DEV), torch.tensor(lens), 64 ** -0.5)
     assert torch.isfinite(ref).all() and rel_err(got.float(), ref) < 8e-3
+
+
+@pytest.mark.parametrize("N", [17, 20, 257])
+def test_attention_bf16_tail_scores_are_one_chain(vl, N):
+    """The score of a key behind the tensor-core part is formed in channel order: large terms that cancel next to each
+    other leave the small ones behind them whole.  Every other score is 0, so the last key's weight shows its score of
+    3; weights and output are rounded to bf16 (2^-9 each, the sums in fp32)."""
+    _, layers = vl
+    k = torch.zeros(1, 1, N, 64)
+    k[..., -1, :2] = torch.tensor([2.0 ** 24, -2.0 ** 24])
+    k[..., -1, [4, 8, 12]] = 1.0
+    v = torch.zeros(1, 1, N, 64)
+    v[..., -1, :] = 1.0
+    q = torch.ones(1, 40, 64)
+    got = layers.batched_sparse_attention(q.bfloat16().to(DEV), k.bfloat16().to(DEV), v.bfloat16().to(DEV), torch.tensor([40]), 1.0)
+    w = math.exp(3.0) / (N - 1 + math.exp(3.0))
+    assert float((got.float() - w).abs().max()) < 2.0 ** -8 * w
+
+
+@pytest.mark.parametrize("dtype,bound", [(torch.bfloat16, 8e-3)])
+@pytest.mark.parametrize("N,far", [(17, 16), (33, 32), (257, 256), (257, 128), (400, 200), (600, 300), (1025, 600)])
+def test_attention_leading_keys_of_weight_zero(vl, dtype, bound, N, far):
+    """The first `far` keys of every row have scores of -inf (whole chunks of them): weight zero, and the row is finite as
+    long as one other score is."""
+    _, layers = vl
+    g = torch.Generator().manual_seed(N)
+    lens = [5, 130]
+    q = (torch.randn(2, sum(lens), 64, generator=g).abs() + 0.5).to(dtype)
+    k, v = (torch.randn(2, 2, N, 64, generator=g).to(dtype) for _ in range(2))
+    k[:, :, :far] = -3e38
+    ref = O.batched_sparse_attention_forward(q.float(), k.float(), v.float(), torch.tensor(lens), 64 ** -0.5)
+    got = layers.batched_sparse_attention(q.to(DEV), k.to(DEV), v.to(DEV), torch.tensor(lens), 64 ** -0.5)
+    assert torch.isfinite(ref).all() and rel_err(got.float(), ref) < bound
 
 
 def test_attention_strided_views(vl):

@@ -15,8 +15,8 @@
 //                      straight from the TMA image of the [keys, d] rows; accumulator in TMEM
 //                      columns [64, 128), which are free once the first 128 keys are consumed: their
 //                      products run while the exp2 of the rest does (DeiT-S, 7 images: 680 -> 675 us)
-//   O  = O*alpha + O_c in registers of the softmax threads (online-softmax rescale, started by the
-//                      tail keys), then the 1/rowsum and the bf16 store.
+//   O  = O*alpha + O_c in registers of the softmax threads (online-softmax rescale), then the
+//                      tail keys, the 1/rowsum and the bf16 store.
 // Warp 0 lane 0 issues TMA (Q is double-buffered so the next item's Q and K stream in during
 // the current softmax), warp 1 lane 0 issues MMA, warps 2-5 do softmax and output.
 // q, k, v are read in place from the Linear outputs through strided tensor maps.
@@ -276,15 +276,15 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
 #pragma unroll
             for (int i = 0; i < HD; ++i) o[i] = 0.f;
             const uint8_t* qrow = base + SM_Q + qb * (QT * HD * 2) + r * 128;
-            if (tail > 0 && live) {
-                // ---- the last n_keys % 16 keys on CUDA cores, one online-softmax step per key.  They come first: their
-                // rows arrived with Q, and the scores of the chunk are still being loaded and multiplied (behind the
-                // chunk this step took 1500 of the 17 k cycles of a lone item: DeiT-Ti, one image, 527 -> 515 us).
-                const uint8_t* tb = base + SM_TAIL + qb * (2 * TAIL_ROWS * HD * 2);
+            // ---- the last n_keys % 16 keys run on CUDA cores.  Their scores (one fmaf chain in channel order each) are
+            // formed here: the rows arrived with Q, and the scores of the chunk are still being loaded and multiplied.
+            const uint8_t* tb = base + SM_TAIL + qb * (2 * TAIL_ROWS * HD * 2);
+            float tail_s[TAIL_ROWS];
+            if (live) {
+#pragma unroll 1
                 for (int t = 0; t < tail; ++t) {
                     const uint4* krow = reinterpret_cast<const uint4*>(tb + t * (HD * 2));
-                    const uint4* vrow = reinterpret_cast<const uint4*>(tb + (TAIL_ROWS + t) * (HD * 2));
-                    float d4[4] = {0.f, 0.f, 0.f, 0.f};
+                    float sdot = 0.f;
 #pragma unroll
                     for (int ch = 0; ch < HD / 8; ++ch) {
                         Vec<bf16> qv, kv;
@@ -294,24 +294,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
                         qv.to_float(qf);
                         kv.to_float(kf);
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) d4[i & 3] = fmaf(qf[i], kf[i], d4[i & 3]);
+                        for (int i = 0; i < 8; ++i) sdot = fmaf(qf[i], kf[i], sdot);
                     }
-                    const float sdot = (d4[0] + d4[1]) + (d4[2] + d4[3]);
-                    const float m_new = fmaxf(m, sdot);
-                    const float m_at = m_new == -INFINITY ? 0.f : m_new;      // (a score of -inf has weight zero)
-                    const float alpha = fast_exp2((m - m_at) * scale_log2e);
-                    const float p = fast_exp2((sdot - m_at) * scale_log2e);
-                    l = l * alpha + p;
-                    m = m_new;
-#pragma unroll
-                    for (int ch = 0; ch < HD / 8; ++ch) {
-                        Vec<bf16> vv;
-                        float vf[8];
-                        vv.raw = vrow[ch];
-                        vv.to_float(vf);
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) o[8 * ch + i] = fmaf(o[8 * ch + i], alpha, p * vf[i]);
-                    }
+                    tail_s[t] = sdot;
                 }
             }
             for (int c = 0; c < n_chunks && ok; ++c, ++g) {
@@ -355,8 +340,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
                 }
                 const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
                 const float m_new = fmaxf(m, mx);
-                const float alpha = fast_exp2((m - m_new) * scale_log2e);       // 0 while m is -inf
-                const float mb = m_new * scale_log2e;
+                const float m_at = m_new == -INFINITY ? 0.f : m_new;            // (scores of -inf have weight zero)
+                const float alpha = fast_exp2((m - m_at) * scale_log2e);        // 0 while m is -inf
+                const float mb = m_at * scale_log2e;
                 float ls4[4] = {0.f, 0.f, 0.f, 0.f};
                 for (int blk = 0; blk < nblk; ++blk) {
                     tmem_ld_wait();
@@ -415,6 +401,27 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
             if (!live) {
                 mbar_arrive(&q_free[qb]);
                 continue;
+            }
+            // ---- one online-softmax step per tail key, behind the chunks: a row's terms are added in the order of its keys
+#pragma unroll 1
+            for (int t = 0; t < tail; ++t) {
+                const uint4* vrow = reinterpret_cast<const uint4*>(tb + (TAIL_ROWS + t) * (HD * 2));
+                const float sdot = tail_s[t];
+                const float m_new = fmaxf(m, sdot);
+                const float m_at = m_new == -INFINITY ? 0.f : m_new;
+                const float alpha = fast_exp2((m - m_at) * scale_log2e);
+                const float p = fast_exp2((sdot - m_at) * scale_log2e);
+                l = l * alpha + p;
+                m = m_new;
+#pragma unroll
+                for (int ch = 0; ch < HD / 8; ++ch) {
+                    Vec<bf16> vv;
+                    float vf[8];
+                    vv.raw = vrow[ch];
+                    vv.to_float(vf);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) o[8 * ch + i] = fmaf(o[8 * ch + i], alpha, p * vf[i]);
+                }
             }
             // ---- normalise, then out through the warp's own 32 rows of the Q tile (no longer needed) so that
             // eight lanes write one full 128-byte line of a row instead of every lane a piece of its own row
