@@ -554,3 +554,25 @@ def test_forward_with_swapped_in_weights_updated_in_place(kind):
         want = fresh._forward_eval(img, use_plans=False)
         for _ in range(3):
             assert torch.equal(functional_call(m, ema, (img,)), want)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16])
+@pytest.mark.parametrize("kind", ["deit", "pvt"])
+def test_image_gives_the_same_bits_in_any_batch(kind, dtype):
+    """Logits and counts of an image do not depend on how many images are with it: sums are formed in the same order
+    whatever the number of tiles a launch has."""
+    from vtpack_b200 import synthetic
+    from vtpack_b200.models.dge.pvt_dge import pvt_dge_s124_tiny_256
+    if kind == "deit":
+        m = synthetic.build_model("small", DEV, dtype, depth=3, seed=0)
+    else:
+        m = pvt_dge_s124_tiny_256()
+        m.load_state_dict(O.make_pvt_state_dict(O.PVT_CONFIGS["tiny"], seed=0), strict=True)
+        m = m.eval().to(device=DEV, dtype=dtype)
+    img = O.make_images(80, 256, seed=3).to(DEV)
+    want = m(img)
+    counts = [c.clone() for c in m.last_counts]
+    for n in (1, 2, 7, 19, 40):
+        got = m(img[:n].contiguous())
+        assert torch.equal(got, want[:n]), n
+        assert all(torch.equal(a, b[:n]) for a, b in zip(m.last_counts, counts))

@@ -31,15 +31,14 @@ struct LinearArgs {
     const float2* ln_stats = nullptr; const float* ln_s = nullptr;
     int ln_mode = 0, ln_dim = 0, ln_slots = 0; float ln_eps = 0.f;
     // When set, every stored row leaves (sum, sum of squares) of its outputs here, one slot per
-    // (column range, epilogue warp): plain stores, so the result does not depend on timing.
-    // linear_stat_slots(N, m_max) tells the consumer how many slots a row has.
+    // (column tile, epilogue warp): plain stores, so the result does not depend on timing.
+    // linear_stat_slots(N) tells the consumer how many slots a row has.
     float2* emit_stats = nullptr;
 };
 
-int linear_stat_slots(int N, int m_max);   // float2 slots per row a tcgen05 GEMM with N output columns fills
-int linear_stat_slots_max(int N);          // ... at most, whatever the number of rows
+int linear_stat_slots(int N);              // float2 slots per row a tcgen05 GEMM with N output columns fills
 
-struct LnFold { const float2* stats; const float* s; int mode, dim; float eps; float2* emit; int slots, emit_cols; };
+struct LnFold { const float2* stats; const float* s; int mode, dim; float eps; float2* emit; int slots; };
 
 int linear_validate(const LinearArgs& p);
 int linear_cuda_cores(const LinearArgs& p, cudaStream_t st);   // fp32 or bf16 inputs, CUDA cores

@@ -228,16 +228,17 @@ linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
     // partial round are cut into `parts` column strips of BN / parts columns, one strip per group, so that
     // the round costs a fraction of a tile instead of a whole one with most SMs idle.  Strips use their
     // own W boxes (tw2 / tw3) and a narrower MMA.  A problem with fewer tiles than SMs is all last round.
-    // Kernels that leave row statistics (EPI_EMIT) split down to the column range one statistic covers.
+    // Kernels that leave row statistics (EPI_EMIT) do not split: a statistic is one sum over a whole tile's columns, so
+    // that a row's sums do not depend on how many rows there are (cut into strips, DeiT's bf16 logits of one image
+    // differed by 1 % between batches, through gates that near-ties flip).
     const int full_items = (total / n_groups) * n_groups;
     int parts = 1;
     {
         const int R = total - full_items, G = n_groups;
-        if (R > 0) {
-            const int most = (EPI & EPI_EMIT) ? BN / L.p[0].ln.emit_cols : BN / 64;
-            if (BN == 256) parts = (R * 4 <= G && most >= 4) ? 4 : (R * 2 <= G && most >= 2 ? 2 : 1);
-            else if (BN == 192) parts = (R * 3 <= G && most >= 3) ? 3 : 1;
-            else parts = (R * 2 <= G && most >= 2) ? 2 : 1;
+        if (!(EPI & EPI_EMIT) && R > 0) {
+            if (BN == 256) parts = (R * 4 <= G) ? 4 : (R * 2 <= G ? 2 : 1);
+            else if (BN == 192) parts = (R * 3 <= G) ? 3 : 1;
+            else parts = (R * 2 <= G) ? 2 : 1;
         }
     }
     // j-th work item of this CTA: problem p, this CTA's rows m0.., columns ct0 .. ct0 + width of its output.  The last
@@ -486,12 +487,9 @@ linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
                     asm volatile("prefetch.global.L1 [%0];" ::"l"(nxt));
                 }
             }
-            float e1 = 0.f, e2 = 0.f;     // sum and sum of squares of this thread's outputs of a statistics range
-            auto emit = [&](int sl) {     // leaves them at the end of the range
-                if ((EPI & EPI_EMIT) && ((sl + 1) * 64 % ln.emit_cols == 0 || sl + 1 == NSLAB)) {
-                    ln.emit[(size_t)(m0 + row) * ln.slots + (nt0 + sl * 64) / ln.emit_cols * 4 + qsub] = make_float2(e1, e2);
-                    e1 = e2 = 0.f;
-                }
+            float e1 = 0.f, e2 = 0.f;     // sum and sum of squares of this thread's outputs
+            auto emit = [&]() {
+                if (EPI & EPI_EMIT) ln.emit[(size_t)(m0 + row) * ln.slots + wi.nt * 4 + qsub] = make_float2(e1, e2);
             };
             auto wait_acc = [&]() {
                 ok = mbar_wait(&acc_full[buf], aph, abort_flag, status, STATUS_GEMM_EPILOGUE);
@@ -582,9 +580,9 @@ linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&slab_full[sb]);                // this warp's part of the slab is in place
                     ++slab_no;
-                    emit(sl);
                 }
                 if (!ok) break;
+                emit();
                 continue;
             }
             // ---- boundary tile / row-remapped / fp32 output: store straight from registers
@@ -662,9 +660,9 @@ linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
                     }
                     OutVec<OutT>::store8(y + orow * ldy + n, v);
                 }
-                if (row_ok) emit(sl);
             }
             if (!ok) break;
+            if (row_ok) emit();
         }
     }
     if (*abort_flag) {
@@ -755,20 +753,7 @@ static int pick_bn(int N) {
     return bn;
 }
 
-// Columns one row statistic of an EPI_EMIT launch covers: a whole tile, or less where even the worst-case tile
-// count leaves SMs idle, so that tiles can be cut into strips.  More slots cost the consumer more reads per row:
-// at DeiT-S batch 256 24 slots instead of 8 slow the forward by 2.7 %.  (The packed rows of a DGE block are about
-// a third of the worst case, hence the factor 2 of the middle range.)
-static int stat_cols(int N, int m_max) {
-    const int bn = pick_bn(N);
-    const long long tiles = (long long)ceil_div(N, bn) * ceil_div(m_max, TM);
-    if (tiles * 2 <= sm_count()) return 64;
-    if (tiles <= 2ll * sm_count()) return bn == 256 ? 128 : 64;
-    return bn;
-}
-// (ranges of the last tile beyond N leave zeros, so whole tiles count)
-int linear_stat_slots(int N, int m_max) { return ceil_div(N, pick_bn(N)) * (pick_bn(N) / stat_cols(N, m_max)) * 4; }
-int linear_stat_slots_max(int N) { return ceil_div(N, pick_bn(N)) * (pick_bn(N) / 64) * 4; }
+int linear_stat_slots(int N) { return ceil_div(N, pick_bn(N)) * 4; }
 
 template <int BN, typename OutT>
 static int fill_problem(TcProblem& q, const LinearArgs& p) {
@@ -809,7 +794,7 @@ static int fill_problem(TcProblem& q, const LinearArgs& p) {
     q.m_max = p.m_max; q.m_dev = p.m_dev; q.N = p.N;
     q.rm = RowMap{p.out_grp, p.out_skip, p.res_mod, p.res_off};
     q.ln = LnFold{p.ln_stats, p.ln_s, p.ln_mode, p.ln_dim, p.ln_eps, p.emit_stats,
-                  p.emit_stats ? linear_stat_slots(p.N, p.m_max) : p.ln_slots, stat_cols(p.N, p.m_max)};
+                  p.emit_stats ? linear_stat_slots(p.N) : p.ln_slots};
     return VTP_OK;
 }
 
@@ -850,7 +835,7 @@ static int launch_tc(const LinearArgs& p, const LinearArgs* p1, cudaStream_t st)
     // batch 256, graph: 3.78 ms without, 3.98 ms with).
     const bool early = tiles <= groups;
     // few tiles are cut into column strips, one per CTA (see the kernel): launch a CTA for each of those
-    tiles *= (EPI & EPI_EMIT) ? BN / stat_cols(p.N, p.m_max) : BN / 64;
+    if (!(EPI & EPI_EMIT)) tiles *= BN / 64;
     const int grid = CG * (int)(tiles < groups ? tiles : groups);
     const cudaError_t le = launch_kernel(kern, early, CG, dim3(grid), dim3(TC_THREADS), (size_t)S::TOTAL, st, L, p.K, device_status_ptr());
     if (le != cudaSuccess) {
