@@ -556,7 +556,7 @@ def test_forward_with_swapped_in_weights_updated_in_place(kind):
             assert torch.equal(functional_call(m, ema, (img,)), want)
 
 
-@pytest.mark.parametrize("dtype", [torch.bfloat16])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("kind", ["deit", "pvt"])
 def test_image_gives_the_same_bits_in_any_batch(kind, dtype):
     """Logits and counts of an image do not depend on how many images are with it: sums are formed in the same order

@@ -579,3 +579,22 @@ def test_linear_fp32_non_finite_operands(vl, M, N, K):
     # a chain of K roundings on one side, the split's bound (see above) on the other
     assert bool(((got.double() - chain.double())[ok].abs() <= (K + 4) * 2.0 ** -23 * mag).all())
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("N,K", [(384, 320), (384, 384), (192, 700), (384, 768), (256, 1536), (129, 1540)])
+def test_linear_fp32_rows_do_not_depend_on_the_launch(vl, N, K):
+    """The bits of a row are the same in launches of 1 to 20,000 rows: reductions split over four CTAs, over two and not
+    at all, narrow and wide tiles, whole and ragged k-blocks in one, two and four groups."""
+    from vtpack_b200 import _lib
+    from vtpack_b200.runtime import ptr, stream_ptr
+    g = torch.Generator(DEV).manual_seed(N + K)
+    x = torch.randn(20000, K, device=DEV, generator=g)
+    w = torch.randn(N, K, device=DEV, generator=g) * 0.1
+    outs = {}
+    for M in (1, 128, 700, 1400, 3000, 20000):
+        y = torch.empty(M, N, device=DEV)
+        _lib.check(_lib.lib().vtp_linear(ptr(x), K, ptr(w), None, None, 0, ptr(y), N, 0, M, None, N, K, 0, stream_ptr(x.device)))
+        outs[M] = y
+    for M, y in outs.items():
+        assert torch.equal(y, outs[20000][:M]), M
+    assert _lib.device_status() == 0

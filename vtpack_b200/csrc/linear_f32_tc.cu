@@ -17,7 +17,11 @@
 //
 // A long reduction with few tiles (fc2 of a small batch: 54 tiles, 24 k-blocks) is split over the CTAs of a cluster:
 // each takes a share of the k-blocks, they exchange their partial sums through distributed shared memory, and each
-// finishes a slice of the tile's columns.
+// finishes a slice of the tile's columns.  The sums are formed the same way whether it is split or not, so that a
+// row's bits depend on K alone and not on how many rows and tiles a launch has: the k-blocks are cut into one, two or
+// four groups by their number, a group is added up from zero, and the groups are added as (0 + 1) + (2 + 3).  A CTA
+// with several groups keeps the sums of the earlier ones in tensor memory (three loads and stores a tile: DeiT-S, 12
+// images, 2453 -> 2507 us against sums that were grouped by the number of tiles).
 //
 // Persistent, one CTA per SM, 128 x BN tiles (BN = 64 where 128-wide tiles would leave SMs idle):
 //   warps 0-10 / 0-14  fetch the next k-block with 16-byte loads one k-block ahead (in registers), split it and write the
@@ -48,6 +52,7 @@ constexpr int F_EPI = 256;              // epilogue threads
 // same: the port is the bound, see above.)
 constexpr int conv_warps(int bn) { return bn == 128 ? 11 : 15; }
 constexpr int F_STAGES = 2;
+constexpr int F_TMEM = 4;              // in tile widths: two accumulators, two group sums
 
 template <int BN>
 struct F32Smem {
@@ -63,6 +68,7 @@ struct F32Args {
     const float* a; long long lda; const float* w; const float* bias; const float* res; long long ldr;
     float* y; long long ldy;
     int m_max; const int32_t* m_dev; int N, K; int gelu, wide;       // wide: 32-byte loads
+    int groups_log2;                                                  // groups of k-blocks, see f32_groups_log2
     RowMap rm;
 };
 
@@ -131,7 +137,37 @@ __device__ __forceinline__ void redo_nonfinite(float (&acc)[NC], const F32Args& 
     }
 }
 
-// SPLIT: CTAs of a cluster that share a tile's reduction (1: none).
+// Groups of k-blocks that are added up apart: at least three k-blocks each.  More splits would leave a CTA less work
+// than the exchange costs.
+static int f32_groups_log2(int num_kb) { return num_kb >= 12 ? 2 : num_kb >= 6 ? 1 : 0; }
+
+// acc (op) a sum kept in tensor memory, 32 columns at a time
+template <int CW>
+__device__ __forceinline__ void stash_store(uint32_t taddr, const float (&acc)[CW]) {
+    __syncwarp();
+#pragma unroll
+    for (int c0 = 0; c0 < CW; c0 += 16) {
+        uint32_t r[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(acc[c0 + i]);
+        tmem_st_32x16(taddr + c0, r);
+    }
+    tmem_st_wait();
+}
+template <int CW>
+__device__ __forceinline__ void stash_add(uint32_t taddr, float (&acc)[CW]) {
+#pragma unroll
+    for (int c0 = 0; c0 < CW; c0 += 32) {
+        uint32_t r[32];
+        __syncwarp();
+        tmem_ld_32x32(taddr + c0, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) acc[c0 + i] += __uint_as_float(r[i]);
+    }
+}
+
+// SPLIT: CTAs of a cluster that share a tile's reduction (1: none); it divides the number of groups.
 template <int BN, int SPLIT>
 __global__ void __launch_bounds__(conv_warps(BN) * 32 + 32 + F_EPI, 1)
 linear_f32_tc_kernel(const F32Args g, int* status) {
@@ -163,7 +199,7 @@ linear_f32_tc_kernel(const F32Args g, int* status) {
         fence_barrier_init();
     }
     if (warp == NCW) {
-        tmem_alloc(tmem_slot, 2 * BN);
+        tmem_alloc(tmem_slot, F_TMEM * BN);
         tmem_relinquish();
     }
     tc_fence_before_sync();
@@ -289,6 +325,8 @@ linear_f32_tc_kernel(const F32Args g, int* status) {
         const uint32_t tacc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * CW;
         const uint32_t stage = smem_u32(base + F_STAGES * S::STAGE) + ew * (32 * 128);
         const bool vec = g.N % 4 == 0 && g.ldy % 4 == 0 && (!g.res || g.ldr % 4 == 0);
+        const int own_groups = (1 << g.groups_log2) / SPLIT;         // this CTA's: 1, 2 or 4
+        const uint32_t tsum = tacc + 2 * BN;             // sums of its earlier groups: 0 (+ 1), and 2
         int it = 0, n_done = 0;                           // k-blocks, tiles
         bool ok = true;
         for (int tile = first_tile; tile < total && ok; tile += tile_step, ++n_done) {
@@ -296,6 +334,7 @@ linear_f32_tc_kernel(const F32Args g, int* status) {
             float acc[CW];
 #pragma unroll
             for (int i = 0; i < CW; ++i) acc[i] = 0.f;
+            int grp = 0;
             for (int kb = 0; kb < num_kb; ++kb, ++it) {
                 const int s = it & 1;
                 ok = mbar_wait(&acc_full[s], (it >> 1) & 1, abort_flag, status, STATUS_GEMM_EPILOGUE);
@@ -313,6 +352,16 @@ linear_f32_tc_kernel(const F32Args g, int* status) {
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&acc_empty[s]);
+                if constexpr (SPLIT < 4) {
+                    // the CTA has one group, or this k-block does not end one
+                    if (own_groups == 1 || kb + 1 != (all_kb * (rank * own_groups + grp + 1) >> g.groups_log2) - kb0) continue;
+                    if (grp & 1) stash_add<CW>(tsum + (SPLIT == 1 ? (grp >> 1) * BN : 0), acc);
+                    if (SPLIT == 1 && grp == 3) stash_add<CW>(tsum, acc);            // (0 + 1) + (2 + 3)
+                    if (++grp == own_groups) continue;
+                    stash_store<CW>(tsum + (SPLIT == 1 && grp == 3 ? BN : 0), acc);
+#pragma unroll
+                    for (int i = 0; i < CW; ++i) acc[i] = 0.f;
+                }
             }
             if (!ok) break;
             if constexpr (SPLIT > 1) {
@@ -344,13 +393,20 @@ linear_f32_tc_kernel(const F32Args g, int* status) {
 #pragma unroll
                         for (int j = 0; j < SC; ++j) own[j] = acc[d * SC + j];
                     }
+                // four partial sums: this CTA's pair first, then the other pair's sum (slots are in source order without
+                // this CTA: 1 2 3, 0 2 3, 0 1 3, 0 1 2)
+                const uint32_t mine = stage + lane * 16 + (SPLIT == 4 && rank >= 2 ? 2 : 0) * (SC * 128);
+                const uint32_t other = stage + lane * 16 + (rank >= 2 ? 0 : 1) * (SC * 128);
 #pragma unroll
-                for (int o = 0; o < SPLIT - 1; ++o)
-#pragma unroll
-                    for (int j = 0; j < SC / 4; ++j) {
-                        const float4 p = lds_f4(stage + o * (SC * 128) + j * 512 + lane * 16);
-                        own[4 * j] += p.x; own[4 * j + 1] += p.y; own[4 * j + 2] += p.z; own[4 * j + 3] += p.w;
+                for (int j = 0; j < SC / 4; ++j) {
+                    const float4 p = lds_f4(mine + j * 512);
+                    own[4 * j] += p.x; own[4 * j + 1] += p.y; own[4 * j + 2] += p.z; own[4 * j + 3] += p.w;
+                    if constexpr (SPLIT == 4) {
+                        const float4 a = lds_f4(other + j * 512), c = lds_f4(other + SC * 128 + j * 512);
+                        own[4 * j] += a.x + c.x; own[4 * j + 1] += a.y + c.y;
+                        own[4 * j + 2] += a.z + c.z; own[4 * j + 3] += a.w + c.w;
                     }
+                }
                 __syncwarp();
                 if (lane == 0) {
 #pragma unroll
@@ -437,7 +493,7 @@ linear_f32_tc_kernel(const F32Args g, int* status) {
     tc_fence_before_sync();
     __syncthreads();
     if (SPLIT > 1) cluster_sync_all();           // no partner signals this CTA's barriers any more
-    if (warp == NCW) tmem_dealloc(tmem_base, 2 * BN);
+    if (warp == NCW) tmem_dealloc(tmem_base, F_TMEM * BN);
 }
 
 template <int BN, int SPLIT>
@@ -482,16 +538,16 @@ int linear_f32_tcgen05(const LinearArgs& p, cudaStream_t st) {
     auto aligned32 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 31u) == 0; };
     g.wide = p.K % 8 == 0 && p.lda % 8 == 0 && aligned32(p.a) && aligned32(p.w);
     g.rm = RowMap{p.out_grp, p.out_skip, p.res_mod, p.res_off};
+    g.groups_log2 = f32_groups_log2(ceil_div(p.K, FK));
     // With a device-side row count the worst case is about three times the packed rows of a DGE block.
     const long long sms = sm_count(), likely = p.m_dev ? 3 : 1;
     // 128-wide tiles only where they keep the SMs busy for two rounds
     const long long wide = (long long)ceil_div(p.N, 128) * ceil_div(p.m_max, FM);
     if (wide >= 2 * likely * sms) return launch_f32<128, 1>(g, st);
-    // a reduction is split where the tiles leave SMs idle and every CTA keeps at least three k-blocks
+    // a reduction is split where the tiles leave SMs idle
     const long long tiles = (long long)ceil_div(p.N, 64) * ceil_div(p.m_max, FM);
-    const int num_kb = ceil_div(p.K, FK);
-    if (num_kb >= 12 && tiles * 4 <= likely * sms) return launch_f32<64, 4>(g, st);
-    if (num_kb >= 6 && tiles * 2 <= likely * sms) return launch_f32<64, 2>(g, st);
+    if (g.groups_log2 == 2 && tiles * 4 <= likely * sms) return launch_f32<64, 4>(g, st);
+    if (g.groups_log2 >= 1 && tiles * 2 <= likely * sms) return launch_f32<64, 2>(g, st);
     return launch_f32<64, 1>(g, st);
 }
 
