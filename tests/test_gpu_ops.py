@@ -263,11 +263,11 @@ def test_attention_bf16_tail_scores_are_one_chain(vl, N):
     assert float((got.float() - w).abs().max()) < 2.0 ** -8 * w
 
 
-@pytest.mark.parametrize("dtype,bound", [(torch.bfloat16, 8e-3)])
+@pytest.mark.parametrize("dtype,bound,flags", [(torch.bfloat16, 8e-3, 0), (torch.bfloat16, 8e-3, 4), (torch.float32, 1e-5, 0)])
 @pytest.mark.parametrize("N,far", [(17, 16), (33, 32), (257, 256), (257, 128), (400, 200), (600, 300), (1025, 600)])
-def test_attention_leading_keys_of_weight_zero(vl, dtype, bound, N, far):
+def test_attention_leading_keys_of_weight_zero(vl, dtype, bound, flags, N, far):
     """The first `far` keys of every row have scores of -inf (whole chunks of them): weight zero, and the row is finite as
-    long as one other score is."""
+    long as one other score is; tensor cores, CUDA cores (flag 4) and fp32."""
     _, layers = vl
     g = torch.Generator().manual_seed(N)
     lens = [5, 130]
@@ -275,7 +275,7 @@ def test_attention_leading_keys_of_weight_zero(vl, dtype, bound, N, far):
     k, v = (torch.randn(2, 2, N, 64, generator=g).to(dtype) for _ in range(2))
     k[:, :, :far] = -3e38
     ref = O.batched_sparse_attention_forward(q.float(), k.float(), v.float(), torch.tensor(lens), 64 ** -0.5)
-    got = layers.batched_sparse_attention(q.to(DEV), k.to(DEV), v.to(DEV), torch.tensor(lens), 64 ** -0.5)
+    got = layers.batched_sparse_attention(q.to(DEV), k.to(DEV), v.to(DEV), torch.tensor(lens), 64 ** -0.5, flags=flags)
     assert torch.isfinite(ref).all() and rel_err(got.float(), ref) < bound
 
 

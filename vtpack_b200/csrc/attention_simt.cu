@@ -161,11 +161,13 @@ attn_simt_kernel(const T* __restrict__ q, long long q_rs, long long q_hs, const 
                 }
 #pragma unroll
                 for (int w = 8; w > 0; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
-                const float m_new = fmaxf(m[i], mx), alpha = expf(m[i] - m_new);      // 0 on the first chunk
+                const float m_new = fmaxf(m[i], mx);
+                const float m_at = m_new == -INFINITY ? 0.f : m_new;  // (scores of -inf have weight zero, a chunk of them too)
+                const float alpha = expf(m[i] - m_at);               // 0 while m is -inf
                 float sum = 0.f;
 #pragma unroll
                 for (int j = 0; j < AKJ; ++j) {
-                    const float p = expf(s[i][j] - m_new);           // keys beyond the chunk: exp(-inf) = 0
+                    const float p = expf(s[i][j] - m_at);            // keys beyond the chunk: exp(-inf) = 0
                     P[(ty * 4 + i) * SPITCH + tx + 16 * j] = p;
                     sum += p;
                 }
