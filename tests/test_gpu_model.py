@@ -487,7 +487,7 @@ def test_repeated_forwards_replay_one_capture(kind, dtype):
 @pytest.mark.parametrize("kind", ["deit", "pvt"])
 def test_replayed_forward_follows_settings_and_streams(kind):
     """What the launches take by value (softmax scale, LayerNorm epsilon) may change between calls of a model whose
-    launches have been captured, and the calls may come from different streams."""
+    launches have been captured, in ``forward`` and in ``forward_graph``, and the calls may come from different streams."""
     from vtpack_b200 import synthetic
     from vtpack_b200.models.dge.pvt_dge import pvt_dge_s124_tiny_256
 
@@ -507,6 +507,8 @@ def test_replayed_forward_follows_settings_and_streams(kind):
 
     img = O.make_images(2, 256, seed=3).to(DEV)
     m, changes = make(), []
+    logits = torch.empty(2, 1000, device=DEV)
+    graph = (lambda: m.forward_graph(img, logits)) if kind == "deit" else (lambda: m.forward_graph(img))
     for change in (None, scale, eps):
         if change is not None:
             change(m)
@@ -517,6 +519,7 @@ def test_replayed_forward_follows_settings_and_streams(kind):
         want = fresh(img)
         for _ in range(3):
             assert torch.equal(m(img), want)
+            assert torch.equal(graph(), want)
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):

@@ -451,6 +451,13 @@ class VisionTransformer(nn.Module):
             return self._forward_train(x)
         return self._forward_eval(x, logits_out)
 
+    def _shape_struct(self, B, dtype):
+        """What the launches of an eval forward take by value, settings that may change between calls (softmax scale,
+        LayerNorm epsilon, flags) among them: part of the key of everything captured."""
+        G, blk0 = self.img_size // self.patch_size, self.blocks[0]
+        return _shape_struct(dtype, B, G, G, 1, self.embed_dim, blk0.attn.num_heads, blk0.mlp.fc1.out_features,
+                             self.split_sizes, self.norm.eps, self.flags, blk0.attn.scale)
+
     def _forward_eval(self, x, logits_out=None, use_plans=True):
         require_cuda(x)
         if x.dtype not in (torch.float32, torch.bfloat16):
@@ -459,9 +466,7 @@ class VisionTransformer(nn.Module):
         B = x.shape[0]
         dtype = self.compute_dtype()
         G = self.img_size // self.patch_size
-        blk0 = self.blocks[0]
-        s = _shape_struct(dtype, B, G, G, 1, self.embed_dim, blk0.attn.num_heads, blk0.mlp.fc1.out_features,
-                          self.split_sizes, self.norm.eps, self.flags, blk0.attn.scale)
+        s = self._shape_struct(B, dtype)
         m, blocks = self._pack_model(dtype)
         m.image_dtype = dtype_code(x.dtype)
         lib = _lib.lib()
@@ -578,11 +583,12 @@ def _graph_forward(model, x, logits_out):
     A captured graph holds raw addresses: the input and output buffers, the packed (and folded)
     weights, the per-device scratch and the optional gate bias.  It is dropped, and captured
     again, when a parameter has changed since (load_state_dict, an optimizer step), when the
-    scratch buffer has been replaced by a larger one, or when another gate bias tensor is set."""
+    scratch buffer has been replaced by a larger one, when another gate bias tensor is set, or
+    when a setting that the launches take by value has changed."""
     model._pack_model(model.compute_dtype())       # repacks after a parameter change and drops stale graphs
     bias = model.gate_image_bias
     key = (x.data_ptr(), tuple(x.shape), x.dtype, logits_out.data_ptr(), None if bias is None else bias.data_ptr(),
-           model.trace, int(model.flags))
+           model.trace, bytes(model._shape_struct(x.shape[0], model.compute_dtype())))
     g = model._graphs.get(key)
     if g is not None and g.scratch_gen != scratch_generation(x.device):
         g = None

@@ -293,10 +293,11 @@ class PyramidVisionTransformer(nn.Module):
         calls, its address and shape may not); returns the graph's own output tensor, overwritten by the next
         call.  The stages are sequenced from Python through some sixty small launches per forward; replaying
         them as one graph removes the host work between them.  The graph is captured again when a parameter
-        has changed, when the per-device scratch buffer has been replaced, or for another input buffer."""
+        or a setting that the launches take by value has changed, when the per-device scratch buffer has been
+        replaced, or for another input buffer."""
         if self.training:
             raise RuntimeError("forward_graph is an eval-mode path")
-        key = (x.data_ptr(), tuple(x.shape), x.dtype, self._param_generation())
+        key = (x.data_ptr(), tuple(x.shape), x.dtype, self._param_generation(), self._launch_config())
         g = self._graph
         if g is None or g["key"] != key or g["scratch_gen"] != self._scratch_gen(x.device):
             cur = torch.cuda.current_stream(x.device)
