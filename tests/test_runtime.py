@@ -1,8 +1,12 @@
 """CPU tests of the host-side plumbing: what makes a model pack its weights again and drop its captured launches."""
+import gc
+import weakref
+
+import pytest
 import torch
 from torch.func import functional_call
 
-from vtpack_b200.models.dge import deit_dge
+from vtpack_b200.models.dge import deit_dge, pvt_dge
 from vtpack_b200.models.dge.deit_dge import _param_key
 
 
@@ -37,3 +41,40 @@ def test_weight_key_follows_tensors_in_the_parameters_place():
     with torch.no_grad():
         m.model.head.weight.add_(1.0)
     assert m() not in keys
+
+
+class _Plan:
+    pass
+
+
+@pytest.fixture
+def no_capture(monkeypatch):
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+
+
+@pytest.mark.parametrize("move", ["update", "replace"])
+def test_pvt_plans_of_replaced_weights_are_dropped(no_capture, move):
+    """A plan holds its weights' device copies: none of the old ones is left when the weights are others."""
+    m = pvt_dge.pvt_dge_s124_tiny_256()
+    made = []
+
+    def capture():
+        p = _Plan()
+        made.append(weakref.ref(p))
+        return p
+
+    for step in range(3):
+        m._param_generation()
+        for key in ("a", "b"):
+            for _ in range(20):
+                m._plans.get(key, lambda p: True, capture)
+        gc.collect()
+        assert len(made) == 2 * (step + 1) and sum(r() is not None for r in made) == 2
+        with torch.no_grad():
+            if move == "update":
+                m.head.bias.add_(1.0)
+            else:
+                m.head.bias = torch.nn.Parameter(m.head.bias.clone())
+    m._param_generation()
+    gc.collect()
+    assert all(r() is None for r in made)

@@ -369,7 +369,11 @@ class PyramidVisionTransformer(nn.Module):
     def _param_generation(self):
         if self._pack.watch is None:
             self._pack.watch = ParamWatch(self)
-        return self._pack.watch.generation()
+        gen = self._pack.watch.generation()
+        if gen != self._pack.key:
+            self._pack.key = gen
+            self._plans.clear()        # they hold the old weights' copies on the device
+        return gen
 
     def _launch_config(self):
         """What the blocks' launches take by value besides shapes: it may be changed between calls."""
@@ -451,7 +455,8 @@ class PyramidVisionTransformer(nn.Module):
             return outputs
         plan = None
         if use_plans:
-            plan = self._plans.get((B, S, dtype, self._param_generation(), self._launch_config()),
+            self._param_generation()                  # drops the plans of other weights
+            plan = self._plans.get((B, S, dtype, self._launch_config()),
                                    lambda p: p.scratch_gen == self._scratch_gen(dev),
                                    lambda: self._capture_trunk(B, sides, ld, dtype, cols, y, tokens, dev))
         front()
