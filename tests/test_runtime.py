@@ -78,3 +78,21 @@ def test_pvt_plans_of_replaced_weights_are_dropped(no_capture, move):
     m._param_generation()
     gc.collect()
     assert all(r() is None for r in made)
+
+
+def test_replay_registers_its_stream_with_all_that_the_plan_holds(monkeypatch):
+    """The allocator may not hand on a plan's memory while a stream that replayed it still works on it, whichever stream
+    that was and whoever else has let go of the buffers."""
+    class Graph:
+        def replay(self):
+            pass
+
+    seen = []
+    monkeypatch.setattr(torch.Tensor, "record_stream", lambda t, s: seen.append((t.data_ptr(), s)))
+    held = [torch.zeros(3) for _ in range(5)]
+    keep = (held[0], {"a": held[1], "b": (1.0, held[2])}, [{"c": held[3]}, None])
+    plan = deit_dge._CapturedTrunk(Graph(), keep, 0, held[4])
+    for stream in ("x", "y", "x"):
+        monkeypatch.setattr(torch.cuda, "current_stream", lambda d=None, s=stream: s)
+        plan.replay(None)
+    assert sorted(seen) == sorted((t.data_ptr(), s) for t in held for s in "xy")

@@ -557,19 +557,31 @@ class _CapturedForward:
         self.graph, self.keep, self.scratch_gen = graph, keep, scratch_gen
 
 
+def _tensors_in(nest):
+    """The tensors of nested tuples, lists and dicts."""
+    if isinstance(nest, torch.Tensor):
+        yield nest
+    elif isinstance(nest, (tuple, list, dict)):
+        for v in (nest.values() if isinstance(nest, dict) else nest):
+            yield from _tensors_in(v)
+
+
 class _CapturedTrunk(_CapturedForward):
     """A captured trunk and the query counts its launches leave behind."""
 
     def __init__(self, graph, keep, scratch_gen, counts):
         super().__init__(graph, keep, scratch_gen)
         self.counts = counts
-        self.stream = torch.cuda.current_stream(counts.device)        # the stream the counts were allocated on
+        self.streams = set()
 
     def replay(self, device, then=None):
         """Replays the launches, runs `then`, and returns a copy of the counts."""
         cur = torch.cuda.current_stream(device)
-        if cur != self.stream:
-            self.counts.record_stream(cur)        # the plan may be dropped while this stream still works on it
+        if cur not in self.streams:
+            # the plan may be dropped while this stream still works on its memory: weights, scratch buffers, counts
+            for t in _tensors_in((self.keep, self.counts)):
+                t.record_stream(cur)
+            self.streams.add(cur)
         self.graph.replay()
         if then is not None:
             then()
