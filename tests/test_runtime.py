@@ -1,5 +1,7 @@
 """CPU tests of the host-side plumbing: what makes a model pack its weights again and drop its captured launches."""
+import copy
 import gc
+import pickle
 import weakref
 
 import pytest
@@ -96,3 +98,23 @@ def test_replay_registers_its_stream_with_all_that_the_plan_holds(monkeypatch):
         monkeypatch.setattr(torch.cuda, "current_stream", lambda d=None, s=stream: s)
         plan.replay(None)
     assert sorted(seen) == sorted((t.data_ptr(), s) for t in held for s in "xy")
+
+
+@pytest.mark.parametrize("make", [_tiny, pvt_dge.pvt_dge_s124_tiny_256])
+def test_whole_models_saved_before_there_were_plans_load(make, no_capture):
+    """Files of whole models, also from a version without watches and plans, load into models that work; a copy starts
+    without plans."""
+    m = make()
+    old = dict(m.__dict__)
+    for name in ("_plans", "_graph") + (("_pack",) if "_graph" in old else ()):
+        old.pop(name, None)
+    fresh = type(m).__new__(type(m))
+    fresh.__setstate__(old)
+    for model in (fresh, copy.deepcopy(m), pickle.loads(pickle.dumps(m))):
+        key = _param_key(model, torch.float32)
+        assert key == _param_key(model, torch.float32)
+        assert model._plans.get("a", lambda p: True, _Plan) is None
+        if isinstance(model, pvt_dge.PyramidVisionTransformer):
+            assert model._graph is None and model._param_generation() == model._param_generation()
+    pack = pickle.loads(pickle.dumps(m.blocks[0]._pack if hasattr(m, "blocks") else m.block1[0]._pack))
+    assert pack.watch is None and deit_dge._WeightPack.__new__(deit_dge._WeightPack).watch is None

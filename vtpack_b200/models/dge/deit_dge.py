@@ -160,12 +160,12 @@ class DropPath(nn.Module):
 class _WeightPack:
     """Device pointers of one block's parameters in the layout the C ABI wants: matrices
     in the compute dtype, vectors fp32.  Rebuilt when a parameter changes."""
+    watch = None                              # (packs in files of whole models may lack it)
 
     def __init__(self):
         self.key = None
         self.tensors = None
         self.struct = None
-        self.watch = None
 
     def __reduce__(self):                     # addresses mean nothing to a copy of the module
         return (_WeightPack, ())
@@ -399,6 +399,10 @@ class VisionTransformer(nn.Module):
         for m in self.modules():
             if isinstance(m, DynamicGrainedEncoder):
                 m.router.init_parameters()
+
+    def __setstate__(self, state):            # files of whole models may come from before there were plans
+        super().__setstate__(state)
+        self.__dict__.setdefault("_plans", LaunchPlans())
 
     @torch.jit.ignore
     def no_weight_decay(self):

@@ -275,6 +275,12 @@ class PyramidVisionTransformer(nn.Module):
         self._plans = LaunchPlans(4)
         self._graph = None
 
+    def __setstate__(self, state):            # files of whole models may come from before there were plans
+        super().__setstate__(state)
+        self.__dict__.setdefault("_pack", _WeightPack())
+        self.__dict__.setdefault("_plans", LaunchPlans(4))
+        self.__dict__.setdefault("_graph", None)
+
     def _const(self, name, sources, make, extra=()):
         """A tensor derived from parameters only (a weight matrix in GEMM layout and dtype, fp32 copies of bias and
         LayerNorm vectors, the resized position rows): made once and kept until one of ``sources`` changes, so an
