@@ -118,3 +118,12 @@ def test_whole_models_saved_before_there_were_plans_load(make, no_capture):
             assert model._graph is None and model._param_generation() == model._param_generation()
     pack = pickle.loads(pickle.dumps(m.blocks[0]._pack if hasattr(m, "blocks") else m.block1[0]._pack))
     assert pack.watch is None and deit_dge._WeightPack.__new__(deit_dge._WeightPack).watch is None
+
+
+def test_stage_forward_refuses_tokens_of_another_width(monkeypatch):
+    """The stage's launches take the width from the blocks: narrower tokens would be read and written beyond their end."""
+    monkeypatch.setattr(pvt_dge, "require_cuda", lambda *t: None)
+    stage = pvt_dge.pvt_dge_s124_tiny_256().block1
+    monkeypatch.setattr(pvt_dge, "_launch_stage", lambda *a: pytest.fail("launched"))
+    with pytest.raises(ValueError, match="32 channels"):
+        pvt_dge.stage_forward(stage, torch.zeros(1, 64, 32), 8, 8)

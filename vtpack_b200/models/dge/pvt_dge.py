@@ -156,6 +156,8 @@ def stage_forward(blocks, x, H, W):
     require_cuda(x)
     x = x.contiguous()
     B, N, C = x.shape
+    if C != blocks[0].dim:
+        raise ValueError(f"stage_forward: tokens of {C} channels for blocks of {blocks[0].dim}")
     out = torch.empty_like(x)
     counts = torch.empty(len(blocks), B, dtype=torch.int32, device=x.device)
     _launch_stage(blocks, x.dtype, B, N, H, W, ptr(x), ptr(out), ptr(counts), x.device, stream_ptr(x.device))
