@@ -4,6 +4,7 @@ import gc
 import pickle
 import weakref
 
+import numpy as np
 import pytest
 import torch
 from torch.func import functional_call
@@ -106,6 +107,7 @@ def test_whole_models_saved_before_there_were_plans_load(make, no_capture):
     without plans."""
     m = make()
     old = dict(m.__dict__)
+    old["_consts"] = {"norm": ((), None)}                    # an entry of another form
     for name in ("_plans", "_graph") + (("_pack",) if "_graph" in old else ()):
         old.pop(name, None)
     fresh = type(m).__new__(type(m))
@@ -115,7 +117,8 @@ def test_whole_models_saved_before_there_were_plans_load(make, no_capture):
         assert key == _param_key(model, torch.float32)
         assert model._plans.get("a", lambda p: True, _Plan) is None
         if isinstance(model, pvt_dge.PyramidVisionTransformer):
-            assert model._graph is None and model._param_generation() == model._param_generation()
+            assert model._graph is None and "_consts" not in model.__dict__
+            assert model._param_generation() == model._param_generation()
     pack = pickle.loads(pickle.dumps(m.blocks[0]._pack if hasattr(m, "blocks") else m.block1[0]._pack))
     assert pack.watch is None and deit_dge._WeightPack.__new__(deit_dge._WeightPack).watch is None
 
@@ -127,3 +130,16 @@ def test_stage_forward_refuses_tokens_of_another_width(monkeypatch):
     monkeypatch.setattr(pvt_dge, "_launch_stage", lambda *a: pytest.fail("launched"))
     with pytest.raises(ValueError, match="32 channels"):
         pvt_dge.stage_forward(stage, torch.zeros(1, 64, 32), 8, 8)
+
+
+def test_constants_follow_a_tensor_that_took_the_address_of_another():
+    """Weights handed over as new tensors on every call (functional_call) may lie where the ones before lay."""
+    m = pvt_dge.pvt_dge_s124_tiny_256()
+    memory = np.zeros(4, dtype=np.float32)
+    for value in (1.0, 2.0):
+        memory[:] = value
+        source = torch.from_numpy(memory)                    # another tensor at the same address, version 0
+        got = m._const("c", (source,), lambda: source.detach().clone())
+        assert got.tolist() == [value] * 4
+        assert m._const("c", (source,), lambda: None) is got
+        del source

@@ -279,20 +279,22 @@ class PyramidVisionTransformer(nn.Module):
 
     def __setstate__(self, state):            # files of whole models may come from before there were plans
         super().__setstate__(state)
+        self.__dict__.pop("_consts", None)    # made again from the weights that were loaded
         self.__dict__.setdefault("_pack", _WeightPack())
         self.__dict__.setdefault("_plans", LaunchPlans(4))
         self.__dict__.setdefault("_graph", None)
 
     def _const(self, name, sources, make, extra=()):
         """A tensor derived from parameters only (a weight matrix in GEMM layout and dtype, fp32 copies of bias and
-        LayerNorm vectors, the resized position rows): made once and kept until one of ``sources`` changes, so an
-        eval forward launches no conversion copies of its own."""
+        LayerNorm vectors, the resized position rows): made once and kept until one of ``sources`` changes or is
+        another tensor, so an eval forward launches no conversion copies of its own.  The entry holds its sources: a
+        tensor that took the place and the address of a freed one would look the same."""
         cache = self.__dict__.setdefault("_consts", {})
         key = tuple((p.data_ptr(), p._version, p.dtype) for p in sources) + tuple(extra)
         hit = cache.get(name)
-        if hit is None or hit[0] != key:
+        if hit is None or hit[0] != key or any(a is not b for a, b in zip(hit[2], sources)):
             with torch.no_grad():
-                hit = (key, make())
+                hit = (key, make(), tuple(sources))
             cache[name] = hit
         return hit[1]
 
