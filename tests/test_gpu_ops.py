@@ -598,3 +598,39 @@ def test_linear_fp32_rows_do_not_depend_on_the_launch(vl, N, K):
     for M, y in outs.items():
         assert torch.equal(y, outs[20000][:M]), M
     assert _lib.device_status() == 0
+
+
+def test_threads_that_launch_give_their_memory_back(vl):
+    """What a launching thread keeps (its encoded tensor maps, about 256 KB) goes with it."""
+    import threading
+
+    from vtpack_b200 import _lib
+    from vtpack_b200.runtime import ptr, stream_ptr
+    x, w = (torch.randn(128, 64, device=DEV).bfloat16() for _ in range(2))
+    y = torch.empty(128, 128, device=DEV, dtype=torch.bfloat16)
+
+    done = []
+
+    class Info(ctypes.Structure):
+        _fields_ = [(n, ctypes.c_size_t) for n in ("arena", "ordblks", "smblks", "hblks", "hblkhd", "usmblks", "fsmblks",
+                                                   "uordblks", "fordblks", "keepcost")]
+
+    libc = ctypes.CDLL("libc.so.6")
+    libc.mallinfo2.restype = Info
+
+    def launch():
+        y.zero_()                                # (makes the device's context current in this thread)
+        _lib.check(_lib.lib().vtp_linear(ptr(x), 64, ptr(w), None, None, 0, ptr(y), 128, 1, 128, None, 128, 64, 0, stream_ptr(x.device)))
+        done.append(1)
+
+    def threads(n):
+        for _ in range(n):
+            t = threading.Thread(target=launch)
+            t.start()
+            t.join()
+        info = libc.mallinfo2()
+        return info.uordblks + info.hblkhd           # bytes in use, in the arenas and in mappings of their own
+
+    before = threads(16)
+    assert threads(128) - before < 128 * 128 * 1024 and len(done) == 144
+    torch.cuda.synchronize()

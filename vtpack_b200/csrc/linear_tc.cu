@@ -36,6 +36,9 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <memory>
+#include <new>
+
 #include "linear.h"
 #include "runtime.h"
 #include "sm100.cuh"
@@ -720,8 +723,10 @@ int make_tmap_bf16(CUtensorMap* map, const void* base, int rank, const unsigned 
     for (int i = 0; i + 1 < rank; ++i) key.strides[i] = strides_bytes[i];
     unsigned long long h = (unsigned long long)reinterpret_cast<uintptr_t>(base) * 0x9E3779B97F4A7C15ull;
     for (int i = 0; i < rank; ++i) h = (h ^ (key.dims[i] * 31 + key.box[i])) * 0xBF58476D1CE4E5B9ull;
-    static thread_local TmapSlot* slots = nullptr;      // lives as long as the thread that launches
-    if (!slots) slots = static_cast<TmapSlot*>(calloc(kTmapSlots, sizeof(TmapSlot)));
+    static thread_local std::unique_ptr<TmapSlot[]> slots;      // freed when the thread that launches ends
+    static_assert(alignof(TmapSlot) >= alignof(CUtensorMap) && __STDCPP_DEFAULT_NEW_ALIGNMENT__ < alignof(CUtensorMap),
+                  "an array from operator new starts on the alignment the driver asks of a map (an aligned new)");
+    if (!slots) slots.reset(new (std::nothrow) TmapSlot[kTmapSlots]());
     TmapSlot* slot = slots ? &slots[(h >> 40) % kTmapSlots] : nullptr;
     if (slot && memcmp(&slot->key, &key, sizeof(key)) == 0) {
         *map = slot->map;
