@@ -438,8 +438,8 @@ def test_pvt_model_other_input_size_and_pyramid(golden_dir):
 @pytest.mark.parametrize("kind", ["deit", "pvt"])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_repeated_forwards_replay_one_capture(kind, dtype):
-    """The second forward of a shape captures the launches between the image kernel and the head, later ones replay
-    them: images and logits at other addresses, two batch sizes in turn, a larger batch that replaces the scratch
+    """A forward captures the launches between the image kernel and the head once its shape has earned it (here: the
+    second one), later ones replay them: images and logits at other addresses, two batch sizes in turn, a larger batch that replaces the scratch
     buffer and changed weights give bit for bit what a first (launch by launch) forward gives."""
     from vtpack_b200 import _lib, synthetic
     from vtpack_b200.models.dge.pvt_dge import pvt_dge_s124_tiny_256
@@ -451,6 +451,7 @@ def test_repeated_forwards_replay_one_capture(kind, dtype):
             m = pvt_dge_s124_tiny_256()
             m.load_state_dict(O.make_pvt_state_dict(O.PVT_CONFIGS["tiny"], seed=seed), strict=True)
             m = m.eval().to(device=DEV, dtype=dtype)
+        m._plans.earn = 2
         return m
 
     def first(seed, img):                                    # a model that has never run before
@@ -507,6 +508,7 @@ def test_replayed_forward_follows_settings_and_streams(kind):
 
     img = O.make_images(2, 256, seed=3).to(DEV)
     m, changes = make(), []
+    m._plans.earn = 2
     logits = torch.empty(2, 1000, device=DEV)
     graph = (lambda: m.forward_graph(img, logits)) if kind == "deit" else (lambda: m.forward_graph(img))
     for change in (None, scale, eps):
@@ -547,6 +549,7 @@ def test_forward_with_swapped_in_weights_updated_in_place(kind):
 
     img = O.make_images(2, 256, seed=3).to(DEV)
     m, fresh = make(), make()
+    m._plans.earn = 2
     ema = {k: v.detach().clone() for k, v in m.named_parameters()}
     for step in range(3):
         if step:

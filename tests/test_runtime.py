@@ -2,6 +2,7 @@
 import copy
 import gc
 import pickle
+import random
 import weakref
 
 import numpy as np
@@ -9,6 +10,7 @@ import pytest
 import torch
 from torch.func import functional_call
 
+from vtpack_b200 import runtime
 from vtpack_b200.models.dge import deit_dge, pvt_dge
 from vtpack_b200.models.dge.deit_dge import _param_key
 
@@ -106,6 +108,7 @@ def test_whole_models_saved_before_there_were_plans_load(make, no_capture):
     """Files of whole models, also from a version without watches and plans, load into models that work; a copy starts
     without plans."""
     m = make()
+    m._plans.earn = 3
     old = dict(m.__dict__)
     old["_consts"] = {"norm": ((), None)}                    # an entry of another form
     for name in ("_plans", "_graph") + (("_pack",) if "_graph" in old else ()):
@@ -143,3 +146,39 @@ def test_constants_follow_a_tensor_that_took_the_address_of_another():
         assert got.tolist() == [value] * 4
         assert m._const("c", (source,), lambda: None) is got
         del source
+
+
+def test_plans_are_earned_by_calls(no_capture):
+    """A shape that is seen often gets a plan and keeps it; many shapes in turn pay for few captures, and for fewer the
+    longer it goes on."""
+    plans, made = runtime.LaunchPlans(most=4, earn=8), []
+
+    def call(key):
+        def capture():
+            made.append(key)
+            return _Plan()
+        return plans.get(key, lambda p: True, capture)
+
+    got = [call("a") for _ in range(20)]
+    assert got[:7] == [None] * 7 and all(p is got[7] for p in got[7:]) and made == ["a"]
+    rng = random.Random(0)
+    for _ in range(2000):
+        call(rng.randrange(30))                              # within the shapes that calls are counted for
+    first = len(made)
+    for _ in range(2000):
+        call(rng.randrange(30))
+    assert first < 2000 / 8 / 1.5 and len(made) - first < first / 2
+    assert len(plans._plans) == 4 and len(plans._calls) <= 32
+    for key in range(1000, 3000):
+        assert call(key) is None
+    assert len(plans._calls) <= 32
+
+
+def test_a_plan_that_no_longer_fits_is_made_again_at_once(no_capture):
+    plans = runtime.LaunchPlans(most=4, earn=2)
+    assert plans.get("a", lambda p: True, _Plan) is None
+    p = plans.get("a", lambda p: True, _Plan)
+    q = plans.get("a", lambda p: False, _Plan)
+    assert q is not p and plans.get("a", lambda p: True, _Plan) is q
+    plans.clear()
+    assert plans.get("a", lambda p: True, _Plan) is None and copy.deepcopy(plans).earn == 2
