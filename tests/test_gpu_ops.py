@@ -634,3 +634,31 @@ def test_threads_that_launch_give_their_memory_back(vl):
     before = threads(16)
     assert threads(128) - before < 128 * 128 * 1024 and len(done) == 144
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("K", [64, 384, 768])
+@pytest.mark.parametrize("ex,ew", [(-112, 0), (-118, 0), (-126, 0), (-135, 0), (0, -122), (-122, 40), (-140, 60), (60, -118),
+                                   (-118, 120), (-65, -65), (-72, -72), (100, -100), (95, 0), (60, 60)])
+def test_linear_fp32_split_terms_over_the_exponent_range(vl, K, ex, ew):
+    """Operands around 2^ex and 2^ew, subnormal ones, subnormal results and sums too large for the scaled products
+    among them: the bound of the split on every output, plus half the smallest number for a result that is subnormal
+    itself; over the whole result no further from float64 than the CUDA-core kernel's fmaf chain."""
+    from vtpack_b200 import _lib
+    from vtpack_b200.runtime import ptr, stream_ptr
+    g = torch.Generator(DEV).manual_seed(K + ex)
+    M, N = 130, 72
+    x = (torch.randn(M, K, device=DEV, generator=g).double() * 2.0 ** ex).float()
+    w = (torch.randn(N, K, device=DEV, generator=g).double() * 0.1 * 2.0 ** ew).float()
+    ref, mag = x.double() @ w.double().t(), x.abs().double() @ w.abs().double().t()
+
+    def run(flags):
+        y = torch.full((M, N), float("nan"), device=DEV)
+        _lib.check(_lib.lib().vtp_linear(ptr(x), K, ptr(w), None, None, 0, ptr(y), N, 0, M, None, N, K, flags, stream_ptr(x.device)))
+        return y.double()
+
+    got, chain = run(0), run(_lib.FLAG_CUDA_CORES)
+    # the largest sums are those of the chain itself, K roundings
+    assert bool(((got - ref).abs() <= (4 + (K if ex + ew >= 90 else K / 64)) * 2.0 ** -23 * mag + 2.0 ** -149).all())
+    e = [float((t - ref).norm() / ref.norm()) for t in (got, chain)]
+    assert e[0] <= e[1] + 2.0 ** -24
+    assert _lib.device_status() == 0

@@ -2,9 +2,12 @@
 //
 //   y[m, n] = act(sum_k a[m,k] w[n,k] + bias[n]) + res[m, n],   everything fp32
 //
-// Every operand element is split into three bf16 terms, x = h + m + l (8 significant bits each, so the three hold
+// Every operand element is split into three bf16 terms, 2^16 x = h + m + l (8 significant bits each, so the three hold
 // the 24 bits of an fp32 number), and a k-block's product is the sum of six bf16 products accumulated in fp32:
-//   l*h + h*l + m*m + m*h + h*m + h*h      (smallest first; the three left out are below 2^-24 of |a||w|).
+//   l*h + h*l + m*m + m*h + h*m + h*h      (smallest first; the sum of the three left out is below 2^-23 of |a||w|,
+// m*l and l*m below 2^-24 each).  The factor 2^16 takes the last bit of the smallest fp32 number, 2^-149, to that of
+// the smallest bf16 number, 2^-133, so that the split is exact for every finite operand (without it, operands below
+// 2^-111 lost bits: 2e-5 of the result at 2^-118); a finished sum is multiplied by 2^-32.  (DeiT-S, 12 images: 1 %.)
 // The tensor core keeps an accumulator for one k-block (64) only; epilogue warps add the k-blocks in fp32
 // registers, rounding to nearest, so a long reduction does not collect the accumulator's own rounding.  Measured
 // against float64 the result is as close as the CUDA-core kernel's sequential fmaf chain (tests/test_gpu_ops.py).
@@ -30,10 +33,10 @@
 //   eight warps  add finished accumulators to their registers (one row x BN / 2 columns per thread); after the last
 //                k-block bias / GELU / residual and 128-byte stores through a per-warp shared-memory transpose
 //
-// An infinite or NaN operand (and a finite one within 2^-9 of the largest fp32 number, whose first term rounds up to
-// inf) turns every sum it enters into NaN through its second term, inf - inf.  Sums that come out non-finite are
-// therefore worked out again as a plain fmaf chain over the fp32 operands (redo_nonfinite): results are infinite, NaN
-// or finite where that chain's are.  The check is one fmaf per output.
+// An infinite or NaN operand (and a finite one of 2^112 or more, whose first term is inf) turns every sum it enters into
+// NaN through its second term, inf - inf, and a sum of 2^96 or more comes out infinite.  Sums that come out non-finite
+// are therefore worked out again as a plain fmaf chain over the fp32 operands (unscale_or_redo): results are infinite,
+// NaN or finite where that chain's are.  The check is one fmaf per output.
 //
 // Replaces nn.Linear q/kv/proj/fc1/fc2/head, nn.GELU and the residual adds of
 // vtpack/models/dge/deit_dge.py:38-44,72-74,96,127-128 when the model runs in fp32.
@@ -52,6 +55,7 @@ constexpr int F_EPI = 256;              // epilogue threads
 // same: the port is the bound, see above.)
 constexpr int conv_warps(int bn) { return bn == 128 ? 11 : 15; }
 constexpr int F_STAGES = 2;
+constexpr float F_SCALE = 65536.f, F_UNSCALE = 1.f / (65536.f * 65536.f);     // of an operand, of a sum of products
 constexpr int F_TMEM = 4;              // in tile widths: two accumulators, two group sums
 
 template <int BN>
@@ -81,7 +85,7 @@ __device__ __forceinline__ void ldg_f8(const float* p, float4& lo, float4& hi) {
 
 // Eight fp32 values -> the three bf16 terms, packed eight to 16 bytes.  h is rounded to nearest (half away), so what
 // is left over has either sign and the products that are left out do not add up; m and l cut the rest in two.
-// All exact, in integer and fp32 adds and byte permutes (the bf16 conversion instruction has a fraction of their rate).
+// All exact (the products with F_SCALE too, up to the largest number), in integer and fp32 adds and byte permutes (the bf16 conversion instruction has a fraction of their rate).
 __device__ __forceinline__ void split8(const float4& x0, const float4& x1, uint4 (&t)[3]) {
     const float v[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
     uint32_t w[3][4];
@@ -90,7 +94,7 @@ __device__ __forceinline__ void split8(const float4& x0, const float4& x1, uint4
         uint32_t h[2], m[2], l[2];
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-            const float x = v[2 * i + j];
+            const float x = v[2 * i + j] * F_SCALE;
             h[j] = (__float_as_uint(x) + 0x8000u) & 0xFFFF0000u;
             const float r = x - __uint_as_float(h[j]);
             m[j] = __float_as_uint(r) & 0xFFFF0000u;
@@ -104,13 +108,16 @@ __device__ __forceinline__ void split8(const float4& x0, const float4& x1, uint4
     for (int p = 0; p < 3; ++p) t[p] = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
 }
 
-// acc: NC columns n0.. of row m0 + lane.  Rows with a sum that is not finite are worked out again, a row at a time, a
-// lane per column (K and lda are multiples of four floats, see linear_f32_tc_supported).
+// acc: NC columns n0.. of row m0 + lane, sums of scaled products, which are scaled back.  Rows with a sum that is not
+// finite are worked out again, a row at a time, a lane per column (K and lda are multiples of four floats, see linear_f32_tc_supported).
 template <int NC>
-__device__ __forceinline__ void redo_nonfinite(float (&acc)[NC], const F32Args& g, int M, int m0, int n0, int lane) {
+__device__ __forceinline__ void unscale_or_redo(float (&acc)[NC], const F32Args& g, int M, int m0, int n0, int lane) {
     float t = 0.f;
 #pragma unroll
-    for (int i = 0; i < NC; ++i) t = fmaf(acc[i], 0.f, t);              // inf * 0 and NaN * 0 are NaN
+    for (int i = 0; i < NC; ++i) {
+        t = fmaf(acc[i], 0.f, t);              // inf * 0 and NaN * 0 are NaN
+        acc[i] *= F_UNSCALE;
+    }
     unsigned bad = __ballot_sync(0xffffffffu, t != t && m0 + lane < M);
     while (bad) {
         const int r = __ffs(bad) - 1;
@@ -413,7 +420,7 @@ linear_f32_tc_kernel(const F32Args g, int* status) {
                     for (int d = 0; d < SPLIT; ++d)
                         if (d != rank) mbar_arrive_release_cluster(mapa_u32(smem_u32(part_free), d));
                 }
-                redo_nonfinite<SC>(own, g, M, m0, n0 + rank * SC, lane);
+                unscale_or_redo<SC>(own, g, M, m0, n0 + rank * SC, lane);
                 const int m = m0 + lane;
                 if (m >= M) continue;
                 float* y = g.y + map_out_row(g.rm, m) * g.ldy;
@@ -441,7 +448,7 @@ linear_f32_tc_kernel(const F32Args g, int* status) {
                 }
                 continue;
             }
-            redo_nonfinite<CW>(acc, g, M, m0, n0, lane);
+            unscale_or_redo<CW>(acc, g, M, m0, n0, lane);
             // 32 columns at a time through the warp's transpose buffer (rows of eight 16-byte chunks, XOR-swizzled):
             // a lane then holds four columns of a row and eight lanes a whole 128-byte line
 #pragma unroll
