@@ -362,22 +362,10 @@ def model_roofline(model, batch, counts, ms_per_step, pk, image_bytes, fine):
 
 
 def launches_per_forward(model):
-    """Nominal kernel count of one forward, the figure that `gpu_launches` has always been formed from (nine kernels
-    around the blocks, cls rows and count resets among them).  Four of those nine have since been merged into others:
-    `counted_launches` is what is launched now."""
-    depth = len(model.blocks)
-    if model.compute_dtype() == torch.bfloat16 and not model.flags:
-        C = model.embed_dim
-        # the q and kv projections share one launch when both widths are whole 64-column slabs
-        paired = C >= 64 and C % 64 == 0
-        return 9 + (7 if paired else 8) * depth
-    return 5 + 12 * depth
-
-
-def counted_launches(model):
     """Kernels of this library in one forward: im2col (which writes the cls rows and starts the counts), patch-embed
     Linear, first gate, final LayerNorm and head; per block pool, q + kv, attention, proj, fc1, fc2 and unpool (which
-    leaves the next block's gate decisions).  fp32 blocks launch q and kv apart and the LayerNorm in front of fc1."""
+    leaves the next block's gate decisions).  q and kv share one launch when both widths are whole 64-column slabs;
+    fp32 blocks launch them apart, and the LayerNorm in front of fc1 too."""
     depth = len(model.blocks)
     if model.compute_dtype() == torch.bfloat16 and not model.flags:
         C = model.embed_dim
@@ -393,25 +381,28 @@ def profile_case(which):
     lib = _lib.lib()
     dev = torch.device("cuda", 0)
     torch.cuda.set_device(dev)
-    if which == "linear_kv":            # the kv projection of DeiT-S at batch 256: M=65792, N=768, K=384
+    if which in ("linear_kv", "linear_f32"):    # the kv projection of DeiT-S at batch 256: M=65792, N=768, K=384
         M, N, K = 65792, 768, 384
-        x = torch.randn(M, K, device=dev).bfloat16()
-        w = (torch.randn(N, K, device=dev) * 0.05).bfloat16()
+        dt = torch.bfloat16 if which == "linear_kv" else torch.float32
+        x = torch.randn(M, K, device=dev).to(dt)
+        w = (torch.randn(N, K, device=dev) * 0.05).to(dt)
         b = torch.randn(N, device=dev)
-        y = torch.empty(M, N, device=dev, dtype=torch.bfloat16)
+        y = torch.empty(M, N, device=dev, dtype=dt)
         for _ in range(3):
-            _lib.check(lib.vtp_linear(x.data_ptr(), K, w.data_ptr(), b.data_ptr(), None, 0, y.data_ptr(), N, 1, M,
-                                      None, N, K, 0, None))
-    elif which == "attention":          # 256 images x 6 heads, 114 queries per image, 257 keys
+            _lib.check(lib.vtp_linear(x.data_ptr(), K, w.data_ptr(), b.data_ptr(), None, 0, y.data_ptr(), N,
+                                      1 if dt == torch.bfloat16 else 0, M, None, N, K, 0, None))
+    elif which in ("attention", "attention_f32"):    # 256 images x 6 heads, 114 queries per image, 257 keys
         B, N, h, Li, d = 256, 257, 6, 114, 64
         C, L = h * d, B * Li
-        q = torch.randn(L, C, device=dev).bfloat16()
-        kv = torch.randn(B, N, 2 * C, device=dev).bfloat16()
-        out = torch.empty(L, C, device=dev, dtype=torch.bfloat16)
+        dt = torch.bfloat16 if which == "attention" else torch.float32
+        q = torch.randn(L, C, device=dev).to(dt)
+        kv = torch.randn(B, N, 2 * C, device=dev).to(dt)
+        out = torch.empty(L, C, device=dev, dtype=dt)
         off = (torch.arange(B + 1, device=dev) * Li).int()
         for _ in range(3):
-            _lib.check(lib.vtp_sparse_attention(q.data_ptr(), C, d, kv.data_ptr(), kv.data_ptr() + C * 2, N * 2 * C,
-                                                2 * C, d, out.data_ptr(), C, d, 1, B, N, h, d, off.data_ptr(), L, 257,
+            _lib.check(lib.vtp_sparse_attention(q.data_ptr(), C, d, kv.data_ptr(),
+                                                kv.data_ptr() + C * kv.element_size(), N * 2 * C, 2 * C, d,
+                                                out.data_ptr(), C, d, 1 if dt == torch.bfloat16 else 0, B, N, h, d, off.data_ptr(), L, 257,
                                                 d ** -0.5, 0, None))
     elif which == "block":              # one DeiT-S DGE block at batch 256 (gate, pool, GEMMs, attention, unpool)
         model = synthetic.build_model("small", dev, torch.bfloat16, depth=2)
@@ -830,7 +821,7 @@ def main():
                          "data loader hands over)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-stage-profile", action="store_true")
-    ap.add_argument("--profile", default=None, choices=["linear_kv", "attention", "block", "train_ops", "pvt_stage1", "pvt_model"],
+    ap.add_argument("--profile", default=None, choices=["linear_kv", "linear_f32", "attention", "attention_f32", "block", "train_ops", "pvt_stage1", "pvt_model"],
                     help="run a small case of one kernel family (for ncu) and exit")
     ap.add_argument("--layer-sweep", action="store_true",
                     help="time one DGE layer over gate skew against the dense block and exit")
@@ -982,10 +973,7 @@ def main():
                     "h2d_copy_alone_gbs_per_gpu": round(h2d_gbs, 1),
                     "h2d_note": "pinned-host-to-device copy of one step's images with nothing else running, all "
                                 "ranks at once, max over ranks"},
-            # per forward: im2col, cls rows, patch-embed GEMM, final LayerNorm, head GEMM, first block's gate,
-            # and per block: count, patch list, pool, 5 GEMMs, attention, unpool
             "gpu_launches": args.steps * launches_per_forward(model),
-            "gpu_launches_counted": args.steps * counted_launches(model),
             "clocks": clocks, "device_status": status, "peaks": pk_src,
             "rank_step_ms": {"max": ms_total / args.steps, "min": float(ms_min.item()) / args.steps},
         }

@@ -14,7 +14,8 @@
 //   O_c = P V_c        tcgen05.mma with A = P from TMEM and B = V chunk as an MN-major operand
 //                      straight from the TMA image of the [keys, d] rows; accumulator in TMEM
 //                      columns [64, 128), which are free once the first 128 keys are consumed: their
-//                      products run while the exp2 of the rest does (DeiT-S, 7 images: 680 -> 675 us)
+//                      products run while the exp2 of the rest does (DeiT-Ti, one image: 526 -> 522 us;
+//                      from 7 images on the gain is within the 1 % that two runs differ by)
 //   O  = O*alpha + O_c in registers of the softmax threads (online-softmax rescale), then the
 //                      tail keys, the 1/rowsum and the bf16 store.
 // Warp 0 lane 0 issues TMA (Q is double-buffered so the next item's Q and K stream in during
@@ -277,7 +278,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
             for (int i = 0; i < HD; ++i) o[i] = 0.f;
             const uint8_t* qrow = base + SM_Q + qb * (QT * HD * 2) + r * 128;
             // ---- the last n_keys % 16 keys run on CUDA cores.  Their scores (one fmaf chain in channel order each) are
-            // formed here: the rows arrived with Q, and the scores of the chunk are still being loaded and multiplied.
+            // formed here: the rows arrived with Q, and the scores of the chunk are still being loaded and multiplied
+            // (behind the chunk: DeiT-Ti, one image, 529 instead of 521 us; DeiT-S, 7 images, 687 instead of 680 us).
             const uint8_t* tb = base + SM_TAIL + qb * (2 * TAIL_ROWS * HD * 2);
             float tail_s[TAIL_ROWS];
             if (live) {
