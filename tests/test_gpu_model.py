@@ -582,3 +582,39 @@ def test_image_gives_the_same_bits_in_any_batch(kind, dtype):
         got = m(img[:n].contiguous())
         assert torch.equal(got, want[:n]), n
         assert all(torch.equal(a, b[:n]) for a, b in zip(m.last_counts, counts))
+
+
+@pytest.mark.parametrize("forced", [False, True])
+@pytest.mark.parametrize("extra", [0, 1])
+def test_packed_rows_listed_or_derived_by_the_pool(extra, forced):
+    """Many regions and images have the rows of a block's packed queries listed, few have the pool work them out: the same
+    bits and counts for an image, in the block that starts and in the one whose counts that one starts."""
+    from functools import partial
+
+    from vtpack_b200 import _lib
+    from vtpack_b200.models.dge import pvt_dge
+    torch.manual_seed(0)
+    blocks = [pvt_dge.Block(64, 1, mlp_ratio=2, qkv_bias=True, norm_layer=partial(torch.nn.LayerNorm, eps=1e-6), sr_ratio=8,
+                            split_sizes=[4, 2, 1]).eval().to(device=DEV, dtype=torch.bfloat16) for _ in range(2)]
+    if extra:                                                # a token in front of the grid: no spatial reduction
+        blocks = [pvt_dge.Block(64, 1, mlp_ratio=2, qkv_bias=True, sr_ratio=1, split_sizes=[4, 2, 1]).eval()
+                  .to(device=DEV, dtype=torch.bfloat16) for _ in range(2)]
+    for b in blocks:
+        torch.nn.init.normal_(b.dge.router.gate.weight, std=0.2)
+        torch.nn.init.zeros_(b.dge.router.gate.bias)
+    G, B = (32, 64) if extra else (64, 40)                   # 64 and 256 regions per image
+    x = torch.randn(B, G * G + extra, 64, device=DEV).bfloat16()
+    gate = torch.randn(B, G // 4, G // 4, 3, device=DEV) if forced else None
+
+    def run(n):
+        if forced:
+            y = blocks[0](x[:n].contiguous(), G, G, forced_gate=gate[:n].contiguous())
+            return y, [blocks[0].dge.states["batches_device"].clone()]
+        y = pvt_dge.stage_forward(blocks, x[:n].contiguous(), G, G)
+        return y, [b.dge.states["batches_device"].clone() for b in blocks]
+
+    many, counts = run(B)
+    for n in (1, 3):
+        few, c = run(n)
+        assert torch.equal(few, many[:n]) and all(torch.equal(p, q[:n]) for p, q in zip(c, counts))
+    assert len(set(counts[0].tolist())) > 1 and _lib.device_status() == 0

@@ -142,6 +142,14 @@ static bool block_chains(const vtp_dge_shape& s, const vtp_block_weights& w, con
     return block_folds(s, w) == block_folds(s, next);
 }
 
+// Whether the pool of a block that nothing prepared works out the packed rows itself: every warp of its B * R CTAs then
+// adds up the counts of the images in front and the grains of the regions in front.  From B * R * (B + R) of about
+// 500,000 on that costs more than the two launches of the patch-list kernels (one block with 64 channels, derived
+// against listed: 256 regions, 8 images 110.5 / 109.3 us, 32 images 242 / 234, 256 images 1442 / 1384; 576 regions, 128
+// images 1778 / 1627; 64 regions of 128 channels, 16 images 91.0 / 92.2, 96 images 283 / 281).  Where the gate has counted
+// already, deriving saves a launch more.
+static bool pool_derives_rows(long long B, long long R, bool counted) { return B * R * (B + R) < (counted ? 2000000 : 500000); }
+
 // Position of a block inside a model forward: whether the previous block's unpool already
 // produced this block's gate decisions and token statistics (in scratch slot `parity`), and
 // the block that follows, whose gate and statistics this block's unpool can produce.
@@ -198,6 +206,7 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
     // chained: gate decisions, per-image counts and token statistics came from the previous
     // block's unpool; the pool kernel then also derives the row offsets itself
     const bool chained = chain.have_gate && by_region && !forced_logits;
+    const bool derive = by_region && (chained || pool_derives_rows(s.B, Hr * Wr, chain.counts_started));
     VTP_REQUIRE(!chain.image_bias || by_region, VTP_ERR_UNSUPPORTED,
                 "block: a per-image gate bias needs the region-parallel gate (4x4-token regions)");
 
@@ -205,7 +214,7 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
         stats_x_ready = fold_q;
         rc = VTP_OK;
     } else if (forced_logits) {
-        rc = by_region ? count_queries(forced_logits, idx, sp, s.B, Hr * Wr, s.num_extra, counts, st)
+        rc = derive ? count_queries(forced_logits, idx, sp, s.B, Hr * Wr, s.num_extra, counts, st)
                        : vtp_gate_argmax(forced_logits, s.B * Hr * Wr, s.n_splits, idx, st);
     } else if (by_region) {
         RegionGateArgs ga;
@@ -220,16 +229,16 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
                              s.n_splits, b.logits[par], idx, st);
     }
     if (rc || (rc = marks.mark(1))) return rc;
-    // the region-parallel pool derives the packed rows from the counts; only the patch-list path needs the list
-    if (!by_region)
-        rc = index_to_patch(idx, 0, sp, s.B, Hr, Wr, s.region, s.num_extra, counts, b.offsets, b.patches, nullptr,
-                            nullptr, st);
+    if (!derive)
+        rc = index_to_patch(idx, 0, sp, s.B, Hr, Wr, s.region, s.num_extra, counts, b.offsets,
+                            by_region ? nullptr : b.patches, nullptr, by_region ? b.region_first : nullptr, st);
     else if (!chained && !forced_logits && !chain.counts_started)
         rc = count_queries(nullptr, idx, sp, s.B, Hr * Wr, s.num_extra, counts, st);
     if (rc || (rc = marks.mark(2))) return rc;
     if (by_region) {
         RegionPoolArgs pa;
         pa.g = g; pa.sp = sp; pa.x = x_in; pa.idx = idx; pa.comp = b.comp; pa.eps = s.eps;
+        pa.offsets = b.offsets; pa.region_first = derive ? nullptr : b.region_first;
         pa.counts = counts; pa.offsets_out = b.offsets; pa.region_first_out = b.region_first;
         const bool will_chain = chain.next && block_chains(s, w, *chain.next);
         pa.counts_next = will_chain ? counts_next : nullptr;

@@ -241,9 +241,9 @@ pool_region_kernel(const T* __restrict__ x, RegionGeom g, const int32_t* __restr
 #pragma unroll
             for (int o = G / 2; o > 0; o >>= 1) base += __shfl_xor_sync(0xffffffffu, base, o);
             dst_row = base + t;
-            // start the next block's per-image count at the extra tokens; its gate adds the rest
-            if (t == 0 && sub == 0 && counts_next) counts_next[b] = g.num_extra;
         }
+        // start the next block's per-image count at the extra tokens; its gate adds the rest
+        if (t == 0 && sub == 0 && counts_next) counts_next[b] = g.num_extra;
         Vec<T> row[CPL];
         load_row<T, CPL>(row, x + src_row * g.C, sub, G);
         store_row<T, CPL>(row, comp + (size_t)dst_row * g.C, sub, G);
@@ -293,11 +293,11 @@ pool_region_kernel(const T* __restrict__ x, RegionGeom g, const int32_t* __restr
             if (rr == 0) {
                 offsets_out[b] = img_base;
                 if (b == g.B - 1) offsets_out[g.B] = img_base + counts[b];
-                // a grid without extra tokens has no extra-token CTA to start the next block's count
-                if (counts_next && g.num_extra == 0) counts_next[b] = 0;
             }
         }
     }
+    // a grid without extra tokens has no extra-token CTA to start the next block's count
+    if (rr == 0 && w == 0 && lane == 0 && counts_next && g.num_extra == 0) counts_next[b] = 0;
 
     // per token: statistics / explicit LayerNorm, and at the finest grain the token is its own patch
     float acc[CPL][VN];                          // in-order sum of this group's tokens (of the current half)
