@@ -2,13 +2,13 @@
 // an independent check of the tcgen05 kernel.
 //
 // One CTA of four warps owns 32 packed queries of one (image, head) and walks the keys in chunks of up to 144 with an
-// online softmax.  A thread owns four query rows: of the scores it holds up to nine keys per row (keys tx, tx + 16,
+// online softmax. A thread owns four query rows: of the scores it holds up to nine keys per row (keys tx, tx + 16,
 // ...), of the output four channels, both in registers, so an inner step is 36 (or 16) fused multiply-adds per nine
-// (five) shared-memory vectors and the FMA pipe is the bound.  257 keys are two chunks of 136 and 121.  The sixteen
-// threads that share a row exchange its maximum and sum with shuffles.  Warps without live rows only stage K and V;
-// images with fewer queries launch CTAs that exit.  DeiT-S, 12 images in fp32: 71 us per launch for the form with
-// one score per thread and step and the whole score row in shared memory, 42 us for this one with synchronous staging,
-// 30 us with K and V copied asynchronously and unrolled steps.
+// (five) shared-memory vectors; busiest are the issue slots and the shared-memory port (64 % each; FMA pipe 47 %, 256
+// images). 257 keys are two chunks of 136 and 121. The sixteen threads that share a row exchange its maximum and sum
+// with shuffles. Warps without live rows only stage K and V; images with fewer queries launch CTAs that exit. DeiT-S,
+// 12 images in fp32: 71 us per launch for the form with one score per thread and step and the whole score row in shared
+// memory, 42 us for this one with synchronous staging, 30 us with K and V copied asynchronously and unrolled steps.
 //
 // Replaces batched_sparse_attention_forward
 // (vtpack/layers/csrc/batched_sparse_gemm/batched_sparse_gemm.cu:219-305): scale is applied
