@@ -137,7 +137,8 @@ __device__ __forceinline__ float warp_max(float v) {
 // the stream has completed and its writes are visible; what stands before it overlaps that kernel's tail.
 // griddep_launch() lets the kernel behind this one start once every CTA of this grid has called it.  It comes
 // AFTER the wait: a kernel that has started then knows that everything up to the kernel before its
-// predecessor has completed, so it may read constants (weights) before its own wait.
+// predecessor has completed.  What stands before the wait reads no tensor, weights included: the predecessor may be
+// the kernel that writes them.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_begin() { griddep_wait(); griddep_launch(); }
