@@ -618,3 +618,24 @@ def test_packed_rows_listed_or_derived_by_the_pool(extra, forced):
         few, c = run(n)
         assert torch.equal(few, many[:n]) and all(torch.equal(p, q[:n]) for p, q in zip(c, counts))
     assert len(set(counts[0].tolist())) > 1 and _lib.device_status() == 0
+
+
+def test_image_with_more_regions_than_a_list_holds():
+    """12544 regions do not fit the listing kernel's shared memory: the pool works their rows out.  The image is a smaller
+    one, whose 6272 regions are listed, twice: doubled keys leave a softmax average as it is, so its halves are the smaller
+    one's result but for the order of fp32 sums over 1568 and 3136 keys (3136 * 2^-24 = 1.9e-4 at worst)."""
+    from functools import partial
+
+    from vtpack_b200 import _lib
+    from vtpack_b200.models.dge import pvt_dge
+    torch.manual_seed(0)
+    blk = pvt_dge.Block(64, 1, mlp_ratio=2, qkv_bias=True, norm_layer=partial(torch.nn.LayerNorm, eps=1e-6), sr_ratio=8,
+                        split_sizes=[4, 2, 1]).eval().to(DEV)
+    H, W = 224, 448
+    x, gate = torch.randn(1, H * W, 64, device=DEV), torch.randn(1, H // 4, W // 4, 3, device=DEV)
+    small = blk(x, H, W, forced_gate=gate)
+    n = int(blk.dge.states["batches_device"])
+    big = blk(torch.cat((x, x), 1), 2 * H, W, forced_gate=torch.cat((gate, gate), 1))
+    assert int(blk.dge.states["batches_device"]) == 2 * n and _lib.device_status() == 0
+    for half in big.split(H * W, 1):
+        assert float((half - small).norm() / small.norm()) < 1.9e-4

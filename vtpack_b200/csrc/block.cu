@@ -147,8 +147,11 @@ static bool block_chains(const vtp_dge_shape& s, const vtp_block_weights& w, con
 // 500,000 on that costs more than the two launches of the patch-list kernels (one block with 64 channels, derived
 // against listed: 256 regions, 8 images 110.5 / 109.3 us, 32 images 242 / 234, 256 images 1442 / 1384; 576 regions, 128
 // images 1778 / 1627; 64 regions of 128 channels, 16 images 91.0 / 92.2, 96 images 283 / 281).  Where the gate has counted
-// already, deriving saves a launch more.
-static bool pool_derives_rows(long long B, long long R, bool counted) { return B * R * (B + R) < (counted ? 2000000 : 500000); }
+// already, deriving saves a launch more.  An image's regions are listed from shared memory (48 KB), so more than 8192 of
+// them are always derived.
+static bool pool_derives_rows(long long B, long long R, bool counted) {
+    return R > 8192 || B * R * (B + R) < (counted ? 2000000 : 500000);
+}
 
 // Position of a block inside a model forward: whether the previous block's unpool already
 // produced this block's gate decisions and token statistics (in scratch slot `parity`), and
