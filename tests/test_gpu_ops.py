@@ -600,6 +600,47 @@ def test_linear_fp32_rows_do_not_depend_on_the_launch(vl, N, K):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("N,K", [(8, 64), (72, 64), (192, 768), (200, 128), (256, 192), (384, 384), (392, 320), (768, 384), (1536, 256)])
+@pytest.mark.parametrize("gelu,res", [(False, False), (True, False), (False, True), (True, True)])
+def test_linear_bf16_rows_do_not_depend_on_the_launch(vl, N, K, gelu, res):
+    """The bits of a row are the same from the kernel of small problems, from single CTAs and from pairs, in whole tiles, strips
+    and narrow last tiles, with all rows of a warp valid and with some; rows beyond the device's row count stay as they were; and
+    the values are those of a float64 product: a sum of K <= 768 terms in fp32 (1e-5) rounded once to bf16 (2^-8 of the result);
+    GELU adds its fit's 2.7e-4 and, with u = 2^-11 the rounding of fp16, 1.13 u |x| for its argument, 0.9 u |x| for the four
+    roundings on the way to tanh's argument (a sech^2 a <= 0.45), 0.5 u |x| for tanh.approx and u |x| for the result: 4 u |x|."""
+    from vtpack_b200 import _lib
+    from vtpack_b200.runtime import ptr, stream_ptr
+    g = torch.Generator(DEV).manual_seed(N + K)
+    rows = 20000
+    x = torch.randn(rows, K, device=DEV, generator=g).bfloat16()
+    w = (torch.randn(N, K, device=DEV, generator=g) * K ** -0.5).bfloat16()
+    b = torch.randn(N, device=DEV, generator=g)
+    r = torch.randn(rows, N, device=DEV, generator=g).bfloat16() if res else None
+
+    def run(m_max, m_dev=None):
+        y = torch.full((m_max, N), 7.0, device=DEV, dtype=torch.bfloat16)
+        _lib.check(_lib.lib().vtp_linear(ptr(x), K, ptr(w), ptr(b), ptr(r), N, ptr(y), N, 1, m_max, ptr(m_dev), N, K, int(gelu),
+                                         stream_ptr(x.device)))
+        return y
+    full = run(rows)
+    ref = x.double() @ w.double().T + b.double()
+    bound = 1e-5 + (2.7e-4 + 2.0 ** -9 * ref.abs() if gelu else 0.0)
+    if gelu:
+        ref = torch.nn.functional.gelu(ref)
+    if res:
+        ref = ref + r.double()
+    err = (full.double() - ref).abs() - (2.0 ** -8 * ref.abs() + bound)
+    assert float(err.max()) <= 0
+    for M in (1, 31, 32, 33, 127, 128, 129, 257, 1000, 2970, 9475):
+        assert torch.equal(run(M), full[:M]), M
+    for M in (0, 1, 90, 2048, 3001):
+        y = run(rows, torch.tensor([M], dtype=torch.int32, device=DEV))
+        assert torch.equal(y[:M], full[:M]) and bool((y[M:] == 7.0).all()), M
+        y = run(4096, torch.tensor([M], dtype=torch.int32, device=DEV))
+        assert torch.equal(y[:M], full[:M]) and bool((y[M:] == 7.0).all()), M
+    assert _lib.device_status() == 0
+
+
 def test_threads_that_launch_give_their_memory_back(vl):
     """What a launching thread keeps (its encoded tensor maps, about 256 KB) goes with it."""
     import threading

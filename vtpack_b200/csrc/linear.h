@@ -25,20 +25,20 @@ struct LinearArgs {
     // LayerNorm folded into the GEMM (tcgen05 kernel only): `a` holds the raw rows, `w` holds
     // W*diag(gamma), ln_s[n] = sum_k w[n,k], bias[n] = sum_k beta[k] W[n,k] + b[n]; then
     //   LN(a) W^T + b = rstd[m] * (acc[m,n] - mean[m] * ln_s[n]) + bias[n].
-    // ln_mode 1: ln_stats[m] = (mean, rstd).  ln_mode 2: ln_stats[m * ln_slots + i], i < ln_slots,
-    // are partial (sum, sum of squares) over ln_dim elements in total (written by the GEMM that
+    // ln_mode 1: ln_stats[m] = (mean, rstd).  ln_mode 2: ln_stats[m * ln_slots + i], 64 i < ln_dim,
+    // are (sum, sum of squares) over 64 of the row's ln_dim elements each (written by the GEMM that
     // produced the rows, see emit_stats); variance = E[x^2] - mean^2, rstd = rsqrt(var + ln_eps).
     const float2* ln_stats = nullptr; const float* ln_s = nullptr;
     int ln_mode = 0, ln_dim = 0, ln_slots = 0; float ln_eps = 0.f;
-    // When set, every stored row leaves (sum, sum of squares) of its outputs here, one slot per
-    // (column tile, epilogue warp): plain stores, so the result does not depend on timing.
-    // linear_stat_slots(N) tells the consumer how many slots a row has.
+    // When set, every stored row leaves (sum, sum of squares) of its outputs here, one slot per 64 columns: plain
+    // stores, so the result does not depend on timing, nor, the columns being added in a fixed order, on the tiles.
+    // Slots of a row are linear_stat_slots(N) apart (an even number, for the consumer's 16-byte loads).
     float2* emit_stats = nullptr;
 };
 
-int linear_stat_slots(int N);              // float2 slots per row a tcgen05 GEMM with N output columns fills
+int linear_stat_slots(int N);              // float2 slots a tcgen05 GEMM with N output columns takes per row
 
-struct LnFold { const float2* stats; const float* s; int mode, dim; float eps; float2* emit; int slots; };
+struct LnFold { const float2* stats; const float* s; int mode, dim; float eps; float2* emit; int slots, used; };
 
 int linear_validate(const LinearArgs& p);
 int linear_cuda_cores(const LinearArgs& p, cudaStream_t st);   // fp32 or bf16 inputs, CUDA cores

@@ -3,29 +3,38 @@
 //
 //   y[m, n] = act(sum_k a[m,k] w[n,k] + bias[n]) + res[m, n]
 //
-// Persistent, warp-specialised: one CTA per SM walks 128 x BN output tiles (n fastest, so the
-// CTAs running at the same time share an A row tile in L2).
-//   warp 0   (one lane)  TMA producer: fills a STAGES-deep ring of {A 128x64, W BNx64} tiles;
-//                        the ring runs across tile boundaries, so the next tile's operands
-//                        stream in during the current tile's epilogue
-//   warp 1   (one lane)  issues tcgen05.mma (M=128, N=BN, K=16) into one of two TMEM
-//                        accumulators and commits each stage back to the producer
-//   warps 2-17           epilogue: read the finished accumulator with tcgen05.ld (warp w may
-//                        touch TMEM lanes 32*(w%4)..+31 = tile rows; four warps share a lane
-//                        quarter and split the columns), apply bias / GELU / residual, then
-//                        write the tile 64 columns at a time into one of two swizzled staging
-//                        slabs (full 128-byte lines, no partial sectors) and signal it full
-//                        on an mbarrier: the warps never wait for each other inside a tile.  The accumulator goes back to the MMA warp as soon as its
-//                        last columns are in registers.  Tiles that touch the last valid row,
-//                        row-remapped outputs and fp32 outputs store straight from registers.
-//   warp 18  (one lane)  store thread: waits for a full slab, hands it to a TMA store, waits until
-//                        the store has read it, then marks it free again or, when there is a
-//                        residual, has the TMA load the residual of the slab after next into it.
+// linear_tc_kernel is persistent and warp-specialised: one CTA per SM, alone or in pairs (cta_group::2), walks 128 x BN or
+// 256 x BN output tiles (n fastest, so the CTAs running at the same time share an A row tile in L2).
+//   producer warps  (one lane each) TMA: fill a ring of {A 128x64, W BNx64} k-blocks in turn; the ring runs across tile
+//                   boundaries, so the next tile's operands stream in during the current tile's epilogue
+//   MMA warp        (one lane) issues tcgen05.mma (K = 16 at a time) into one of two TMEM accumulators and commits each stage
+//                   back to the producers
+//   epilogue warps  one per TMEM lane quarter (the 32 rows it may read) and 64-column slab of the tile: tcgen05.ld, bias /
+//                   LayerNorm fold / GELU / residual, then through a 4 KB staging buffer of the warp's own (full 128-byte lines)
+//                   to its own TMA store.  No warp waits for another one's part of the tile.  Warps with rows beyond the last
+//                   valid one and row-remapped outputs copy the buffer out themselves; fp32 outputs go straight from registers.
 // The two accumulators let the MMA of tile i+1 overlap the epilogue of tile i.
 // The tiles left for the last, partial round of the grid are cut into two to four column strips
 // (their own W boxes, a narrower MMA), one per CTA, so that round costs a fraction of a tile.
 // The number of valid rows is read from device memory: tiles beyond it do not exist, rows
 // beyond it are never stored.
+// linear_tc_small_kernel (below) is the form for problems of few tiles.
+//
+// What bounds it, and what was measured (B200, launches replayed back to back in a graph, us; the kernel before: one CTA per
+// tile, staging slabs shared by all epilogue warps, a store thread):
+//                                                         before   now   cuBLAS (no epilogue)
+//   65792 x 768, K = 384 (DeiT-S kv, 256 images)           43.3   41.2   39.1    HBM and L2 writes: without stores 29.8
+//   23040 x 1536, K = 384, GELU (fc1)                      34.0   29.8   28.6    epilogue and writes
+//   23040 x 384, K = 1536, residual (fc2)                  39.0   30.8   25.5    2.4 rounds of tiles, their tail
+//   8481 x 1536, K = 768 (DeiT-B kv, 33 images)            24.6   21.7   18.1    2.8 rounds, start (4 us) and tail
+//   2970 x 768, K = 3072, residual (DeiT-B fc2)            21.0   17.5   13.9    one round
+//   172000 x 512, K = 64, GELU (PVT stage 1 fc1)           63.4   42.5   36.2    epilogue instructions, HBM (floor 31)
+//   393216 x 64, K = 64                                    28.3   19.5   18.0    HBM (floor 16)
+//   50176 x 3072, K = 768                                 199    183    201      tensor core under the power limit
+//   90 x 768, K = 192, GELU (DeiT-Ti fc1, one image)        5.5    3.3    2.6    latency (small kernel)
+//   90 x 192, K = 768, residual (DeiT-Ti fc2)               6.6    4.7    3.2    latency (small kernel): 48 MMA steps in a row
+// A k-block's loads cost their producer thread 265 to 450 cycles (try_wait 42, an arrival that the next try_wait waits behind
+// 130, the loads themselves), the MMAs of 192 or 256 columns 384 or 512: three producers take k-blocks in turn.
 //
 // Every mbarrier wait is bounded (see sm100.cuh); a wait that gives up ORs a code into the
 // device status word and the CTA unwinds.
@@ -33,7 +42,6 @@
 // Replaces nn.Linear q/kv/proj/fc1/fc2/head, nn.GELU and the residual adds of
 // vtpack/models/dge/deit_dge.py:38-44,72-74,96,127-128 (cuBLAS + ATen kernels there).
 #include <cuda_fp16.h>
-#include <stdlib.h>
 #include <string.h>
 
 #include <memory>
@@ -48,62 +56,37 @@ namespace vtp {
 using namespace sm100;
 
 constexpr int TBM = 128;   // tile rows of one CTA = TMEM lanes
-// CTAs per MMA tile.  2: the CTAs of a cluster of two share 256-row tiles (tcgen05 cta_group::2): each stages
-// its own 128 rows of A and half of the tile's W rows, the rank-0 CTA issues the MMAs, each CTA runs the
-// epilogue of its own 128 rows.  A CTA then stages and the tensor core reads 8 KB per 128 x 256 x 16 MMA step
-// instead of 12 KB; with one CTA per tile the shared-memory operand reads, not the tensor core, set the pace.
-#ifndef VTP_LINEAR_CTA_GROUP
-#define VTP_LINEAR_CTA_GROUP 1
-#endif
-constexpr int CG = VTP_LINEAR_CTA_GROUP;
-static_assert(CG == 1 || CG == 2, "one CTA or a pair per tile");
-constexpr int TM = TBM * CG;   // tile rows of the CTA group
-// Staging slabs of the epilogue (128 rows x 64 columns each); half as many TMA stores may be reading them at
-// a time.  A store's shared-memory read takes longer than the epilogue needs to fill the next slab, so with
-// two slabs the epilogue waits on the store; the pair kernel's smaller operand stages leave room for four.
-// A narrow Linear (N <= 128) with one k-block per tile, or two and a residual to fetch, spends its time in the
-// epilogue's hand-offs: it runs with a ring of SHALLOW_RING stages, gives the shared memory to four staging
-// slabs and keeps its bias slice across tiles (measured at 1 M rows, K = N = 64: 80 -> 71 us, with a residual
-// 117 -> 85 us; wide tiles with GELU and K = 128 without a residual were faster on the deep ring).
-constexpr int SHALLOW_RING = 3;
-constexpr int staging_slabs(int stages) { return CG == 2 ? 4 : (stages <= SHALLOW_RING ? 4 : 2); }
-// depth of the operand ring for a tile width: what fits beside the staging slabs
-constexpr int ring_stages(int bn) { return CG == 2 ? (bn == 128 ? 6 : 5) : (bn == 128 ? 5 : 4); }
 constexpr int TBK = 64;    // 64 bf16 = one 128-byte swizzle row
-constexpr int EPI_THREADS = 512;  // 16 epilogue warps, four per TMEM lane quarter
-constexpr int TC_THREADS = 64 + EPI_THREADS + 32;   // + the store warp
+constexpr int SLAB = 64;   // columns a warp takes through its staging buffer at a time: 128-byte rows
+constexpr int SLAB_BYTES = 32 * SLAB * 2;
+constexpr int SMEM_MAX = 232448;
 
-template <int BN, int STAGES>
-struct TcSmem {
+// EPI: what the epilogue does besides the bias, fixed at compile time so that a kernel only
+// issues the instructions of the variant it is (a runtime flag would be if-converted and the
+// GELU / LayerNorm arithmetic issued, predicated off, by every GEMM).
+constexpr int EPI_GELU = 1, EPI_LN = 2, EPI_EMIT = 4, EPI_RES = 8;
+
+template <int BN, int CG>
+struct TcConf {
+    static constexpr int EW = BN / SLAB * 4;             // epilogue warps: one per TMEM lane quarter and 64-column slab
+    static constexpr int PRODUCERS = 3;                  // warps that take the k-blocks in turn
+    static constexpr int FIRST_EPI = PRODUCERS + 1;      // ... behind the MMA warp
+    static constexpr int THREADS = (FIRST_EPI + EW) * 32;
     static constexpr int A_BYTES = TBM * TBK * 2;
-    static constexpr int B_BYTES = (BN / CG) * TBK * 2;   // this CTA's share of the W rows
+    static constexpr int B_BYTES = (BN / CG) * TBK * 2;  // this CTA's share of the W rows
+    static constexpr int STAGING = EW * SLAB_BYTES;
+    static constexpr int CTRL = 1024;                    // barriers, then the launch's scalars at CTRL_SCALARS
+    static constexpr int CTRL_SCALARS = 512;
+    // as deep a ring as fits; dynamic shared memory is only promised 16-byte alignment and the ring wants 1024, so
+    // the kernel checks that what is left behind the aligned base fits (in practice the base is aligned already)
+    static constexpr int FIT = (SMEM_MAX - STAGING - CTRL) / (A_BYTES + B_BYTES);
+    static constexpr int STAGES = FIT > 8 ? 8 : FIT;
     static constexpr int RING = STAGES * (A_BYTES + B_BYTES);
-    static constexpr int NSTG = staging_slabs(STAGES);
-    static constexpr int STORES_IN_FLIGHT = NSTG / 2;
-    static constexpr int STAGE_OUT = NSTG * TBM * 128;   // 128-row x 64-column bf16 slabs
-    static constexpr int BIAS = 2 * BN * 4;           // the bias and LayerNorm-fold slices of the tile in the epilogue
-    static constexpr int USED = RING + STAGE_OUT + BIAS + 512 /* barriers */;
-    // Dynamic shared memory is only promised 16-byte alignment; the ring wants 1024.  In
-    // practice the base is already aligned; the kernel checks that what is left fits.
-    static constexpr int TOTAL = (USED + 1024 <= 232448) ? USED + 1024 : 232448;
-    static_assert(USED <= 232448, "shared memory budget");
-    static constexpr int TMEM_COLS = (2 * BN <= 256) ? 256 : 512;
-};
-
-template <typename OutT> struct OutVec;
-template <> struct OutVec<bf16> {
-    // 8 values -> one 16-byte store
-    static __device__ __forceinline__ void store8(bf16* p, const float* v) {
-        Vec<bf16> o;
-        o.from_float(v);
-        o.store(p);
-    }
-};
-template <> struct OutVec<float> {
-    static __device__ __forceinline__ void store8(float* p, const float* v) {
-        reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
-        reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
-    }
+    static constexpr int USED = RING + STAGING + CTRL;
+    static constexpr int TOTAL = (USED + 1024 <= SMEM_MAX) ? USED + 1024 : SMEM_MAX;
+    static constexpr int TMEM_COLS = 2 * BN <= 256 ? 256 : 512;
+    static_assert(STAGES >= 3, "operand ring");
+    static_assert((2 * STAGES + 4 + EW) * 8 + 8 <= CTRL_SCALARS, "barrier area");
 };
 
 // erf-GELU of eight values, packed two per register in fp16, as 0.5 x (1 + tanh(x (k0 + k1 x^2))) with
@@ -134,29 +117,136 @@ __device__ __forceinline__ void gelu8(float* v) {
     }
 }
 
-// EPI: what the epilogue does besides the bias, fixed at compile time so that a kernel only
-// issues the instructions of the variant it is (a runtime flag would be if-converted and the
-// GELU / LayerNorm arithmetic issued, predicated off, by every GEMM).
-constexpr int EPI_GELU = 1, EPI_LN = 2, EPI_EMIT = 4;
+// Unsigned division by a number the host knows: multiply by ceil(2^32 / d), then take back the one the estimate may
+// be over (it is never under).  A runtime division is about forty dependent instructions on the way to a CTA's first load.
+struct FastDiv { uint32_t d, magic; };
+__device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv& f) {
+    if (f.d == 1) return n;
+    uint32_t q = __umulhi(n, f.magic);
+    if (q * f.d > n) --q;          // (n and d are below 2^31)
+    return q;
+}
 
-// One GEMM problem of a launch: its tensor maps and epilogue operands.
-struct TcProblem {
-    CUtensorMap ta, tw, tw2, tw3, ty, tr;    // A, W (tile / half / quarter height boxes), output, residual
+// One GEMM problem of a launch: its tensor maps, and the scalars the kernel reads.  Each CTA copies the scalars of a launch
+// to shared memory before it waits for the kernel in front: parameters are cold in every launch, and read where they are
+// needed each line of them is a miss of some 500 cycles on the way to the first load, and another on the way to the first store.
+struct TcScalars {
     const float* bias; const bf16* res; long long ldr;
     void* y; long long ldy;
-    int m_max; const int32_t* m_dev; int N;
-    int use_tma_store;
+    const int32_t* m_dev; int m_max; int N;
+    FastDiv n_tiles;
     RowMap rm; LnFold ln;
+    int use_tma_store;
 };
+struct TcMaps { CUtensorMap ta, tw, tws, ty, tr; };   // A, W (a whole tile's rows / 64 columns' rows), output, residual
 // A launch works through one problem or two independent ones (same K, tile shape and epilogue kind): the
 // tiles of the second fill the last, partial round of the first, and one launch's ramp and tail is saved.
-struct TcLaunch { TcProblem p[2]; int n; };
+struct TcSharedScalars { TcScalars p[2]; FastDiv groups; };
+struct TcLaunch { TcMaps m[2]; TcSharedScalars s; };
+static_assert(sizeof(TcSharedScalars) % 4 == 0 && sizeof(TcSharedScalars) <= 512, "copied to shared memory in words");
 
-template <int BN, int STAGES, typename OutT, int EPI, int NPROB>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+__device__ const float g_no_bias[8] = {};      // what a Linear without a bias adds
+
+// A row's folded LayerNorm, LN(a) W^T + b = ln_a * acc + (ln_b * s[n] + bias[n]), from its statistics.
+__device__ __forceinline__ void row_fold(const LnFold& ln, int m, float& ln_a, float& ln_b) {
+    if (ln.mode == 2) {
+        // (sum, sum of squares) of each 64-column slab of the row, left by the GEMM that produced it; added in order
+        const float4* sp = reinterpret_cast<const float4*>(ln.stats + (size_t)m * ln.slots);
+        const int used = ln.used;
+        const float dim = (float)ln.dim, eps = ln.eps;
+        float s1 = 0.f, s2 = 0.f;
+        for (int i0 = 0; 2 * i0 < used; i0 += 4) {
+            float4 v4[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)                    // independent 16-byte loads, one latency
+                v4[i] = (2 * (i0 + i) < used) ? sp[i0 + i] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                s1 += v4[i].x; s2 += v4[i].y;
+                if (2 * (i0 + i) + 1 < used) { s1 += v4[i].z; s2 += v4[i].w; }
+            }
+        }
+        const float mean = s1 / dim;
+        ln_a = rsqrtf(fmaxf(s2 / dim - mean * mean, 0.f) + eps);
+        ln_b = -ln_a * mean;
+    } else {
+        const float2 st = ln.stats[m];
+        ln_a = st.y;
+        ln_b = -st.y * st.x;
+    }
+}
+
+// The work items of one CTA group, in order.  Everything an item is worked out from is kept in registers: the first one
+// stands between the kernel in front and this one's first load.
+template <int BN, int CG, int NPROB>
+struct Schedule {
+    int M[NPROB], N[NPROB];
+    FastDiv nt[NPROB];
+    uint32_t G, tot0, full_items, strips, group;
+    int parts;
+    struct Item { int p, m0, ct0, width; };     // problem, first row of this CTA, output columns ct0 .. ct0 + width
+
+    __device__ __forceinline__ Schedule(const TcSharedScalars& L, bool void_launch) {
+        uint32_t total = 0;
+        tot0 = 0;
+#pragma unroll
+        for (int i = 0; i < NPROB; ++i) {
+            const int32_t* m_dev = L.p[i].m_dev;
+            M[i] = L.p[i].m_max;
+            N[i] = L.p[i].N;
+            nt[i] = L.p[i].n_tiles;
+            if (m_dev) M[i] = min(max(*reinterpret_cast<const volatile int32_t*>(m_dev), 0), M[i]);
+            if (i == 1) tot0 = total;
+            total += (uint32_t)((M[i] + TBM * CG - 1) / (TBM * CG)) * nt[i].d;
+        }
+        if (void_launch) total = 0;
+        G = L.groups.d;
+        group = blockIdx.x / CG;
+        // Tail splitting.  A CTA group takes tiles group, group + G, ...; the R tiles left for the last, partial round are
+        // cut into `parts` column strips of BN / parts columns, one per group, so that the round costs a fraction of a
+        // tile instead of a whole one with most SMs idle.  A problem with fewer tiles than groups is all last round.
+        // (Every sum of the epilogue covers at most one 64-column slab, so a row's bits do not depend on the strips.)
+        full_items = total < G ? 0 : fast_div(total, L.groups) * G;
+        const uint32_t R = total - full_items;
+        parts = 1;
+        if (BN == 256) parts = (R * 4 <= G) ? 4 : (R * 2 <= G ? 2 : 1);
+        else if (BN == 192) parts = (R * 3 <= G) ? 3 : 1;
+        else if (BN == 128) parts = (R * 2 <= G) ? 2 : 1;
+        strips = R * (uint32_t)parts;
+    }
+    __device__ __forceinline__ bool at(uint32_t j, Item& it) const {
+        uint32_t tile = group + j * G, sub = 0;
+        int strip = BN;
+        if (tile >= full_items) {
+            const uint32_t u = tile - full_items;
+            if (u >= strips) return false;
+            const uint32_t q = parts == 3 ? u / 3u : u >> (parts == 4 ? 2 : parts - 1);
+            tile = full_items + q;
+            sub = u - q * (uint32_t)parts;
+            strip = parts == 1 ? BN : (parts == 2 ? BN / 2 : SLAB);
+        }
+        it.p = (NPROB == 2 && tile >= tot0) ? 1 : 0;       // one-problem launches index their problem statically
+        const bool second = NPROB == 2 && it.p;
+        const uint32_t lt = tile - (second ? tot0 : 0);
+        const FastDiv n_tiles = second ? nt[NPROB - 1] : nt[0];
+        const uint32_t mt = fast_div(lt, n_tiles);
+        const int nt0 = (int)(lt - mt * n_tiles.d) * BN;
+        it.m0 = (int)mt * (TBM * CG) + (CG == 2 ? (int)cluster_ctarank() * TBM : 0);
+        // the last column tile is as wide as the columns left, in 64s
+        const int tile_w = min(BN, ((second ? N[NPROB - 1] : N[0]) - nt0 + SLAB - 1) & ~(SLAB - 1));
+        it.ct0 = nt0 + (int)sub * strip;
+        it.width = min(strip, tile_w - (int)sub * strip);
+        return true;                                       // (a strip beyond a narrow tile's columns has no width)
+    }
+};
+
+template <int BN, int CG, int EPI, bool F32, int NPROB>
+__global__ void __launch_bounds__(TcConf<BN, CG>::THREADS, 1)
 linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
-    using S = TcSmem<BN, STAGES>;
-    constexpr int NSTG = S::NSTG, STORES_IN_FLIGHT = S::STORES_IN_FLIGHT;
+    using S = TcConf<BN, CG>;
+    using Sched = Schedule<BN, CG, NPROB>;
+    using Item = typename Sched::Item;
+    constexpr int STAGES = S::STAGES, EW = S::EW, PRODUCERS = S::PRODUCERS;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* smem_a = base;
@@ -166,42 +256,49 @@ linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
         return;
     }
     uint8_t* smem_out = base + S::RING;
-    float* bias_s = reinterpret_cast<float*>(base + S::RING + S::STAGE_OUT);
-    uint64_t* full = reinterpret_cast<uint64_t*>(base + S::RING + S::STAGE_OUT + S::BIAS);
+    uint8_t* ctrl = smem_out + S::STAGING;
+    uint64_t* full = reinterpret_cast<uint64_t*>(ctrl);
     uint64_t* empty = full + STAGES;
     uint64_t* acc_full = empty + STAGES;       // [2]
     uint64_t* acc_empty = acc_full + 2;        // [2]
-    uint64_t* res_full = acc_empty + 2;        // [NSTG] residual slab landed in the staging buffer
-    uint64_t* slab_full = res_full + NSTG;     // [NSTG] every epilogue warp has written its part of the staging slab
-    uint64_t* slab_free = slab_full + NSTG;    // [NSTG] the TMA store has read the staging slab
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(slab_free + NSTG);
-    static_assert((2 * STAGES + 4 + 3 * NSTG) * 8 + 8 <= 512, "barrier area");
+    uint64_t* res_full = acc_empty + 2;        // [EW] the warp's residual slab has landed
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(res_full + EW);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const TcSharedScalars& sc = *reinterpret_cast<const TcSharedScalars*>(ctrl + S::CTRL_SCALARS);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const int num_kb = K / TBK;
     const int rank = CG == 2 ? (int)cluster_ctarank() : 0;             // this CTA within its group
-    const int n_groups = (int)gridDim.x / CG, group = (int)blockIdx.x / CG;
 
-    if (threadIdx.x == 0) {
+    // not zero: an earlier launch gave up on a wait and this one does nothing (fetched here, beside the set-up)
+    int status_word = 0;
+    if (status) status_word = *reinterpret_cast<volatile int*>(status);
+    for (int i = threadIdx.x; i < (int)sizeof(TcSharedScalars) / 4; i += S::THREADS)
+        reinterpret_cast<uint32_t*>(ctrl + S::CTRL_SCALARS)[i] = reinterpret_cast<const uint32_t*>(&L.s)[i];
+    if (warp == 0 && elect_one()) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], CG * (EPI_THREADS / 32));   // rank 0's: the epilogue warps of the whole group
+            mbar_init(&acc_empty[b], CG * EW);       // rank 0's: the epilogue warps of the whole group
         }
-        for (int b = 0; b < NSTG; ++b) {
-            mbar_init(&res_full[b], 1);
-            mbar_init(&slab_full[b], EPI_THREADS / 32);
-            mbar_init(&slab_free[b], 1);
-        }
+        for (int b = 0; b < EW; ++b) mbar_init(&res_full[b], 1);
         *abort_flag = 0;
         fence_barrier_init();
-        for (int i = 0; i < NPROB; ++i) { prefetch_tmap(&L.p[i].ta); prefetch_tmap(&L.p[i].tw); }
+        for (int i = 0; i < NPROB; ++i) {
+            prefetch_tmap(&L.m[i].ta);
+            prefetch_tmap(&L.m[i].tw);
+            prefetch_tmap(&L.m[i].tws);
+        }
     }
-    if (warp == 1) {
+    if (warp == PRODUCERS) {
         if (CG == 2) { tmem_alloc_pair(tmem_slot, S::TMEM_COLS); tmem_relinquish_pair(); }
         else { tmem_alloc(tmem_slot, S::TMEM_COLS); tmem_relinquish(); }
+    }
+    if (warp == 1 && elect_one()) {
+        for (int i = 0; i < NPROB; ++i) {
+            prefetch_tmap(&L.m[i].ty);
+            if (EPI & EPI_RES) prefetch_tmap(&L.m[i].tr);
+        }
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -212,487 +309,291 @@ linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
     // Everything above is independent of the kernel in front of this one on the stream; from
     // here on its results (row count, operands, residual, statistics) are read.
     pdl_begin();
-    // valid rows, column tiles and tile count of each problem
-    int Mp[2], ntp[2], totp[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        Mp[i] = ntp[i] = totp[i] = 0;
-        if (i < NPROB) {
-            Mp[i] = L.p[i].m_max;
-            if (L.p[i].m_dev) Mp[i] = min(*reinterpret_cast<const volatile int32_t*>(L.p[i].m_dev), L.p[i].m_max);
-            ntp[i] = (L.p[i].N + BN - 1) / BN;
-            totp[i] = ((Mp[i] + TM - 1) / TM) * ntp[i];
-        }
-    }
-    // no tiles for this CTA, or an earlier CTA gave up on a wait (the launch is void): skip the work
-    const bool void_launch = status && (*reinterpret_cast<volatile int*>(status) & STATUS_WAIT_MASK) != 0;
-    const int total = void_launch ? 0 : totp[0] + totp[1];
-    // Tail splitting.  A CTA group takes tiles group, + n_groups, ...; the R tiles left for the last,
-    // partial round are cut into `parts` column strips of BN / parts columns, one strip per group, so that
-    // the round costs a fraction of a tile instead of a whole one with most SMs idle.  Strips use their
-    // own W boxes (tw2 / tw3) and a narrower MMA.  A problem with fewer tiles than SMs is all last round.
-    // Kernels that leave row statistics (EPI_EMIT) do not split: a statistic is one sum over a whole tile's columns, so
-    // that a row's sums do not depend on how many rows there are (cut into strips, DeiT's bf16 logits of one image
-    // differed by 1 % between batches, through gates that near-ties flip).
-    const int full_items = (total / n_groups) * n_groups;
-    int parts = 1;
-    {
-        const int R = total - full_items, G = n_groups;
-        if (!(EPI & EPI_EMIT) && R > 0) {
-            if (BN == 256) parts = (R * 4 <= G) ? 4 : (R * 2 <= G ? 2 : 1);
-            else if (BN == 192) parts = (R * 3 <= G) ? 3 : 1;
-            else parts = (R * 2 <= G) ? 2 : 1;
-        }
-    }
-    // j-th work item of this CTA: problem p, this CTA's rows m0.., columns ct0 .. ct0 + width of its output.  The last
-    // column tile of a problem whose N is not a multiple of BN is as wide as the columns left, in 64s.
-    struct Item { int p, m0, nt, ct0, width; };
-    auto item_at = [&](int j, Item& it) -> bool {
-        const int idx = group + j * n_groups;
-        int tile, sub = 0, pr = 1;
-        if (idx < full_items) {
-            tile = idx;
-        } else {
-            const int u = idx - full_items;
-            if (u >= (total - full_items) * parts) return false;
-            tile = full_items + u / parts;
-            sub = u % parts;
-            pr = parts;
-        }
-        it.p = (NPROB == 2 && tile >= totp[0]) ? 1 : 0;       // one-problem launches index their problem statically
-        const int lt = tile - (it.p ? totp[0] : 0);
-        const int n_tiles = ntp[it.p];
-        it.m0 = (lt / n_tiles) * TM + rank * TBM;
-        it.nt = lt % n_tiles;
-        int tile_w = BN;
-        if (NPROB == 2) {
-            // narrow last column tile where a W box of that height exists (128 or 64 columns at BN = 256)
-            const int cols_left = ((L.p[it.p].N - it.nt * BN + 63) / 64) * 64;
-            if (BN == 256 && (cols_left == 64 || cols_left == 128)) tile_w = cols_left;
-        }
-        it.width = pr == 1 ? tile_w : BN / pr;
-        it.ct0 = it.nt * BN + sub * it.width;
-        return sub * it.width < tile_w;        // a strip beyond a narrow tile's columns does not exist
-    };
+    const Sched sched(sc, (status_word & STATUS_WAIT_MASK) != 0);
 
-    if (warp == 0) {
-        if (lane == 0) {
-            // ------------------------------------------------------------ TMA producer
-            int it = 0;
+    // The two loops below run in one thread each, and a k-block has a few hundred cycles: shared memory goes by 32-bit
+    // addresses that advance with the ring.
+    const uint32_t full_a = smem_u32(full), empty_a = smem_u32(empty);
+    if (warp < PRODUCERS) {
+        if (elect_one()) {
+            // ------------------------------------------------------------ TMA producers
+            // A k-block costs its producer some 400 cycles (the wait, the barrier, two loads), which is about what the tensor core
+            // takes for it: three warps take them in turn.
+            const uint32_t ring_a = smem_u32(smem_a), ring_b = smem_u32(smem_b);
+            int s = 0, turn = warp;
+            uint32_t ph = 1, filled = 0;
             bool ok = true;
             Item wi;
-            for (int j = 0; ok && item_at(j, wi); ++j) {
-                // the W box that holds this CTA's share of the item's columns
-                const TcProblem& P = L.p[wi.p];
-                const CUtensorMap* wm = wi.width == BN ? &P.tw : ((BN == 256 && wi.width == 64) ? &P.tw3 : &P.tw2);
+            for (uint32_t j = 0; ok && sched.at(j, wi); ++j) {
+                if (wi.width <= 0) continue;
+                const TcMaps& P = L.m[wi.p];
+                const bool whole = wi.width == BN;
                 const int wshare = wi.width / CG;
                 const uint32_t bytes = CG * (S::A_BYTES + (uint32_t)wshare * TBK * 2);     // of the whole group
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1;
-                    ok = mbar_wait(&empty[s], ph ^ 1, abort_flag, status, STATUS_GEMM_PRODUCER);
-                    if (!ok) break;
-#if defined(VTP_LINEAR_EXPERIMENT) && (VTP_LINEAR_EXPERIMENT & 1)
-                    // measurement build: no operand traffic, the MMAs run on whatever the ring holds
-                    (void)bytes; (void)wm;
-                    mbar_arrive(&full[s]);
-#else
-                    if (CG == 1) {
-                        mbar_arrive_expect_tx(&full[s], bytes);
-                        tma_load_2d(smem_a + s * S::A_BYTES, &P.ta, &full[s], kb * TBK, wi.m0);
-                        tma_load_2d(smem_b + s * S::B_BYTES, wm, &full[s], kb * TBK, wi.ct0);
-                    } else {
-                        // both CTAs' bytes are counted on rank 0's barrier, which its MMA thread waits on
-                        if (rank == 0) mbar_arrive_expect_tx(&full[s], bytes);
-                        const uint32_t fb = mapa_u32(smem_u32(&full[s]), 0);
-                        tma_load_2d_pair(smem_a + s * S::A_BYTES, &P.ta, fb, kb * TBK, wi.m0);
-                        tma_load_2d_pair(smem_b + s * S::B_BYTES, wm, fb, kb * TBK, wi.ct0 + rank * wshare);
+                const int wrow = wi.ct0 + rank * wshare;
+                for (int x = 0; x < K; x += TBK) {
+                    if (turn == 0) {
+                        const uint32_t fb = full_a + 8 * s, da = ring_a + s * S::A_BYTES, db = ring_b + s * S::B_BYTES;
+                        ok = mbar_wait_a(empty_a + 8 * s, ph, abort_flag, status, STATUS_GEMM_PRODUCER);
+                        if (!ok) break;
+                        // (both CTAs' bytes of a pair are counted on rank 0's barrier, which its MMA thread waits on)
+                        if (CG == 1 || rank == 0) mbar_arrive_expect_tx_a(fb, bytes);
+                        const uint32_t lead = CG == 1 ? fb : mapa_u32(fb, 0);
+                        tma_load_2d_a<CG>(da, &P.ta, lead, x, wi.m0);
+                        if (whole) tma_load_2d_a<CG>(db, &P.tw, lead, x, wrow);
+                        else for (int c = 0; c < wshare; c += SLAB / CG) tma_load_2d_a<CG>(db + c * (TBK * 2), &P.tws, lead, x, wrow + c);
+                        turn = PRODUCERS;
                     }
-#endif
+                    --turn;
+                    ++filled;
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
             }
-            if (CG == 2 && ok) {
+            if (CG == 2 && ok && warp == 0) {
                 // The MMA thread's last commits arrive on this CTA's `empty` barriers, from the partner for
                 // rank 1: wait for them, so that nothing is signalled into a CTA that has retired.
-                for (int s = 0; s < STAGES && ok; ++s) {
-                    if (it <= s) break;
-                    const int uses = (it - s + STAGES - 1) / STAGES;
-                    ok = mbar_wait(&empty[s], (uses - 1) & 1, abort_flag, status, STATUS_GEMM_PRODUCER);
+                for (int i = 0; i < STAGES && ok; ++i) {
+                    if (filled <= (uint32_t)i) break;
+                    const uint32_t uses = (filled - i + STAGES - 1) / STAGES;
+                    ok = mbar_wait_a(empty_a + 8 * i, (uses - 1) & 1, abort_flag, status, STATUS_GEMM_PRODUCER);
                 }
             }
         }
         __syncwarp();
-    } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+    } else if (warp == PRODUCERS) {
+        if (rank == 0 && elect_one()) {
             // -------------------------------------------------------------- MMA issuer (of the group)
-            int it = 0, lt = 0;
+            int s = 0, lt = 0;
+            uint32_t ph = 0;
             bool ok = true;
+            const uint64_t adesc0 = smem_desc_sw128(smem_u32(smem_a));
+            const uint64_t bdesc0 = smem_desc_sw128(smem_u32(smem_b));
             Item wi;
-            for (int j = 0; ok && item_at(j, wi); ++j, ++lt) {
-                const uint32_t idesc = idesc_bf16_f32(TM, wi.width, 0, 0);
+            for (uint32_t j = 0; ok && sched.at(j, wi); ++j) {
+                if (wi.width <= 0) continue;
+                const uint32_t idesc = idesc_bf16_f32(TBM * CG, wi.width, 0, 0);
                 const int buf = lt & 1;
-                const uint32_t aph = (lt >> 1) & 1;
-                ok = mbar_wait(&acc_empty[buf], aph ^ 1, abort_flag, status, STATUS_GEMM_MMA);
+                ok = mbar_wait(&acc_empty[buf], ((lt >> 1) & 1) ^ 1, abort_flag, status, STATUS_GEMM_MMA);
                 if (!ok) break;
                 tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + buf * BN;
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1;
-                    ok = mbar_wait(&full[s], ph, abort_flag, status, STATUS_GEMM_MMA);
+                for (int x = 0; x < K; x += TBK) {
+                    ok = mbar_wait_a(full_a + 8 * s, ph, abort_flag, status, STATUS_GEMM_MMA);
                     if (!ok) break;
                     tc_fence_after_sync();
-                    const uint64_t adesc = smem_desc_sw128(smem_u32(smem_a + s * S::A_BYTES));
-                    const uint64_t bdesc = smem_desc_sw128(smem_u32(smem_b + s * S::B_BYTES));
+                    const uint64_t adesc = adesc0 + (uint64_t)(s * (S::A_BYTES >> 4));
+                    const uint64_t bdesc = bdesc0 + (uint64_t)(s * (S::B_BYTES >> 4));
 #pragma unroll
                     for (int k = 0; k < TBK / 16; ++k) {
                         // 16 bf16 of K = 32 bytes = 2 descriptor address units inside the swizzle row
-                        if (CG == 2) umma_ss_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
-                        else umma_ss(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                        if (CG == 2) umma_ss_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (x | k) != 0 ? 1u : 0u);
+                        else umma_ss(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (x | k) != 0 ? 1u : 0u);
                     }
-                    if (CG == 2) umma_commit_pair(&empty[s]); else umma_commit(&empty[s]);
+                    umma_commit_a<CG>(empty_a + 8 * s);
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
-                if (ok) { if (CG == 2) umma_commit_pair(&acc_full[buf]); else umma_commit(&acc_full[buf]); }
+                if (ok) umma_commit_a<CG>(smem_u32(&acc_full[buf]));
+                ++lt;
             }
-        }
-        __syncwarp();
-    } else if (warp == 2 + EPI_THREADS / 32) {
-        if (lane == 0 && L.p[0].use_tma_store) {
-            // -------------------------------------------------------------- store thread
-            // Walks the staged slabs in the epilogue's order: (item j, slab sl) of every item whose 128 rows
-            // are all valid (the items with the last, partial rows come last and store from registers).
-            struct Cursor { int j, sl; Item it; bool ok; };
-            // the staged items: all 128 rows valid.  (Items with the last, partial rows of a problem store from
-            // registers; they are skipped here exactly as the epilogue warps skip the staging for them.)
-            auto staged = [&](const Item& it) { return it.m0 + TBM <= Mp[it.p]; };
-            auto seek = [&](Cursor& c) {                  // first staged item at or after c.j
-                for (;;) {
-                    if (!item_at(c.j, c.it)) { c.ok = false; return; }
-                    if (staged(c.it)) { c.ok = true; return; }
-                    ++c.j;
-                }
-            };
-            auto first = [&]() { Cursor c; c.j = 0; c.sl = 0; seek(c); return c; };
-            auto advance = [&](Cursor& c) {
-                if (++c.sl == c.it.width / 64) { c.sl = 0; ++c.j; seek(c); }
-            };
-            auto load_residual = [&](const Cursor& c, int b) {
-                mbar_arrive_expect_tx(&res_full[b], TBM * 128);
-                tma_load_2d(smem_out + b * (TBM * 128), &L.p[c.it.p].tr, &res_full[b], c.it.ct0 + c.sl * 64, c.it.m0);
-            };
-            Cursor cur = first(), ahead = cur;        // `ahead` runs NSTG slabs in front (residual prefetch)
-            const bool res = L.p[0].res != nullptr;
-            if (res) {
-                for (int b = 0; b < NSTG && ahead.ok; ++b) { load_residual(ahead, b); advance(ahead); }
-            }
-            bool ok = true;
-            for (int slab_no = 0; cur.ok && ok; ++slab_no, advance(cur)) {
-                const int b = slab_no % NSTG;
-                ok = mbar_wait(&slab_full[b], (slab_no / NSTG) & 1, abort_flag, status, STATUS_GEMM_EPILOGUE);
-                if (!ok) break;
-#if !(defined(VTP_LINEAR_EXPERIMENT) && (VTP_LINEAR_EXPERIMENT & 2))     // measurement build: no output traffic
-                tma_store_2d(&L.p[cur.it.p].ty, smem_out + b * (TBM * 128), cur.it.ct0 + cur.sl * 64, cur.it.m0);
-#endif
-                bulk_commit_group();
-                // every store but the newest STORES_IN_FLIGHT - 1 has read its slab: the slab of the last of those
-                // can be written again (with a residual: it receives the residual of the slab NSTG further on)
-                bulk_wait_group_read<STORES_IN_FLIGHT - 1>();
-                if (slab_no >= STORES_IN_FLIGHT - 1) {
-                    const int fb = (slab_no - (STORES_IN_FLIGHT - 1)) % NSTG;
-                    if (res) {
-                        if (ahead.ok) { load_residual(ahead, fb); advance(ahead); }
-                    } else {
-                        mbar_arrive(&slab_free[fb]);
-                    }
-                }
-            }
-            bulk_wait_group0();                       // every TMA store has landed before the CTA retires
         }
         __syncwarp();
     } else {
         // ------------------------------------------------------------------- epilogue
+        // A warp works on its own: TMEM lanes 32 * (warp % 4) .. + 31 (the rows it may read) of one 64-column slab of each
+        // item, through a staging buffer of its own that its own TMA store empties; no warp waits for another.
+        const int e = warp - S::FIRST_EPI;
+        const int quarter = warp & 3;
+        const int sl = e >> 2;                        // slab of an item
+        const bool leader = elect_one();
+        uint8_t* buf_s = smem_out + e * SLAB_BYTES;   // residual in, result out
         // the accumulator goes back to the MMA thread, which runs in the group's rank-0 CTA
         auto release_acc = [&](int b) {
-            if (CG == 2) mbar_arrive_cluster(mapa_u32(smem_u32(&acc_empty[b]), 0));
-            else mbar_arrive(&acc_empty[b]);
+            tc_fence_before_sync();
+            __syncwarp();
+            if (leader) {
+                if (CG == 2) mbar_arrive_cluster(mapa_u32(smem_u32(&acc_empty[b]), 0));
+                else mbar_arrive(&acc_empty[b]);
+            }
         };
-        const int quarter = warp & 3;                 // TMEM lane quarter this warp may read
-        const int qsub = (warp - 2) >> 2;             // which of the four warps of that quarter
-        const int row = quarter * 32 + lane;          // tile row = TMEM lane
-        int lt = 0, slab_no = 0;
-        int held_p = -1, held_ct0 = -1, held_width = -1;   // the bias slice that is in shared memory
+        int lt = 0;
+        uint32_t res_ph = 0;
         bool ok = true;
         Item wi;
-        for (int j = 0; ok && item_at(j, wi); ++j, ++lt) {
-            const TcProblem& P = L.p[wi.p];
-            const int M = Mp[wi.p], N = P.N;
-            const float* __restrict__ bias = P.bias;
-            const bf16* __restrict__ res = (EPI & EPI_LN) ? nullptr : P.res;     // (no launch folds and adds)
-            const LnFold& ln = P.ln;
-            const int m0 = wi.m0;
-            const int nt0 = wi.ct0;                   // first output column of the item
-            const int NSLAB = wi.width / 64;          // 64-column slabs in it
+        for (uint32_t j = 0; ok && sched.at(j, wi); ++j) {
+            if (wi.width <= 0) continue;
+            const TcScalars& P = sc.p[wi.p];
+            const TcMaps& T = L.m[wi.p];
+            const int M = (NPROB == 2 && wi.p) ? sched.M[NPROB - 1] : sched.M[0], N = P.N;
             const int buf = lt & 1;
             const uint32_t aph = (lt >> 1) & 1;
-            const bool tma_path = P.use_tma_store && m0 + TBM <= M;
-            // A CTA whose tiles keep to one column range (a Linear no wider than a tile, or a column-tile count
-            // that divides the grid) loads the slice once: a short-K tile is too brief to hide a global load and
-            // two barriers of the sixteen warps in.
-            const bool new_slice = tma_path && !(STAGES <= SHALLOW_RING && wi.p == held_p && nt0 == held_ct0 &&
-                                                 wi.width == held_width);
-            if (new_slice) {
-                // this tile's bias slice -> shared memory (one value per thread), so the column
-                // loop reads it as a broadcast instead of through the global-load path
-                named_barrier(1, EPI_THREADS);                       // nobody reads the previous slice any more
-                held_p = wi.p; held_ct0 = nt0; held_width = wi.width;
-                const int te = threadIdx.x - 64;
-                if (te < wi.width) {
-                    bias_s[te] = (bias && nt0 + te < N) ? __ldg(bias + nt0 + te) : 0.f;
-                    if (EPI & EPI_LN) bias_s[BN + te] = (nt0 + te < N) ? __ldg(ln.s + nt0 + te) : 0.f;
+            ++lt;
+            const int wrow0 = wi.m0 + quarter * 32;         // the warp's first row
+            const int n0 = wi.ct0 + sl * SLAB;
+            const bool active = wrow0 < M && sl * SLAB < wi.width;
+            // the residual of 32 valid rows comes by TMA, mapped rows and those beside the last valid one are copied by the warp
+            const bool res_tma = P.rm.res_mod <= 0 && wrow0 + 32 <= M;
+            float2 b2[8], s2[8];                                       // bias and fold vector of this thread's columns
+            float ln_a = 1.f, ln_b = 0.f;                              // of row `lane` of the warp
+            if (active) {
+                // what the slab needs besides the accumulator travels while the MMAs run
+                // (the columns of a partial slab beyond N read the last ones; what is made of them is not stored)
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const int nb = min(n0 + 8 * c, N - 8) + 2 * (lane & 3);
+                    b2[c] = __ldg(reinterpret_cast<const float2*>(P.bias ? P.bias + nb : g_no_bias));
+                    if (EPI & EPI_LN) s2[c] = __ldg(reinterpret_cast<const float2*>(P.ln.s + nb));
                 }
-            }
-            // Where the epilogue is the bound (GELU without a fold, and bias only in the short-K variant: the Linears of PVT's
-            // first stages) the accumulator is waited for before anything else.  The loads ahead of the wait that small
-            // launches gain from lengthen the instruction stream of the whole-tile path too: M = 131072, N = 512, K = 64 with
-            // GELU 51.6 us this way, 55.2 with them; M = 1048576, N = K = 64 65.9 / 68.2.  The other variants hide it
-            // (DeiT-S, 256 images: 3.34 ms with every variant this way, 3.28 with none).
-            constexpr bool WAIT_FIRST = EPI == EPI_GELU || (EPI == 0 && STAGES <= SHALLOW_RING);
-            if (WAIT_FIRST) {
-                ok = mbar_wait(&acc_full[buf], aph, abort_flag, status, STATUS_GEMM_EPILOGUE);
-                if (!ok) break;
-                tc_fence_after_sync();
-            }
-            const uint32_t tacc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BN;
-            // folded LayerNorm: out = ln_a * acc + ln_b * s[n] + bias[n]
-            // (the statistics are fetched while the MMAs of the tile are still running)
-            float ln_a = 1.f, ln_b = 0.f;
-            if ((EPI & EPI_LN) && m0 + row < M) {
-                float2 st;
-                if (ln.mode == 2) {
-                    // partial (sum, sum of squares) left by the GEMM that produced the rows, one slot
-                    // per (column tile, epilogue warp of the lane quarter); added in a fixed order
-                    st = make_float2(0.f, 0.f);
-                    const float4* sp = reinterpret_cast<const float4*>(ln.stats + (size_t)(m0 + row) * ln.slots);
-                    for (int i0 = 0; 2 * i0 < ln.slots; i0 += 8) {
-                        float4 v4[8];
-#pragma unroll
-                        for (int i = 0; i < 8; ++i)                    // independent 16-byte loads, one latency
-                            v4[i] = (2 * (i0 + i) < ln.slots) ? sp[i0 + i] : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) { st.x += v4[i].x; st.y += v4[i].y; st.x += v4[i].z; st.y += v4[i].w; }
-                    }
-                } else {
-                    st = ln.stats[m0 + row];
-                }
-                float mean = st.x, rstd = st.y;
-                if (ln.mode == 2) {
-                    mean = st.x / (float)ln.dim;
-                    rstd = rsqrtf(fmaxf(st.y / (float)ln.dim - mean * mean, 0.f) + ln.eps);
-                }
-                ln_a = rstd;
-                ln_b = -rstd * mean;
-            }
-            if (EPI & EPI_LN) {
-                // warm L1 with the row statistics the next tile of this CTA will start with
-                Item nxt;
-                const int mn = (item_at(j + 1, nxt) && nxt.p == wi.p) ? nxt.m0 + row : M;
-                if (mn < M) {
-                    const float2* nxt = ln.stats + (size_t)mn * (ln.mode == 2 ? ln.slots : 1);
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(nxt));
-                }
-            }
-            float e1 = 0.f, e2 = 0.f;     // sum and sum of squares of this thread's outputs
-            auto emit = [&]() {
-                if (EPI & EPI_EMIT) ln.emit[(size_t)(m0 + row) * ln.slots + wi.nt * 4 + qsub] = make_float2(e1, e2);
-            };
-            auto wait_acc = [&]() {
-                ok = mbar_wait(&acc_full[buf], aph, abort_flag, status, STATUS_GEMM_EPILOGUE);
-                if (ok) tc_fence_after_sync();
-            };
-            if (tma_path) {
-                if (!WAIT_FIRST) {
-                    wait_acc();
-                    if (!ok) break;
-                }
-                // ---- full tile: registers -> swizzled staging slab -> TMA store
-                // The slab loop is unrolled (two register sets take the tensor-memory loads in turn, so nothing is
-                // copied) and every shared-memory access goes through a 32-bit shared-space address worked out once
-                // per tile: the tensor core pays for each instruction these sixteen warps issue.
-                if (new_slice) named_barrier(1, EPI_THREADS);        // bias slice complete
-                const uint32_t cell0 = (uint32_t)row * 128u + ((uint32_t)((qsub * 2) ^ (row & 7)) << 4);
-                const uint32_t cell1 = (uint32_t)row * 128u + ((uint32_t)((qsub * 2 + 1) ^ (row & 7)) << 4);
-                const uint32_t stage_a = smem_u32(smem_out);
-                const uint32_t vec_a = smem_u32(bias_s) + (uint32_t)qsub * 64u;     // this thread's 16 columns of slab 0
-                uint32_t rbuf[2][16];
-                __syncwarp();
-                tmem_ld_32x16(tacc + qsub * 16, rbuf[0]);
-#pragma unroll
-                for (int sl = 0; sl < BN / 64; ++sl) {
-                    if (sl >= NSLAB || !ok) continue;
-                    uint32_t (&r)[16] = rbuf[sl & 1];
-                    // the additive part of this slab's 16 columns (bias, or bias + ln_b * s for a folded
-                    // LayerNorm), fetched from shared memory while the accumulator columns are on their way
-                    float cadd[16];
-#pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4) {
-                        const float4 b = lds_f4(vec_a + (uint32_t)sl * 256u + q4 * 16u);
-                        cadd[4 * q4] = b.x; cadd[4 * q4 + 1] = b.y; cadd[4 * q4 + 2] = b.z; cadd[4 * q4 + 3] = b.w;
-                        if (EPI & EPI_LN) {
-                            const float4 sv = lds_f4(vec_a + (uint32_t)BN * 4u + (uint32_t)sl * 256u + q4 * 16u);
-                            cadd[4 * q4] = fmaf(ln_b, sv.x, b.x); cadd[4 * q4 + 1] = fmaf(ln_b, sv.y, b.y);
-                            cadd[4 * q4 + 2] = fmaf(ln_b, sv.z, b.z); cadd[4 * q4 + 3] = fmaf(ln_b, sv.w, b.w);
-                        }
-                    }
-                    tmem_ld_wait();
-                    if (sl + 1 < NSLAB) {
-                        __syncwarp();
-                        tmem_ld_32x16(tacc + (sl + 1) * 64 + qsub * 16, rbuf[(sl + 1) & 1]);     // next slab in flight
-                    } else {
-                        tc_fence_before_sync();
-                        __syncwarp();
-                        if (lane == 0) release_acc(buf);                        // accumulator is free
-                    }
-                    const int sb = slab_no % NSTG;                                // staging slab of this one
-                    const uint32_t srow_a = stage_a + (uint32_t)sb * (TBM * 128);
-                    if (res) {
-                        // the residual of this slab is in the staging slab (so the slab is free, too)
-                        ok = mbar_wait(&res_full[sb], (slab_no / NSTG) & 1, abort_flag, status,
-                                       STATUS_GEMM_EPILOGUE);
-                    } else if (slab_no >= NSTG) {
-                        // the store of the slab that used this staging slab last has read it
-                        ok = mbar_wait(&slab_free[sb], ((slab_no / NSTG) - 1) & 1, abort_flag, status,
-                                       STATUS_GEMM_EPILOGUE);
-                    }
-                    if (!ok) continue;
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        const uint32_t cell = srow_a + (j ? cell1 : cell0);
-                        float vj[8];
-                        if (EPI & EPI_LN) {
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) vj[i] = fmaf(ln_a, __uint_as_float(r[8 * j + i]), cadd[8 * j + i]);
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) vj[i] = __uint_as_float(r[8 * j + i]) + cadd[8 * j + i];
-                        }
-                        if (EPI & EPI_GELU) gelu8(vj);
-                        if (res) {
-                            Vec<bf16> rv;
-                            float rf[8];
-                            rv.raw = lds_u4(cell);                               // residual slab, same layout
-                            rv.to_float(rf);
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) vj[i] += rf[i];
-                        }
-                        if ((EPI & EPI_EMIT) && nt0 + sl * 64 + (qsub * 2 + j) * 8 < N) {
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) { e1 += vj[i]; e2 = fmaf(vj[i], vj[i], e2); }
-                        }
-                        Vec<bf16> ov;
-                        ov.from_float(vj);
-                        sts_u4(cell, ov.raw);
-                    }
-                    fence_proxy_async_smem();
+                if (EPI & EPI_RES) {
+                    if (leader) bulk_wait_group_read0();               // the last item's store has read the buffer
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&slab_full[sb]);                // this warp's part of the slab is in place
-                    ++slab_no;
+                    if (!res_tma) {
+                        const int c = lane & 7;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const int rr = i * 4 + (lane >> 3);
+                            uint4 v = make_uint4(0, 0, 0, 0);
+                            if (wrow0 + rr < M && n0 + c * 8 < N)
+                                v = *reinterpret_cast<const uint4*>(P.res + map_res_row(P.rm, wrow0 + rr) * P.ldr + n0 + c * 8);
+                            *reinterpret_cast<uint4*>(buf_s + rr * 128 + ((c ^ (rr & 7)) << 4)) = v;
+                        }
+                        __syncwarp();
+                    } else if (leader) {
+                        mbar_arrive_expect_tx(&res_full[e], SLAB_BYTES);
+                        tma_load_2d(buf_s, &T.tr, &res_full[e], n0, wrow0);
+                    }
                 }
-                if (!ok) break;
-                emit();
+                if ((EPI & EPI_LN) && wrow0 + lane < M) row_fold(P.ln, wrow0 + lane, ln_a, ln_b);
+            }
+            ok = mbar_wait(&acc_full[buf], aph, abort_flag, status, STATUS_GEMM_EPILOGUE);
+            if (!ok) break;
+            tc_fence_after_sync();
+            if (!active) {
+                release_acc(buf);
                 continue;
             }
-            // ---- boundary tile / row-remapped / fp32 output: store straight from registers
-            const int m = m0 + row;
-            const bool row_ok = m < M;
-            const long long orow = map_out_row(P.rm, row_ok ? m : m0);
-            const long long rrow = map_res_row(P.rm, row_ok ? m : m0);
-            OutT* __restrict__ y = static_cast<OutT*>(P.y);
-            const long long ldy = P.ldy, ldr = P.ldr;
-            // same column split as the staged path (16 columns of each 64-column slab per warp), so a
-            // row's statistics do not depend on which kind of tile it falls in
-#pragma unroll 1
-            for (int sl = 0; sl < NSLAB; ++sl) {
-                const int n0 = nt0 + sl * 64 + qsub * 16;
-                // what the columns need from global memory, requested before the accumulator is waited for (unless
-                // WAIT_FIRST): a small problem is a chain of latencies
-                float bb[16], ss[16];
-                uint4 rraw[2];
-                if (!WAIT_FIRST) {
+            if ((EPI & EPI_RES) && res_tma) {
+                ok = mbar_wait(&res_full[e], res_ph, abort_flag, status, STATUS_GEMM_EPILOGUE);
+                res_ph ^= 1;
+                if (!ok) break;
+            }
+            // A thread holds columns 8 c + 2 (lane % 4), + 1 of rows lane / 4 + 8 k: a bias or fold vector value serves four rows
+            // of eight lanes.  (With a whole row to a thread every value of those vectors is a load of the whole warp, and the
+            // sixteen warps' loads, four passes for 16 bytes each, took as long as the tile's MMAs.)
+            const uint32_t tacc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BN + sl * SLAB;
+            float fa[4], fb[4];
+            if (EPI & EPI_LN) {
 #pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4) {
-                        const bool in = n0 + 8 * (q4 >> 1) < N;
-                        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-                        const float4 b4 = (bias && in) ? __ldg(reinterpret_cast<const float4*>(bias + n0) + q4) : z;
-                        bb[4 * q4] = b4.x; bb[4 * q4 + 1] = b4.y; bb[4 * q4 + 2] = b4.z; bb[4 * q4 + 3] = b4.w;
-                        if (EPI & EPI_LN) {
-                            const float4 s4 = in ? __ldg(reinterpret_cast<const float4*>(ln.s + n0) + q4) : z;
-                            ss[4 * q4] = s4.x; ss[4 * q4 + 1] = s4.y; ss[4 * q4 + 2] = s4.z; ss[4 * q4 + 3] = s4.w;
-                        }
-                    }
-                    if (res) {
-#pragma unroll
-                        for (int j = 0; j < 2; ++j)
-                            if (n0 + 8 * j < N && row_ok) rraw[j] = *reinterpret_cast<const uint4*>(res + rrow * ldr + n0 + 8 * j);
-                    }
-                    if (sl == 0) {
-                        wait_acc();
-                        if (!ok) break;
-                    }
-                }
-                uint32_t r[16];
-                __syncwarp();                 // tcgen05.ld is warp-collective
-                tmem_ld_32x16(tacc + sl * 64 + qsub * 16, r);
-                tmem_ld_wait();
-                if (sl + 1 == NSLAB) {
-                    // every column of this warp's slice is in registers: release the accumulator
-                    tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) release_acc(buf);
-                }
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const int n = n0 + 8 * j;
-                    if (n >= N || !row_ok) continue;
-                    float v[8];
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[8 * j + i]);
-                    if (WAIT_FIRST) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) bb[8 * j + i] = 0.f;
-                        if (bias) {
-                            const float4 b0 = __ldg(reinterpret_cast<const float4*>(bias + n));
-                            const float4 b1 = __ldg(reinterpret_cast<const float4*>(bias + n) + 1);
-                            bb[8 * j] = b0.x; bb[8 * j + 1] = b0.y; bb[8 * j + 2] = b0.z; bb[8 * j + 3] = b0.w;
-                            bb[8 * j + 4] = b1.x; bb[8 * j + 5] = b1.y; bb[8 * j + 6] = b1.z; bb[8 * j + 7] = b1.w;
-                        }
-                    }
-                    if (EPI & EPI_LN) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) v[i] = fmaf(ln_a, v[i], fmaf(ln_b, ss[8 * j + i], bb[8 * j + i]));
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) v[i] += bb[8 * j + i];
-                    }
-                    if (EPI & EPI_GELU) gelu8(v);
-                    if (res) {
-                        Vec<bf16> rv;
-                        float rf[8];
-                        if (WAIT_FIRST) rv.load(res + rrow * ldr + n);
-                        else rv.raw = rraw[j];
-                        rv.to_float(rf);
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) v[i] += rf[i];
-                    }
-                    if (EPI & EPI_EMIT) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) { e1 += v[i]; e2 = fmaf(v[i], v[i], e2); }
-                    }
-                    OutVec<OutT>::store8(y + orow * ldy + n, v);
+                for (int k = 0; k < 4; ++k) {
+                    fa[k] = __shfl_sync(0xffffffffu, ln_a, (lane >> 2) + 8 * k);
+                    fb[k] = __shfl_sync(0xffffffffu, ln_b, (lane >> 2) + 8 * k);
                 }
             }
-            if (!ok) break;
-            if (row_ok) emit();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {                      // 16 rows at a time
+                uint32_t r[32];
+                __syncwarp();                                  // tcgen05.ld is warp-collective
+                tmem_ld_16x256b_x8(tacc + (static_cast<uint32_t>(16 * h) << 16), r);
+                tmem_ld_wait();
+                if (h == 1) release_acc(buf);                  // the warp's last columns are in registers
+                // 16-byte cells for four 8 x 8 matrices at a time: rows 16 h + 0..7 and + 8..15 of chunks c and c + 1
+                const int mrow = 16 * h + (lane & 15);
+                const uint32_t cells = smem_u32(buf_s) + (uint32_t)mrow * 128u, cx = (uint32_t)(mrow & 7);
+                if (h == 0 && !(EPI & EPI_RES) && !F32) {
+                    if (leader) bulk_wait_group_read0();       // the last item's store has read the buffer
+                    __syncwarp();
+                }
+                float p1[2][4], p2[2][4];                      // EPI_EMIT: sums and sums of squares, 16 columns each, of the two rows
+#pragma unroll
+                for (int c = 0; c < 8; c += 2) {
+                    const uint32_t cell = cells + (((uint32_t)(c + (lane >> 4)) ^ cx) << 4);
+                    uint32_t rv[4], o[4];
+                    if (EPI & EPI_RES) ldmatrix_x4(cell, rv);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {              // matrix i: chunk c + i / 2, rows + 8 * (i % 2)
+                        const int cc = c + (i >> 1), k = 2 * h + (i & 1);
+                        const float a0 = __uint_as_float(r[4 * cc + 2 * (i & 1)]), a1 = __uint_as_float(r[4 * cc + 2 * (i & 1) + 1]);
+                        float v0, v1;
+                        if (EPI & EPI_LN) {
+                            v0 = fmaf(fa[k], a0, fmaf(fb[k], s2[cc].x, b2[cc].x));
+                            v1 = fmaf(fa[k], a1, fmaf(fb[k], s2[cc].y, b2[cc].y));
+                        } else {
+                            v0 = a0 + b2[cc].x;
+                            v1 = a1 + b2[cc].y;
+                        }
+                        if (EPI & EPI_GELU) {
+                            const uint32_t g = gelu_pair_f16(v0, v1);
+                            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&g));
+                            v0 = f.x;
+                            v1 = f.y;
+                        }
+                        if (EPI & EPI_RES) {
+                            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&rv[i]));
+                            v0 += f.x;
+                            v1 += f.y;
+                        }
+                        if (EPI & EPI_EMIT) {
+                            const bool in = n0 + 8 * cc < N;
+                            const float z0 = in ? v0 : 0.f, z1 = in ? v1 : 0.f;
+                            const float q1 = z0 + z1, q2 = fmaf(z1, z1, __fmul_rn(z0, z0));
+                            if (i < 2) { p1[i][c >> 1] = q1; p2[i][c >> 1] = q2; }
+                            else { p1[i & 1][c >> 1] += q1; p2[i & 1][c >> 1] += q2; }
+                        }
+                        if (F32) {
+                            const int rr = wrow0 + (lane >> 2) + 8 * k;
+                            if (rr < M && n0 + 8 * cc < N)
+                                *reinterpret_cast<float2*>(static_cast<float*>(P.y) + map_out_row(P.rm, rr) * P.ldy + n0 + 8 * cc + 2 * (lane & 3)) =
+                                    make_float2(v0, v1);
+                        } else {
+                            const __nv_bfloat162 t = __floats2bfloat162_rn(v0, v1);
+                            o[i] = *reinterpret_cast<const uint32_t*>(&t);
+                        }
+                    }
+                    if (!F32) stmatrix_x4(cell, o);
+                }
+                if (EPI & EPI_EMIT) {
+                    // (16 + 16) + (16 + 16) columns of a lane, then the four lanes of a row: (0 + 1) + (2 + 3)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        float e1 = (p1[i][0] + p1[i][1]) + (p1[i][2] + p1[i][3]), e2 = (p2[i][0] + p2[i][1]) + (p2[i][2] + p2[i][3]);
+                        e1 += __shfl_xor_sync(0xffffffffu, e1, 1); e2 += __shfl_xor_sync(0xffffffffu, e2, 1);
+                        e1 += __shfl_xor_sync(0xffffffffu, e1, 2); e2 += __shfl_xor_sync(0xffffffffu, e2, 2);
+                        const int rr = wrow0 + 16 * h + 8 * i + (lane >> 2);
+                        if ((lane & 3) == 0 && rr < M) P.ln.emit[(size_t)rr * P.ln.slots + n0 / SLAB] = make_float2(e1, e2);
+                    }
+                }
+            }
+            if (F32) continue;
+            if (P.use_tma_store && wrow0 + 32 <= M) {
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (leader) {
+                    tma_store_2d(&T.ty, buf_s, n0, wrow0);
+                    bulk_commit_group();
+                }
+            } else {
+                // rows beyond M among the warp's, or mapped rows: eight lanes copy a row's 128 bytes
+                __syncwarp();
+                const int c = lane & 7;
+                bf16* y = static_cast<bf16*>(P.y) + n0 + c * 8;
+                const bool in = n0 + c * 8 < N;
+                const int rows = M - wrow0;
+                const long long ldy = P.ldy;
+                const bool mapped = P.rm.out_grp > 0;
+                bf16* yr = y + (wrow0 + (lane >> 3)) * ldy;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int rr = i * 4 + (lane >> 3);
+                    const uint4 v = lds_u4(smem_u32(buf_s) + rr * 128 + ((c ^ (rr & 7)) << 4));
+                    if (mapped) yr = y + map_out_row(P.rm, wrow0 + rr) * ldy;
+                    if (rr < rows && in) *reinterpret_cast<uint4*>(yr) = v;
+                    yr += 4 * ldy;
+                }
+                fence_proxy_async_smem();                      // (a TMA residual may be the buffer's next content)
+                __syncwarp();
+            }
         }
+        if (leader) bulk_wait_group0();               // every TMA store has landed before the CTA retires
+        __syncwarp();
     }
     if (*abort_flag) {
         // Unwinding after a wait gave up: give copies still in flight time to land before
@@ -703,10 +604,220 @@ linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
     tc_fence_before_sync();
     __syncthreads();
     if (CG == 2) cluster_sync_all();     // the partner no longer reads this CTA's operands or signals its barriers
-    if (warp == 1) {
+    if (warp == PRODUCERS) {
         if (CG == 2) tmem_dealloc_pair(tmem_base, S::TMEM_COLS);
         else tmem_dealloc(tmem_base, S::TMEM_COLS);
     }
+}
+
+// ------------------------------------------------------------------------------ small problems
+// The same products for problems of no more 128 x 64 tiles than SMs, where a launch is a chain of latencies: one tile per CTA,
+// which tile it is known before the wait for the kernel in front (the loads do not wait for the row count, only the stores
+// do), sixteen epilogue warps with 16 columns each that go straight between registers and global memory.  Same MMA steps and
+// sums in the same order as linear_tc_kernel: a row's bits do not depend on which of the two it comes from.
+struct SmallConf {
+    static constexpr int BN = 64, STAGES = 8, PRODUCERS = 3, FIRST_EPI = 4, EW = 16, THREADS = (FIRST_EPI + EW) * 32;
+    static constexpr int A_BYTES = TBM * TBK * 2, B_BYTES = BN * TBK * 2;
+    static constexpr int RING = STAGES * (A_BYTES + B_BYTES);
+    static constexpr int SUMS = TBM * 16 * 8;            // EPI_EMIT: (sum, sum of squares) of four columns of a row each
+    static constexpr int USED = RING + SUMS + 256;
+    static constexpr int TOTAL = USED + 1024;
+    static_assert(TOTAL <= SMEM_MAX, "shared memory budget");
+};
+struct SmallLaunch { CUtensorMap ta[2], tw[2]; TcScalars p[2]; int grid0; };     // n_tiles: 64-column tiles of a row
+
+template <int EPI, bool F32, int NPROB>
+__global__ void __launch_bounds__(SmallConf::THREADS, 1)
+linear_tc_small_kernel(const __grid_constant__ SmallLaunch L, int K, int* status) {
+    using S = SmallConf;
+    constexpr int STAGES = S::STAGES, PRODUCERS = S::PRODUCERS;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const uint32_t ring_a = smem_u32(base), ring_b = ring_a + STAGES * S::A_BYTES;
+    float2* sums = reinterpret_cast<float2*>(base + S::RING);
+    uint64_t* full = reinterpret_cast<uint64_t*>(base + S::RING + S::SUMS);
+    uint64_t* empty = full + STAGES;
+    uint64_t* acc_full = empty + STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const uint32_t full_a = smem_u32(full), empty_a = smem_u32(empty);
+
+    const int prob = (NPROB == 2 && (int)blockIdx.x >= L.grid0) ? 1 : 0;
+    const TcScalars& P = L.p[prob];
+    const uint32_t tile = blockIdx.x - (prob ? L.grid0 : 0);
+    const uint32_t mt = fast_div(tile, P.n_tiles);
+    const int m0 = (int)mt * TBM, ct0 = (int)(tile - mt * P.n_tiles.d) * S::BN;
+    const int nkb = K / TBK;
+
+    if (warp == 0 && elect_one()) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        mbar_init(acc_full, 1);
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (warp == 1 && elect_one()) { prefetch_tmap(&L.ta[prob]); prefetch_tmap(&L.tw[prob]); }
+    if (warp == PRODUCERS) { tmem_alloc(tmem_slot, 64); tmem_relinquish(); }
+    // an earlier launch gave up on a wait: this one does nothing
+    const bool void_launch = status && (*reinterpret_cast<volatile int*>(status) & STATUS_WAIT_MASK) != 0;
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+    pdl_begin();
+
+    if (void_launch) {
+    } else if (warp < PRODUCERS) {
+        if (elect_one()) {
+            for (int kb = warp; kb < nkb; kb += PRODUCERS) {
+                const int s = kb % STAGES;
+                if (kb >= STAGES && !mbar_wait_a(empty_a + 8 * s, ((kb / STAGES) & 1) ^ 1, abort_flag, status, STATUS_GEMM_PRODUCER)) break;
+                mbar_arrive_expect_tx_a(full_a + 8 * s, S::A_BYTES + S::B_BYTES);
+                tma_load_2d_a<1>(ring_a + s * S::A_BYTES, &L.ta[prob], full_a + 8 * s, kb * TBK, m0);
+                tma_load_2d_a<1>(ring_b + s * S::B_BYTES, &L.tw[prob], full_a + 8 * s, kb * TBK, ct0);
+            }
+        }
+        __syncwarp();
+    } else if (warp == PRODUCERS) {
+        if (elect_one()) {
+            const uint64_t adesc0 = smem_desc_sw128(ring_a), bdesc0 = smem_desc_sw128(ring_b);
+            const uint32_t idesc = idesc_bf16_f32(TBM, S::BN, 0, 0);
+            bool ok = true;
+            for (int kb = 0; kb < nkb; ++kb) {
+                const int s = kb % STAGES;
+                ok = mbar_wait_a(full_a + 8 * s, (kb / STAGES) & 1, abort_flag, status, STATUS_GEMM_MMA);
+                if (!ok) break;
+                tc_fence_after_sync();
+                const uint64_t adesc = adesc0 + (uint64_t)(s * (S::A_BYTES >> 4)), bdesc = bdesc0 + (uint64_t)(s * (S::B_BYTES >> 4));
+#pragma unroll
+                for (int k = 0; k < TBK / 16; ++k) umma_ss(tmem_base, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                if (kb + STAGES < nkb) umma_commit_a<1>(empty_a + 8 * s);
+            }
+            if (ok) umma_commit_a<1>(smem_u32(acc_full));
+        }
+        __syncwarp();
+    } else {
+        const int g = (warp - S::FIRST_EPI) >> 2;         // which 16 columns of the tile
+        const int row = (warp & 3) * 32 + lane;           // tile row = TMEM lane
+        const int m = m0 + row, n0 = ct0 + g * 16, N = P.N;
+        int M = P.m_max;
+        if (P.m_dev) M = min(max(*reinterpret_cast<const volatile int32_t*>(P.m_dev), 0), M);
+        // what the outputs need besides the accumulator travels while the operands are loaded and multiplied
+        const bool live = m0 + (warp & 3) * 32 < M;       // the warp has rows
+        const bool row_ok = m < M;
+        const bool c0 = n0 < N, c1 = n0 + 8 < N;          // its columns exist, eight at a time
+        float add[16], sv[16], ln_a = 1.f;
+        uint4 rv[2];
+        if (live && c0) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int nb = min(n0 + 8 * (q >> 1), N - 8);
+                const float* bias = P.bias ? P.bias + nb : g_no_bias;
+                const float4 b4 = __ldg(reinterpret_cast<const float4*>(bias) + (q & 1));
+                add[4 * q] = b4.x; add[4 * q + 1] = b4.y; add[4 * q + 2] = b4.z; add[4 * q + 3] = b4.w;
+                if (EPI & EPI_LN) {
+                    const float4 s4 = __ldg(reinterpret_cast<const float4*>(P.ln.s + nb) + (q & 1));
+                    sv[4 * q] = s4.x; sv[4 * q + 1] = s4.y; sv[4 * q + 2] = s4.z; sv[4 * q + 3] = s4.w;
+                }
+            }
+            if ((EPI & EPI_RES) && row_ok) {
+                const bf16* r = P.res + map_res_row(P.rm, m) * P.ldr + n0;
+                rv[0] = *reinterpret_cast<const uint4*>(r);
+                rv[1] = c1 ? *reinterpret_cast<const uint4*>(r + 8) : make_uint4(0, 0, 0, 0);
+            }
+            if (EPI & EPI_LN) {
+                float ln_b = 0.f;
+                if (row_ok) row_fold(P.ln, m, ln_a, ln_b);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) add[i] = fmaf(ln_b, sv[i], add[i]);
+            }
+        }
+        const long long orow = map_out_row(P.rm, row_ok ? m : m0);
+        const bool ok = mbar_wait(acc_full, 0, abort_flag, status, STATUS_GEMM_EPILOGUE);
+        if (ok && live) {
+            tc_fence_after_sync();
+            uint32_t r[16];
+            float e1[4] = {0.f, 0.f, 0.f, 0.f}, e2[4] = {0.f, 0.f, 0.f, 0.f};
+            __syncwarp();
+            tmem_ld_32x16(tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + g * 16, r);
+            tmem_ld_wait();
+            if (c0) {
+                uint4 out[2];
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    float v[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float acc = __uint_as_float(r[8 * c + i]);
+                        v[i] = (EPI & EPI_LN) ? fmaf(ln_a, acc, add[8 * c + i]) : acc + add[8 * c + i];
+                    }
+                    if (EPI & EPI_GELU) gelu8(v);
+                    if (EPI & EPI_RES) {
+                        Vec<bf16> w;
+                        float rf[8];
+                        w.raw = rv[c];
+                        w.to_float(rf);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) v[i] += rf[i];
+                    }
+                    if (EPI & EPI_EMIT) {
+                        // as in linear_tc_kernel: columns 2 q, 2 q + 1 of the first and of the second eight
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const float z0 = (c == 0 || c1) ? v[2 * q] : 0.f, z1 = (c == 0 || c1) ? v[2 * q + 1] : 0.f;
+                            const float q1 = z0 + z1, q2 = fmaf(z1, z1, __fmul_rn(z0, z0));
+                            if (c == 0) { e1[q] = q1; e2[q] = q2; }
+                            else { e1[q] += q1; e2[q] += q2; }
+                        }
+                    }
+                    if (F32) {
+                        if (row_ok && (c == 0 || c1)) {
+                            float* y = static_cast<float*>(P.y) + orow * P.ldy + n0 + 8 * c;
+                            reinterpret_cast<float4*>(y)[0] = make_float4(v[0], v[1], v[2], v[3]);
+                            reinterpret_cast<float4*>(y)[1] = make_float4(v[4], v[5], v[6], v[7]);
+                        }
+                    } else {
+                        Vec<bf16> ov;
+                        ov.from_float(v);
+                        out[c] = ov.raw;
+                    }
+                }
+                if (!F32 && row_ok) {
+                    bf16* y = static_cast<bf16*>(P.y) + orow * P.ldy + n0;
+                    *reinterpret_cast<uint4*>(y) = out[0];
+                    if (c1) *reinterpret_cast<uint4*>(y + 8) = out[1];
+                }
+            }
+            if (EPI & EPI_EMIT) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) sums[(g * 4 + q) * TBM + row] = make_float2(e1[q], e2[q]);
+            }
+        }
+        if ((EPI & EPI_EMIT) && live) {
+            // the four warps of these rows (all of them get here): a column pair's 16 columns of each, (0 + 1) + (2 + 3), then the
+            // pairs, (0 + 1) + (2 + 3)
+            named_barrier(1 + (warp & 3), 128);
+            if (g == 0 && row_ok && ok) {
+                float t1[4], t2[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float2 a = sums[(0 * 4 + q) * TBM + row], b = sums[(1 * 4 + q) * TBM + row];
+                    const float2 c = sums[(2 * 4 + q) * TBM + row], d = sums[(3 * 4 + q) * TBM + row];
+                    t1[q] = (a.x + b.x) + (c.x + d.x);
+                    t2[q] = (a.y + b.y) + (c.y + d.y);
+                }
+                P.ln.emit[(size_t)m * P.ln.slots + ct0 / SLAB] = make_float2((t1[0] + t1[1]) + (t1[2] + t1[3]), (t2[0] + t2[1]) + (t2[2] + t2[3]));
+            }
+        }
+    }
+    if (*abort_flag) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000) { }          // let copies in flight land before releasing memory
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == PRODUCERS) tmem_dealloc(tmem_base, 64);
 }
 
 // ------------------------------------------------------------------------------ host
@@ -784,97 +895,126 @@ static int pick_bn(int N) {
     return bn;
 }
 
-int linear_stat_slots(int N) { return ceil_div(N, pick_bn(N)) * 4; }
+int linear_stat_slots(int N) { return (int)round_up(ceil_div(N, SLAB), 2); }
 
-template <int BN, typename OutT>
-static int fill_problem(TcProblem& q, const LinearArgs& p) {
-    {
-        const unsigned long long dims[2] = {(unsigned long long)p.K, (unsigned long long)p.m_max};
-        const unsigned long long strides[1] = {(unsigned long long)p.lda * 2ull};
-        const unsigned box[2] = {TBK, TBM};
-        if (int rc = make_tmap_bf16(&q.ta, p.a, 2, dims, strides, box)) return rc;
-    }
-    {
-        // W boxes: a whole tile, and the column strips of split tail tiles / narrow last tiles (half, or a
-        // third for BN = 192, and a quarter)
-        const unsigned long long dims[2] = {(unsigned long long)p.K, (unsigned long long)p.N};
-        const unsigned long long strides[1] = {(unsigned long long)p.K * 2ull};
-        // (each CTA of a group loads its share of the rows: box heights divide by CG)
-        const unsigned box[2] = {TBK, BN / CG};
-        if (int rc = make_tmap_bf16(&q.tw, p.w, 2, dims, strides, box)) return rc;
-        const unsigned box2[2] = {TBK, (BN == 256 ? 128u : 64u) / CG};
-        if (int rc = make_tmap_bf16(&q.tw2, p.w, 2, dims, strides, box2)) return rc;
-        const unsigned box3[2] = {TBK, 64u / CG};
-        if (int rc = make_tmap_bf16(&q.tw3, p.w, 2, dims, strides, box3)) return rc;
-    }
-    // Output map for the TMA-store epilogue (bf16 output, rows not remapped).
-    q.use_tma_store = (sizeof(OutT) == 2 && p.out_grp == 0) ? 1 : 0;
-    q.ty = q.tw;
-    q.tr = q.tw;
-    if (q.use_tma_store) {
-        const unsigned long long dims[2] = {(unsigned long long)p.N, (unsigned long long)p.m_max};
-        const unsigned long long strides[1] = {(unsigned long long)p.ldy * 2ull};
-        const unsigned box[2] = {64, TBM};
-        if (int rc = make_tmap_bf16(&q.ty, p.y, 2, dims, strides, box)) return rc;
-        if (p.res) {
-            const unsigned long long rstrides[1] = {(unsigned long long)p.ldr * 2ull};
-            if (int rc = make_tmap_bf16(&q.tr, p.res, 2, dims, rstrides, box)) return rc;
-        }
-    }
+static FastDiv make_fast_div(uint32_t d) {
+    return FastDiv{d, d == 1 ? 0u : (uint32_t)(((1ull << 32) + d - 1) / d)};
+}
+
+static void fill_scalars(TcScalars& q, const LinearArgs& p, bool f32, int bn) {
     q.bias = p.bias; q.res = (const bf16*)p.res; q.ldr = p.ldr; q.y = p.y; q.ldy = p.ldy;
     q.m_max = p.m_max; q.m_dev = p.m_dev; q.N = p.N;
+    q.n_tiles = make_fast_div((uint32_t)ceil_div(p.N, bn));
+    q.use_tma_store = (!f32 && p.out_grp == 0) ? 1 : 0;
     q.rm = RowMap{p.out_grp, p.out_skip, p.res_mod, p.res_off};
     q.ln = LnFold{p.ln_stats, p.ln_s, p.ln_mode, p.ln_dim, p.ln_eps, p.emit_stats,
-                  p.emit_stats ? linear_stat_slots(p.N) : p.ln_slots};
+                  p.emit_stats ? linear_stat_slots(p.N) : p.ln_slots, ceil_div(p.ln_dim, SLAB)};
+}
+
+// A [m_max, K] in boxes of one k-block of a CTA's rows; W [N, K] in boxes of `rows` rows.
+static int operand_maps(CUtensorMap* ta, CUtensorMap* tw, const LinearArgs& p, unsigned rows) {
+    const unsigned long long da[2] = {(unsigned long long)p.K, (unsigned long long)p.m_max};
+    const unsigned long long sa[1] = {(unsigned long long)p.lda * 2ull};
+    const unsigned ba[2] = {TBK, TBM};
+    if (ta) if (int rc = make_tmap_bf16(ta, p.a, 2, da, sa, ba)) return rc;
+    const unsigned long long dw[2] = {(unsigned long long)p.K, (unsigned long long)p.N};
+    const unsigned long long sw[1] = {(unsigned long long)p.K * 2ull};
+    const unsigned bw[2] = {TBK, rows};
+    return make_tmap_bf16(tw, p.w, 2, dw, sw, bw);
+}
+
+template <int BN, int CG>
+static int fill_problem(TcMaps& t, TcScalars& q, const LinearArgs& p, bool f32) {
+    fill_scalars(q, p, f32, BN);
+    // W boxes: a whole tile, and 64 columns of a strip or a narrow last tile (each CTA of a group loads its share)
+    if (int rc = operand_maps(&t.ta, &t.tw, p, BN / CG)) return rc;
+    if (int rc = operand_maps(nullptr, &t.tws, p, SLAB / CG)) return rc;
+    // Output and residual maps: 32 rows of a slab (bf16 output, rows not remapped).
+    t.ty = t.tw;
+    t.tr = t.tw;
+    const unsigned box[2] = {SLAB, 32};
+    const unsigned long long dims[2] = {(unsigned long long)p.N, (unsigned long long)p.m_max};
+    if (q.use_tma_store) {
+        const unsigned long long strides[1] = {(unsigned long long)p.ldy * 2ull};
+        if (int rc = make_tmap_bf16(&t.ty, p.y, 2, dims, strides, box)) return rc;
+    }
+    if (p.res && p.res_mod <= 0) {
+        const unsigned long long strides[1] = {(unsigned long long)p.ldr * 2ull};
+        if (int rc = make_tmap_bf16(&t.tr, p.res, 2, dims, strides, box)) return rc;
+    }
     return VTP_OK;
 }
 
-// p1 = null: one problem.  Otherwise two problems of the same K and epilogue kind in one launch.
-template <int BN, int STAGES, typename OutT, int EPI>
-static int launch_tc(const LinearArgs& p, const LinearArgs* p1, cudaStream_t st) {
-    using S = TcSmem<BN, STAGES>;
-    TcLaunch L;
-    L.n = p1 ? 2 : 1;
-    if (int rc = fill_problem<BN, OutT>(L.p[0], p)) return rc;
-    if (p1) {
-        if (int rc = fill_problem<BN, OutT>(L.p[1], *p1)) return rc;
-    } else {
-        L.p[1] = L.p[0];
-    }
-    if (p1 && !(BN == 256 && EPI == EPI_LN && sizeof(OutT) == 2))
-        return fail(VTP_ERR_UNSUPPORTED, "linear (tcgen05): two-problem launches are built for 256-wide LayerNorm-fold tiles");
-    auto kern = (p1 && BN == 256 && EPI == EPI_LN && sizeof(OutT) == 2) ? linear_tc_kernel<BN, STAGES, OutT, EPI, (BN == 256 && EPI == EPI_LN && sizeof(OutT) == 2) ? 2 : 1>
-                                                                       : linear_tc_kernel<BN, STAGES, OutT, EPI, 1>;
-    static bool attr_set[64][2] = {};   // per instantiation, device and problem count
+// Reserves the dynamic shared memory of a kernel once per device.
+template <typename Kernel>
+static int reserve_smem(Kernel kern, int bytes, bool (&done)[64]) {
     int dev = 0;
     cudaGetDevice(&dev);
-    const int np = p1 ? 1 : 0;
-    if (dev < 0 || dev >= 64 || !attr_set[dev][np]) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
-        if (e != cudaSuccess) {
-            set_error("linear (tcgen05): cannot reserve %d bytes of shared memory: %s", S::TOTAL,
-                      cudaGetErrorString(e));
-            return (int)e;
-        }
-        if (dev >= 0 && dev < 64) attr_set[dev][np] = true;
+    if (dev >= 0 && dev < 64 && done[dev]) return VTP_OK;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) {
+        set_error("linear (tcgen05): cannot reserve %d bytes of shared memory: %s", bytes, cudaGetErrorString(e));
+        return (int)e;
     }
-    long long tiles = (long long)ceil_div(p.N, BN) * ceil_div(p.m_max, TM);
-    if (p1) tiles += (long long)ceil_div(p1->N, BN) * ceil_div(p1->m_max, TM);
-    const int groups = sm_count() / CG;
-    // Few tiles start early (launch_kernel): then most SMs are free and the set-up overlaps the kernel in front.
-    // With every SM taken there is nothing to overlap, and a chain of early launches measured slower (DeiT-S,
-    // batch 256, graph: 3.78 ms without, 3.98 ms with).
-    const bool early = tiles <= groups;
-    // few tiles are cut into column strips, one per CTA (see the kernel): launch a CTA for each of those
-    if (!(EPI & EPI_EMIT)) tiles *= BN / 64;
-    const int grid = CG * (int)(tiles < groups ? tiles : groups);
-    const cudaError_t le = launch_kernel(kern, early, CG, dim3(grid), dim3(TC_THREADS), (size_t)S::TOTAL, st, L, p.K, device_status_ptr());
-    if (le != cudaSuccess) {
+    if (dev >= 0 && dev < 64) done[dev] = true;
+    return VTP_OK;
+}
+
+static int launched(cudaError_t e) {
+    if (e != cudaSuccess) {
         cudaGetLastError();
-        set_error("linear (tcgen05): %s", cudaGetErrorString(le));
-        return (int)le;
+        set_error("linear (tcgen05): %s", cudaGetErrorString(e));
+        return (int)e;
     }
     return check_launch("linear (tcgen05)");
+}
+
+// p1 = null: one problem.  Otherwise two problems of the same K and epilogue kind in one launch.
+template <int BN, int CG, int EPI, bool F32, int NPROB>
+static int launch_tc(const LinearArgs& p, const LinearArgs* p1, cudaStream_t st) {
+    using S = TcConf<BN, CG>;
+    TcLaunch L;
+    if (int rc = fill_problem<BN, CG>(L.m[0], L.s.p[0], p, F32)) return rc;
+    if (NPROB == 2) {
+        if (int rc = fill_problem<BN, CG>(L.m[1], L.s.p[1], *p1, F32)) return rc;
+    } else {
+        L.m[1] = L.m[0];
+        L.s.p[1] = L.s.p[0];
+    }
+    auto kern = linear_tc_kernel<BN, CG, EPI, F32, NPROB>;
+    static bool reserved[64] = {};   // per instantiation and device
+    if (int rc = reserve_smem(kern, S::TOTAL, reserved)) return rc;
+    long long tiles = (long long)ceil_div(p.N, BN) * ceil_div(p.m_max, TBM * CG);
+    if (NPROB == 2) tiles += (long long)ceil_div(p1->N, BN) * ceil_div(p1->m_max, TBM * CG);
+    const int groups = sm_count() / CG;
+    // few tiles are cut into column strips, one per CTA group (see Schedule): launch a group for each of those
+    tiles *= BN / SLAB;
+    const int used = (int)(tiles < groups ? tiles : groups);
+    L.s.groups = make_fast_div((uint32_t)used);
+    // Every launch starts early (launch_kernel): a CTA takes an SM by itself and sets itself up while the kernel in front ends
+    // (DeiT-S, 256 images: 3.35 -> 3.31 ms; DeiT-B, 33 images: 1.55 -> 1.47; PVT-small, 96 images: 2.78 -> 2.69).
+    return launched(launch_kernel(kern, true, CG, dim3(CG * used), dim3(S::THREADS), (size_t)S::TOTAL, st, L, p.K, device_status_ptr()));
+}
+
+// 128 x 64 tiles of a problem.  As many as SMs at most run as linear_tc_small_kernel: all at once, one per SM.  (DeiT-Ti, one
+// image: 505 us per forward with the persistent kernel alone, 395 with both; DeiT-S, 7 images: 662 and 586.)
+static long long small_tiles(const LinearArgs& p) { return (long long)ceil_div(p.m_max, TBM) * ceil_div(p.N, SmallConf::BN); }
+
+template <int EPI, bool F32, int NPROB>
+static int launch_small(const LinearArgs& p, const LinearArgs* p1, cudaStream_t st) {
+    SmallLaunch L;
+    for (int i = 0; i < 2; ++i) {
+        const LinearArgs& q = (NPROB == 2 && i) ? *p1 : p;
+        if (int rc = operand_maps(&L.ta[i], &L.tw[i], q, SmallConf::BN)) return rc;
+        fill_scalars(L.p[i], q, F32, SmallConf::BN);
+    }
+    L.grid0 = (int)small_tiles(p);
+    const int grid = L.grid0 + (NPROB == 2 ? (int)small_tiles(*p1) : 0);
+    auto kern = linear_tc_small_kernel<EPI, F32, NPROB>;
+    static bool reserved[64] = {};   // per instantiation and device
+    if (int rc = reserve_smem(kern, SmallConf::TOTAL, reserved)) return rc;
+    return launched(launch_kernel(kern, true, 1, dim3(grid), dim3(SmallConf::THREADS), (size_t)SmallConf::TOTAL, st, L, p.K,
+                                  device_status_ptr()));
 }
 
 static int check_tc_args(const LinearArgs& p) {
@@ -882,7 +1022,7 @@ static int check_tc_args(const LinearArgs& p) {
     VTP_REQUIRE(p.K % TBK == 0, VTP_ERR_SHAPE, "linear (tcgen05): K=%d must be a multiple of %d", p.K, TBK);
     VTP_REQUIRE(p.N % 8 == 0, VTP_ERR_SHAPE, "linear (tcgen05): N=%d must be a multiple of 8", p.N);
     VTP_REQUIRE(p.ln_mode == 0 || (p.ln_stats && p.ln_s && p.out_grp == 0 &&
-                                   (p.ln_mode == 1 || (p.ln_dim > 0 && p.ln_slots > 0 && p.ln_slots % 2 == 0))),
+                                   (p.ln_mode == 1 || (p.ln_dim > 0 && p.ln_slots >= ceil_div(p.ln_dim, SLAB) && p.ln_slots % 2 == 0))),
                 VTP_ERR_NULL, "linear (tcgen05): folded LayerNorm needs row statistics and the column sums");
     VTP_REQUIRE(p.ln_mode == 0 || !p.res, VTP_ERR_UNSUPPORTED, "linear (tcgen05): a folded LayerNorm takes no residual");
     VTP_REQUIRE(p.lda % 8 == 0 && p.ldy % 8 == 0 && (!p.res || p.ldr % 8 == 0), VTP_ERR_ALIGN,
@@ -891,18 +1031,22 @@ static int check_tc_args(const LinearArgs& p) {
 }
 
 // Two independent Linears that follow the same kind of LayerNorm fold (the q and kv projections of a block)
-// in ONE launch of 128 x 256 tiles: the tiles of the second problem fill the last, partial round of the first,
+// in ONE launch of 256-wide tiles: the tiles of the second problem fill the last, partial round of the first,
 // and one launch's ramp and tail is saved.  Both: bf16 output, bias + folded LayerNorm (ln_mode 1), no
 // residual, no row remap; N a multiple of 64.
 bool linear_pair_supported(const LinearArgs& a, const LinearArgs& b) {
     auto ok = [](const LinearArgs& p) {
-        // whole 64-column slabs: a last tile of 64 or 128 columns is a narrow tile, one of 192 a full tile whose
-        // W rows beyond N the TMA load fills with zeros and whose last slab the TMA store drops
         return p.dtype == VTP_BF16 && p.ln_mode == 1 && !p.res && !p.emit_stats && p.out_grp == 0 && p.flags == 0 &&
                p.m_max > 0 && p.N >= 64 && p.N % 64 == 0;
     };
     return ok(a) && ok(b) && a.K == b.K;
 }
+
+// Whether two CTAs should share 256-row tiles (cta_group::2).  Each then loads and multiplies half of the tile's W rows, which
+// pays once a tile has several k-blocks: 65792 x 768 with K = 384 48.1 -> 41.2 us, 23040 x 384 with K = 1536 37.1 -> 30.8.  With
+// K = 64 or 128, or tiles of 128 columns, the pair's longer set-up costs more than that: 393216 x 64 with K = 64 19.5 -> 21.7,
+// 172000 x 64 with K = 512 37.6 -> 39.6, 172000 x 512 with K = 64 42.5 -> 43.9.
+static bool pairs_pay(int bn, int K) { return bn >= 192 && K >= 256; }
 
 int linear_tcgen05_pair(const LinearArgs& a, const LinearArgs& b, cudaStream_t st) {
     if (int rc = linear_validate(a)) return rc;
@@ -910,34 +1054,45 @@ int linear_tcgen05_pair(const LinearArgs& a, const LinearArgs& b, cudaStream_t s
     if (int rc = check_tc_args(a)) return rc;
     if (int rc = check_tc_args(b)) return rc;
     VTP_REQUIRE(linear_pair_supported(a, b), VTP_ERR_UNSUPPORTED, "linear (tcgen05): these two problems cannot share a launch");
-    return launch_tc<256, ring_stages(256), bf16, EPI_LN>(a, &b, st);
+    if (small_tiles(a) + small_tiles(b) <= sm_count()) return launch_small<EPI_LN, false, 2>(a, &b, st);
+    if (pairs_pay(256, a.K)) return launch_tc<256, 2, EPI_LN, false, 2>(a, &b, st);
+    return launch_tc<256, 1, EPI_LN, false, 2>(a, &b, st);
 }
 
 int linear_tcgen05(const LinearArgs& p, cudaStream_t st) {
     if (p.m_max == 0) return VTP_OK;
     if (int rc = check_tc_args(p)) return rc;
     const int bn = pick_bn(p.N);
+    const bool pairs = pairs_pay(bn, p.K);
+    const bool small = small_tiles(p) <= sm_count();
     const bool f32 = (p.flags & VTP_FLAG_OUT_F32) != 0;
-    const int epi = ((p.flags & VTP_FLAG_GELU) ? EPI_GELU : 0) | (p.ln_mode ? EPI_LN : 0) | (p.emit_stats ? EPI_EMIT : 0);
+    const int epi = ((p.flags & VTP_FLAG_GELU) ? EPI_GELU : 0) | (p.ln_mode ? EPI_LN : 0) | (p.emit_stats ? EPI_EMIT : 0) |
+                    (p.res ? EPI_RES : 0);
+    // rare kinds in one tile width (a row's bits do not depend on it)
     if (f32) {
-        VTP_REQUIRE(epi == 0, VTP_ERR_UNSUPPORTED, "linear (tcgen05): fp32 output supports bias and residual only");
-        if (bn == 256) return launch_tc<256, ring_stages(256), float, 0>(p, nullptr, st);
-        if (bn == 192) return launch_tc<192, ring_stages(192), float, 0>(p, nullptr, st);
-        return launch_tc<128, ring_stages(128), float, 0>(p, nullptr, st);
+        if (small && epi == 0) return launch_small<0, true, 1>(p, nullptr, st);
+        if (small && epi == EPI_RES) return launch_small<EPI_RES, true, 1>(p, nullptr, st);
+        if (epi == 0) return launch_tc<128, 1, 0, true, 1>(p, nullptr, st);
+        if (epi == EPI_RES) return launch_tc<128, 1, EPI_RES, true, 1>(p, nullptr, st);
+        return fail(VTP_ERR_UNSUPPORTED, "linear (tcgen05): fp32 output supports bias and residual only");
     }
-    const bool shallow = CG == 1 && bn == 128 && (p.K <= TBK || (p.K <= 2 * TBK && p.res));
-#define VTP_TC_CASE(E)                                                  \
-    if (epi == (E)) {                                                   \
-        if (shallow) return launch_tc<128, SHALLOW_RING, bf16, (E)>(p, nullptr, st);            \
-        if (bn == 256) return launch_tc<256, ring_stages(256), bf16, (E)>(p, nullptr, st);      \
-        if (bn == 192) return launch_tc<192, ring_stages(192), bf16, (E)>(p, nullptr, st);      \
-        return launch_tc<128, ring_stages(128), bf16, (E)>(p, nullptr, st);                     \
+    if (small && epi == (EPI_GELU | EPI_RES)) return launch_small<EPI_GELU | EPI_RES, false, 1>(p, nullptr, st);
+    if (epi == (EPI_GELU | EPI_RES)) return launch_tc<128, 1, EPI_GELU | EPI_RES, false, 1>(p, nullptr, st);
+#define VTP_TC_CASE(E)                                                                   \
+    if (epi == (E)) {                                                                    \
+        if (small) return launch_small<(E), false, 1>(p, nullptr, st);                   \
+        if (pairs && bn == 256) return launch_tc<256, 2, (E), false, 1>(p, nullptr, st); \
+        if (pairs && bn == 192) return launch_tc<192, 2, (E), false, 1>(p, nullptr, st); \
+        if (bn == 256) return launch_tc<256, 1, (E), false, 1>(p, nullptr, st);          \
+        if (bn == 192) return launch_tc<192, 1, (E), false, 1>(p, nullptr, st);          \
+        return launch_tc<128, 1, (E), false, 1>(p, nullptr, st);                         \
     }
     VTP_TC_CASE(0)
     VTP_TC_CASE(EPI_GELU)
+    VTP_TC_CASE(EPI_RES)
     VTP_TC_CASE(EPI_LN)
     VTP_TC_CASE(EPI_LN | EPI_GELU)
-    VTP_TC_CASE(EPI_EMIT)
+    VTP_TC_CASE(EPI_EMIT | EPI_RES)
 #undef VTP_TC_CASE
     return fail(VTP_ERR_UNSUPPORTED, "linear (tcgen05): epilogue combination %d is not instantiated", epi);
 }

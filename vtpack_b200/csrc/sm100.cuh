@@ -31,23 +31,26 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// One try: the thread may be SUSPENDED by the hardware for up to `kSuspendHintNs` while the phase is
-// incomplete and is woken when it completes.  Without the hint a waiting thread comes back at once and
-// a polling loop fills the issue slots of its SM sub-partition, at the expense of the warps that work.
-#ifndef VTP_SUSPEND_HINT_NS
-#define VTP_SUSPEND_HINT_NS 20000
-#endif
-constexpr uint32_t kSuspendHintNs = VTP_SUSPEND_HINT_NS;
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
+// One try; the hardware may park the thread for a while of its own choosing.  (With a suspend-time hint a try costs 77 cycles
+// instead of 42 even when the phase has completed.)
+__device__ __forceinline__ bool mbar_try_wait_a(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(kSuspendHintNs)
+        : "r"(bar), "r"(parity)
         : "memory");
     return ok != 0;
+}
+
+// True in one lane of a converged warp.  Unlike with `lane == 0` the compiler then knows that one thread runs what
+// follows: a TMA load issues in about 10 cycles behind another one instead of 65, a tcgen05.commit in 45 fewer.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
 }
 
 // About one second at 2 GHz.  A wait that runs this long means a copy or MMA that will
@@ -55,14 +58,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // so that the kernel can unwind instead of hanging the GPU.
 constexpr long long kWaitLimitCycles = 2000000000LL;
 
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                          int* status, int code) {
-    if (mbar_try_wait(bar, parity)) return true;
+// The tries come in runs without anything else between them: a thread that feeds the tensor core waits here for most of
+// its k-blocks, and reading the clock on the way in costs it the phase it would have seen.
+__device__ __forceinline__ bool mbar_wait_a(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+#pragma unroll 1
+    for (int i = 0; i < 1024; ++i)
+        if (mbar_try_wait_a(bar, parity)) return true;
     const long long t0 = clock64();
     for (;;) {
 #pragma unroll 1
-        for (int i = 0; i < 32; ++i)
-            if (mbar_try_wait(bar, parity)) return true;
+        for (int i = 0; i < 1024; ++i)
+            if (mbar_try_wait_a(bar, parity)) return true;
         if (*abort_flag) return false;
         if (clock64() - t0 > kWaitLimitCycles) {
             *abort_flag = 1;
@@ -70,6 +76,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
             return false;
         }
     }
+}
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+    return mbar_wait_a(smem_u32(bar), parity, abort_flag, status, code);
 }
 
 // Shared-memory accesses by 32-bit shared-space address (a generic pointer costs 64-bit address arithmetic
@@ -108,6 +117,24 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* m, uin
         : "memory");
 }
 
+// The forms by shared-space address; for a pair of CTAs (cta_group 2) `bar` is a barrier of the rank-0 CTA.
+__device__ __forceinline__ void mbar_arrive_expect_tx_a(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+template <int CTA_GROUP>
+__device__ __forceinline__ void tma_load_2d_a(uint32_t dst, const CUtensorMap* m, uint32_t bar, int x, int y) {
+    if (CTA_GROUP == 1)
+        asm volatile(
+            "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+            ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(y)
+            : "memory");
+    else
+        asm volatile(
+            "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+            ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(y)
+            : "memory");
+}
+
 // Tile store shared (this CTA) -> global, tracked by the bulk async-group of the issuing thread.
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* src, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
@@ -117,9 +144,6 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* s
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // Waits until the shared-memory source of every committed bulk group has been read.
 __device__ __forceinline__ void bulk_wait_group_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// ... of every committed bulk group but the newest N.
-template <int N>
-__device__ __forceinline__ void bulk_wait_group_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 // Waits until every committed bulk group has completed.
 __device__ __forceinline__ void bulk_wait_group0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // Barrier among `count` threads (a multiple of 32) on hardware barrier `id` (1..15).
@@ -231,10 +255,10 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
         uint32_t ok;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
             "selp.u32 %0, 1, 0, p;\n\t}"
             : "=r"(ok)
-            : "r"(smem_u32(bar)), "r"(parity), "r"(kSuspendHintNs)
+            : "r"(smem_u32(bar)), "r"(parity)
             : "memory");
         if (ok) return true;
         if (*abort_flag) return false;
@@ -244,14 +268,6 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
             return false;
         }
     }
-}
-// Tile load into THIS CTA's shared memory whose bytes are counted on an mbarrier of the pair's
-// rank-0 CTA (`leader_bar`, a shared::cluster address).
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m, uint32_t leader_bar, int x, int y) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(leader_bar), "r"(x), "r"(y)
-        : "memory");
 }
 // TMEM allocation for the pair: the same warp of BOTH CTAs executes it with the same arguments.
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* dst_smem, uint32_t ncols) {
@@ -276,13 +292,15 @@ __device__ __forceinline__ void umma_ss_pair(uint32_t tmem_d, uint64_t adesc, ui
         ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// Arrives on the mbarrier at `bar`'s offset in BOTH CTAs once every pair MMA issued so far by this
-// thread has completed: one commit per CTA, the partner's barrier addressed through the cluster window.
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
-    const uint32_t own = smem_u32(bar);
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(own) : "memory");
-    const uint32_t other = mapa_u32(own, cluster_ctarank() ^ 1u);
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(other) : "memory");
+// umma_commit by shared-space address; for a pair it arrives on the barrier of that offset in both CTAs.
+template <int CTA_GROUP>
+__device__ __forceinline__ void umma_commit_a(uint32_t bar) {
+    if (CTA_GROUP == 1)
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                     ::"r"(bar), "h"(static_cast<unsigned short>(3))
+                     : "memory");
 }
 
 // ------------------------------------------------------------------ TMEM -> registers
@@ -309,6 +327,30 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
         : "r"(taddr)
         : "memory");
 }
+// 16 lanes x 64 columns: register 4 c + 2 i + j of thread t holds lane t / 4 + 8 i, column 8 c + 2 (t % 4) + j (the accumulator
+// layout of the warp-level matrix instructions, so ldmatrix / stmatrix match it).
+__device__ __forceinline__ void tmem_ld_16x256b_x8(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
+}
+// Four 8 x 8 matrices of 16-bit elements between shared memory and that layout: thread t gives the address of row t % 8 of
+// matrix t / 8 and holds columns 2 (t % 4), + 1 of row t / 4 of matrix i in r[i].
+__device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void stmatrix_x4(uint32_t addr, const uint32_t (&r)[4]) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};"
+                 ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
+}
 // registers -> TMEM, 32 lanes x 16 consecutive 32-bit columns (thread i writes lane base + i).
 __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
@@ -316,12 +358,6 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r
         "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
           "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
