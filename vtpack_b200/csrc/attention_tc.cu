@@ -18,10 +18,16 @@
 //                      from 7 images on the gain is within the 1 % that two runs differ by)
 //   O  = O*alpha + O_c in registers of the softmax threads (online-softmax rescale), then the
 //                      tail keys, the 1/rowsum and the bf16 store.
-// Warp 0 lane 0 issues TMA (Q is double-buffered so the next item's Q and K stream in during
-// the current softmax), warp 1 lane 0 issues MMA, warps 2-5 do softmax and output.
+// Warp 0 issues TMA (Q is double-buffered so the next item's Q and K stream in during
+// the current softmax), warp 1 issues MMA, warps 2-5 do softmax and output.
 // q, k, v are read in place from the Linear outputs through strided tensor maps.
 // Every mbarrier wait is bounded (sm100.cuh).
+//
+// An item (128 queries, 257 keys) is a chain of scores, maximum, exp2, P V and output: 1400 + 1500 + 5300 + 1500 + 3000 cycles
+// (clock64) with two items on the SM, hardly less alone.  Two threads a row (eight softmax warps) measured 68 us where this
+// takes 59 (256 images x 6 heads) and 73 where it takes 56 (1025 keys).  What a chunk costs beside the sweeps: one arrival per warp
+// instead of one per thread, loads and MMAs from an elected thread, offsets kept in shared memory and scanned a run of images per
+// lane: DeiT-S at 512 px 1830 -> 1770 us, 256 images 3384 -> 3357, DeiT-Ti with one image 396 -> 392.
 //
 // Replaces batched_sparse_attention_forward
 // (vtpack/layers/csrc/batched_sparse_gemm/batched_sparse_gemm.cu:219-305: per image two
@@ -40,6 +46,8 @@ constexpr int KC_MAX = 256;        // keys per tensor-core chunk, upper bound
 constexpr int O_COL = 64;          // TMEM column of the P*V accumulator
 constexpr int P_SPLIT = 128;       // keys of a chunk's first part of P, in columns [0, 64); the rest of P from column 128 on
 constexpr int ATT_TMEM_COLS = 256;
+constexpr int SOFTMAX_WARPS = 4;
+constexpr int OFFSETS_KEPT = 512;  // images whose offsets are copied to shared memory beside the tile prefix
 
 constexpr int SM_Q = 0;                               // two Q buffers
 constexpr int SM_K = SM_Q + 2 * QT * HD * 2;          // 32768
@@ -66,9 +74,8 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                  : "memory");
 }
 
-// item w -> (image, head, first packed row, valid rows); tile_prefix is in shared memory
-__device__ __forceinline__ AttnItem attn_item(int w, int heads, int B, const int* tile_prefix,
-                                              const int32_t* __restrict__ offsets) {
+// item w -> (image, head, first packed row, valid rows); tile_prefix is in shared memory, so are the offsets of a moderate batch
+__device__ __forceinline__ AttnItem attn_item(int w, int heads, int B, const int* tile_prefix, const int32_t* offsets) {
     const int tg = w / heads;
     int lo = 0, hi = B;                        // largest b with tile_prefix[b] <= tg
     while (hi - lo > 1) {
@@ -108,17 +115,21 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     int* tile_prefix = reinterpret_cast<int*>(base + SM_PREFIX);
+    int32_t* offs_s = tile_prefix + B + 1;
     AttnItem* items = reinterpret_cast<AttnItem*>(base + SM_ITEM);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
-    if (threadIdx.x == 32) {
-        for (int i = 0; i < 2; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_free[i], QT); }
+    // (a launch does nothing after one that gave up on a wait; the word travels beside the set-up)
+    int status_word = 0;
+    if (status) status_word = *reinterpret_cast<volatile int*>(status);
+    if (warp == 1 && elect_one()) {
+        for (int i = 0; i < 2; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_free[i], SOFTMAX_WARPS); }
         mbar_init(k_full, 1); mbar_init(k_free, 1);
         mbar_init(v_full, 1); mbar_init(v_free, 1);
-        mbar_init(s_full, 1); mbar_init(p_full, QT); mbar_init(p_half, QT);
-        mbar_init(o_full, 1); mbar_init(o_free, QT);
+        mbar_init(s_full, 1); mbar_init(p_full, SOFTMAX_WARPS); mbar_init(p_half, SOFTMAX_WARPS);
+        mbar_init(o_full, 1); mbar_init(o_free, SOFTMAX_WARPS);
         *abort_flag = 0;
         fence_barrier_init();
         prefetch_tmap(&tmap_q);
@@ -133,54 +144,62 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     // offsets, q, k and v below do.
     pdl_begin();
     // tile_prefix[b] = number of 128-query tiles of the images in front of b.  All threads fetch the
-    // per-image tile counts at once (one global-load latency), then warp 0 scans them in shared memory.
+    // per-image tile counts at once (one global-load latency), then warp 0 scans them in shared memory, a run of images per
+    // lane.
     // (the offsets come from the caller: a count outside [0, max_q] is clamped, so the item list
     // always fits the grid's bound, and rows at or beyond l_max are never stored below)
+    const bool keep = B <= OFFSETS_KEPT;
     for (int b = threadIdx.x; b < B; b += blockDim.x) {
-        int cnt = offsets[b + 1] - offsets[b];
+        const int o0 = offsets[b], o1 = offsets[b + 1];
+        int cnt = o1 - o0;
 #if VTP_INDEX_GUARDS
-        if (cnt < 0 || cnt > max_q || offsets[b] < 0 || offsets[b + 1] > l_max) {
+        if (cnt < 0 || cnt > max_q || o0 < 0 || o1 > l_max) {
             if (status && blockIdx.x == 0) atomicOr(status, STATUS_BAD_INDEX);
-            cnt = (offsets[b] < 0) ? 0 : min(max(cnt, 0), max_q);
+            cnt = (o0 < 0) ? 0 : min(max(cnt, 0), max_q);
         }
 #endif
         tile_prefix[b] = (cnt + QT - 1) / QT;
+        if (keep) {
+            offs_s[b] = o0;
+            if (b + 1 == B) offs_s[B] = o1;
+        }
     }
     __syncthreads();
     if (warp == 0) {
-        int run = 0;
-        for (int b0 = 0; b0 < B; b0 += 32) {
-            const int b = b0 + lane;
-            const int tiles = b < B ? tile_prefix[b] : 0;
-            int incl = tiles;
+        const int per = (B + 31) / 32, b0 = min(lane * per, B), b1 = min(b0 + per, B);
+        int sum = 0;
+        for (int b = b0; b < b1; ++b) sum += tile_prefix[b];
+        int incl = sum;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int nb = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += nb;
-            }
-            __syncwarp();
-            if (b < B) tile_prefix[b] = run + incl - tiles;
-            run += __shfl_sync(0xffffffffu, incl, 31);
+        for (int o = 1; o < 32; o <<= 1) {
+            const int nb = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += nb;
         }
-        if (lane == 0) tile_prefix[B] = run;
+        int run = incl - sum;
+        for (int b = b0; b < b1; ++b) {
+            const int tiles = tile_prefix[b];
+            tile_prefix[b] = run;
+            run += tiles;
+        }
+        if (lane == 31) tile_prefix[B] = incl;
     }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    const bool void_launch = status && (*reinterpret_cast<volatile int*>(status) & STATUS_WAIT_MASK) != 0;
-    const int n_work = void_launch ? 0 : tile_prefix[B] * heads;
+    const int n_work = (status_word & STATUS_WAIT_MASK) != 0 ? 0 : tile_prefix[B] * heads;
     const int n_main = (n_keys / 16) * 16;          // keys handled by the tensor cores
     const int tail = n_keys - n_main;               // 0..15 keys handled on CUDA cores
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ------------------------------------------------------------ TMA producer
+            const int32_t* offs = keep ? offs_s : offsets;
             const uint32_t kv_bytes = (uint32_t)KC * HD * 2;
             int li = 0, g = 0;
             bool ok = true;
             for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++li) {
-                const AttnItem it = attn_item(w, heads, B, tile_prefix, offsets);
+                const AttnItem it = attn_item(w, heads, B, tile_prefix, offs);
                 const int qb = li & 1;
                 ok = mbar_wait(&q_free[qb], ((li >> 1) & 1) ^ 1, abort_flag, status, STATUS_ATTN_LOAD);
                 if (!ok) break;
@@ -209,7 +228,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // -------------------------------------------------------------- MMA issuer
             const uint32_t idesc_s = idesc_bf16_f32(QT, KC, 0, 0);
             const uint32_t idesc_o = idesc_bf16_f32(QT, HD, 0, 1);     // B = V, MN-major
@@ -260,6 +279,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         // ------------------------------------------------------- softmax + output warps
         const int r = (warp & 3) * 32 + lane;                     // query row = TMEM lane
         const uint32_t lane_base = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+        auto arrive = [&](uint64_t* bar) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar);
+        };
         int li = 0, g = 0;
         bool ok = true;
         for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++li) {
@@ -307,11 +330,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
                 if (!ok) break;
                 tc_fence_after_sync();
                 if (!live) {
-                    mbar_arrive(p_half);
-                    mbar_arrive(p_full);
+                    arrive(p_half);
+                    arrive(p_full);
                     ok = mbar_wait(o_full, ph, abort_flag, status, STATUS_ATTN_SOFTMAX);
                     if (!ok) break;
-                    mbar_arrive(o_free);
+                    arrive(o_free);
                     continue;
                 }
                 const int n_valid = min(KC, n_main - c * KC);
@@ -375,13 +398,13 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
                     if (c0 + 32 == P_SPLIT || (blk + 1 == nblk && c0 < P_SPLIT)) {
                         tmem_st_wait();
                         tc_fence_before_sync();
-                        mbar_arrive(p_half);
+                        arrive(p_half);
                     }
                 }
                 const float lsum = (ls4[0] + ls4[1]) + (ls4[2] + ls4[3]);
                 tmem_st_wait();
                 tc_fence_before_sync();
-                mbar_arrive(p_full);
+                arrive(p_full);
                 l = l * alpha + lsum;
                 m = m_new;
                 ok = mbar_wait(o_full, ph, abort_flag, status, STATUS_ATTN_SOFTMAX);
@@ -397,11 +420,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
                     for (int i = 0; i < 32; ++i) o[c0 + i] = fmaf(o[c0 + i], alpha, __uint_as_float(t[i]));
                 }
                 tc_fence_before_sync();
-                mbar_arrive(o_free);
+                arrive(o_free);
             }
             if (!ok) break;
             if (!live) {
-                mbar_arrive(&q_free[qb]);
+                arrive(&q_free[qb]);
                 continue;
             }
             // ---- one online-softmax step per tail key, behind the chunks: a row's terms are added in the order of its keys
@@ -454,7 +477,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
                 __syncwarp();
                 fence_proxy_async_smem();                       // the next Q tile is written by TMA
             }
-            mbar_arrive(&q_free[qb]);
+            arrive(&q_free[qb]);
         }
     }
     if (*abort_flag) {
@@ -497,7 +520,7 @@ int attention_tcgen05(const AttnArgs& p, cudaStream_t st) {
         if (int rc = make_tmap_bf16(&tk, p.k, 3, dims, strides, box)) return rc;
         if (int rc = make_tmap_bf16(&tv, p.v, 3, dims, strides, box)) return rc;
     }
-    const int smem = SM_PREFIX + (p.B + 1) * 4 + 1024;
+    const int smem = SM_PREFIX + (p.B + 1) * 4 * (p.B <= OFFSETS_KEPT ? 2 : 1) + 1024;
     static int attr_smem[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
