@@ -11,8 +11,7 @@
 
 namespace vtp {
 
-int token_im2col(const void* x, int dtype, int B, int H, int W, int C, int sr, void* cols, cudaStream_t st,
-                 const float2* stats = nullptr, const float* lnw = nullptr, const float* lnb = nullptr);  // patch_embed.cu
+int token_im2col(const void* x, int dtype, int B, int H, int W, int C, int sr, void* cols, cudaStream_t st);  // patch_embed.cu
 
 int patch_im2col(const void* images, int image_dtype, int B, int S, int P, int dtype, void* cols, int ld,
                  const void* cls_token, const void* pos_embed, int C, void* x, int32_t* counts, cudaStream_t st);   // patch_embed.cu
@@ -193,8 +192,8 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
                 "block: spatial reduction needs the sr and sr_norm parameters");
     const int n_keys = keys_per_image(s);
     // LayerNorm folded into the GEMM epilogues (bf16 tensor-core path with prepared weights): norm1 into q and
-    // norm2 into fc1.  A PVT block's keys need LayerNorm rows all the same; the im2col in front of the reducing
-    // convolution normalises them on the way from the token statistics.  Without a reduction kv folds norm1 too.
+    // norm2 into fc1.  A PVT block's keys need LayerNorm rows all the same; the pool kernel writes them as the rows of the reducing
+    // convolution.  Without a reduction kv folds norm1 too.
     const bool fold_q = block_folds(s, w);
     const bool fold = fold_q && !reduce;
     // norm2 into fc1 only where the reduction is long enough to hide it: with K <= 128 the Linear is bound by its
@@ -248,6 +247,8 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
         if (fold_q) {
             pa.stats_x = stats_x; pa.stats_q = b.stats_q;
             pa.stats_x_ready = stats_x_ready;
+            // (the rows of the reducing convolution come with it)
+            if (reduce) { pa.sr = s.sr_ratio; pa.cols = b.sr_cols; pa.lnw = w.norm1_w; pa.lnb = w.norm1_b; }
         }
         else { pa.lnw = w.norm1_w; pa.lnb = w.norm1_b; pa.xn = b.xn; pa.qn = b.qn; }
         rc = region_pool(pa, s.dtype, st);
@@ -267,8 +268,7 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
         if ((rc = linear(lq, st)) || (rc = marks.mark(4))) return rc;
         // x_ = norm(sr(LN1(x) as [B,C,H,W])): the stride-sr convolution as im2col rows times a matrix
         const int krows = s.B * n_keys, KS = s.sr_ratio * s.sr_ratio * C;
-        if (fold_q) rc = token_im2col(x_in, s.dtype, s.B, s.H, s.W, C, s.sr_ratio, b.sr_cols, st, stats_x, w.norm1_w, w.norm1_b);
-        else rc = token_im2col(b.xn, s.dtype, s.B, s.H, s.W, C, s.sr_ratio, b.sr_cols, st);
+        if (!fold_q) rc = token_im2col(b.xn, s.dtype, s.B, s.H, s.W, C, s.sr_ratio, b.sr_cols, st);
         if (rc) return rc;
         LinearArgs lsr;
         lsr.a = b.sr_cols; lsr.lda = KS; lsr.w = w.sr_w; lsr.bias = w.sr_b; lsr.y = b.sr_out; lsr.ldy = C;

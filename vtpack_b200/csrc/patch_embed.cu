@@ -152,10 +152,8 @@ im2col_kernel(const I* __restrict__ img, long long total8, int S, int P, T* __re
 // Replaces the permute / reshape in front of attn.sr (vtpack/models/dge/pvt_dge.py:82-83).
 template <typename T, typename IDX>
 __global__ void __launch_bounds__(256)
-token_im2col_kernel(const T* __restrict__ x, long long total_vec, int H, int W, int C, int sr, T* __restrict__ cols,
-                    const float2* __restrict__ stats, const float* __restrict__ lnw, const float* __restrict__ lnb) {
+token_im2col_kernel(const T* __restrict__ x, long long total_vec, int H, int W, int C, int sr, T* __restrict__ cols) {
     pdl_begin();
-    // stats != null: the rows gathered are LayerNorm(x), normalised on the way from each token's (mean, rstd)
     // (IDX: unsigned when the vector count fits 32 bits, see im2col4_kernel)
     constexpr int VN = Vec<T>::N;
     const int run = sr * C / VN;                  // 16-byte vectors per window row
@@ -170,29 +168,11 @@ token_im2col_kernel(const T* __restrict__ x, long long total_vec, int H, int W, 
         const long long tok = (b * H + (long long)oy * sr + dy) * W + (long long)ox * sr;
         Vec<T> t;
         t.load(x + tok * C + (long long)i * VN);
-        if (stats) {
-            const int e0 = i * VN;                        // element of the window row: token e0 / C, channel e0 % C
-            const float2 ms = stats[tok + e0 / C];
-            const int ch = e0 % C;
-            float f[VN], gw[VN], gb[VN];
-            t.to_float(f);
-#pragma unroll
-            for (int k4 = 0; k4 < VN / 4; ++k4) {          // ch is a multiple of VN: 16-byte loads of the LayerNorm vectors
-                const float4 w4 = __ldg(reinterpret_cast<const float4*>(lnw + ch) + k4);
-                const float4 b4 = __ldg(reinterpret_cast<const float4*>(lnb + ch) + k4);
-                gw[4 * k4] = w4.x; gw[4 * k4 + 1] = w4.y; gw[4 * k4 + 2] = w4.z; gw[4 * k4 + 3] = w4.w;
-                gb[4 * k4] = b4.x; gb[4 * k4 + 1] = b4.y; gb[4 * k4 + 2] = b4.z; gb[4 * k4 + 3] = b4.w;
-            }
-#pragma unroll
-            for (int k = 0; k < VN; ++k) f[k] = (f[k] - ms.x) * ms.y * gw[k] + gb[k];
-            t.from_float(f);
-        }
         t.store(cols + ((((b * Ho + oy) * Wo + ox) * sr + dy) * (long long)run + i) * VN);
     }
 }
 
-int token_im2col(const void* x, int dtype, int B, int H, int W, int C, int sr, void* cols, cudaStream_t st,
-                 const float2* stats, const float* lnw, const float* lnb) {
+int token_im2col(const void* x, int dtype, int B, int H, int W, int C, int sr, void* cols, cudaStream_t st) {
     const int vn = dtype == VTP_BF16 ? 8 : 4;
     VTP_REQUIRE(C % vn == 0, VTP_ERR_SHAPE, "spatial reduction: C=%d must be a multiple of %d", C, vn);
     const long long total = (long long)B * H * W * C / vn;
@@ -200,11 +180,11 @@ int token_im2col(const void* x, int dtype, int B, int H, int W, int C, int sr, v
     const int grid = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
     const bool small = total < (1ll << 31);
     if (dtype == VTP_BF16) {
-        if (small) launch_chain(token_im2col_kernel<bf16, unsigned>, dim3(grid), dim3(256), 0, st, (const bf16*)x, total, H, W, C, sr, (bf16*)cols, stats, lnw, lnb);
-        else launch_chain(token_im2col_kernel<bf16, long long>, dim3(grid), dim3(256), 0, st, (const bf16*)x, total, H, W, C, sr, (bf16*)cols, stats, lnw, lnb);
+        if (small) launch_chain(token_im2col_kernel<bf16, unsigned>, dim3(grid), dim3(256), 0, st, (const bf16*)x, total, H, W, C, sr, (bf16*)cols);
+        else launch_chain(token_im2col_kernel<bf16, long long>, dim3(grid), dim3(256), 0, st, (const bf16*)x, total, H, W, C, sr, (bf16*)cols);
     } else {
-        if (small) launch_chain(token_im2col_kernel<float, unsigned>, dim3(grid), dim3(256), 0, st, (const float*)x, total, H, W, C, sr, (float*)cols, stats, lnw, lnb);
-        else launch_chain(token_im2col_kernel<float, long long>, dim3(grid), dim3(256), 0, st, (const float*)x, total, H, W, C, sr, (float*)cols, stats, lnw, lnb);
+        if (small) launch_chain(token_im2col_kernel<float, unsigned>, dim3(grid), dim3(256), 0, st, (const float*)x, total, H, W, C, sr, (float*)cols);
+        else launch_chain(token_im2col_kernel<float, long long>, dim3(grid), dim3(256), 0, st, (const float*)x, total, H, W, C, sr, (float*)cols);
     }
     return check_launch("spatial reduction im2col");
 }
@@ -250,7 +230,7 @@ extern "C" int vtp_token_im2col(const void* x, int dtype, int B, int H, int W, i
     VTP_REQUIRE(B > 0 && H > 0 && W > 0 && C > 0 && ratio > 0 && H % ratio == 0 && W % ratio == 0, VTP_ERR_SHAPE,
                 "token im2col: grid %dx%d / ratio %d", H, W, ratio);
     VTP_REQUIRE(aligned16(x) && aligned16(cols), VTP_ERR_ALIGN, "token im2col: unaligned pointer");
-    return token_im2col(x, dtype, B, H, W, C, ratio, cols, static_cast<cudaStream_t>(stream), nullptr, nullptr, nullptr);
+    return token_im2col(x, dtype, B, H, W, C, ratio, cols, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int vtp_add_rows(const void* x, int x_mod, const void* addend, int a_mod, int a_off, void* out, int out_grp,

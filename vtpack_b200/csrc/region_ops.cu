@@ -199,7 +199,10 @@ __device__ __forceinline__ void publish_partials(float* part, float (&acc)[CPL][
 // Seven CTAs per SM (at most 73 registers, a few spilled words): the kernel is bound by how many
 // regions are in flight, and measured faster over the whole forward than at the 88 registers / five
 // CTAs the compiler picks on its own (six: +0.5 %, seven: +0.9 %, eight: +0.8 %).
-constexpr int POOL_LN = 0, POOL_STATS = 1, POOL_PLAIN = 2;
+// POOL_COLS:  POOL_STATS, and LayerNorm(x) as the rows of the strided convolution in front of the keys (a block with a spatial
+//             reduction): token (y, x) is element (y % sr, x % sr) of window (y / sr, x / sr).  The tokens are in registers
+//             here; a gather of its own read them again (PVT-small, 96 images: 2678 -> 2640 us, PVT-tiny, 3 images, 450 -> 444).
+constexpr int POOL_LN = 0, POOL_STATS = 1, POOL_PLAIN = 2, POOL_COLS = 3;
 // (A thread of a narrow-row layout holds one or two 16-byte vectors of a region: such kernels run with 16 or 12 CTAs per SM
 // (a few spilled words in the unpool; measured faster all the same), and the kernel is bound by how many regions are in flight.)
 template <typename T, int G, int CPL, int MODE>
@@ -211,9 +214,9 @@ pool_region_kernel(const T* __restrict__ x, RegionGeom g, const int32_t* __restr
                    T* __restrict__ comp, float2* __restrict__ stats_x, float2* __restrict__ stats_q,
                    float2* __restrict__ stats_acc, int write_stats_x, const float* __restrict__ lnw,
                    const float* __restrict__ lnb, float eps, T* __restrict__ xn, T* __restrict__ qn, int sum_only,
-                   int* status) {
+                   int sr, int* status) {
     pdl_begin();
-    constexpr bool STATS = MODE == POOL_STATS, EXPLICIT_LN = MODE == POOL_LN;
+    constexpr bool COLS = MODE == POOL_COLS, STATS = MODE == POOL_STATS || COLS, EXPLICIT_LN = MODE == POOL_LN;
     using L = Lay<T, G, CPL>;
     constexpr int VN = L::VN, GROUPS = L::GROUPS, TPG = L::TPG;
     extern __shared__ float part[];          // [4 grid rows][2 halves][C] partial sums
@@ -313,10 +316,32 @@ pool_region_kernel(const T* __restrict__ x, RegionGeom g, const int32_t* __restr
             if (write_stats_x) {
                 st = mean_rstd(row_sums<T, G, CPL>(f), g.C, eps);
                 if (sub == 0) stats_x[tok0 + j] = st;
-            } else if (step == 1) {
+            } else if (COLS || step == 1) {
                 st = stats_x[tok0 + j];
             }
             if (step == 1 && sub == 0) { stats_q[prow] = st; if (stats_acc) stats_acc[prow] = make_float2(0.f, 0.f); }
+            if (COLS) {
+                // (xn: the convolution's rows)
+                const int ty = ry * RG + w, tx = rx * RG + col, wy = ty / sr, wx = tx / sr;
+                const size_t win = ((size_t)b * (g.Hr * RG / sr) + wy) * (g.W / sr) + wx;
+                T* dst = xn + ((win * sr + (ty - wy * sr)) * sr + (tx - wx * sr)) * g.C;
+#pragma unroll
+                for (int ch = 0; ch < CPL; ++ch) {
+                    const int c0 = (sub + G * ch) * VN;
+                    float o[VN];
+#pragma unroll
+                    for (int i4 = 0; i4 < VN / 4; ++i4) {
+                        const float4 w4 = __ldg(reinterpret_cast<const float4*>(lnw + c0) + i4);
+                        const float4 b4 = __ldg(reinterpret_cast<const float4*>(lnb + c0) + i4);
+                        const float gw[4] = {w4.x, w4.y, w4.z, w4.w}, gb[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) o[4 * i4 + i] = (f[ch][4 * i4 + i] - st.x) * st.y * gw[i] + gb[i];
+                    }
+                    Vec<T> ov;
+                    ov.from_float(o);
+                    ov.store(dst + c0);
+                }
+            }
         } else if (EXPLICIT_LN) {
             ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, xn + (tok0 + j) * g.C);
             if (step == 1) ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, qn + (size_t)prow * g.C);
@@ -616,20 +641,25 @@ static void launch_pool_t(const RegionPoolArgs& a, cudaStream_t st) {
     const int R = a.g.Hr * a.g.Wr;
     const int grid = a.g.B * R + ceil_div(a.g.B * a.g.num_extra, RG * (32 / G));
     const size_t smem = (size_t)8 * a.g.C * sizeof(float);
-    if (a.stats_q)
+    if (a.stats_q && a.sr > 1)
+        launch_chain(pool_region_kernel<T, G, CPL, POOL_COLS>, dim3(grid), dim3(128), smem, st, 
+            (const T*)a.x, a.g, a.idx, a.region_first, a.offsets, a.counts, a.offsets_out, a.region_first_out,
+            a.counts_next, a.sp, (T*)a.comp, a.stats_x, a.stats_q, a.stats_acc, a.stats_x_ready ? 0 : 1, a.lnw,
+            a.lnb, a.eps, (T*)a.cols, nullptr, 0, a.sr, nullptr);
+    else if (a.stats_q)
         launch_chain(pool_region_kernel<T, G, CPL, POOL_STATS>, dim3(grid), dim3(128), smem, st, 
             (const T*)a.x, a.g, a.idx, a.region_first, a.offsets, a.counts, a.offsets_out, a.region_first_out,
             a.counts_next, a.sp, (T*)a.comp, a.stats_x, a.stats_q, a.stats_acc, a.stats_x_ready ? 0 : 1, nullptr,
-            nullptr, a.eps, nullptr, nullptr, 0, nullptr);
+            nullptr, a.eps, nullptr, nullptr, 0, 1, nullptr);
     else if (a.xn && a.qn)
         launch_chain(pool_region_kernel<T, G, CPL, POOL_LN>, dim3(grid), dim3(128), smem, st, 
             (const T*)a.x, a.g, a.idx, a.region_first, a.offsets, a.counts, a.offsets_out, a.region_first_out,
-            a.counts_next, a.sp, (T*)a.comp, nullptr, nullptr, nullptr, 0, a.lnw, a.lnb, a.eps, (T*)a.xn, (T*)a.qn, 0, nullptr);
+            a.counts_next, a.sp, (T*)a.comp, nullptr, nullptr, nullptr, 0, a.lnw, a.lnb, a.eps, (T*)a.xn, (T*)a.qn, 0, 1, nullptr);
     else
         launch_chain(pool_region_kernel<T, G, CPL, POOL_PLAIN>, dim3(grid), dim3(128), smem, st, 
             (const T*)a.x, a.g, a.idx, a.region_first, a.offsets, a.counts, a.offsets_out, a.region_first_out,
             a.counts_next, a.sp, (T*)a.comp, nullptr, nullptr, nullptr, 0, nullptr, nullptr, a.eps, nullptr, nullptr,
-            a.sum_only ? 1 : 0, device_status_ptr());
+            a.sum_only ? 1 : 0, 1, device_status_ptr());
 }
 
 template <typename T, int G, int CPL>

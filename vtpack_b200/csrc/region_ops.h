@@ -34,6 +34,9 @@ struct RegionPoolArgs {
     bool stats_x_ready = false;              // stats_x was already written (by the previous block's unpool)
     const float* lnw = nullptr; const float* lnb = nullptr; float eps = 1e-6f;
     void* xn = nullptr; void* qn = nullptr;
+    // With the statistics and sr > 1 (a divisor of both grid sides, no extra tokens): also LayerNorm(x) (lnw, lnb) in `cols`, as rows of
+    // the stride-sr convolution, [B * (H / sr) * (W / sr), sr * sr * C] with column (dy, dx, c).
+    int sr = 1; void* cols = nullptr;
     // With neither statistics nor LayerNorm rows asked for: plain pooled rows, as means or (sum_only) as the
     // sums of each patch's tokens, which is the gradient of the replicate-unpool for its packed rows.
     bool sum_only = false;
