@@ -327,6 +327,25 @@ def test_pvt_block_stages(C, heads, H, sr, mr, extra, dtype):
     assert err < (1e-4 if dtype == torch.float32 else 2e-2), err
 
 
+@pytest.mark.parametrize("C,heads", [(64, 1), (128, 2), (320, 5)])
+@pytest.mark.parametrize("H,W,sr", [(12, 24, 3), (24, 8, 2), (16, 16, 4), (60, 20, 5), (32, 48, 8)])
+def test_pvt_block_reduction_windows(C, heads, H, W, sr):
+    """Windows of the spatial reduction that lie inside a 4 x 4 region, cover several and straddle them, on grids that are not
+    square: the rows the pool writes for the convolution (bf16) against the fp32 oracle on the same bf16 weights and tokens, with the
+    bound of the stage shapes."""
+    from vtpack_b200 import _lib
+    w = O.round_bf16(O.make_pvt_block_weights(C, 2, sr, seed=7))
+    x = O.make_tokens(3, H * W, C, seed=8).bfloat16().float()
+    gate = O.make_gate_logits(3, H // 4, W // 4, 3, seed=9)
+    tr = {}
+    ref = O.dge_block_forward(x, w, heads, (4, 2, 1), forced_gate=gate, trace=tr, grid=(H, W), sr_ratio=sr)
+    blk = _pvt_block(C, heads, 2, sr, w, torch.bfloat16)
+    out = blk(x.to(DEV).bfloat16(), H, W, forced_gate=gate)
+    assert _lib.device_status() == 0
+    assert blk.dge.states["batches_device"].tolist() == tr["batches"].tolist()
+    assert rel_err(out.float(), ref) < 2e-2
+
+
 @pytest.mark.parametrize("C,heads,H,sr,mr,extra", [(64, 1, 64, 8, 8, 0), (128, 2, 32, 4, 8, 0), (320, 5, 16, 2, 4, 0),
                                                    (512, 8, 8, 1, 4, 1)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
