@@ -1,0 +1,46 @@
+"""Rules of the kernels that keep a failed launch from spreading, read off the CUDA sources: what they guard against cannot be
+made to happen on a GPU that others share."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "vtpack_b200", "csrc")
+WAITING = {"linear_tc_kernel": "linear_tc.cu", "linear_tc_small_kernel": "linear_tc.cu", "attn_tc_kernel": "attention_tc.cu",
+           "linear_f32_tc_kernel": "linear_f32_tc.cu"}
+
+
+def source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        text = re.sub(r"/\*.*?\*/", " ", f.read(), flags=re.S)
+    return re.sub(r"//[^\n]*", "", text)
+
+
+def body(name, text):
+    """From the opening brace of function `name` to the one that closes it."""
+    at = text.index("{", re.search(r"\b%s\(" % name, text).start())
+    depth = 0
+    for i in range(at, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0:
+            return text[at:i]
+    raise AssertionError(name)
+
+
+@pytest.mark.parametrize("kernel", sorted(WAITING))
+def test_stores_hang_on_a_status_word_read_behind_the_wait(kernel):
+    """Nothing is written after a launch that gave up on a wait.  The kernel in front, which may be the one that gives up, has
+    completed only behind griddepcontrol.wait, so the last look at the word lies there; and two threads that look for themselves
+    can decide differently, so every look is one thread's."""
+    text = body(kernel, source(WAITING[kernel]))
+    looks = [m.start() for m in re.finditer(r"launch_is_void\(", text)]
+    assert len([at for at in looks if at > text.index("pdl_begin()")]) == 1
+    for at in looks:
+        guard = max(m.end() for m in re.finditer(r"if \(threadIdx\.x == ([^()]|\([^()]*\))*\)", text[:at]))
+        assert ";" not in text[guard:at] and "{" not in text[guard:at]
+
+
+def test_no_other_code_looks_at_the_wait_codes():
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".h", ".cuh")) and name != "common.cuh":
+            assert "STATUS_WAIT_MASK" not in source(name), name

@@ -114,6 +114,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     uint64_t* p_half = bars + 12;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* void_s = reinterpret_cast<int*>(tmem_slot + 2);
     int* tile_prefix = reinterpret_cast<int*>(base + SM_PREFIX);
     int32_t* offs_s = tile_prefix + B + 1;
     AttnItem* items = reinterpret_cast<AttnItem*>(base + SM_ITEM);
@@ -121,9 +122,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
-    // (a launch does nothing after one that gave up on a wait; the word travels beside the set-up)
-    int status_word = 0;
-    if (status) status_word = *reinterpret_cast<volatile int*>(status);
     if (warp == 1 && elect_one()) {
         for (int i = 0; i < 2; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_free[i], SOFTMAX_WARPS); }
         mbar_init(k_full, 1); mbar_init(k_free, 1);
@@ -149,6 +147,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     // (the offsets come from the caller: a count outside [0, max_q] is clamped, so the item list
     // always fits the grid's bound, and rows at or beyond l_max are never stored below)
     const bool keep = B <= OFFSETS_KEPT;
+    if (threadIdx.x == blockDim.x - 1) *void_s = launch_is_void(status) ? 1 : 0;
     for (int b = threadIdx.x; b < B; b += blockDim.x) {
         const int o0 = offsets[b], o1 = offsets[b + 1];
         int cnt = o1 - o0;
@@ -187,7 +186,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    const int n_work = (status_word & STATUS_WAIT_MASK) != 0 ? 0 : tile_prefix[B] * heads;
+    const int n_work = *void_s ? 0 : tile_prefix[B] * heads;
     const int n_main = (n_keys / 16) * 16;          // keys handled by the tensor cores
     const int tail = n_keys - n_main;               // 0..15 keys handled on CUDA cores
 

@@ -78,8 +78,15 @@ enum : int {
     STATUS_GEMM_PRODUCER = 1, STATUS_GEMM_MMA = 2, STATUS_GEMM_EPILOGUE = 4,
     STATUS_ATTN_LOAD = 8, STATUS_ATTN_MMA = 16, STATUS_ATTN_SOFTMAX = 32,
     STATUS_BAD_INDEX = 64,      // a caller-supplied patch row or row offset pointed outside the declared arrays
-    STATUS_WAIT_MASK = 63,      // the bounded-wait codes: while one is set, tensor-core launches return at once
+    STATUS_WAIT_MASK = 63,      // the bounded-wait codes: while one is set, tensor-core launches write nothing (launch_is_void)
 };
+// Whether an earlier launch gave up on a wait: nothing is written any more.  The word may be set by the kernel in front, so what
+// decides about the stores is read behind the wait for that kernel; what is known in front of it saves the work too.  Launches
+// on other streams may set the word at any time: ONE thread reads it and tells those that must decide alike (the roles of a
+// CTA, the CTAs of a cluster) through shared memory.
+__device__ __forceinline__ bool launch_is_void(const int* status) {
+    return status && (*reinterpret_cast<const volatile int*>(status) & STATUS_WAIT_MASK) != 0;
+}
 
 // Index guards: kernels that follow caller-supplied indices (patch lists, packed-row offsets) check them
 // against the declared shapes, skip what does not fit and OR STATUS_BAD_INDEX into the status word.

@@ -191,6 +191,7 @@ linear_f32_tc_kernel(const F32Args g, int* status) {
     uint64_t* part_free = bars + 9;               // the other CTAs have added the ones this CTA sent them
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* void_s = reinterpret_cast<int*>(tmem_slot + 2);   // [2] launch_is_void in front of the wait and behind it
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
@@ -209,18 +210,19 @@ linear_f32_tc_kernel(const F32Args g, int* status) {
         tmem_alloc(tmem_slot, F_TMEM * BN);
         tmem_relinquish();
     }
+    if (threadIdx.x == (NCW + 1) * 32) void_s[0] = launch_is_void(status) ? 1 : 0;
     tc_fence_before_sync();
     __syncthreads();
     if (SPLIT > 1) cluster_sync_all();            // the partners' barriers exist
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    const bool known_void = lead_word<SPLIT>(void_s) != 0;
     pdl_begin();
 
     int M = g.m_max;
     if (g.m_dev) M = min(*reinterpret_cast<const volatile int32_t*>(g.m_dev), g.m_max);
-    const bool void_launch = status && (*reinterpret_cast<volatile int*>(status) & STATUS_WAIT_MASK) != 0;
     const int n_tiles = (g.N + BN - 1) / BN;
-    const int total = void_launch ? 0 : ((M + FM - 1) / FM) * n_tiles;
+    const int total = known_void ? 0 : ((M + FM - 1) / FM) * n_tiles;
     const int rank = SPLIT > 1 ? (int)cluster_ctarank() : 0;
     const int all_kb = (g.K + FK - 1) / FK;
     const int kb0 = all_kb * rank / SPLIT, num_kb = all_kb * (rank + 1) / SPLIT - kb0;    // this CTA's k-blocks
@@ -335,6 +337,10 @@ linear_f32_tc_kernel(const F32Args g, int* status) {
         const bool vec = g.N % 4 == 0 && g.ldy % 4 == 0 && (!g.res || g.ldr % 4 == 0);
         const int own_groups = (1 << g.groups_log2) / SPLIT;         // this CTA's: 1, 2 or 4
         const uint32_t tsum = tacc + 2 * BN;             // sums of its earlier groups: 0 (+ 1), and 2
+        // in a launch that turns out to be void the sums still change hands, but this CTA has no rows to store
+        if (threadIdx.x == (NCW + 1) * 32) void_s[1] = launch_is_void(status) ? 1 : 0;
+        named_barrier(1, F_EPI);
+        if (void_s[1] != 0) M = 0;
         int it = 0, n_done = 0;                           // k-blocks, tiles
         bool ok = true;
         for (int tile = first_tile; tile < total && ok; tile += tile_step, ++n_done) {

@@ -86,7 +86,7 @@ struct TcConf {
     static constexpr int TOTAL = (USED + 1024 <= SMEM_MAX) ? USED + 1024 : SMEM_MAX;
     static constexpr int TMEM_COLS = 2 * BN <= 256 ? 256 : 512;
     static_assert(STAGES >= 3, "operand ring");
-    static_assert((2 * STAGES + 4 + EW) * 8 + 8 <= CTRL_SCALARS, "barrier area");
+    static_assert((2 * STAGES + 4 + EW) * 8 + 16 <= CTRL_SCALARS, "barrier area");
 };
 
 // erf-GELU of eight values, packed two per register in fp16, as 0.5 x (1 + tanh(x (k0 + k1 x^2))) with
@@ -264,15 +264,15 @@ linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
     uint64_t* res_full = acc_empty + 2;        // [EW] the warp's residual slab has landed
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(res_full + EW);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* void_s = reinterpret_cast<int*>(tmem_slot + 2);               // [2] launch_is_void in front of the wait and behind it
     const TcSharedScalars& sc = *reinterpret_cast<const TcSharedScalars*>(ctrl + S::CTRL_SCALARS);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int rank = CG == 2 ? (int)cluster_ctarank() : 0;             // this CTA within its group
 
-    // not zero: an earlier launch gave up on a wait and this one does nothing (fetched here, beside the set-up)
-    int status_word = 0;
-    if (status) status_word = *reinterpret_cast<volatile int*>(status);
+    bool void_launch = false;
+    if (threadIdx.x == S::FIRST_EPI * 32) void_launch = launch_is_void(status);
     for (int i = threadIdx.x; i < (int)sizeof(TcSharedScalars) / 4; i += S::THREADS)
         reinterpret_cast<uint32_t*>(ctrl + S::CTRL_SCALARS)[i] = reinterpret_cast<const uint32_t*>(&L.s)[i];
     if (warp == 0 && elect_one()) {
@@ -300,16 +300,18 @@ linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
             if (EPI & EPI_RES) prefetch_tmap(&L.m[i].tr);
         }
     }
+    if (threadIdx.x == S::FIRST_EPI * 32) void_s[0] = void_launch ? 1 : 0;
     tc_fence_before_sync();
     __syncthreads();
     if (CG == 2) cluster_sync_all();     // the partner's barriers exist before anything arrives on them
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    const bool known_void = lead_word<CG>(void_s) != 0;
 
     // Everything above is independent of the kernel in front of this one on the stream; from
     // here on its results (row count, operands, residual, statistics) are read.
     pdl_begin();
-    const Sched sched(sc, (status_word & STATUS_WAIT_MASK) != 0);
+    const Sched sched(sc, known_void);
 
     // The two loops below run in one thread each, and a k-block has a few hundred cycles: shared memory goes by 32-bit
     // addresses that advance with the ring.
@@ -415,6 +417,10 @@ linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
                 else mbar_arrive(&acc_empty[b]);
             }
         };
+        // In a launch that turns out to be void the accumulators still change hands, but this CTA has no rows.
+        if (threadIdx.x == S::FIRST_EPI * 32) void_s[1] = launch_is_void(status) ? 1 : 0;
+        named_barrier(1, EW * 32);
+        const bool stores = void_s[1] == 0;
         int lt = 0;
         uint32_t res_ph = 0;
         bool ok = true;
@@ -423,7 +429,7 @@ linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
             if (wi.width <= 0) continue;
             const TcScalars& P = sc.p[wi.p];
             const TcMaps& T = L.m[wi.p];
-            const int M = (NPROB == 2 && wi.p) ? sched.M[NPROB - 1] : sched.M[0], N = P.N;
+            const int M = !stores ? 0 : (NPROB == 2 && wi.p) ? sched.M[NPROB - 1] : sched.M[0], N = P.N;
             const int buf = lt & 1;
             const uint32_t aph = (lt >> 1) & 1;
             ++lt;
@@ -640,6 +646,7 @@ linear_tc_small_kernel(const __grid_constant__ SmallLaunch L, int K, int* status
     uint64_t* acc_full = empty + STAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* void_s = reinterpret_cast<int*>(tmem_slot + 2);               // [2] launch_is_void in front of the wait and behind it
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const uint32_t full_a = smem_u32(full), empty_a = smem_u32(empty);
@@ -659,15 +666,15 @@ linear_tc_small_kernel(const __grid_constant__ SmallLaunch L, int K, int* status
     }
     if (warp == 1 && elect_one()) { prefetch_tmap(&L.ta[prob]); prefetch_tmap(&L.tw[prob]); }
     if (warp == PRODUCERS) { tmem_alloc(tmem_slot, 64); tmem_relinquish(); }
-    // an earlier launch gave up on a wait: this one does nothing
-    const bool void_launch = status && (*reinterpret_cast<volatile int*>(status) & STATUS_WAIT_MASK) != 0;
+    if (threadIdx.x == S::FIRST_EPI * 32) void_s[0] = launch_is_void(status) ? 1 : 0;
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    const bool known_void = void_s[0] != 0;
     pdl_begin();
 
-    if (void_launch) {
+    if (known_void) {
     } else if (warp < PRODUCERS) {
         if (elect_one()) {
             for (int kb = warp; kb < nkb; kb += PRODUCERS) {
@@ -701,8 +708,12 @@ linear_tc_small_kernel(const __grid_constant__ SmallLaunch L, int K, int* status
         const int g = (warp - S::FIRST_EPI) >> 2;         // which 16 columns of the tile
         const int row = (warp & 3) * 32 + lane;           // tile row = TMEM lane
         const int m = m0 + row, n0 = ct0 + g * 16, N = P.N;
+        // (a launch that turns out to be void forms its products and has no rows to store)
+        if (threadIdx.x == S::FIRST_EPI * 32) void_s[1] = launch_is_void(status) ? 1 : 0;
         int M = P.m_max;
         if (P.m_dev) M = min(max(*reinterpret_cast<const volatile int32_t*>(P.m_dev), 0), M);
+        named_barrier(5, S::EW * 32);
+        if (void_s[1] != 0) M = 0;
         // what the outputs need besides the accumulator travels while the operands are loaded and multiplied
         const bool live = m0 + (warp & 3) * 32 < M;       // the warp has rows
         const bool row_ok = m < M;

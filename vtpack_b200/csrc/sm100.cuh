@@ -269,6 +269,14 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
         }
     }
 }
+// A word of the rank-0 CTA's shared memory, written there in front of the last barrier of the cluster (CTAS = 1: of the CTA).
+template <int CTAS>
+__device__ __forceinline__ int lead_word(const int* slot) {
+    if (CTAS == 1) return *slot;
+    int v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(mapa_u32(smem_u32(slot), 0)) : "memory");
+    return v;
+}
 // TMEM allocation for the pair: the same warp of BOTH CTAs executes it with the same arguments.
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* dst_smem, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)),
