@@ -641,6 +641,25 @@ def test_linear_bf16_rows_do_not_depend_on_the_launch(vl, N, K, gelu, res):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("N,K", [(72, 64), (192, 768), (384, 384), (768, 384), (1536, 256)])
+def test_linear_bf16_without_a_bias(vl, N, K):
+    """The same bits with no bias as with one of zeros, from the kernel of small problems, single CTAs and pairs."""
+    from vtpack_b200 import _lib
+    from vtpack_b200.runtime import ptr, stream_ptr
+    g = torch.Generator(DEV).manual_seed(N + K)
+    x = torch.randn(20000, K, device=DEV, generator=g).bfloat16()
+    w = (torch.randn(N, K, device=DEV, generator=g) * K ** -0.5).bfloat16()
+    zeros = torch.zeros(N, device=DEV)
+    for M in (5, 20000):
+        y = torch.full((2, M, N), 7.0, device=DEV, dtype=torch.bfloat16)
+        for i, b in enumerate((None, zeros)):
+            _lib.check(_lib.lib().vtp_linear(ptr(x), K, ptr(w), ptr(b), None, 0, ptr(y[i]), N, 1, M, None, N, K, 0,
+                                             stream_ptr(x.device)))
+        assert torch.equal(y[0], y[1])
+        assert rel_err(y[0].float(), x[:M].double() @ w.double().T) < 2.0 ** -8       # one rounding of the output to bf16
+    assert _lib.device_status() == 0
+
+
 def test_threads_that_launch_give_their_memory_back(vl):
     """What a launching thread keeps (its encoded tensor maps, about 256 KB) goes with it."""
     import threading

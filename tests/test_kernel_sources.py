@@ -44,3 +44,16 @@ def test_no_other_code_looks_at_the_wait_codes():
     for name in sorted(os.listdir(CSRC)):
         if name.endswith((".cu", ".h", ".cuh")) and name != "common.cuh":
             assert "STATUS_WAIT_MASK" not in source(name), name
+
+
+def test_device_arrays_state_their_alignment():
+    """An array of the library's own is aligned to its element type unless it says more, and the kernels read such arrays through
+    vector types (the linker happens to align them well enough: nothing else would show it)."""
+    found = 0
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".h", ".cuh")):
+            for line in re.findall(r"^(?:static )?__device__ (?!__forceinline__)[^;{]*\[[^;]*;", source(name), flags=re.M):
+                said = re.search(r"(?:__align__|alignas)\((\d+)\)", line)
+                assert said and int(said.group(1)) >= 16, (name, line)
+                found += 1
+    assert found >= 2

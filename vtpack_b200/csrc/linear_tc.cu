@@ -145,7 +145,7 @@ struct TcSharedScalars { TcScalars p[2]; FastDiv groups; };
 struct TcLaunch { TcMaps m[2]; TcSharedScalars s; };
 static_assert(sizeof(TcSharedScalars) % 4 == 0 && sizeof(TcSharedScalars) <= 512, "copied to shared memory in words");
 
-__device__ const float g_no_bias[8] = {};      // what a Linear without a bias adds
+__device__ const __align__(16) float g_no_bias[8] = {};      // what a Linear without a bias adds, read up to 16 bytes at a time
 
 // A row's folded LayerNorm, LN(a) W^T + b = ln_a * acc + (ln_b * s[n] + bias[n]), from its statistics.
 __device__ __forceinline__ void row_fold(const LnFold& ln, int m, float& ln_a, float& ln_b) {
