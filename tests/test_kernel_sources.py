@@ -57,3 +57,29 @@ def test_device_arrays_state_their_alignment():
                 assert said and int(said.group(1)) >= 16, (name, line)
                 found += 1
     assert found >= 2
+
+
+@pytest.mark.parametrize("stages", range(3, 9))
+def test_pair_producers_wait_for_every_last_commit(stages):
+    """Before a CTA of a pair ends, its producers wait for the commit of every stage's last fill.  A wait goes by the parity of a
+    barrier's phase, so it means what it says only if the commit before has been seen: here the MMA thread is as late as the
+    waits in front allow, and no wait may pass on an older commit."""
+    text = body("linear_tc_kernel", source("linear_tc.cu"))
+    drain = text[text.index("if (CG == 2 && ok"):text.index("rank == 0 && elect_one()")]
+    own = re.search(r"f % PRODUCERS == \(uint32_t\)warp", drain) is not None      # else producer 0 waits for all, by stage
+    producers = 3
+    for filled in range(1, 6 * stages):
+        last = sorted(range(max(0, filled - stages), filled), key=lambda f: f if own else f % stages)
+        waited = set()
+        for w in range(producers):
+            mine = [f for f in range(filled) if f % producers == w]
+            done = mine[-1] - stages + 1 if mine else 0         # k-blocks committed for sure: all up to the last one waited for
+            for f in last:
+                if own and f % producers != w or not own and w != 0:
+                    continue
+                phases = len(range(f % stages, max(done, 0), stages))
+                passes = (phases - 1) & 1 == (f // stages) & 1     # (a fresh barrier passes a wait on parity 1)
+                assert not passes, (filled, w, f)
+                done = f + 1                                     # commits are in order
+                waited.add(f)
+        assert waited == set(last)

@@ -351,14 +351,13 @@ linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
                     if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
             }
-            if (CG == 2 && ok && warp == 0) {
-                // The MMA thread's last commits arrive on this CTA's `empty` barriers, from the partner for
-                // rank 1: wait for them, so that nothing is signalled into a CTA that has retired.
-                for (int i = 0; i < STAGES && ok; ++i) {
-                    if (filled <= (uint32_t)i) break;
-                    const uint32_t uses = (filled - i + STAGES - 1) / STAGES;
-                    ok = mbar_wait_a(empty_a + 8 * i, (uses - 1) & 1, abort_flag, status, STATUS_GEMM_PRODUCER);
-                }
+            if (CG == 2 && ok) {
+                // The MMA thread's last commits arrive on this CTA's `empty` barriers, from the partner for rank 1: wait for
+                // them, so that nothing is signalled into a CTA that has retired.  Each producer for its own last fills: it
+                // has seen the stage's commit before, so the parity is that of the commit it means.
+                for (uint32_t f = filled > (uint32_t)STAGES ? filled - STAGES : 0; f < filled && ok; ++f)
+                    if (f % PRODUCERS == (uint32_t)warp)
+                        ok = mbar_wait_a(empty_a + 8 * (f % STAGES), (f / STAGES) & 1, abort_flag, status, STATUS_GEMM_PRODUCER);
             }
         }
         __syncwarp();
