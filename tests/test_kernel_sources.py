@@ -83,3 +83,24 @@ def test_pair_producers_wait_for_every_last_commit(stages):
                 done = f + 1                                     # commits are in order
                 waited.add(f)
         assert waited == set(last)
+
+
+@pytest.mark.parametrize("kernel", sorted(WAITING))
+def test_lanes_that_wait_together_go_on_together(kernel):
+    """A wait gives up after about a second, lane by lane.  Where a whole warp waits, warp-wide instructions follow, which a lane
+    that went to unwind never reaches: such waits are decided by a vote, or no lane leaves.  Others are those of one elected thread."""
+    text = body(kernel, source(WAITING[kernel]))
+    elected = []
+    for m in re.finditer(r"if \((rank == 0 && )?elect_one\(\)\) \{", text):
+        depth, i = 1, m.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[i], 0)
+            i += 1
+        elected.append((m.end(), i))
+    waits = [(m.start(), m.group(1)) for m in re.finditer(r"\bmbar_(\w*wait\w*)\(", text)]
+    assert len(waits) >= 3
+    for at, name in waits:
+        one = any(a <= at < b for a, b in elected)
+        # (the warps that split fp32 operands have only __syncwarp behind it, which a lane that leaves still runs as often)
+        runs_out = "num_kb - kb; n > 0; --n) __syncwarp();" in text[at:at + 400]
+        assert name in (("wait", "wait_a") if one or runs_out else ("wait_warp", "wait_cluster_warp")), (name, text[at:at + 80])

@@ -287,7 +287,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++li) {
             const int qb = li & 1;
             // the producer worked out which (image, head, rows) this item is; it arrives with the Q tile
-            ok = mbar_wait(&q_full[qb], (li >> 1) & 1, abort_flag, status, STATUS_ATTN_SOFTMAX);
+            ok = mbar_wait_warp(&q_full[qb], (li >> 1) & 1, abort_flag, status, STATUS_ATTN_SOFTMAX);
             if (!ok) break;
             const AttnItem it = items[qb];
             // a warp whose 32 rows all lie beyond the item's queries only keeps the barriers moving: its rows
@@ -325,13 +325,13 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
             }
             for (int c = 0; c < n_chunks && ok; ++c, ++g) {
                 const uint32_t ph = g & 1;
-                ok = mbar_wait(s_full, ph, abort_flag, status, STATUS_ATTN_SOFTMAX);
+                ok = mbar_wait_warp(s_full, ph, abort_flag, status, STATUS_ATTN_SOFTMAX);
                 if (!ok) break;
                 tc_fence_after_sync();
                 if (!live) {
                     arrive(p_half);
                     arrive(p_full);
-                    ok = mbar_wait(o_full, ph, abort_flag, status, STATUS_ATTN_SOFTMAX);
+                    ok = mbar_wait_warp(o_full, ph, abort_flag, status, STATUS_ATTN_SOFTMAX);
                     if (!ok) break;
                     arrive(o_free);
                     continue;
@@ -406,7 +406,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
                 arrive(p_full);
                 l = l * alpha + lsum;
                 m = m_new;
-                ok = mbar_wait(o_full, ph, abort_flag, status, STATUS_ATTN_SOFTMAX);
+                ok = mbar_wait_warp(o_full, ph, abort_flag, status, STATUS_ATTN_SOFTMAX);
                 if (!ok) break;
                 tc_fence_after_sync();
 #pragma unroll

@@ -469,7 +469,7 @@ linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
                 }
                 if ((EPI & EPI_LN) && wrow0 + lane < M) row_fold(P.ln, wrow0 + lane, ln_a, ln_b);
             }
-            ok = mbar_wait(&acc_full[buf], aph, abort_flag, status, STATUS_GEMM_EPILOGUE);
+            ok = mbar_wait_warp(&acc_full[buf], aph, abort_flag, status, STATUS_GEMM_EPILOGUE);
             if (!ok) break;
             tc_fence_after_sync();
             if (!active) {
@@ -477,7 +477,7 @@ linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
                 continue;
             }
             if ((EPI & EPI_RES) && res_tma) {
-                ok = mbar_wait(&res_full[e], res_ph, abort_flag, status, STATUS_GEMM_EPILOGUE);
+                ok = mbar_wait_warp(&res_full[e], res_ph, abort_flag, status, STATUS_GEMM_EPILOGUE);
                 res_ph ^= 1;
                 if (!ok) break;
             }
@@ -744,7 +744,7 @@ linear_tc_small_kernel(const __grid_constant__ SmallLaunch L, int K, int* status
             }
         }
         const long long orow = map_out_row(P.rm, row_ok ? m : m0);
-        const bool ok = mbar_wait(acc_full, 0, abort_flag, status, STATUS_GEMM_EPILOGUE);
+        const bool ok = mbar_wait_warp(acc_full, 0, abort_flag, status, STATUS_GEMM_EPILOGUE);
         if (ok && live) {
             tc_fence_after_sync();
             uint32_t r[16];

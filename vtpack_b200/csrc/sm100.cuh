@@ -80,8 +80,11 @@ __device__ __forceinline__ bool mbar_wait_a(uint32_t bar, uint32_t parity, volat
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
     return mbar_wait_a(smem_u32(bar), parity, abort_flag, status, code);
 }
-
-// Shared-memory accesses by 32-bit shared-space address (a generic pointer costs 64-bit address arithmetic
+// The same for all lanes of a converged warp: at the limit a lane can still see the phase that another one has given up on, and
+// the warp-wide instructions behind the wait would then stand for ever for lanes that have gone to unwind.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code));
+}// Shared-memory accesses by 32-bit shared-space address (a generic pointer costs 64-bit address arithmetic
 // and a generic load / store per access).
 __device__ __forceinline__ float4 lds_f4(uint32_t addr) {
     float4 v;
@@ -248,9 +251,11 @@ __device__ __forceinline__ void stc_f4(uint32_t cluster_addr, float4 v) {
 __device__ __forceinline__ void mbar_arrive_release_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
-                                                  int code) {
+// For all lanes of a converged warp, see mbar_wait_warp.
+__device__ __forceinline__ bool mbar_wait_cluster_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
+                                                       int code) {
     const long long t0 = clock64();
+    bool done;
     for (;;) {
         uint32_t ok;
         asm volatile(
@@ -260,14 +265,15 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
             : "=r"(ok)
             : "r"(smem_u32(bar)), "r"(parity)
             : "memory");
-        if (ok) return true;
-        if (*abort_flag) return false;
+        done = ok != 0;
+        if (done || *abort_flag) break;
         if (clock64() - t0 > kWaitLimitCycles) {
             *abort_flag = 1;
             if (status) atomicOr(status, code);
-            return false;
+            break;
         }
     }
+    return __all_sync(0xffffffffu, done);
 }
 // A word of the rank-0 CTA's shared memory, written there in front of the last barrier of the cluster (CTAS = 1: of the CTA).
 template <int CTAS>
