@@ -327,6 +327,23 @@ def test_pvt_block_stages(C, heads, H, sr, mr, extra, dtype):
     assert err < (1e-4 if dtype == torch.float32 else 2e-2), err
 
 
+def _visible_keys(C, sr):
+    """Weights of a PVT block whose output shows its keys: tokens small beside their LayerNorm, attention sharp and wide, the MLP
+    faint, random LayerNorm gains and biases.  In the oracle, rows of the reducing convolution that are wrong change the largest
+    output by (15 shapes of test_pvt_block_reduction_windows) 0.3 to 1.5 of itself where rows or columns of the grid are
+    mirrored or rolled, window elements or images exchanged, channels rolled, norm1's gain and bias left out, zeros or noise
+    given; by 0.10 to 0.34 where one 4 x 4 region is zero, by 0.027 to 0.12 where one token is."""
+    w = O.make_pvt_block_weights(C, 2, sr, seed=7)
+    g = torch.Generator().manual_seed(11)
+    for n in ("norm1", "attn.norm"):
+        w[n + ".weight"] = 1 + 0.5 * torch.randn(C, generator=g)
+        w[n + ".bias"] = 0.5 * torch.randn(C, generator=g)
+    for n in ("q", "kv", "proj"):
+        w[f"attn.{n}.weight"] = w[f"attn.{n}.weight"] * (5 * (C / 64) ** -0.5)
+    w["mlp.fc2.weight"] = w["mlp.fc2.weight"] * 0.01
+    return O.round_bf16(w)
+
+
 @pytest.mark.parametrize("C,heads", [(64, 1), (128, 2), (320, 5)])
 @pytest.mark.parametrize("H,W,sr", [(12, 24, 3), (24, 8, 2), (16, 16, 4), (60, 20, 5), (32, 48, 8)])
 def test_pvt_block_reduction_windows(C, heads, H, W, sr):
@@ -334,8 +351,8 @@ def test_pvt_block_reduction_windows(C, heads, H, W, sr):
     square: the rows the pool writes for the convolution (bf16) against the fp32 oracle on the same bf16 weights and tokens, with the
     bound of the stage shapes."""
     from vtpack_b200 import _lib
-    w = O.round_bf16(O.make_pvt_block_weights(C, 2, sr, seed=7))
-    x = O.make_tokens(3, H * W, C, seed=8).bfloat16().float()
+    w = _visible_keys(C, sr)
+    x = (O.make_tokens(3, H * W, C, seed=8) * 2.0 ** -6).bfloat16().float()
     gate = O.make_gate_logits(3, H // 4, W // 4, 3, seed=9)
     tr = {}
     ref = O.dge_block_forward(x, w, heads, (4, 2, 1), forced_gate=gate, trace=tr, grid=(H, W), sr_ratio=sr)
@@ -343,7 +360,8 @@ def test_pvt_block_reduction_windows(C, heads, H, W, sr):
     out = blk(x.to(DEV).bfloat16(), H, W, forced_gate=gate)
     assert _lib.device_status() == 0
     assert blk.dge.states["batches_device"].tolist() == tr["batches"].tolist()
-    assert rel_err(out.float(), ref) < 2e-2
+    err = rel_err(out.float(), ref)
+    assert err < 2e-2, err
 
 
 @pytest.mark.parametrize("C,heads,H,sr,mr,extra", [(64, 1, 64, 8, 8, 0), (128, 2, 32, 4, 8, 0), (320, 5, 16, 2, 4, 0),
