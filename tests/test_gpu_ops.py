@@ -155,8 +155,8 @@ def test_linear_fp32(vl, M, N, K, gelu, res):
 
 @pytest.mark.parametrize("M,N,K", [(1, 64, 64), (130, 192, 192), (257, 768, 192), (64, 1000, 384), (300, 384, 1536),
                                    (1024, 1536, 384),
-                                   # narrow, short-K Linears (PVT stages 1 and 2): several tiles per CTA, so the
-                                   # staging slabs and the held bias slice go round more than once
+                                   # narrow, short-K Linears (PVT stages 1 and 2): several tiles per CTA, so the operand
+                                   # ring, the accumulators and the staging buffers go round more than once
                                    (148 * 128 * 5 + 77, 64, 64), (148 * 128 * 3, 128, 64), (148 * 128 * 3 + 5, 128, 128)])
 @pytest.mark.parametrize("gelu,res", [(False, False), (True, False), (False, True)])
 def test_linear_bf16_tensor_cores(vl, M, N, K, gelu, res):
@@ -277,6 +277,20 @@ def test_attention_leading_keys_of_weight_zero(vl, dtype, bound, flags, N, far):
     ref = O.batched_sparse_attention_forward(q.float(), k.float(), v.float(), torch.tensor(lens), 64 ** -0.5)
     got = layers.batched_sparse_attention(q.to(DEV), k.to(DEV), v.to(DEV), torch.tensor(lens), 64 ** -0.5, flags=flags)
     assert torch.isfinite(ref).all() and rel_err(got.float(), ref) < bound
+
+
+@pytest.mark.parametrize("B", [1, 31, 33, 512, 513, 2000])
+def test_attention_bf16_many_images(vl, B):
+    """Images of 0 to 3 queries, with one of 131 in the middle and one of 130 at the end (two tiles each, the second one ragged):
+    the scan over the images' tiles, a run of images to a lane, and the offsets, which up to 512 images are kept in shared
+    memory.  Bound as above."""
+    _lib, layers = vl
+    lens = [(7 * i + 1) % 4 for i in range(B)]
+    lens[B // 2], lens[-1] = 131, 130
+    q, k, v, ref = _attn_case(torch.bfloat16, B, 17, 1, lens, seed=B)
+    got = layers.batched_sparse_attention(q.to(DEV), k.to(DEV), v.to(DEV), torch.tensor(lens), 64 ** -0.5)
+    assert _lib.device_status() == 0
+    assert got.shape == ref.shape and rel_err(got.float(), ref) < 8e-3
 
 
 def test_attention_strided_views(vl):
