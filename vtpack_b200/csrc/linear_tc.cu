@@ -1007,7 +1007,10 @@ static int launch_tc(const LinearArgs& p, const LinearArgs* p1, cudaStream_t st)
 }
 
 // 128 x 64 tiles of a problem.  As many as SMs at most run as linear_tc_small_kernel: all at once, one per SM.  (DeiT-Ti, one
-// image: 505 us per forward with the persistent kernel alone, 395 with both; DeiT-S, 7 images: 662 and 586.)
+// image: 505 us per forward with the persistent kernel alone, 395 with both; DeiT-S, 7 images: 662 and 586.  Launches on both
+// sides of the line, us, small / persistent kernel:  1536, K = 384, GELU: 96 tiles 4.6 / 6.2, 144 4.7 / 6.8, 216 8.5 / 7.0, 288
+// 8.9 / 7.3;  384, K = 1536, residual: 108 tiles 7.8 / 8.9, 144 7.8 / 9.5, 222 14.7 / 11.5;  768, K = 192, GELU: 108 tiles 3.9 / 4.7,
+// 144 4.1 / 4.8, 216 7.4 / 5.4.)
 static long long small_tiles(const LinearArgs& p) { return (long long)ceil_div(p.m_max, TBM) * ceil_div(p.N, SmallConf::BN); }
 
 template <int EPI, bool F32, int NPROB>
@@ -1054,8 +1057,11 @@ bool linear_pair_supported(const LinearArgs& a, const LinearArgs& b) {
 
 // Whether two CTAs should share 256-row tiles (cta_group::2).  Each then loads and multiplies half of the tile's W rows, which
 // pays once a tile has several k-blocks: 65792 x 768 with K = 384 48.1 -> 41.2 us, 23040 x 384 with K = 1536 37.1 -> 30.8.  With
-// K = 64 or 128, or tiles of 128 columns, the pair's longer set-up costs more than that: 393216 x 64 with K = 64 19.5 -> 21.7,
-// 172000 x 64 with K = 512 37.6 -> 39.6, 172000 x 512 with K = 64 42.5 -> 43.9.
+// K = 64, or tiles of 128 columns, the pair's longer set-up costs more than that: 393216 x 64 with K = 64 19.5 -> 21.7,
+// 172000 x 64 with K = 512 37.6 -> 39.6, 172000 x 512 with K = 64 42.5 -> 43.9.  From K = 128 to 256 it depends on the launch: many
+// rounds of tiles gain, one or two lose (K = 192: 65792 x 576 24.6 -> 21.2, 65792 x 384 14.4 -> 14.2, 22000 x 192 6.1 -> 6.8, 22000 x
+// 768 12.7 -> 13.8, 8000 x 768 8.0 -> 8.8; K = 256: 65792 x 768 36.1 -> 30.3, 65792 x 512 25.8 -> 21.7, 22000 x 1024 15.4 -> 15.8, 8000 x
+// 1024 8.9 -> 9.7).  The line keeps K = 192, the projections and fc1 of DeiT-Ti, on single CTAs; no other model has a K between.
 static bool pairs_pay(int bn, int K) { return bn >= 192 && K >= 256; }
 
 int linear_tcgen05_pair(const LinearArgs& a, const LinearArgs& b, cudaStream_t st) {

@@ -53,8 +53,8 @@ __device__ __forceinline__ bool elect_one() {
     return p != 0;
 }
 
-// About one second at 2 GHz.  A wait that runs this long means a copy or MMA that will
-// never complete; the waiter records `code`, raises the CTA's abort flag and returns false
+// About one second at 2 GHz, counted from the 1024th try of a wait on.  A wait that runs this long means a copy or MMA that
+// will never complete; the waiter records `code`, raises the CTA's abort flag and returns false
 // so that the kernel can unwind instead of hanging the GPU.
 constexpr long long kWaitLimitCycles = 2000000000LL;
 
