@@ -27,8 +27,9 @@ STAGES = ["router_gate", "patch_list", "pool_ln1", "q_proj", "kv_proj", "attenti
           "fc2", "unpool_add"]
 # DRAM bytes (read + written) of one launch of the dominant kernel on the roofline's workload (the kv
 # projection at batch 256: M=65792, N=768, K=384), from the ncu capture summarised in
-# profiles/linear_tc_kv_projection_m65792_n768_k384.md; scaled by the row count for other batch sizes
-NCU_TRAFFIC_BYTES_PER_ROW = (51173888 + 43880448) / 65792
+# profiles/linear_tc_kv_projection_m65792_n768_k384.md, over the launch's operand and output bytes (below 1: part of the
+# output is still in L2 when the kernel ends); other shapes are scaled by their own bytes
+NCU_TRAFFIC_PER_BYTE = (51157760 + 45900800) / ((65792 * 384 + 2 * 384 * 384 + 65792 * 768) * 2)
 
 
 def peaks():
@@ -317,9 +318,9 @@ def kv_launch_roofline(model, batch, device, pk, iters=20):
             "achieved": round(ach, 1), "peak": pk["bf16_tflops"], "unit": "TFLOP/s",
             "frac": round(ach / pk["bf16_tflops"], 3), "peak_kind": "burst cuBLAS bf16 (launch timed on its own)",
             "frac_of_sustained_peak": round(ach / pk["bf16_tflops_sustained"], 3),
-            "traffic": int(NCU_TRAFFIC_BYTES_PER_ROW * M),
+            "traffic": int(NCU_TRAFFIC_PER_BYTE * (M * C + 2 * C * C + M * 2 * C) * 2),
             "traffic_note": "constant: dram read + write bytes of one launch from the committed ncu capture "
-                            "(profiles/), scaled by the row count; not measured in this run",
+                            "(profiles/), scaled by the algorithmic bytes; not measured in this run",
             "algorithmic_bytes": (M * C + 2 * C * C + M * 2 * C) * 2, "launch_us": round(us, 2),
             "timing": f"{iters} launches back to back between two CUDA events; "
                       f"{(M * C + M * 2 * C) * 2 / 1e6:.0f} MB per launch (> L2)"}
