@@ -1061,7 +1061,8 @@ bool linear_pair_supported(const LinearArgs& a, const LinearArgs& b) {
 // 172000 x 64 with K = 512 37.6 -> 39.6, 172000 x 512 with K = 64 42.5 -> 43.9.  From K = 128 to 256 it depends on the launch: many
 // rounds of tiles gain, one or two lose (K = 192: 65792 x 576 24.6 -> 21.2, 65792 x 384 14.4 -> 14.2, 22000 x 192 6.1 -> 6.8, 22000 x
 // 768 12.7 -> 13.8, 8000 x 768 8.0 -> 8.8; K = 256: 65792 x 768 36.1 -> 30.3, 65792 x 512 25.8 -> 21.7, 22000 x 1024 15.4 -> 15.8, 8000 x
-// 1024 8.9 -> 9.7).  The line keeps K = 192, the projections and fc1 of DeiT-Ti, on single CTAs; no other model has a K between.
+// 1024 8.9 -> 9.7).  The line keeps K = 192 (DeiT-Ti) on single CTAs, and K = 128 (stage 2 of PVT, where 43000 x 512
+// would go 12.4 -> 11.7 and 100000 x 256 13.5 -> 13.0); no model has K = 256 with tiles this wide.
 static bool pairs_pay(int bn, int K) { return bn >= 192 && K >= 256; }
 
 int linear_tcgen05_pair(const LinearArgs& a, const LinearArgs& b, cudaStream_t st) {
