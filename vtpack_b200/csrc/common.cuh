@@ -34,7 +34,7 @@ int sm_count();
 // Launches `kernel`; with `early` it may start while the previous kernel on the stream is finishing (programmatic
 // dependent launch; a programmatic edge when the stream is being captured into a graph).  Every kernel launched
 // through here begins with pdl_begin(), or calls griddep_wait() before it touches anything an earlier kernel wrote
-// and griddep_launch() after that.  `cluster_x` > 1 cuts the grid into clusters.
+// (but for a first look at the status word, see launch_is_void) and griddep_launch() after that.  `cluster_x` > 1 cuts the grid into clusters.
 template <typename... KArgs, typename... Args>
 cudaError_t launch_kernel(void (*kernel)(KArgs...), bool early, int cluster_x, dim3 grid, dim3 block, size_t smem,
                           cudaStream_t st, Args&&... args) {
