@@ -75,6 +75,39 @@ def test_all_fine_equals_dense_block_fp32():
     assert rel_err(a, ref) < 1e-4 and rel_err(b, ref) < 1e-4
 
 
+@pytest.mark.parametrize("C,B,mlp_ratio,special", [
+    (256, 1, 0.84375, False),       # 216 hidden channels: a reduction that is not whole k-blocks; two rows of tiles and one row more
+    (256, 2, 4.0, True), (256, 5, 1.65625, False), (256, 40, 1.0, False),
+    (384, 1, 4.0, False), (384, 12, 4.0, False), (384, 4, 4.0, True),
+    (768, 1, 4.0, False), (768, 2, 4.0, True),
+])
+def test_block_fp32_terms_same_bits_as_rows(C, B, mlp_ratio, special):
+    """An fp32 block's Linears take their operands as three bf16 terms, split by the kernels in front of them; the dense block's
+    Linears split fp32 rows themselves.  With every region at the finest grain the two blocks do the same arithmetic
+    (channels that the pool spreads over whole warps: LayerNorm sums in the same order), so the outputs are the same bits, where operands or
+    sums are infinite, NaN, near the largest or subnormal too."""
+    from vtpack_b200 import _lib
+    from vtpack_b200.models.dge.deit_dge import Block
+    torch.manual_seed(C + B)
+    blk = Block(C, C // 64, mlp_ratio=mlp_ratio, qkv_bias=True, split_sizes=[4, 2, 1]).to(DEV).eval()
+    x = torch.randn(B, 257, C, device=DEV)
+    if special:
+        with torch.no_grad():
+            w1, w2 = blk.mlp.fc1.weight, blk.mlp.fc2.weight
+            w1[5, 3], w1[64, 7], w1[70] = 2.0 ** 113, -3.4e38, 1e-41        # (a row of subnormal numbers)
+            w2[9, 2], w2[10, 1], w2[11, 0] = float("inf"), float("nan"), 2.0 ** 111
+            blk.attn.proj.weight[17, 5] = -float("inf")
+        x[0, 40, 3] = 1e30
+    gate = torch.zeros(B, 4, 4, 3)
+    gate[..., 0] = 1
+    with torch.no_grad():
+        # (the cls row goes through the unpool's sum, ref + (q - comp), which rounds)
+        a, b = blk(x, forced_gate=gate)[:, 1:], blk(x, dense=True)[:, 1:]
+    assert _lib.device_status() == 0
+    assert bool(torch.isfinite(a).all()) != special
+    assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.nan_to_num(nan=0.0), b.nan_to_num(nan=0.0))
+
+
 def test_layer_512px_skewed_fp32():
     """32x32 grid (N=1025, 64 regions); even images all-coarse, odd all-fine."""
     sd = O.make_state_dict(128, 1, 2, img_size=512, seed=10)

@@ -10,6 +10,8 @@ struct AttnArgs {
     const void* k = nullptr; const void* v = nullptr;
     long long kv_bs = 0, kv_rs = 0, kv_hs = 0;
     void* out = nullptr; long long o_rs = 0, o_hs = 0;
+    long long o_terms = 0;              // fp32: > 0: out takes terms (f32_terms.cuh), o_rs and o_hs count bf16, and the terms of
+                                        // an element are o_terms apart
     int dtype = VTP_F32;
     int B = 0, n_keys = 0, heads = 0, head_dim = 0;
     const int32_t* offsets = nullptr;   // device int32 [B+1]

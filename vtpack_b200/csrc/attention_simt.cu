@@ -14,6 +14,7 @@
 // (vtpack/layers/csrc/batched_sparse_gemm/batched_sparse_gemm.cu:219-305): scale is applied
 // to Q K^T before the softmax exactly as the reference passes it as the GEMM alpha (:275).
 #include "attention.h"
+#include "f32_terms.cuh"
 #include "runtime.h"
 
 namespace vtp {
@@ -74,7 +75,7 @@ __global__ void __launch_bounds__(128, 2)
 attn_simt_kernel(const T* __restrict__ q, long long q_rs, long long q_hs, const T* __restrict__ k,
                  const T* __restrict__ v, long long kv_bs, long long kv_rs, long long kv_hs,
                  T* __restrict__ out, long long o_rs, long long o_hs, int n_keys, int n_chunks, int kc,
-                 const int32_t* __restrict__ offsets, int l_max, float scale, int* status) {
+                 const int32_t* __restrict__ offsets, int l_max, float scale, int* status, long long o_terms) {
     constexpr int AKC = 16 * AKJ, SPITCH = AKC + 4;      // chunk, row pitch of the probabilities
     pdl_begin();
     extern __shared__ float smem[];
@@ -215,6 +216,13 @@ attn_simt_kernel(const T* __restrict__ q, long long q_rs, long long q_hs, const 
         const int qi = ty * 4 + i;
         if (qi >= nq) continue;
         const float inv = 1.f / l[i];
+        if constexpr (sizeof(T) == 4) {
+            if (o_terms) {
+                const float v[4] = {o[i][0] * inv, o[i][1] * inv, o[i][2] * inv, o[i][3] * inv};
+                store_terms4(reinterpret_cast<bf16*>(out) + (long long)(row0 + qi) * o_rs + h * o_hs + tx * 4, (size_t)o_terms, v);
+                continue;
+            }
+        }
         T* p = out + (long long)(row0 + qi) * o_rs + h * o_hs + tx * 4;
 #pragma unroll
         for (int j = 0; j < 4; ++j) p[j] = from_f32<T>(o[i][j] * inv);
@@ -238,7 +246,7 @@ static int launch_simt_j(const AttnArgs& p, cudaStream_t st) {
     // a query tile never straddles images; images with fewer queries launch CTAs that exit
     launch_kernel(kern, false, 1, dim3(ceil_div(p.max_q, AQ), p.heads, p.B), dim3(128), (size_t)smem, st,
                   (const T*)p.q, p.q_rs, p.q_hs, (const T*)p.k, (const T*)p.v, p.kv_bs, p.kv_rs, p.kv_hs, (T*)p.out, p.o_rs,
-                  p.o_hs, p.n_keys, ceil_div(p.n_keys, kc), kc, p.offsets, p.l_max, p.scale, device_status_ptr());
+                  p.o_hs, p.n_keys, ceil_div(p.n_keys, kc), kc, p.offsets, p.l_max, p.scale, device_status_ptr(), p.o_terms);
     return check_launch("attention (CUDA cores)");
 }
 

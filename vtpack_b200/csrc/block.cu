@@ -33,12 +33,28 @@ struct BlockScratch {
     float2 *stats_x[2], *stats_q, *stats_acc;
     void *comp, *xn, *qn, *qp, *kv, *ao, *q1, *hid;
     void *sr_cols, *sr_out, *sr_norm;       // spatial reduction (PVT blocks): im2col rows, reduced tokens, their LayerNorm
+    void *q_wt, *kv_wt, *proj_wt, *fc1_wt, *fc2_wt, *sr_wt;     // the matrices as terms (block_terms)
     long long bytes;
 };
 
 // keys per image: the tokens, or the grid reduced by sr_ratio in each direction
 static int keys_per_image(const vtp_dge_shape& s) {
     return s.sr_ratio > 1 ? (s.H / s.sr_ratio) * (s.W / s.sr_ratio) : s.num_extra + s.H * s.W;
+}
+
+static RegionGeom region_geom(const vtp_dge_shape& s) {
+    RegionGeom g;
+    g.B = s.B; g.Hr = s.H / s.region; g.Wr = s.W / s.region; g.W = s.W; g.N = s.num_extra + s.H * s.W; g.C = s.C;
+    g.num_extra = s.num_extra; g.region = s.region;
+    return g;
+}
+
+// Whether the Linears of an fp32 block take their operands as terms (f32_terms.cuh): their inputs are written that way by the
+// kernels in front, and the matrices are split beside the pooling.
+static bool block_terms(const vtp_dge_shape& s) {
+    const long long reduced = (long long)s.B * s.H * s.W * s.C / 8;
+    return s.dtype == VTP_F32 && !(s.flags & VTP_FLAG_CUDA_CORES) && s.C % 8 == 0 && s.hidden % 8 == 0 && s.region > 0 &&
+           region_ops_supported(region_geom(s), s.dtype) && (s.sr_ratio <= 1 || reduced < (1ll << 32));
 }
 
 static BlockScratch carve_block(const vtp_dge_shape& s, void* ws) {
@@ -61,20 +77,32 @@ static BlockScratch carve_block(const vtp_dge_shape& s, void* ws) {
     b.stats_x[1] = (float2*)c.take(rows * 8);
     b.stats_q = (float2*)c.take(rows * 8);
     b.stats_acc = (float2*)c.take(rows * 8 * linear_stat_slots(s.C));
+    const bool terms = block_terms(s);
+    const long long et = terms ? 6 : e;     // of what a Linear reads
     b.comp = c.take(rows * s.C * e);
-    b.xn = c.take(rows * s.C * e);
-    b.qn = c.take(rows * s.C * e);
+    b.xn = c.take(rows * s.C * et);
+    b.qn = c.take(rows * s.C * et);
     b.qp = c.take(rows * s.C * e);
     b.kv = c.take(rows * 2 * s.C * e);
-    b.ao = c.take(rows * s.C * e);
+    b.ao = c.take(rows * s.C * et);
     b.q1 = c.take(rows * s.C * e);
-    b.hid = c.take(rows * s.hidden * e);
+    b.hid = c.take(rows * s.hidden * et);
     b.sr_cols = b.sr_out = b.sr_norm = nullptr;
     if (s.sr_ratio > 1) {
         const long long krows = (long long)s.B * keys_per_image(s);
-        b.sr_cols = c.take(rows * s.C * e);             // [B*keys, sr*sr*C] = as many elements as the tokens
+        b.sr_cols = c.take(rows * s.C * et);            // [B*keys, sr*sr*C] = as many elements as the tokens
         b.sr_out = c.take(krows * s.C * e);
-        b.sr_norm = c.take(krows * s.C * e);
+        b.sr_norm = c.take(krows * s.C * et);
+    }
+    b.q_wt = b.kv_wt = b.proj_wt = b.fc1_wt = b.fc2_wt = b.sr_wt = nullptr;
+    if (terms) {
+        const long long cc = (long long)s.C * s.C * 6, ch = (long long)s.C * s.hidden * 6;
+        b.q_wt = c.take(cc);
+        b.kv_wt = c.take(2 * cc);
+        b.proj_wt = c.take(cc);
+        b.fc1_wt = c.take(ch);
+        b.fc2_wt = c.take(ch);
+        if (s.sr_ratio > 1) b.sr_wt = c.take(cc * s.sr_ratio * s.sr_ratio);
     }
     b.bytes = c.off;
     return b;
@@ -117,13 +145,6 @@ static bool has_folded_weights(const vtp_block_weights& w) {
 
 static bool has_folded_q_fc1(const vtp_block_weights& w) {
     return w.q_wf && w.q_s && w.q_c && w.fc1_wf && w.fc1_s && w.fc1_c;
-}
-
-static RegionGeom region_geom(const vtp_dge_shape& s) {
-    RegionGeom g;
-    g.B = s.B; g.Hr = s.H / s.region; g.Wr = s.W / s.region; g.W = s.W; g.N = s.num_extra + s.H * s.W; g.C = s.C;
-    g.num_extra = s.num_extra; g.region = s.region;
-    return g;
 }
 
 // Whether a block of this shape runs with norm1 folded into q and norm2 into fc1 (bf16 tensor-core path,
@@ -208,6 +229,16 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
     // chained: gate decisions, per-image counts and token statistics came from the previous
     // block's unpool; the pool kernel then also derives the row offsets itself
     const bool chained = chain.have_gate && by_region && !forced_logits;
+    const bool terms = block_terms(s);
+    if (terms)
+        VTP_REQUIRE(aligned16(w.q_w) && aligned16(w.kv_w) && aligned16(w.proj_w) && aligned16(w.fc1_w) && aligned16(w.fc2_w) &&
+                        aligned16(w.sr_w), VTP_ERR_ALIGN, "block: matrices must be 16-byte aligned");
+    auto run_linear = [&](LinearArgs& p, const void* w_terms, bool out_terms) {
+        if (!terms) return linear(p, st);
+        p.w = w_terms;
+        p.out_terms = out_terms;
+        return linear_f32_terms(p, st);
+    };
     const bool derive = by_region && (chained || pool_derives_rows(s.B, Hr * Wr, chain.counts_started));
     VTP_REQUIRE(!chain.image_bias || by_region, VTP_ERR_UNSUPPORTED,
                 "block: a per-image gate bias needs the region-parallel gate (4x4-token regions)");
@@ -251,6 +282,16 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
             if (reduce) { pa.sr = s.sr_ratio; pa.cols = b.sr_cols; pa.lnw = w.norm1_w; pa.lnb = w.norm1_b; }
         }
         else { pa.lnw = w.norm1_w; pa.lnb = w.norm1_b; pa.xn = b.xn; pa.qn = b.qn; }
+        if (terms) {
+            pa.qn_terms = true;
+            pa.xn_terms = !reduce;           // (the gather of a reduction splits its rows itself)
+            pa.split.add(w.q_w, b.q_wt, C, C);
+            pa.split.add(w.kv_w, b.kv_wt, 2 * C, C);
+            pa.split.add(w.proj_w, b.proj_wt, C, C);
+            pa.split.add(w.fc1_w, b.fc1_wt, s.hidden, C);
+            pa.split.add(w.fc2_w, b.fc2_wt, C, s.hidden);
+            if (reduce) pa.split.add(w.sr_w, b.sr_wt, C, s.sr_ratio * s.sr_ratio * C);
+        }
         rc = region_pool(pa, s.dtype, st);
     } else {
         rc = vtp_pool(x_in, s.dtype, s.B, N, C, s.W, s.num_extra, b.patches, L_dev, rows, b.comp, w.norm1_w,
@@ -265,16 +306,18 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
 
     const void* keys_in = fold ? x_in : b.xn;
     if (reduce) {
-        if ((rc = linear(lq, st)) || (rc = marks.mark(4))) return rc;
+        if ((rc = run_linear(lq, b.q_wt, false)) || (rc = marks.mark(4))) return rc;
         // x_ = norm(sr(LN1(x) as [B,C,H,W])): the stride-sr convolution as im2col rows times a matrix
         const int krows = s.B * n_keys, KS = s.sr_ratio * s.sr_ratio * C;
-        if (!fold_q) rc = token_im2col(b.xn, s.dtype, s.B, s.H, s.W, C, s.sr_ratio, b.sr_cols, st);
+        if (terms) rc = token_im2col_terms(b.xn, s.B, s.H, s.W, C, s.sr_ratio, b.sr_cols, st);
+        else if (!fold_q) rc = token_im2col(b.xn, s.dtype, s.B, s.H, s.W, C, s.sr_ratio, b.sr_cols, st);
         if (rc) return rc;
         LinearArgs lsr;
         lsr.a = b.sr_cols; lsr.lda = KS; lsr.w = w.sr_w; lsr.bias = w.sr_b; lsr.y = b.sr_out; lsr.ldy = C;
         lsr.dtype = s.dtype; lsr.m_max = krows; lsr.N = C; lsr.K = KS; lsr.flags = kflag;
-        if ((rc = linear(lsr, st))) return rc;
-        rc = vtp_layernorm(b.sr_out, s.dtype, krows, nullptr, C, C, w.sr_norm_w, w.sr_norm_b, s.sr_eps, b.sr_norm, st);
+        if ((rc = run_linear(lsr, b.sr_wt, false))) return rc;
+        rc = terms ? layernorm_terms(b.sr_out, krows, nullptr, C, w.sr_norm_w, w.sr_norm_b, s.sr_eps, b.sr_norm, st)
+                   : vtp_layernorm(b.sr_out, s.dtype, krows, nullptr, C, C, w.sr_norm_w, w.sr_norm_b, s.sr_eps, b.sr_norm, st);
         if (rc) return rc;
         keys_in = b.sr_norm;
     }
@@ -286,8 +329,8 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
         // the two projections do not depend on each other: one launch, the q tiles fill the kv tail
         if ((rc = linear_tcgen05_pair(lkv, lq, st))) return rc;
     } else {
-        if (!reduce && ((rc = linear(lq, st)) || (rc = marks.mark(4)))) return rc;
-        if ((rc = linear(lkv, st)) || (rc = marks.mark(5))) return rc;
+        if (!reduce && ((rc = run_linear(lq, b.q_wt, false)) || (rc = marks.mark(4)))) return rc;
+        if ((rc = run_linear(lkv, b.kv_wt, false)) || (rc = marks.mark(5))) return rc;
     }
 
     AttnArgs at;
@@ -295,7 +338,8 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
     at.q = b.qp; at.q_rs = C; at.q_hs = d;
     at.k = b.kv; at.v = static_cast<const char*>(b.kv) + (long long)C * e;
     at.kv_bs = (long long)n_keys * 2 * C; at.kv_rs = 2 * C; at.kv_hs = d;
-    at.out = b.ao; at.o_rs = C; at.o_hs = d;
+    at.out = b.ao; at.o_rs = terms ? 3 * C : C; at.o_hs = d;
+    at.o_terms = terms ? C : 0;
     at.dtype = s.dtype; at.B = s.B; at.n_keys = n_keys; at.heads = s.heads; at.head_dim = d;
     at.offsets = b.offsets; at.l_max = rows; at.max_q = N; at.scale = attn_scale(s); at.flags = kflag;
     if ((rc = attention(at, st)) || (rc = marks.mark(6))) return rc;
@@ -304,10 +348,11 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
     lp.a = b.ao; lp.lda = C; lp.w = w.proj_w; lp.bias = w.proj_b; lp.res = b.comp; lp.ldr = C; lp.y = b.q1;
     lp.ldy = C; lp.dtype = s.dtype; lp.m_max = rows; lp.m_dev = L_dev; lp.N = C; lp.K = C; lp.flags = kflag;
     if (fold_fc1) lp.emit_stats = b.stats_acc;
-    if ((rc = linear(lp, st)) || (rc = marks.mark(7))) return rc;
+    if ((rc = run_linear(lp, b.proj_wt, false)) || (rc = marks.mark(7))) return rc;
 
     if (!fold_fc1) {
-        rc = vtp_layernorm(b.q1, s.dtype, rows, L_dev, C, C, w.norm2_w, w.norm2_b, s.eps, b.qn, st);
+        rc = terms ? layernorm_terms(b.q1, rows, L_dev, C, w.norm2_w, w.norm2_b, s.eps, b.qn, st)
+                   : vtp_layernorm(b.q1, s.dtype, rows, L_dev, C, C, w.norm2_w, w.norm2_b, s.eps, b.qn, st);
         if (rc) return rc;
     }
     if ((rc = marks.mark(8))) return rc;
@@ -318,12 +363,12 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
     l1.flags = kflag | VTP_FLAG_GELU;
     if (fold_fc1) { l1.ln_mode = 2; l1.ln_stats = b.stats_acc; l1.ln_s = w.fc1_s; l1.ln_dim = C; l1.ln_eps = s.eps;
                 l1.ln_slots = linear_stat_slots(C); }
-    if ((rc = linear(l1, st)) || (rc = marks.mark(9))) return rc;
+    if ((rc = run_linear(l1, b.fc1_wt, true)) || (rc = marks.mark(9))) return rc;
 
     LinearArgs l2;   // q2 = q1 + hid W2^T + b   (into the q-projection buffer, dead by now)
     l2.a = b.hid; l2.lda = s.hidden; l2.w = w.fc2_w; l2.bias = w.fc2_b; l2.res = b.q1; l2.ldr = C; l2.y = b.qp;
     l2.ldy = C; l2.dtype = s.dtype; l2.m_max = rows; l2.m_dev = L_dev; l2.N = C; l2.K = s.hidden; l2.flags = kflag;
-    if ((rc = linear(l2, st)) || (rc = marks.mark(10))) return rc;
+    if ((rc = run_linear(l2, b.fc2_wt, false)) || (rc = marks.mark(10))) return rc;
 
     if (by_region) {
         RegionUnpoolArgs ua;

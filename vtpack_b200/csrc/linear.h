@@ -34,6 +34,8 @@ struct LinearArgs {
     // stores, so the result does not depend on timing, nor, the columns being added in a fixed order, on the tiles.
     // Slots of a row are linear_stat_slots(N) apart (an even number, for the consumer's 16-byte loads).
     float2* emit_stats = nullptr;
+    // fp32 only: y takes the three bf16 terms of every row, [3][N], instead of fp32 values (f32_terms.cuh).
+    bool out_terms = false;
 };
 
 int linear_stat_slots(int N);              // float2 slots a tcgen05 GEMM with N output columns takes per row
@@ -45,9 +47,21 @@ int linear_cuda_cores(const LinearArgs& p, cudaStream_t st);   // fp32 or bf16 i
 int linear_tcgen05(const LinearArgs& p, cudaStream_t st);      // bf16 inputs, tcgen05 + TMA
 bool linear_f32_tc_supported(const LinearArgs& p);
 int linear_f32_tcgen05(const LinearArgs& p, cudaStream_t st);  // fp32 inputs as three bf16 terms each, tcgen05
+int linear_f32_terms(const LinearArgs& p, cudaStream_t st);    // fp32 with a and w as rows of terms (f32_terms.cuh), lda unused
 int linear(const LinearArgs& p, cudaStream_t st);              // picks by dtype / flags
 bool linear_pair_supported(const LinearArgs& a, const LinearArgs& b);
 int linear_tcgen05_pair(const LinearArgs& a, const LinearArgs& b, cudaStream_t st);   // two problems, one launch
+
+// Unsigned division by a number the host knows: multiply by ceil(2^32 / d), then take back the one the estimate may
+// be over (it is never under).  A runtime division is about forty dependent instructions on the way to a CTA's first load.
+struct FastDiv { uint32_t d, magic; };
+inline FastDiv make_fast_div(uint32_t d) { return FastDiv{d, d == 1 ? 0u : (uint32_t)(((1ull << 32) + d - 1) / d)}; }
+__device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv& f) {
+    if (f.d == 1) return n;
+    uint32_t q = __umulhi(n, f.magic);
+    if (q * f.d > n) --q;          // (n and d are below 2^31)
+    return q;
+}
 
 struct RowMap { int out_grp, out_skip, res_mod, res_off; };
 __device__ __forceinline__ long long map_out_row(const RowMap& r, int m) {

@@ -39,8 +39,11 @@
 // NaN or finite where that chain's are.  The check is one fmaf per output.
 //
 // Replaces nn.Linear q/kv/proj/fc1/fc2/head, nn.GELU and the residual adds of
-// vtpack/models/dge/deit_dge.py:38-44,72-74,96,127-128 when the model runs in fp32.
+// vtpack/models/dge/deit_dge.py:38-44,72-74,96,127-128 in fp32, where the operands are fp32 rows: single Linears, patch embedding,
+// head and dense blocks.  The Linears of DGE blocks are linear_f32_terms.cu.
+#include "f32_terms.cuh"
 #include "linear.h"
+#include "linear_f32.cuh"
 #include "runtime.h"
 #include "sm100.cuh"
 
@@ -48,15 +51,11 @@ namespace vtp {
 
 using namespace sm100;
 
-constexpr int FM = 128;                 // tile rows = TMEM lanes
-constexpr int FK = 64;                  // k-block: one 128-byte row of bf16 per operand term
 constexpr int F_EPI = 256;              // epilogue threads
 // Converter warps: as many as the registers of an SM allow beside the tile's accumulators.  (Eight measured the
 // same: the port is the bound, see above.)
 constexpr int conv_warps(int bn) { return bn == 128 ? 11 : 15; }
 constexpr int F_STAGES = 2;
-constexpr float F_SCALE = 65536.f, F_UNSCALE = 1.f / (65536.f * 65536.f);     // of an operand, of a sum of products
-constexpr int F_TMEM = 4;              // in tile widths: two accumulators, two group sums
 
 template <int BN>
 struct F32Smem {
@@ -83,9 +82,7 @@ __device__ __forceinline__ void ldg_f8(const float* p, float4& lo, float4& hi) {
                  : "l"(p));
 }
 
-// Eight fp32 values -> the three bf16 terms, packed eight to 16 bytes.  h is rounded to nearest (half away), so what
-// is left over has either sign and the products that are left out do not add up; m and l cut the rest in two.
-// All exact (the products with F_SCALE too, up to the largest number), in integer and fp32 adds and byte permutes (the bf16 conversion instruction has a fraction of their rate).
+// Eight fp32 values -> the three bf16 terms, packed eight to 16 bytes.
 __device__ __forceinline__ void split8(const float4& x0, const float4& x1, uint4 (&t)[3]) {
     const float v[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
     uint32_t w[3][4];
@@ -93,13 +90,7 @@ __device__ __forceinline__ void split8(const float4& x0, const float4& x1, uint4
     for (int i = 0; i < 4; ++i) {
         uint32_t h[2], m[2], l[2];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const float x = v[2 * i + j] * F_SCALE;
-            h[j] = (__float_as_uint(x) + 0x8000u) & 0xFFFF0000u;
-            const float r = x - __uint_as_float(h[j]);
-            m[j] = __float_as_uint(r) & 0xFFFF0000u;
-            l[j] = __float_as_uint(r - __uint_as_float(m[j]));
-        }
+        for (int j = 0; j < 2; ++j) split_scaled(v[2 * i + j] * F_SCALE, h[j], m[j], l[j]);
         w[0][i] = __byte_perm(h[0], h[1], 0x7632);       // the upper halves of both: element 2 i in the low half
         w[1][i] = __byte_perm(m[0], m[1], 0x7632);
         w[2][i] = __byte_perm(l[0], l[1], 0x7632);
@@ -141,36 +132,6 @@ __device__ __forceinline__ void unscale_or_redo(float (&acc)[NC], const F32Args&
                 if (lane == r) acc[c0 + i] = v;
             }
         }
-    }
-}
-
-// Groups of k-blocks that are added up apart: at least three k-blocks each.  More splits would leave a CTA less work
-// than the exchange costs.
-static int f32_groups_log2(int num_kb) { return num_kb >= 12 ? 2 : num_kb >= 6 ? 1 : 0; }
-
-// acc (op) a sum kept in tensor memory, 32 columns at a time
-template <int CW>
-__device__ __forceinline__ void stash_store(uint32_t taddr, const float (&acc)[CW]) {
-    __syncwarp();
-#pragma unroll
-    for (int c0 = 0; c0 < CW; c0 += 16) {
-        uint32_t r[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(acc[c0 + i]);
-        tmem_st_32x16(taddr + c0, r);
-    }
-    tmem_st_wait();
-}
-template <int CW>
-__device__ __forceinline__ void stash_add(uint32_t taddr, float (&acc)[CW]) {
-#pragma unroll
-    for (int c0 = 0; c0 < CW; c0 += 32) {
-        uint32_t r[32];
-        __syncwarp();
-        tmem_ld_32x32(taddr + c0, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) acc[c0 + i] += __uint_as_float(r[i]);
     }
 }
 

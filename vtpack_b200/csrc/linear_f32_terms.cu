@@ -1,0 +1,538 @@
+// fp32 Linear on tcgen05 tensor cores with operands that arrive as terms (f32_terms.cuh), for the blocks of fp32 models.
+//
+//   y[m, n] = act(sum_k a[m,k] w[n,k] + bias[n]) + res[m, n]
+//
+// The products and sums are those of linear_f32_tc.cu, in the same order, so a row's bits are the same: six bf16 products of
+// terms per k-block of 64, smallest first, a fresh TMEM accumulator for each k-block, k-blocks added in fp32 registers in one,
+// two or four groups that K alone decides, sums that come out infinite or NaN worked out again from the decoded operands.
+// There every CTA splits the rows it multiplies: a row of the weights once per 128 rows of the batch, a row of the batch once per
+// 64 columns, and the splitting bounds it.  Here the kernels that produce the operands leave terms, once, and TMA brings them.
+//
+// Persistent, one CTA per SM, 128 x BN tiles:
+//   warp 0        (one lane) TMA: the three terms of a k-block of a and of w, two stages; a product starts when its own two have
+//                 landed
+//   warp 1        (one lane) issues the MMAs into one of two TMEM accumulators, one per k-block
+//   16 warps      one per TMEM lane quarter and quarter of the columns: add finished accumulators to their registers; after the last
+//                 k-block bias / GELU / residual, 64 bytes of a row per store through a per-warp transpose buffer
+// A long reduction with few tiles is split over the CTAs of a cluster as in linear_f32_tc.cu.
+#include <string.h>
+
+#include "f32_terms.cuh"
+#include "linear.h"
+#include "linear_f32.cuh"
+#include "runtime.h"
+
+namespace vtp {
+
+constexpr int FT_EPI_WARPS = 16, FT_FIRST_EPI = 2, FT_THREADS = (FT_FIRST_EPI + FT_EPI_WARPS) * 32;
+constexpr int FT_STAGES = 2;
+constexpr int FT_OUT = 32 * 64;          // bytes of a warp's transpose buffer: 32 rows x 16 fp32 columns
+
+template <int BN>
+struct FtSmem {
+    static constexpr int A_TERM = FM * FK * 2, B_TERM = BN * FK * 2;
+    static constexpr int STAGE = 3 * (A_TERM + B_TERM);
+    static constexpr int USED = FT_STAGES * STAGE + FT_EPI_WARPS * FT_OUT + 256;
+    static constexpr int TOTAL = USED + 1024;                   // the operand tiles want 1024-byte alignment
+    static_assert(TOTAL <= 232448, "shared memory budget");
+};
+
+struct FtArgs {
+    const bf16* a; const bf16* w; const float* bias; const float* res; long long ldr;
+    float* y; long long ldy;
+    const int32_t* m_dev; int m_max, N, K, groups_log2;
+    FastDiv n_tiles, step;               // column tiles of a row of tiles, CTAs (clusters) of the grid
+};
+// a [m_max][3][K], w [N][3][K] as maps {K, 3, rows} with boxes of 64 elements of one term of a tile's rows; w also in boxes of half
+// and of a quarter of a tile's columns.
+struct FtMaps { CUtensorMap a, w[3]; };
+
+// The work items of a CTA (SPLIT of a cluster), in order: tiles first, first + step, ...; where they are cut, the tiles of the
+// last, partial round are two or four column strips, one per CTA, so that it takes a fraction of a tile's time.
+// (A row's bits do not depend on it: a column's sums are the same in any tile.)
+template <int BN>
+struct FtItems {
+    FastDiv n_tiles;
+    uint32_t full, strips, step, first;
+    int cut;                                     // log2 of the strips of a tile
+    __device__ __forceinline__ FtItems(uint32_t total, const FtArgs& g, uint32_t first_, bool strips_pay) : n_tiles(g.n_tiles), step(g.step.d), first(first_) {
+        full = !strips_pay ? total : total < step ? 0 : fast_div(total, g.step) * step;
+        const uint32_t rest = total - full;
+        cut = BN == 128 && rest * 4 <= step ? 2 : rest * 2 <= step ? 1 : 0;
+        strips = rest << cut;
+    }
+    // (a strip beyond the columns of a narrow tile is an item like any other: its sums are not stored)
+    struct Item { int mt, n0, cut; };            // row of tiles, first column, log2 of BN / columns
+    __device__ __forceinline__ bool at(uint32_t j, Item& it) const {
+        uint32_t tile = first + j * step, sub = 0;
+        it.cut = 0;
+        if (tile >= full) {
+            const uint32_t u = tile - full;
+            if (u >= strips) return false;
+            tile = full + (u >> cut);
+            sub = u & ((1u << cut) - 1);
+            it.cut = cut;
+        }
+        const uint32_t mt = fast_div(tile, n_tiles);
+        it.mt = (int)mt;
+        it.n0 = (int)(tile - mt * n_tiles.d) * BN + (int)sub * (BN >> it.cut);
+        return true;
+    }
+};
+
+// Where the terms of a k-block lie: two sets of three slots for a and three for w, which k-blocks take in turn.  Terms are read for
+// the last time in the order l, m, h but needed in the order (l, h), (h, l), (m, m): the next k-block of a set takes each slot as
+// it falls free, so that its loads are spread over the products of the one before and each is under way for the time of
+// eight products or more.
+struct FtSlots {
+    int a[3] = {0, 1, 2}, b[3] = {0, 1, 2};      // of h, m, l
+    // sets[0] becomes the other set's, sets[1] this one's for its next k-block: a's l stays, its h goes where m was, m where h was; w's h
+    // goes where l was, its l where m was, m where h was
+    static __device__ __forceinline__ void next(FtSlots (&sets)[2]) {
+        const FtSlots s = sets[0];
+        sets[0] = sets[1];
+        sets[1].a[0] = s.a[1]; sets[1].a[1] = s.a[0]; sets[1].a[2] = s.a[2];
+        sets[1].b[0] = s.b[2]; sets[1].b[1] = s.b[0]; sets[1].b[2] = s.b[1];
+    }
+};
+
+__device__ __forceinline__ float term_at(const bf16* row, int K, int k) {
+    const unsigned short* t = reinterpret_cast<const unsigned short*>(row) + k;
+    return join_terms(__ldg(t), __ldg(t + K), __ldg(t + 2 * (size_t)K));
+}
+// acc: NC columns n0.. of row m0 + lane, sums of scaled products, which are scaled back.  Rows with a sum that is not finite are
+// worked out again as an fmaf chain, a row at a time, a lane per column (see linear_f32_tc.cu).
+template <int NC>
+__device__ __forceinline__ void unscale_or_redo(float (&acc)[NC], const FtArgs& g, int M, int m0, int n0, int lane) {
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+        t = fmaf(acc[i], 0.f, t);              // inf * 0 and NaN * 0 are NaN
+        acc[i] *= F_UNSCALE;
+    }
+    unsigned bad = __ballot_sync(0xffffffffu, t != t && m0 + lane < M);
+    while (bad) {
+        const int r = __ffs(bad) - 1;
+        bad &= bad - 1;
+        const bf16* a = g.a + (size_t)(m0 + r) * 3 * g.K;
+        static_assert(NC <= 32, "a lane per column");
+        const int n = n0 + lane;
+        float s = 0.f;
+        if (lane < NC && n < g.N) {
+            const bf16* w = g.w + (size_t)n * 3 * g.K;
+#pragma unroll 1
+            for (int k = 0; k < g.K; ++k) s = fmaf(term_at(a, g.K, k), term_at(w, g.K, k), s);
+        }
+#pragma unroll
+        for (int i = 0; i < NC; ++i) {
+            const float v = __shfl_sync(0xffffffffu, s, i);
+            if (lane == r) acc[i] = v;
+        }
+    }
+}
+
+// Four output columns of row m from column n on, N and n multiples of four.  HIDDEN: GELU, stored as terms; else + res, as fp32.
+template <bool HIDDEN>
+__device__ __forceinline__ void finish4(const FtArgs& g, int m, int n, const float4& s, const float4& bias, const float4& res) {
+    float v[4] = {s.x + bias.x, s.y + bias.y, s.z + bias.z, s.w + bias.w};
+    if (HIDDEN) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = gelu_erf(v[i]);
+        store_terms4(reinterpret_cast<bf16*>(g.y) + (size_t)m * 3 * g.N + n, (size_t)g.N, v);
+    } else {
+        if (g.res) { v[0] += res.x; v[1] += res.y; v[2] += res.z; v[3] += res.w; }
+        *reinterpret_cast<float4*>(g.y + (size_t)m * g.ldy + n) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+}
+
+// SPLIT: CTAs of a cluster that share a tile's reduction (1: none); it divides the number of groups.
+template <int BN, int SPLIT, bool HIDDEN>
+__global__ void __launch_bounds__(FT_THREADS, 1)
+linear_f32_terms_kernel(const __grid_constant__ FtMaps maps, const __grid_constant__ FtArgs g, int* status) {
+    using S = FtSmem<BN>;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint64_t* bars = reinterpret_cast<uint64_t*>(base + FT_STAGES * S::STAGE + FT_EPI_WARPS * FT_OUT);
+    uint64_t* full = bars;                        // [2][3] per set of slots: the terms of the first product have landed, those of the
+                                                  //     second, the other two (FtSlots)
+    uint64_t* empty = bars + 6;                   // [2][3] the slots that these go to have been read
+    uint64_t* acc_full = bars + 12;               // [2]
+    uint64_t* acc_empty = bars + 14;              // [2]
+    uint64_t* part_full = bars + 16;              // the other CTAs' partial sums of this CTA's columns have arrived
+    uint64_t* part_free = bars + 17;              // the other CTAs have added the ones this CTA sent them
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* void_s = reinterpret_cast<int*>(tmem_slot + 2);   // [2] launch_is_void in front of the wait and behind it
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 6; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&acc_full[i], 1);
+            mbar_init(&acc_empty[i], FT_EPI_WARPS);
+        }
+        mbar_init(part_full, 1);
+        mbar_init(part_free, SPLIT > 1 ? (SPLIT - 1) * FT_EPI_WARPS : 1);
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (warp == 1) {
+        tmem_alloc(tmem_slot, F_TMEM * BN);
+        tmem_relinquish();
+    }
+    if (warp == FT_FIRST_EPI && elect_one()) {
+        prefetch_tmap(&maps.a);
+        for (int i = 0; i < 3; ++i) prefetch_tmap(&maps.w[i]);
+    }
+    // (parameters are cold in every launch, each line of them is a miss: not on the way to the first load)
+    if (warp == FT_FIRST_EPI + 2 && lane < (int)(sizeof(FtArgs) / 4))
+        asm volatile("" ::"r"(reinterpret_cast<const uint32_t*>(&g)[lane]));
+    if (threadIdx.x == (FT_FIRST_EPI + 1) * 32) void_s[0] = launch_is_void(status) ? 1 : 0;
+    tc_fence_before_sync();
+    __syncthreads();
+    if (SPLIT > 1) cluster_sync_all();            // the partners' barriers exist
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+    const bool known_void = lead_word<SPLIT>(void_s) != 0;
+    pdl_begin();
+
+    int M = g.m_max;
+    if (g.m_dev) M = min(max(*reinterpret_cast<const volatile int32_t*>(g.m_dev), 0), M);
+    const uint32_t total = known_void ? 0 : (uint32_t)((M + FM - 1) / FM) * g.n_tiles.d;
+    const int rank = SPLIT > 1 ? (int)cluster_ctarank() : 0;
+    const int all_kb = (g.K + FK - 1) / FK;
+    const int kb0 = all_kb * rank / SPLIT, num_kb = all_kb * (rank + 1) / SPLIT - kb0;    // this CTA's k-blocks
+    const FtItems<BN> items(total, g, blockIdx.x / SPLIT, SPLIT == 1);
+    // (term of a, term of w) of the products, smallest first; the first three bring every term once
+    constexpr int TA[6] = {2, 0, 1, 1, 0, 0}, TB[6] = {0, 2, 1, 0, 1, 0};
+    FtSlots sets[2];
+    typename FtItems<BN>::Item wi;
+    int it = 0;                                   // k-blocks so far
+    bool ok = true;
+
+    if (warp == 0) {
+        if (elect_one()) {
+            // ------------------------------------------------------------ TMA producer
+            const uint32_t sbase = smem_u32(base);
+            for (uint32_t j = 0; ok && items.at(j, wi); ++j) {
+                const CUtensorMap* wmap = &maps.w[wi.cut];
+                const uint32_t b_term = S::B_TERM >> wi.cut;
+                for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                    const int s = it & 1;
+                    const FtSlots& in = sets[0];
+                    const uint32_t sa = sbase + s * S::STAGE, sb = sa + 3 * S::A_TERM;
+                    const int k = (kb0 + kb) * FK;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        ok = mbar_wait(&empty[3 * s + c], ((it >> 1) & 1) ^ 1, abort_flag, status, STATUS_GEMM_PRODUCER);
+                        if (!ok) break;
+                        const uint32_t bar = smem_u32(&full[3 * s + c]);
+                        mbar_arrive_expect_tx_a(bar, S::A_TERM + b_term);
+                        tma_load_3d_a(sa + in.a[TA[c]] * S::A_TERM, &maps.a, bar, k, TA[c], wi.mt * FM);
+                        tma_load_3d_a(sb + in.b[TB[c]] * S::B_TERM, wmap, bar, k, TB[c], wi.n0);
+                    }
+                    if (!ok) break;
+                    FtSlots::next(sets);
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (elect_one()) {
+            // -------------------------------------------------------------- MMA issuer
+            const uint32_t sbase = smem_u32(base);
+            for (uint32_t j = 0; ok && items.at(j, wi); ++j) {
+                const uint32_t idesc = idesc_bf16_f32(FM, BN >> wi.cut, 0, 0);
+                for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                    const int s = it & 1;
+                    const uint32_t ph = (it >> 1) & 1;
+                    ok = mbar_wait(&acc_empty[s], ph ^ 1, abort_flag, status, STATUS_GEMM_MMA);
+                    if (!ok) break;
+                    const FtSlots& in = sets[0];
+                    const uint32_t sa = sbase + s * S::STAGE, sb = sa + 3 * S::A_TERM;
+#pragma unroll
+                    for (int c = 0; c < 6; ++c) {
+                        if (c < 3) {
+                            ok = mbar_wait(&full[3 * s + c], ph, abort_flag, status, STATUS_GEMM_MMA);
+                            if (!ok) break;
+                            tc_fence_after_sync();
+                        }
+                        const uint64_t ad = smem_desc_sw128(sa + in.a[TA[c]] * S::A_TERM);
+                        const uint64_t bd = smem_desc_sw128(sb + in.b[TB[c]] * S::B_TERM);
+#pragma unroll
+                        for (int k = 0; k < FK / 16; ++k)
+                            umma_ss(tmem_base + s * BN, ad + 2 * k, bd + 2 * k, idesc, (c | k) != 0 ? 1u : 0u);
+                        // l of both has been read; m of both; h
+                        if (c == 1 || c >= 4) umma_commit(&empty[3 * s + (c == 1 ? 0 : c - 3)]);
+                    }
+                    if (!ok) break;
+                    umma_commit(&acc_full[s]);
+                    FtSlots::next(sets);
+                }
+            }
+        }
+        __syncwarp();
+    } else {
+        // ------------------------------------------------------------------- epilogue
+        constexpr int CW = BN / 4;                       // columns of a warp
+        const int ew = warp - FT_FIRST_EPI;
+        const int quarter = warp & 3;                    // TMEM lane quarter this warp may read
+        const int col = (ew >> 2) * CW;                  // its first column of an item
+        const uint32_t tacc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + col;
+        const uint32_t stage = smem_u32(base + FT_STAGES * S::STAGE) + ew * FT_OUT;
+        const int own_groups = (1 << g.groups_log2) / SPLIT;         // this CTA's: 1, 2 or 4
+        const uint32_t tsum = tacc + 2 * BN;             // sums of its earlier groups: 0 (+ 1), and 2
+        const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        // in a launch that turns out to be void the sums still change hands, but this CTA has no rows to store
+        if (threadIdx.x == FT_FIRST_EPI * 32) void_s[1] = launch_is_void(status) ? 1 : 0;
+        named_barrier(1, FT_EPI_WARPS * 32);
+        if (void_s[1] != 0) M = 0;
+        int n_sent = 0;                                   // exchanges
+        for (uint32_t j = 0; ok && items.at(j, wi); ++j) {
+            const int m0 = wi.mt * FM + quarter * 32, n0 = wi.n0 + col;
+            const bool has = col < (BN >> wi.cut);        // a strip leaves some warps without columns
+            // What an output needs besides its sum travels while the operands are loaded and multiplied.  SPLIT: SC columns of row
+            // `lane`, else of every sixteen columns four of rows lane / 4 + 8 q.
+            constexpr int SC = CW / SPLIT;
+            constexpr int NV = SPLIT > 1 ? SC / 4 : CW / 4;
+            float4 res[HIDDEN ? 1 : NV], bias[SPLIT > 1 ? NV : CW / 16];
+            auto col_of = [&](int v) { return SPLIT > 1 ? n0 + rank * SC + 4 * v : n0 + (v >> 2) * 16 + (lane & 3) * 4; };
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                const int m = SPLIT > 1 ? m0 + lane : m0 + (v & 3) * 8 + (lane >> 2), n = col_of(v);
+                if (!HIDDEN) res[v] = g.res && has && m < M && n < g.N ? *reinterpret_cast<const float4*>(g.res + (size_t)m * g.ldr + n) : zero4;
+                if (SPLIT > 1 || (v & 3) == 0)
+                    bias[SPLIT > 1 ? v : v >> 2] = g.bias && has && n < g.N ? __ldg(reinterpret_cast<const float4*>(g.bias + n)) : zero4;
+            }
+            float acc[CW];
+#pragma unroll
+            for (int i = 0; i < CW; ++i) acc[i] = 0.f;
+            int grp = 0;
+            for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                const int s = it & 1;
+                ok = mbar_wait_warp(&acc_full[s], (it >> 1) & 1, abort_flag, status, STATUS_GEMM_EPILOGUE);
+                if (!ok) break;
+                tc_fence_after_sync();
+                if (has) stash_add<CW, 16>(tacc + s * BN, acc);
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_empty[s]);
+                if constexpr (SPLIT < 4) {
+                    // the CTA has one group, or this k-block does not end one
+                    if (own_groups == 1 || kb + 1 != (all_kb * (rank * own_groups + grp + 1) >> g.groups_log2) - kb0) continue;
+                    if (grp & 1) stash_add<CW, 16>(tsum + (SPLIT == 1 ? (grp >> 1) * BN : 0), acc);
+                    if (SPLIT == 1 && grp == 3) stash_add<CW, 16>(tsum, acc);            // (0 + 1) + (2 + 3)
+                    if (++grp == own_groups) continue;
+                    stash_store<CW>(tsum + (SPLIT == 1 && grp == 3 ? BN : 0), acc);
+#pragma unroll
+                    for (int i = 0; i < CW; ++i) acc[i] = 0.f;
+                }
+            }
+            if (!ok) break;
+            if constexpr (SPLIT > 1) {
+                // every CTA of the cluster finishes SC of this warp's columns: the others' partial sums of them come
+                // through distributed shared memory (one slot per source CTA in the transpose buffers), 512
+                // consecutive bytes per store
+                constexpr int ROUNDS = (SPLIT - 1) * SC * 128 > FT_OUT ? 2 : 1, XC = SC / ROUNDS;     // what the slots hold
+                static_assert((SPLIT - 1) * XC * 128 <= FT_OUT && XC % 4 == 0, "the exchange fits the warp's transpose buffer");
+                float own[SC];
+                typename FtItems<BN>::Item next;
+#pragma unroll
+                for (int d = 0; d < SPLIT; ++d)                   // (a runtime index would put acc into local memory)
+                    if (d == rank) {
+#pragma unroll
+                        for (int i = 0; i < SC; ++i) own[i] = acc[d * SC + i];
+                    }
+#pragma unroll
+                for (int x = 0; x < ROUNDS; ++x, ++n_sent) {
+                    if (n_sent > 0) ok = mbar_wait_cluster_warp(part_free, (n_sent - 1) & 1, abort_flag, status, STATUS_GEMM_EPILOGUE);
+                    if (!ok) break;
+#pragma unroll
+                    for (int d = 0; d < SPLIT; ++d) {
+                        if (d == rank) continue;
+                        const uint32_t dst = mapa_u32(stage, d) + (rank < d ? rank : rank - 1) * (XC * 128) + lane * 16;
+                        const uint32_t bar = mapa_u32(smem_u32(part_full), d);
+#pragma unroll
+                        for (int i = 0; i < XC / 4; ++i) {
+                            const int c = d * SC + x * XC + 4 * i;
+                            stc_async_f4(dst + i * 512, make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]), bar);
+                        }
+                    }
+                    // (bytes may arrive before they are expected: the phase also waits for this arrival)
+                    if (threadIdx.x == FT_FIRST_EPI * 32) mbar_arrive_expect_tx(part_full, (SPLIT - 1) * FT_EPI_WARPS * XC * 128);
+                    ok = mbar_wait_cluster_warp(part_full, n_sent & 1, abort_flag, status, STATUS_GEMM_EPILOGUE);
+                    if (!ok) break;
+                    // four partial sums: this CTA's pair first, then the other pair's sum (slots are in source order without
+                    // this CTA: 1 2 3, 0 2 3, 0 1 3, 0 1 2)
+                    const uint32_t mine = stage + lane * 16 + (SPLIT == 4 && rank >= 2 ? 2 : 0) * (XC * 128);
+                    const uint32_t other = stage + lane * 16 + (rank >= 2 ? 0 : 1) * (XC * 128);
+#pragma unroll
+                    for (int i = 0; i < XC / 4; ++i) {
+                        float* o = own + x * XC + 4 * i;
+                        const float4 p = lds_f4(mine + i * 512);
+                        o[0] += p.x; o[1] += p.y; o[2] += p.z; o[3] += p.w;
+                        if constexpr (SPLIT == 4) {
+                            const float4 c = lds_f4(other + i * 512), d = lds_f4(other + XC * 128 + i * 512);
+                            o[0] += c.x + d.x; o[1] += c.y + d.y; o[2] += c.z + d.z; o[3] += c.w + d.w;
+                        }
+                    }
+                    // (nothing follows the last exchange of the last item)
+                    __syncwarp();
+                    if (lane == 0 && (x + 1 < ROUNDS || items.at(j + 1, next))) {
+#pragma unroll
+                        for (int d = 0; d < SPLIT; ++d)
+                            if (d != rank) mbar_arrive_release_cluster(mapa_u32(smem_u32(part_free), d));
+                    }
+                }
+                if (!ok) break;
+                unscale_or_redo<SC>(own, g, M, m0, n0 + rank * SC, lane);
+                if (m0 + lane < M) {
+#pragma unroll
+                    for (int v = 0; v < NV; ++v)
+                        if (col_of(v) < g.N)
+                            finish4<HIDDEN>(g, m0 + lane, col_of(v), make_float4(own[4 * v], own[4 * v + 1], own[4 * v + 2], own[4 * v + 3]),
+                                            bias[v], res[HIDDEN ? 0 : v]);
+                }
+            } else if (has) {
+                unscale_or_redo<CW>(acc, g, M, m0, n0, lane);
+                // 16 columns at a time through the warp's transpose buffer (rows of four 16-byte chunks, XOR-swizzled): a lane
+                // then holds four columns of a row and four lanes 64 consecutive bytes
+#pragma unroll
+                for (int b = 0; b < CW / 16; ++b) {
+                    __syncwarp();                             // the previous block has been read
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        sts_u4(stage + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4),
+                               make_uint4(__float_as_uint(acc[16 * b + 4 * i]), __float_as_uint(acc[16 * b + 4 * i + 1]),
+                                          __float_as_uint(acc[16 * b + 4 * i + 2]), __float_as_uint(acc[16 * b + 4 * i + 3])));
+                    __syncwarp();
+                    const int n = n0 + 16 * b + (lane & 3) * 4;
+                    auto finish = [&](int q) {
+                        const int rr = q * 8 + (lane >> 2);
+                        const float4 v = lds_f4(stage + rr * 64 + (((lane & 3) ^ ((rr >> 1) & 3)) << 4));
+                        if (m0 + rr < M && n < g.N) finish4<HIDDEN>(g, m0 + rr, n, v, bias[b], res[HIDDEN ? 0 : 4 * b + q]);
+                    };
+                    if constexpr (HIDDEN) {
+                        // (not unrolled: most launches run this once per warp, and then what it costs is its fetch)
+#pragma unroll 1
+                        for (int q = 0; q < 4; ++q) finish(q);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) finish(q);
+                    }
+                }
+            }
+        }
+    }
+    if (*abort_flag) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000) { }     // let copies and MMAs in flight finish before releasing memory
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    if (SPLIT > 1) cluster_sync_all();           // no partner signals this CTA's barriers any more
+    if (warp == 1) tmem_dealloc(tmem_base, F_TMEM * BN);
+}
+
+template <int BN, int SPLIT, bool HIDDEN>
+static int launch_terms(FtArgs& g, const FtMaps& maps, cudaStream_t st) {
+    auto kern = linear_f32_terms_kernel<BN, SPLIT, HIDDEN>;
+    static bool attr_set[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !attr_set[dev]) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FtSmem<BN>::TOTAL);
+        if (e != cudaSuccess) {
+            set_error("linear (fp32 terms): cannot reserve %d bytes of shared memory: %s", FtSmem<BN>::TOTAL, cudaGetErrorString(e));
+            return (int)e;
+        }
+        if (dev >= 0 && dev < 64) attr_set[dev] = true;
+    }
+    long long tiles = (long long)ceil_div(g.N, BN) * ceil_div(g.m_max, FM);
+    if (SPLIT == 1) tiles *= BN / 32;                        // few tiles are cut into strips (FtItems): a CTA for each
+    const int grid = (int)(tiles * SPLIT <= sm_count() ? tiles * SPLIT : sm_count() / SPLIT * SPLIT);
+    g.n_tiles = make_fast_div((uint32_t)ceil_div(g.N, BN));
+    g.step = make_fast_div((uint32_t)(grid / SPLIT));
+    const cudaError_t le = launch_kernel(kern, true, SPLIT, dim3(grid), dim3(FT_THREADS), (size_t)FtSmem<BN>::TOTAL, st, maps, g,
+                                         device_status_ptr());
+    if (le != cudaSuccess) {
+        cudaGetLastError();
+        set_error("linear (fp32 terms): %s", cudaGetErrorString(le));
+        return (int)le;
+    }
+    return check_launch("linear (fp32 terms)");
+}
+
+// What a launch of this tile width and split takes, in cycles: rounds of tiles, the k-blocks of each, a tile's end (GELU and the
+// exchange of a split among it; clusters of four do not fill the chip).  Fitted to the launches below (us; * what it picks):
+//                                        64 / 1    64 / 2    64 / 4   128 / 1   128 / 2   128 / 4
+//   3084 x 768, K = 384                    21.0      24.5               19.0*     25.4
+//   1100 x 384, K = 384                     9.5       8.3*              10.6      11.4
+//   1100 x 1536, K = 384, GELU             18.4      22.0               16.3*     26.3
+//   1100 x 384, K = 1536, residual         26.6      18.1      21.5     27.6      23.0      15.7*
+//   771 x 1536, K = 768                    26.8      25.4      43.8     21.0*     25.2      37.9
+//   270 x 768, K = 768, residual           15.0      11.4*     14.8     16.3      15.7      11.4
+//   270 x 768, K = 3072, residual          48.2      29.1      32.3     49.4      36.4      22.3*
+//   180 x 192, K = 768, residual           14.0      10.7       7.4*    15.4      15.0      10.5
+//   4400 x 768, K = 192, GELU              18.0                         17.4*
+static double terms_cost(int bn, int split, bool hidden, long long m, int N, int num_kb, int sms) {
+    const bool wide = bn == 128;
+    const double kb_cost = wide ? 2050 : 1640;
+    const double end = (split == 1 ? (wide ? 3000 : 1500) : split == 2 ? (wide ? 5000 : 2500) : (wide ? 7500 : 3000)) +
+                       (hidden ? (wide ? 6000 : 3500) : 0);
+    const long long tiles = (m + FM - 1) / FM * ceil_div(N, bn), lanes = split == 4 ? sms * 9 / 40 : sms / split;
+    const long long full = tiles / lanes, rest = tiles - full * lanes;
+    double rounds = (double)full;
+    if (rest) rounds += split > 1 ? 1.0 : (wide && rest * 4 <= lanes) ? 0.65 : rest * 2 <= lanes ? 0.8 : 1.0;
+    return rounds * (ceil_div(num_kb, split) * kb_cost + end);
+}
+
+int linear_f32_terms_as(const LinearArgs& p, int bn, int split, cudaStream_t st) {
+    FtArgs g;
+    g.a = (const bf16*)p.a; g.w = (const bf16*)p.w; g.bias = p.bias; g.res = (const float*)p.res; g.ldr = p.ldr;
+    g.y = (float*)p.y; g.ldy = p.ldy; g.m_max = p.m_max; g.m_dev = p.m_dev; g.N = p.N; g.K = p.K;
+    g.groups_log2 = f32_groups_log2(ceil_div(p.K, FK));
+    FtMaps maps;
+    const unsigned long long strides[2] = {(unsigned long long)p.K * 2, (unsigned long long)p.K * 6};
+    const unsigned long long da[3] = {(unsigned long long)p.K, 3, (unsigned long long)p.m_max};
+    const unsigned long long dw[3] = {(unsigned long long)p.K, 3, (unsigned long long)p.N};
+    const unsigned ba[3] = {FK, 1, FM};
+    if (int rc = make_tmap_bf16(&maps.a, p.a, 3, da, strides, ba)) return rc;
+    for (int i = 0; i < 3; ++i) {
+        const unsigned bw[3] = {FK, 1, (unsigned)(bn >> (bn == 128 ? i : i > 0))};      // (64-wide tiles are cut in two only)
+        if (int rc = make_tmap_bf16(&maps.w[i], p.w, 3, dw, strides, bw)) return rc;
+    }
+#define VTP_TERMS_CASE(BN, SPLIT) \
+    if (bn == BN && split == SPLIT) return p.out_terms ? launch_terms<BN, SPLIT, true>(g, maps, st) : launch_terms<BN, SPLIT, false>(g, maps, st)
+    VTP_TERMS_CASE(128, 1);
+    VTP_TERMS_CASE(128, 2);
+    VTP_TERMS_CASE(128, 4);
+    VTP_TERMS_CASE(64, 1);
+    VTP_TERMS_CASE(64, 2);
+    VTP_TERMS_CASE(64, 4);
+#undef VTP_TERMS_CASE
+    return fail(VTP_ERR_UNSUPPORTED, "linear (fp32 terms): no kernel for tiles of %d columns, %d CTAs", bn, split);
+}
+
+int linear_f32_terms(const LinearArgs& p, cudaStream_t st) {
+    if (int rc = linear_validate(p)) return rc;
+    VTP_REQUIRE(p.dtype == VTP_F32 && p.N % 8 == 0 && p.K % 8 == 0 && p.ldy % 4 == 0 && (!p.res || p.ldr % 4 == 0), VTP_ERR_SHAPE,
+                "linear (fp32 terms): N=%d K=%d", p.N, p.K);
+    VTP_REQUIRE(p.ln_mode == 0 && !p.emit_stats && p.out_grp == 0 && p.res_mod == 0 && p.out_terms == ((p.flags & VTP_FLAG_GELU) != 0) &&
+                    !(p.out_terms && p.res), VTP_ERR_UNSUPPORTED,
+                "linear (fp32 terms): plain rows, either GELU and terms out or an optional residual and fp32 out");
+    if (p.m_max == 0) return VTP_OK;
+    const int num_kb = ceil_div(p.K, FK), sms = sm_count();
+    // With a device-side row count the worst case is about three times the packed rows of a DGE block.
+    const long long m = p.m_dev ? ceil_div(p.m_max, 3) : p.m_max;
+    int bn = 64, split = 1;
+    double best = 0;
+    for (int b = 64; b <= 128; b *= 2)
+        for (int s = 1; s <= (1 << f32_groups_log2(num_kb)); s *= 2) {
+            const double c = terms_cost(b, s, p.out_terms, m, p.N, num_kb, sms);
+            if (best == 0 || c < best) { best = c; bn = b; split = s; }
+        }
+    return linear_f32_terms_as(p, bn, split, st);
+}
+
+}  // namespace vtp

@@ -117,16 +117,6 @@ __device__ __forceinline__ void gelu8(float* v) {
     }
 }
 
-// Unsigned division by a number the host knows: multiply by ceil(2^32 / d), then take back the one the estimate may
-// be over (it is never under).  A runtime division is about forty dependent instructions on the way to a CTA's first load.
-struct FastDiv { uint32_t d, magic; };
-__device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv& f) {
-    if (f.d == 1) return n;
-    uint32_t q = __umulhi(n, f.magic);
-    if (q * f.d > n) --q;          // (n and d are below 2^31)
-    return q;
-}
-
 // One GEMM problem of a launch: its tensor maps, and the scalars the kernel reads.  Each CTA copies the scalars of a launch
 // to shared memory before it waits for the kernel in front: parameters are cold in every launch, and read where they are
 // needed each line of them is a miss of some 500 cycles on the way to the first load, and another on the way to the first store.
@@ -906,10 +896,6 @@ static int pick_bn(int N) {
 }
 
 int linear_stat_slots(int N) { return (int)round_up(ceil_div(N, SLAB), 2); }
-
-static FastDiv make_fast_div(uint32_t d) {
-    return FastDiv{d, d == 1 ? 0u : (uint32_t)(((1ull << 32) + d - 1) / d)};
-}
 
 static void fill_scalars(TcScalars& q, const LinearArgs& p, bool f32, int bn) {
     q.bias = p.bias; q.res = (const bf16*)p.res; q.ldr = p.ldr; q.y = p.y; q.ldy = p.ldy;

@@ -4,7 +4,7 @@
 //
 // Replaces PatchEmbed, the cls-token concat and the position-embedding add of
 // VisionTransformer.forward_features (vtpack/models/dge/deit_dge.py:268-275).
-#include "common.cuh"
+#include "f32_terms.cuh"
 
 namespace vtp {
 
@@ -186,6 +186,37 @@ int token_im2col(const void* x, int dtype, int B, int H, int W, int C, int sr, v
         if (small) launch_chain(token_im2col_kernel<float, unsigned>, dim3(grid), dim3(256), 0, st, (const float*)x, total, H, W, C, sr, (float*)cols);
         else launch_chain(token_im2col_kernel<float, long long>, dim3(grid), dim3(256), 0, st, (const float*)x, total, H, W, C, sr, (float*)cols);
     }
+    return check_launch("spatial reduction im2col");
+}
+
+// The same for fp32 tokens with the rows as terms, [3][sr * sr * C]: a thread moves eight values.
+__global__ void __launch_bounds__(256)
+token_im2col_terms_kernel(const float* __restrict__ x, unsigned total, int H, int W, int C, int sr, bf16* __restrict__ cols) {
+    pdl_begin();
+    const unsigned run = (unsigned)(sr * C / 8), Wo = (unsigned)(W / sr), Ho = (unsigned)(H / sr);
+    const size_t n = (size_t)sr * sr * C;
+    for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < total; v += gridDim.x * blockDim.x) {
+        const unsigned i = v % run;
+        unsigned r = v / run;                     // (b, oy, ox, dy) with dy fastest
+        const unsigned dy = r % (unsigned)sr; r /= (unsigned)sr;
+        const unsigned ox = r % Wo; r /= Wo;
+        const unsigned oy = r % Ho, b = r / Ho;
+        const float4* src = reinterpret_cast<const float4*>(x + (((size_t)b * H + oy * sr + dy) * W + ox * sr) * C + (size_t)i * 8);
+        const float4 lo = src[0], hi = src[1];
+        const float f[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        bf16* dst = cols + (((size_t)b * Ho + oy) * Wo + ox) * 3 * n + (size_t)dy * sr * C + (size_t)i * 8;
+        store_terms4(dst, n, f);
+        store_terms4(dst + 4, n, f + 4);
+    }
+}
+
+int token_im2col_terms(const void* x, int B, int H, int W, int C, int sr, void* cols, cudaStream_t st) {
+    // (a block has fewer than 2^30 tokens; at eight values a unit their index has to fit 32 bits)
+    const long long total = (long long)B * H * W * C / 8;
+    VTP_REQUIRE(C % 8 == 0 && total < (1ll << 32), VTP_ERR_SHAPE, "spatial reduction: %lld values of C=%d", total * 8, C);
+    if (total == 0) return VTP_OK;
+    const int grid = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
+    launch_chain(token_im2col_terms_kernel, dim3(grid), dim3(256), 0, st, (const float*)x, (unsigned)total, H, W, C, sr, (bf16*)cols);
     return check_launch("spatial reduction im2col");
 }
 

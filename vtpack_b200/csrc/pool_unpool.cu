@@ -39,7 +39,7 @@ template <typename T, int MAXCH>
 __device__ __forceinline__ void ln_row_store(const float (&f)[MAXCH][Vec<T>::N], int lane,
                                              int nchunks, int C, const float (&w)[MAXCH][Vec<T>::N],
                                              const float (&bb)[MAXCH][Vec<T>::N], float eps,
-                                             T* __restrict__ dst, const T* __restrict__ add_row = nullptr) {
+                                             T* __restrict__ y, size_t row, bool terms = false, const T* __restrict__ add_row = nullptr) {
     constexpr int VN = Vec<T>::N;
     float s = 0.f;
 #pragma unroll
@@ -70,9 +70,7 @@ __device__ __forceinline__ void ln_row_store(const float (&f)[MAXCH][Vec<T>::N],
 #pragma unroll
                 for (int i = 0; i < VN; ++i) o[i] += af[i];
             }
-            Vec<T> ov;
-            ov.from_float(o);
-            ov.store(dst + chunk * VN);
+            store_row_vec<T>(y, row, C, chunk * VN, o, terms);
         }
     }
 }
@@ -161,8 +159,7 @@ pool_kernel(const T* __restrict__ x, int B, int N, int C, int W, int num_extra,
                             for (int i = 0; i < VN; ++i) sum[ch][i] += f[ch][i];
                         }
                         if (WITH_LN && xn)
-                            ln_row_store<T, MAXCH>(f, lane, nchunks, C, w, bb, eps,
-                                                   xn + (row0 + (size_t)dy * W + dx0 + j) * C);
+                            ln_row_store<T, MAXCH>(f, lane, nchunks, C, w, bb, eps, xn, row0 + (size_t)dy * W + dx0 + j);
                     }
                 }
             }
@@ -179,7 +176,7 @@ pool_kernel(const T* __restrict__ x, int B, int N, int C, int W, int num_extra,
                 ov.store(comp + (size_t)p * C + chunk * VN);
             }
         }
-        if (WITH_LN && qn) ln_row_store<T, MAXCH>(sum, lane, nchunks, C, w, bb, eps, qn + (size_t)p * C);
+        if (WITH_LN && qn) ln_row_store<T, MAXCH>(sum, lane, nchunks, C, w, bb, eps, qn, (size_t)p);
     }
 }
 
@@ -355,6 +352,7 @@ static int elem_grid(long long elems) {
 struct RowAdd {
     const void* addend = nullptr;
     int a_mod = 1, a_off = 0, out_grp = 1, out_stride = 1, out_off = 0;
+    bool terms = false;      // fp32: y takes the terms of every row (f32_terms.cuh)
 };
 
 template <typename T, int MAXCH>
@@ -388,10 +386,10 @@ layernorm_kernel(const T* __restrict__ x, int rows_max, const int32_t* __restric
         }
         if (add.addend) {
             const size_t orow = (size_t)(r / add.out_grp) * add.out_stride + add.out_off + r % add.out_grp;
-            ln_row_store<T, MAXCH>(f, lane, nchunks, C, w, bb, eps, y + orow * C,
+            ln_row_store<T, MAXCH>(f, lane, nchunks, C, w, bb, eps, y, orow, false,
                                    static_cast<const T*>(add.addend) + ((size_t)(r % add.a_mod) + add.a_off) * C);
         } else {
-            ln_row_store<T, MAXCH>(f, lane, nchunks, C, w, bb, eps, y + (size_t)r * C);
+            ln_row_store<T, MAXCH>(f, lane, nchunks, C, w, bb, eps, y, (size_t)r, add.terms);
         }
     }
 }
@@ -458,9 +456,7 @@ layernorm_narrow_kernel(const T* __restrict__ x, int rows_max, const int32_t* __
                 for (int i = 0; i < VN; ++i) o[i] += af[i];
                 orow = (size_t)(r / add.out_grp) * add.out_stride + add.out_off + r % add.out_grp;
             }
-            Vec<T> ov;
-            ov.from_float(o);
-            ov.store(y + orow * C + sub * VN);
+            store_row_vec<T>(y, orow, C, sub * VN, o, add.terms);
         }
     }
 }
@@ -558,6 +554,13 @@ static int launch_ln(const void* x, int rows_max, const int32_t* rows_dev, int C
     else return fail(VTP_ERR_SHAPE, "layernorm: C=%d too large", C);
 #undef VTP_LN
     return check_launch("layernorm");
+}
+
+int layernorm_terms(const void* x, int rows_max, const int32_t* rows_dev, int C, const float* w, const float* b, float eps, void* y,
+                    cudaStream_t st) {
+    RowAdd out;
+    out.terms = true;
+    return rows_max == 0 ? VTP_OK : launch_ln<float>(x, rows_max, rows_dev, C, C, w, b, eps, y, st, out);
 }
 
 static int check_rows(const char* what, int dtype, int C, const void* a, const void* b) {

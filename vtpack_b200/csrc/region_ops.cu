@@ -101,7 +101,7 @@ __device__ __forceinline__ float2 mean_rstd(float2 s, int C, float eps) {
 template <typename T, int G, int CPL>
 __device__ __forceinline__ void ln_store(const float (&f)[CPL][Vec<T>::N], int sub, int C,
                                          const float* __restrict__ lnw, const float* __restrict__ lnb, float eps,
-                                         T* dst) {
+                                         T* y, size_t row, bool terms) {
     constexpr int VN = Vec<T>::N;
     float s = 0.f;
 #pragma unroll
@@ -121,9 +121,7 @@ __device__ __forceinline__ void ln_store(const float (&f)[CPL][Vec<T>::N], int s
         float o[VN];
 #pragma unroll
         for (int i = 0; i < VN; ++i) o[i] = (f[ch][i] - mean) * rstd * __ldg(lnw + c0 + i) + __ldg(lnb + c0 + i);
-        Vec<T> ov;
-        ov.from_float(o);
-        ov.store(dst + c0);
+        store_row_vec<T>(y, row, C, c0, o, terms);
     }
 }
 
@@ -205,17 +203,19 @@ __device__ __forceinline__ void publish_partials(float* part, float (&acc)[CPL][
 constexpr int POOL_LN = 0, POOL_STATS = 1, POOL_PLAIN = 2, POOL_COLS = 3;
 // (A thread of a narrow-row layout holds one or two 16-byte vectors of a region: such kernels run with 16 or 12 CTAs per SM
 // (a few spilled words in the unpool; measured faster all the same), and the kernel is bound by how many regions are in flight.)
+template <typename T, int G, int CPL>
+constexpr int pool_ctas() { return Lay<T, G, CPL>::TPG * CPL <= 1 ? 16 : Lay<T, G, CPL>::TPG * CPL <= 2 ? 12 : 7; }
+// (terms: POOL_LN of fp32 rows only; 1: xn, 2: qn as terms)
 template <typename T, int G, int CPL, int MODE>
-__global__ void __launch_bounds__(128, (Lay<T, G, CPL>::TPG * CPL <= 1) ? 16 : ((Lay<T, G, CPL>::TPG * CPL <= 2) ? 12 : 7))
-pool_region_kernel(const T* __restrict__ x, RegionGeom g, const int32_t* __restrict__ idx,
+__device__ __forceinline__ void
+pool_region(const T* __restrict__ x, RegionGeom g, const int32_t* __restrict__ idx,
                    const int32_t* __restrict__ region_first, const int32_t* __restrict__ offsets,
                    const int32_t* __restrict__ counts, int32_t* __restrict__ offsets_out,
                    int32_t* __restrict__ region_first_out, int32_t* __restrict__ counts_next, Splits sp,
                    T* __restrict__ comp, float2* __restrict__ stats_x, float2* __restrict__ stats_q,
                    float2* __restrict__ stats_acc, int write_stats_x, const float* __restrict__ lnw,
                    const float* __restrict__ lnb, float eps, T* __restrict__ xn, T* __restrict__ qn, int sum_only,
-                   int sr, int* status) {
-    pdl_begin();
+                   int sr, int* status, int terms) {
     constexpr bool COLS = MODE == POOL_COLS, STATS = MODE == POOL_STATS || COLS, EXPLICIT_LN = MODE == POOL_LN;
     using L = Lay<T, G, CPL>;
     constexpr int VN = L::VN, GROUPS = L::GROUPS, TPG = L::TPG;
@@ -262,8 +262,8 @@ pool_region_kernel(const T* __restrict__ x, RegionGeom g, const int32_t* __restr
             }
             if (sub == 0) { stats_q[dst_row] = st; if (stats_acc) stats_acc[dst_row] = make_float2(0.f, 0.f); }
         } else if (EXPLICIT_LN) {
-            ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, xn + src_row * g.C);
-            ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, qn + (size_t)dst_row * g.C);
+            ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, xn, src_row, terms & 1);
+            ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, qn, (size_t)dst_row, terms & 2);
         }
         return;
     }
@@ -343,8 +343,8 @@ pool_region_kernel(const T* __restrict__ x, RegionGeom g, const int32_t* __restr
                 }
             }
         } else if (EXPLICIT_LN) {
-            ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, xn + (tok0 + j) * g.C);
-            if (step == 1) ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, qn + (size_t)prow * g.C);
+            ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, xn, tok0 + j, terms & 1);
+            if (step == 1) ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, qn, (size_t)prow, terms & 2);
         }
         if (step == 1) {
             store_row<T, CPL>(rows[j], comp + (size_t)prow * g.C, sub, G);
@@ -397,9 +397,42 @@ pool_region_kernel(const T* __restrict__ x, RegionGeom g, const int32_t* __restr
         const float2 st = mean_rstd(row_sums<T, G, CPL>(acc), g.C, eps);
         if (sub == 0) { stats_q[row] = st; if (stats_acc) stats_acc[row] = make_float2(0.f, 0.f); }
     } else {
-        if (EXPLICIT_LN) ln_store<T, G, CPL>(acc, sub, g.C, lnw, lnb, eps, qn + (size_t)row * g.C);
+        if (EXPLICIT_LN) ln_store<T, G, CPL>(acc, sub, g.C, lnw, lnb, eps, qn, (size_t)row, terms & 2);
         round_store<T, CPL>(acc, comp + (size_t)row * g.C, sub, G);
     }
+}
+
+template <typename T, int G, int CPL, int MODE>
+__global__ void __launch_bounds__(128, (pool_ctas<T, G, CPL>()))
+pool_region_kernel(const T* __restrict__ x, RegionGeom g, const int32_t* __restrict__ idx,
+                   const int32_t* __restrict__ region_first, const int32_t* __restrict__ offsets,
+                   const int32_t* __restrict__ counts, int32_t* __restrict__ offsets_out,
+                   int32_t* __restrict__ region_first_out, int32_t* __restrict__ counts_next, Splits sp,
+                   T* __restrict__ comp, float2* __restrict__ stats_x, float2* __restrict__ stats_q,
+                   float2* __restrict__ stats_acc, int write_stats_x, const float* __restrict__ lnw,
+                   const float* __restrict__ lnb, float eps, T* __restrict__ xn, T* __restrict__ qn, int sum_only,
+                   int sr, int* status) {
+    pdl_begin();
+    pool_region<T, G, CPL, MODE>(x, g, idx, region_first, offsets, counts, offsets_out, region_first_out, counts_next, sp, comp,
+                                 stats_x, stats_q, stats_acc, write_stats_x, lnw, lnb, eps, xn, qn, sum_only, sr, status, 0);
+}
+// The pool of an fp32 block whose Linears take terms.  The CTAs behind the pool's split the block's matrices, which nothing in
+// front of this kernel needs: the pool waits on its rows, the split on its own, and a launch is saved.
+template <int G, int CPL>
+__global__ void __launch_bounds__(128, (pool_ctas<float, G, CPL>()))
+pool_region_terms_kernel(const float* __restrict__ x, RegionGeom g, const int32_t* __restrict__ idx,
+                         const int32_t* __restrict__ region_first, const int32_t* __restrict__ offsets,
+                         const int32_t* __restrict__ counts, int32_t* __restrict__ offsets_out,
+                         int32_t* __restrict__ region_first_out, int32_t* __restrict__ counts_next, Splits sp,
+                         float* __restrict__ comp, const float* __restrict__ lnw, const float* __restrict__ lnb, float eps,
+                         float* __restrict__ xn, float* __restrict__ qn, int terms, int pool_grid, TermSplit split) {
+    pdl_begin();
+    if ((int)blockIdx.x >= pool_grid) {
+        split_matrices(split, (int)blockIdx.x - pool_grid);
+        return;
+    }
+    pool_region<float, G, CPL, POOL_LN>(x, g, idx, region_first, offsets, counts, offsets_out, region_first_out, counts_next, sp,
+                                        comp, nullptr, nullptr, nullptr, 0, lnw, lnb, eps, xn, qn, 0, 1, nullptr, terms);
 }
 
 // ------------------------------------------------------------------------ router gate
@@ -641,6 +674,14 @@ static void launch_pool_t(const RegionPoolArgs& a, cudaStream_t st) {
     const int R = a.g.Hr * a.g.Wr;
     const int grid = a.g.B * R + ceil_div(a.g.B * a.g.num_extra, RG * (32 / G));
     const size_t smem = (size_t)8 * a.g.C * sizeof(float);
+    if constexpr (sizeof(T) == 4) {
+        if (a.qn_terms) {
+            launch_chain(pool_region_terms_kernel<G, CPL>, dim3(grid + a.split.ctas()), dim3(128), smem, st, (const float*)a.x, a.g,
+                a.idx, a.region_first, a.offsets, a.counts, a.offsets_out, a.region_first_out, a.counts_next, a.sp, (float*)a.comp,
+                a.lnw, a.lnb, a.eps, (float*)a.xn, (float*)a.qn, a.xn_terms ? 3 : 2, grid, a.split);
+            return;
+        }
+    }
     if (a.stats_q && a.sr > 1)
         launch_chain(pool_region_kernel<T, G, CPL, POOL_COLS>, dim3(grid), dim3(128), smem, st, 
             (const T*)a.x, a.g, a.idx, a.region_first, a.offsets, a.counts, a.offsets_out, a.region_first_out,

@@ -1,7 +1,7 @@
 // Internal interface of the region-parallel kernels (router gate, pooling, unpooling).
 #pragma once
 
-#include "common.cuh"
+#include "f32_terms.cuh"
 
 namespace vtp {
 
@@ -34,6 +34,8 @@ struct RegionPoolArgs {
     bool stats_x_ready = false;              // stats_x was already written (by the previous block's unpool)
     const float* lnw = nullptr; const float* lnb = nullptr; float eps = 1e-6f;
     void* xn = nullptr; void* qn = nullptr;
+    bool xn_terms = false, qn_terms = false; // fp32: these rows as terms (f32_terms.cuh)
+    TermSplit split;                         // with qn_terms: matrices to split beside the pooling
     // With the statistics and sr > 1 (a divisor of both grid sides, no extra tokens): also LayerNorm(x) (lnw, lnb) in `cols`, as rows of
     // the stride-sr convolution, [B * (H / sr) * (W / sr), sr * sr * C] with column (dy, dx, c).
     int sr = 1; void* cols = nullptr;

@@ -138,6 +138,13 @@ __device__ __forceinline__ void tma_load_2d_a(uint32_t dst, const CUtensorMap* m
             : "memory");
 }
 
+__device__ __forceinline__ void tma_load_3d_a(uint32_t dst, const CUtensorMap* m, uint32_t bar, int x, int y, int z) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(y), "r"(z)
+        : "memory");
+}
+
 // Tile store shared (this CTA) -> global, tracked by the bulk async-group of the issuing thread.
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* src, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
@@ -246,6 +253,13 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
 // them at cluster scope; the waiter acquires at cluster scope.
 __device__ __forceinline__ void stc_f4(uint32_t cluster_addr, float4 v) {
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                 : "memory");
+}
+// The same with the bytes counted on a barrier of that CTA, which then needs no arrival that releases them (such an arrival waits for
+// the stores in front of it to get there, about a microsecond).
+__device__ __forceinline__ void stc_async_f4(uint32_t cluster_addr, float4 v, uint32_t cluster_bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(cluster_addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(cluster_bar)
                  : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_release_cluster(uint32_t cluster_addr) {
