@@ -81,11 +81,12 @@ def test_all_fine_equals_dense_block_fp32():
     (384, 1, 4.0, False), (384, 12, 4.0, False), (384, 4, 4.0, True),
     (768, 1, 4.0, False), (768, 2, 4.0, True),
 ])
-def test_block_fp32_terms_same_bits_as_rows(C, B, mlp_ratio, special):
-    """An fp32 block's Linears take their operands as three bf16 terms, split by the kernels in front of them; the dense block's
-    Linears split fp32 rows themselves.  With every region at the finest grain the two blocks do the same arithmetic
-    (channels that the pool spreads over whole warps: LayerNorm sums in the same order), so the outputs are the same bits, where operands or
-    sums are infinite, NaN, near the largest or subnormal too."""
+def test_block_fp32_on_terms_vs_dense_block(C, B, mlp_ratio, special):
+    """An fp32 block's Linears and attention take their operands as three bf16 terms, split by the kernels in front of them; the
+    dense block's Linears split fp32 rows themselves and its attention runs on CUDA cores.  With every region at the finest grain
+    the two blocks are the same function; they differ by the attention's rounding only, some 2^-22 of a row's largest value
+    (probabilities with errors of a few 2^-24, sums of 257 of them), carried through two Linears.  Where operands or sums are
+    infinite, NaN, near the largest or subnormal the same values have to be infinite or NaN."""
     from vtpack_b200 import _lib
     from vtpack_b200.models.dge.deit_dge import Block
     torch.manual_seed(C + B)
@@ -101,11 +102,59 @@ def test_block_fp32_terms_same_bits_as_rows(C, B, mlp_ratio, special):
     gate = torch.zeros(B, 4, 4, 3)
     gate[..., 0] = 1
     with torch.no_grad():
-        # (the cls row goes through the unpool's sum, ref + (q - comp), which rounds)
+        # (the cls row goes through the unpool's sum, ref + (q - comp))
         a, b = blk(x, forced_gate=gate)[:, 1:], blk(x, dense=True)[:, 1:]
     assert _lib.device_status() == 0
     assert bool(torch.isfinite(a).all()) != special
-    assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.nan_to_num(nan=0.0), b.nan_to_num(nan=0.0))
+    assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+    fin = torch.isfinite(b)
+    assert torch.equal(a[~fin & ~a.isnan()], b[~fin & ~b.isnan()])
+    scale = torch.where(fin, b, 0.0).double().abs().amax(dim=-1, keepdim=True).clamp_min(1e-30)
+    assert float((torch.where(fin, a - b, 0.0).double().abs() / scale).max()) < 2e-6
+
+
+@pytest.mark.parametrize("n_grid,heads,special", [(4, 1, ""), (8, 2, ""), (12, 3, "inf key"), (16, 2, "nan value"), (16, 6, "huge"),
+                                                  (20, 1, "minus inf"), (24, 2, ""), (32, 1, "huge")])
+def test_attention_fp32_on_terms(n_grid, heads, special):
+    """The fp32 attention of a block at 17 to 1025 keys (one key behind whole blocks of 64, one to four chunks of up to five
+    blocks), 1 to 1025 queries an image, in float64 and, where scores or values are infinite, NaN or overflow the terms'
+    sums, as the CUDA-core kernel has them (the dense block)."""
+    from vtpack_b200 import _lib
+    from vtpack_b200.models.dge.deit_dge import Block
+    torch.manual_seed(n_grid)
+    C, B, N = 64 * heads, 3, n_grid * n_grid + 1
+    blk = Block(C, heads, mlp_ratio=1.0, qkv_bias=True, split_sizes=[4, 2, 1]).to(DEV).eval()
+    with torch.no_grad():
+        blk.attn.q.weight *= 8          # (scores that spread over some units)
+        blk.attn.kv.weight *= 4
+    x = torch.randn(B, N, C, device=DEV)
+    gate = torch.zeros(B, n_grid // 4, n_grid // 4, 3)
+    gate[0, ..., 2], gate[1, ..., 0], gate[2, ..., 1] = 1, 1, 1
+    kv = blk.attn.kv
+    with torch.no_grad():
+        if special == "inf key":
+            kv.bias[3] = float("inf")
+        elif special == "nan value":
+            kv.bias[C + 5] = float("nan")
+        elif special == "huge":
+            kv.bias[C + 7], kv.bias[2] = 2.0 ** 118, 2.0 ** 97
+            blk.attn.q.bias[2] = 1e-3
+        elif special == "minus inf":
+            kv.bias[1], blk.attn.q.bias[1] = -float("inf"), 9.0
+        out = blk(x, forced_gate=gate)
+        assert _lib.device_status() == 0
+        if special:
+            fine = torch.zeros(B, n_grid // 4, n_grid // 4, 3)
+            fine[..., 0] = 1
+            a, b = blk(x, forced_gate=fine)[:, 1:], blk(x, dense=True)[:, 1:]
+            assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+            fin = torch.isfinite(b)
+            scale = torch.where(fin, b, 0.0).double().abs().amax(dim=-1, keepdim=True).clamp_min(1e-30)
+            assert float((torch.where(fin, a - b, 0.0).double().abs() / scale).max()) < 1e-5
+        else:
+            w = {k: v.double().cpu() for k, v in blk.state_dict().items()}
+            ref = O.dge_block_forward(x.double().cpu(), w, heads, (4, 2, 1), forced_gate=gate.double(), eps=1e-5)
+            assert rel_err(out, ref) < 2e-6
 
 
 def test_layer_512px_skewed_fp32():

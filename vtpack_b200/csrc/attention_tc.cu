@@ -33,6 +33,7 @@
 // (vtpack/layers/csrc/batched_sparse_gemm/batched_sparse_gemm.cu:219-305: per image two
 // cuBLAS strided-batched GEMMs around a cuDNN softmax, scores round-tripping through HBM).
 #include "attention.h"
+#include "attention_items.cuh"
 #include "runtime.h"
 #include "sm100.cuh"
 
@@ -40,8 +41,6 @@ namespace vtp {
 
 using namespace sm100;
 
-constexpr int QT = 128;            // queries per item = TMEM lanes
-constexpr int HD = 64;             // head dim
 constexpr int KC_MAX = 256;        // keys per tensor-core chunk, upper bound
 constexpr int O_COL = 64;          // TMEM column of the P*V accumulator
 constexpr int P_SPLIT = 128;       // keys of a chunk's first part of P, in columns [0, 64); the rest of P from column 128 on
@@ -65,30 +64,11 @@ __device__ __forceinline__ float fast_exp2(float x) {
     return y;
 }
 
-struct AttnItem { int b, h, row0, nq; };
-
 // Plain bulk copy global -> shared of `bytes` (a multiple of 16, both ends 16-byte aligned), counted on `bar`.
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
-}
-
-// item w -> (image, head, first packed row, valid rows); tile_prefix is in shared memory, so are the offsets of a moderate batch
-__device__ __forceinline__ AttnItem attn_item(int w, int heads, int B, const int* tile_prefix, const int32_t* offsets) {
-    const int tg = w / heads;
-    int lo = 0, hi = B;                        // largest b with tile_prefix[b] <= tg
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (tile_prefix[mid] <= tg) lo = mid; else hi = mid;
-    }
-    AttnItem it;
-    it.b = lo;
-    it.h = w - tg * heads;
-    const int t = tg - tile_prefix[lo];
-    it.row0 = offsets[lo] + t * QT;
-    it.nq = min(QT, offsets[lo + 1] - it.row0);
-    return it;
 }
 
 __global__ void __launch_bounds__(192, 2)
@@ -141,47 +121,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     // Nothing above depends on the kernel in front of this one on the stream; the packed-row
     // offsets, q, k and v below do.
     pdl_begin();
-    // tile_prefix[b] = number of 128-query tiles of the images in front of b.  All threads fetch the
-    // per-image tile counts at once (one global-load latency), then warp 0 scans them in shared memory, a run of images per
-    // lane.
-    // (the offsets come from the caller: a count outside [0, max_q] is clamped, so the item list
-    // always fits the grid's bound, and rows at or beyond l_max are never stored below)
     const bool keep = B <= OFFSETS_KEPT;
     if (threadIdx.x == blockDim.x - 1) *void_s = launch_is_void(status) ? 1 : 0;
-    for (int b = threadIdx.x; b < B; b += blockDim.x) {
-        const int o0 = offsets[b], o1 = offsets[b + 1];
-        int cnt = o1 - o0;
-#if VTP_INDEX_GUARDS
-        if (cnt < 0 || cnt > max_q || o0 < 0 || o1 > l_max) {
-            if (status && blockIdx.x == 0) atomicOr(status, STATUS_BAD_INDEX);
-            cnt = (o0 < 0) ? 0 : min(max(cnt, 0), max_q);
-        }
-#endif
-        tile_prefix[b] = (cnt + QT - 1) / QT;
-        if (keep) {
-            offs_s[b] = o0;
-            if (b + 1 == B) offs_s[B] = o1;
-        }
-    }
-    __syncthreads();
-    if (warp == 0) {
-        const int per = (B + 31) / 32, b0 = min(lane * per, B), b1 = min(b0 + per, B);
-        int sum = 0;
-        for (int b = b0; b < b1; ++b) sum += tile_prefix[b];
-        int incl = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int nb = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += nb;
-        }
-        int run = incl - sum;
-        for (int b = b0; b < b1; ++b) {
-            const int tiles = tile_prefix[b];
-            tile_prefix[b] = run;
-            run += tiles;
-        }
-        if (lane == 31) tile_prefix[B] = incl;
-    }
+    list_tiles(offsets, B, max_q, l_max, status, tile_prefix, keep ? offs_s : nullptr);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();

@@ -57,6 +57,11 @@ static bool block_terms(const vtp_dge_shape& s) {
            region_ops_supported(region_geom(s), s.dtype) && (s.sr_ratio <= 1 || reduced < (1ll << 32));
 }
 
+// ... and its attention too.
+static bool attn_terms(const vtp_dge_shape& s) {
+    return block_terms(s) && s.C == s.heads * 64 && attention_f32_terms_pays(keys_per_image(s));
+}
+
 static BlockScratch carve_block(const vtp_dge_shape& s, void* ws) {
     const long long e = (long long)elem_size(s.dtype);
     const int N = s.num_extra + s.H * s.W;
@@ -82,8 +87,9 @@ static BlockScratch carve_block(const vtp_dge_shape& s, void* ws) {
     b.comp = c.take(rows * s.C * e);
     b.xn = c.take(rows * s.C * et);
     b.qn = c.take(rows * s.C * et);
-    b.qp = c.take(rows * s.C * e);
-    b.kv = c.take(rows * 2 * s.C * e);
+    const long long ea = attn_terms(s) ? 6 : e;     // of what the attention reads
+    b.qp = c.take(rows * s.C * ea);
+    b.kv = c.take(rows * 2 * s.C * ea);
     b.ao = c.take(rows * s.C * et);
     b.q1 = c.take(rows * s.C * e);
     b.hid = c.take(rows * s.hidden * et);
@@ -229,7 +235,7 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
     // chained: gate decisions, per-image counts and token statistics came from the previous
     // block's unpool; the pool kernel then also derives the row offsets itself
     const bool chained = chain.have_gate && by_region && !forced_logits;
-    const bool terms = block_terms(s);
+    const bool terms = block_terms(s), terms_attn = attn_terms(s);
     if (terms)
         VTP_REQUIRE(aligned16(w.q_w) && aligned16(w.kv_w) && aligned16(w.proj_w) && aligned16(w.fc1_w) && aligned16(w.fc2_w) &&
                         aligned16(w.sr_w), VTP_ERR_ALIGN, "block: matrices must be 16-byte aligned");
@@ -306,7 +312,7 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
 
     const void* keys_in = fold ? x_in : b.xn;
     if (reduce) {
-        if ((rc = run_linear(lq, b.q_wt, false)) || (rc = marks.mark(4))) return rc;
+        if ((rc = run_linear(lq, b.q_wt, terms_attn)) || (rc = marks.mark(4))) return rc;
         // x_ = norm(sr(LN1(x) as [B,C,H,W])): the stride-sr convolution as im2col rows times a matrix
         const int krows = s.B * n_keys, KS = s.sr_ratio * s.sr_ratio * C;
         if (terms) rc = token_im2col_terms(b.xn, s.B, s.H, s.W, C, s.sr_ratio, b.sr_cols, st);
@@ -329,8 +335,8 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
         // the two projections do not depend on each other: one launch, the q tiles fill the kv tail
         if ((rc = linear_tcgen05_pair(lkv, lq, st))) return rc;
     } else {
-        if (!reduce && ((rc = run_linear(lq, b.q_wt, false)) || (rc = marks.mark(4)))) return rc;
-        if ((rc = run_linear(lkv, b.kv_wt, false)) || (rc = marks.mark(5))) return rc;
+        if (!reduce && ((rc = run_linear(lq, b.q_wt, terms_attn)) || (rc = marks.mark(4)))) return rc;
+        if ((rc = run_linear(lkv, b.kv_wt, terms_attn)) || (rc = marks.mark(5))) return rc;
     }
 
     AttnArgs at;
@@ -342,7 +348,7 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
     at.o_terms = terms ? C : 0;
     at.dtype = s.dtype; at.B = s.B; at.n_keys = n_keys; at.heads = s.heads; at.head_dim = d;
     at.offsets = b.offsets; at.l_max = rows; at.max_q = N; at.scale = attn_scale(s); at.flags = kflag;
-    if ((rc = attention(at, st)) || (rc = marks.mark(6))) return rc;
+    if ((rc = terms_attn ? attention_f32_terms(at, st) : attention(at, st)) || (rc = marks.mark(6))) return rc;
 
     LinearArgs lp;   // q1 = comp + attn_out Wp^T + b   (and, when folding, the row sums LN2 needs)
     lp.a = b.ao; lp.lda = C; lp.w = w.proj_w; lp.bias = w.proj_b; lp.res = b.comp; lp.ldr = C; lp.y = b.q1;

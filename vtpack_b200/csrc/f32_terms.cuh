@@ -39,14 +39,27 @@ __device__ __forceinline__ float join_terms(uint32_t h, uint32_t m, uint32_t l) 
     return (__uint_as_float(h << 16) + (__uint_as_float(m << 16) + __uint_as_float(l << 16))) * (1.f / F_SCALE);
 }
 
-// Four consecutive values, the first of them element `at` of a row whose h terms start at `row` and whose terms are n apart.
+// Four consecutive values, the h terms to `row` on, terms n apart.
 __device__ __forceinline__ void store_terms4(bf16* row, size_t n, const float* v) {
-    uint32_t t[3][4];
+    uint32_t t[3][4], most = 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) split_terms(v[i], t[0][i], t[1][i], t[2][i]);
+    for (int i = 0; i < 4; ++i) {
+        const float x = v[i] * F_SCALE;
+        most = max(most, __float_as_uint(x) & 0x7FFFFFFFu);
+        split_scaled(x, t[0][i], t[1][i], t[2][i]);
+    }
+    if (most >= 0x7F7F8000u) {             // one whose h, rounded, is infinite
+#pragma unroll
+        for (int i = 0; i < 4; ++i) split_terms(v[i], t[0][i], t[1][i], t[2][i]);
+    }
 #pragma unroll
     for (int p = 0; p < 3; ++p)
         *reinterpret_cast<uint2*>(row + p * n) = make_uint2(__byte_perm(t[p][0], t[p][1], 0x7632), __byte_perm(t[p][2], t[p][3], 0x7632));
+}
+// 32 bytes to a 32-byte boundary.
+__device__ __forceinline__ void stg_u8(void* p, const uint32_t (&r)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 // Vec<T>::N values of element `col` on of row `row` of y: T as they are, or (T = float, terms) as terms.
 template <typename T>

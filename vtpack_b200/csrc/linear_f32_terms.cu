@@ -131,13 +131,17 @@ __device__ __forceinline__ void unscale_or_redo(float (&acc)[NC], const FtArgs& 
     }
 }
 
-// Four output columns of row m from column n on, N and n multiples of four.  HIDDEN: GELU, stored as terms; else + res, as fp32.
-template <bool HIDDEN>
+// What the outputs are: + res, as fp32; as terms; GELU, as terms.
+constexpr int FT_ROWS = 0, FT_TERMS = 1, FT_HIDDEN = 2;
+// Four output columns of row m from column n on, N and n multiples of four.
+template <int OUT>
 __device__ __forceinline__ void finish4(const FtArgs& g, int m, int n, const float4& s, const float4& bias, const float4& res) {
     float v[4] = {s.x + bias.x, s.y + bias.y, s.z + bias.z, s.w + bias.w};
-    if (HIDDEN) {
+    if (OUT != FT_ROWS) {
+        if (OUT == FT_HIDDEN) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = gelu_erf(v[i]);
+            for (int i = 0; i < 4; ++i) v[i] = gelu_erf(v[i]);
+        }
         store_terms4(reinterpret_cast<bf16*>(g.y) + (size_t)m * 3 * g.N + n, (size_t)g.N, v);
     } else {
         if (g.res) { v[0] += res.x; v[1] += res.y; v[2] += res.z; v[3] += res.w; }
@@ -146,7 +150,7 @@ __device__ __forceinline__ void finish4(const FtArgs& g, int m, int n, const flo
 }
 
 // SPLIT: CTAs of a cluster that share a tile's reduction (1: none); it divides the number of groups.
-template <int BN, int SPLIT, bool HIDDEN>
+template <int BN, int SPLIT, int OUT>
 __global__ void __launch_bounds__(FT_THREADS, 1)
 linear_f32_terms_kernel(const __grid_constant__ FtMaps maps, const __grid_constant__ FtArgs g, int* status) {
     using S = FtSmem<BN>;
@@ -295,12 +299,12 @@ linear_f32_terms_kernel(const __grid_constant__ FtMaps maps, const __grid_consta
             // `lane`, else of every sixteen columns four of rows lane / 4 + 8 q.
             constexpr int SC = CW / SPLIT;
             constexpr int NV = SPLIT > 1 ? SC / 4 : CW / 4;
-            float4 res[HIDDEN ? 1 : NV], bias[SPLIT > 1 ? NV : CW / 16];
+            float4 res[OUT != FT_ROWS ? 1 : NV], bias[SPLIT > 1 ? NV : CW / 16];
             auto col_of = [&](int v) { return SPLIT > 1 ? n0 + rank * SC + 4 * v : n0 + (v >> 2) * 16 + (lane & 3) * 4; };
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
                 const int m = SPLIT > 1 ? m0 + lane : m0 + (v & 3) * 8 + (lane >> 2), n = col_of(v);
-                if (!HIDDEN) res[v] = g.res && has && m < M && n < g.N ? *reinterpret_cast<const float4*>(g.res + (size_t)m * g.ldr + n) : zero4;
+                if (OUT == FT_ROWS) res[v] = g.res && has && m < M && n < g.N ? *reinterpret_cast<const float4*>(g.res + (size_t)m * g.ldr + n) : zero4;
                 if (SPLIT > 1 || (v & 3) == 0)
                     bias[SPLIT > 1 ? v : v >> 2] = g.bias && has && n < g.N ? __ldg(reinterpret_cast<const float4*>(g.bias + n)) : zero4;
             }
@@ -390,8 +394,8 @@ linear_f32_terms_kernel(const __grid_constant__ FtMaps maps, const __grid_consta
 #pragma unroll
                     for (int v = 0; v < NV; ++v)
                         if (col_of(v) < g.N)
-                            finish4<HIDDEN>(g, m0 + lane, col_of(v), make_float4(own[4 * v], own[4 * v + 1], own[4 * v + 2], own[4 * v + 3]),
-                                            bias[v], res[HIDDEN ? 0 : v]);
+                            finish4<OUT>(g, m0 + lane, col_of(v), make_float4(own[4 * v], own[4 * v + 1], own[4 * v + 2], own[4 * v + 3]),
+                                            bias[v], res[OUT != FT_ROWS ? 0 : v]);
                 }
             } else if (has) {
                 unscale_or_redo<CW>(acc, g, M, m0, n0, lane);
@@ -410,9 +414,9 @@ linear_f32_terms_kernel(const __grid_constant__ FtMaps maps, const __grid_consta
                     auto finish = [&](int q) {
                         const int rr = q * 8 + (lane >> 2);
                         const float4 v = lds_f4(stage + rr * 64 + (((lane & 3) ^ ((rr >> 1) & 3)) << 4));
-                        if (m0 + rr < M && n < g.N) finish4<HIDDEN>(g, m0 + rr, n, v, bias[b], res[HIDDEN ? 0 : 4 * b + q]);
+                        if (m0 + rr < M && n < g.N) finish4<OUT>(g, m0 + rr, n, v, bias[b], res[OUT != FT_ROWS ? 0 : 4 * b + q]);
                     };
-                    if constexpr (HIDDEN) {
+                    if constexpr (OUT == FT_HIDDEN) {
                         // (not unrolled: most launches run this once per warp, and then what it costs is its fetch)
 #pragma unroll 1
                         for (int q = 0; q < 4; ++q) finish(q);
@@ -434,9 +438,9 @@ linear_f32_terms_kernel(const __grid_constant__ FtMaps maps, const __grid_consta
     if (warp == 1) tmem_dealloc(tmem_base, F_TMEM * BN);
 }
 
-template <int BN, int SPLIT, bool HIDDEN>
+template <int BN, int SPLIT, int OUT>
 static int launch_terms(FtArgs& g, const FtMaps& maps, cudaStream_t st) {
-    auto kern = linear_f32_terms_kernel<BN, SPLIT, HIDDEN>;
+    auto kern = linear_f32_terms_kernel<BN, SPLIT, OUT>;
     static bool attr_set[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -503,7 +507,9 @@ int linear_f32_terms_as(const LinearArgs& p, int bn, int split, cudaStream_t st)
         if (int rc = make_tmap_bf16(&maps.w[i], p.w, 3, dw, strides, bw)) return rc;
     }
 #define VTP_TERMS_CASE(BN, SPLIT) \
-    if (bn == BN && split == SPLIT) return p.out_terms ? launch_terms<BN, SPLIT, true>(g, maps, st) : launch_terms<BN, SPLIT, false>(g, maps, st)
+    if (bn == BN && split == SPLIT) return !p.out_terms ? launch_terms<BN, SPLIT, FT_ROWS>(g, maps, st) \
+                                             : (p.flags & VTP_FLAG_GELU) ? launch_terms<BN, SPLIT, FT_HIDDEN>(g, maps, st) \
+                                                                         : launch_terms<BN, SPLIT, FT_TERMS>(g, maps, st)
     VTP_TERMS_CASE(128, 1);
     VTP_TERMS_CASE(128, 2);
     VTP_TERMS_CASE(128, 4);
@@ -518,9 +524,9 @@ int linear_f32_terms(const LinearArgs& p, cudaStream_t st) {
     if (int rc = linear_validate(p)) return rc;
     VTP_REQUIRE(p.dtype == VTP_F32 && p.N % 8 == 0 && p.K % 8 == 0 && p.ldy % 4 == 0 && (!p.res || p.ldr % 4 == 0), VTP_ERR_SHAPE,
                 "linear (fp32 terms): N=%d K=%d", p.N, p.K);
-    VTP_REQUIRE(p.ln_mode == 0 && !p.emit_stats && p.out_grp == 0 && p.res_mod == 0 && p.out_terms == ((p.flags & VTP_FLAG_GELU) != 0) &&
+    VTP_REQUIRE(p.ln_mode == 0 && !p.emit_stats && p.out_grp == 0 && p.res_mod == 0 && (p.out_terms || !(p.flags & VTP_FLAG_GELU)) &&
                     !(p.out_terms && p.res), VTP_ERR_UNSUPPORTED,
-                "linear (fp32 terms): plain rows, either GELU and terms out or an optional residual and fp32 out");
+                "linear (fp32 terms): plain rows; GELU only with terms out, a residual only with fp32 out");
     if (p.m_max == 0) return VTP_OK;
     const int num_kb = ceil_div(p.K, FK), sms = sm_count();
     // With a device-side row count the worst case is about three times the packed rows of a DGE block.
@@ -529,7 +535,7 @@ int linear_f32_terms(const LinearArgs& p, cudaStream_t st) {
     double best = 0;
     for (int b = 64; b <= 128; b *= 2)
         for (int s = 1; s <= (1 << f32_groups_log2(num_kb)); s *= 2) {
-            const double c = terms_cost(b, s, p.out_terms, m, p.N, num_kb, sms);
+            const double c = terms_cost(b, s, (p.flags & VTP_FLAG_GELU) != 0, m, p.N, num_kb, sms);
             if (best == 0 || c < best) { best = c; bn = b; split = s; }
         }
     return linear_f32_terms_as(p, bn, split, st);
