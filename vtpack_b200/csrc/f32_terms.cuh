@@ -78,7 +78,7 @@ __device__ __forceinline__ void store_row_vec(T* y, size_t row, int C, int col, 
 // The matrices of a block, split on every call: a forward then follows whatever was done to the parameters, and the terms of
 // one block stay in L2 until its Linears read them.
 struct TermSplit {
-    static constexpr int MOST = 6, PER_CTA = 512;      // units of eight values
+    static constexpr int MOST = 6, PER_THREAD = 2;     // units of eight values
     const float* src[MOST] = {}; bf16* dst[MOST] = {};
     int K[MOST] = {};                                  // values per row, a multiple of 8
     unsigned units[MOST] = {};
@@ -87,33 +87,35 @@ struct TermSplit {
         src[n] = static_cast<const float*>(s); dst[n] = static_cast<bf16*>(d); K[n] = k;
         units[n++] = (unsigned)((long long)rows * k / 8);
     }
-    int ctas() const {
+    int ctas(int threads) const {
         int c = 0;
-        for (int i = 0; i < n; ++i) c += (int)((units[i] + PER_CTA - 1) / PER_CTA);
+        for (int i = 0; i < n; ++i) c += (int)((units[i] + PER_THREAD * threads - 1) / (PER_THREAD * threads));
         return c;
     }
 };
-// Share `cta` of the split, by a CTA of 128 threads: four units a thread, all loaded before the first is split.
+// Share `cta` of the split: two units a thread, both loaded before the first is split.
+template <int THREADS>
 __device__ __forceinline__ void split_matrices(const TermSplit& s, int cta) {
+    constexpr int PT = TermSplit::PER_THREAD;
 #pragma unroll 1
     for (int i = 0; i < TermSplit::MOST; ++i) {
-        const int ctas = (int)((s.units[i] + TermSplit::PER_CTA - 1) / TermSplit::PER_CTA);
+        const int ctas = (int)((s.units[i] + PT * THREADS - 1) / (PT * THREADS));
         if (cta >= ctas) { cta -= ctas; continue; }
         const float* src = s.src[i];
         bf16* dst = s.dst[i];
-        const unsigned K8 = (unsigned)s.K[i] / 8, units = s.units[i], u0 = (unsigned)cta * TermSplit::PER_CTA + threadIdx.x;
-        float4 v[4][2];
+        const unsigned K8 = (unsigned)s.K[i] / 8, units = s.units[i], u0 = (unsigned)cta * (PT * THREADS) + threadIdx.x;
+        float4 v[PT][2];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const unsigned u = u0 + j * 128;
+        for (int j = 0; j < PT; ++j) {
+            const unsigned u = u0 + j * THREADS;
             if (u < units) {
                 v[j][0] = __ldg(reinterpret_cast<const float4*>(src + (size_t)u * 8));
                 v[j][1] = __ldg(reinterpret_cast<const float4*>(src + (size_t)u * 8) + 1);
             }
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const unsigned u = u0 + j * 128;
+        for (int j = 0; j < PT; ++j) {
+            const unsigned u = u0 + j * THREADS;
             if (u >= units) return;
             const unsigned r = u / K8, c = u - r * K8;
             const float f[8] = {v[j][0].x, v[j][0].y, v[j][0].z, v[j][0].w, v[j][1].x, v[j][1].y, v[j][1].z, v[j][1].w};

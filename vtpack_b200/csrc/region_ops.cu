@@ -1,11 +1,11 @@
 // Region-parallel token movers used by the fused block forward: router gate, multi-grain
 // pooling (with LayerNorm statistics or explicit LayerNorm rows) and replicate-unpool with
-// residual.  One CTA of four warps owns one 4x4 region of the token grid, whatever grain
-// the gate picked for it: warp w owns grid row w.  A token row is spread over a GROUP of G
-// lanes, each lane holding CPL chunks of 16 bytes (C = G * CPL * 16 bytes exactly, e.g.
-// 16 lanes x 3 chunks at C=384 bf16), so no lane idles and no access needs a bounds check;
-// a warp holds 32/G groups.  All 16 rows of a region are requested before any arithmetic,
-// every region costs the same, and nothing depends on walking the patch list.
+// residual.  One CTA owns one 4x4 region of the token grid, whatever grain the gate picked
+// for it.  A token row is spread over a GROUP of G lanes, each lane holding CPL chunks of 16
+// bytes (C = G * CPL * 16 bytes exactly, e.g. 16 lanes x 3 chunks at C=384 bf16), so no lane
+// idles and no access needs a bounds check; a group owns TPG neighbouring tokens of a grid
+// row.  All 16 rows of a region are requested before any arithmetic, every region costs the
+// same, and nothing depends on walking the patch list.
 // Sums that span tokens go through shared memory: each group sums its own tokens in order,
 // then the partial sums of a patch are added top-left to bottom-right (the reference adds
 // the same tokens in one sequential chain; results differ by fp32 rounding only).
@@ -19,13 +19,22 @@
 
 namespace vtp {
 
-constexpr int RG = 4;              // tokens per region side = warps per CTA
+constexpr int RG = 4;              // tokens per region side
 
+// bf16: four warps, one per grid row, so a group owns 1, 2 or 4 tokens.  fp32: a token per group, 4, 8 or 16 warps.  What a region
+// takes is its longest chain, and an fp32 batch has few regions: DeiT-S, 12 images, pool 16.0 -> 8.0 us, unpool 10.7 -> 6.1 (gate,
+// pool and unpool of bf16 in the same form: DeiT-S, 256 images, 19.6 / 17.1 / 38.5 -> 35 / 26 / 45, DeiT-B, 33 images, pool 7.6 ->
+// 11.0, unpool 14.8 -> 15.1, 7 images no faster: there regions in flight count, and each warp of theirs moves fewer bytes).
 template <typename T, int G, int CPL>
 struct Lay {
     static constexpr int VN = Vec<T>::N;
-    static constexpr int GROUPS = 32 / G;          // token rows a warp holds at once
-    static constexpr int TPG = RG / GROUPS;        // tokens of a grid row per group (4, 2 or 1)
+    static constexpr int GROUPS = 32 / G;                                  // groups of a warp
+    static constexpr int TPG = sizeof(T) == 4 ? 1 : RG / GROUPS;           // tokens of a group
+    static constexpr int THREADS = RG * RG / TPG * G;
+    // Sums that span tokens go through rows of C floats in shared memory: the two halves of each grid row, or (TPG == 4) whole
+    // grid rows too; groups of a whole warp with one token each leave that.
+    static constexpr bool BY_TOKEN = TPG == 1 && G == 32;
+    static constexpr int SLOTS = BY_TOKEN ? RG * RG : RG * 2;
 };
 
 // group-wide sum over the G lanes that share a row
@@ -97,11 +106,11 @@ __device__ __forceinline__ float2 mean_rstd(float2 s, int C, float eps) {
     return make_float2(mean, rsqrtf(fmaxf(s.y / (float)C - mean * mean, 0.f) + eps));
 }
 
-// explicit LayerNorm of a row (two-pass) and store
+// explicit LayerNorm of a row (two-pass), stored in one place or two
 template <typename T, int G, int CPL>
 __device__ __forceinline__ void ln_store(const float (&f)[CPL][Vec<T>::N], int sub, int C,
                                          const float* __restrict__ lnw, const float* __restrict__ lnb, float eps,
-                                         T* y, size_t row, bool terms) {
+                                         T* y, size_t row, bool terms, T* y2 = nullptr, size_t row2 = 0, bool terms2 = false) {
     constexpr int VN = Vec<T>::N;
     float s = 0.f;
 #pragma unroll
@@ -122,6 +131,7 @@ __device__ __forceinline__ void ln_store(const float (&f)[CPL][Vec<T>::N], int s
 #pragma unroll
         for (int i = 0; i < VN; ++i) o[i] = (f[ch][i] - mean) * rstd * __ldg(lnw + c0 + i) + __ldg(lnb + c0 + i);
         store_row_vec<T>(y, row, C, c0, o, terms);
+        if (y2) store_row_vec<T>(y2, row2, C, c0, o, terms2);
     }
 }
 
@@ -156,24 +166,22 @@ __device__ __forceinline__ int derive_first(const int32_t* __restrict__ counts, 
     return part_sum + num_extra + own;
 }
 
-// Each group leaves the in-order sum of its tokens of grid row w in shared memory.
-// Slot layout: part[(w * 2 + half) * C], half 0 = left two tokens of the row, 1 = right two.
-// A group that owns the whole row (TPG == 4) fills slot (w, 0) only, unless it was told to
-// split (`left` holds the first two tokens, `acc` the last two).  Groups that own a single
-// token (TPG == 1) are paired through shared memory.  Ends with the CTA barrier.
+// Each group `gi` leaves the in-order sum `acc` of its tokens in shared memory.  Slot layout: part[(w * 2 + half) * C], half 0 = left
+// two tokens of grid row w, 1 = right two.  A group that owns a whole row (TPG == 4) fills slot (w, 0) only, unless it was told to
+// split.  Groups that own a single token are paired through shared memory, or (BY_TOKEN) leave it in a slot of its own.
+// Ends with the CTA barrier.
 template <typename T, int G, int CPL>
-__device__ __forceinline__ void publish_partials(float* part, float (&acc)[CPL][Vec<T>::N], int w, int grp, int sub,
-                                                 int C) {
-    constexpr int TPG = Lay<T, G, CPL>::TPG;
-    if (TPG == 4) {
-        smem_store<T, CPL>(part + (size_t)(w * 2) * C, acc, sub, G);
-    } else if (TPG == 2) {
-        smem_store<T, CPL>(part + (size_t)(w * 2 + grp) * C, acc, sub, G);
+__device__ __forceinline__ void publish_partials(float* part, float (&acc)[CPL][Vec<T>::N], int gi, int sub, int C) {
+    using L = Lay<T, G, CPL>;
+    if (L::TPG == 4) {
+        smem_store<T, CPL>(part + (size_t)(gi * 2) * C, acc, sub, G);
+    } else if (L::TPG == 2 || L::BY_TOKEN) {
+        smem_store<T, CPL>(part + (size_t)gi * C, acc, sub, G);
     } else {
-        float* slot = part + (size_t)(w * 2 + (grp >> 1)) * C;
-        if ((grp & 1) == 0) smem_store<T, CPL>(slot, acc, sub, G);
+        float* slot = part + (size_t)(gi >> 1) * C;
+        if ((gi & 1) == 0) smem_store<T, CPL>(slot, acc, sub, G);
         __syncwarp();
-        if ((grp & 1) == 1) {
+        if ((gi & 1) == 1) {
             float tmp[CPL][Vec<T>::N];
             zero_f<T, CPL>(tmp);
             smem_add<T, CPL>(tmp, slot, sub, G);          // even token first, then the odd one
@@ -185,6 +193,25 @@ __device__ __forceinline__ void publish_partials(float* part, float (&acc)[CPL][
         }
     }
     __syncthreads();
+}
+// acc += the left or right half (tokens) of grid row w, or (HALVES == 2) the whole row.  The order in which a region's tokens are
+// added does not depend on TPG where G does not.
+template <typename T, int G, int CPL, int HALVES>
+__device__ __forceinline__ void add_row(float (&acc)[CPL][Vec<T>::N], const float* part, int w, int half, int sub, int C) {
+    using L = Lay<T, G, CPL>;
+    if (L::BY_TOKEN) {
+        float sum[CPL][Vec<T>::N];
+        zero_f<T, CPL>(sum);
+#pragma unroll
+        for (int j = 0; j < 2 * HALVES; ++j) smem_add<T, CPL>(sum, part + (size_t)(w * RG + 2 * half + j) * C, sub, G);
+#pragma unroll
+        for (int ch = 0; ch < CPL; ++ch)
+#pragma unroll
+            for (int i = 0; i < Vec<T>::N; ++i) acc[ch][i] += sum[ch][i];
+    } else {
+        smem_add<T, CPL>(acc, part + (size_t)(w * 2 + half) * C, sub, G);
+        if (HALVES == 2 && L::TPG != 4) smem_add<T, CPL>(acc, part + (size_t)(w * 2 + 1) * C, sub, G);
+    }
 }
 
 // ------------------------------------------------------------------------------- pool
@@ -204,11 +231,14 @@ constexpr int POOL_LN = 0, POOL_STATS = 1, POOL_PLAIN = 2, POOL_COLS = 3;
 // (A thread of a narrow-row layout holds one or two 16-byte vectors of a region: such kernels run with 16 or 12 CTAs per SM
 // (a few spilled words in the unpool; measured faster all the same), and the kernel is bound by how many regions are in flight.)
 template <typename T, int G, int CPL>
-constexpr int pool_ctas() { return Lay<T, G, CPL>::TPG * CPL <= 1 ? 16 : Lay<T, G, CPL>::TPG * CPL <= 2 ? 12 : 7; }
+constexpr int pool_ctas() {
+    if (Lay<T, G, CPL>::THREADS != 128) return G == 16 ? (CPL <= 2 ? 6 : 4) : CPL <= 2 ? 3 : CPL <= 3 ? 2 : 1;
+    return Lay<T, G, CPL>::TPG * CPL <= 1 ? 16 : Lay<T, G, CPL>::TPG * CPL <= 2 ? 12 : 7;
+}
 // (terms: POOL_LN of fp32 rows only; 1: xn, 2: qn as terms)
 template <typename T, int G, int CPL, int MODE>
 __device__ __forceinline__ void
-pool_region(const T* __restrict__ x, RegionGeom g, const int32_t* __restrict__ idx,
+pool_region(const int rid, const T* __restrict__ x, RegionGeom g, const int32_t* __restrict__ idx,
                    const int32_t* __restrict__ region_first, const int32_t* __restrict__ offsets,
                    const int32_t* __restrict__ counts, int32_t* __restrict__ offsets_out,
                    int32_t* __restrict__ region_first_out, int32_t* __restrict__ counts_next, Splits sp,
@@ -219,15 +249,16 @@ pool_region(const T* __restrict__ x, RegionGeom g, const int32_t* __restrict__ i
     constexpr bool COLS = MODE == POOL_COLS, STATS = MODE == POOL_STATS || COLS, EXPLICIT_LN = MODE == POOL_LN;
     using L = Lay<T, G, CPL>;
     constexpr int VN = L::VN, GROUPS = L::GROUPS, TPG = L::TPG;
-    extern __shared__ float part[];          // [4 grid rows][2 halves][C] partial sums
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int grp = lane / G, sub = lane % G;
+    extern __shared__ float part[];          // [SLOTS][C] partial sums
+    __shared__ int first_s;
+    const int lane = threadIdx.x & 31, sub = lane % G;
+    const int gi = (int)(threadIdx.x >> 5) * GROUPS + lane / G;      // the group, its tokens: row w, columns col0 .. col0 + TPG - 1
+    const int w = gi * TPG / RG, col0 = gi * TPG % RG;
     const int R = g.Hr * g.Wr;
-    const int rid = blockIdx.x;
 
     if (rid >= g.B * R) {
         // ---- extra (cls) tokens: one per group, copied
-        const int e = ((rid - g.B * R) * RG + w) * GROUPS + grp;
+        const int e = (rid - g.B * R) * (RG * RG / TPG) + gi;
         if (e >= g.B * g.num_extra) return;
         const int b = e / g.num_extra, t = e % g.num_extra;
         const size_t src_row = (size_t)b * g.N + t;
@@ -273,8 +304,7 @@ pool_region(const T* __restrict__ x, RegionGeom g, const int32_t* __restrict__ i
     const int k = min(max(idx[rid], 0), sp.n - 1);
     const int s = sp.v[k];                     // sub-patches per region side: 4, 2 or 1
     const int step = RG / s;
-    // this group's tokens: grid row w, columns grp*TPG .. grp*TPG + TPG - 1
-    const size_t tok0 = (size_t)b * g.N + g.num_extra + (size_t)(ry * RG + w) * g.W + rx * RG + grp * TPG;
+    const size_t tok0 = (size_t)b * g.N + g.num_extra + (size_t)(ry * RG + w) * g.W + rx * RG + col0;
 
     Vec<T> rows[TPG][CPL];
 #pragma unroll
@@ -289,18 +319,30 @@ pool_region(const T* __restrict__ x, RegionGeom g, const int32_t* __restrict__ i
             return;
         }
     } else {
-        int img_base;
-        first = derive_first(counts, idx, b, rr, R, sp, g.num_extra, lane, &img_base);
-        if (w == 0 && lane == 0) {
-            region_first_out[rid] = first;
-            if (rr == 0) {
-                offsets_out[b] = img_base;
-                if (b == g.B - 1) offsets_out[g.B] = img_base + counts[b];
+        // One warp adds up the counts in front while the rows are on their way: with every warp doing it PVT-small's stage 1, 96
+        // images, takes 65.8 us instead of 57.5 (DeiT-B, 33 images: 1443 / 1433 us); of two tokens a group, where the barrier
+        // costs more (DeiT-S, 256 images: 16.5 / 17.0 us), each warp does.
+        constexpr bool EACH = TPG == 2;
+        if (EACH || threadIdx.x < 32) {
+            int img_base;
+            const int at = derive_first(counts, idx, b, rr, R, sp, g.num_extra, lane, &img_base);
+            first = at;
+            if (threadIdx.x == 0) {
+                first_s = at;
+                region_first_out[rid] = at;
+                if (rr == 0) {
+                    offsets_out[b] = img_base;
+                    if (b == g.B - 1) offsets_out[g.B] = img_base + counts[b];
+                }
             }
+        }
+        if (!EACH) {
+            __syncthreads();
+            first = first_s;
         }
     }
     // a grid without extra tokens has no extra-token CTA to start the next block's count
-    if (rr == 0 && w == 0 && lane == 0 && counts_next && g.num_extra == 0) counts_next[b] = 0;
+    if (rr == 0 && threadIdx.x == 0 && counts_next && g.num_extra == 0) counts_next[b] = 0;
 
     // per token: statistics / explicit LayerNorm, and at the finest grain the token is its own patch
     float acc[CPL][VN];                          // in-order sum of this group's tokens (of the current half)
@@ -309,7 +351,7 @@ pool_region(const T* __restrict__ x, RegionGeom g, const int32_t* __restrict__ i
     for (int j = 0; j < TPG; ++j) {
         float f[CPL][VN];
         to_f<T, CPL>(f, rows[j]);
-        const int col = grp * TPG + j;                        // column inside the grid row
+        const int col = col0 + j;                             // column inside the grid row
         const int prow = first + w * RG + col;                // packed row if step == 1
         if (STATS) {
             float2 st = make_float2(0.f, 1.f);
@@ -343,8 +385,7 @@ pool_region(const T* __restrict__ x, RegionGeom g, const int32_t* __restrict__ i
                 }
             }
         } else if (EXPLICIT_LN) {
-            ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, xn, tok0 + j, terms & 1);
-            if (step == 1) ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, qn, (size_t)prow, terms & 2);
+            ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, xn, tok0 + j, terms & 1, step == 1 ? qn : nullptr, (size_t)prow, terms & 2);
         }
         if (step == 1) {
             store_row<T, CPL>(rows[j], comp + (size_t)prow * g.C, sub, G);
@@ -366,24 +407,20 @@ pool_region(const T* __restrict__ x, RegionGeom g, const int32_t* __restrict__ i
         smem_store<T, CPL>(part + (size_t)(w * 2 + 1) * g.C, acc, sub, G);
         __syncthreads();
     } else {
-        publish_partials<T, G, CPL>(part, acc, w, grp, sub, g.C);
+        publish_partials<T, G, CPL>(part, acc, gi, sub, g.C);
     }
-    const bool row_in_one_slot = (TPG == 4) && step == 4;     // slot (w, 0) holds the whole grid row
 
-    // finishing: unit u = w * GROUPS + grp takes patch u.  step 2: four patches (dy, dx); step 4: one.
-    const int u = w * GROUPS + grp;
-    if (u >= s * s) return;
-    const int dy = (step == 2) ? (u >> 1) : 0;
-    const int dx = (step == 2) ? (u & 1) : 0;
+    // finishing: group gi takes patch gi.  step 2: four patches (dy, dx); step 4: one.
+    if (gi >= s * s) return;
+    const int dy = (step == 2) ? (gi >> 1) : 0;
+    const int dx = (step == 2) ? (gi & 1) : 0;
     zero_f<T, CPL>(acc);
     if (step == 2) {
-        smem_add<T, CPL>(acc, part + (size_t)((2 * dy) * 2 + dx) * g.C, sub, G);
-        smem_add<T, CPL>(acc, part + (size_t)((2 * dy + 1) * 2 + dx) * g.C, sub, G);
+        add_row<T, G, CPL, 1>(acc, part, 2 * dy, dx, sub, g.C);
+        add_row<T, G, CPL, 1>(acc, part, 2 * dy + 1, dx, sub, g.C);
     } else {
-        for (int r2 = 0; r2 < RG; ++r2) {
-            smem_add<T, CPL>(acc, part + (size_t)(r2 * 2) * g.C, sub, G);
-            if (!row_in_one_slot) smem_add<T, CPL>(acc, part + (size_t)(r2 * 2 + 1) * g.C, sub, G);
-        }
+#pragma unroll 1
+        for (int r2 = 0; r2 < RG; ++r2) add_row<T, G, CPL, 2>(acc, part, r2, 0, sub, g.C);
     }
     // step * step is 4 or 16: multiplying by its reciprocal is the division, bit for bit
     const float inv_denom = sum_only ? 1.0f : 1.0f / (float)(step * step);
@@ -403,7 +440,7 @@ pool_region(const T* __restrict__ x, RegionGeom g, const int32_t* __restrict__ i
 }
 
 template <typename T, int G, int CPL, int MODE>
-__global__ void __launch_bounds__(128, (pool_ctas<T, G, CPL>()))
+__global__ void __launch_bounds__((Lay<T, G, CPL>::THREADS), (pool_ctas<T, G, CPL>()))
 pool_region_kernel(const T* __restrict__ x, RegionGeom g, const int32_t* __restrict__ idx,
                    const int32_t* __restrict__ region_first, const int32_t* __restrict__ offsets,
                    const int32_t* __restrict__ counts, int32_t* __restrict__ offsets_out,
@@ -413,25 +450,28 @@ pool_region_kernel(const T* __restrict__ x, RegionGeom g, const int32_t* __restr
                    const float* __restrict__ lnb, float eps, T* __restrict__ xn, T* __restrict__ qn, int sum_only,
                    int sr, int* status) {
     pdl_begin();
-    pool_region<T, G, CPL, MODE>(x, g, idx, region_first, offsets, counts, offsets_out, region_first_out, counts_next, sp, comp,
+    pool_region<T, G, CPL, MODE>((int)blockIdx.x, x, g, idx, region_first, offsets, counts, offsets_out, region_first_out, counts_next, sp, comp,
                                  stats_x, stats_q, stats_acc, write_stats_x, lnw, lnb, eps, xn, qn, sum_only, sr, status, 0);
 }
-// The pool of an fp32 block whose Linears take terms.  The CTAs behind the pool's split the block's matrices, which nothing in
-// front of this kernel needs: the pool waits on its rows, the split on its own, and a launch is saved.
+// The pool of an fp32 block whose Linears take terms.  The CTAs in front of the pool's split the block's matrices, and do not wait
+// for the kernel in front: that is always one of the same call (the gate, or the unpool of the block before), which let this one start
+// only once everything before itself had completed, whatever wrote the parameters and the Linears that read the last
+// block's terms among it.  So the split runs beside the end of that kernel (behind the pool's CTAs, in a kernel that
+// started late: DeiT-S, 12 images, 17.3 us a block instead of 16.0).
 template <int G, int CPL>
-__global__ void __launch_bounds__(128, (pool_ctas<float, G, CPL>()))
+__global__ void __launch_bounds__((Lay<float, G, CPL>::THREADS), (pool_ctas<float, G, CPL>()))
 pool_region_terms_kernel(const float* __restrict__ x, RegionGeom g, const int32_t* __restrict__ idx,
                          const int32_t* __restrict__ region_first, const int32_t* __restrict__ offsets,
                          const int32_t* __restrict__ counts, int32_t* __restrict__ offsets_out,
                          int32_t* __restrict__ region_first_out, int32_t* __restrict__ counts_next, Splits sp,
                          float* __restrict__ comp, const float* __restrict__ lnw, const float* __restrict__ lnb, float eps,
-                         float* __restrict__ xn, float* __restrict__ qn, int terms, int pool_grid, TermSplit split) {
-    pdl_begin();
-    if ((int)blockIdx.x >= pool_grid) {
-        split_matrices(split, (int)blockIdx.x - pool_grid);
+                         float* __restrict__ xn, float* __restrict__ qn, int terms, int split_grid, TermSplit split) {
+    if ((int)blockIdx.x < split_grid) {
+        split_matrices<Lay<float, G, CPL>::THREADS>(split, (int)blockIdx.x);
         return;
     }
-    pool_region<float, G, CPL, POOL_LN>(x, g, idx, region_first, offsets, counts, offsets_out, region_first_out, counts_next, sp,
+    pdl_begin();
+    pool_region<float, G, CPL, POOL_LN>((int)blockIdx.x - split_grid, x, g, idx, region_first, offsets, counts, offsets_out, region_first_out, counts_next, sp,
                                         comp, nullptr, nullptr, nullptr, 0, lnw, lnb, eps, xn, qn, 0, 1, nullptr, terms);
 }
 
@@ -445,13 +485,10 @@ __device__ __forceinline__ void gate_from_partials(const float* part, int C, int
                                                    int32_t* __restrict__ idx_out, int rid, int32_t* counts_img,
                                                    const Splits& sp, const float* __restrict__ img_bias) {
     constexpr int VN = Vec<T>::N;
-    constexpr bool both_halves = Lay<T, G, CPL>::TPG != 4;
     float acc[CPL][VN];
     zero_f<T, CPL>(acc);
-    for (int r2 = 0; r2 < RG; ++r2) {
-        smem_add<T, CPL>(acc, part + (size_t)(r2 * 2) * C, sub, G);
-        if (both_halves) smem_add<T, CPL>(acc, part + (size_t)(r2 * 2 + 1) * C, sub, G);
-    }
+#pragma unroll 1
+    for (int r2 = 0; r2 < RG; ++r2) add_row<T, G, CPL, 2>(acc, part, r2, 0, sub, C);
     // the region mean: 1/16 is a power of two, so the product equals the quotient
 #pragma unroll
     for (int ch = 0; ch < CPL; ++ch)
@@ -489,21 +526,27 @@ __device__ __forceinline__ void gate_from_partials(const float* part, int C, int
 // out[b,tok] = ref[b,tok] + (q[p] - comp[p]) for the patch p that covers the token; optionally
 // also the next block's token statistics, router gate decisions and per-image counts.
 template <typename T, int G, int CPL>
-__global__ void __launch_bounds__(128, (Lay<T, G, CPL>::TPG * CPL <= 1) ? 16 : ((Lay<T, G, CPL>::TPG * CPL <= 2) ? 12 : 4))
+constexpr int unpool_ctas() {
+    if (Lay<T, G, CPL>::THREADS != 128) return G == 16 ? (CPL <= 2 ? 6 : 3) : CPL <= 2 ? 3 : CPL <= 3 ? 2 : 1;
+    return Lay<T, G, CPL>::TPG * CPL <= 1 ? 16 : Lay<T, G, CPL>::TPG * CPL <= 2 ? 12 : 4;
+}
+template <typename T, int G, int CPL>
+__global__ void __launch_bounds__((Lay<T, G, CPL>::THREADS), (unpool_ctas<T, G, CPL>()))
 unpool_region_kernel(const T* __restrict__ q, const T* __restrict__ comp, const T* ref, T* out, RegionGeom g,
                      const int32_t* __restrict__ idx, const int32_t* __restrict__ region_first,
                      const int32_t* __restrict__ offsets, Splits sp, NextBlock nx) {
     pdl_begin();
     using L = Lay<T, G, CPL>;
     constexpr int VN = L::VN, GROUPS = L::GROUPS, TPG = L::TPG;
-    extern __shared__ float part[];          // [4 grid rows][2 halves][C] row sums of the output (next gate)
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int grp = lane / G, sub = lane % G;
+    extern __shared__ float part[];          // [SLOTS][C] sums of the output (next gate)
+    const int lane = threadIdx.x & 31, sub = lane % G;
+    const int gi = (int)(threadIdx.x >> 5) * GROUPS + lane / G;
+    const int w = gi * TPG / RG, col0 = gi * TPG % RG;
     const int R = g.Hr * g.Wr;
     const int rid = blockIdx.x;
 
     if (rid >= g.B * R) {
-        const int e = ((rid - g.B * R) * RG + w) * GROUPS + grp;
+        const int e = (rid - g.B * R) * (RG * RG / TPG) + gi;
         if (e >= g.B * g.num_extra) return;
         const int b = e / g.num_extra, t = e % g.num_extra;
         const size_t tok = (size_t)b * g.N + t;
@@ -531,7 +574,7 @@ unpool_region_kernel(const T* __restrict__ q, const T* __restrict__ comp, const 
     const int s = sp.v[k];
     const int step = RG / s;
     const int first = region_first[rid];
-    const size_t tok0 = (size_t)b * g.N + g.num_extra + (size_t)(ry * RG + w) * g.W + rx * RG + grp * TPG;
+    const size_t tok0 = (size_t)b * g.N + g.num_extra + (size_t)(ry * RG + w) * g.W + rx * RG + col0;
     const int prow = first + (w / step) * s;            // packed row of this grid row's first patch
 
     // every row this group needs, requested up front: TPG reference rows and the patch rows they map to.
@@ -542,7 +585,7 @@ unpool_region_kernel(const T* __restrict__ q, const T* __restrict__ comp, const 
     Vec<T> rrow[TPG][CPL], qrow[TPG][CPL], crow[TPG][CPL];
 #pragma unroll
     for (int j = 0; j < TPG; ++j) {
-        const int col = grp * TPG + j;
+        const int col = col0 + j;
         if (!fine) load_row<T, CPL>(rrow[j], ref + (tok0 + j) * g.C, sub, G);
         if (j == 0 || (col % step) == 0) {               // a new patch starts at this column
             const int p = prow + col / step;
@@ -556,7 +599,7 @@ unpool_region_kernel(const T* __restrict__ q, const T* __restrict__ comp, const 
     zero_f<T, CPL>(d);
 #pragma unroll
     for (int j = 0; j < TPG; ++j) {
-        const int col = grp * TPG + j;
+        const int col = col0 + j;
         if (j == 0 || (col % step) == 0) {
             to_f<T, CPL>(d, qrow[j]);
             if (!fine) {
@@ -595,8 +638,8 @@ unpool_region_kernel(const T* __restrict__ q, const T* __restrict__ comp, const 
     }
     if (!nx.gw) return;
     // ---- the next block's router gate on the region this CTA has just written
-    publish_partials<T, G, CPL>(part, acc, w, grp, sub, g.C);
-    if (w != 0 || grp != 0) return;
+    publish_partials<T, G, CPL>(part, acc, gi, sub, g.C);
+    if (gi != 0) return;
     gate_from_partials<T, G, CPL>(part, g.C, sub, nx.gw, nx.gb, nx.S, nx.logits, nx.idx, rid,
                                   nx.counts ? nx.counts + b : nullptr, sp,
                                   nx.image_bias ? nx.image_bias + (size_t)b * nx.S : nullptr);
@@ -605,7 +648,7 @@ unpool_region_kernel(const T* __restrict__ q, const T* __restrict__ comp, const 
 // Stand-alone gate (first block of a model, or a block called on its own); optionally also
 // writes the LayerNorm statistics of every token row it reads.
 template <typename T, int G, int CPL>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__((Lay<T, G, CPL>::THREADS))
 gate_region_kernel(const T* __restrict__ x, RegionGeom g, const float* __restrict__ gw,
                    const float* __restrict__ gb, int S, float* __restrict__ logits_out,
                    int32_t* __restrict__ idx_out, float2* __restrict__ stats_x, float eps,
@@ -613,14 +656,15 @@ gate_region_kernel(const T* __restrict__ x, RegionGeom g, const float* __restric
     pdl_begin();
     using L = Lay<T, G, CPL>;
     constexpr int VN = L::VN, GROUPS = L::GROUPS, TPG = L::TPG;
-    extern __shared__ float part[];          // [4][2][C]
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int grp = lane / G, sub = lane % G;
+    extern __shared__ float part[];          // [SLOTS][C]
+    const int lane = threadIdx.x & 31, sub = lane % G;
+    const int gi = (int)(threadIdx.x >> 5) * GROUPS + lane / G;
+    const int w = gi * TPG / RG, col0 = gi * TPG % RG;
     const int R = g.Hr * g.Wr;
     const int rid = blockIdx.x;
     if (rid >= g.B * R) {
         // extra (cls) tokens only matter for the statistics
-        const int e = ((rid - g.B * R) * RG + w) * GROUPS + grp;
+        const int e = (rid - g.B * R) * (RG * RG / TPG) + gi;
         if (!stats_x || e >= g.B * g.num_extra) return;
         const size_t tok = (size_t)(e / g.num_extra) * g.N + e % g.num_extra;
         Vec<T> row[CPL];
@@ -633,7 +677,7 @@ gate_region_kernel(const T* __restrict__ x, RegionGeom g, const float* __restric
     }
     const int b = rid / R, rr = rid % R;
     const int ry = rr / g.Wr, rx = rr % g.Wr;
-    const size_t tok0 = (size_t)b * g.N + g.num_extra + (size_t)(ry * RG + w) * g.W + rx * RG + grp * TPG;
+    const size_t tok0 = (size_t)b * g.N + g.num_extra + (size_t)(ry * RG + w) * g.W + rx * RG + col0;
     Vec<T> rows[TPG][CPL];
 #pragma unroll
     for (int j = 0; j < TPG; ++j) load_row<T, CPL>(rows[j], x + (tok0 + j) * g.C, sub, G);
@@ -652,8 +696,8 @@ gate_region_kernel(const T* __restrict__ x, RegionGeom g, const float* __restric
 #pragma unroll
             for (int i = 0; i < VN; ++i) acc[ch][i] += f[ch][i];
     }
-    publish_partials<T, G, CPL>(part, acc, w, grp, sub, g.C);
-    if (w != 0 || grp != 0) return;
+    publish_partials<T, G, CPL>(part, acc, gi, sub, g.C);
+    if (gi != 0) return;
     gate_from_partials<T, G, CPL>(part, g.C, sub, gw, gb, S, logits_out, idx_out, rid, counts ? counts + b : nullptr, sp,
                                   image_bias ? image_bias + (size_t)b * S : nullptr);
 }
@@ -669,35 +713,51 @@ static bool pick_layout(int nchunks, int* G, int* CPL) {
     return false;
 }
 
+template <typename L>
+static size_t region_smem(int C) { return (size_t)L::SLOTS * C * sizeof(float); }
+// (static shared memory counts towards the 48 KB that need no leave)
+template <typename Kernel>
+static void allow_smem(Kernel kern, size_t bytes) {
+    if (bytes > 47 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
 template <typename T, int G, int CPL>
 static void launch_pool_t(const RegionPoolArgs& a, cudaStream_t st) {
     const int R = a.g.Hr * a.g.Wr;
-    const int grid = a.g.B * R + ceil_div(a.g.B * a.g.num_extra, RG * (32 / G));
-    const size_t smem = (size_t)8 * a.g.C * sizeof(float);
+    using L = Lay<T, G, CPL>;
+    const int grid = a.g.B * R + ceil_div(a.g.B * a.g.num_extra, RG * RG / L::TPG);
+    const dim3 block(L::THREADS);
+    const size_t smem = region_smem<L>(a.g.C);
     if constexpr (sizeof(T) == 4) {
         if (a.qn_terms) {
-            launch_chain(pool_region_terms_kernel<G, CPL>, dim3(grid + a.split.ctas()), dim3(128), smem, st, (const float*)a.x, a.g,
+            const int split_grid = a.split.ctas(L::THREADS);
+            allow_smem(pool_region_terms_kernel<G, CPL>, smem);
+            launch_kernel(pool_region_terms_kernel<G, CPL>, true, 1, dim3(split_grid + grid), block, smem, st, (const float*)a.x, a.g,
                 a.idx, a.region_first, a.offsets, a.counts, a.offsets_out, a.region_first_out, a.counts_next, a.sp, (float*)a.comp,
-                a.lnw, a.lnb, a.eps, (float*)a.xn, (float*)a.qn, a.xn_terms ? 3 : 2, grid, a.split);
+                a.lnw, a.lnb, a.eps, (float*)a.xn, (float*)a.qn, a.xn_terms ? 3 : 2, split_grid, a.split);
             return;
         }
     }
+    auto launch = [&](auto kern, auto... args) {
+        allow_smem(kern, smem);
+        launch_chain(kern, dim3(grid), block, smem, st, args...);
+    };
     if (a.stats_q && a.sr > 1)
-        launch_chain(pool_region_kernel<T, G, CPL, POOL_COLS>, dim3(grid), dim3(128), smem, st, 
+        launch(pool_region_kernel<T, G, CPL, POOL_COLS>,
             (const T*)a.x, a.g, a.idx, a.region_first, a.offsets, a.counts, a.offsets_out, a.region_first_out,
             a.counts_next, a.sp, (T*)a.comp, a.stats_x, a.stats_q, a.stats_acc, a.stats_x_ready ? 0 : 1, a.lnw,
             a.lnb, a.eps, (T*)a.cols, nullptr, 0, a.sr, nullptr);
     else if (a.stats_q)
-        launch_chain(pool_region_kernel<T, G, CPL, POOL_STATS>, dim3(grid), dim3(128), smem, st, 
+        launch(pool_region_kernel<T, G, CPL, POOL_STATS>,
             (const T*)a.x, a.g, a.idx, a.region_first, a.offsets, a.counts, a.offsets_out, a.region_first_out,
             a.counts_next, a.sp, (T*)a.comp, a.stats_x, a.stats_q, a.stats_acc, a.stats_x_ready ? 0 : 1, nullptr,
             nullptr, a.eps, nullptr, nullptr, 0, 1, nullptr);
     else if (a.xn && a.qn)
-        launch_chain(pool_region_kernel<T, G, CPL, POOL_LN>, dim3(grid), dim3(128), smem, st, 
+        launch(pool_region_kernel<T, G, CPL, POOL_LN>,
             (const T*)a.x, a.g, a.idx, a.region_first, a.offsets, a.counts, a.offsets_out, a.region_first_out,
             a.counts_next, a.sp, (T*)a.comp, nullptr, nullptr, nullptr, 0, a.lnw, a.lnb, a.eps, (T*)a.xn, (T*)a.qn, 0, 1, nullptr);
     else
-        launch_chain(pool_region_kernel<T, G, CPL, POOL_PLAIN>, dim3(grid), dim3(128), smem, st, 
+        launch(pool_region_kernel<T, G, CPL, POOL_PLAIN>,
             (const T*)a.x, a.g, a.idx, a.region_first, a.offsets, a.counts, a.offsets_out, a.region_first_out,
             a.counts_next, a.sp, (T*)a.comp, nullptr, nullptr, nullptr, 0, nullptr, nullptr, a.eps, nullptr, nullptr,
             a.sum_only ? 1 : 0, 1, device_status_ptr());
@@ -706,16 +766,22 @@ static void launch_pool_t(const RegionPoolArgs& a, cudaStream_t st) {
 template <typename T, int G, int CPL>
 static void launch_unpool_t(const RegionUnpoolArgs& a, cudaStream_t st) {
     const int R = a.g.Hr * a.g.Wr;
-    const int grid = a.g.B * R + ceil_div(a.g.B * a.g.num_extra, RG * (32 / G));
-    launch_chain(unpool_region_kernel<T, G, CPL>, dim3(grid), dim3(128), (size_t)8 * a.g.C * sizeof(float), st, 
+    using L = Lay<T, G, CPL>;
+    const int grid = a.g.B * R + ceil_div(a.g.B * a.g.num_extra, RG * RG / L::TPG);
+    const size_t smem = a.next.gw ? region_smem<L>(a.g.C) : 0;
+    allow_smem(unpool_region_kernel<T, G, CPL>, smem);
+    launch_chain(unpool_region_kernel<T, G, CPL>, dim3(grid), dim3(L::THREADS), smem, st,
         (const T*)a.q, (const T*)a.comp, (const T*)a.ref, (T*)a.out, a.g, a.idx, a.region_first, a.offsets, a.sp, a.next);
 }
 
 template <typename T, int G, int CPL>
 static void launch_gate_t(const RegionGateArgs& a, cudaStream_t st) {
     const int R = a.g.Hr * a.g.Wr;
-    const int grid = a.g.B * R + (a.stats_x ? ceil_div(a.g.B * a.g.num_extra, RG * (32 / G)) : 0);
-    launch_chain(gate_region_kernel<T, G, CPL>, dim3(grid), dim3(128), (size_t)8 * a.g.C * sizeof(float), st, 
+    using L = Lay<T, G, CPL>;
+    const int grid = a.g.B * R + (a.stats_x ? ceil_div(a.g.B * a.g.num_extra, RG * RG / L::TPG) : 0);
+    const size_t smem = region_smem<L>(a.g.C);
+    allow_smem(gate_region_kernel<T, G, CPL>, smem);
+    launch_chain(gate_region_kernel<T, G, CPL>, dim3(grid), dim3(L::THREADS), smem, st,
         (const T*)a.x, a.g, a.gw, a.gb, a.S, a.logits_out, a.idx_out, a.stats_x, a.eps, a.image_bias, a.counts, a.sp);
 }
 
