@@ -11,6 +11,11 @@ from ..runtime import dtype_code, ptr, require_cuda, stream_ptr
 _MODES = {"point": 0, "channel": 1}
 
 
+def _dense(t, dtype):
+    """t in this type, contiguous (itself where it is)."""
+    return t if t.dtype is dtype and t.is_contiguous() else t.to(dtype).contiguous()
+
+
 def _dims(input, grid):
     B, H, W, C = input.shape
     return B, H, W, C, grid.shape[1], grid.shape[2]
@@ -25,9 +30,7 @@ class _BilinearAttention(Function):
         if mode not in _MODES:
             raise NotImplementedError(f"Mode {mode} is not supported")
         require_cuda(input, grid, weight)
-        input = input.contiguous()
-        grid = grid.to(input.dtype).contiguous()
-        weight = weight.to(input.dtype).contiguous()
+        input, grid, weight = _dense(input, input.dtype), _dense(grid, input.dtype), _dense(weight, input.dtype)
         B, H, W, C, G, P = _dims(input, grid)
         assert grid.shape == (B, G, P, 2) and weight.shape == (B, G, P if mode == "point" else C), \
             "grid must be [B,G,P,2] and weight [B,G,P] (point) or [B,G,C] (channel)"
@@ -43,7 +46,7 @@ class _BilinearAttention(Function):
     @once_differentiable
     def backward(ctx, grad_output):
         input, grid, weight = ctx.saved_tensors
-        grad_output = grad_output.to(input.dtype).contiguous()
+        grad_output = _dense(grad_output, input.dtype)
         B, H, W, C, G, P = _dims(input, grid)
         grad_input, grad_grid, grad_weight = torch.empty_like(input), torch.empty_like(grid), torch.empty_like(weight)
         _lib.check(_lib.lib().vtp_bilinear_attention_backward(

@@ -19,8 +19,16 @@ def dtype_code(t: torch.dtype) -> int:
     raise TypeError(f"vtpack_b200 supports float32 and bfloat16, got {t}")
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)     # (absent from builds of torch without CUDA)
+
+
 def stream_ptr(device=None) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """The current stream of `device` as the library takes it.  Asked for its number only: making the Stream object costs
+    4 us, as much as the launch that follows."""
+    if _raw_stream is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    index = None if device is None else torch.device(device).index
+    return _raw_stream(torch.cuda.current_device() if index is None else index)
 
 
 def require_cuda(*tensors):
@@ -35,7 +43,7 @@ def ptr(t):
 
 _scratch = {}       # (device type, index, use) -> buffer
 _scratch_gen = {}   # (device type, index, use) -> how many times the buffer was replaced
-_scratch_users = {}  # (device type, index, use) -> streams that have been handed the current buffer
+_scratch_users = {}  # (device type, index, use) -> {stream number: stream} that have been handed the current buffer
 
 
 def scratch(device, nbytes: int, use: str = "block") -> torch.Tensor:
@@ -49,18 +57,18 @@ def scratch(device, nbytes: int, use: str = "block") -> torch.Tensor:
     (``scratch_generation`` changes)."""
     key = (device.type, device.index, use)
     buf = _scratch.get(key)
-    cur = torch.cuda.current_stream(device)
     if buf is None or buf.numel() < nbytes:
         if buf is not None:
-            for st in _scratch_users.get(key, ()):
+            for st in _scratch_users.get(key, {}).values():
                 buf.record_stream(st)          # kernels queued on st may still be using the old buffer
         buf = torch.empty(max(int(nbytes), 1), dtype=torch.uint8, device=device)
         _scratch[key] = buf
         _scratch_gen[key] = _scratch_gen.get(key, 0) + 1
-        _scratch_users[key] = []
-    users = _scratch_users.setdefault(key, [])
-    if all(u.cuda_stream != cur.cuda_stream for u in users):
-        users.append(cur)
+        _scratch_users[key] = {}
+    users = _scratch_users.setdefault(key, {})
+    number = stream_ptr(device)
+    if number not in users:
+        users[number] = torch.cuda.current_stream(device)
     return buf
 
 
