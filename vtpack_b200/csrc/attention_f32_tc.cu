@@ -145,9 +145,38 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         tmem_relinquish();
     }
     if (warp == 2 && lane < (int)(sizeof(AfArgs) / 4)) asm volatile("" ::"r"(reinterpret_cast<const uint32_t*>(&g)[lane]));
+    // Loads of one thread of warp 0: an item and its Q; a slot of K (which = 0) or V of blocks blk and, where there is one, blk + 1
+    auto load_q = [&](const AttnItem& it, int slot) {
+        items[slot] = it;
+        mbar_arrive_expect_tx(q_full, 3 * AF_PLANE);
+        for (int t = 0; t < 3; ++t) tma_load_3d_a(smem_u32(base + t * AF_PLANE), &tmap_q, smem_u32(q_full), it.h * HD, t, it.row0);
+    };
+    auto load_kv = [&](const AttnItem& it, int s, int which, int blk, int halves) {
+        mbar_arrive_expect_tx(&kv_full[s], 3 * halves * (AF_PLANE / 2));
+        for (int t = 0; t < 3; ++t)
+            for (int i = 0; i < halves; ++i)
+                tma_load_4d_a(smem_u32(base + AF_SM_KV + (s * 3 + t) * AF_PLANE + i * (AF_PLANE / 2)), &tmap_kv, smem_u32(&kv_full[s]),
+                              which * g.C + it.h * HD, t, (blk + i) * 64, it.b);
+    };
+    __syncthreads();                                 // (the barriers exist)
     pdl_begin();
-    if (threadIdx.x == blockDim.x - 1) *void_s = launch_is_void(status) ? 1 : 0;
-    list_tiles(g.offsets, g.B, g.max_q, g.l_max, status, tile_prefix, offs);
+    // (of up to 32 images warp 0 lists the items alone and sends for the first one's Q and first keys before the others know the list)
+    const bool few = g.B <= FEW_IMAGES;
+    int o0 = 0, o1 = 0;
+    if (few && warp == 0 && lane < g.B) { o0 = g.offsets[lane]; o1 = g.offsets[lane + 1]; }
+    if (threadIdx.x == 0) *void_s = launch_is_void(status) ? 1 : 0;
+    AttnItem first_item;
+    if (!few) {
+        list_tiles(g.offsets, g.B, g.max_q, g.l_max, status, tile_prefix, offs);
+    } else if (warp == 0) {
+        __syncwarp();
+        const int n_tiles = list_few_tiles(o0, o1, g.B, g.max_q, g.l_max, status, tile_prefix, offs, blockIdx.x, g.heads, first_item);
+        if (*void_s == 0 && (int)blockIdx.x < n_tiles * g.heads && elect_one()) {
+            load_q(first_item, 0);
+            load_kv(first_item, 0, 0, 0, min(2, g.n_blocks / g.n_chunks));       // (the first chunk has so many blocks)
+        }
+        __syncwarp();
+    }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -165,24 +194,22 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             int n = 0, s = 0;                        // slots filled; the next one
             uint32_t ph = 1;
             for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++li) {
-                const AttnItem it = attn_item(w, g.heads, g.B, tile_prefix, offs);
-                ok = mbar_wait(q_free, (li & 1) ^ 1, abort_flag, status, STATUS_ATTN_LOAD);
-                if (!ok) break;
-                items[li & 1] = it;
-                mbar_arrive_expect_tx(q_full, 3 * AF_PLANE);
-                for (int t = 0; t < 3; ++t) tma_load_3d_a(smem_u32(base + t * AF_PLANE), &tmap_q, smem_u32(q_full), it.h * HD, t, it.row0);
+                const bool sent = few && li == 0;         // (its Q and first slot of K are under way)
+                const AttnItem it = sent ? first_item : attn_item(w, g.heads, g.B, tile_prefix, offs);
+                if (!sent) {
+                    ok = mbar_wait(q_free, (li & 1) ^ 1, abort_flag, status, STATUS_ATTN_LOAD);
+                    if (!ok) break;
+                    load_q(it, li & 1);
+                }
                 for (int c = 0; c < g.n_chunks && ok; ++c) {
                     const int b0 = first_block(c), b1 = first_block(c + 1);
                     for (int v = 0; v < 2 && ok; ++v) {
                         for (int blk = b0; blk < b1; blk += 2, ++n) {
-                            ok = mbar_wait(&kv_free[s], ph, abort_flag, status, STATUS_ATTN_LOAD);
-                            if (!ok) break;
-                            const int halves = min(2, b1 - blk);
-                            mbar_arrive_expect_tx(&kv_full[s], 3 * halves * (AF_PLANE / 2));
-                            for (int t = 0; t < 3; ++t)
-                                for (int i = 0; i < halves; ++i)
-                                    tma_load_4d_a(smem_u32(base + AF_SM_KV + (s * 3 + t) * AF_PLANE + i * (AF_PLANE / 2)), &tmap_kv,
-                                                  smem_u32(&kv_full[s]), v * g.C + it.h * HD, t, (blk + i) * 64, it.b);
+                            if (!sent || n > 0) {
+                                ok = mbar_wait(&kv_free[s], ph, abort_flag, status, STATUS_ATTN_LOAD);
+                                if (!ok) break;
+                                load_kv(it, s, v, blk, min(2, b1 - blk));
+                            }
                             if (++s == AF_SLOTS) { s = 0; ph ^= 1; }
                         }
                     }

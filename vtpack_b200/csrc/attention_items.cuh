@@ -71,4 +71,42 @@ __device__ __forceinline__ AttnItem attn_item(int w, int heads, int B, const int
     return it;
 }
 
+// The same for up to 32 images by one warp alone, which also works out item `w`, so that its loads are under way before the other
+// warps know the list: o0, o1 are offsets[lane] and offsets[lane + 1] (lane < B, else 0).  Returns the number of tiles; `it` holds only if
+// w is below that times heads.
+constexpr int FEW_IMAGES = 32;
+__device__ __forceinline__ int list_few_tiles(int o0, int o1, int B, int max_q, int l_max, int* status, int* tile_prefix, int32_t* offs,
+                                              int w, int heads, AttnItem& it) {
+    const int lane = threadIdx.x & 31;
+    int cnt = o1 - o0;
+#if VTP_INDEX_GUARDS
+    if (cnt < 0 || cnt > max_q || o0 < 0 || o1 > l_max) {
+        if (status && blockIdx.x == 0) atomicOr(status, STATUS_BAD_INDEX);
+        cnt = (o0 < 0) ? 0 : min(max(cnt, 0), max_q);
+    }
+#endif
+    const int tiles = lane < B ? (cnt + QT - 1) / QT : 0;
+    int incl = tiles;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int nb = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += nb;
+    }
+    const int excl = incl - tiles, total = __shfl_sync(0xffffffffu, incl, 31);
+    if (lane < B) {
+        tile_prefix[lane] = excl;
+        offs[lane] = o0;
+        if (lane + 1 == B) { tile_prefix[B] = total; offs[B] = o1; }
+    }
+    const int tg = w / heads;
+    // the last image whose first tile is not behind tile tg (as attn_item finds it)
+    const int b = 31 - __clz(__ballot_sync(0xffffffffu, lane < B && excl <= tg));
+    const int first = __shfl_sync(0xffffffffu, o0, b), end = __shfl_sync(0xffffffffu, o1, b);
+    it.b = b;
+    it.h = w - tg * heads;
+    it.row0 = first + (tg - __shfl_sync(0xffffffffu, excl, b)) * QT;
+    it.nq = min(QT, end - it.row0);
+    return total;
+}
+
 }  // namespace vtp
