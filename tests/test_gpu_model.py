@@ -703,6 +703,24 @@ def test_image_gives_the_same_bits_in_any_batch(kind, dtype):
         assert all(torch.equal(a, b[:n]) for a, b in zip(m.last_counts, counts))
 
 
+@pytest.mark.parametrize("C,B,fine", [(192, 9, 0.0), (192, 16, 0.5), (192, 20, 1.0), (384, 4, 0.0), (384, 9, 1.0), (768, 2, 0.5), (768, 4, 1.0)])
+def test_q_and_kv_in_one_launch_same_bits_for_an_image(C, B, fine):
+    """q and kv of a block in 128 x 64 tiles (an image alone), 128 x 128 tiles (as many as SMs; 192 q columns fill one and a half) and the
+    persistent kernel's, with few and with all rows that the host allows for."""
+    from vtpack_b200 import _lib
+    torch.manual_seed(C + B)
+    sd = O.round_bf16(O.make_state_dict(C, 1, C // 64, seed=B))
+    blk = _block(C, C // 64, sd, torch.bfloat16)
+    x = torch.randn(B, 257, C, device=DEV).bfloat16()
+    gate = torch.zeros(B, 4, 4, 3, device=DEV)
+    gate[..., 2] = 1
+    gate[..., 0] = torch.where(torch.rand(B, 4, 4, device=DEV) < fine, 2.0, 0.0)
+    out = blk(x, forced_gate=gate)
+    for b in range(B):
+        assert torch.equal(blk(x[b:b + 1].contiguous(), forced_gate=gate[b:b + 1]), out[b:b + 1]), b
+    assert _lib.device_status() == 0
+
+
 @pytest.mark.parametrize("forced", [False, True])
 @pytest.mark.parametrize("extra", [0, 1])
 def test_packed_rows_listed_or_derived_by_the_pool(extra, forced):

@@ -606,12 +606,13 @@ linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
 }
 
 // ------------------------------------------------------------------------------ small problems
-// The same products for problems of no more 128 x 64 tiles than SMs, where a launch is a chain of latencies: one tile per CTA,
+// The same products for problems of no more 128 x 64 or 128 x 128 tiles than SMs, where a launch is a chain of latencies: one tile per CTA,
 // which tile it is known before the wait for the kernel in front (the loads do not wait for the row count, only the stores
-// do), sixteen epilogue warps with 16 columns each that go straight between registers and global memory.  Same MMA steps and
+// do), sixteen epilogue warps with 16 columns of each 64 that go straight between registers and global memory.  Same MMA steps and
 // sums in the same order as linear_tc_kernel: a row's bits do not depend on which of the two it comes from.
+template <int BN_>
 struct SmallConf {
-    static constexpr int BN = 64, STAGES = 8, PRODUCERS = 3, FIRST_EPI = 4, EW = 16, THREADS = (FIRST_EPI + EW) * 32;
+    static constexpr int BN = BN_, STAGES = BN == 64 ? 8 : 6, PRODUCERS = 3, FIRST_EPI = 4, EW = 16, THREADS = (FIRST_EPI + EW) * 32;
     static constexpr int A_BYTES = TBM * TBK * 2, B_BYTES = BN * TBK * 2;
     static constexpr int RING = STAGES * (A_BYTES + B_BYTES);
     static constexpr int SUMS = TBM * 16 * 8;            // EPI_EMIT: (sum, sum of squares) of four columns of a row each
@@ -619,12 +620,15 @@ struct SmallConf {
     static constexpr int TOTAL = USED + 1024;
     static_assert(TOTAL <= SMEM_MAX, "shared memory budget");
 };
-struct SmallLaunch { CUtensorMap ta[2], tw[2]; TcScalars p[2]; int grid0; };     // n_tiles: 64-column tiles of a row
+// n_tiles: tiles of a row; grid0: CTAs of the first problem; at_once: CTAs that are sure to start together
+struct SmallLaunch { CUtensorMap ta[2], tw[2]; TcScalars p[2]; int grid0, at_once; };
 
-template <int EPI, bool F32, int NPROB>
-__global__ void __launch_bounds__(SmallConf::THREADS, 1)
+template <int BN, int EPI, bool F32, int NPROB>
+__global__ void __launch_bounds__(SmallConf<BN>::THREADS, 1)
 linear_tc_small_kernel(const __grid_constant__ SmallLaunch L, int K, int* status) {
-    using S = SmallConf;
+    using S = SmallConf<BN>;
+    constexpr int H = BN / SLAB;                                       // 64-column halves of a tile
+    static_assert(H == 1 || !(EPI & EPI_EMIT), "one half's row sums at a time");
     constexpr int STAGES = S::STAGES, PRODUCERS = S::PRODUCERS;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -654,7 +658,7 @@ linear_tc_small_kernel(const __grid_constant__ SmallLaunch L, int K, int* status
         fence_barrier_init();
     }
     if (warp == 1 && elect_one()) { prefetch_tmap(&L.ta[prob]); prefetch_tmap(&L.tw[prob]); }
-    if (warp == PRODUCERS) { tmem_alloc(tmem_slot, 64); tmem_relinquish(); }
+    if (warp == PRODUCERS) { tmem_alloc(tmem_slot, BN); tmem_relinquish(); }
     if (threadIdx.x == S::FIRST_EPI * 32) void_s[0] = launch_is_void(status) ? 1 : 0;
     tc_fence_before_sync();
     __syncthreads();
@@ -662,8 +666,10 @@ linear_tc_small_kernel(const __grid_constant__ SmallLaunch L, int K, int* status
     const uint32_t tmem_base = *tmem_slot;
     const bool known_void = void_s[0] != 0;
     pdl_begin();
+    // a CTA that starts when others have ended looks first whether its rows exist
+    const bool none = (int)blockIdx.x >= L.at_once && P.m_dev && m0 >= *reinterpret_cast<const volatile int32_t*>(P.m_dev);
 
-    if (known_void) {
+    if (known_void || none) {
     } else if (warp < PRODUCERS) {
         if (elect_one()) {
             for (int kb = warp; kb < nkb; kb += PRODUCERS) {
@@ -694,9 +700,9 @@ linear_tc_small_kernel(const __grid_constant__ SmallLaunch L, int K, int* status
         }
         __syncwarp();
     } else {
-        const int g = (warp - S::FIRST_EPI) >> 2;         // which 16 columns of the tile
+        const int g = (warp - S::FIRST_EPI) >> 2;         // which 16 columns of a half
         const int row = (warp & 3) * 32 + lane;           // tile row = TMEM lane
-        const int m = m0 + row, n0 = ct0 + g * 16, N = P.N;
+        const int m = m0 + row, N = P.N;
         // (a launch that turns out to be void forms its products and has no rows to store)
         if (threadIdx.x == S::FIRST_EPI * 32) void_s[1] = launch_is_void(status) ? 1 : 0;
         int M = P.m_max;
@@ -706,108 +712,117 @@ linear_tc_small_kernel(const __grid_constant__ SmallLaunch L, int K, int* status
         // what the outputs need besides the accumulator travels while the operands are loaded and multiplied
         const bool live = m0 + (warp & 3) * 32 < M;       // the warp has rows
         const bool row_ok = m < M;
-        const bool c0 = n0 < N, c1 = n0 + 8 < N;          // its columns exist, eight at a time
-        float add[16], sv[16], ln_a = 1.f;
-        uint4 rv[2];
-        if (live && c0) {
+        float add[H][16], ln_a = 1.f, ln_b = 0.f;
+        uint4 rv[H][2];
+        if ((EPI & EPI_LN) && live && row_ok) row_fold(P.ln, m, ln_a, ln_b);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int nb = min(n0 + 8 * (q >> 1), N - 8);
-                const float* bias = P.bias ? P.bias + nb : g_no_bias;
-                const float4 b4 = __ldg(reinterpret_cast<const float4*>(bias) + (q & 1));
-                add[4 * q] = b4.x; add[4 * q + 1] = b4.y; add[4 * q + 2] = b4.z; add[4 * q + 3] = b4.w;
-                if (EPI & EPI_LN) {
-                    const float4 s4 = __ldg(reinterpret_cast<const float4*>(P.ln.s + nb) + (q & 1));
-                    sv[4 * q] = s4.x; sv[4 * q + 1] = s4.y; sv[4 * q + 2] = s4.z; sv[4 * q + 3] = s4.w;
+        for (int h = 0; h < H; ++h) {
+            const int n0 = ct0 + h * SLAB + g * 16;
+            const bool c1 = n0 + 8 < N;               // its columns exist, eight at a time
+            if (live && n0 < N) {
+                float sv[16];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int nb = min(n0 + 8 * (q >> 1), N - 8);
+                    const float* bias = P.bias ? P.bias + nb : g_no_bias;
+                    const float4 b4 = __ldg(reinterpret_cast<const float4*>(bias) + (q & 1));
+                    add[h][4 * q] = b4.x; add[h][4 * q + 1] = b4.y; add[h][4 * q + 2] = b4.z; add[h][4 * q + 3] = b4.w;
+                    if (EPI & EPI_LN) {
+                        const float4 s4 = __ldg(reinterpret_cast<const float4*>(P.ln.s + nb) + (q & 1));
+                        sv[4 * q] = s4.x; sv[4 * q + 1] = s4.y; sv[4 * q + 2] = s4.z; sv[4 * q + 3] = s4.w;
+                    }
                 }
-            }
-            if ((EPI & EPI_RES) && row_ok) {
-                const bf16* r = P.res + map_res_row(P.rm, m) * P.ldr + n0;
-                rv[0] = *reinterpret_cast<const uint4*>(r);
-                rv[1] = c1 ? *reinterpret_cast<const uint4*>(r + 8) : make_uint4(0, 0, 0, 0);
-            }
-            if (EPI & EPI_LN) {
-                float ln_b = 0.f;
-                if (row_ok) row_fold(P.ln, m, ln_a, ln_b);
+                if ((EPI & EPI_RES) && row_ok) {
+                    const bf16* r = P.res + map_res_row(P.rm, m) * P.ldr + n0;
+                    rv[h][0] = *reinterpret_cast<const uint4*>(r);
+                    rv[h][1] = c1 ? *reinterpret_cast<const uint4*>(r + 8) : make_uint4(0, 0, 0, 0);
+                }
+                if (EPI & EPI_LN) {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) add[i] = fmaf(ln_b, sv[i], add[i]);
+                    for (int i = 0; i < 16; ++i) add[h][i] = fmaf(ln_b, sv[i], add[h][i]);
+                }
             }
         }
         const long long orow = map_out_row(P.rm, row_ok ? m : m0);
         const bool ok = mbar_wait_warp(acc_full, 0, abort_flag, status, STATUS_GEMM_EPILOGUE);
-        if (ok && live) {
-            tc_fence_after_sync();
-            uint32_t r[16];
-            float e1[4] = {0.f, 0.f, 0.f, 0.f}, e2[4] = {0.f, 0.f, 0.f, 0.f};
-            __syncwarp();
-            tmem_ld_32x16(tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + g * 16, r);
-            tmem_ld_wait();
-            if (c0) {
-                uint4 out[2];
+        if (ok && live) tc_fence_after_sync();
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    float v[8];
+        for (int h = 0; h < H; ++h) {
+            const int n0 = ct0 + h * SLAB + g * 16;
+            const bool c1 = n0 + 8 < N;
+            if (ok && live) {
+                uint32_t r[16];
+                float e1[4] = {0.f, 0.f, 0.f, 0.f}, e2[4] = {0.f, 0.f, 0.f, 0.f};
+                __syncwarp();
+                tmem_ld_32x16(tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + h * SLAB + g * 16, r);
+                tmem_ld_wait();
+                if (n0 < N) {
+                    uint4 out[2];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const float acc = __uint_as_float(r[8 * c + i]);
-                        v[i] = (EPI & EPI_LN) ? fmaf(ln_a, acc, add[8 * c + i]) : acc + add[8 * c + i];
-                    }
-                    if (EPI & EPI_GELU) gelu8(v);
-                    if (EPI & EPI_RES) {
-                        Vec<bf16> w;
-                        float rf[8];
-                        w.raw = rv[c];
-                        w.to_float(rf);
+                    for (int c = 0; c < 2; ++c) {
+                        float v[8];
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) v[i] += rf[i];
-                    }
-                    if (EPI & EPI_EMIT) {
-                        // as in linear_tc_kernel: columns 2 q, 2 q + 1 of the first and of the second eight
+                        for (int i = 0; i < 8; ++i) {
+                            const float acc = __uint_as_float(r[8 * c + i]);
+                            v[i] = (EPI & EPI_LN) ? fmaf(ln_a, acc, add[h][8 * c + i]) : acc + add[h][8 * c + i];
+                        }
+                        if (EPI & EPI_GELU) gelu8(v);
+                        if (EPI & EPI_RES) {
+                            Vec<bf16> w;
+                            float rf[8];
+                            w.raw = rv[h][c];
+                            w.to_float(rf);
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            const float z0 = (c == 0 || c1) ? v[2 * q] : 0.f, z1 = (c == 0 || c1) ? v[2 * q + 1] : 0.f;
-                            const float q1 = z0 + z1, q2 = fmaf(z1, z1, __fmul_rn(z0, z0));
-                            if (c == 0) { e1[q] = q1; e2[q] = q2; }
-                            else { e1[q] += q1; e2[q] += q2; }
+                            for (int i = 0; i < 8; ++i) v[i] += rf[i];
+                        }
+                        if (EPI & EPI_EMIT) {
+                            // as in linear_tc_kernel: columns 2 q, 2 q + 1 of the first and of the second eight
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                const float z0 = (c == 0 || c1) ? v[2 * q] : 0.f, z1 = (c == 0 || c1) ? v[2 * q + 1] : 0.f;
+                                const float q1 = z0 + z1, q2 = fmaf(z1, z1, __fmul_rn(z0, z0));
+                                if (c == 0) { e1[q] = q1; e2[q] = q2; }
+                                else { e1[q] += q1; e2[q] += q2; }
+                            }
+                        }
+                        if (F32) {
+                            if (row_ok && (c == 0 || c1)) {
+                                float* y = static_cast<float*>(P.y) + orow * P.ldy + n0 + 8 * c;
+                                reinterpret_cast<float4*>(y)[0] = make_float4(v[0], v[1], v[2], v[3]);
+                                reinterpret_cast<float4*>(y)[1] = make_float4(v[4], v[5], v[6], v[7]);
+                            }
+                        } else {
+                            Vec<bf16> ov;
+                            ov.from_float(v);
+                            out[c] = ov.raw;
                         }
                     }
-                    if (F32) {
-                        if (row_ok && (c == 0 || c1)) {
-                            float* y = static_cast<float*>(P.y) + orow * P.ldy + n0 + 8 * c;
-                            reinterpret_cast<float4*>(y)[0] = make_float4(v[0], v[1], v[2], v[3]);
-                            reinterpret_cast<float4*>(y)[1] = make_float4(v[4], v[5], v[6], v[7]);
-                        }
-                    } else {
-                        Vec<bf16> ov;
-                        ov.from_float(v);
-                        out[c] = ov.raw;
+                    if (!F32 && row_ok) {
+                        bf16* y = static_cast<bf16*>(P.y) + orow * P.ldy + n0;
+                        *reinterpret_cast<uint4*>(y) = out[0];
+                        if (c1) *reinterpret_cast<uint4*>(y + 8) = out[1];
                     }
                 }
-                if (!F32 && row_ok) {
-                    bf16* y = static_cast<bf16*>(P.y) + orow * P.ldy + n0;
-                    *reinterpret_cast<uint4*>(y) = out[0];
-                    if (c1) *reinterpret_cast<uint4*>(y + 8) = out[1];
+                if (EPI & EPI_EMIT) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) sums[(g * 4 + q) * TBM + row] = make_float2(e1[q], e2[q]);
                 }
             }
-            if (EPI & EPI_EMIT) {
+            if ((EPI & EPI_EMIT) && live) {
+                // the four warps of these rows (all of them get here): a column pair's 16 columns of each, (0 + 1) + (2 + 3), then the
+                // pairs, (0 + 1) + (2 + 3)
+                named_barrier(1 + (warp & 3), 128);
+                if (g == 0 && row_ok && ok) {
+                    float t1[4], t2[4];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) sums[(g * 4 + q) * TBM + row] = make_float2(e1[q], e2[q]);
-            }
-        }
-        if ((EPI & EPI_EMIT) && live) {
-            // the four warps of these rows (all of them get here): a column pair's 16 columns of each, (0 + 1) + (2 + 3), then the
-            // pairs, (0 + 1) + (2 + 3)
-            named_barrier(1 + (warp & 3), 128);
-            if (g == 0 && row_ok && ok) {
-                float t1[4], t2[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float2 a = sums[(0 * 4 + q) * TBM + row], b = sums[(1 * 4 + q) * TBM + row];
-                    const float2 c = sums[(2 * 4 + q) * TBM + row], d = sums[(3 * 4 + q) * TBM + row];
-                    t1[q] = (a.x + b.x) + (c.x + d.x);
-                    t2[q] = (a.y + b.y) + (c.y + d.y);
+                    for (int q = 0; q < 4; ++q) {
+                        const float2 a = sums[(0 * 4 + q) * TBM + row], b = sums[(1 * 4 + q) * TBM + row];
+                        const float2 c = sums[(2 * 4 + q) * TBM + row], d = sums[(3 * 4 + q) * TBM + row];
+                        t1[q] = (a.x + b.x) + (c.x + d.x);
+                        t2[q] = (a.y + b.y) + (c.y + d.y);
+                    }
+                    P.ln.emit[(size_t)m * P.ln.slots + ct0 / SLAB] = make_float2((t1[0] + t1[1]) + (t1[2] + t1[3]), (t2[0] + t2[1]) + (t2[2] + t2[3]));
                 }
-                P.ln.emit[(size_t)m * P.ln.slots + ct0 / SLAB] = make_float2((t1[0] + t1[1]) + (t1[2] + t1[3]), (t2[0] + t2[1]) + (t2[2] + t2[3]));
             }
         }
     }
@@ -817,7 +832,7 @@ linear_tc_small_kernel(const __grid_constant__ SmallLaunch L, int K, int* status
     }
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == PRODUCERS) tmem_dealloc(tmem_base, 64);
+    if (warp == PRODUCERS) tmem_dealloc(tmem_base, BN);
 }
 
 // ------------------------------------------------------------------------------ host
@@ -992,28 +1007,35 @@ static int launch_tc(const LinearArgs& p, const LinearArgs* p1, cudaStream_t st)
     return launched(launch_kernel(kern, true, CG, dim3(CG * used), dim3(S::THREADS), (size_t)S::TOTAL, st, L, p.K, device_status_ptr()));
 }
 
-// 128 x 64 tiles of a problem.  As many as SMs at most run as linear_tc_small_kernel: all at once, one per SM.  (DeiT-Ti, one
+// 128 x bn tiles of a problem.  As many of 64 columns as SMs at most run as linear_tc_small_kernel: all at once, one per SM.  (DeiT-Ti, one
 // image: 505 us per forward with the persistent kernel alone, 395 with both; DeiT-S, 7 images: 662 and 586.  Launches on both
 // sides of the line, us, small / persistent kernel:  1536, K = 384, GELU: 96 tiles 4.6 / 6.2, 144 4.7 / 6.8, 216 8.5 / 7.0, 288
 // 8.9 / 7.3;  384, K = 1536, residual: 108 tiles 7.8 / 8.9, 144 7.8 / 9.5, 222 14.7 / 11.5;  768, K = 192, GELU: 108 tiles 3.9 / 4.7,
 // 144 4.1 / 4.8, 216 7.4 / 5.4.)
-static long long small_tiles(const LinearArgs& p) { return (long long)ceil_div(p.m_max, TBM) * ceil_div(p.N, SmallConf::BN); }
+// Two problems in one launch also run that way as 128 x 128 tiles, if those are no more than SMs (q and kv of DeiT-S, 7 images: 7.0 -> 5.8
+// us; forwards, of the same tree but for this: DeiT-S 7 images 562 / 550; DeiT-S 9, DeiT-Ti 16 and DeiT-B 4 images are the last batches that
+// fit).  One problem gains nothing by them: 1536, K = 384, 539 of 1799 rows 6.6 / 6.5, all of them 11.4 / 8.4.
+static long long small_tiles(const LinearArgs& p, int bn, bool likely = false) {
+    // (with a device-side row count the worst case is about three times the packed rows of a DGE block)
+    return (long long)ceil_div(likely && p.m_dev ? ceil_div(p.m_max, 2) : p.m_max, TBM) * ceil_div(p.N, bn);
+}
 
-template <int EPI, bool F32, int NPROB>
+template <int BN, int EPI, bool F32, int NPROB>
 static int launch_small(const LinearArgs& p, const LinearArgs* p1, cudaStream_t st) {
+    using S = SmallConf<BN>;
     SmallLaunch L;
     for (int i = 0; i < 2; ++i) {
         const LinearArgs& q = (NPROB == 2 && i) ? *p1 : p;
-        if (int rc = operand_maps(&L.ta[i], &L.tw[i], q, SmallConf::BN)) return rc;
-        fill_scalars(L.p[i], q, F32, SmallConf::BN);
+        if (int rc = operand_maps(&L.ta[i], &L.tw[i], q, BN)) return rc;
+        fill_scalars(L.p[i], q, F32, BN);
     }
-    L.grid0 = (int)small_tiles(p);
-    const int grid = L.grid0 + (NPROB == 2 ? (int)small_tiles(*p1) : 0);
-    auto kern = linear_tc_small_kernel<EPI, F32, NPROB>;
+    L.grid0 = (int)small_tiles(p, BN);
+    L.at_once = sm_count();
+    const int grid = L.grid0 + (NPROB == 2 ? (int)small_tiles(*p1, BN) : 0);
+    auto kern = linear_tc_small_kernel<BN, EPI, F32, NPROB>;
     static bool reserved[64] = {};   // per instantiation and device
-    if (int rc = reserve_smem(kern, SmallConf::TOTAL, reserved)) return rc;
-    return launched(launch_kernel(kern, true, 1, dim3(grid), dim3(SmallConf::THREADS), (size_t)SmallConf::TOTAL, st, L, p.K,
-                                  device_status_ptr()));
+    if (int rc = reserve_smem(kern, S::TOTAL, reserved)) return rc;
+    return launched(launch_kernel(kern, true, 1, dim3(grid), dim3(S::THREADS), (size_t)S::TOTAL, st, L, p.K, device_status_ptr()));
 }
 
 static int check_tc_args(const LinearArgs& p) {
@@ -1057,7 +1079,8 @@ int linear_tcgen05_pair(const LinearArgs& a, const LinearArgs& b, cudaStream_t s
     if (int rc = check_tc_args(a)) return rc;
     if (int rc = check_tc_args(b)) return rc;
     VTP_REQUIRE(linear_pair_supported(a, b), VTP_ERR_UNSUPPORTED, "linear (tcgen05): these two problems cannot share a launch");
-    if (small_tiles(a) + small_tiles(b) <= sm_count()) return launch_small<EPI_LN, false, 2>(a, &b, st);
+    if (small_tiles(a, 64) + small_tiles(b, 64) <= sm_count()) return launch_small<64, EPI_LN, false, 2>(a, &b, st);
+    if (small_tiles(a, 128, true) + small_tiles(b, 128, true) <= sm_count()) return launch_small<128, EPI_LN, false, 2>(a, &b, st);
     if (pairs_pay(256, a.K)) return launch_tc<256, 2, EPI_LN, false, 2>(a, &b, st);
     return launch_tc<256, 1, EPI_LN, false, 2>(a, &b, st);
 }
@@ -1067,23 +1090,23 @@ int linear_tcgen05(const LinearArgs& p, cudaStream_t st) {
     if (int rc = check_tc_args(p)) return rc;
     const int bn = pick_bn(p.N);
     const bool pairs = pairs_pay(bn, p.K);
-    const bool small = small_tiles(p) <= sm_count();
+    const bool small = small_tiles(p, 64) <= sm_count();
     const bool f32 = (p.flags & VTP_FLAG_OUT_F32) != 0;
     const int epi = ((p.flags & VTP_FLAG_GELU) ? EPI_GELU : 0) | (p.ln_mode ? EPI_LN : 0) | (p.emit_stats ? EPI_EMIT : 0) |
                     (p.res ? EPI_RES : 0);
     // rare kinds in one tile width (a row's bits do not depend on it)
     if (f32) {
-        if (small && epi == 0) return launch_small<0, true, 1>(p, nullptr, st);
-        if (small && epi == EPI_RES) return launch_small<EPI_RES, true, 1>(p, nullptr, st);
+        if (small && epi == 0) return launch_small<64, 0, true, 1>(p, nullptr, st);
+        if (small && epi == EPI_RES) return launch_small<64, EPI_RES, true, 1>(p, nullptr, st);
         if (epi == 0) return launch_tc<128, 1, 0, true, 1>(p, nullptr, st);
         if (epi == EPI_RES) return launch_tc<128, 1, EPI_RES, true, 1>(p, nullptr, st);
         return fail(VTP_ERR_UNSUPPORTED, "linear (tcgen05): fp32 output supports bias and residual only");
     }
-    if (small && epi == (EPI_GELU | EPI_RES)) return launch_small<EPI_GELU | EPI_RES, false, 1>(p, nullptr, st);
+    if (small && epi == (EPI_GELU | EPI_RES)) return launch_small<64, EPI_GELU | EPI_RES, false, 1>(p, nullptr, st);
     if (epi == (EPI_GELU | EPI_RES)) return launch_tc<128, 1, EPI_GELU | EPI_RES, false, 1>(p, nullptr, st);
 #define VTP_TC_CASE(E)                                                                   \
     if (epi == (E)) {                                                                    \
-        if (small) return launch_small<(E), false, 1>(p, nullptr, st);                   \
+        if (small) return launch_small<64, (E), false, 1>(p, nullptr, st);               \
         if (pairs && bn == 256) return launch_tc<256, 2, (E), false, 1>(p, nullptr, st); \
         if (pairs && bn == 192) return launch_tc<192, 2, (E), false, 1>(p, nullptr, st); \
         if (bn == 256) return launch_tc<256, 1, (E), false, 1>(p, nullptr, st);          \
