@@ -334,6 +334,10 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
     if (fold && !marks.events && linear_pair_supported(lkv, lq)) {
         // the two projections do not depend on each other: one launch, the q tiles fill the kv tail
         if ((rc = linear_tcgen05_pair(lkv, lq, st))) return rc;
+    } else if (terms && !reduce && !marks.events) {
+        lq.w = b.q_wt; lkv.w = b.kv_wt;
+        lq.out_terms = lkv.out_terms = terms_attn;
+        if ((rc = linear_f32_terms_pair(lkv, lq, st))) return rc;
     } else {
         if (!reduce && ((rc = run_linear(lq, b.q_wt, terms_attn)) || (rc = marks.mark(4)))) return rc;
         if ((rc = run_linear(lkv, b.kv_wt, terms_attn)) || (rc = marks.mark(5))) return rc;

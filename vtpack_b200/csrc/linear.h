@@ -48,6 +48,7 @@ int linear_tcgen05(const LinearArgs& p, cudaStream_t st);      // bf16 inputs, t
 bool linear_f32_tc_supported(const LinearArgs& p);
 int linear_f32_tcgen05(const LinearArgs& p, cudaStream_t st);  // fp32 inputs as three bf16 terms each, tcgen05
 int linear_f32_terms(const LinearArgs& p, cudaStream_t st);    // fp32 with a and w as rows of terms (f32_terms.cuh), lda unused
+int linear_f32_terms_pair(const LinearArgs& a, const LinearArgs& b, cudaStream_t st);    // two of them, in one launch if that is shorter
 int linear(const LinearArgs& p, cudaStream_t st);              // picks by dtype / flags
 bool linear_pair_supported(const LinearArgs& a, const LinearArgs& b);
 int linear_tcgen05_pair(const LinearArgs& a, const LinearArgs& b, cudaStream_t st);   // two problems, one launch

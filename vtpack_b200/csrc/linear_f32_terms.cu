@@ -37,32 +37,50 @@ struct FtSmem {
     static_assert(TOTAL <= 232448, "shared memory budget");
 };
 
-struct FtArgs {
+struct FtProblem {
     const bf16* a; const bf16* w; const float* bias; const float* res; long long ldr;
     float* y; long long ldy;
-    const int32_t* m_dev; int m_max, N, K, groups_log2;
-    FastDiv n_tiles, step;               // column tiles of a row of tiles, CTAs (clusters) of the grid
+    const int32_t* m_dev; int m_max, N;
+    FastDiv n_tiles;                     // column tiles of a row of tiles
+};
+// A launch works through one problem or two independent ones (same K and kind of output): the tiles of the second fill the last, partial
+// round of the first (q and kv of DeiT-S, 12 images, 31.6 us in two launches, 22.0 in one).
+struct FtArgs {
+    FtProblem p[2];
+    int K, groups_log2;
+    FastDiv step;                        // CTAs (clusters) of the grid
 };
 // a [m_max][3][K], w [N][3][K] as maps {K, 3, rows} with boxes of 64 elements of one term of a tile's rows; w also in boxes of half
 // and of a quarter of a tile's columns.
 struct FtMaps { CUtensorMap a, w[3]; };
+struct FtMapsOf { FtMaps p[2]; };
 
 // The work items of a CTA (SPLIT of a cluster), in order: tiles first, first + step, ...; where they are cut, the tiles of the
 // last, partial round are two or four column strips, one per CTA, so that it takes a fraction of a tile's time.
 // (A row's bits do not depend on it: a column's sums are the same in any tile.)
-template <int BN>
+template <int BN, int NPROB>
 struct FtItems {
-    FastDiv n_tiles;
-    uint32_t full, strips, step, first;
+    FastDiv n_tiles[NPROB];
+    uint32_t tot0, full, strips, step, first;
     int cut;                                     // log2 of the strips of a tile
-    __device__ __forceinline__ FtItems(uint32_t total, const FtArgs& g, uint32_t first_, bool strips_pay) : n_tiles(g.n_tiles), step(g.step.d), first(first_) {
+    // M: rows of the problems; a void launch that is known has no items
+    __device__ __forceinline__ FtItems(const int (&M)[NPROB], bool known_void, const FtArgs& g, uint32_t first_, bool strips_pay) : step(g.step.d), first(first_) {
+        uint32_t total = 0;
+        tot0 = 0;
+#pragma unroll
+        for (int i = 0; i < NPROB; ++i) {
+            n_tiles[i] = g.p[i].n_tiles;
+            if (i == 1) tot0 = total;
+            total += (uint32_t)((M[i] + FM - 1) / FM) * n_tiles[i].d;
+        }
+        if (known_void) total = 0;
         full = !strips_pay ? total : total < step ? 0 : fast_div(total, g.step) * step;
         const uint32_t rest = total - full;
         cut = BN == 128 && rest * 4 <= step ? 2 : rest * 2 <= step ? 1 : 0;
         strips = rest << cut;
     }
     // (a strip beyond the columns of a narrow tile is an item like any other: its sums are not stored)
-    struct Item { int mt, n0, cut; };            // row of tiles, first column, log2 of BN / columns
+    struct Item { int p, mt, n0, cut; };         // problem, row of tiles, first column, log2 of BN / columns
     __device__ __forceinline__ bool at(uint32_t j, Item& it) const {
         uint32_t tile = first + j * step, sub = 0;
         it.cut = 0;
@@ -73,9 +91,12 @@ struct FtItems {
             sub = u & ((1u << cut) - 1);
             it.cut = cut;
         }
-        const uint32_t mt = fast_div(tile, n_tiles);
+        it.p = NPROB == 2 && tile >= tot0 ? 1 : 0;
+        if (NPROB == 2 && it.p) tile -= tot0;
+        const FastDiv nt = NPROB == 2 && it.p ? n_tiles[NPROB - 1] : n_tiles[0];
+        const uint32_t mt = fast_div(tile, nt);
         it.mt = (int)mt;
-        it.n0 = (int)(tile - mt * n_tiles.d) * BN + (int)sub * (BN >> it.cut);
+        it.n0 = (int)(tile - mt * nt.d) * BN + (int)sub * (BN >> it.cut);
         return true;
     }
 };
@@ -103,7 +124,7 @@ __device__ __forceinline__ float term_at(const bf16* row, int K, int k) {
 // acc: NC columns n0.. of row m0 + lane, sums of scaled products, which are scaled back.  Rows with a sum that is not finite are
 // worked out again as an fmaf chain, a row at a time, a lane per column (see linear_f32_tc.cu).
 template <int NC>
-__device__ __forceinline__ void unscale_or_redo(float (&acc)[NC], const FtArgs& g, int M, int m0, int n0, int lane) {
+__device__ __forceinline__ void unscale_or_redo(float (&acc)[NC], const FtProblem& g, int K, int M, int m0, int n0, int lane) {
     float t = 0.f;
 #pragma unroll
     for (int i = 0; i < NC; ++i) {
@@ -114,14 +135,14 @@ __device__ __forceinline__ void unscale_or_redo(float (&acc)[NC], const FtArgs& 
     while (bad) {
         const int r = __ffs(bad) - 1;
         bad &= bad - 1;
-        const bf16* a = g.a + (size_t)(m0 + r) * 3 * g.K;
+        const bf16* a = g.a + (size_t)(m0 + r) * 3 * K;
         static_assert(NC <= 32, "a lane per column");
         const int n = n0 + lane;
         float s = 0.f;
         if (lane < NC && n < g.N) {
-            const bf16* w = g.w + (size_t)n * 3 * g.K;
+            const bf16* w = g.w + (size_t)n * 3 * K;
 #pragma unroll 1
-            for (int k = 0; k < g.K; ++k) s = fmaf(term_at(a, g.K, k), term_at(w, g.K, k), s);
+            for (int k = 0; k < K; ++k) s = fmaf(term_at(a, K, k), term_at(w, K, k), s);
         }
 #pragma unroll
         for (int i = 0; i < NC; ++i) {
@@ -135,7 +156,7 @@ __device__ __forceinline__ void unscale_or_redo(float (&acc)[NC], const FtArgs& 
 constexpr int FT_ROWS = 0, FT_TERMS = 1, FT_HIDDEN = 2;
 // Four output columns of row m from column n on, N and n multiples of four.
 template <int OUT>
-__device__ __forceinline__ void finish4(const FtArgs& g, int m, int n, const float4& s, const float4& bias, const float4& res) {
+__device__ __forceinline__ void finish4(const FtProblem& g, int m, int n, const float4& s, const float4& bias, const float4& res) {
     float v[4] = {s.x + bias.x, s.y + bias.y, s.z + bias.z, s.w + bias.w};
     if (OUT != FT_ROWS) {
         if (OUT == FT_HIDDEN) {
@@ -150,9 +171,9 @@ __device__ __forceinline__ void finish4(const FtArgs& g, int m, int n, const flo
 }
 
 // SPLIT: CTAs of a cluster that share a tile's reduction (1: none); it divides the number of groups.
-template <int BN, int SPLIT, int OUT>
+template <int BN, int SPLIT, int OUT, int NPROB>
 __global__ void __launch_bounds__(FT_THREADS, 1)
-linear_f32_terms_kernel(const __grid_constant__ FtMaps maps, const __grid_constant__ FtArgs g, int* status) {
+linear_f32_terms_kernel(const __grid_constant__ FtMapsOf maps, const __grid_constant__ FtArgs g, int* status) {
     using S = FtSmem<BN>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -185,12 +206,14 @@ linear_f32_terms_kernel(const __grid_constant__ FtMaps maps, const __grid_consta
         tmem_relinquish();
     }
     if (warp == FT_FIRST_EPI && elect_one()) {
-        prefetch_tmap(&maps.a);
-        for (int i = 0; i < 3; ++i) prefetch_tmap(&maps.w[i]);
+        for (int p = 0; p < NPROB; ++p) {
+            prefetch_tmap(&maps.p[p].a);
+            for (int i = 0; i < 3; ++i) prefetch_tmap(&maps.p[p].w[i]);
+        }
     }
     // (parameters are cold in every launch, each line of them is a miss: not on the way to the first load)
-    if (warp == FT_FIRST_EPI + 2 && lane < (int)(sizeof(FtArgs) / 4))
-        asm volatile("" ::"r"(reinterpret_cast<const uint32_t*>(&g)[lane]));
+    if (warp == FT_FIRST_EPI + 2)
+        for (int i = lane; i < (int)(sizeof(FtArgs) / 4); i += 32) asm volatile("" ::"r"(reinterpret_cast<const uint32_t*>(&g)[i]));
     if (threadIdx.x == (FT_FIRST_EPI + 1) * 32) void_s[0] = launch_is_void(status) ? 1 : 0;
     tc_fence_before_sync();
     __syncthreads();
@@ -200,17 +223,20 @@ linear_f32_terms_kernel(const __grid_constant__ FtMaps maps, const __grid_consta
     const bool known_void = lead_word<SPLIT>(void_s) != 0;
     pdl_begin();
 
-    int M = g.m_max;
-    if (g.m_dev) M = min(max(*reinterpret_cast<const volatile int32_t*>(g.m_dev), 0), M);
-    const uint32_t total = known_void ? 0 : (uint32_t)((M + FM - 1) / FM) * g.n_tiles.d;
+    int rows[NPROB];
+#pragma unroll
+    for (int i = 0; i < NPROB; ++i) {
+        rows[i] = g.p[i].m_max;
+        if (g.p[i].m_dev) rows[i] = min(max(*reinterpret_cast<const volatile int32_t*>(g.p[i].m_dev), 0), rows[i]);
+    }
     const int rank = SPLIT > 1 ? (int)cluster_ctarank() : 0;
     const int all_kb = (g.K + FK - 1) / FK;
     const int kb0 = all_kb * rank / SPLIT, num_kb = all_kb * (rank + 1) / SPLIT - kb0;    // this CTA's k-blocks
-    const FtItems<BN> items(total, g, blockIdx.x / SPLIT, SPLIT == 1);
+    const FtItems<BN, NPROB> items(rows, known_void, g, blockIdx.x / SPLIT, SPLIT == 1);
     // (term of a, term of w) of the products, smallest first; the first three bring every term once
     constexpr int TA[6] = {2, 0, 1, 1, 0, 0}, TB[6] = {0, 2, 1, 0, 1, 0};
     FtSlots sets[2];
-    typename FtItems<BN>::Item wi;
+    typename FtItems<BN, NPROB>::Item wi;
     int it = 0;                                   // k-blocks so far
     bool ok = true;
 
@@ -219,7 +245,8 @@ linear_f32_terms_kernel(const __grid_constant__ FtMaps maps, const __grid_consta
             // ------------------------------------------------------------ TMA producer
             const uint32_t sbase = smem_u32(base);
             for (uint32_t j = 0; ok && items.at(j, wi); ++j) {
-                const CUtensorMap* wmap = &maps.w[wi.cut];
+                const FtMaps& mp = maps.p[NPROB == 2 ? wi.p : 0];
+                const CUtensorMap* wmap = &mp.w[wi.cut];
                 const uint32_t b_term = S::B_TERM >> wi.cut;
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it & 1;
@@ -232,7 +259,7 @@ linear_f32_terms_kernel(const __grid_constant__ FtMaps maps, const __grid_consta
                         if (!ok) break;
                         const uint32_t bar = smem_u32(&full[3 * s + c]);
                         mbar_arrive_expect_tx_a(bar, S::A_TERM + b_term);
-                        tma_load_3d_a(sa + in.a[TA[c]] * S::A_TERM, &maps.a, bar, k, TA[c], wi.mt * FM);
+                        tma_load_3d_a(sa + in.a[TA[c]] * S::A_TERM, &mp.a, bar, k, TA[c], wi.mt * FM);
                         tma_load_3d_a(sb + in.b[TB[c]] * S::B_TERM, wmap, bar, k, TB[c], wi.n0);
                     }
                     if (!ok) break;
@@ -290,9 +317,11 @@ linear_f32_terms_kernel(const __grid_constant__ FtMaps maps, const __grid_consta
         // in a launch that turns out to be void the sums still change hands, but this CTA has no rows to store
         if (threadIdx.x == FT_FIRST_EPI * 32) void_s[1] = launch_is_void(status) ? 1 : 0;
         named_barrier(1, FT_EPI_WARPS * 32);
-        if (void_s[1] != 0) M = 0;
+        const bool stores = void_s[1] == 0;
         int n_sent = 0;                                   // exchanges
         for (uint32_t j = 0; ok && items.at(j, wi); ++j) {
+            const FtProblem& q = g.p[NPROB == 2 ? wi.p : 0];
+            const int M = !stores ? 0 : NPROB == 2 && wi.p ? rows[NPROB - 1] : rows[0];
             const int m0 = wi.mt * FM + quarter * 32, n0 = wi.n0 + col;
             const bool has = col < (BN >> wi.cut);        // a strip leaves some warps without columns
             // What an output needs besides its sum travels while the operands are loaded and multiplied.  SPLIT: SC columns of row
@@ -304,9 +333,9 @@ linear_f32_terms_kernel(const __grid_constant__ FtMaps maps, const __grid_consta
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
                 const int m = SPLIT > 1 ? m0 + lane : m0 + (v & 3) * 8 + (lane >> 2), n = col_of(v);
-                if (OUT == FT_ROWS) res[v] = g.res && has && m < M && n < g.N ? *reinterpret_cast<const float4*>(g.res + (size_t)m * g.ldr + n) : zero4;
+                if (OUT == FT_ROWS) res[v] = q.res && has && m < M && n < q.N ? *reinterpret_cast<const float4*>(q.res + (size_t)m * q.ldr + n) : zero4;
                 if (SPLIT > 1 || (v & 3) == 0)
-                    bias[SPLIT > 1 ? v : v >> 2] = g.bias && has && n < g.N ? __ldg(reinterpret_cast<const float4*>(g.bias + n)) : zero4;
+                    bias[SPLIT > 1 ? v : v >> 2] = q.bias && has && n < q.N ? __ldg(reinterpret_cast<const float4*>(q.bias + n)) : zero4;
             }
             float acc[CW];
 #pragma unroll
@@ -340,7 +369,7 @@ linear_f32_terms_kernel(const __grid_constant__ FtMaps maps, const __grid_consta
                 constexpr int ROUNDS = (SPLIT - 1) * SC * 128 > FT_OUT ? 2 : 1, XC = SC / ROUNDS;     // what the slots hold
                 static_assert((SPLIT - 1) * XC * 128 <= FT_OUT && XC % 4 == 0, "the exchange fits the warp's transpose buffer");
                 float own[SC];
-                typename FtItems<BN>::Item next;
+                typename FtItems<BN, NPROB>::Item next;
 #pragma unroll
                 for (int d = 0; d < SPLIT; ++d)                   // (a runtime index would put acc into local memory)
                     if (d == rank) {
@@ -389,16 +418,16 @@ linear_f32_terms_kernel(const __grid_constant__ FtMaps maps, const __grid_consta
                     }
                 }
                 if (!ok) break;
-                unscale_or_redo<SC>(own, g, M, m0, n0 + rank * SC, lane);
+                unscale_or_redo<SC>(own, q, g.K, M, m0, n0 + rank * SC, lane);
                 if (m0 + lane < M) {
 #pragma unroll
                     for (int v = 0; v < NV; ++v)
-                        if (col_of(v) < g.N)
-                            finish4<OUT>(g, m0 + lane, col_of(v), make_float4(own[4 * v], own[4 * v + 1], own[4 * v + 2], own[4 * v + 3]),
+                        if (col_of(v) < q.N)
+                            finish4<OUT>(q, m0 + lane, col_of(v), make_float4(own[4 * v], own[4 * v + 1], own[4 * v + 2], own[4 * v + 3]),
                                             bias[v], res[OUT != FT_ROWS ? 0 : v]);
                 }
             } else if (has) {
-                unscale_or_redo<CW>(acc, g, M, m0, n0, lane);
+                unscale_or_redo<CW>(acc, q, g.K, M, m0, n0, lane);
                 // 16 columns at a time through the warp's transpose buffer (rows of four 16-byte chunks, XOR-swizzled): a lane
                 // then holds four columns of a row and four lanes 64 consecutive bytes
 #pragma unroll
@@ -411,18 +440,18 @@ linear_f32_terms_kernel(const __grid_constant__ FtMaps maps, const __grid_consta
                                           __float_as_uint(acc[16 * b + 4 * i + 2]), __float_as_uint(acc[16 * b + 4 * i + 3])));
                     __syncwarp();
                     const int n = n0 + 16 * b + (lane & 3) * 4;
-                    auto finish = [&](int q) {
-                        const int rr = q * 8 + (lane >> 2);
+                    auto finish = [&](int r8) {
+                        const int rr = r8 * 8 + (lane >> 2);
                         const float4 v = lds_f4(stage + rr * 64 + (((lane & 3) ^ ((rr >> 1) & 3)) << 4));
-                        if (m0 + rr < M && n < g.N) finish4<OUT>(g, m0 + rr, n, v, bias[b], res[OUT != FT_ROWS ? 0 : 4 * b + q]);
+                        if (m0 + rr < M && n < q.N) finish4<OUT>(q, m0 + rr, n, v, bias[b], res[OUT != FT_ROWS ? 0 : 4 * b + r8]);
                     };
                     if constexpr (OUT == FT_HIDDEN) {
                         // (not unrolled: most launches run this once per warp, and then what it costs is its fetch)
 #pragma unroll 1
-                        for (int q = 0; q < 4; ++q) finish(q);
+                        for (int r8 = 0; r8 < 4; ++r8) finish(r8);
                     } else {
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) finish(q);
+                        for (int r8 = 0; r8 < 4; ++r8) finish(r8);
                     }
                 }
             }
@@ -438,9 +467,9 @@ linear_f32_terms_kernel(const __grid_constant__ FtMaps maps, const __grid_consta
     if (warp == 1) tmem_dealloc(tmem_base, F_TMEM * BN);
 }
 
-template <int BN, int SPLIT, int OUT>
-static int launch_terms(FtArgs& g, const FtMaps& maps, cudaStream_t st) {
-    auto kern = linear_f32_terms_kernel<BN, SPLIT, OUT>;
+template <int BN, int SPLIT, int OUT, int NPROB>
+static int launch_terms(FtArgs& g, const FtMapsOf& maps, cudaStream_t st) {
+    auto kern = linear_f32_terms_kernel<BN, SPLIT, OUT, NPROB>;
     static bool attr_set[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -452,10 +481,13 @@ static int launch_terms(FtArgs& g, const FtMaps& maps, cudaStream_t st) {
         }
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    long long tiles = (long long)ceil_div(g.N, BN) * ceil_div(g.m_max, FM);
+    long long tiles = 0;
+    for (int i = 0; i < NPROB; ++i) {
+        g.p[i].n_tiles = make_fast_div((uint32_t)ceil_div(g.p[i].N, BN));
+        tiles += (long long)ceil_div(g.p[i].N, BN) * ceil_div(g.p[i].m_max, FM);
+    }
     if (SPLIT == 1) tiles *= BN / 32;                        // few tiles are cut into strips (FtItems): a CTA for each
     const int grid = (int)(tiles * SPLIT <= sm_count() ? tiles * SPLIT : sm_count() / SPLIT * SPLIT);
-    g.n_tiles = make_fast_div((uint32_t)ceil_div(g.N, BN));
     g.step = make_fast_div((uint32_t)(grid / SPLIT));
     const cudaError_t le = launch_kernel(kern, true, SPLIT, dim3(grid), dim3(FT_THREADS), (size_t)FtSmem<BN>::TOTAL, st, maps, g,
                                          device_status_ptr());
@@ -479,24 +511,22 @@ static int launch_terms(FtArgs& g, const FtMaps& maps, cudaStream_t st) {
 //   270 x 768, K = 3072, residual          48.2      29.1      32.3     49.4      36.4      22.3*
 //   180 x 192, K = 768, residual           14.0      10.7       7.4*    15.4      15.0      10.5
 //   4400 x 768, K = 192, GELU              18.0                         17.4*
-static double terms_cost(int bn, int split, bool hidden, long long m, int N, int num_kb, int sms) {
+// (tiles: of a launch without splits, 128 rows x bn columns, the second problem's included)
+static double terms_cost(int bn, int split, bool hidden, long long tiles, int num_kb, int sms) {
     const bool wide = bn == 128;
     const double kb_cost = wide ? 2050 : 1640;
     const double end = (split == 1 ? (wide ? 3000 : 1500) : split == 2 ? (wide ? 5000 : 2500) : (wide ? 7500 : 3000)) +
                        (hidden ? (wide ? 6000 : 3500) : 0);
-    const long long tiles = (m + FM - 1) / FM * ceil_div(N, bn), lanes = split == 4 ? sms * 9 / 40 : sms / split;
+    const long long lanes = split == 4 ? sms * 9 / 40 : sms / split;
     const long long full = tiles / lanes, rest = tiles - full * lanes;
     double rounds = (double)full;
     if (rest) rounds += split > 1 ? 1.0 : (wide && rest * 4 <= lanes) ? 0.65 : rest * 2 <= lanes ? 0.8 : 1.0;
     return rounds * (ceil_div(num_kb, split) * kb_cost + end);
 }
 
-int linear_f32_terms_as(const LinearArgs& p, int bn, int split, cudaStream_t st) {
-    FtArgs g;
-    g.a = (const bf16*)p.a; g.w = (const bf16*)p.w; g.bias = p.bias; g.res = (const float*)p.res; g.ldr = p.ldr;
-    g.y = (float*)p.y; g.ldy = p.ldy; g.m_max = p.m_max; g.m_dev = p.m_dev; g.N = p.N; g.K = p.K;
-    g.groups_log2 = f32_groups_log2(ceil_div(p.K, FK));
-    FtMaps maps;
+static int fill_terms(FtProblem& q, FtMaps& maps, const LinearArgs& p, int bn) {
+    q.a = (const bf16*)p.a; q.w = (const bf16*)p.w; q.bias = p.bias; q.res = (const float*)p.res; q.ldr = p.ldr;
+    q.y = (float*)p.y; q.ldy = p.ldy; q.m_max = p.m_max; q.m_dev = p.m_dev; q.N = p.N;
     const unsigned long long strides[2] = {(unsigned long long)p.K * 2, (unsigned long long)p.K * 6};
     const unsigned long long da[3] = {(unsigned long long)p.K, 3, (unsigned long long)p.m_max};
     const unsigned long long dw[3] = {(unsigned long long)p.K, 3, (unsigned long long)p.N};
@@ -506,10 +536,27 @@ int linear_f32_terms_as(const LinearArgs& p, int bn, int split, cudaStream_t st)
         const unsigned bw[3] = {FK, 1, (unsigned)(bn >> (bn == 128 ? i : i > 0))};      // (64-wide tiles are cut in two only)
         if (int rc = make_tmap_bf16(&maps.w[i], p.w, 3, dw, strides, bw)) return rc;
     }
+    return VTP_OK;
+}
+
+// p1: null, or a second problem (split 1 only).
+static int linear_f32_terms_as(const LinearArgs& p, const LinearArgs* p1, int bn, int split, cudaStream_t st) {
+    FtArgs g;
+    FtMapsOf maps;
+    g.K = p.K;
+    g.groups_log2 = f32_groups_log2(ceil_div(p.K, FK));
+    if (int rc = fill_terms(g.p[0], maps.p[0], p, bn)) return rc;
+    if (p1) {
+        if (int rc = fill_terms(g.p[1], maps.p[1], *p1, bn)) return rc;
+        if (bn == 128) return p.out_terms ? launch_terms<128, 1, FT_TERMS, 2>(g, maps, st) : launch_terms<128, 1, FT_ROWS, 2>(g, maps, st);
+        return p.out_terms ? launch_terms<64, 1, FT_TERMS, 2>(g, maps, st) : launch_terms<64, 1, FT_ROWS, 2>(g, maps, st);
+    }
+    g.p[1] = g.p[0];
+    maps.p[1] = maps.p[0];
 #define VTP_TERMS_CASE(BN, SPLIT) \
-    if (bn == BN && split == SPLIT) return !p.out_terms ? launch_terms<BN, SPLIT, FT_ROWS>(g, maps, st) \
-                                             : (p.flags & VTP_FLAG_GELU) ? launch_terms<BN, SPLIT, FT_HIDDEN>(g, maps, st) \
-                                                                         : launch_terms<BN, SPLIT, FT_TERMS>(g, maps, st)
+    if (bn == BN && split == SPLIT) return !p.out_terms ? launch_terms<BN, SPLIT, FT_ROWS, 1>(g, maps, st) \
+                                             : (p.flags & VTP_FLAG_GELU) ? launch_terms<BN, SPLIT, FT_HIDDEN, 1>(g, maps, st) \
+                                                                         : launch_terms<BN, SPLIT, FT_TERMS, 1>(g, maps, st)
     VTP_TERMS_CASE(128, 1);
     VTP_TERMS_CASE(128, 2);
     VTP_TERMS_CASE(128, 4);
@@ -520,25 +567,56 @@ int linear_f32_terms_as(const LinearArgs& p, int bn, int split, cudaStream_t st)
     return fail(VTP_ERR_UNSUPPORTED, "linear (fp32 terms): no kernel for tiles of %d columns, %d CTAs", bn, split);
 }
 
-int linear_f32_terms(const LinearArgs& p, cudaStream_t st) {
+static int check_terms(const LinearArgs& p) {
     if (int rc = linear_validate(p)) return rc;
     VTP_REQUIRE(p.dtype == VTP_F32 && p.N % 8 == 0 && p.K % 8 == 0 && p.ldy % 4 == 0 && (!p.res || p.ldr % 4 == 0), VTP_ERR_SHAPE,
                 "linear (fp32 terms): N=%d K=%d", p.N, p.K);
     VTP_REQUIRE(p.ln_mode == 0 && !p.emit_stats && p.out_grp == 0 && p.res_mod == 0 && (p.out_terms || !(p.flags & VTP_FLAG_GELU)) &&
                     !(p.out_terms && p.res), VTP_ERR_UNSUPPORTED,
                 "linear (fp32 terms): plain rows; GELU only with terms out, a residual only with fp32 out");
-    if (p.m_max == 0) return VTP_OK;
+    return VTP_OK;
+}
+
+// With a device-side row count the worst case is about three times the packed rows of a DGE block.
+static long long likely_tiles(const LinearArgs& p, int bn) {
+    return (long long)ceil_div(p.m_dev ? ceil_div(p.m_max, 3) : p.m_max, FM) * ceil_div(p.N, bn);
+}
+static double best_terms(const LinearArgs& p, int* bn, int* split) {
     const int num_kb = ceil_div(p.K, FK), sms = sm_count();
-    // With a device-side row count the worst case is about three times the packed rows of a DGE block.
-    const long long m = p.m_dev ? ceil_div(p.m_max, 3) : p.m_max;
-    int bn = 64, split = 1;
     double best = 0;
     for (int b = 64; b <= 128; b *= 2)
         for (int s = 1; s <= (1 << f32_groups_log2(num_kb)); s *= 2) {
-            const double c = terms_cost(b, s, (p.flags & VTP_FLAG_GELU) != 0, m, p.N, num_kb, sms);
-            if (best == 0 || c < best) { best = c; bn = b; split = s; }
+            const double c = terms_cost(b, s, (p.flags & VTP_FLAG_GELU) != 0, likely_tiles(p, b), num_kb, sms);
+            if (best == 0 || c < best) { best = c; *bn = b; *split = s; }
         }
-    return linear_f32_terms_as(p, bn, split, st);
+    return best;
+}
+
+int linear_f32_terms(const LinearArgs& p, cudaStream_t st) {
+    if (int rc = check_terms(p)) return rc;
+    if (p.m_max == 0) return VTP_OK;
+    int bn = 64, split = 1;
+    best_terms(p, &bn, &split);
+    return linear_f32_terms_as(p, nullptr, bn, split, st);
+}
+
+// Two problems that do not depend on each other, with the same K and kind of output: in one launch where that looks the shorter (a launch
+// costs some 4000 cycles beside its tiles; one of both splits no reduction).
+int linear_f32_terms_pair(const LinearArgs& a, const LinearArgs& b, cudaStream_t st) {
+    if (int rc = check_terms(a)) return rc;
+    if (int rc = check_terms(b)) return rc;
+    const int num_kb = ceil_div(a.K, FK), sms = sm_count();
+    int bn = 64, split = 1;
+    const double apart = best_terms(a, &bn, &split) + best_terms(b, &bn, &split) + 4000;
+    double together = 0;
+    for (int w = 64; w <= 128; w *= 2) {
+        const double c = terms_cost(w, 1, false, likely_tiles(a, w) + likely_tiles(b, w), num_kb, sms);
+        if (together == 0 || c < together) { together = c; bn = w; }
+    }
+    const bool fit = a.K == b.K && a.out_terms == b.out_terms && !((a.flags | b.flags) & VTP_FLAG_GELU) && a.m_max > 0 && b.m_max > 0;
+    if (fit && together < apart) return linear_f32_terms_as(a, &b, bn, 1, st);
+    if (int rc = linear_f32_terms(a, st)) return rc;
+    return linear_f32_terms(b, st);
 }
 
 }  // namespace vtp
