@@ -11,11 +11,13 @@
 // (8 bf16 / 4 fp32): 4 instances per warp at C = 64 in bf16.  A point's corner arithmetic and the reductions over
 // the channels are then paid once per 16 bytes instead of once per channel pair, and the input gradient leaves as
 // one vector red per corner.
-// Measured on 32 maps of 64 x 64 x 64, 9 points, bf16, point mode: forward + backward 525 -> 245 us (now 71 + 163
-// us) against a warp per instance with a channel pair per lane.  Bound: the issue slots (76 % busy) and, in the
-// backward, the SM's request port to L2 (69 %: 4 x 128 bytes of reds per point); DRAM 5 %.  Tried and not kept, same
-// inputs: contiguous query ranges per SM for the L1 (71 -> 76 / 163 -> 157 us), packed f32x2 arithmetic (70 / 163 us),
-// a point's corners worked out by one lane and handed round by shuffles (78 / 159 us), no reds at all 136 us.
+// Measured on 32 maps of 64 x 64 x 64, 9 points, bf16, point mode: forward + backward 525 -> 245 us (71 + 163 us) against a
+// warp per instance with a channel pair per lane, 187 (65 + 122) with the backward's sums formed from four dot products and
+// taps outside the map as zeroed raw words.  Bound: the issue slots and, in the backward, the SM's request port to L2 (69 % at 163 us: 4 x 128 bytes of reds
+// per point); DRAM 5 %.  Tried and not kept, with the sums as they were: contiguous query ranges per SM for the L1 (71 -> 76 / 163 ->
+// 157 us), packed f32x2 arithmetic (70 / 163 us), a point's corners worked out by one lane and handed round by shuffles (78 /
+// 159 us), no reds at all 136 us; and the corners' weights times the point's in front of the channels, whose rounding is the
+// larger one (forward 71 -> 69 us, relative error in fp32 6.0e-8 -> 7.8e-8).
 #include <initializer_list>
 
 #include "common.cuh"
@@ -61,6 +63,12 @@ template <typename T, int V> struct Pack {
         v.load(p);
         v.to_float(f);
     }
+    // zeros unless `in`
+    static __device__ __forceinline__ void load_if(bool in, const T* p, float (&f)[V]) {
+        Vec<T> v = {};
+        if (in) v.load(p);
+        v.to_float(f);
+    }
     static __device__ __forceinline__ void store(T* p, const float (&f)[V]) {
         Vec<T> v;
         v.from_float(f);
@@ -79,11 +87,19 @@ template <typename T, int V> struct Pack {
     }
 };
 template <> struct Pack<float, 1> {
+    static __device__ __forceinline__ void load_if(bool in, const float* p, float (&f)[1]) {
+        for (int v = 0; v < 1; ++v) f[v] = 0.f;
+        if (in) load(p, f);
+    }
     static __device__ __forceinline__ void load(const float* p, float (&f)[1]) { f[0] = *p; }
     static __device__ __forceinline__ void store(float* p, const float (&f)[1]) { *p = f[0]; }
     static __device__ __forceinline__ void atomic_add(float* p, const float (&f)[1]) { atomicAdd(p, f[0]); }
 };
 template <> struct Pack<float, 2> {
+    static __device__ __forceinline__ void load_if(bool in, const float* p, float (&f)[2]) {
+        for (int v = 0; v < 2; ++v) f[v] = 0.f;
+        if (in) load(p, f);
+    }
     static __device__ __forceinline__ void load(const float* p, float (&f)[2]) {
         const float2 v = *reinterpret_cast<const float2*>(p);
         f[0] = v.x; f[1] = v.y;
@@ -96,6 +112,10 @@ template <> struct Pack<float, 2> {
     }
 };
 template <> struct Pack<bf16, 1> {
+    static __device__ __forceinline__ void load_if(bool in, const bf16* p, float (&f)[1]) {
+        for (int v = 0; v < 1; ++v) f[v] = 0.f;
+        if (in) load(p, f);
+    }
     static __device__ __forceinline__ void load(const bf16* p, float (&f)[1]) { f[0] = __bfloat162float(*p); }
     static __device__ __forceinline__ void store(bf16* p, const float (&f)[1]) { *p = __float2bfloat16_rn(f[0]); }
     static __device__ __forceinline__ void atomic_add(bf16* p, const float (&f)[1]) {
@@ -103,6 +123,10 @@ template <> struct Pack<bf16, 1> {
     }
 };
 template <> struct Pack<bf16, 2> {
+    static __device__ __forceinline__ void load_if(bool in, const bf16* p, float (&f)[2]) {
+        for (int v = 0; v < 2; ++v) f[v] = 0.f;
+        if (in) load(p, f);
+    }
     static __device__ __forceinline__ void load(const bf16* p, float (&f)[2]) {
         const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
         f[0] = v.x; f[1] = v.y;
@@ -120,12 +144,10 @@ struct Taps {
     float lt[V], rt[V], lb[V], rb[V];
     __device__ __forceinline__ void load(const T* __restrict__ img, const Corner& k, int W, int C, int c) {
         const size_t o = ((size_t)k.y0 * W + k.x0) * C + c;   // only dereferenced where in-bounds
-#pragma unroll
-        for (int v = 0; v < V; ++v) lt[v] = rt[v] = lb[v] = rb[v] = 0.f;
-        if (k.in_lt) Pack<T, V>::load(img + o, lt);
-        if (k.in_rt) Pack<T, V>::load(img + o + C, rt);
-        if (k.in_lb) Pack<T, V>::load(img + o + (size_t)W * C, lb);
-        if (k.in_rb) Pack<T, V>::load(img + o + (size_t)W * C + C, rb);
+        Pack<T, V>::load_if(k.in_lt, img + o, lt);
+        Pack<T, V>::load_if(k.in_rt, img + o + C, rt);
+        Pack<T, V>::load_if(k.in_lb, img + o + (size_t)W * C, lb);
+        Pack<T, V>::load_if(k.in_rb, img + o + (size_t)W * C + C, rb);
     }
     __device__ __forceinline__ float value(const Corner& k, int v) const {
         return k.w_lt * lt[v] + k.w_rt * rt[v] + k.w_lb * lb[v] + k.w_rb * rb[v];
@@ -133,12 +155,13 @@ struct Taps {
 };
 
 template <typename T, int V>
-__device__ __forceinline__ void scatter(T* __restrict__ gimg, const Corner& k, int W, int C, int c, const float (&g)[V]) {
+__device__ __forceinline__ void scatter(T* __restrict__ gimg, const Corner& k, int W, int C, int c, const float (&up)[V], float sc) {
     const size_t o = ((size_t)k.y0 * W + k.x0) * C + c;
     float t[V];
 #define VTP_BA_SCATTER(IN, OFF, WT)                              \
     if (IN) {                                                    \
-        _Pragma("unroll") for (int v = 0; v < V; ++v) t[v] = g[v] * (WT); \
+        const float a = sc * (WT);                               \
+        _Pragma("unroll") for (int v = 0; v < V; ++v) t[v] = up[v] * a; \
         Pack<T, V>::atomic_add(gimg + o + (OFF), t);             \
     }
     VTP_BA_SCATTER(k.in_lt, 0, k.w_lt)
@@ -237,8 +260,9 @@ bilinear_attention_bwd_kernel(const T* __restrict__ grad_out, const T* __restric
     constexpr bool VEC = V == Vec<T>::N;
     const int lane = threadIdx.x & 31, gl = lane % LG, sub = lane / LG;
     const long long n_inst = (long long)B * G;
-    for (long long first = ((long long)blockIdx.x * BA_WARPS + (threadIdx.x >> 5)) * PW; first < n_inst;
-         first += (long long)gridDim.x * BA_WARPS * PW) {
+    const int warps = (int)(blockDim.x >> 5);
+    for (long long first = ((long long)blockIdx.x * warps + (threadIdx.x >> 5)) * PW; first < n_inst;
+         first += (long long)gridDim.x * warps * PW) {
         const bool own = first + sub < n_inst;           // a group past the end goes along for the shuffles
         const long long inst = own ? first + sub : first;
         const int Hb = own ? H : 0;                      // and touches no pixel
@@ -261,30 +285,34 @@ bilinear_attention_bwd_kernel(const T* __restrict__ grad_out, const T* __restric
             const Corner k = corners_of(sane(xy.x, W), sane(xy.y, H), Hb, W);
             // scale turning up[] into g = d(loss) / d(sample(b, p, c))
             const float sc = POINT ? to_f32(weight[(size_t)inst * P + p]) : to_f32(grad_out[(size_t)inst * P + p]);
-            float gix = 0.f, giy = 0.f, giw = 0.f;
+            // Everything that is summed over the channels is a combination of four sums, up times each corner: four multiply-adds a
+            // channel instead of sixteen
+            float d_lt = 0.f, d_rt = 0.f, d_lb = 0.f, d_rb = 0.f;
 #pragma unroll
             for (int j = 0; j < J; ++j) {
                 const int c = (gl + LG * j) * V;
                 if (c < C) {
-                    float g[V];
-#pragma unroll
-                    for (int v = 0; v < V; ++v) g[v] = up[j][v] * sc;
                     Taps<T, V> t;
                     t.load(img, k, W, C, c);
-                    scatter<T, V>(gimg, k, W, C, c, g);
+                    scatter<T, V>(gimg, k, W, C, c, up[j], sc);
 #pragma unroll
                     for (int v = 0; v < V; ++v) {
-                        // d(sample)/dx and d(sample)/dy of the bilinear form
-                        gix += g[v] * ((t.rt[v] - t.lt[v]) * (1.f - k.ty) + (t.rb[v] - t.lb[v]) * k.ty);
-                        giy += g[v] * ((t.lb[v] - t.lt[v]) * (1.f - k.tx) + (t.rb[v] - t.rt[v]) * k.tx);
-                        if (POINT) giw += t.value(k, v) * up[j][v];
-                        else gw_c[j][v] += t.value(k, v) * sc;
+                        d_lt = fmaf(up[j][v], t.lt[v], d_lt);
+                        d_rt = fmaf(up[j][v], t.rt[v], d_rt);
+                        d_lb = fmaf(up[j][v], t.lb[v], d_lb);
+                        d_rb = fmaf(up[j][v], t.rb[v], d_rb);
+                        if (!POINT) gw_c[j][v] += t.value(k, v) * sc;
                     }
                 }
             }
-            gix = group_sum<LG>(gix);
-            giy = group_sum<LG>(giy);
-            if (POINT) giw = group_sum<LG>(giw);
+            d_lt = group_sum<LG>(d_lt);
+            d_rt = group_sum<LG>(d_rt);
+            d_lb = group_sum<LG>(d_lb);
+            d_rb = group_sum<LG>(d_rb);
+            // d(sample)/dx and d(sample)/dy of the bilinear form
+            const float gix = sc * ((d_rt - d_lt) * (1.f - k.ty) + (d_rb - d_lb) * k.ty);
+            const float giy = sc * ((d_lb - d_lt) * (1.f - k.tx) + (d_rb - d_rt) * k.tx);
+            const float giw = k.w_lt * d_lt + k.w_rt * d_rt + k.w_lb * d_lb + k.w_rb * d_rb;
             if (gl == 0 && own) {
                 grad_grid[((size_t)inst * P + p) * 2] = from_f32<T>(gix);
                 grad_grid[((size_t)inst * P + p) * 2 + 1] = from_f32<T>(giy);
@@ -390,9 +418,11 @@ extern "C" int vtp_bilinear_attention_backward(const void* grad_out, const void*
     const BaLayout lay = mode == 0 ? ba_layout(dtype, C, grid, {input, grad_input, grad_out})
                                    : ba_layout(dtype, C, grid, {input, grad_input, weight, grad_weight});
     const int blocks = ba_grid((long long)B * G, 32 / lay.lanes);
+    // What one block could hold is worked off by one warp: its reds arrive in one order, and the smallest gradients repeat bit for bit.
+    const int warps = (long long)B * G <= BA_WARPS * (32 / lay.lanes) ? 1 : BA_WARPS;
 #define VTP_BA_BWD(T, V, LG)                                                                                 \
     (mode == 0 ? bilinear_attention_bwd_kernel<T, true, V, LG> : bilinear_attention_bwd_kernel<T, false, V, LG>) \
-        <<<blocks, BA_WARPS * 32, 0, st>>>((const T*)grad_out, (const T*)input, (const T*)grid, (const T*)weight, \
+        <<<blocks, warps * 32, 0, st>>>((const T*)grad_out, (const T*)input, (const T*)grid, (const T*)weight, \
                                            (T*)grad_input, (T*)grad_grid, (T*)grad_weight, B, H, W, C, G, P)
     if (dtype == VTP_F32) VTP_BA_DISPATCH(float, 4, VTP_BA_BWD);
     else VTP_BA_DISPATCH(bf16, 8, VTP_BA_BWD);
