@@ -157,6 +157,23 @@ def test_attention_fp32_on_terms(n_grid, heads, special):
             assert rel_err(out, ref) < 2e-6
 
 
+@pytest.mark.parametrize("B", [33, 256, 257])
+def test_block_fp32_items_of_runs_of_images(B):
+    """The items of the fp32 attention are listed in three ways, for up to 32, up to 256 and more images: an image's bits are those
+    it has in a batch of 16."""
+    from vtpack_b200 import _lib
+    from vtpack_b200.models.dge.deit_dge import Block
+    torch.manual_seed(B)
+    blk = Block(64, 1, mlp_ratio=1.0, qkv_bias=True, split_sizes=[4, 2, 1]).to(DEV).eval()
+    x = torch.randn(B, 145, 64, device=DEV)
+    gate = torch.eye(3)[torch.randint(0, 3, (B, 3, 3))]
+    with torch.no_grad():
+        whole = blk(x, forced_gate=gate)
+        parts = torch.cat([blk(x[i:i + 16].contiguous(), forced_gate=gate[i:i + 16]) for i in range(0, B, 16)])
+    assert _lib.device_status() == 0
+    assert torch.equal(whole, parts)
+
+
 def test_layer_512px_skewed_fp32():
     """32x32 grid (N=1025, 64 regions); even images all-coarse, odd all-fine."""
     sd = O.make_state_dict(128, 1, 2, img_size=512, seed=10)

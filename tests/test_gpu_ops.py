@@ -293,6 +293,21 @@ def test_attention_bf16_many_images(vl, B):
     assert got.shape == ref.shape and rel_err(got.float(), ref) < 8e-3
 
 
+@pytest.mark.parametrize("B", [32, 34, 63, 65, 129, 255, 256, 257])
+def test_attention_items_of_runs_of_images(vl, B):
+    """Up to 32, up to 256 and more images have their items listed in three ways, the first two by one warp that looks for its own
+    first item among runs of one to eight images: images without queries in front, at the end, in the middle and over whole runs,
+    a partial last run, one to three tiles an image.  Bound as above."""
+    _lib, layers = vl
+    lens = [(0, 5, 130, 0, 257, 1, 128, 0, 129)[(i * i + i // 9) % 9] for i in range(B)]
+    lens[0] = lens[-1] = lens[-2] = 0
+    lens[B // 3:B // 3 + 17] = [0] * len(lens[B // 3:B // 3 + 17])
+    q, k, v, ref = _attn_case(torch.bfloat16, B, 17, 3, lens, seed=B)
+    got = layers.batched_sparse_attention(q.to(DEV), k.to(DEV), v.to(DEV), torch.tensor(lens), 64 ** -0.5)
+    assert _lib.device_status() == 0
+    assert got.shape == ref.shape and rel_err(got.float(), ref) < 8e-3
+
+
 def test_attention_strided_views(vl):
     """q / k / v as permuted views of Linear outputs, as the model passes them."""
     _, layers = vl

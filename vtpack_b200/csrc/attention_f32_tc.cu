@@ -160,17 +160,22 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     };
     __syncthreads();                                 // (the barriers exist)
     pdl_begin();
-    // (of up to 32 images warp 0 lists the items alone and sends for the first one's Q and first keys before the others know the list)
+    // (of up to 256 images warp 0 lists the items alone and sends for the first one's Q and first keys before the others know the list)
     const bool few = g.B <= FEW_IMAGES;
-    int o0 = 0, o1 = 0;
-    if (few && warp == 0 && lane < g.B) { o0 = g.offsets[lane]; o1 = g.offsets[lane + 1]; }
-    if (threadIdx.x == 0) *void_s = launch_is_void(status) ? 1 : 0;
+    FewImages<1> one_each;
+    FewImages<FEW_PER> some_each;
+    if (few && warp == 0) {
+        if (g.B <= 32) one_each.load(g.offsets, g.B);
+        else some_each.load(g.offsets, g.B);
+    }
+    if (threadIdx.x == (few ? 0 : blockDim.x - 1)) *void_s = launch_is_void(status) ? 1 : 0;
     AttnItem first_item;
     if (!few) {
         list_tiles(g.offsets, g.B, g.max_q, g.l_max, status, tile_prefix, offs);
     } else if (warp == 0) {
         __syncwarp();
-        const int n_tiles = list_few_tiles(o0, o1, g.B, g.max_q, g.l_max, status, tile_prefix, offs, blockIdx.x, g.heads, first_item);
+        const int n_tiles = g.B <= 32 ? one_each.list(g.B, g.max_q, g.l_max, status, tile_prefix, offs, blockIdx.x, g.heads, first_item)
+                                     : some_each.list(g.B, g.max_q, g.l_max, status, tile_prefix, offs, blockIdx.x, g.heads, first_item);
         if (*void_s == 0 && (int)blockIdx.x < n_tiles * g.heads && elect_one()) {
             load_q(first_item, 0);
             load_kv(first_item, 0, 0, 0, min(2, g.n_blocks / g.n_chunks));       // (the first chunk has so many blocks)

@@ -71,42 +71,67 @@ __device__ __forceinline__ AttnItem attn_item(int w, int heads, int B, const int
     return it;
 }
 
-// The same for up to 32 images by one warp alone, which also works out item `w`, so that its loads are under way before the other
-// warps know the list: o0, o1 are offsets[lane] and offsets[lane + 1] (lane < B, else 0).  Returns the number of tiles; `it` holds only if
-// w is below that times heads.
-constexpr int FEW_IMAGES = 32;
-__device__ __forceinline__ int list_few_tiles(int o0, int o1, int B, int max_q, int l_max, int* status, int* tile_prefix, int32_t* offs,
-                                              int w, int heads, AttnItem& it) {
-    const int lane = threadIdx.x & 31;
-    int cnt = o1 - o0;
-#if VTP_INDEX_GUARDS
-    if (cnt < 0 || cnt > max_q || o0 < 0 || o1 > l_max) {
-        if (status && blockIdx.x == 0) atomicOr(status, STATUS_BAD_INDEX);
-        cnt = (o0 < 0) ? 0 : min(max(cnt, 0), max_q);
-    }
-#endif
-    const int tiles = lane < B ? (cnt + QT - 1) / QT : 0;
-    int incl = tiles;
+// The same for up to 32 * PER images by one warp alone, a run of up to PER images per lane, which also works out item `w`, so that
+// its loads are under way before the other warps know the list.  Two steps, so that the caller can look at other memory while the
+// offsets are under way.  Batches of up to 32 images have a form of their own: with eight images per lane, DeiT-Ti of 12 images
+// takes 516 us instead of 507 (523 with list_tiles), DeiT-B of 8 images 935 instead of 925 (940).
+constexpr int FEW_PER = 8, FEW_IMAGES = 32 * FEW_PER;
+template <int PER>
+struct FewImages {
+    int o[PER + 1];                // offsets of the lane's images b0 .. b0 + n - 1 and of the one behind them
+    int b0, n;
+
+    __device__ __forceinline__ void load(const int32_t* __restrict__ offsets, int B) {
+        const int lane = threadIdx.x & 31, per = PER == 1 ? 1 : (B + 31) / 32;
+        b0 = min(lane * per, B);
+        n = min(per, B - b0);
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int nb = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += nb;
+        for (int i = 0; i <= PER; ++i) o[i] = (n > 0 && i <= n) ? offsets[b0 + i] : 0;
     }
-    const int excl = incl - tiles, total = __shfl_sync(0xffffffffu, incl, 31);
-    if (lane < B) {
-        tile_prefix[lane] = excl;
-        offs[lane] = o0;
-        if (lane + 1 == B) { tile_prefix[B] = total; offs[B] = o1; }
+
+    // Returns the number of tiles; `it` holds only if w is below that times heads.
+    __device__ __forceinline__ int list(int B, int max_q, int l_max, int* status, int* tile_prefix, int32_t* offs, int w, int heads,
+                                        AttnItem& it) const {
+        const int lane = threadIdx.x & 31;
+        int before[PER], sum = 0;              // tiles of the lane's images in front of an image
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            int cnt = i < n ? o[i + 1] - o[i] : 0;
+#if VTP_INDEX_GUARDS
+            if (i < n && (cnt < 0 || cnt > max_q || o[i] < 0 || o[i + 1] > l_max)) {
+                if (status && blockIdx.x == 0) atomicOr(status, STATUS_BAD_INDEX);
+                cnt = (o[i] < 0) ? 0 : min(max(cnt, 0), max_q);
+            }
+#endif
+            before[i] = sum;
+            sum += (cnt + QT - 1) / QT;
+        }
+        int incl = sum;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int nb = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += nb;
+        }
+        const int excl = incl - sum, total = __shfl_sync(0xffffffffu, incl, 31);
+        // the last image whose first tile is not behind tile tg (as attn_item finds it): the last of the lane's and the lane that has it
+        const int tg = w / heads;
+        int b = 0, row0 = 0, end = 0;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            if (i >= n) continue;
+            const int first = excl + before[i];
+            tile_prefix[b0 + i] = first;
+            offs[b0 + i] = o[i];
+            if (first <= tg) { b = b0 + i; row0 = o[i] + (tg - first) * QT; end = o[i + 1]; }
+            if (b0 + i + 1 == B) { tile_prefix[B] = total; offs[B] = o[i + 1]; }
+        }
+        const int from = 31 - __clz(__ballot_sync(0xffffffffu, n > 0 && excl <= tg));
+        it.b = __shfl_sync(0xffffffffu, b, from);
+        it.h = w - tg * heads;
+        it.row0 = __shfl_sync(0xffffffffu, row0, from);
+        it.nq = min(QT, __shfl_sync(0xffffffffu, end, from) - it.row0);
+        return total;
     }
-    const int tg = w / heads;
-    // the last image whose first tile is not behind tile tg (as attn_item finds it)
-    const int b = 31 - __clz(__ballot_sync(0xffffffffu, lane < B && excl <= tg));
-    const int first = __shfl_sync(0xffffffffu, o0, b), end = __shfl_sync(0xffffffffu, o1, b);
-    it.b = b;
-    it.h = w - tg * heads;
-    it.row0 = first + (tg - __shfl_sync(0xffffffffu, excl, b)) * QT;
-    it.nq = min(QT, end - it.row0);
-    return total;
-}
+};
 
 }  // namespace vtp

@@ -145,18 +145,24 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     // Nothing above depends on the kernel in front of this one on the stream; the packed-row
     // offsets, q, k and v below do.
     pdl_begin();
-    // The items.  Of up to 32 images warp 0 lists them alone and sends for the first one's operands before the others know the list:
-    // DeiT-Ti, one image, 8.3 -> 7.9 us a launch, DeiT-S, 7 images, 10.1 -> 9.3.
+    // The items.  Of up to 256 images warp 0 lists them alone and sends for the first one's operands before the others know the list
+    // (all threads listing them first / this): DeiT-Ti, one image, 8.3 / 7.9 us a launch, DeiT-S, 7 images, 10.1 / 9.3; the forward of
+    // PVT-tiny, 48 images, 986 / 975 us, DeiT-Ti, 96 images, 1015 / 1011, 200 images, 1679 / 1657.
     const bool few = B <= FEW_IMAGES, keep = B <= OFFSETS_KEPT;
-    int o0 = 0, o1 = 0;
-    if (few && warp == 0 && lane < B) { o0 = offsets[lane]; o1 = offsets[lane + 1]; }
-    if (threadIdx.x == 0) *void_s = launch_is_void(status) ? 1 : 0;
+    FewImages<1> one_each;
+    FewImages<FEW_PER> some_each;
+    if (few && warp == 0) {
+        if (B <= 32) one_each.load(offsets, B);
+        else some_each.load(offsets, B);
+    }
+    if (threadIdx.x == (few ? 0 : blockDim.x - 1)) *void_s = launch_is_void(status) ? 1 : 0;
     AttnItem first_item;
     if (!few) {
         list_tiles(offsets, B, max_q, l_max, status, tile_prefix, keep ? offs_s : nullptr);
     } else if (warp == 0) {
         __syncwarp();
-        const int n_tiles = list_few_tiles(o0, o1, B, max_q, l_max, status, tile_prefix, offs_s, blockIdx.x, heads, first_item);
+        const int n_tiles = B <= 32 ? one_each.list(B, max_q, l_max, status, tile_prefix, offs_s, blockIdx.x, heads, first_item)
+                                   : some_each.list(B, max_q, l_max, status, tile_prefix, offs_s, blockIdx.x, heads, first_item);
         if (*void_s == 0 && (int)blockIdx.x < n_tiles * heads && elect_one()) {
             load_q(first_item, 0);
             load_k(first_item, 0);
