@@ -738,6 +738,46 @@ def test_q_and_kv_in_one_launch_same_bits_for_an_image(C, B, fine):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("B", [1, 10, 40, 150])
+@pytest.mark.parametrize("C", [64, 128, 320])
+def test_q_and_kv_in_one_launch_behind_a_reduction(C, B, dtype):
+    """q, which folds norm1 in bf16, and kv of reduced keys, which does not, as one launch (tiles of 64 and 128 columns all at once, the
+    persistent kernel's narrow and wide ones) and as two, which is how a block with events between its stages runs: the same bits,
+    biases of -0 included."""
+    import ctypes
+
+    from vtpack_b200 import _lib
+    from vtpack_b200.models.dge import pvt_dge
+    torch.manual_seed(C + B)
+    blk = pvt_dge.Block(C, C // 64, mlp_ratio=1, qkv_bias=True, sr_ratio=2, split_sizes=[4, 2, 1]).eval()
+    with torch.no_grad():
+        for p in blk.parameters():
+            if p.is_floating_point():
+                torch.nn.init.normal_(p, std=0.2)
+        blk.attn.kv.bias[: 2 * C: 3] = -0.0
+    blk = blk.to(device=DEV, dtype=dtype)
+    x = torch.randn(B, 256, C, device=DEV).to(dtype)
+    gate = torch.randn(B, 4, 4, 3, device=DEV)
+    got = blk(x, 16, 16, forced_gate=gate)
+    s = pvt_dge._shape_struct(dtype, B, 16, 16, 0, C, C // 64, C, [4, 2, 1], blk.norm1.eps, 0, blk.attn.scale)
+    s.sr_ratio, s.sr_eps = 2, float(blk.attn.norm.eps)
+    w, lib = pvt_dge._pack_block(blk, dtype), _lib.lib()
+    n = lib.vtp_block_workspace_bytes(ctypes.byref(s))
+    ws, out = torch.empty(n, dtype=torch.uint8, device=DEV), torch.empty_like(x)
+    counts = torch.empty(B, dtype=torch.int32, device=DEV)
+    events = [torch.cuda.Event(enable_timing=True) for _ in range(12)]
+    for e in events:
+        e.record()
+    arr = (ctypes.c_void_p * 12)(*[e.cuda_event for e in events])
+    _lib.check(lib.vtp_dge_block_forward_timed(ctypes.byref(s), ctypes.byref(w), x.data_ptr(), out.data_ptr(), gate.data_ptr(),
+                                               counts.data_ptr(), ws.data_ptr(), n, arr, 12,
+                                               torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
+    assert bool(got.isfinite().all()) and torch.equal(got, out)
+
+
 @pytest.mark.parametrize("forced", [False, True])
 @pytest.mark.parametrize("extra", [0, 1])
 def test_packed_rows_listed_or_derived_by_the_pool(extra, forced):

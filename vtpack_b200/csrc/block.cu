@@ -310,9 +310,17 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
     lq.y = b.qp; lq.ldy = C; lq.dtype = s.dtype; lq.m_max = rows; lq.m_dev = L_dev; lq.N = C; lq.K = C; lq.flags = kflag;
     if (fold_q) { lq.ln_mode = 1; lq.ln_stats = b.stats_q; lq.ln_s = w.q_s; }
 
-    const void* keys_in = fold ? x_in : b.xn;
+    LinearArgs lkv;  // kv = LN(x) Wkv^T + b, rows stay [b, key, {k,v}, head, d]
+    lkv.a = reduce ? b.sr_norm : fold ? x_in : b.xn; lkv.lda = C; lkv.w = fold ? w.kv_wf : w.kv_w; lkv.bias = fold ? w.kv_c : w.kv_b;
+    lkv.y = b.kv; lkv.ldy = 2 * C; lkv.dtype = s.dtype; lkv.m_max = s.B * n_keys; lkv.N = 2 * C; lkv.K = C; lkv.flags = kflag;
+    if (fold) { lkv.ln_mode = 1; lkv.ln_stats = stats_x; lkv.ln_s = w.kv_s; }
+    // The two projections do not depend on each other: one launch, the q tiles fill the kv tail.  Behind a reduction as well, where q
+    // waits for the keys although it need not (apart / together: PVT-tiny, 3 / 33 / 96 images, 460 / 803 / 1493 us and 440 / 791 / 1470;
+    // PVT-small, 1 and 96 images, 783 / 2704 and 751 / 2657; in fp32, 1 image, 1228 and 1149).
+    const bool pair_bf16 = fold_q && !marks.events && linear_pair_supported(lkv, lq), pair_f32 = terms && !marks.events;
+    if (!pair_bf16 && !pair_f32 && ((rc = run_linear(lq, b.q_wt, terms_attn)) || (rc = marks.mark(4)))) return rc;
+
     if (reduce) {
-        if ((rc = run_linear(lq, b.q_wt, terms_attn)) || (rc = marks.mark(4))) return rc;
         // x_ = norm(sr(LN1(x) as [B,C,H,W])): the stride-sr convolution as im2col rows times a matrix
         const int krows = s.B * n_keys, KS = s.sr_ratio * s.sr_ratio * C;
         if (terms) rc = token_im2col_terms(b.xn, s.B, s.H, s.W, C, s.sr_ratio, b.sr_cols, st);
@@ -325,23 +333,18 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
         rc = terms ? layernorm_terms(b.sr_out, krows, nullptr, C, w.sr_norm_w, w.sr_norm_b, s.sr_eps, b.sr_norm, st)
                    : vtp_layernorm(b.sr_out, s.dtype, krows, nullptr, C, C, w.sr_norm_w, w.sr_norm_b, s.sr_eps, b.sr_norm, st);
         if (rc) return rc;
-        keys_in = b.sr_norm;
     }
-    LinearArgs lkv;  // kv = LN(x) Wkv^T + b, rows stay [b, key, {k,v}, head, d]
-    lkv.a = keys_in; lkv.lda = C; lkv.w = fold ? w.kv_wf : w.kv_w; lkv.bias = fold ? w.kv_c : w.kv_b;
-    lkv.y = b.kv; lkv.ldy = 2 * C; lkv.dtype = s.dtype; lkv.m_max = s.B * n_keys; lkv.N = 2 * C; lkv.K = C; lkv.flags = kflag;
-    if (fold) { lkv.ln_mode = 1; lkv.ln_stats = stats_x; lkv.ln_s = w.kv_s; }
-    if (fold && !marks.events && linear_pair_supported(lkv, lq)) {
-        // the two projections do not depend on each other: one launch, the q tiles fill the kv tail
-        if ((rc = linear_tcgen05_pair(lkv, lq, st))) return rc;
-    } else if (terms && !reduce && !marks.events) {
+    if (pair_bf16) {
+        rc = linear_tcgen05_pair(lkv, lq, st);
+    } else if (pair_f32) {
         lq.w = b.q_wt; lkv.w = b.kv_wt;
         lq.out_terms = lkv.out_terms = terms_attn;
-        if ((rc = linear_f32_terms_pair(lkv, lq, st))) return rc;
+        rc = linear_f32_terms_pair(lkv, lq, st);
     } else {
-        if (!reduce && ((rc = run_linear(lq, b.q_wt, terms_attn)) || (rc = marks.mark(4)))) return rc;
-        if ((rc = run_linear(lkv, b.kv_wt, terms_attn)) || (rc = marks.mark(5))) return rc;
+        rc = run_linear(lkv, b.kv_wt, terms_attn);
+        if (!rc) rc = marks.mark(5);
     }
+    if (rc) return rc;
 
     AttnArgs at;
     const long long e = (long long)elem_size(s.dtype);

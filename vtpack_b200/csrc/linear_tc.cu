@@ -137,7 +137,8 @@ static_assert(sizeof(TcSharedScalars) % 4 == 0 && sizeof(TcSharedScalars) <= 512
 
 __device__ const __align__(16) float g_no_bias[8] = {};      // what a Linear without a bias adds, read up to 16 bytes at a time
 
-// A row's folded LayerNorm, LN(a) W^T + b = ln_a * acc + (ln_b * s[n] + bias[n]), from its statistics.
+// A row's folded LayerNorm, LN(a) W^T + b = ln_a * acc + (ln_b * s[n] + bias[n]), from its statistics.  The problem of a pair that
+// folds none (mode 0; its s[n] are g_no_bias) gets 1 * acc + (-0 * 0 + bias[n]), which is acc + bias[n] to the last bit.
 __device__ __forceinline__ void row_fold(const LnFold& ln, int m, float& ln_a, float& ln_b) {
     if (ln.mode == 2) {
         // (sum, sum of squares) of each 64-column slab of the row, left by the GEMM that produced it; added in order
@@ -159,6 +160,9 @@ __device__ __forceinline__ void row_fold(const LnFold& ln, int m, float& ln_a, f
         const float mean = s1 / dim;
         ln_a = rsqrtf(fmaxf(s2 / dim - mean * mean, 0.f) + eps);
         ln_b = -ln_a * mean;
+    } else if (ln.mode == 0) {
+        ln_a = 1.f;
+        ln_b = -0.f;
     } else {
         const float2 st = ln.stats[m];
         ln_a = st.y;
@@ -436,7 +440,7 @@ linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
                 for (int c = 0; c < 8; ++c) {
                     const int nb = min(n0 + 8 * c, N - 8) + 2 * (lane & 3);
                     b2[c] = __ldg(reinterpret_cast<const float2*>(P.bias ? P.bias + nb : g_no_bias));
-                    if (EPI & EPI_LN) s2[c] = __ldg(reinterpret_cast<const float2*>(P.ln.s + nb));
+                    if (EPI & EPI_LN) s2[c] = __ldg(reinterpret_cast<const float2*>(NPROB == 2 && !P.ln.s ? g_no_bias : P.ln.s + nb));
                 }
                 if (EPI & EPI_RES) {
                     if (leader) bulk_wait_group_read0();               // the last item's store has read the buffer
@@ -728,7 +732,7 @@ linear_tc_small_kernel(const __grid_constant__ SmallLaunch L, int K, int* status
                     const float4 b4 = __ldg(reinterpret_cast<const float4*>(bias) + (q & 1));
                     add[h][4 * q] = b4.x; add[h][4 * q + 1] = b4.y; add[h][4 * q + 2] = b4.z; add[h][4 * q + 3] = b4.w;
                     if (EPI & EPI_LN) {
-                        const float4 s4 = __ldg(reinterpret_cast<const float4*>(P.ln.s + nb) + (q & 1));
+                        const float4 s4 = __ldg(reinterpret_cast<const float4*>(NPROB == 2 && !P.ln.s ? g_no_bias : P.ln.s + nb) + (q & 1));
                         sv[4 * q] = s4.x; sv[4 * q + 1] = s4.y; sv[4 * q + 2] = s4.z; sv[4 * q + 3] = s4.w;
                     }
                 }
@@ -1051,16 +1055,15 @@ static int check_tc_args(const LinearArgs& p) {
     return VTP_OK;
 }
 
-// Two independent Linears that follow the same kind of LayerNorm fold (the q and kv projections of a block)
-// in ONE launch of 256-wide tiles: the tiles of the second problem fill the last, partial round of the first,
-// and one launch's ramp and tail is saved.  Both: bf16 output, bias + folded LayerNorm (ln_mode 1), no
-// residual, no row remap; N a multiple of 64.
+// Two independent Linears of the same K (the q and kv projections of a block) in ONE launch: the tiles of the second problem fill
+// the last, partial round of the first, and one launch's ramp and tail is saved.  Both: bf16 output, bias, no residual, no row
+// remap, N a multiple of 64; one or both fold a LayerNorm (ln_mode 1: a block that reduces its keys folds only q's).
 bool linear_pair_supported(const LinearArgs& a, const LinearArgs& b) {
     auto ok = [](const LinearArgs& p) {
-        return p.dtype == VTP_BF16 && p.ln_mode == 1 && !p.res && !p.emit_stats && p.out_grp == 0 && p.flags == 0 &&
+        return p.dtype == VTP_BF16 && (p.ln_mode == 1 || (p.ln_mode == 0 && !p.ln_s)) && !p.res && !p.emit_stats && p.out_grp == 0 && p.flags == 0 &&
                p.m_max > 0 && p.N >= 64 && p.N % 64 == 0;
     };
-    return ok(a) && ok(b) && a.K == b.K;
+    return ok(a) && ok(b) && a.K == b.K && a.ln_mode + b.ln_mode > 0;
 }
 
 // Whether two CTAs should share 256-row tiles (cta_group::2).  Each then loads and multiplies half of the tile's W rows, which
@@ -1081,6 +1084,9 @@ int linear_tcgen05_pair(const LinearArgs& a, const LinearArgs& b, cudaStream_t s
     VTP_REQUIRE(linear_pair_supported(a, b), VTP_ERR_UNSUPPORTED, "linear (tcgen05): these two problems cannot share a launch");
     if (small_tiles(a, 64) + small_tiles(b, 64) <= sm_count()) return launch_small<64, EPI_LN, false, 2>(a, &b, st);
     if (small_tiles(a, 128, true) + small_tiles(b, 128, true) <= sm_count()) return launch_small<128, EPI_LN, false, 2>(a, &b, st);
+    // (narrow tiles where most of the work, the problem of more rows, has no more than 128 columns: the queries of PVT's first two stages,
+    // whose keys are few; PVT-tiny, 96 images, 1470 us)
+    if (pick_bn((a.m_max > b.m_max ? a : b).N) == 128) return launch_tc<128, 1, EPI_LN, false, 2>(a, &b, st);
     if (pairs_pay(256, a.K)) return launch_tc<256, 2, EPI_LN, false, 2>(a, &b, st);
     return launch_tc<256, 1, EPI_LN, false, 2>(a, &b, st);
 }
