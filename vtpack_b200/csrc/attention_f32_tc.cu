@@ -105,6 +105,7 @@ __device__ __noinline__ void redo_row(const AfArgs& g, int b, int h, long long r
 
 template <bool V> struct Masked { static constexpr bool value = V; };
 
+template <int PER>
 __global__ void __launch_bounds__(AF_THREADS, 1)
 attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_kv,
                    const __grid_constant__ AfArgs g, int* status) {
@@ -161,21 +162,16 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     __syncthreads();                                 // (the barriers exist)
     pdl_begin();
     // (of up to 256 images warp 0 lists the items alone and sends for the first one's Q and first keys before the others know the list)
-    const bool few = g.B <= FEW_IMAGES;
-    FewImages<1> one_each;
-    FewImages<FEW_PER> some_each;
-    if (few && warp == 0) {
-        if (g.B <= 32) one_each.load(g.offsets, g.B);
-        else some_each.load(g.offsets, g.B);
-    }
+    const bool few = PER == 1 || g.B <= FEW_IMAGES;
+    FewImages<PER> images;
+    if (few && warp == 0) images.load(g.offsets, g.B);
     if (threadIdx.x == (few ? 0 : blockDim.x - 1)) *void_s = launch_is_void(status) ? 1 : 0;
     AttnItem first_item;
     if (!few) {
         list_tiles(g.offsets, g.B, g.max_q, g.l_max, status, tile_prefix, offs);
     } else if (warp == 0) {
         __syncwarp();
-        const int n_tiles = g.B <= 32 ? one_each.list(g.B, g.max_q, g.l_max, status, tile_prefix, offs, blockIdx.x, g.heads, first_item)
-                                     : some_each.list(g.B, g.max_q, g.l_max, status, tile_prefix, offs, blockIdx.x, g.heads, first_item);
+        const int n_tiles = images.list(g.B, g.max_q, g.l_max, status, tile_prefix, offs, blockIdx.x, g.heads, first_item);
         if (*void_s == 0 && (int)blockIdx.x < n_tiles * g.heads && elect_one()) {
             load_q(first_item, 0);
             load_kv(first_item, 0, 0, 0, min(2, g.n_blocks / g.n_chunks));       // (the first chunk has so many blocks)
@@ -509,11 +505,15 @@ int attention_f32_terms(const AttnArgs& p, cudaStream_t st) {
         if (int rc = make_tmap_bf16(&tkv, p.k, 4, dims, strides, box)) return rc;
     }
     const int smem = AF_SM_PREFIX + 2 * (p.B + 1) * 4 + 1024;
-    static int attr_smem[64] = {};
+    // (batches of up to 32 images have a kernel of their own, whose code a small launch is through sooner: FewImages)
+    const bool one_each = p.B <= 32;
+    auto kern = one_each ? attn_f32_tc_kernel<1> : attn_f32_tc_kernel<FEW_PER>;
+    static int reserved[2][64] = {};
+    int* attr_smem = reserved[one_each];
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || attr_smem[dev] < smem) {
-        const cudaError_t e = cudaFuncSetAttribute(attn_f32_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) {
             set_error("attention (fp32 terms): cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
             return (int)e;
@@ -522,7 +522,7 @@ int attention_f32_terms(const AttnArgs& p, cudaStream_t st) {
     }
     const long long worst = (long long)p.B * ceil_div(p.max_q, QT) * p.heads;
     const int grid = (int)(worst < sm_count() ? worst : sm_count());
-    const cudaError_t le = launch_kernel(attn_f32_tc_kernel, true, 1, dim3(grid), dim3(AF_THREADS), (size_t)smem, st, tq, tkv, g,
+    const cudaError_t le = launch_kernel(kern, true, 1, dim3(grid), dim3(AF_THREADS), (size_t)smem, st, tq, tkv, g,
                                          device_status_ptr());
     if (le != cudaSuccess) {
         cudaGetLastError();

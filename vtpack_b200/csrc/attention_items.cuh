@@ -73,8 +73,9 @@ __device__ __forceinline__ AttnItem attn_item(int w, int heads, int B, const int
 
 // The same for up to 32 * PER images by one warp alone, a run of up to PER images per lane, which also works out item `w`, so that
 // its loads are under way before the other warps know the list.  Two steps, so that the caller can look at other memory while the
-// offsets are under way.  Batches of up to 32 images have a form of their own: with eight images per lane, DeiT-Ti of 12 images
-// takes 516 us instead of 507 (523 with list_tiles), DeiT-B of 8 images 935 instead of 925 (940).
+// offsets are under way.  Batches of up to 32 images have a form and kernels of
+// their own (DeiT-Ti, 12 images: 519 us with list_tiles, 516 with eight images per lane, 513 with both forms in one kernel, 509
+// apart; DeiT-B, 8 images: 937, 935, 934 and 927).
 constexpr int FEW_PER = 8, FEW_IMAGES = 32 * FEW_PER;
 template <int PER>
 struct FewImages {

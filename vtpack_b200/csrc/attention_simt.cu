@@ -1,4 +1,4 @@
-// Variable-length-query attention on CUDA cores, fp32 arithmetic (fp32 or bf16 storage): the fp32 product path, and
+// Variable-length-query attention on CUDA cores, fp32 arithmetic (fp32 or bf16 storage): fp32 of single calls and of fewer than 128 keys, and
 // an independent check of the tcgen05 kernel.
 //
 // One CTA of four warps owns 32 packed queries of one (image, head) and walks the keys in chunks of up to 144 with an

@@ -71,6 +71,7 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                  : "memory");
 }
 
+template <int PER>
 __global__ void __launch_bounds__(192, 2)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                const __grid_constant__ CUtensorMap tmap_v, const bf16* __restrict__ kptr,
@@ -148,21 +149,16 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     // The items.  Of up to 256 images warp 0 lists them alone and sends for the first one's operands before the others know the list
     // (all threads listing them first / this): DeiT-Ti, one image, 8.3 / 7.9 us a launch, DeiT-S, 7 images, 10.1 / 9.3; the forward of
     // PVT-tiny, 48 images, 986 / 975 us, DeiT-Ti, 96 images, 1015 / 1011, 200 images, 1679 / 1657.
-    const bool few = B <= FEW_IMAGES, keep = B <= OFFSETS_KEPT;
-    FewImages<1> one_each;
-    FewImages<FEW_PER> some_each;
-    if (few && warp == 0) {
-        if (B <= 32) one_each.load(offsets, B);
-        else some_each.load(offsets, B);
-    }
+    const bool few = PER == 1 || B <= FEW_IMAGES, keep = B <= OFFSETS_KEPT;
+    FewImages<PER> images;
+    if (few && warp == 0) images.load(offsets, B);
     if (threadIdx.x == (few ? 0 : blockDim.x - 1)) *void_s = launch_is_void(status) ? 1 : 0;
     AttnItem first_item;
     if (!few) {
         list_tiles(offsets, B, max_q, l_max, status, tile_prefix, keep ? offs_s : nullptr);
     } else if (warp == 0) {
         __syncwarp();
-        const int n_tiles = B <= 32 ? one_each.list(B, max_q, l_max, status, tile_prefix, offs_s, blockIdx.x, heads, first_item)
-                                   : some_each.list(B, max_q, l_max, status, tile_prefix, offs_s, blockIdx.x, heads, first_item);
+        const int n_tiles = images.list(B, max_q, l_max, status, tile_prefix, offs_s, blockIdx.x, heads, first_item);
         if (*void_s == 0 && (int)blockIdx.x < n_tiles * heads && elect_one()) {
             load_q(first_item, 0);
             load_k(first_item, 0);
@@ -498,11 +494,15 @@ int attention_tcgen05(const AttnArgs& p, cudaStream_t st) {
         if (int rc = make_tmap_bf16(&tv, p.v, 3, dims, strides, box)) return rc;
     }
     const int smem = SM_PREFIX + (p.B + 1) * 4 * (p.B <= OFFSETS_KEPT ? 2 : 1) + 1024;
-    static int attr_smem[64] = {};
+    // (batches of up to 32 images have a kernel of their own, whose code a small launch is through sooner: FewImages)
+    const bool one_each = p.B <= 32;
+    auto kern = one_each ? attn_tc_kernel<1> : attn_tc_kernel<FEW_PER>;
+    static int reserved[2][64] = {};
+    int* attr_smem = reserved[one_each];
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || attr_smem[dev] < smem) {
-        const cudaError_t e = cudaFuncSetAttribute(attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) {
             set_error("attention (tcgen05): cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
             return (int)e;
@@ -511,7 +511,7 @@ int attention_tcgen05(const AttnArgs& p, cudaStream_t st) {
     }
     const long long worst = (long long)p.B * ceil_div(p.max_q, QT) * p.heads;
     const int grid = (int)(worst < 2ll * sm_count() ? worst : 2ll * sm_count());
-    const cudaError_t le = launch_kernel(attn_tc_kernel, worst <= sm_count(), 1, dim3(grid), dim3(192), (size_t)smem, st, tq, tk, tv,
+    const cudaError_t le = launch_kernel(kern, worst <= sm_count(), 1, dim3(grid), dim3(192), (size_t)smem, st, tq, tk, tv,
                                       (const bf16*)p.k, (const bf16*)p.v, p.q_hs, p.kv_bs, p.kv_rs, p.kv_hs, (bf16*)p.out,
                                       p.o_rs, p.o_hs, p.B, p.heads, p.n_keys, KC, n_chunks, p.offsets, p.l_max, p.max_q,
                                       p.scale * 1.4426950408889634f, device_status_ptr());

@@ -145,7 +145,8 @@ __device__ __forceinline__ float warp_max(float v) {
 // griddep_launch() lets the kernel behind this one start once every CTA of this grid has called it.  It comes
 // AFTER the wait: a kernel that has started then knows that everything up to the kernel before its
 // predecessor has completed.  What stands before the wait reads no tensor, weights included: the predecessor may be
-// the kernel that writes them.
+// the kernel that writes them.  (One kernel whose predecessor is always of the same call reads weights there:
+// pool_region_terms_kernel.)
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_begin() { griddep_wait(); griddep_launch(); }

@@ -12,6 +12,9 @@
 // registers, rounding to nearest, so a long reduction does not collect the accumulator's own rounding.  Measured
 // against float64 the result is as close as the CUDA-core kernel's sequential fmaf chain (tests/test_gpu_ops.py).
 //
+// For fp32 operands as they are: single Linears, the patch embedding, the head, dense blocks.  The Linears of a DGE block read operands
+// that are terms already (linear_f32_terms.cu); figures of a forward below are from when they ran here.
+//
 // Bound: the SM's shared-memory / L1 port (128 bytes per clock).  A k-block of a 128 x 64 tile passes 96 KB of loads
 // through the L1, 72 KB of operand writes and 144 KB of operand reads (24 MMAs), 2450 cycles, which is its measured
 // time; fewer MMAs or no operand writes shorten it in proportion, more converter warps do not.  32-byte loads move the
