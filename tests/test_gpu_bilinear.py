@@ -88,6 +88,42 @@ def test_bilinear_attention_channel_layouts(op, dtype, mode, C, shift):
         assert rel_err(t.float(), ref) < bound, name
 
 
+@pytest.mark.parametrize("mode", ["point", "channel"])
+@pytest.mark.parametrize("C", [64, 48, 20])
+@pytest.mark.parametrize("kind", ["noise", "offset 100", "offset 1000", "smooth", "vertical edge", "horizontal edge"])
+def test_bilinear_attention_gradients_of_maps_with_common_parts(op, kind, C, mode):
+    """fp32 gradients of the points and weights where neighbouring pixels share most of their value, where they differ a lot across an
+    edge and where taps outside the map are zero: every component within 2^-24 times the roundings on its way, of the sum of
+    what it is formed from.  Derivatives: a difference, its product, up to eight channels of a lane, five steps of shuffles, the
+    fractions, products and sum of the two rows, the scale; weight gradients: three roundings a corner weight, four products
+    and sums, the channels (point mode) or the points (channel mode)."""
+    B, H, W, P = 2, 20, 17, 5
+    inp, grid, weight, grad_out = BO.make_bilinear_inputs(B, H, W, C, H * W, P, seed=C, mode=mode)
+    if kind.startswith("offset"):
+        inp += float(kind.split()[1])
+    elif kind == "smooth":
+        ys, xs = torch.meshgrid(torch.arange(H) / 7.0, torch.arange(W) / 9.0, indexing="ij")
+        inp = 5.0 + torch.sin(xs + ys)[None, :, :, None] + 1e-3 * inp
+    elif kind == "vertical edge":
+        inp[:, :, W // 2:] += 1000.0
+    elif kind == "horizontal edge":
+        inp[:, H // 2:] += 1000.0
+    r = [t.double() for t in (inp, grid, weight, grad_out)]
+    want = getattr(BO, f"bilinear_attention_{mode}wise_backward")(r[3], *r[:3])
+    (lt, rt, lb, rb), _, _, tx, ty = BO._taps(*r[:2])
+    tx, ty = tx[..., None], ty[..., None]
+    up, sc = (r[3], r[2]) if mode == "point" else (r[2], r[3])
+    up, sc = up[:, :, None, :].abs(), sc.abs()
+    of_x = (up * ((rt - lt).abs() * (1 - ty) + (rb - lb).abs() * ty)).sum(-1) * sc
+    of_y = (up * ((lb - lt).abs() * (1 - tx) + (rb - rt).abs() * tx)).sum(-1) * sc
+    value = (1 - tx) * (1 - ty) * lt.abs() + tx * (1 - ty) * rt.abs() + (1 - tx) * ty * lb.abs() + tx * ty * rb.abs()
+    of_w = (value * up).sum(-1) if mode == "point" else (value * sc[..., None]).sum(2)
+    _, _, gg, gw = _run(op, inp, grid, weight, grad_out, mode)
+    for name, got, ref, of, roundings in (("x", gg[..., 0], want[1][..., 0], of_x, 20), ("y", gg[..., 1], want[1][..., 1], of_y, 20),
+                                          ("weight", gw, want[2], of_w, 20)):
+        assert bool(((got.double().cpu() - ref).abs() <= roundings * 2.0 ** -24 * of).all()), name
+
+
 def test_bilinear_attention_points_outside_and_non_finite(op):
     """Points far outside the map, at infinity or NaN read zero and leave zero gradients; nothing is
     dereferenced out of bounds."""

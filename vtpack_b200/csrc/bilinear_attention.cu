@@ -12,12 +12,14 @@
 // the channels are then paid once per 16 bytes instead of once per channel pair, and the input gradient leaves as
 // one vector red per corner.
 // Measured on 32 maps of 64 x 64 x 64, 9 points, bf16, point mode: forward + backward 525 -> 245 us (71 + 163 us) against a
-// warp per instance with a channel pair per lane, 187 (65 + 122) with the backward's sums formed from four dot products and
-// taps outside the map as zeroed raw words.  Bound: the issue slots and, in the backward, the SM's request port to L2 (69 % at 163 us: 4 x 128 bytes of reds
-// per point); DRAM 5 %.  Tried and not kept, with the sums as they were: contiguous query ranges per SM for the L1 (71 -> 76 / 163 ->
-// 157 us), packed f32x2 arithmetic (70 / 163 us), a point's corners worked out by one lane and handed round by shuffles (78 /
-// 159 us), no reds at all 136 us; and the corners' weights times the point's in front of the channels, whose rounding is the
-// larger one (forward 71 -> 69 us, relative error in fp32 6.0e-8 -> 7.8e-8).
+// warp per instance with a channel pair per lane, 203 (65 + 138) with the backward's derivatives formed from four dot products
+// and taps outside the map as zeroed raw words.  Bound: the issue slots and, in the backward, the SM's request port to L2 (69 % at
+// 163 us: 4 x 128 bytes of reds per point); DRAM 5 %.  Tried and not kept, with the sums as they were: contiguous query ranges per SM
+// for the L1 (71 -> 76 / 163 -> 157 us), packed f32x2 arithmetic (70 / 163 us), a point's corners worked out by one lane and handed
+// round by shuffles (78 / 159 us), no reds at all 136 us; and what is faster and less exact, relative errors in fp32: the corners' weights times
+// the point's in front of the channels (forward 71 -> 69 us, 6.0e-8 -> 7.8e-8), derivatives from sums of taps (138 -> 120 us, point
+// gradients of a map with an offset of 100 7.9e-8 -> 6.8e-6), weight gradients from one tap's sum and the differences' (138
+// -> 130 us, 8.2e-8 -> 1.6e-7).
 #include <initializer_list>
 
 #include "common.cuh"
@@ -285,9 +287,11 @@ bilinear_attention_bwd_kernel(const T* __restrict__ grad_out, const T* __restric
             const Corner k = corners_of(sane(xy.x, W), sane(xy.y, H), Hb, W);
             // scale turning up[] into g = d(loss) / d(sample(b, p, c))
             const float sc = POINT ? to_f32(weight[(size_t)inst * P + p]) : to_f32(grad_out[(size_t)inst * P + p]);
-            // Everything that is summed over the channels is a combination of four sums, up times each corner: four multiply-adds a
-            // channel instead of sixteen
-            float d_lt = 0.f, d_rt = 0.f, d_lb = 0.f, d_rb = 0.f;
+            // The derivatives are combinations of four sums over the channels, up times the difference of two taps.  (The differences are
+            // formed per channel: sums of up times each tap cost four subtractions less, but where neighbouring pixels share most of
+            // their value their difference has lost its digits; and each of the four has its own sum, because an edge in
+            // the map or its border makes any one of them as small beside the others.)
+            float d_xt = 0.f, d_xb = 0.f, d_yl = 0.f, d_yr = 0.f, giw = 0.f;
 #pragma unroll
             for (int j = 0; j < J; ++j) {
                 const int c = (gl + LG * j) * V;
@@ -297,22 +301,23 @@ bilinear_attention_bwd_kernel(const T* __restrict__ grad_out, const T* __restric
                     scatter<T, V>(gimg, k, W, C, c, up[j], sc);
 #pragma unroll
                     for (int v = 0; v < V; ++v) {
-                        d_lt = fmaf(up[j][v], t.lt[v], d_lt);
-                        d_rt = fmaf(up[j][v], t.rt[v], d_rt);
-                        d_lb = fmaf(up[j][v], t.lb[v], d_lb);
-                        d_rb = fmaf(up[j][v], t.rb[v], d_rb);
+                        d_xt = fmaf(up[j][v], t.rt[v] - t.lt[v], d_xt);
+                        d_xb = fmaf(up[j][v], t.rb[v] - t.lb[v], d_xb);
+                        d_yl = fmaf(up[j][v], t.lb[v] - t.lt[v], d_yl);
+                        d_yr = fmaf(up[j][v], t.rb[v] - t.rt[v], d_yr);
+                        if (POINT) giw += t.value(k, v) * up[j][v];
                         if (!POINT) gw_c[j][v] += t.value(k, v) * sc;
                     }
                 }
             }
-            d_lt = group_sum<LG>(d_lt);
-            d_rt = group_sum<LG>(d_rt);
-            d_lb = group_sum<LG>(d_lb);
-            d_rb = group_sum<LG>(d_rb);
+            d_xt = group_sum<LG>(d_xt);
+            d_xb = group_sum<LG>(d_xb);
+            d_yl = group_sum<LG>(d_yl);
+            d_yr = group_sum<LG>(d_yr);
+            if (POINT) giw = group_sum<LG>(giw);
             // d(sample)/dx and d(sample)/dy of the bilinear form
-            const float gix = sc * ((d_rt - d_lt) * (1.f - k.ty) + (d_rb - d_lb) * k.ty);
-            const float giy = sc * ((d_lb - d_lt) * (1.f - k.tx) + (d_rb - d_rt) * k.tx);
-            const float giw = k.w_lt * d_lt + k.w_rt * d_rt + k.w_lb * d_lb + k.w_rb * d_rb;
+            const float gix = sc * (d_xt * (1.f - k.ty) + d_xb * k.ty);
+            const float giy = sc * (d_yl * (1.f - k.tx) + d_yr * k.tx);
             if (gl == 0 && own) {
                 grad_grid[((size_t)inst * P + p) * 2] = from_f32<T>(gix);
                 grad_grid[((size_t)inst * P + p) * 2 + 1] = from_f32<T>(giy);
