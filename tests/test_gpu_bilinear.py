@@ -124,19 +124,49 @@ def test_bilinear_attention_gradients_of_maps_with_common_parts(op, kind, C, mod
         assert bool(((got.double().cpu() - ref).abs() <= roundings * 2.0 ** -24 * of).all()), name
 
 
-def test_bilinear_attention_points_outside_and_non_finite(op):
+@pytest.mark.parametrize("G", [10, 150])
+def test_bilinear_attention_points_outside_and_non_finite(op, G):
     """Points far outside the map, at infinity or NaN read zero and leave zero gradients; nothing is
-    dereferenced out of bounds."""
-    inp, grid, weight, grad_out = BO.make_bilinear_inputs(2, 6, 6, 32, 10, 4, seed=5, mode="point")
+    dereferenced out of bounds.  Queries of one block and of several.  The input gradient is a sum of atomic adds in any order: two runs
+    differ by a rounding a term at most, of the sum of the terms' magnitudes (the gradient of the operands' magnitudes)."""
+    inp, grid, weight, grad_out = BO.make_bilinear_inputs(2, 6, 6, 32, G, 4, seed=5, mode="point")
     grid[0, :, 0, :] = 1e30
     grid[0, :, 1, :] = -1e30
     grid[1, :, 2, 0] = float("inf")
     grid[1, :, 3, 1] = float("nan")
     finite = grid.clone()
     finite[~torch.isfinite(finite) | (finite.abs() > 1e6)] = -3.0          # an equivalent all-outside point
-    y, gi, _, gw = _run(op, inp, grid, weight, grad_out, "point")
-    y2, gi2, _, gw2 = _run(op, inp, finite, weight, grad_out, "point")
-    assert torch.isfinite(y).all() and torch.equal(y, y2) and torch.equal(gi, gi2) and torch.equal(gw, gw2)
+    y, gi, gg, gw = _run(op, inp, grid, weight, grad_out, "point")
+    y2, gi2, gg2, gw2 = _run(op, inp, finite, weight, grad_out, "point")
+    assert torch.isfinite(y).all() and torch.equal(y, y2) and torch.equal(gg, gg2) and torch.equal(gw, gw2)
+    assert not bool(gg[0, :, :2].any()) and not bool(gg[1, :, 2:].any()) and not bool(gw[0, :, :2].any())
+    of = _run(op, inp, finite, weight.abs(), grad_out.abs(), "point")[1].double()
+    assert bool(((gi - gi2).double().abs() <= 2 * (4 * G) * 2.0 ** -24 * of).all())
+
+
+@pytest.mark.parametrize("dtype,C,G", [(torch.bfloat16, 32, 64), (torch.float32, 64, 16), (torch.float32, 128, 8)])
+def test_bilinear_attention_smallest_backward_uses_the_whole_block(op, dtype, C, G):
+    """As many queries as one block holds take about what a few more take (64 of them 41 us when one warp worked them all off, 11 now)."""
+    from vtpack_b200 import _lib
+
+    def us(G):
+        t = [v.to(DEV, dtype) for v in BO.make_bilinear_inputs(1, 8, 8, C, G, 9, seed=1, mode="point")]
+        inp, grid, weight, grad_out = t
+        grads = [torch.empty_like(v) for v in t[:3]]
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        best = float("inf")
+        for _ in range(8):
+            e[0].record()
+            for _ in range(20):
+                _lib.check(_lib.lib().vtp_bilinear_attention_backward(
+                    grad_out.data_ptr(), inp.data_ptr(), grid.data_ptr(), weight.data_ptr(), *(g.data_ptr() for g in grads),
+                    0 if dtype == torch.float32 else 1, 0, 1, 8, 8, C, G, 9, torch.cuda.current_stream().cuda_stream))
+            e[1].record()
+            torch.cuda.synchronize()
+            best = min(best, e[0].elapsed_time(e[1]) * 50)
+        return best
+
+    assert us(G) < 1.9 * us(G + G // 4)
 
 
 def test_dpvt_attention_usage(op):

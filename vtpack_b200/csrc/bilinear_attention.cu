@@ -251,7 +251,8 @@ bilinear_attention_fwd_kernel(const T* __restrict__ input, const T* __restrict__
 }
 
 // --------------------------------------------------------------------------- backward
-// grad_input must be zero on entry (the host wrapper clears it on the same stream).
+// grad_input must be zero on entry (the host wrapper clears it on the same stream).  It is a sum of reds, whose order, and with it the last
+// bits, may change from call to call; the other two gradients repeat bit for bit.
 template <typename T, bool POINT, int V, int LG>
 __global__ void __launch_bounds__(BA_WARPS * 32)
 bilinear_attention_bwd_kernel(const T* __restrict__ grad_out, const T* __restrict__ input, const T* __restrict__ grid,
@@ -262,9 +263,8 @@ bilinear_attention_bwd_kernel(const T* __restrict__ grad_out, const T* __restric
     constexpr bool VEC = V == Vec<T>::N;
     const int lane = threadIdx.x & 31, gl = lane % LG, sub = lane / LG;
     const long long n_inst = (long long)B * G;
-    const int warps = (int)(blockDim.x >> 5);
-    for (long long first = ((long long)blockIdx.x * warps + (threadIdx.x >> 5)) * PW; first < n_inst;
-         first += (long long)gridDim.x * warps * PW) {
+    for (long long first = ((long long)blockIdx.x * BA_WARPS + (threadIdx.x >> 5)) * PW; first < n_inst;
+         first += (long long)gridDim.x * BA_WARPS * PW) {
         const bool own = first + sub < n_inst;           // a group past the end goes along for the shuffles
         const long long inst = own ? first + sub : first;
         const int Hb = own ? H : 0;                      // and touches no pixel
@@ -423,11 +423,9 @@ extern "C" int vtp_bilinear_attention_backward(const void* grad_out, const void*
     const BaLayout lay = mode == 0 ? ba_layout(dtype, C, grid, {input, grad_input, grad_out})
                                    : ba_layout(dtype, C, grid, {input, grad_input, weight, grad_weight});
     const int blocks = ba_grid((long long)B * G, 32 / lay.lanes);
-    // What one block could hold is worked off by one warp: its reds arrive in one order, and the smallest gradients repeat bit for bit.
-    const int warps = (long long)B * G <= BA_WARPS * (32 / lay.lanes) ? 1 : BA_WARPS;
 #define VTP_BA_BWD(T, V, LG)                                                                                 \
     (mode == 0 ? bilinear_attention_bwd_kernel<T, true, V, LG> : bilinear_attention_bwd_kernel<T, false, V, LG>) \
-        <<<blocks, warps * 32, 0, st>>>((const T*)grad_out, (const T*)input, (const T*)grid, (const T*)weight, \
+        <<<blocks, BA_WARPS * 32, 0, st>>>((const T*)grad_out, (const T*)input, (const T*)grid, (const T*)weight, \
                                            (T*)grad_input, (T*)grad_grid, (T*)grad_weight, B, H, W, C, G, P)
     if (dtype == VTP_F32) VTP_BA_DISPATCH(float, 4, VTP_BA_BWD);
     else VTP_BA_DISPATCH(bf16, 8, VTP_BA_BWD);
