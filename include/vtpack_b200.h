@@ -388,7 +388,7 @@ typedef struct {
                          vtpack/models/dge/deit_dge.py:52-53); 0 selects head_dim^-0.5 */
 } vtp_dge_shape;
 
-/* Scratch bytes vtp_dge_block_forward needs for this shape (16-byte aligned slices). */
+/* Scratch bytes vtp_dge_block_forward needs for this shape, in a workspace on any 16-byte boundary. */
 long long vtp_block_workspace_bytes(const vtp_dge_shape* s);
 
 /*

@@ -157,6 +157,48 @@ def test_attention_fp32_on_terms(n_grid, heads, special):
             assert rel_err(out, ref) < 2e-6
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("what", ["block", "dense block", "pvt stage", "model"])
+def test_workspace_on_any_16_byte_boundary(what, dtype, monkeypatch):
+    """A workspace has to lie on a 16-byte boundary and be as long as the library says: one that begins 16 bytes behind a 32-byte
+    boundary gives the same bits, nothing is refused and nothing is written around it."""
+    from vtpack_b200 import _lib
+    from vtpack_b200.models.dge import deit_dge, pvt_dge
+    torch.manual_seed(5)
+    if what == "model":
+        net = deit_dge.VisionTransformer(img_size=256, patch_size=16, embed_dim=128, depth=2, num_heads=2, mlp_ratio=2, qkv_bias=True,
+                                         num_classes=16, split_sizes=[4, 2, 1])
+        args = (torch.randn(2, 3, 256, 256),)
+    elif what == "pvt stage":
+        net = pvt_dge.Block(128, 2, mlp_ratio=2, qkv_bias=True, sr_ratio=2, split_sizes=[4, 2, 1])
+        args = (torch.randn(2, 32 * 32, 128), 32, 32)                         # 256 keys
+    else:
+        net = deit_dge.Block(128, 2, mlp_ratio=2, qkv_bias=True, split_sizes=[4, 2, 1])
+        args = (torch.randn(2, 257, 128),)
+    net = net.to(DEV, dtype).eval()
+    args = tuple(a.to(DEV, dtype) if torch.is_tensor(a) else a for a in args)
+    kwargs = {"dense": True} if what == "dense block" else {}
+    with torch.no_grad():
+        want = net(*args, **kwargs)
+    taken = []
+
+    def shifted(device, nbytes, use="block"):
+        buf = torch.full((nbytes + 64 + 32,), 0xA5, dtype=torch.uint8, device=device)
+        at = (16 - buf.data_ptr()) % 32
+        taken.append((buf, at, nbytes))
+        return buf[at:at + nbytes]
+
+    for module in (deit_dge, pvt_dge):
+        monkeypatch.setattr(module, "scratch", shifted)
+    with torch.no_grad():
+        got = net(*args, **kwargs)
+    assert _lib.device_status() == 0
+    assert taken and torch.equal(got, want)
+    for buf, at, nbytes in taken:
+        assert (buf.data_ptr() + at) % 32 == 16
+        assert bool((buf[:at] == 0xA5).all()) and bool((buf[at + nbytes:] == 0xA5).all())
+
+
 @pytest.mark.parametrize("B", [33, 256, 257])
 def test_block_fp32_items_of_runs_of_images(B):
     """The items of the fp32 attention are listed in three ways, for up to 32, up to 256 and more images: an image's bits are those

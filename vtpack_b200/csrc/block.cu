@@ -16,10 +16,15 @@ int token_im2col(const void* x, int dtype, int B, int H, int W, int C, int sr, v
 int patch_im2col(const void* images, int image_dtype, int B, int S, int P, int dtype, void* cols, int ld,
                  const void* cls_token, const void* pos_embed, int C, void* x, int32_t* counts, cudaStream_t st);   // patch_embed.cu
 
+// Slices of a workspace, on 32-byte boundaries (the fp32 attention stores 32 bytes at a time): a workspace only has to lie on a
+// 16-byte one, and the 16 bytes that may be skipped for it are counted in its size.
 struct Carver {
     char* base;
     long long off = 0;
-    explicit Carver(void* p) : base(static_cast<char*>(p)) {}
+    explicit Carver(void* p) : base(static_cast<char*>(p)) {
+        if (reinterpret_cast<uintptr_t>(p) % 32 == 16) base += 16;
+    }
+    long long bytes() const { return off + 16; }
     void* take(long long bytes) {
         void* r = base ? base + off : nullptr;
         off += round_up(bytes, 256);
@@ -110,7 +115,7 @@ static BlockScratch carve_block(const vtp_dge_shape& s, void* ws) {
         b.fc2_wt = c.take(ch);
         if (s.sr_ratio > 1) b.sr_wt = c.take(cc * s.sr_ratio * s.sr_ratio);
     }
-    b.bytes = c.off;
+    b.bytes = c.bytes();
     return b;
 }
 
@@ -472,7 +477,7 @@ static ModelScratch carve_model(const vtp_dge_shape& s, const vtp_model_weights&
     r.x = c.take((long long)s.B * N * s.C * e);
     r.cls_n = c.take((long long)s.B * s.C * e);
     r.block_ws = c.take(carve_block(s, nullptr).bytes);
-    r.bytes = c.off;
+    r.bytes = c.bytes();
     return r;
 }
 
