@@ -157,6 +157,34 @@ def test_attention_fp32_on_terms(n_grid, heads, special):
             assert rel_err(out, ref) < 2e-6
 
 
+def _block_us(blk, x, gate, n):
+    best = float("inf")
+    e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+    with torch.no_grad():
+        blk(x, forced_gate=gate)
+        for _ in range(4):
+            e[0].record()
+            for _ in range(n):
+                blk(x, forced_gate=gate)
+            e[1].record()
+            torch.cuda.synchronize()
+            best = min(best, e[0].elapsed_time(e[1]) * 1e3 / n)
+    return best
+
+
+def test_block_fp32_with_a_nan_weight_takes_little_longer():
+    """One NaN in fc2's weights makes a column of every row one that is worked out again from the decoded operands: that takes two or
+    three times a finite block (by scalar loads, a row at a time: 45 times)."""
+    from vtpack_b200.models.dge.deit_dge import Block
+    torch.manual_seed(0)
+    blk = Block(384, 6, mlp_ratio=4, qkv_bias=True, split_sizes=[4, 2, 1]).to(DEV).eval()
+    x, gate = torch.randn(12, 257, 384, device=DEV), torch.randn(12, 4, 4, 3, device=DEV)
+    finite = _block_us(blk, x, gate, 20)
+    with torch.no_grad():
+        blk.mlp.fc2.weight[9, 2] = float("nan")
+    assert _block_us(blk, x, gate, 5) < 12 * finite
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("what", ["block", "dense block", "pvt stage", "model"])
 def test_workspace_on_any_16_byte_boundary(what, dtype, monkeypatch):

@@ -44,20 +44,6 @@ struct AfArgs {
     const int32_t* offsets; float scale;
 };
 
-// Eight consecutive values of a row whose terms are n apart.
-__device__ __forceinline__ void join8(const bf16* p, size_t n, float (&f)[8]) {
-    uint4 t[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) t[i] = __ldg(reinterpret_cast<const uint4*>(p + i * n));
-    const uint32_t* h = &t[0].x;
-    const uint32_t* m = &t[1].x;
-    const uint32_t* l = &t[2].x;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int s = (i & 1) * 16;
-        f[i] = join_terms((h[i >> 1] >> s) & 0xFFFFu, (m[i >> 1] >> s) & 0xFFFFu, (l[i >> 1] >> s) & 0xFFFFu);
-    }
-}
 // 32 channels from d0 on of one query row, as chains of fused multiply-adds over the decoded operands.
 __device__ __noinline__ void redo_row(const AfArgs& g, int b, int h, long long row, int d0) {
     const bf16* q = g.q + row * 3 * g.C + h * HD;

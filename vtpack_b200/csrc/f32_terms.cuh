@@ -1,4 +1,5 @@
-// fp32 rows as three bf16 terms: the form in which the fp32 Linear on tensor cores takes its operands (linear_f32_tc.cu).
+// fp32 rows as three bf16 terms: the form in which the Linears and the attention of fp32 blocks take their operands (linear_f32_terms.cu,
+// attention_f32_tc.cu).  linear_f32_tc.cu splits fp32 rows into the same terms on the way.
 //
 // 2^16 x = h + m + l with 8 significant bits each, so the three hold the 24 bits of an fp32 number.  The factor 2^16 takes the
 // last bit of the smallest fp32 number, 2^-149, to that of the smallest bf16 number, 2^-133, so that the split is exact for
@@ -37,6 +38,21 @@ __device__ __forceinline__ void split_terms(float v, uint32_t& h, uint32_t& m, u
 __device__ __forceinline__ float join_terms(uint32_t h, uint32_t m, uint32_t l) {      // bf16 bits in the lower halves
     if ((h & 0x7F80u) == 0x7F80u) return __uint_as_float(m << 16 | l);
     return (__uint_as_float(h << 16) + (__uint_as_float(m << 16) + __uint_as_float(l << 16))) * (1.f / F_SCALE);
+}
+
+// Eight consecutive values of a row whose terms are n apart.
+__device__ __forceinline__ void join8(const bf16* p, size_t n, float (&f)[8]) {
+    uint4 t[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) t[i] = __ldg(reinterpret_cast<const uint4*>(p + i * n));
+    const uint32_t* h = &t[0].x;
+    const uint32_t* m = &t[1].x;
+    const uint32_t* l = &t[2].x;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int s = (i & 1) * 16;
+        f[i] = join_terms((h[i >> 1] >> s) & 0xFFFFu, (m[i >> 1] >> s) & 0xFFFFu, (l[i >> 1] >> s) & 0xFFFFu);
+    }
 }
 
 // Four consecutive values, the h terms to `row` on, terms n apart.

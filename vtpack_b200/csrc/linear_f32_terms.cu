@@ -117,39 +117,17 @@ struct FtSlots {
     }
 };
 
-__device__ __forceinline__ float term_at(const bf16* row, int K, int k) {
-    const unsigned short* t = reinterpret_cast<const unsigned short*>(row) + k;
-    return join_terms(__ldg(t), __ldg(t + K), __ldg(t + 2 * (size_t)K));
-}
-// acc: NC columns n0.. of row m0 + lane, sums of scaled products, which are scaled back.  Rows with a sum that is not finite are
-// worked out again as an fmaf chain, a row at a time, a lane per column (see linear_f32_tc.cu).
+// acc: NC columns of row m0 + lane, sums of scaled products, which are scaled back.  Returns the rows of the warp that have a sum that is
+// not finite: those are not stored, redo_rows works them out again.
 template <int NC>
-__device__ __forceinline__ void unscale_or_redo(float (&acc)[NC], const FtProblem& g, int K, int M, int m0, int n0, int lane) {
+__device__ __forceinline__ unsigned unscale(float (&acc)[NC], int M, int m0, int lane) {
     float t = 0.f;
 #pragma unroll
     for (int i = 0; i < NC; ++i) {
         t = fmaf(acc[i], 0.f, t);              // inf * 0 and NaN * 0 are NaN
         acc[i] *= F_UNSCALE;
     }
-    unsigned bad = __ballot_sync(0xffffffffu, t != t && m0 + lane < M);
-    while (bad) {
-        const int r = __ffs(bad) - 1;
-        bad &= bad - 1;
-        const bf16* a = g.a + (size_t)(m0 + r) * 3 * K;
-        static_assert(NC <= 32, "a lane per column");
-        const int n = n0 + lane;
-        float s = 0.f;
-        if (lane < NC && n < g.N) {
-            const bf16* w = g.w + (size_t)n * 3 * K;
-#pragma unroll 1
-            for (int k = 0; k < K; ++k) s = fmaf(term_at(a, K, k), term_at(w, K, k), s);
-        }
-#pragma unroll
-        for (int i = 0; i < NC; ++i) {
-            const float v = __shfl_sync(0xffffffffu, s, i);
-            if (lane == r) acc[i] = v;
-        }
-    }
+    return __ballot_sync(0xffffffffu, t != t && m0 + lane < M);
 }
 
 // What the outputs are: + res, as fp32; as terms; GELU, as terms.
@@ -167,6 +145,45 @@ __device__ __forceinline__ void finish4(const FtProblem& g, int m, int n, const 
     } else {
         if (g.res) { v[0] += res.x; v[1] += res.y; v[2] += res.z; v[3] += res.w; }
         *reinterpret_cast<float4*>(g.y + (size_t)m * g.ldy + n) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+}
+
+// Columns n0 .. n0 + cols - 1 of rows m0 + lane, those of `bad`, as fmaf chains over the decoded operands (see linear_f32_tc.cu).  Sixteen
+// columns at a time, all rows of the warp at once: an operand that is not finite is a column of the weights or a row of the batch in
+// front, and then most rows are bad.  A lane decodes its own row and column lane % 16, the columns go round by shuffles.  (A DeiT-S
+// block, 12 images, us: all finite 98, a NaN among the weights of fc2 330; a row at a time, a lane per column, by scalar loads 4500;
+// fp32 rows in linear_f32_tc.cu 1700.)
+template <int OUT>
+__device__ __noinline__ void redo_rows(const FtProblem& g, int K, int M, int m0, int n0, int cols, unsigned bad, int lane) {
+    constexpr int CH = 16;
+    const int m = min(m0 + lane, M - 1);
+    const bf16* a = g.a + (size_t)m * 3 * K;
+#pragma unroll 1
+    for (int c0 = 0; c0 < cols; c0 += CH) {
+        const bf16* w = g.w + (size_t)min(n0 + c0 + (lane & (CH - 1)), g.N - 1) * 3 * K;
+        float s[CH];
+#pragma unroll
+        for (int c = 0; c < CH; ++c) s[c] = 0.f;
+#pragma unroll 1
+        for (int k = 0; k < K; k += 8) {
+            float x[8], y[8];
+            join8(a + k, (size_t)K, x);
+            join8(w + k, (size_t)K, y);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int c = 0; c < CH; ++c) s[c] = fmaf(x[i], __shfl_sync(0xffffffffu, y[i], c), s[c]);
+        }
+        if (!(bad >> lane & 1)) continue;
+#pragma unroll
+        for (int c = 0; c < CH; c += 4) {
+            const int n = n0 + c0 + c;
+            if (c0 + c >= cols || n >= g.N) continue;
+            const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+            finish4<OUT>(g, m, n, make_float4(s[c], s[c + 1], s[c + 2], s[c + 3]),
+                         g.bias ? __ldg(reinterpret_cast<const float4*>(g.bias + n)) : zero4,
+                         OUT == FT_ROWS && g.res ? *reinterpret_cast<const float4*>(g.res + (size_t)m * g.ldr + n) : zero4);
+        }
     }
 }
 
@@ -418,16 +435,17 @@ linear_f32_terms_kernel(const __grid_constant__ FtMapsOf maps, const __grid_cons
                     }
                 }
                 if (!ok) break;
-                unscale_or_redo<SC>(own, q, g.K, M, m0, n0 + rank * SC, lane);
-                if (m0 + lane < M) {
+                const unsigned bad = unscale<SC>(own, M, m0, lane);
+                if (m0 + lane < M && !(bad >> lane & 1)) {
 #pragma unroll
                     for (int v = 0; v < NV; ++v)
                         if (col_of(v) < q.N)
                             finish4<OUT>(q, m0 + lane, col_of(v), make_float4(own[4 * v], own[4 * v + 1], own[4 * v + 2], own[4 * v + 3]),
                                             bias[v], res[OUT != FT_ROWS ? 0 : v]);
                 }
+                if (bad) redo_rows<OUT>(q, g.K, M, m0, n0 + rank * SC, SC, bad, lane);
             } else if (has) {
-                unscale_or_redo<CW>(acc, q, g.K, M, m0, n0, lane);
+                const unsigned bad = unscale<CW>(acc, M, m0, lane);
                 // 16 columns at a time through the warp's transpose buffer (rows of four 16-byte chunks, XOR-swizzled): a lane
                 // then holds four columns of a row and four lanes 64 consecutive bytes
 #pragma unroll
@@ -443,7 +461,7 @@ linear_f32_terms_kernel(const __grid_constant__ FtMapsOf maps, const __grid_cons
                     auto finish = [&](int r8) {
                         const int rr = r8 * 8 + (lane >> 2);
                         const float4 v = lds_f4(stage + rr * 64 + (((lane & 3) ^ ((rr >> 1) & 3)) << 4));
-                        if (m0 + rr < M && n < q.N) finish4<OUT>(q, m0 + rr, n, v, bias[b], res[OUT != FT_ROWS ? 0 : 4 * b + r8]);
+                        if (m0 + rr < M && n < q.N && !(bad >> rr & 1)) finish4<OUT>(q, m0 + rr, n, v, bias[b], res[OUT != FT_ROWS ? 0 : 4 * b + r8]);
                     };
                     if constexpr (OUT == FT_HIDDEN) {
                         // (not unrolled: most launches run this once per warp, and then what it costs is its fetch)
@@ -454,6 +472,8 @@ linear_f32_terms_kernel(const __grid_constant__ FtMapsOf maps, const __grid_cons
                         for (int r8 = 0; r8 < 4; ++r8) finish(r8);
                     }
                 }
+                // (behind the stores, where a call has no outputs to keep)
+                if (bad) redo_rows<OUT>(q, g.K, M, m0, n0, CW, bad, lane);
             }
         }
     }
