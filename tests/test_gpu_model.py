@@ -185,6 +185,19 @@ def test_block_fp32_with_a_nan_weight_takes_little_longer():
     assert _block_us(blk, x, gate, 5) < 12 * finite
 
 
+def test_block_fp32_with_a_nan_among_the_values_takes_little_longer():
+    """A NaN in v's bias makes every row of the attention, and of the Linears behind it, one that is worked out again: 15 times a finite
+    block (41 times with every lane decoding all keys for itself)."""
+    from vtpack_b200.models.dge.deit_dge import Block
+    torch.manual_seed(0)
+    blk = Block(384, 6, mlp_ratio=4, qkv_bias=True, split_sizes=[4, 2, 1]).to(DEV).eval()
+    x, gate = torch.randn(12, 257, 384, device=DEV), torch.randn(12, 4, 4, 3, device=DEV)
+    finite = _block_us(blk, x, gate, 20)
+    with torch.no_grad():
+        blk.attn.kv.bias[384 + 5] = float("nan")
+    assert _block_us(blk, x, gate, 5) < 27 * finite
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("what", ["block", "dense block", "pvt stage", "model"])
 def test_workspace_on_any_16_byte_boundary(what, dtype, monkeypatch):

@@ -2,7 +2,7 @@
 //
 // The products are formed like those of the fp32 Linears: six bf16 products of terms, smallest first, into a fresh TMEM
 // accumulator per 64 channels (scores) or 64 keys (P V), which fp32 registers add up; the softmax is fp32 with expf.  A row with a
-// score or an output that is not finite is worked out again on its own from the decoded operands (redo_row).
+// score or an output that is not finite is worked out again from the decoded operands (redo_rows).
 //
 // Work item = 128 packed queries of one (image, head) (attention_items.cuh); persistent, one CTA per SM; keys in chunks of up to
 // 320, five blocks of 64:
@@ -44,22 +44,33 @@ struct AfArgs {
     const int32_t* offsets; float scale;
 };
 
-// 32 channels from d0 on of one query row, as chains of fused multiply-adds over the decoded operands.
-__device__ __noinline__ void redo_row(const AfArgs& g, int b, int h, long long row, int d0) {
-    const bf16* q = g.q + row * 3 * g.C + h * HD;
+// 32 channels from d0 on of a query row per lane, as chains of fused multiply-adds over the decoded operands; `put`: whether the lane
+// stores its row (the others come along, with a row that exists).  A key and its value are decoded once, two channels and
+// one a lane, and go round by shuffles.  (A DeiT-S block, 12 images, with a NaN among the biases of v, us: 1440; each lane decoding all of
+// the keys 4000; the CUDA-core attention and fp32 Linears 3200.)
+__device__ __noinline__ void redo_rows(const AfArgs& g, int b, int h, long long row, int d0, int lane, bool put) {
     const bf16* k = g.kv + (long long)b * g.n_keys * 6 * g.C + h * HD;
     const bf16* v = k + g.C + d0;
-    auto score = [&](int key) {
-        const bf16* kr = k + (long long)key * 6 * g.C;
-        float s = 0.f;
-#pragma unroll 2
-        for (int d = 0; d < HD; d += 8) {
-            float x[8], y[8];
-            join8(q + d, g.C, x);
-            join8(kr + d, 2 * g.C, y);
+    float q[HD];
+    {
+        const bf16* at = g.q + row * 3 * g.C + h * HD;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) s = fmaf(x[i], y[i], s);
+        for (int d = 0; d < HD; d += 8) {
+            float x[8];
+            join8(at + d, g.C, x);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) q[d + i] = x[i];
         }
+    }
+    auto score = [&](int key) {
+        const bf16* kr = k + (long long)key * 6 * g.C + 2 * lane;
+        uint32_t t[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) t[i] = __ldg(reinterpret_cast<const uint32_t*>(kr + (size_t)i * 2 * g.C));
+        const float y[2] = {join_terms(t[0] & 0xFFFFu, t[1] & 0xFFFFu, t[2] & 0xFFFFu), join_terms(t[0] >> 16, t[1] >> 16, t[2] >> 16)};
+        float s = 0.f;
+#pragma unroll
+        for (int d = 0; d < HD; ++d) s = fmaf(q[d], __shfl_sync(0xffffffffu, y[d & 1], d >> 1), s);
         return s * g.scale;
     };
     float m = -INFINITY, l = 0.f, o[32];
@@ -72,14 +83,12 @@ __device__ __noinline__ void redo_row(const AfArgs& g, int b, int h, long long r
     for (int key = 0; key < g.n_keys; ++key) {
         const float p = expf(score(key) - m_at);
         l += p;
+        const unsigned short* vr = reinterpret_cast<const unsigned short*>(v + (long long)key * 6 * g.C) + lane;
+        const float x = join_terms(__ldg(vr), __ldg(vr + 2 * g.C), __ldg(vr + 4 * (size_t)g.C));
 #pragma unroll
-        for (int c = 0; c < 32; c += 8) {
-            float x[8];
-            join8(v + (long long)key * 6 * g.C + c, 2 * g.C, x);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) o[c + i] = fmaf(p, x[i], o[c + i]);
-        }
+        for (int c = 0; c < 32; ++c) o[c] = fmaf(p, __shfl_sync(0xffffffffu, x, c), o[c]);
     }
+    if (!put) return;
     const float inv = 1.f / l;
     bf16* dst = reinterpret_cast<bf16*>(g.out) + row * 3 * g.C + h * HD + d0;
 #pragma unroll
@@ -415,28 +424,28 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             }
             bad += swap_row(bad);
             if (!ok) break;
-            if (r >= it.nq || it.row0 + r >= g.l_max) continue;
-            const long long row = it.row0 + r;
-            if (bad != bad) {
-                redo_row(g, it.b, it.h, row, hf * 32);
-                continue;
-            }
-            bf16* dst = reinterpret_cast<bf16*>(g.out) + row * 3 * g.C + it.h * HD + hf * 32;
+            const bool exists = r < it.nq && it.row0 + r < g.l_max, again = exists && bad != bad;
+            const long long row = it.row0 + (exists ? r : 0);
+            if (exists && !again) {
+                bf16* dst = reinterpret_cast<bf16*>(g.out) + row * 3 * g.C + it.h * HD + hf * 32;
 #pragma unroll
-            for (int e = 0; e < 32; e += 16) {
-                uint32_t w3[3][8];
+                for (int e = 0; e < 32; e += 16) {
+                    uint32_t w3[3][8];
 #pragma unroll
-                for (int x = 0; x < 16; x += 2) {
-                    uint32_t tt[3][2];
+                    for (int x = 0; x < 16; x += 2) {
+                        uint32_t tt[3][2];
 #pragma unroll
-                    for (int y = 0; y < 2; ++y) split_scaled(o[e + x + y] * F_SCALE, tt[0][y], tt[1][y], tt[2][y]);      // (below 2^96)
+                        for (int y = 0; y < 2; ++y) split_scaled(o[e + x + y] * F_SCALE, tt[0][y], tt[1][y], tt[2][y]);      // (below 2^96)
 #pragma unroll
-                    for (int q = 0; q < 3; ++q) w3[q][x >> 1] = __byte_perm(tt[q][0], tt[q][1], 0x7632);
+                        for (int q = 0; q < 3; ++q) w3[q][x >> 1] = __byte_perm(tt[q][0], tt[q][1], 0x7632);
+                    }
+                    // (32 bytes a store: each touches a line per lane, which is what a store costs here)
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) stg_u8(dst + (size_t)q * g.C + e, w3[q]);
                 }
-                // (32 bytes a store: each touches a line per lane, which is what a store costs here)
-#pragma unroll
-                for (int q = 0; q < 3; ++q) stg_u8(dst + (size_t)q * g.C + e, w3[q]);
             }
+            // (behind the stores, where a call has no outputs to keep)
+            if (__any_sync(0xffffffffu, again)) redo_rows(g, it.b, it.h, row, hf * 32, lane, again);
         }
     }
     if (*abort_flag) {
