@@ -803,10 +803,11 @@ def test_image_gives_the_same_bits_in_any_batch(kind, dtype):
         assert all(torch.equal(a, b[:n]) for a, b in zip(m.last_counts, counts))
 
 
-@pytest.mark.parametrize("C,B,fine", [(192, 9, 0.0), (192, 16, 0.5), (192, 20, 1.0), (384, 4, 0.0), (384, 9, 1.0), (768, 2, 0.5), (768, 4, 1.0)])
+@pytest.mark.parametrize("C,B,fine", [(192, 9, 0.0), (192, 15, 1.0), (192, 16, 0.5), (192, 20, 1.0), (384, 4, 0.0), (384, 8, 1.0),
+                                      (384, 9, 1.0), (768, 2, 0.5), (768, 3, 1.0), (768, 4, 1.0)])
 def test_q_and_kv_in_one_launch_same_bits_for_an_image(C, B, fine):
-    """q and kv of a block in 128 x 64 tiles (an image alone), 128 x 128 tiles (as many as SMs; 192 q columns fill one and a half) and the
-    persistent kernel's, with few and with all rows that the host allows for."""
+    """q and kv of a block in 128 x 64 tiles (an image alone), 128 x 128 tiles (as many as SMs, or some more where all rows exist: 15 and 16, 8,
+    4 images; 192 q columns fill one and a half) and the persistent kernel's, with few and with all rows that the host allows for."""
     from vtpack_b200 import _lib
     torch.manual_seed(C + B)
     sd = O.round_bf16(O.make_state_dict(C, 1, C // 64, seed=B))

@@ -610,9 +610,9 @@ linear_tc_kernel(const __grid_constant__ TcLaunch L, int K, int* status) {
 }
 
 // ------------------------------------------------------------------------------ small problems
-// The same products for problems of no more 128 x 64 or 128 x 128 tiles than SMs, where a launch is a chain of latencies: one tile per CTA,
-// which tile it is known before the wait for the kernel in front (the loads do not wait for the row count, only the stores
-// do), sixteen epilogue warps with 16 columns of each 64 that go straight between registers and global memory.  Same MMA steps and
+// The same products for problems of no more 128 x 64 tiles than SMs, or 128 x 128 tiles (linear_tcgen05_pair), where a launch is a chain of
+// latencies: one tile per CTA, which tile it is known before the wait for the kernel in front (the loads do not wait for the row
+// count, only the stores do), sixteen epilogue warps with 16 columns of each 64 that go straight between registers and global memory.  Same MMA steps and
 // sums in the same order as linear_tc_kernel: a row's bits do not depend on which of the two it comes from.
 template <int BN_>
 struct SmallConf {
@@ -1016,12 +1016,19 @@ static int launch_tc(const LinearArgs& p, const LinearArgs* p1, cudaStream_t st)
 // sides of the line, us, small / persistent kernel:  1536, K = 384, GELU: 96 tiles 4.6 / 6.2, 144 4.7 / 6.8, 216 8.5 / 7.0, 288
 // 8.9 / 7.3;  384, K = 1536, residual: 108 tiles 7.8 / 8.9, 144 7.8 / 9.5, 222 14.7 / 11.5;  768, K = 192, GELU: 108 tiles 3.9 / 4.7,
 // 144 4.1 / 4.8, 216 7.4 / 5.4.)
-// Two problems in one launch also run that way as 128 x 128 tiles, if those are no more than SMs (q and kv of DeiT-S, 7 images: 7.0 -> 5.8
-// us; forwards, of the same tree but for this: DeiT-S 7 images 562 / 550; DeiT-S 9, DeiT-Ti 16 and DeiT-B 4 images are the last batches that
-// fit).  One problem gains nothing by them: 1536, K = 384, 539 of 1799 rows 6.6 / 6.5, all of them 11.4 / 8.4.
+// Two problems in one launch also run that way as 128 x 128 tiles, if those of all of one's rows and of seven tenths of the rows that
+// the other's count on the device allows are no more than SMs (q and kv of DeiT-S, 7 images: 7.0 -> 5.8 us).  Blocks, us, at a fifth /
+// half / three quarters / all of the regions on the finest grain, this way and by the persistent kernel: DeiT-S, 7 images 43.2 43.7 44.4
+// 45.5 and 44.0 44.5 45.0 47.4; 8 images 42.4 43.5 46.1 49.4 and 44.8 45.2 48.0 48.3; DeiT-Ti, 16 images 37.3 37.9 41.1 43.4 and 38.0
+// 39.9 42.4 41.3; DeiT-B, 4 images 54.2 55.2 60.5 62.9 and 56.1 58.4 61.9 61.9; PVT stage 3, 18 images 53.7 55.8 57.9 61.7 and 54.7 57.1
+// 59.9 60.2.  Up to here it gains more than it loses: with all regions on the finest grain the tiles are some more than SMs,
+// and each of those waits until one is free.  Beyond the line that costs more than the rest gains: DeiT-S, 9 images 43.2 45.0 51.1
+// 52.0 and 43.8 46.2 48.5 49.7; PVT stage 3, 25 images 58.0 61.2 66.3 67.3 and 58.9 61.9 64.8 65.6.
+// Where the queries are most of the rows and have no more columns than a tile (PVT stage 1, 8 images 63.2 65.9 73.9 74.7 and 62.1
+// 66.0 72.0 72.6) it gains nothing.  One problem gains nothing either: 1536, K = 384, 539 of 1799 rows 6.6 / 6.5, all of them 11.4 / 8.4.
 static long long small_tiles(const LinearArgs& p, int bn, bool likely = false) {
-    // (with a device-side row count the worst case is about three times the packed rows of a DGE block)
-    return (long long)ceil_div(likely && p.m_dev ? ceil_div(p.m_max, 2) : p.m_max, TBM) * ceil_div(p.N, bn);
+    const int rows = likely && p.m_dev ? (int)((7ll * p.m_max + 9) / 10) : p.m_max;
+    return (long long)ceil_div(rows, TBM) * ceil_div(p.N, bn);
 }
 
 template <int BN, int EPI, bool F32, int NPROB>
@@ -1083,10 +1090,12 @@ int linear_tcgen05_pair(const LinearArgs& a, const LinearArgs& b, cudaStream_t s
     if (int rc = check_tc_args(b)) return rc;
     VTP_REQUIRE(linear_pair_supported(a, b), VTP_ERR_UNSUPPORTED, "linear (tcgen05): these two problems cannot share a launch");
     if (small_tiles(a, 64) + small_tiles(b, 64) <= sm_count()) return launch_small<64, EPI_LN, false, 2>(a, &b, st);
-    if (small_tiles(a, 128, true) + small_tiles(b, 128, true) <= sm_count()) return launch_small<128, EPI_LN, false, 2>(a, &b, st);
+    const bool narrow = pick_bn((a.m_max > b.m_max ? a : b).N) == 128;
+    if ((!narrow || a.m_max == b.m_max) && small_tiles(a, 128, true) + small_tiles(b, 128, true) <= sm_count())
+        return launch_small<128, EPI_LN, false, 2>(a, &b, st);
     // (narrow tiles where most of the work, the problem of more rows, has no more than 128 columns: the queries of PVT's first two stages,
     // whose keys are few; PVT-tiny, 96 images, 1470 us)
-    if (pick_bn((a.m_max > b.m_max ? a : b).N) == 128) return launch_tc<128, 1, EPI_LN, false, 2>(a, &b, st);
+    if (narrow) return launch_tc<128, 1, EPI_LN, false, 2>(a, &b, st);
     if (pairs_pay(256, a.K)) return launch_tc<256, 2, EPI_LN, false, 2>(a, &b, st);
     return launch_tc<256, 1, EPI_LN, false, 2>(a, &b, st);
 }
