@@ -105,3 +105,13 @@ def test_lanes_that_wait_together_go_on_together(kernel):
         # (the warps that split fp32 operands have only __syncwarp behind it, which a lane that leaves still runs as often)
         runs_out = "num_kb - kb; n > 0; --n) __syncwarp();" in text[at:at + 400]
         assert name in (("wait", "wait_a") if one or runs_out else ("wait_warp", "wait_cluster_warp")), (name, text[at:at + 80])
+
+
+def test_shared_memory_is_reserved_for_the_largest_launch():
+    """A kernel's limit of shared memory is set once per device.  Set to what a launch takes that depends on the call, a thread could
+    lower what another has just raised for a larger batch and is about to launch with."""
+    for name in ("attention_tc.cu", "attention_f32_tc.cu"):
+        sizes = re.findall(r"cudaFuncSetAttribute\(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (\w+)\)", source(name))
+        assert sizes, name
+        for size in sizes:
+            assert re.search(r"constexpr int [^;]*\b%s = " % size, source(name)), (name, size)

@@ -36,7 +36,8 @@ constexpr int AF_SM_ITEM = AF_SM_BAR + 256;              // two items
 constexpr int AF_SM_ROW = AF_SM_ITEM + 64;               // float [2][2 halves][128 rows], exchanged between the two threads of a row
 constexpr int AF_SM_PREFIX = AF_SM_ROW + 2048;           // int32 [B + 1] tile prefix, [B + 1] offsets
 constexpr int AF_MOST_IMAGES = 4000;
-static_assert(AF_SM_PREFIX + 2 * (AF_MOST_IMAGES + 1) * 4 + 1024 <= 232448, "shared memory budget");
+constexpr int AF_SM_MOST = AF_SM_PREFIX + 2 * (AF_MOST_IMAGES + 1) * 4 + 1024;
+static_assert(AF_SM_MOST <= 232448, "shared memory budget");
 
 struct AfArgs {
     const bf16* q; const bf16* kv; float* out;           // q [l_max][3][C], kv [B n_keys][3][2 C], out [l_max][3][C] terms
@@ -503,17 +504,17 @@ int attention_f32_terms(const AttnArgs& p, cudaStream_t st) {
     // (batches of up to 32 images have a kernel of their own, whose code a small launch is through sooner: FewImages)
     const bool one_each = p.B <= 32;
     auto kern = one_each ? attn_f32_tc_kernel<1> : attn_f32_tc_kernel<FEW_PER>;
-    static int reserved[2][64] = {};
-    int* attr_smem = reserved[one_each];
+    // (what the largest launch takes, whatever this one does: two threads may get here with different batches)
+    static bool reserved[2][64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64 || attr_smem[dev] < smem) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (dev < 0 || dev >= 64 || !reserved[one_each][dev]) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AF_SM_MOST);
         if (e != cudaSuccess) {
-            set_error("attention (fp32 terms): cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
+            set_error("attention (fp32 terms): cannot reserve %d bytes of shared memory: %s", AF_SM_MOST, cudaGetErrorString(e));
             return (int)e;
         }
-        if (dev >= 0 && dev < 64) attr_smem[dev] = smem;
+        if (dev >= 0 && dev < 64) reserved[one_each][dev] = true;
     }
     const long long worst = (long long)p.B * ceil_div(p.max_q, QT) * p.heads;
     const int grid = (int)(worst < sm_count() ? worst : sm_count());

@@ -462,13 +462,15 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     if (warp == 0) tmem_dealloc(tmem_base, ATT_TMEM_COLS);
 }
 
-int attention_tcgen05_max_images() { return 16384; }
+constexpr int MOST_IMAGES = 16384, SM_MOST = SM_PREFIX + (MOST_IMAGES + 1) * 4 + 1024;
+static_assert(SM_MOST <= 232448, "shared memory budget");
+int attention_tcgen05_max_images() { return MOST_IMAGES; }
 
 int attention_tcgen05(const AttnArgs& p, cudaStream_t st) {
     VTP_REQUIRE(p.dtype == VTP_BF16, VTP_ERR_DTYPE, "attention (tcgen05): bf16 only");
     VTP_REQUIRE(p.head_dim == HD, VTP_ERR_UNSUPPORTED, "attention (tcgen05): head_dim %d (only %d)", p.head_dim, HD);
     VTP_REQUIRE(p.n_keys >= 16, VTP_ERR_UNSUPPORTED, "attention (tcgen05): needs at least 16 keys, got %d", p.n_keys);
-    VTP_REQUIRE(p.B <= 16384, VTP_ERR_SHAPE, "attention (tcgen05): %d images (at most 16384)", p.B);
+    VTP_REQUIRE(p.B <= MOST_IMAGES, VTP_ERR_SHAPE, "attention (tcgen05): %d images (at most %d)", p.B, MOST_IMAGES);
     VTP_REQUIRE(p.q_rs % 8 == 0 && p.q_hs % 8 == 0 && p.kv_rs % 8 == 0 && p.kv_hs % 8 == 0 && p.kv_bs % 8 == 0 &&
                     p.o_rs % 8 == 0 && p.o_hs % 8 == 0,
                 VTP_ERR_ALIGN, "attention (tcgen05): strides must be multiples of 16 bytes");
@@ -497,17 +499,17 @@ int attention_tcgen05(const AttnArgs& p, cudaStream_t st) {
     // (batches of up to 32 images have a kernel of their own, whose code a small launch is through sooner: FewImages)
     const bool one_each = p.B <= 32;
     auto kern = one_each ? attn_tc_kernel<1> : attn_tc_kernel<FEW_PER>;
-    static int reserved[2][64] = {};
-    int* attr_smem = reserved[one_each];
+    // (what the largest launch takes, whatever this one does: two threads may get here with different batches)
+    static bool reserved[2][64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64 || attr_smem[dev] < smem) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (dev < 0 || dev >= 64 || !reserved[one_each][dev]) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_MOST);
         if (e != cudaSuccess) {
-            set_error("attention (tcgen05): cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
+            set_error("attention (tcgen05): cannot reserve %d bytes of shared memory: %s", SM_MOST, cudaGetErrorString(e));
             return (int)e;
         }
-        if (dev >= 0 && dev < 64) attr_smem[dev] = smem;
+        if (dev >= 0 && dev < 64) reserved[one_each][dev] = true;
     }
     const long long worst = (long long)p.B * ceil_div(p.max_q, QT) * p.heads;
     const int grid = (int)(worst < 2ll * sm_count() ? worst : 2ll * sm_count());
