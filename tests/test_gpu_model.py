@@ -257,6 +257,65 @@ def test_block_fp32_items_of_runs_of_images(B):
     assert torch.equal(whole, parts)
 
 
+def test_block_fp32_more_images_than_one_attention_launch_takes():
+    """The fp32 attention on tensor cores lists the items of up to 4000 images in a launch: images on both sides of that number have the
+    bits they have in a batch of their own."""
+    from vtpack_b200 import _lib
+    from vtpack_b200.models.dge.deit_dge import Block
+    torch.manual_seed(1)
+    blk = Block(64, 1, mlp_ratio=1.0, qkv_bias=True, split_sizes=[4, 2, 1]).to(DEV).eval()
+    B = 4007
+    x = torch.randn(B, 145, 64, device=DEV)
+    gate = torch.eye(3)[torch.randint(0, 3, (B, 3, 3))]
+    with torch.no_grad():
+        whole = blk(x, forced_gate=gate)
+        for i in (0, 2000, 3992, 4000):
+            n = min(8, B - i)
+            assert torch.equal(blk(x[i:i + n].contiguous(), forced_gate=gate[i:i + n]), whole[i:i + n]), i
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("B", [1, 12])
+@pytest.mark.parametrize("forced", [False, True])
+@pytest.mark.parametrize("C,sr", [(128, 1), (384, 1), (128, 2)])
+def test_block_fp32_weights_written_directly_in_front(C, sr, forced, B):
+    """The matrices of an fp32 block are split by CTAs that do not wait for the kernel in front of theirs: a call that follows the kernels
+    which write its parameters, without anything between them, uses what they wrote."""
+    from vtpack_b200 import _lib
+    from vtpack_b200.models.dge import deit_dge, pvt_dge
+    torch.manual_seed(C + B)
+    if sr == 1:
+        blk, n, args = deit_dge.Block(C, C // 64, mlp_ratio=4, qkv_bias=True, split_sizes=[4, 2, 1]), 257, ()
+    else:
+        blk, n, args = pvt_dge.Block(C, C // 64, mlp_ratio=4, qkv_bias=True, sr_ratio=sr, split_sizes=[4, 2, 1]), 256, (16, 16)
+    blk = blk.to(DEV).eval()
+    params = [p for p in blk.parameters() if p.is_floating_point()]
+    x = torch.randn(B, n, C, device=DEV)
+    kw = {"forced_gate": torch.randn(B, 4, 4, 3, device=DEV)} if forced else {}
+    sets = [[torch.randn_like(p) * 0.05 for p in params] for _ in range(3)]
+    outs, want = [], []
+    with torch.no_grad():
+        for s in sets:
+            for p, v in zip(params, s):
+                p.copy_(v)
+            torch.cuda.synchronize()
+            want.append(blk(x, *args, **kw))
+            torch.cuda.synchronize()
+        for i in range(120):
+            if i % 2:
+                torch._foreach_copy_(params, sets[i % 3])
+            else:                                             # one kernel a parameter, another one last each time
+                k = i // 2 % len(params)
+                for p, v in list(zip(params, sets[i % 3]))[k + 1:] + list(zip(params, sets[i % 3]))[:k + 1]:
+                    p.copy_(v)
+            outs.append(blk(x, *args, **kw))
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
+    assert not torch.equal(want[0], want[1])
+    for i, out in enumerate(outs):
+        assert torch.equal(out, want[i % 3]), i
+
+
 def test_layer_512px_skewed_fp32():
     """32x32 grid (N=1025, 64 regions); even images all-coarse, odd all-fine."""
     sd = O.make_state_dict(128, 1, 2, img_size=512, seed=10)
