@@ -457,7 +457,10 @@ pool_region_kernel(const T* __restrict__ x, RegionGeom g, const int32_t* __restr
 // for the kernel in front: that is always one of the same call (the gate, or the unpool of the block before), which let this one start
 // only once everything before itself had completed, whatever wrote the parameters and the Linears that read the last
 // block's terms among it.  So the split runs beside the end of that kernel (behind the pool's CTAs, in a kernel that
-// started late: DeiT-S, 12 images, 17.3 us a block instead of 16.0).
+// started late: DeiT-S, 12 images, 17.3 us a block instead of 16.0).  It starts early whatever its grid: early / late, us a block, DeiT-S, 12
+// images 98.2 / 99.4, 128 images 503.8 / 504.3, DeiT-B, 40 images 650.1 / 650.6, DeiT-Ti, 200 images 341.2 / 340.5.
+// The split is most of what few images move, and still less than splitting in every Linear took (terms / fp32 rows): DeiT-B, 1
+// image, pool 24.6 / 21.9 us by itself and the block 104 / 131, 2 images 30.8 / 22.5 and 148 / 199.
 template <int G, int CPL>
 __global__ void __launch_bounds__((Lay<float, G, CPL>::THREADS), (pool_ctas<float, G, CPL>()))
 pool_region_terms_kernel(const float* __restrict__ x, RegionGeom g, const int32_t* __restrict__ idx,
