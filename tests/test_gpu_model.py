@@ -186,7 +186,7 @@ def test_block_fp32_with_a_nan_weight_takes_little_longer():
 
 
 def test_block_fp32_with_a_nan_among_the_values_takes_little_longer():
-    """A NaN in v's bias makes every row of the attention, and of the Linears behind it, one that is worked out again: 15 times a finite
+    """A NaN in v's bias makes every row of the attention, and of the Linears behind it, one that is worked out again: 14 times a finite
     block (41 times with every lane decoding all keys for itself)."""
     from vtpack_b200.models.dge.deit_dge import Block
     torch.manual_seed(0)

@@ -47,7 +47,7 @@ struct AfArgs {
 
 // 32 channels from d0 on of a query row per lane, as chains of fused multiply-adds over the decoded operands; `put`: whether the lane
 // stores its row (the others come along, with a row that exists).  A key and its value are decoded once, two channels and
-// one a lane, and go round by shuffles.  (A DeiT-S block, 12 images, with a NaN among the biases of v, us: 1440; each lane decoding all of
+// one a lane, and go round by shuffles.  (A DeiT-S block, 12 images, with a NaN among the biases of v, us: 1360; each lane decoding all of
 // the keys 4000; the CUDA-core attention and fp32 Linears 3200.)
 __device__ __noinline__ void redo_rows(const AfArgs& g, int b, int h, long long row, int d0, int lane, bool put) {
     const bf16* k = g.kv + (long long)b * g.n_keys * 6 * g.C + h * HD;

@@ -151,10 +151,10 @@ __device__ __forceinline__ void finish4(const FtProblem& g, int m, int n, const 
 // Columns n0 .. n0 + cols - 1 of rows m0 + lane, those of `bad`, as fmaf chains over the decoded operands (see linear_f32_tc.cu).  Sixteen
 // columns at a time, all rows of the warp at once: an operand that is not finite is a column of the weights or a row of the batch in
 // front, and then most rows are bad.  A lane decodes its own row and column lane % 16, the columns go round by shuffles.  (A DeiT-S
-// block, 12 images, us: all finite 98, a NaN among the weights of fc2 330; a row at a time, a lane per column, by scalar loads 4500;
-// fp32 rows in linear_f32_tc.cu 1700.)
+// block, 12 images, us: all finite 98, a NaN among the weights of fc2 228; a row at a time, a lane per column, by scalar loads 4500;
+// fp32 rows in linear_f32_tc.cu 1700.  Inlined: as a function of its own it cost DeiT-S, 12 images, 11 of 1217 us where all is finite.)
 template <int OUT>
-__device__ __noinline__ void redo_rows(const FtProblem& g, int K, int M, int m0, int n0, int cols, unsigned bad, int lane) {
+__device__ __forceinline__ void redo_rows(const FtProblem& g, int K, int M, int m0, int n0, int cols, unsigned bad, int lane) {
     constexpr int CH = 16;
     const int m = min(m0 + lane, M - 1);
     const bf16* a = g.a + (size_t)m * 3 * K;
@@ -472,7 +472,7 @@ linear_f32_terms_kernel(const __grid_constant__ FtMapsOf maps, const __grid_cons
                         for (int r8 = 0; r8 < 4; ++r8) finish(r8);
                     }
                 }
-                // (behind the stores, where a call has no outputs to keep)
+                // (behind the stores, where there are no outputs to keep beside it)
                 if (bad) redo_rows<OUT>(q, g.K, M, m0, n0, CW, bad, lane);
             }
         }
