@@ -362,16 +362,19 @@ def model_roofline(model, batch, counts, ms_per_step, pk, image_bytes, fine):
                     "unpool bytes are what the kernel moves (fine regions read neither ref nor comp)"}
 
 
-def launches_per_forward(model):
-    """Kernels of this library in one forward: im2col (which writes the cls rows and starts the counts), patch-embed
+def launches_per_forward(model, images):
+    """Kernels of this library in one forward.  In bf16: im2col (which writes the cls rows and starts the counts), patch-embed
     Linear, first gate, final LayerNorm and head; per block pool, q + kv, attention, proj, fc1, fc2 and unpool (which
-    leaves the next block's gate decisions).  q and kv share one launch when both widths are whole 64-column slabs;
-    fp32 blocks launch them apart, and the LayerNorm in front of fc1 too."""
+    leaves the next block's gate decisions).  q and kv share one launch when both widths are whole 64-column slabs.
+    Other forwards are counted by the profiler: whether fp32 blocks launch q and kv together depends on the batch."""
     depth = len(model.blocks)
     if model.compute_dtype() == torch.bfloat16 and not model.flags:
         C = model.embed_dim
         return 5 + (7 if C >= 64 and C % 64 == 0 else 8) * depth
-    return 5 + 9 * depth
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        model._forward_eval(images, None, use_plans=False)
+        torch.cuda.synchronize()
+    return sum(e.count for e in prof.key_averages() if "vtp::" in e.key)
 
 
 def profile_case(which):
@@ -974,7 +977,7 @@ def main():
                     "h2d_copy_alone_gbs_per_gpu": round(h2d_gbs, 1),
                     "h2d_note": "pinned-host-to-device copy of one step's images with nothing else running, all "
                                 "ranks at once, max over ranks"},
-            "gpu_launches": args.steps * launches_per_forward(model),
+            "gpu_launches": args.steps * launches_per_forward(model, img_dev),
             "clocks": clocks, "device_status": status, "peaks": pk_src,
             "rank_step_ms": {"max": ms_total / args.steps, "min": float(ms_min.item()) / args.steps},
         }
