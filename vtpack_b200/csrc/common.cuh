@@ -64,7 +64,8 @@ cudaError_t launch_kernel(void (*kernel)(KArgs...), bool early, int cluster_x, d
 // Kernels with several CTAs per SM start early only when the grid is small.  CTAs that start early are placed on
 // the SMs that have room first, as many as fit there, and stay packed on those: a latency-bound chain of small
 // kernels gains (DeiT-Ti, one image: 790 -> 570 us launch by launch), a large grid would be left unevenly spread
-// (DeiT-S, 12 images in fp32: 5.8 -> 8.2 ms with every kernel starting early).
+// (DeiT-S, 12 images in fp32: 5.8 -> 8.2 ms with every kernel starting early).  The fp32 pool starts early whatever its grid, because of the
+// matrices it splits (figures at pool_region_terms_kernel).
 template <typename... KArgs, typename... Args>
 cudaError_t launch_chain(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
     const bool early = (long long)grid.x * grid.y * grid.z <= 2ll * sm_count();
