@@ -363,14 +363,7 @@ def model_roofline(model, batch, counts, ms_per_step, pk, image_bytes, fine):
 
 
 def launches_per_forward(model, images):
-    """Kernels of this library in one forward.  In bf16: im2col (which writes the cls rows and starts the counts), patch-embed
-    Linear, first gate, final LayerNorm and head; per block pool, q + kv, attention, proj, fc1, fc2 and unpool (which
-    leaves the next block's gate decisions).  q and kv share one launch when both widths are whole 64-column slabs.
-    Other forwards are counted by the profiler: whether fp32 blocks launch q and kv together depends on the batch."""
-    depth = len(model.blocks)
-    if model.compute_dtype() == torch.bfloat16 and not model.flags:
-        C = model.embed_dim
-        return 5 + (7 if C >= 64 and C % 64 == 0 else 8) * depth
+    """Kernels of this library in one forward, counted by the profiler: which Linears share a launch depends on the batch."""
     with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
         model._forward_eval(images, None, use_plans=False)
         torch.cuda.synchronize()
@@ -999,7 +992,7 @@ def main():
             line["roofline"]["frac_all_launches"] = all_linear["frac_in_step_est"]
             line["kernels"] = rows
             line["kernels_note"] = ("one block (the middle one's weights and the tokens it received in this forward), "
-                                    "q and kv projections as separate launches (the forward pairs them in one); "
+                                    "q and kv projections, and fc1 and fc2, as separate launches (the forward has one for each two); "
                                     "ms_event_bracketed: every stage sits between two event records, which keeps the "
                                     "next launch from queueing behind the running one: an upper bound. ms_in_step_est "
                                     "= that share scaled so that depth x block + front/back equals ms_per_step")

@@ -976,3 +976,50 @@ def test_image_with_more_regions_than_a_list_holds():
     assert int(blk.dge.states["batches_device"]) == 2 * n and _lib.device_status() == 0
     for half in big.split(H * W, 1):
         assert float((half - small).norm() / small.norm()) < 1.9e-4
+
+
+@pytest.mark.parametrize("fine", [0.0, 0.3, 1.0])
+@pytest.mark.parametrize("C,B,grid,sr,ratio", [(64, 8, 64, 8, 8), (128, 33, 32, 4, 8), (192, 79, 16, 1, 4), (320, 96, 16, 2, 4),
+                                               (384, 125, 16, 1, 4), (384, 210, 16, 1, 8)])
+def test_mlp_in_one_launch(C, B, grid, sr, ratio, fine):
+    """fc1 and fc2 as one launch, which large batches take, and as two, which is how a block with events between its stages runs: the
+    same bits.  Few rows, some rounds of 256 rows for every pair of CTAs, a last round whose rows are two pairs' each (384: 2125 and
+    33410 rows), rows that end inside a warp's, and a wider hidden layer."""
+    import ctypes
+
+    from vtpack_b200 import _lib
+    from vtpack_b200.models.dge import deit_dge, pvt_dge
+    torch.manual_seed(C + B)
+    if sr > 1:
+        blk = pvt_dge.Block(C, C // 64, mlp_ratio=ratio, qkv_bias=True, sr_ratio=sr, split_sizes=[4, 2, 1]).eval()
+    else:
+        blk = deit_dge.Block(C, C // 64, mlp_ratio=ratio, qkv_bias=True, split_sizes=[4, 2, 1]).eval()
+    with torch.no_grad():
+        for name, p in blk.named_parameters():
+            if p.is_floating_point():
+                torch.nn.init.normal_(p, mean=float("norm" in name and name.endswith("weight")), std=0.05)
+    blk = blk.to(device=DEV, dtype=torch.bfloat16)
+    extra = int(sr == 1)
+    x = torch.randn(B, grid * grid + extra, C, device=DEV).bfloat16()
+    gate = torch.randn(B, grid // 4, grid // 4, 3, device=DEV)
+    gate[..., 0] = torch.where(torch.rand(gate.shape[:3], device=DEV) < fine, 9.0, -9.0)
+    if fine == 0.0:
+        gate[..., 2] = 9.0
+    got = blk(x, grid, grid, forced_gate=gate) if sr > 1 else blk(x, forced_gate=gate)
+    s = deit_dge._shape_struct(torch.bfloat16, B, grid, grid, extra, C, C // 64, ratio * C, [4, 2, 1], blk.norm1.eps, 0, blk.attn.scale)
+    if sr > 1:
+        s.sr_ratio, s.sr_eps = sr, float(blk.attn.norm.eps)
+    w, lib = (pvt_dge if sr > 1 else deit_dge)._pack_block(blk, torch.bfloat16), _lib.lib()
+    n = lib.vtp_block_workspace_bytes(ctypes.byref(s))
+    ws, out = torch.empty(n, dtype=torch.uint8, device=DEV), torch.empty_like(x)
+    counts = torch.empty(B, dtype=torch.int32, device=DEV)
+    events = [torch.cuda.Event(enable_timing=True) for _ in range(12)]
+    for e in events:
+        e.record()
+    arr = (ctypes.c_void_p * 12)(*[e.cuda_event for e in events])
+    _lib.check(lib.vtp_dge_block_forward_timed(ctypes.byref(s), ctypes.byref(w), x.data_ptr(), out.data_ptr(), gate.data_ptr(),
+                                               counts.data_ptr(), ws.data_ptr(), n, arr, 12,
+                                               torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
+    assert bool(got.isfinite().all()) and torch.equal(got, out)

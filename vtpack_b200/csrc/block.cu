@@ -381,12 +381,15 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
     l1.flags = kflag | VTP_FLAG_GELU;
     if (fold_fc1) { l1.ln_mode = 2; l1.ln_stats = b.stats_acc; l1.ln_s = w.fc1_s; l1.ln_dim = C; l1.ln_eps = s.eps;
                 l1.ln_slots = linear_stat_slots(C); }
-    if ((rc = run_linear(l1, b.fc1_wt, true)) || (rc = marks.mark(9))) return rc;
-
     LinearArgs l2;   // q2 = q1 + hid W2^T + b   (into the q-projection buffer, dead by now)
     l2.a = b.hid; l2.lda = s.hidden; l2.w = w.fc2_w; l2.bias = w.fc2_b; l2.res = b.q1; l2.ldr = C; l2.y = b.qp;
     l2.ldy = C; l2.dtype = s.dtype; l2.m_max = rows; l2.m_dev = L_dev; l2.N = C; l2.K = s.hidden; l2.flags = kflag;
-    if ((rc = run_linear(l2, b.fc2_wt, false)) || (rc = marks.mark(10))) return rc;
+    if (!marks.events && mlp_tcgen05_supported(l1, l2) && mlp_tcgen05_pays(l1)) {
+        if ((rc = mlp_tcgen05(l1, l2, st))) return rc;
+    } else if ((rc = run_linear(l1, b.fc1_wt, true)) || (rc = marks.mark(9)) || (rc = run_linear(l2, b.fc2_wt, false)) ||
+               (rc = marks.mark(10))) {
+        return rc;
+    }
 
     if (by_region) {
         RegionUnpoolArgs ua;

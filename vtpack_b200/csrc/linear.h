@@ -53,6 +53,10 @@ int linear(const LinearArgs& p, cudaStream_t st);              // picks by dtype
 bool linear_pair_supported(const LinearArgs& a, const LinearArgs& b);
 int linear_tcgen05_pair(const LinearArgs& a, const LinearArgs& b, cudaStream_t st);   // two problems, one launch
 
+bool mlp_tcgen05_supported(const LinearArgs& fc1, const LinearArgs& fc2);
+bool mlp_tcgen05_pays(const LinearArgs& fc1);
+int mlp_tcgen05(const LinearArgs& fc1, const LinearArgs& fc2, cudaStream_t st);       // both, the hidden rows on chip
+
 // Unsigned division by a number the host knows: multiply by ceil(2^32 / d), then take back the one the estimate may
 // be over (it is never under).  A runtime division is about forty dependent instructions on the way to a CTA's first load.
 struct FastDiv { uint32_t d, magic; };
