@@ -670,6 +670,35 @@ def test_linear_bf16_rows_do_not_depend_on_the_launch(vl, N, K, gelu, res):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("N,K,gelu,res", [(8, 512, False, False), (64, 4096, False, True), (72, 384, True, False), (200, 768, False, True),
+                                          (384, 1536, False, True), (768, 3072, True, False), (1000, 896, False, False)])
+def test_linear_bf16_long_reductions_of_few_rows(vl, N, K, gelu, res):
+    """Few rows with a long reduction run in tiles that two CTAs share, 64 or 128 columns wide: the bits of the persistent kernel (20,000
+    rows), in whole and narrow last tiles, with all rows of a tile valid, some, or none of a CTA's, and rows beyond the device's count
+    untouched."""
+    from vtpack_b200 import _lib
+    from vtpack_b200.runtime import ptr, stream_ptr
+    g = torch.Generator(DEV).manual_seed(N + K)
+    x = torch.randn(20000, K, device=DEV, generator=g).bfloat16()
+    w = (torch.randn(N, K, device=DEV, generator=g) * K ** -0.5).bfloat16()
+    b = torch.randn(N, device=DEV, generator=g)
+    r = torch.randn(20000, N, device=DEV, generator=g).bfloat16() if res else None
+
+    def run(m_max, m=None):
+        y = torch.full((m_max, N), 7.0, device=DEV, dtype=torch.bfloat16)
+        m_dev = None if m is None else torch.tensor([m], dtype=torch.int32, device=DEV)
+        _lib.check(_lib.lib().vtp_linear(ptr(x), K, ptr(w), ptr(b), ptr(r), N, ptr(y), N, 1, m_max, ptr(m_dev), N, K, int(gelu),
+                                         stream_ptr(x.device)))
+        return y
+    full = run(20000)
+    for M in (1, 32, 33, 63, 64, 65, 128, 129, 257, 700, 1799, 3000):
+        assert torch.equal(run(M), full[:M]), M
+    for m_max, m in ((257, 0), (257, 1), (257, 63), (257, 92), (1799, 644), (1799, 1700), (4000, 2049)):
+        y = run(m_max, m)
+        assert torch.equal(y[:m], full[:m]) and bool((y[m:] == 7.0).all()), (m_max, m)
+    assert _lib.device_status() == 0
+
+
 @pytest.mark.parametrize("N,K", [(72, 64), (192, 768), (384, 384), (768, 384), (1536, 256)])
 def test_linear_bf16_without_a_bias(vl, N, K):
     """The same bits with no bias as with one of zeros, from the kernel of small problems, single CTAs and pairs."""

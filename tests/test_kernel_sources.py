@@ -8,7 +8,8 @@ import pytest
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "vtpack_b200", "csrc")
 WAITING = {"linear_tc_kernel": "linear_tc.cu", "linear_tc_small_kernel": "linear_tc.cu", "attn_tc_kernel": "attention_tc.cu",
            "linear_f32_tc_kernel": "linear_f32_tc.cu", "linear_f32_terms_kernel": "linear_f32_terms.cu",
-           "attn_f32_tc_kernel": "attention_f32_tc.cu", "mlp_tc_kernel": "mlp_tc.cu"}
+           "attn_f32_tc_kernel": "attention_f32_tc.cu", "mlp_tc_kernel": "mlp_tc.cu",
+           "linear_tc_pair_kernel": "linear_tc.cu"}
 
 
 def source(name):

@@ -18,7 +18,7 @@
 // (their own W boxes, a narrower MMA), one per CTA, so that round costs a fraction of a tile.
 // The number of valid rows is read from device memory: tiles beyond it do not exist, rows
 // beyond it are never stored.
-// linear_tc_small_kernel (below) is the form for problems of few tiles.
+// linear_tc_small_kernel and linear_tc_pair_kernel (below) are the forms for problems of few tiles.
 //
 // What bounds it, and what was measured (B200, launches replayed back to back in a graph, us; the kernel before: one CTA per
 // tile, staging slabs shared by all epilogue warps, a store thread):
@@ -32,7 +32,7 @@
 //   393216 x 64, K = 64                                    28.3   19.5   18.0    HBM (floor 16)
 //   50176 x 3072, K = 768                                 199    183    201      tensor core under the power limit
 //   90 x 768, K = 192, GELU (DeiT-Ti fc1, one image)        5.5    3.3    2.6    latency (small kernel)
-//   90 x 192, K = 768, residual (DeiT-Ti fc2)               6.6    4.7    3.2    latency (small kernel): 48 MMA steps in a row
+//   90 x 192, K = 768, residual (DeiT-Ti fc2)               6.6    3.9    3.2    latency (pair kernel; 4.7 before it): 48 MMA steps in a row
 // A k-block's loads cost their producer thread 265 to 450 cycles (try_wait 42, an arrival that the next try_wait waits behind
 // 130, the loads themselves), the MMAs of 192 or 256 columns 384 or 512: three producers take k-blocks in turn.
 //
@@ -767,6 +767,232 @@ linear_tc_small_kernel(const __grid_constant__ SmallLaunch L, int K, int* status
     if (warp == PRODUCERS) tmem_dealloc(tmem_base, BN);
 }
 
+// The same for a long reduction: a pair of CTAs shares a 128 x BN tile, 64 rows of A and half of the columns' W rows each.  A CTA's share of a
+// k-block is 12 or 16 KB instead of 24, and what bounds a CTA is how fast its operands come (64 bytes a clock); the MMAs
+// of a pair with 64 rows each take half of the cycles too.  Accumulator: lanes 0 to 63 hold the CTA's rows and the tile's
+// first half of the columns, lanes 64 to 127 the same rows and the other half.
+template <int BN_>
+struct PairConf {
+    static constexpr int BN = BN_, STAGES = BN == 64 ? 8 : 6, PRODUCERS = 3, FIRST_EPI = 4, EW = 16, THREADS = (FIRST_EPI + EW) * 32;
+    static constexpr int ROWS = TBM / 2, A_BYTES = ROWS * TBK * 2, B_BYTES = BN / 2 * TBK * 2, STAGE = 2 * (A_BYTES + B_BYTES);      // 128 of K
+    static constexpr int RING = STAGES * STAGE;
+    static constexpr int SUMS = ROWS * 32 * 8;           // EPI_EMIT: (sum, sum of squares) of 32 column groups of a row
+    static constexpr int USED = RING + SUMS + 256;
+    static constexpr int TOTAL = USED + 1024;
+    static constexpr int TMEM_COLS = 64;
+    static constexpr int COLS = BN / 8;                  // columns of an epilogue warp
+    static_assert(TOTAL <= SMEM_MAX && B_BYTES % 1024 == 0, "shared memory budget");
+};
+
+template <int BN, int EPI>
+__global__ void __launch_bounds__(PairConf<BN>::THREADS, 1)
+linear_tc_pair_kernel(const __grid_constant__ SmallLaunch L, int K, int* status) {
+    using S = PairConf<BN>;
+    constexpr int STAGES = S::STAGES, PRODUCERS = S::PRODUCERS, COLS = S::COLS;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const uint32_t ring = smem_u32(base);
+    float2* sums = reinterpret_cast<float2*>(base + S::RING);
+    uint64_t* full = reinterpret_cast<uint64_t*>(base + S::RING + S::SUMS);     // rank 0's
+    uint64_t* empty = full + STAGES;
+    uint64_t* acc_full = empty + STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* void_s = reinterpret_cast<int*>(tmem_slot + 2);               // [2] launch_is_void in front of the wait and behind it
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int rank = (int)cluster_ctarank();
+    const uint32_t full_a = smem_u32(full), empty_a = smem_u32(empty);
+
+    const TcScalars& P = L.p[0];
+    const uint32_t tile = blockIdx.x >> 1;
+    const uint32_t mt = fast_div(tile, P.n_tiles);
+    const int m0 = (int)mt * TBM, ct0 = (int)(tile - mt * P.n_tiles.d) * BN;
+    const int n_stages = K / (2 * TBK);
+
+    if (warp == 0 && elect_one()) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        mbar_init(acc_full, 1);
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (warp == 1 && elect_one()) { prefetch_tmap(&L.ta[0]); prefetch_tmap(&L.tw[0]); }
+    if (warp == PRODUCERS) { tmem_alloc_pair(tmem_slot, S::TMEM_COLS); tmem_relinquish_pair(); }
+    if (threadIdx.x == S::FIRST_EPI * 32) void_s[0] = launch_is_void(status) ? 1 : 0;
+    tc_fence_before_sync();
+    __syncthreads();
+    cluster_sync_all();                  // the partner's barriers exist before anything arrives on them
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+    const bool known_void = lead_word<2>(void_s) != 0;
+    pdl_begin();
+    // a pair that starts when others have ended looks first whether its rows exist
+    const bool none = (int)blockIdx.x >= L.at_once && P.m_dev && m0 >= *reinterpret_cast<const volatile int32_t*>(P.m_dev);
+
+    if (known_void || none) {
+    } else if (warp < PRODUCERS) {
+        if (elect_one()) {
+            for (int i = warp; i < n_stages; i += PRODUCERS) {
+                const int s = i % STAGES;
+                if (i >= STAGES && !mbar_wait_a(empty_a + 8 * s, ((i / STAGES) & 1) ^ 1, abort_flag, status, STATUS_GEMM_PRODUCER)) break;
+                // (both CTAs' bytes are counted on rank 0's barrier, which its MMA thread waits on)
+                if (rank == 0) mbar_arrive_expect_tx_a(full_a + 8 * s, 2 * S::STAGE);
+                const uint32_t lead = mapa_u32(full_a + 8 * s, 0), dst = ring + s * S::STAGE;
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    tma_load_2d_a<2>(dst + k * S::A_BYTES, &L.ta[0], lead, (2 * i + k) * TBK, m0 + rank * S::ROWS);
+                    tma_load_2d_a<2>(dst + 2 * S::A_BYTES + k * S::B_BYTES, &L.tw[0], lead, (2 * i + k) * TBK, ct0 + rank * (BN / 2));
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == PRODUCERS) {
+        if (rank == 0 && elect_one()) {
+            constexpr uint32_t idesc = idesc_bf16_f32(TBM, BN, 0, 0);
+            const uint32_t desc0 = (uint32_t)smem_desc_sw128(ring);
+            bool ok = true, peeked = false;
+            int s = 0;
+            uint32_t ph = 0;
+            for (int i = 0; i < n_stages; ++i) {
+                if (!peeked) ok = mbar_wait_a(full_a + 8 * s, ph, abort_flag, status, STATUS_GEMM_MMA);
+                if (!ok) break;
+                tc_fence_after_sync();
+                const bool wrap = s + 1 == STAGES;
+                // (a look behind the MMAs would wait until the tensor core has taken them)
+                peeked = mbar_passed_a(wrap ? full_a : full_a + 8 * (s + 1), wrap ? ph ^ 1 : ph);
+                const uint32_t a = desc0 + s * (S::STAGE >> 4), b = a + (2 * S::A_BYTES >> 4);
+#pragma unroll
+                for (int k = 0; k < 2 * TBK / 16; ++k) {
+                    const uint32_t ad = a + (k >> 2) * (S::A_BYTES >> 4) + 2 * (k & 3), bd = b + (k >> 2) * (S::B_BYTES >> 4) + 2 * (k & 3);
+                    if (k == 0 && i == 0) umma_ss_pair_lo<false>(tmem_base, ad, bd, idesc);
+                    else umma_ss_pair_lo<true>(tmem_base, ad, bd, idesc);
+                }
+                if (i + STAGES < n_stages) umma_commit_a<2>(empty_a + 8 * s);
+                if (wrap) { s = 0; ph ^= 1; }
+                else ++s;
+            }
+            if (ok) umma_commit_a<2>(smem_u32(acc_full));
+        }
+        __syncwarp();
+    } else {
+        const int g = (warp - S::FIRST_EPI) >> 2, quarter = warp & 3;
+        const int half = quarter >> 1, row = (quarter & 1) * 32 + lane;          // of the tile's columns; of the CTA's rows
+        const int wm0 = m0 + rank * S::ROWS + (quarter & 1) * 32, m = wm0 + lane, N = P.N;
+        const int c0 = half * (BN / 2) + g * COLS, n0 = ct0 + c0;
+        // (a launch that turns out to be void forms its products and has no rows to store)
+        if (threadIdx.x == S::FIRST_EPI * 32) void_s[1] = launch_is_void(status) ? 1 : 0;
+        int M = P.m_max;
+        if (P.m_dev) M = min(max(*reinterpret_cast<const volatile int32_t*>(P.m_dev), 0), M);
+        named_barrier(5, S::EW * 32);
+        if (void_s[1] != 0) M = 0;
+        const bool live = wm0 < M, row_ok = m < M;        // the warp, the lane has rows
+        float add[COLS], ln_a = 1.f, ln_b = 0.f;
+        uint4 rv[COLS / 8];
+        if (live) {
+            if ((EPI & EPI_LN) && row_ok) row_fold(P.ln, m, ln_a, ln_b);
+#pragma unroll
+            for (int c = 0; c < COLS / 8; ++c) {
+                const int nb = min(n0 + 8 * c, N - 8);
+                const float* bias = P.bias ? P.bias + nb : g_no_bias;
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const float4 b4 = __ldg(reinterpret_cast<const float4*>(bias) + q);
+                    float* d = add + 8 * c + 4 * q;
+                    d[0] = b4.x; d[1] = b4.y; d[2] = b4.z; d[3] = b4.w;
+                    if (EPI & EPI_LN) {
+                        const float4 s4 = __ldg(reinterpret_cast<const float4*>(P.ln.s + nb) + q);
+                        d[0] = fmaf(ln_b, s4.x, d[0]); d[1] = fmaf(ln_b, s4.y, d[1]); d[2] = fmaf(ln_b, s4.z, d[2]); d[3] = fmaf(ln_b, s4.w, d[3]);
+                    }
+                }
+                rv[c] = make_uint4(0, 0, 0, 0);
+                if ((EPI & EPI_RES) && row_ok && n0 + 8 * c < N)
+                    rv[c] = *reinterpret_cast<const uint4*>(P.res + map_res_row(P.rm, m) * P.ldr + n0 + 8 * c);
+            }
+        }
+        const long long orow = map_out_row(P.rm, row_ok ? m : m0);
+        const bool ok = mbar_wait_warp(acc_full, 0, abort_flag, status, STATUS_GEMM_EPILOGUE);
+        if (ok && live) {
+            tc_fence_after_sync();
+            uint32_t r[COLS];
+            __syncwarp();
+            const uint32_t at = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + g * COLS;
+            if constexpr (COLS == 8) tmem_ld_32x8(at, r);
+            else tmem_ld_32x16(at, r);
+            tmem_ld_wait();
+            float e1[4], e2[4];
+#pragma unroll
+            for (int c = 0; c < COLS / 8; ++c) {
+                const bool in = n0 + 8 * c < N;
+                float v[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float acc = __uint_as_float(r[8 * c + i]);
+                    v[i] = (EPI & EPI_LN) ? fmaf(ln_a, acc, add[8 * c + i]) : acc + add[8 * c + i];
+                }
+                if (EPI & EPI_GELU) gelu8(v);
+                if (EPI & EPI_RES) {
+                    Vec<bf16> w;
+                    float rf[8];
+                    w.raw = rv[c];
+                    w.to_float(rf);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[i] += rf[i];
+                }
+                if (EPI & EPI_EMIT) {
+                    // as in linear_tc_kernel: columns 2 q, 2 q + 1 of each eight
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float z0 = in ? v[2 * q] : 0.f, z1 = in ? v[2 * q + 1] : 0.f;
+                        const float q1 = z0 + z1, q2 = fmaf(z1, z1, __fmul_rn(z0, z0));
+                        if (c == 0) { e1[q] = q1; e2[q] = q2; }
+                        else { e1[q] += q1; e2[q] += q2; }
+                    }
+                }
+                if (row_ok && in) {
+                    Vec<bf16> ov;
+                    ov.from_float(v);
+                    ov.store(static_cast<bf16*>(P.y) + orow * P.ldy + n0 + 8 * c);
+                }
+            }
+            if (EPI & EPI_EMIT) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) sums[((half * 4 + g) * 4 + q) * S::ROWS + row] = make_float2(e1[q], e2[q]);
+            }
+        }
+        if ((EPI & EPI_EMIT) && live) {
+            // the eight warps of these rows (all of them get here): eights make sixteens, these (0 + 1) + (2 + 3), the column pairs the same
+            named_barrier(1 + (quarter & 1), 256);
+            if (g == 0 && (BN == 128 || half == 0) && row_ok && ok && ct0 + half * 64 < N) {
+                float t1[4], t2[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    float2 e[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        if (BN == 128) {
+                            e[k] = sums[((half * 4 + k) * 4 + q) * S::ROWS + row];
+                        } else {
+                            const float2 a = sums[((2 * k) * 4 + q) * S::ROWS + row], b = sums[((2 * k + 1) * 4 + q) * S::ROWS + row];
+                            e[k] = make_float2(a.x + b.x, a.y + b.y);
+                        }
+                    }
+                    t1[q] = (e[0].x + e[1].x) + (e[2].x + e[3].x);
+                    t2[q] = (e[0].y + e[1].y) + (e[2].y + e[3].y);
+                }
+                P.ln.emit[(size_t)m * P.ln.slots + ct0 / SLAB + half] = make_float2((t1[0] + t1[1]) + (t1[2] + t1[3]), (t2[0] + t2[1]) + (t2[2] + t2[3]));
+            }
+        }
+    }
+    if (*abort_flag) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000) { }          // let copies in flight land before releasing memory
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    cluster_sync_all();     // the partner no longer reads this CTA's operands
+    if (warp == PRODUCERS) tmem_dealloc_pair(tmem_base, S::TMEM_COLS);
+}
+
 // ------------------------------------------------------------------------------ host
 
 static EncodeTiledFn g_encode = nullptr;
@@ -941,6 +1167,43 @@ static int launch_small(const LinearArgs& p, const LinearArgs* p1, cudaStream_t 
     return launched(launch_kernel(kern, true, 1, dim3(grid), dim3(S::THREADS), (size_t)S::TOTAL, st, L, p.K, device_status_ptr()));
 }
 
+// Which tiles of linear_tc_pair_kernel a problem takes, 0: none.  All of them run at once, a pair of SMs each: as many tiles as pairs at most.
+// us, this form with 64 and with 128 columns / the forms above (rows valid of those the host has to allow for):
+//   64 x 4096, 192 rows (PVT's first reduction, 3 images)    7.1         / 13.2      128 x 2048, 192 rows          5.0  5.9  /  8.0
+//   320 x 1280, 192 rows                                     4.5  5.3    /  6.1      320 x 1280, 2048 rows (80)   10.0  6.2  /  6.8
+//   192 x 768, 92 of 257 rows (DeiT-Ti fc2, one image)       3.9  4.7    /  4.6      384 x 1536, 92 of 257         4.8  5.8  /  6.8
+//   384 x 1536, 644 of 1799 (90)                             8.0  6.6    /  8.2      768 x 3072, 92 of 257         6.6  7.8  / 11.0
+//   768 x 3072, 368 of 1028 (108)                           10.1  9.7    / 12.6      768 x 3072, 920 of 2570 (252) 16.5 12.3 / 12.6
+//   768 x 768, 92 of 257                                     4.0  4.8    /  4.8      768 x 768, 368 of 1028 (108)  7.2  5.5  /  5.9
+//   384 x 384, 92 of 257                                     3.3  4.2    /  3.6      1536 x 384, 92 of 257 (72)    4.3  4.4  /  4.2
+//   384 x 384, 644 of 1799 (90)                              6.2  4.6    /  4.5      3072 x 768, 92 of 257 (144)   7.8  5.9  /  6.0
+// (In brackets the 128 x 64 tiles, where they come near the 74 pairs or exceed them.)
+static int long_reduction_pairs(const LinearArgs& p) {
+    if (p.K % (2 * TBK) != 0) return 0;
+    const long long pairs = sm_count() / 2;
+    if (small_tiles(p, 64) <= (p.K >= 512 ? pairs : pairs * 4 / 5)) return p.K >= 384 ? 64 : 0;
+    return p.K >= 768 && p.N > 64 && small_tiles(p, 128) <= pairs ? 128 : 0;
+}
+
+template <int BN, int EPI>
+static int launch_pair(const LinearArgs& p, cudaStream_t st) {
+    using S = PairConf<BN>;
+    SmallLaunch L;
+    if (int rc = operand_maps(nullptr, &L.tw[0], p, BN / 2)) return rc;
+    const unsigned long long da[2] = {(unsigned long long)p.K, (unsigned long long)p.m_max}, sa[1] = {(unsigned long long)p.lda * 2ull};
+    const unsigned ba[2] = {TBK, S::ROWS};
+    if (int rc = make_tmap_bf16(&L.ta[0], p.a, 2, da, sa, ba)) return rc;
+    fill_scalars(L.p[0], p, false, BN);
+    L.ta[1] = L.ta[0]; L.tw[1] = L.tw[0]; L.p[1] = L.p[0];
+    const int grid = 2 * (int)small_tiles(p, BN);
+    L.grid0 = grid;
+    L.at_once = sm_count() / 2 * 2;
+    auto kern = linear_tc_pair_kernel<BN, EPI>;
+    static bool reserved[64] = {};   // per instantiation and device
+    if (int rc = reserve_smem(kern, S::TOTAL, reserved)) return rc;
+    return launched(launch_kernel(kern, true, 2, dim3(grid), dim3(S::THREADS), (size_t)S::TOTAL, st, L, p.K, device_status_ptr()));
+}
+
 // Two independent Linears of the same K (the q and kv projections of a block) in ONE launch: the tiles of the second problem fill
 // the last, partial round of the first, and one launch's ramp and tail is saved.  Both: bf16 output, bias, no residual, no row
 // remap, N a multiple of 64; one or both fold a LayerNorm (ln_mode 1: a block that reduces its keys folds only q's).
@@ -995,6 +1258,17 @@ int linear_tcgen05(const LinearArgs& p, cudaStream_t st) {
         if (epi == 0) return launch_tc<128, 1, 0, true, 1>(p, nullptr, st);
         if (epi == EPI_RES) return launch_tc<128, 1, EPI_RES, true, 1>(p, nullptr, st);
         return fail(VTP_ERR_UNSUPPORTED, "linear (tcgen05): fp32 output supports bias and residual only");
+    }
+    const int pair_bn = long_reduction_pairs(p);
+    if (pair_bn) {
+#define VTP_PAIR_CASE(E) if (epi == (E)) return pair_bn == 64 ? launch_pair<64, (E)>(p, st) : launch_pair<128, (E)>(p, st);
+        VTP_PAIR_CASE(0)
+        VTP_PAIR_CASE(EPI_GELU)
+        VTP_PAIR_CASE(EPI_RES)
+        VTP_PAIR_CASE(EPI_LN)
+        VTP_PAIR_CASE(EPI_LN | EPI_GELU)
+        VTP_PAIR_CASE(EPI_EMIT | EPI_RES)
+#undef VTP_PAIR_CASE
     }
     if (small && epi == (EPI_GELU | EPI_RES)) return launch_small<64, EPI_GELU | EPI_RES, false, 1>(p, nullptr, st);
     if (epi == (EPI_GELU | EPI_RES)) return launch_tc<128, 1, EPI_GELU | EPI_RES, false, 1>(p, nullptr, st);

@@ -74,7 +74,7 @@ struct WRing {
         if (!peeked && !mbar_wait_a(full + 8 * s, ph, c.abort_flag, c.status, STATUS_GEMM_MMA)) return false;
         tc_fence_after_sync();
         const bool wrap = s + 1 == STAGES;
-        peeked = mbar_try_wait_a(wrap ? full : full + 8 * (s + 1), wrap ? ph ^ 1 : ph);
+        peeked = mbar_passed_a(wrap ? full : full + 8 * (s + 1), wrap ? ph ^ 1 : ph);
         return true;
     }
     // One box against 64 columns of A

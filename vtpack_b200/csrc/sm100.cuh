@@ -45,6 +45,9 @@ __device__ __forceinline__ bool mbar_try_wait_a(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
+// Whether the phase has completed, as far as one look tells (false: wait).
+__device__ __forceinline__ bool mbar_passed_a(uint32_t bar, uint32_t parity) { return mbar_try_wait_a(bar, parity); }
+
 // True in one lane of a converged warp.  Unlike with `lane == 0` the compiler then knows that one thread runs what
 // follows: a TMA load issues in about 10 cycles behind another one instead of 65, a tcgen05.commit in 45 fewer.
 __device__ __forceinline__ bool elect_one() {
@@ -383,6 +386,12 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr)
         : "memory");
+}
+__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
 }
 // 16 lanes x 64 columns: register 4 c + 2 i + j of thread t holds lane t / 4 + 8 i, column 8 c + 2 (t % 4) + j (the accumulator
 // layout of the warp-level matrix instructions, so ldmatrix / stmatrix match it).
