@@ -184,6 +184,23 @@ int vtp_unpool_grad_regions(const void* grad_out, int dtype, int B, int Hr, int 
                             void* stream);
 
 /*
+ * Gated decompress of the training path (vtpack/layers/dge.py:98-112 with sparse_train), region-parallel, for a patch list that was
+ * made from grain indices (arguments as in vtp_unpool_grad_regions):
+ *   out[b,tok,:] = ref[b,tok,:] + (x[p,:] - comp[p,:]) * gate[region, its grain]   for every token of patch p; extra tokens ungated
+ * x, comp [n_patches, C], gate [B*Hr*Wr, n_splits], ref, out [B, N, C], all of `dtype`; the difference and the product are rounded to it.
+ * The gradient: r[p] the sum of grad_out over the tokens of patch p (rounded), grad_x = r * gate, grad_comp = -grad_x, and
+ * grad_gate (may be null) = the sum over a region's patches of r . (x - comp) for its grain, 0 for the others.
+ */
+int vtp_unpool_gated_regions(const void* x, const void* comp, const void* gate, int dtype, int B, int Hr, int Wr, int region_size,
+                             int C, int num_extra, const int32_t* indices, const int* splits, int n_splits,
+                             const int32_t* region_first, const int32_t* offsets, int n_patches, const void* ref, void* out,
+                             void* stream);
+int vtp_unpool_gated_grad_regions(const void* grad_out, const void* x, const void* comp, const void* gate, int dtype, int B, int Hr,
+                                  int Wr, int region_size, int C, int num_extra, const int32_t* indices, const int* splits,
+                                  int n_splits, const int32_t* region_first, const int32_t* offsets, int n_patches, void* grad_x,
+                                  void* grad_comp, void* grad_gate, void* stream);
+
+/*
  * Ragged batched matrix product of the training path.  For image i and head h
  *   out_i = op(a_i) * op(b_i),  a_i = a[h, a_offsets[i] : a_offsets[i+1], :],  b_i likewise,
  * op = transpose when the matching flag is non-zero; the out_i are stacked along the row axis: image i

@@ -470,3 +470,55 @@ def test_region_rows_of_patch_list(layers, dt, extra, splits):
     start = torch.cumsum(lengths, 0) - lengths
     want = start[:, None] + extra + torch.cumsum(per, 1) - per
     assert torch.equal(first.cpu().long(), want) and torch.equal(idx32.cpu().long(), idx.reshape(B, -1).long())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("B,G,C,extra", [(3, 4, 192, 1), (2, 3, 64, 0), (5, 2, 384, 2), (2, 4, 320, 1), (3, 2, 768, 1), (2, 2, 512, 0)])
+def test_gated_decompress_is_the_sequence_of_operations(layers, dtype, B, G, C, extra):
+    """The gated decompress of the training path as one launch each way against the operations it stands for: output and row gradients
+    bit for bit; the gate's gradient, a sum of n = 16 C products (or fewer) in fp32, within n 2^-24 of the sum of their magnitudes and one
+    rounding of the result.  Gate values that are not quite 1, every grain, an image of one grain."""
+    from vtpack_b200.layers import dge, grained_sample as gs
+    g = torch.Generator(DEV).manual_seed(C + B)
+    N, W = extra + 16 * G * G, 4 * G
+    idx = torch.randint(0, 3, (B, G, G), device=DEV, generator=g)
+    idx[0] = 1
+    gate = torch.zeros(B, G, G, 3, device=DEV).scatter_(3, idx[..., None], 1.0) * (1 + 0.01 * torch.rand(B, G, G, 3, device=DEV, generator=g))
+    patches, _ = gs.grained_sample_index_to_patch(idx, torch.tensor([4, 2, 1]), 4, extra)
+    L = patches.shape[0]
+    leaves = [torch.randn(L, C, device=DEV, generator=g), torch.randn(L, C, device=DEV, generator=g), gate, torch.randn(B, N, C, device=DEV, generator=g)]
+    grad = torch.randn(B, N, C, device=DEV, generator=g).to(dtype)
+    enc = dge.DynamicGrainedEncoder(C, [4, 2, 1], sparse_train=True).to(DEV).train()
+
+    def run(fused):
+        x, comp, gt, ref = (t.to(dtype).requires_grad_(True) for t in leaves)
+        listed = patches if fused else patches.clone()            # (a copy does not say which grains it was made from)
+        enc.states.update(comp=comp, gate=gt, input=ref, patches=listed, size=(4 * G, W), num_extra_tokens=extra)
+        out = enc.decompress(x)
+        assert ("GatedDecompress" in type(out.grad_fn).__name__) == fused
+        return out, torch.autograd.grad(out, (x, comp, gt, ref), grad)
+    out, (gx, gc, gg, gr) = run(True)
+    want, (_, _, wg, wr) = run(False)
+    # the sequence pools the gate over its patches, which in fp32 rounds it: 16 additions of a value of about 1
+    assert torch.equal(out, want) if dtype is torch.bfloat16 else float((out - want).detach().abs().max()) <= 16 * 2.0 ** -24 * 12
+    assert torch.equal(gr, wr)
+    first = patches[:, 1] < 0
+    val = torch.ones(L, 1, device=DEV, dtype=dtype)
+    region = (patches[:, 0] * G + torch.div(patches[:, 1], 4, rounding_mode="floor")) * G + torch.div(patches[:, 2], 4, rounding_mode="floor")
+    picked = gate.to(dtype).gather(3, idx[..., None]).reshape(-1)
+    val[~first, 0] = picked[region[~first]]
+    x, comp, ref = (leaves[i].to(dtype) for i in (0, 1, 3))
+    rows = ((x - comp) * val).requires_grad_(True)
+    y = gs.grained_sample_decompress(rows, patches, ref, 4 * G, W, extra, True)
+    assert torch.equal(out, y)
+    r, = torch.autograd.grad(y, rows, grad)
+    assert torch.equal(gx, r * val) and torch.equal(gc, -(r * val))
+    prod = (r.double() * (x - comp).double())[~first]
+    exact = torch.zeros(B * G * G, device=DEV, dtype=torch.double).index_add_(0, region[~first], prod.sum(1))
+    size = torch.zeros_like(exact).index_add_(0, region[~first], prod.abs().sum(1))
+    got = gg.double().gather(3, idx[..., None]).reshape(-1)
+    eps = 2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -23
+    assert bool(((got - exact).abs() <= 16 * C * 2.0 ** -24 * size + eps * exact.abs()).all())
+    assert int((gg != 0).sum()) <= B * G * G and float((gg - wg).abs().max()) <= 0.05 * float(wg.abs().max()) + 1e-3
+    from vtpack_b200 import _lib
+    assert _lib.device_status() == 0

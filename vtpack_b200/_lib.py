@@ -71,6 +71,11 @@ PROTOTYPES = {
     "vtp_region_layout_supported": (c_int, [c_int, c_int]),
     "vtp_unpool_grad_regions": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
                                         C.POINTER(c_int), c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p]),
+    "vtp_unpool_gated_regions": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
+                                         C.POINTER(c_int), c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p]),
+    "vtp_unpool_gated_grad_regions": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
+                                              c_int, c_void_p, C.POINTER(c_int), c_int, c_void_p, c_void_p, c_int, c_void_p,
+                                              c_void_p, c_void_p, c_void_p]),
     "vtp_batched_sparse_gemm": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_int, c_ll,
                                         c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_ll, c_int,
                                         c_void_p]),

@@ -697,6 +697,44 @@ extern "C" int vtp_unpool_grad_regions(const void* grad_out, int dtype, int B, i
     return region_pool(a, dtype, static_cast<cudaStream_t>(stream));
 }
 
+static int gated_unpool(GatedArgs& a, int dtype, int B, int Hr, int Wr, int region_size, int C, int num_extra, const int32_t* indices,
+                        const int* splits, int n_splits, const int32_t* region_first, const int32_t* offsets, int n_patches, void* stream) {
+    VTP_REQUIRE(a.x && a.comp && a.gate && indices && splits && region_first && offsets, VTP_ERR_NULL, "gated unpool: null pointer");
+    VTP_REQUIRE(dtype == VTP_F32 || dtype == VTP_BF16, VTP_ERR_DTYPE, "gated unpool: dtype %d", dtype);
+    VTP_REQUIRE(B > 0 && Hr > 0 && Wr > 0 && C > 0 && num_extra >= 0 && n_patches >= 0, VTP_ERR_SHAPE, "gated unpool: bad shape");
+    if (int rc = make_splits(&a.sp, splits, n_splits, region_size)) return rc;
+    a.g.B = B; a.g.Hr = Hr; a.g.Wr = Wr; a.g.W = Wr * region_size; a.g.C = C; a.g.num_extra = num_extra;
+    a.g.region = region_size;
+    a.g.N = num_extra + Hr * Wr * region_size * region_size;
+    a.g.l_max = n_patches;       // regions whose rows would not fit are skipped and flagged
+    VTP_REQUIRE(region_ops_supported(a.g, dtype), VTP_ERR_SHAPE, "gated unpool: region size %d / C=%d have no region kernel", region_size, C);
+    for (const void* p : {a.x, a.comp, a.ref, a.grad_out, (const void*)a.out, (const void*)a.grad_x, (const void*)a.grad_comp})
+        VTP_REQUIRE(aligned16(p), VTP_ERR_ALIGN, "gated unpool: unaligned rows");
+    a.idx = indices; a.region_first = region_first; a.offsets = offsets;
+    a.status = device_status_ptr();
+    return region_gated_unpool(a, dtype, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int vtp_unpool_gated_regions(const void* x, const void* comp, const void* gate, int dtype, int B, int Hr, int Wr, int region_size,
+                                        int C, int num_extra, const int32_t* indices, const int* splits, int n_splits,
+                                        const int32_t* region_first, const int32_t* offsets, int n_patches, const void* ref, void* out,
+                                        void* stream) {
+    VTP_REQUIRE(ref && out, VTP_ERR_NULL, "gated unpool: null pointer");
+    GatedArgs a;
+    a.x = x; a.comp = comp; a.gate = gate; a.ref = ref; a.out = out;
+    return gated_unpool(a, dtype, B, Hr, Wr, region_size, C, num_extra, indices, splits, n_splits, region_first, offsets, n_patches, stream);
+}
+
+extern "C" int vtp_unpool_gated_grad_regions(const void* grad_out, const void* x, const void* comp, const void* gate, int dtype, int B, int Hr,
+                                             int Wr, int region_size, int C, int num_extra, const int32_t* indices, const int* splits,
+                                             int n_splits, const int32_t* region_first, const int32_t* offsets, int n_patches, void* grad_x,
+                                             void* grad_comp, void* grad_gate, void* stream) {
+    VTP_REQUIRE(grad_out && grad_x && grad_comp, VTP_ERR_NULL, "gated unpool gradient: null pointer");
+    GatedArgs a;
+    a.grad_out = grad_out; a.x = x; a.comp = comp; a.gate = gate; a.grad_x = grad_x; a.grad_comp = grad_comp; a.grad_gate = grad_gate;
+    return gated_unpool(a, dtype, B, Hr, Wr, region_size, C, num_extra, indices, splits, n_splits, region_first, offsets, n_patches, stream);
+}
+
 extern "C" int vtp_layernorm_add_rows(const void* x, int dtype, int rows, int C, long long in_row_stride, const float* w,
                                       const float* b, float eps, const void* addend, int a_mod, int a_off, void* out,
                                       int out_grp, int out_stride, int out_off, void* stream) {

@@ -72,7 +72,17 @@ struct RegionGateArgs {
     int32_t* counts = nullptr; Splits sp;
 };
 
+// Gated decompress of the training path, or (grad_out) its gradients; rows in one dtype, `gate` [B * R, sp.n] too.
+struct GatedArgs {
+    RegionGeom g; Splits sp;
+    const void *x = nullptr, *comp = nullptr, *gate = nullptr, *ref = nullptr, *grad_out = nullptr;
+    const int32_t *idx = nullptr, *region_first = nullptr, *offsets = nullptr;
+    void *out = nullptr, *grad_x = nullptr, *grad_comp = nullptr, *grad_gate = nullptr;
+    int* status = nullptr;
+};
+
 bool region_ops_supported(const RegionGeom& g, int dtype);
+int region_gated_unpool(const GatedArgs& a, int dtype, cudaStream_t st);
 int region_pool(const RegionPoolArgs& a, int dtype, cudaStream_t st);
 int region_unpool(const RegionUnpoolArgs& a, int dtype, cudaStream_t st);
 int region_gate(const RegionGateArgs& a, int dtype, cudaStream_t st);

@@ -15,6 +15,7 @@ from torch import nn
 from .. import _lib
 from ..runtime import dtype_code, ptr, require_cuda, stream_ptr
 from .grained_sample import (
+    gated_decompress,
     grained_sample_compress,
     grained_sample_compress_dense,
     grained_sample_decompress,
@@ -181,9 +182,13 @@ class DynamicGrainedEncoder(nn.Module):
         """``dge.py:87-112`` with ``self.training``: the gate value (1 in the forward pass, carrying the
         straight-through gradient in the backward pass) multiplies the update of every query."""
         st = self.states
-        x = x - st["comp"]
         H, W = st["size"]
         num_extra_tokens = st["num_extra_tokens"]
+        if self.sparse_train:
+            out = gated_decompress(x, st["comp"], st["gate"], st["input"], st["patches"], W, num_extra_tokens)
+            if out is not None:
+                return out
+        x = x - st["comp"]
         if not self.sparse_train:
             return grained_sample_decompress_dense(x, st["gate"], st["input"], self.splits, self.region_size,
                                                    H, W, num_extra_tokens, True)

@@ -64,6 +64,14 @@ def _mover_args(t, p32, width, num_extra_tokens):
     return (B, N, C, int(width), int(num_extra_tokens), ptr(p32), None, p32.shape[0])
 
 
+def _by_region(regions, offsets, shape, width, num_extra_tokens, dtype):
+    """Whether a patch list, from grain indices, describes these tokens and they have a region kernel."""
+    B, N, C = shape
+    return (regions is not None and offsets is not None and regions[3] == 4 and regions[6] == num_extra_tokens
+            and regions[0].shape[0] == B and N == num_extra_tokens + regions[4] * regions[5] * 16
+            and width == regions[5] * 4 and bool(_lib.lib().vtp_region_layout_supported(dtype_code(dtype), C)))
+
+
 class _GrainedSampleCompress(Function):
     """[B,N,C] -> [L,C] multi-grain mean pooling (``grained_sample.cu:198-239``); the gradient
     hands every token 1/size^2 of its patch's row (``grained_sample.py:26-38``)."""
@@ -125,9 +133,7 @@ class _GrainedSampleDecompress(Function):
         lib = _lib.lib()
         regions, offsets = ctx.regions
         B, N, C = shape
-        if (regions is not None and offsets is not None and regions[3] == 4 and regions[6] == num_extra_tokens
-                and regions[0].shape[0] == B and N == num_extra_tokens + regions[4] * regions[5] * 16
-                and width == regions[5] * 4 and lib.vtp_region_layout_supported(dtype_code(grad_output.dtype), C)):
+        if _by_region(regions, offsets, shape, width, num_extra_tokens, grad_output.dtype):
             # the list came from grain indices: one thread block per region instead of a walk over the list
             idx32, first, splits, region_size, Hr, Wr, _ = regions
             arr = (ctypes.c_int * len(splits))(*splits)
@@ -141,6 +147,55 @@ class _GrainedSampleDecompress(Function):
                 ptr(grad_input), stream_ptr(grad_output.device)))
         grad_ref = grad_output if is_add_ref else torch.zeros_like(grad_output)
         return grad_input, None, grad_ref, None, None, None, None
+
+
+class _GatedDecompress(Function):
+    """ref + replicate((x - comp) * the gate value of the region's grain), extra tokens ungated: ``dge.py:98-112`` of the
+    reference with ``sparse_train``, one launch each way."""
+
+    @staticmethod
+    def forward(ctx, x, comp, gate, ref, regions, offsets):
+        x, comp, gate, ref = x.contiguous(), comp.contiguous(), gate.contiguous(), ref.contiguous()
+        ctx.save_for_backward(x, comp, gate)
+        ctx.regions, ctx.offsets = regions, offsets
+        out = torch.empty_like(ref)
+        _lib.check(_lib.lib().vtp_unpool_gated_regions(
+            ptr(x), ptr(comp), ptr(gate), *_GatedDecompress.geometry(x, regions, offsets), ptr(ref), ptr(out),
+            stream_ptr(x.device)))
+        return out
+
+    @staticmethod
+    def geometry(x, regions, offsets):
+        idx32, first, splits, region_size, Hr, Wr, num_extra_tokens = regions
+        return (dtype_code(x.dtype), idx32.shape[0], Hr, Wr, region_size, x.shape[1], num_extra_tokens, ptr(idx32),
+                (ctypes.c_int * len(splits))(*splits), len(splits), ptr(first), ptr(offsets), x.shape[0])
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, grad_output):
+        x, comp, gate = ctx.saved_tensors
+        grad_output = grad_output.contiguous()
+        grad_x, grad_comp = torch.empty_like(x), torch.empty_like(comp)
+        grad_gate = torch.empty_like(gate) if ctx.needs_input_grad[2] else None
+        _lib.check(_lib.lib().vtp_unpool_gated_grad_regions(
+            ptr(grad_output), ptr(x), ptr(comp), ptr(gate), *_GatedDecompress.geometry(x, ctx.regions, ctx.offsets),
+            ptr(grad_x), ptr(grad_comp), ptr(grad_gate), stream_ptr(x.device)))
+        return grad_x, grad_comp, grad_gate, grad_output, None, None
+
+
+def gated_decompress(x, comp, gate, ref, patches, width, num_extra_tokens):
+    """``_GatedDecompress`` where its kernels take these rows and this patch list, which must be that of the gate's largest
+    values; None where they do not."""
+    regions, offsets = getattr(patches, "_vtp_regions", None), getattr(patches, "_vtp_offsets", None)
+    if (x.dim() != 2 or x.shape != comp.shape or x.shape[0] != patches.shape[0] or x.shape[1] != ref.shape[2]
+            or not (x.dtype is comp.dtype is gate.dtype is ref.dtype) or x.dtype not in (torch.float32, torch.bfloat16)
+            or not (x.is_cuda and comp.is_cuda and gate.is_cuda and ref.is_cuda)
+            or not _by_region(regions, offsets, ref.shape, width, num_extra_tokens, x.dtype)
+            or gate.shape != (ref.shape[0], regions[4], regions[5], len(regions[2]))
+            or (x.data_ptr() | comp.data_ptr() | ref.data_ptr()) % 16 != 0
+            or x.shape[1] * x.element_size() > 3072):              # the widest row that the replicate-unpool takes
+        return None
+    return _GatedDecompress.apply(x, comp, gate, ref, regions, offsets)
 
 
 grained_sample_compress = _GrainedSampleCompress.apply
