@@ -201,6 +201,14 @@ int vtp_unpool_gated_grad_regions(const void* grad_out, const void* x, const voi
                                   void* grad_comp, void* grad_gate, void* stream);
 
 /*
+ * p = softmax(scale * s) of rows of n scores, and the gradient ds = scale * p * (dp - sum(p * dp)); dense rows, `dtype` in and out, in
+ * fp32 between; the output may be the input (s or dp).  The step between the two ragged products of the training path's
+ * attention (vtpack/models/dge/deit_dge.py:90-91).
+ */
+int vtp_scaled_softmax(const void* s, int dtype, long long rows, int n, float scale, void* p, void* stream);
+int vtp_scaled_softmax_grad(const void* p, const void* dp, int dtype, long long rows, int n, float scale, void* ds, void* stream);
+
+/*
  * Ragged batched matrix product of the training path.  For image i and head h
  *   out_i = op(a_i) * op(b_i),  a_i = a[h, a_offsets[i] : a_offsets[i+1], :],  b_i likewise,
  * op = transpose when the matching flag is non-zero; the out_i are stacked along the row axis: image i

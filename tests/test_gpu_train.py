@@ -522,3 +522,64 @@ def test_gated_decompress_is_the_sequence_of_operations(layers, dtype, B, G, C, 
     assert int((gg != 0).sum()) <= B * G * G and float((gg - wg).abs().max()) <= 0.05 * float(wg.abs().max()) + 1e-3
     from vtpack_b200 import _lib
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("lengths,M,heads,d", [([197, 3, 50], 197, 6, 64), ([1, 0, 5], 49, 1, 64), ([17, 64], 64, 2, 64), ([9, 2], 1, 3, 64), ([4, 30], 1100, 2, 64)])
+def test_ragged_attention_is_the_sequence_of_operations(layers, dtype, lengths, M, heads, d):
+    """The training attention as one node against float64 attention of the same inputs, output and both gradients no further off than the
+    separate operations are (plus the two roundings' worth that separates orders of one sum); sums of one key, more keys than a lane
+    keeps, images without queries."""
+    from vtpack_b200.layers import sparse_ops
+    g = torch.Generator(DEV).manual_seed(M)
+    B, L, C = len(lengths), sum(lengths), heads * d
+    ln = torch.tensor(lengths)
+    q0 = torch.randn(L, C, device=DEV, generator=g).to(dtype)
+    kv0 = torch.randn(B, M, 2 * C, device=DEV, generator=g).to(dtype)
+    w = torch.randn(L, C, device=DEV, generator=g).to(dtype)
+    drop, scale = torch.nn.Dropout(0.0), d ** -0.5
+
+    def one(q, kv):
+        return sparse_ops.ragged_attention(q, kv, ln, heads, scale, drop)
+
+    def separate(q, kv):
+        qh = q.reshape(-1, heads, d).permute(1, 0, 2)
+        k, v = (t.reshape(heads, -1, d) for t in kv.reshape(B, M, 2, heads, d).permute(2, 3, 0, 1, 4))
+        n = ln.new_full([B], M)
+        p = (sparse_ops.batched_sparse_gemm(qh, k, ln, n, False, True) * scale).softmax(-1, dtype=v.dtype)
+        return sparse_ops.batched_sparse_gemm(p, v, ln, n, False, False).transpose(0, 1).reshape(-1, C)
+
+    def exact(q, kv):
+        k, v = kv.reshape(B, M, 2, heads, d).permute(2, 0, 3, 1, 4)
+        rows = [((x.reshape(-1, heads, d).transpose(0, 1) @ k[b].transpose(-1, -2)) * scale).softmax(-1) @ v[b]
+                for b, x in enumerate(q.split(lengths))]
+        return torch.cat(rows, 1).transpose(0, 1).reshape(-1, C)
+
+    def run(f, dt):
+        q, kv = q0.to(dt).requires_grad_(True), kv0.to(dt).requires_grad_(True)
+        y = f(q, kv)
+        return [t.double() for t in (y.detach(), *torch.autograd.grad(y, (q, kv), w.to(dt)))]
+    got, old, want = run(one, dtype), run(separate, dtype), run(exact, torch.float64)
+    eps = 2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -23
+    for a, b, e in zip(got, old, want):
+        size = float(e.abs().max())
+        assert float((a - e).norm()) <= float((b - e).norm()) * 1.1 + eps / 4 * float(e.norm())
+        assert float((a - e).abs().max()) <= 1.5 * float((b - e).abs().max()) + 2 * eps * size
+    assert one(q0, kv0[:, :, :-2]) is None and sparse_ops.ragged_attention(q0, kv0, ln, heads, scale, torch.nn.Dropout(0.1)) is None
+
+
+def test_scaled_softmax_of_rows_without_a_value():
+    """Scores of -inf, +inf and NaN, and a negative scale, as softmax(scale * s) gives them."""
+    from vtpack_b200 import _lib
+    from vtpack_b200.runtime import dtype_code, ptr, stream_ptr
+    inf, nan = float("inf"), float("nan")
+    for n in (3, 70, 1200):
+        s = torch.randn(6, n, device=DEV)
+        s[0, 1:], s[1], s[2, 0], s[3, 0] = -inf, -inf, nan, inf
+        for scale in (0.125, -0.5):
+            p = torch.empty_like(s)
+            _lib.check(_lib.lib().vtp_scaled_softmax(ptr(s), dtype_code(s.dtype), 6, n, scale, ptr(p), stream_ptr(s.device)))
+            want = (s.double() * scale).softmax(-1)
+            assert torch.equal(p.isnan(), want.isnan())
+            ok = ~want.isnan()
+            assert float((p.double() - want)[ok].abs().max()) <= 2.0 ** -20

@@ -76,6 +76,8 @@ PROTOTYPES = {
     "vtp_unpool_gated_grad_regions": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                               c_int, c_void_p, C.POINTER(c_int), c_int, c_void_p, c_void_p, c_int, c_void_p,
                                               c_void_p, c_void_p, c_void_p]),
+    "vtp_scaled_softmax": (c_int, [c_void_p, c_int, c_ll, c_int, c_float, c_void_p, c_void_p]),
+    "vtp_scaled_softmax_grad": (c_int, [c_void_p, c_void_p, c_int, c_ll, c_int, c_float, c_void_p, c_void_p]),
     "vtp_batched_sparse_gemm": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_int, c_ll,
                                         c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_ll, c_int,
                                         c_void_p]),

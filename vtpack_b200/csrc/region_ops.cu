@@ -708,7 +708,7 @@ gate_region_kernel(const T* __restrict__ x, RegionGeom g, const float* __restric
 // -------------------------------------------------------------- gated decompress (training)
 // out[b,tok] = ref[b,tok] + (x[p] - comp[p]) * gate[region] for the patch p that covers the token, gate[region] being the value of the
 // region's grain; extra tokens without a gate.  Differences and products are rounded to T, as the separate operations do.  One launch where
-// those took eight, and the gradient one for eleven (DeiT-S layer, 48 images, forward and backward, whose time is the host's: 2.42 -> 2.17 ms).
+// those took eight, and the gradient one for eleven (DeiT-S layer, 48 images, forward and backward, whose time is the host's: 2.43 -> 2.18 ms).
 template <typename T, int G, int CPL>
 __device__ __forceinline__ void gated_rows(float (&d)[CPL][Vec<T>::N], const T* __restrict__ x, const T* __restrict__ comp, size_t p, int C, int sub) {
     Vec<T> xv[CPL], cv[CPL];

@@ -56,9 +56,9 @@ class _Lengths:
 _INLINE_IMAGES = 512            # the library passes the offsets of up to this many images with the launch
 
 
-def _ragged_gemm(a, b, la, lb, ta, tb):
+def _ragged_gemm(a, b, la, lb, ta, tb, out=None):
     """One launch of the ragged product: a [H,La,ka], b [H,Lb,kb] -> the per-image products
-    stacked along dim 1 (``batched_sparse_gemm.cu:150-196``)."""
+    stacked along dim 1 (``batched_sparse_gemm.cu:150-196``), in `out` (dense, of that shape) if it is given."""
     require_cuda(a, b)
     a, b = a.contiguous(), b.contiguous()
     H, B = a.shape[0], la.n
@@ -68,7 +68,8 @@ def _ragged_gemm(a, b, la, lb, ta, tb):
             "a transposed b needs the same number of rows in every image"
     out_rows = B * a.shape[2] if ta else la.total
     out_cols = lb.max if tb else b.shape[2]
-    out = torch.empty(H, out_rows, out_cols, dtype=a.dtype, device=a.device)
+    if out is None:
+        out = torch.empty(H, out_rows, out_cols, dtype=a.dtype, device=a.device)
     lib = _lib.lib()
     head = (ptr(a), ptr(b), ptr(out), dtype_code(a.dtype), H, B, a.shape[1], a.shape[2], b.shape[1], b.shape[2])
     tail = (int(bool(ta)), int(bool(tb)), out_rows, out_cols, stream_ptr(a.device))
@@ -112,3 +113,53 @@ class _BatchedSparseGEMM(Function):
 
 
 batched_sparse_gemm = _BatchedSparseGEMM.apply
+
+
+class _RaggedAttention(Function):
+    """softmax(scale * q k^T) v of every image and head, q [L,C] (an image's queries behind those of the one in front), kv [B,M,2C]
+    -> [L,C]: the two ragged products with the softmax between them (``deit_dge.py:87-95`` of the reference) and the layout changes
+    around them as one node."""
+
+    @staticmethod
+    def forward(ctx, q, kv, q_lengths, heads, scale):
+        L, C = q.shape
+        B, M, _ = kv.shape
+        d = C // heads
+        la, lb = _Lengths(q_lengths), _Lengths(q_lengths.new_full([B], M))
+        qh = q.reshape(L, heads, d).transpose(0, 1).contiguous()
+        kvh = kv.reshape(B, M, 2, heads, d).permute(2, 3, 0, 1, 4).contiguous().view(2, heads, B * M, d)
+        p = _ragged_gemm(qh, kvh[0], la, lb, False, True)
+        _lib.check(_lib.lib().vtp_scaled_softmax(ptr(p), dtype_code(p.dtype), heads * L, M, scale, ptr(p), stream_ptr(p.device)))
+        ctx.save_for_backward(qh, kvh, p)
+        ctx.lengths, ctx.scale, ctx.shapes = (la, lb), scale, (q.shape, kv.shape)
+        return _ragged_gemm(p, kvh[1], la, lb, False, False).transpose(0, 1).reshape(L, C)
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, grad_output):
+        qh, kvh, p = ctx.saved_tensors
+        la, lb = ctx.lengths
+        (L, C), (B, M, _) = ctx.shapes
+        heads, _, d = qh.shape
+        g = grad_output.reshape(L, heads, d).transpose(0, 1).contiguous()
+        grads = torch.empty_like(kvh)
+        _ragged_gemm(p, g, la, la, True, False, out=grads[1])
+        ds = _ragged_gemm(g, kvh[1], la, lb, False, True)
+        _lib.check(_lib.lib().vtp_scaled_softmax_grad(ptr(p), ptr(ds), dtype_code(p.dtype), heads * L, M, ctx.scale, ptr(ds),
+                                                      stream_ptr(p.device)))
+        _ragged_gemm(ds, qh, la, la, True, False, out=grads[0])
+        grad_q = _ragged_gemm(ds, kvh[0], la, lb, False, False).transpose(0, 1).reshape(L, C)
+        grad_kv = grads.view(2, heads, B, M, d).permute(2, 3, 0, 1, 4).reshape(B, M, 2 * C)
+        return grad_q, grad_kv, None, None, None
+
+
+def ragged_attention(q, kv, q_lengths, heads, scale, drop):
+    """``_RaggedAttention`` where it is what the separate operations are: no dropout of its weights (`drop`, the module for it), rows of one
+    supported type on a GPU and lengths that add up; None elsewhere."""
+    if (type(drop) is not torch.nn.Dropout or drop.p != 0.0 or drop._forward_hooks or drop._forward_pre_hooks
+            or drop._backward_hooks or drop._backward_pre_hooks or not isinstance(scale, (int, float)) or q.dim() != 2 or kv.dim() != 3 or q.dtype is not kv.dtype
+            or q.dtype not in (torch.float32, torch.bfloat16) or not (q.is_cuda and kv.is_cuda) or kv.shape[2] != 2 * q.shape[1]
+            or q.shape[1] % heads != 0 or q_lengths.shape != kv.shape[:1] or kv.shape[1] == 0
+            or int(q_lengths.sum()) != q.shape[0]):
+        return None
+    return _RaggedAttention.apply(q, kv, q_lengths, heads, float(scale))

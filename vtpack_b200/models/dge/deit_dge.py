@@ -21,6 +21,7 @@ import torch.nn as nn
 
 from ... import _lib
 from ...layers import DynamicGrainedEncoder, batched_sparse_attention, batched_sparse_gemm
+from ...layers.sparse_ops import ragged_attention
 from ...runtime import (LaunchPlans, ParamWatch, capture_launches, dtype_code, ptr, require_cuda, scratch,
                         scratch_generation, stream_ptr)
 
@@ -122,10 +123,15 @@ class Attention(nn.Module):
         number of queries, else the two ragged products with the softmax between them."""
         B, N, C = x.shape
         h, d = self.num_heads, C // self.num_heads
-        q = self.q(q).reshape(-1, h, d).permute(1, 0, 2)
-        kv = self.kv(x).reshape(B, N, 2, h, d).permute(2, 3, 0, 1, 4)
+        q, kv = self.q(q), self.kv(x)
+        same = int(q_lengths.max() - q_lengths.min()) == 0
+        o = None if same else ragged_attention(q, kv, q_lengths, h, self.scale, self.attn_drop)
+        if o is not None:
+            return self.proj_drop(self.proj(o))
+        q = q.reshape(-1, h, d).permute(1, 0, 2)
+        kv = kv.reshape(B, N, 2, h, d).permute(2, 3, 0, 1, 4)
         k, v = kv[0], kv[1]
-        if int(q_lengths.max() - q_lengths.min()) == 0:
+        if same:
             q = q.reshape(h, B, -1, d)
             attn = (q @ k.transpose(-1, -2)) * self.scale
             attn = self.attn_drop(attn.softmax(dim=-1, dtype=v.dtype))

@@ -18,6 +18,7 @@ import torch.nn as nn
 
 from ... import _lib
 from ...layers import DynamicGrainedEncoder, batched_sparse_attention, batched_sparse_gemm
+from ...layers.sparse_ops import ragged_attention
 from ...runtime import (LaunchPlans, ParamWatch, capture_launches, dtype_code, ptr, require_cuda, scratch,
                         scratch_generation, stream_ptr)
 from .deit_dge import DropPath, Mlp, _CapturedTrunk, _WeightPack, _pack_block, _shape_struct
@@ -50,13 +51,18 @@ class Attention(nn.Module):
         path is ``Block.forward``, which never comes through here."""
         B, N, C = x.shape
         h, d = self.num_heads, C // self.num_heads
-        q = self.q(q).reshape(-1, h, d).permute(1, 0, 2)
+        q = self.q(q)
         if self.sr_ratio > 1:
             x_ = x.permute(0, 2, 1).reshape(B, C, H, W)
             x_ = self.norm(self.sr(x_).reshape(B, C, -1).permute(0, 2, 1))
             kv = self.kv(x_)
         else:
             kv = self.kv(x)
+        if self.training and int(q_lengths.max() - q_lengths.min()) != 0:
+            o = ragged_attention(q, kv, q_lengths, h, self.scale, self.attn_drop)
+            if o is not None:
+                return self.proj_drop(self.proj(o))
+        q = q.reshape(-1, h, d).permute(1, 0, 2)
         kv = kv.reshape(B, -1, 2, h, d).permute(2, 3, 0, 1, 4)
         k, v = kv[0], kv[1]
         n_keys = kv.shape[3]
