@@ -230,3 +230,52 @@ def test_dpvt_attention_module_matches_reference(golden_dir):
         assert rel_err(prm.grad, torch.from_numpy(z[f"grad.{name}"])) < 1e-4, name
         n += 1
     assert n == 8
+
+
+@pytest.mark.parametrize("mode", ["point", "channel"])
+@pytest.mark.parametrize("dtype,C", [(torch.float32, 12), (torch.float32, 44), (torch.float32, 64), (torch.float32, 96), (torch.float32, 256),
+                                     (torch.bfloat16, 24), (torch.bfloat16, 64), (torch.bfloat16, 88), (torch.bfloat16, 136), (torch.bfloat16, 256)])
+@pytest.mark.parametrize("H,W,G", [(29, 37, 29 * 37), (40, 3, 120), (29, 37, 1000)])
+def test_bilinear_attention_of_many_queries_is_that_of_the_general_kernel(op, dtype, mode, C, H, W, G):
+    """Enough queries for several vectors a lane (one to three, whole or part-filled), as tiles of pixels with ragged edges, narrow maps and
+    queries that are not the pixels, against the kernel for single channels (operands one element behind a 16-byte boundary), on maps with
+    infinities and NaN off the way of all but a few queries.  Both sum the same terms in other orders: apart by two times n 2^-24 of the sum of
+    the terms' magnitudes (n terms), and a rounding of the result in bf16 (of every term of grad_input)."""
+    P, lanes = 3, 2
+    B = -(-16 * 32 * 148 // (lanes * G))
+    g = torch.Generator(DEV).manual_seed(C + G)
+    ys, xs = torch.arange(G, device=DEV) // W % H, torch.arange(G, device=DEV) % W
+    t = [torch.randn(B, H, W, C, device=DEV, generator=g),
+         torch.stack([xs, ys], -1)[None, :, None].float() + 3 * torch.randn(B, G, P, 2, device=DEV, generator=g),
+         torch.randn(B, G, P if mode == "point" else C, device=DEV, generator=g),
+         torch.randn(B, G, C if mode == "point" else P, device=DEV, generator=g)]
+    t = [v.to(dtype) for v in t]
+
+    def run(t, shift):
+        def place(v):
+            buf = torch.zeros(v.numel() + shift, dtype=dtype, device=DEV)
+            buf[shift:] = v.flatten()
+            return buf[shift:].view(v.shape).requires_grad_(True)
+        a, gr, w, go = map(place, t)
+        y = op(a, gr, w, mode)
+        return [v.double() for v in (y.detach(), *torch.autograd.grad(y, (a, gr, w), go.detach()))]
+    got, want, size = run(t, 0), run(t, 1), run([t[0].abs(), t[1], t[2].abs(), t[3].abs()], 1)
+    sc, up = (t[2], t[3]) if mode == "point" else (t[3], t[2])
+    size[2] = 2 * float(t[0].abs().max()) * (sc.double().abs() * up.double().abs().sum(-1, keepdim=True))[..., None]
+    x0 = t[1].double().floor().long()
+    hits = torch.zeros(B * H * W, device=DEV)
+    for dx in (0, 1):
+        for dy in (0, 1):
+            x, y = x0[..., 0] + dx, x0[..., 1] + dy
+            ok = (x >= 0) & (x < W) & (y >= 0) & (y < H)
+            at = (torch.arange(B, device=DEV)[:, None, None] * H + y) * W + x
+            hits.index_add_(0, at[ok], torch.ones_like(at[ok], dtype=torch.float32))
+    most = float(hits.max())
+    # two results on either side of a rounding boundary are a unit of the last place apart, 2^-7 of a bf16 number at most
+    eps = 2.0 ** -7 if dtype is torch.bfloat16 else 0.0
+    for name, a, b, of, n in zip(("out", "grad_input", "grad_grid", "grad_weight"), got, want, size, (C + 4 * P + 8, most, C + 8, C + 4 * P + 8)):
+        bound = (2 * n * 2.0 ** -24 + (eps * (most + 1) if name == "grad_input" else 0)) * of + eps * torch.maximum(a.abs(), b.abs())
+        assert bool(((a - b).abs() <= bound + 1e-30).all()), name
+    t[0][0, 1, 1, 0], t[0][0, 2, 2, C - 1] = float("inf"), float("nan")
+    for name, a, b in zip(("out", "grad_input", "grad_grid", "grad_weight"), run(t, 0), run(t, 1)):
+        assert torch.equal(torch.isfinite(a), torch.isfinite(b)), name

@@ -130,6 +130,20 @@ template <typename T> __device__ __forceinline__ T from_f32(float v);
 template <> __device__ __forceinline__ float from_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ bf16 from_f32<bf16>(float v) { return __float2bfloat16_rn(v); }
 
+// Two values at once, each rounded as fmaf, a product and a difference are: half the issue slots.
+#define VTP_PAIR_OP(OP, A, B, MORE, C)                                                                                  \
+    float2 d;                                                                                                           \
+    asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"        \
+        OP ".rn.f32x2 d, a, b" MORE ";\n\tmov.b64 {%0, %1}, d;\n\t}"                                                    \
+        : "=f"(d.x), "=f"(d.y)                                                                                          \
+        : "f"(A.x), "f"(A.y), "f"(B.x), "f"(B.y), "f"(C.x), "f"(C.y));                                                  \
+    return d;
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { VTP_PAIR_OP("fma", a, b, ", c", c) }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { VTP_PAIR_OP("mul", a, b, "", b) }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { VTP_PAIR_OP("sub", a, b, "", b) }
+#undef VTP_PAIR_OP
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -30,16 +30,6 @@ namespace vtp {
 
 using namespace sm100;
 
-// a * b + c of two values at once, each rounded as fmaf rounds it
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
-        "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return d;
-}
-
 struct WaitCtx { volatile int* abort_flag; int* status; };
 
 // A ring of stages, each up to BOXES boxes of W, 64 of K and half of an MMA's columns; for one thread of a CTA that loads, or one of rank 0
