@@ -1023,3 +1023,31 @@ def test_mlp_in_one_launch(C, B, grid, sr, ratio, fine):
     torch.cuda.synchronize()
     assert _lib.device_status() == 0
     assert bool(got.isfinite().all()) and torch.equal(got, out)
+
+
+@pytest.mark.parametrize("C,G,B,extra", [(64, 20, 49, 0), (128, 12, 133, 1), (192, 20, 49, 1), (320, 20, 49, 1), (384, 28, 25, 1), (384, 4, 1187, 0)])
+def test_unpool_of_many_regions_is_that_of_few(C, G, B, extra):
+    """From eight regions a SM on a warp unpools a region, with fewer a block: the same tokens, statistics and next decisions, so the same bits
+    after two blocks that chain, at every grain; region counts that leave warps of the last block idle, with and without extra tokens."""
+    from functools import partial
+
+    from vtpack_b200 import _lib
+    from vtpack_b200.models.dge import pvt_dge
+    torch.manual_seed(C + G)
+    blocks = [pvt_dge.Block(C, C // 64, mlp_ratio=2, qkv_bias=True, norm_layer=partial(torch.nn.LayerNorm, eps=1e-6), sr_ratio=1,
+                            split_sizes=[4, 2, 1]).eval().to(device=DEV, dtype=torch.bfloat16) for _ in range(2)]
+    for b in blocks:
+        torch.nn.init.normal_(b.dge.router.gate.weight, std=0.3)
+        torch.nn.init.zeros_(b.dge.router.gate.bias)
+    x = torch.randn(B, G * G + extra, C, device=DEV).bfloat16()
+    assert B * (G // 4) ** 2 >= 8 * torch.cuda.get_device_properties(0).multi_processor_count and (B * (G // 4) ** 2) % 4
+
+    def run(rows):
+        y = pvt_dge.stage_forward(blocks, rows.contiguous(), G, G)
+        return y, [b.dge.states["batches_device"].clone() for b in blocks]
+    many, counts = run(x)
+    for part in (slice(0, 1), slice(1, 12), slice(B - 5, B)):
+        few, c = run(x[part])
+        assert torch.equal(few, many[part]) and all(torch.equal(p, q[part]) for p, q in zip(c, counts))
+    R = (G // 4) ** 2
+    assert B * extra + B * R < int(counts[1].sum()) < B * extra + 16 * B * R and _lib.device_status() == 0

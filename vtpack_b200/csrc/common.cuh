@@ -140,9 +140,19 @@ template <> __device__ __forceinline__ bf16 from_f32<bf16>(float v) { return __f
     return d;
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { VTP_PAIR_OP("fma", a, b, ", c", c) }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { VTP_PAIR_OP("mul", a, b, "", b) }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { VTP_PAIR_OP("add", a, b, "", b) }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { VTP_PAIR_OP("sub", a, b, "", b) }
 #undef VTP_PAIR_OP
 __device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+// channels 2i and 2i + 1 of a vector
+__device__ __forceinline__ float2 pair_of(const Vec<bf16>& v, int i) {
+    const uint32_t w = i == 0 ? v.raw.x : i == 1 ? v.raw.y : i == 2 ? v.raw.z : v.raw.w;
+    return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+__device__ __forceinline__ void set_pair(Vec<bf16>& v, int i, float2 f) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(f.x, f.y);
+    (i == 0 ? v.raw.x : i == 1 ? v.raw.y : i == 2 ? v.raw.z : v.raw.w) = *reinterpret_cast<const uint32_t*>(&h);
+}
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

@@ -480,18 +480,13 @@ pool_region_terms_kernel(const float* __restrict__ x, RegionGeom g, const int32_
 
 // ------------------------------------------------------------------------ router gate
 // Region mean of the raw tokens (/ 16), n_splits fp32 dot products, argmax with the lowest
-// index winning ties.  `part` holds the partial row sums published by publish_partials;
-// executed by one group of G lanes.
+// index winning ties.  acc: the sum of the region's tokens across group 0 of G lanes, of which the lane with `writes` stores.
 template <typename T, int G, int CPL>
-__device__ __forceinline__ void gate_from_partials(const float* part, int C, int sub, const float* __restrict__ gw,
-                                                   const float* __restrict__ gb, int S, float* __restrict__ logits_out,
-                                                   int32_t* __restrict__ idx_out, int rid, int32_t* counts_img,
-                                                   const Splits& sp, const float* __restrict__ img_bias) {
+__device__ __forceinline__ void gate_of_sum(float (&acc)[CPL][Vec<T>::N], int C, int sub, bool writes, const float* __restrict__ gw,
+                                            const float* __restrict__ gb, int S, float* __restrict__ logits_out,
+                                            int32_t* __restrict__ idx_out, int rid, int32_t* counts_img,
+                                            const Splits& sp, const float* __restrict__ img_bias) {
     constexpr int VN = Vec<T>::N;
-    float acc[CPL][VN];
-    zero_f<T, CPL>(acc);
-#pragma unroll 1
-    for (int r2 = 0; r2 < RG; ++r2) add_row<T, G, CPL, 2>(acc, part, r2, 0, sub, C);
     // the region mean: 1/16 is a power of two, so the product equals the quotient
 #pragma unroll
     for (int ch = 0; ch < CPL; ++ch)
@@ -515,19 +510,53 @@ __device__ __forceinline__ void gate_from_partials(const float* part, int C, int
         }
         pdot = group_sum<G>(pdot) + __ldg(gb + sI);
         if (img_bias) pdot += __ldg(img_bias + sI);          // per-image offset of the logits (forced grain mixes)
-        if (sub == 0 && logits_out) logits_out[(size_t)rid * S + sI] = pdot;
+        if (writes && logits_out) logits_out[(size_t)rid * S + sI] = pdot;
         if (sI == 0 || pdot > best) { best = pdot; best_i = sI; }
     }
-    if (sub == 0) {
+    if (writes) {
         idx_out[rid] = best_i;
         // queries this region contributes to its image (the image's slot starts at num_extra)
         if (counts_img) atomicAdd(counts_img, sp.v[min(best_i, sp.n - 1)] * sp.v[min(best_i, sp.n - 1)]);
     }
 }
+// `part` holds the partial row sums published by publish_partials; executed by one group of G lanes.
+template <typename T, int G, int CPL>
+__device__ __forceinline__ void gate_from_partials(const float* part, int C, int sub, const float* __restrict__ gw,
+                                                   const float* __restrict__ gb, int S, float* __restrict__ logits_out,
+                                                   int32_t* __restrict__ idx_out, int rid, int32_t* counts_img,
+                                                   const Splits& sp, const float* __restrict__ img_bias) {
+    float acc[CPL][Vec<T>::N];
+    zero_f<T, CPL>(acc);
+#pragma unroll 1
+    for (int r2 = 0; r2 < RG; ++r2) add_row<T, G, CPL, 2>(acc, part, r2, 0, sub, C);
+    gate_of_sum<T, G, CPL>(acc, C, sub, sub == 0, gw, gb, S, logits_out, idx_out, rid, counts_img, sp, img_bias);
+}
 
 // ----------------------------------------------------------------------------- unpool
 // out[b,tok] = ref[b,tok] + (q[p] - comp[p]) for the patch p that covers the token; optionally
 // also the next block's token statistics, router gate decisions and per-image counts.
+// an extra (cls) token: its own patch, row p of the packed ones
+template <typename T, int G, int CPL>
+__device__ __forceinline__ void unpool_extra(const T* __restrict__ q, const T* __restrict__ comp, const T* ref, T* out, const RegionGeom& g,
+                                             int b, int t, size_t p, int sub, const NextBlock& nx) {
+    constexpr int VN = Vec<T>::N;
+    const size_t tok = (size_t)b * g.N + t;
+    Vec<T> qv[CPL], cv[CPL], rv[CPL];
+    load_row<T, CPL>(qv, q + p * g.C, sub, G);
+    load_row<T, CPL>(cv, comp + p * g.C, sub, G);
+    load_row<T, CPL>(rv, ref + tok * g.C, sub, G);
+    float qf[CPL][VN], cf[CPL][VN], rf[CPL][VN];
+    to_f<T, CPL>(qf, qv); to_f<T, CPL>(cf, cv); to_f<T, CPL>(rf, rv);
+#pragma unroll
+    for (int ch = 0; ch < CPL; ++ch)
+#pragma unroll
+        for (int i = 0; i < VN; ++i) rf[ch][i] = (qf[ch][i] - cf[ch][i]) + rf[ch][i];
+    round_store<T, CPL>(rf, out + tok * g.C, sub, G);
+    if (nx.stats_x) {
+        const float2 st = mean_rstd(row_sums<T, G, CPL>(rf), g.C, nx.eps);
+        if (sub == 0) nx.stats_x[tok] = st;
+    }
+}
 template <typename T, int G, int CPL>
 constexpr int unpool_ctas() {
     if (Lay<T, G, CPL>::THREADS != 128) return G == 16 ? (CPL <= 2 ? 6 : 3) : CPL <= 2 ? 3 : CPL <= 3 ? 2 : 1;
@@ -552,23 +581,7 @@ unpool_region_kernel(const T* __restrict__ q, const T* __restrict__ comp, const 
         const int e = (rid - g.B * R) * (RG * RG / TPG) + gi;
         if (e >= g.B * g.num_extra) return;
         const int b = e / g.num_extra, t = e % g.num_extra;
-        const size_t tok = (size_t)b * g.N + t;
-        const size_t p = (size_t)(offsets[b] + t);
-        Vec<T> qv[CPL], cv[CPL], rv[CPL];
-        load_row<T, CPL>(qv, q + p * g.C, sub, G);
-        load_row<T, CPL>(cv, comp + p * g.C, sub, G);
-        load_row<T, CPL>(rv, ref + tok * g.C, sub, G);
-        float qf[CPL][VN], cf[CPL][VN], rf[CPL][VN];
-        to_f<T, CPL>(qf, qv); to_f<T, CPL>(cf, cv); to_f<T, CPL>(rf, rv);
-#pragma unroll
-        for (int ch = 0; ch < CPL; ++ch)
-#pragma unroll
-            for (int i = 0; i < VN; ++i) rf[ch][i] = (qf[ch][i] - cf[ch][i]) + rf[ch][i];
-        round_store<T, CPL>(rf, out + tok * g.C, sub, G);
-        if (nx.stats_x) {
-            const float2 st = mean_rstd(row_sums<T, G, CPL>(rf), g.C, nx.eps);
-            if (sub == 0) nx.stats_x[tok] = st;
-        }
+        unpool_extra<T, G, CPL>(q, comp, ref, out, g, b, t, (size_t)(offsets[b] + t), sub, nx);
         return;
     }
     const int b = rid / R, rr = rid % R;
@@ -645,6 +658,132 @@ unpool_region_kernel(const T* __restrict__ q, const T* __restrict__ comp, const 
     if (gi != 0) return;
     gate_from_partials<T, G, CPL>(part, g.C, sub, nx.gw, nx.gb, nx.S, nx.logits, nx.idx, rid,
                                   nx.counts ? nx.counts + b : nullptr, sp,
+                                  nx.image_bias ? nx.image_bias + (size_t)b * nx.S : nullptr);
+}
+
+// The same with a warp per region, for many bf16 regions, bit for bit.  With a block per region 41 us of DeiT-S, 256 images, were 20 % of DRAM's rate and
+// 42 % of the issue slots: 16 warps a SM, of which three wait while one works out the gate.  Here no barrier is left, arithmetic is on pairs
+// of channels and the code is the grain's own; a warp walks down the four grid rows, the next one's values on their way.
+// us of a launch, block -> warp: C = 384, 4096 regions (256 images) 37.7 -> 25.8, 1536 regions 17.0 -> 11.1; C = 64, 24576 regions (PVT-small, 96
+// images) 50.6 -> 33; C = 128, 6144 22.0 -> 15.3; C = 320, 1536 15.2 -> 11.0.  Without the next row's loads 24.0 / 12.2 (C = 384); with a row's vectors
+// loaded one chunk after the other, 24 warps a SM, 31.1 / 16.5.  Bound by HBM and L2 at 60 % (C = 384: 112 MB).
+constexpr int UW_WARPS = 4;
+template <int G, int CPL>
+constexpr int unpool_warp_ctas() { return G * CPL >= 40 ? 3 : G * CPL > 16 ? 4 : G * CPL == 16 ? 6 : 8; }
+
+// What a lane reads for a grid row at a grain of STEP x STEP: all of it on its way at once.
+template <int G, int CPL, int STEP>
+struct UnpoolRow {
+    static constexpr int TPG = RG * G / 32, PATCHES = (TPG + STEP - 1) / STEP;
+    static constexpr bool FINE = STEP == 1;              // (a token is its own patch: see above)
+    Vec<bf16> row[FINE ? 1 : TPG][CPL], q[PATCHES][CPL], c[FINE ? 1 : PATCHES][CPL];
+    __device__ __forceinline__ void load(const bf16* __restrict__ qp, const bf16* __restrict__ cp, const bf16* rp, int C, int sub) {
+        if (!FINE)
+#pragma unroll
+            for (int j = 0; j < TPG; ++j) load_row<bf16, CPL>(row[FINE ? 0 : j], rp + (size_t)j * C, sub, G);
+#pragma unroll
+        for (int j = 0; j < PATCHES; ++j) {
+            load_row<bf16, CPL>(q[j], qp + (size_t)j * C, sub, G);
+            if (!FINE) load_row<bf16, CPL>(c[FINE ? 0 : j], cp + (size_t)j * C, sub, G);
+        }
+    }
+};
+
+// One region's tokens at a grain of STEP x STEP; acc (group 0): their sum.
+template <int G, int CPL, int STEP>
+__device__ __forceinline__ void unpool_rows(float (&acc)[CPL][8], const bf16* __restrict__ q, const bf16* __restrict__ comp, const bf16* ref,
+                                            bf16* out, const RegionGeom& g, size_t tok0, int first, int sub, int grp, const NextBlock& nx) {
+    using U = UnpoolRow<G, CPL, STEP>;
+    constexpr int VN = 8, GROUPS = 32 / G, TPG = U::TPG;
+    auto load = [&](U& u, int w) {
+        const size_t from = (size_t)(first + (w / STEP) * (RG / STEP) + grp * TPG / STEP) * g.C;
+        u.load(q + from, comp + from, ref + (tok0 + (size_t)w * g.W + grp * TPG) * g.C, g.C, sub);
+    };
+    U cur, next;
+    load(cur, 0);
+#pragma unroll 1
+    for (int w = 0; w < RG; ++w) {
+        if (w + 1 < RG) load(next, w + 1);
+        const size_t tok = tok0 + (size_t)w * g.W + grp * TPG;
+        float s1[TPG], s2[TPG];                          // of a token: the sums of row_sums, in its order
+#pragma unroll
+        for (int j = 0; j < TPG; ++j) s1[j] = s2[j] = 0.f;
+#pragma unroll
+        for (int ch = 0; ch < CPL; ++ch) {
+            float2 sum[VN / 2], d[VN / 2];
+#pragma unroll
+            for (int j = 0; j < TPG; ++j) {
+                Vec<bf16> o;
+                if (U::FINE) {
+                    o = cur.q[j / STEP][ch];
+                } else {
+                    if (j % STEP == 0)
+#pragma unroll
+                        for (int i = 0; i < VN / 2; ++i) d[i] = sub2(pair_of(cur.q[j / STEP][ch], i), pair_of(cur.c[U::FINE ? 0 : j / STEP][ch], i));
+#pragma unroll
+                    for (int i = 0; i < VN / 2; ++i) set_pair(o, i, add2(d[i], pair_of(cur.row[U::FINE ? 0 : j][ch], i)));
+                }
+                o.store(out + (tok + j) * g.C + (sub + G * ch) * VN);
+#pragma unroll
+                for (int i = 0; i < VN / 2; ++i) {
+                    const float2 v = pair_of(o, i);                    // the rounded values
+                    s1[j] = s1[j] + v.x + v.y;
+                    s2[j] = fmaf(v.y, v.y, fmaf(v.x, v.x, s2[j]));
+                    sum[i] = j == 0 ? v : add2(sum[i], v);
+                }
+            }
+            if (nx.gw) {
+#pragma unroll
+                for (int i = 0; i < VN; ++i) {
+                    float v = i & 1 ? sum[i / 2].y : sum[i / 2].x;
+                    if (GROUPS == 4) v += __shfl_xor_sync(0xffffffffu, v, G);      // the left or right pair of the row
+                    acc[ch][i] += v;
+                    if (GROUPS >= 2) acc[ch][i] += __shfl_xor_sync(0xffffffffu, v, 16);
+                }
+            }
+        }
+        if (nx.stats_x) {
+#pragma unroll
+            for (int j = 0; j < TPG; ++j) {
+                const float2 st = mean_rstd(make_float2(group_sum<G>(s1[j]), group_sum<G>(s2[j])), g.C, nx.eps);
+                if (sub == 0) nx.stats_x[tok + j] = st;
+            }
+        }
+        cur = next;
+    }
+}
+
+template <int G, int CPL>
+__global__ void __launch_bounds__(UW_WARPS * 32, (unpool_warp_ctas<G, CPL>()))
+unpool_warp_kernel(const bf16* __restrict__ q, const bf16* __restrict__ comp, const bf16* ref, bf16* out, RegionGeom g,
+                   const int32_t* __restrict__ idx, const int32_t* __restrict__ region_first,
+                   const int32_t* __restrict__ offsets, Splits sp, NextBlock nx) {
+    pdl_begin();
+    constexpr int GROUPS = 32 / G;
+    const int lane = threadIdx.x & 31, sub = lane % G, grp = lane / G, warp = threadIdx.x >> 5;
+    const int R = g.Hr * g.Wr, regions = g.B * R, blocks = (regions + UW_WARPS - 1) / UW_WARPS;
+
+    if ((int)blockIdx.x >= blocks) {                     // extra tokens, one per group
+        const int e = (((int)blockIdx.x - blocks) * UW_WARPS + warp) * GROUPS + grp;
+        if (e >= g.B * g.num_extra) return;
+        const int b = e / g.num_extra, t = e % g.num_extra;
+        unpool_extra<bf16, G, CPL>(q, comp, ref, out, g, b, t, (size_t)(offsets[b] + t), sub, nx);
+        return;
+    }
+    const int rid = (int)blockIdx.x * UW_WARPS + warp;
+    if (rid >= regions) return;
+    const int b = rid / R, rr = rid % R;
+    const int ry = rr / g.Wr, rx = rr % g.Wr;
+    const int step = RG / sp.v[min(max(idx[rid], 0), sp.n - 1)];
+    const int first = region_first[rid];
+    const size_t tok0 = (size_t)b * g.N + g.num_extra + (size_t)ry * RG * g.W + rx * RG;
+    float acc[CPL][8];
+    zero_f<bf16, CPL>(acc);
+    if (step == 1) unpool_rows<G, CPL, 1>(acc, q, comp, ref, out, g, tok0, first, sub, grp, nx);
+    else if (step == 2) unpool_rows<G, CPL, 2>(acc, q, comp, ref, out, g, tok0, first, sub, grp, nx);
+    else unpool_rows<G, CPL, 4>(acc, q, comp, ref, out, g, tok0, first, sub, grp, nx);
+    if (nx.gw)
+        gate_of_sum<bf16, G, CPL>(acc, g.C, sub, lane == 0, nx.gw, nx.gb, nx.S, nx.logits, nx.idx, rid, nx.counts ? nx.counts + b : nullptr, sp,
                                   nx.image_bias ? nx.image_bias + (size_t)b * nx.S : nullptr);
 }
 
@@ -969,6 +1108,17 @@ static void launch_unpool_t(const RegionUnpoolArgs& a, cudaStream_t st) {
     const int R = a.g.Hr * a.g.Wr;
     using L = Lay<T, G, CPL>;
     const int grid = a.g.B * R + ceil_div(a.g.B * a.g.num_extra, RG * RG / L::TPG);
+    // A warp per region from eight regions a SM on: with fewer its chain, four grid rows in turn, is longer than that of a block per region.
+    // DeiT-S forward, block | warp, us: 32 images (3.5 a SM) 800 | 838, 64 (6.9) 1130 | 1133, 96 (10.4) 1481 | 1408; DeiT-Ti, 64 images
+    // 796 | 789, 96 939 | 890, 128 1109 | 1036.  Rows of a whole warp (C = 512, 768) are four tokens in a row each: 7 | 21 us, not used.
+    if constexpr (sizeof(T) == 2 && G <= 16 && G * CPL <= 48) {
+        if (a.g.B * R >= 8 * sm_count()) {
+            const int blocks = ceil_div(a.g.B * R, UW_WARPS) + ceil_div(a.g.B * a.g.num_extra, UW_WARPS * L::GROUPS);
+            launch_chain(unpool_warp_kernel<G, CPL>, dim3(blocks), dim3(UW_WARPS * 32), 0, st, (const T*)a.q, (const T*)a.comp, (const T*)a.ref,
+                (T*)a.out, a.g, a.idx, a.region_first, a.offsets, a.sp, a.next);
+            return;
+        }
+    }
     const size_t smem = a.next.gw ? region_smem<L>(a.g.C) : 0;
     allow_smem(unpool_region_kernel<T, G, CPL>, smem);
     launch_chain(unpool_region_kernel<T, G, CPL>, dim3(grid), dim3(L::THREADS), smem, st,
