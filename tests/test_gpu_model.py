@@ -1025,16 +1025,18 @@ def test_mlp_in_one_launch(C, B, grid, sr, ratio, fine):
     assert bool(got.isfinite().all()) and torch.equal(got, out)
 
 
-@pytest.mark.parametrize("C,G,B,extra", [(64, 20, 49, 0), (128, 12, 133, 1), (192, 20, 49, 1), (320, 20, 49, 1), (384, 28, 25, 1), (384, 4, 1187, 0)])
-def test_unpool_of_many_regions_is_that_of_few(C, G, B, extra):
-    """From eight regions a SM on a warp unpools a region, with fewer a block: the same tokens, statistics and next decisions, so the same bits
-    after two blocks that chain, at every grain; region counts that leave warps of the last block idle, with and without extra tokens."""
+@pytest.mark.parametrize("C,G,B,extra,sr", [(64, 20, 49, 0, 1), (128, 12, 133, 1, 1), (192, 20, 49, 1, 1), (320, 20, 49, 1, 1), (384, 28, 25, 1, 1), (384, 4, 1187, 0, 1),
+                                            (64, 20, 49, 0, 4), (128, 20, 49, 0, 4), (320, 20, 49, 0, 2)])
+def test_pool_and_unpool_of_many_regions_are_those_of_few(C, G, B, extra, sr):
+    """From eight regions a SM on a warp pools and unpools a region, with fewer a block: the same tokens, statistics, rows of a spatial reduction and
+    next decisions, so the same bits after two blocks that chain, at every grain; region counts that leave warps of the last block idle, with and
+    without extra tokens."""
     from functools import partial
 
     from vtpack_b200 import _lib
     from vtpack_b200.models.dge import pvt_dge
     torch.manual_seed(C + G)
-    blocks = [pvt_dge.Block(C, C // 64, mlp_ratio=2, qkv_bias=True, norm_layer=partial(torch.nn.LayerNorm, eps=1e-6), sr_ratio=1,
+    blocks = [pvt_dge.Block(C, C // 64, mlp_ratio=2, qkv_bias=True, norm_layer=partial(torch.nn.LayerNorm, eps=1e-6), sr_ratio=sr,
                             split_sizes=[4, 2, 1]).eval().to(device=DEV, dtype=torch.bfloat16) for _ in range(2)]
     for b in blocks:
         torch.nn.init.normal_(b.dge.router.gate.weight, std=0.3)

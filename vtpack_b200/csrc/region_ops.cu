@@ -235,6 +235,79 @@ constexpr int pool_ctas() {
     if (Lay<T, G, CPL>::THREADS != 128) return G == 16 ? (CPL <= 2 ? 6 : 4) : CPL <= 2 ? 3 : CPL <= 3 ? 2 : 1;
     return Lay<T, G, CPL>::TPG * CPL <= 1 ? 16 : Lay<T, G, CPL>::TPG * CPL <= 2 ? 12 : 7;
 }
+// LayerNorm(x) of token (ty, tx) as a part of its window's row (POOL_COLS)
+template <typename T, int G, int CPL>
+__device__ __forceinline__ void cols_row(const float (&f)[CPL][Vec<T>::N], float2 st, int b, int ty, int tx, const RegionGeom& g, int sr, int sub,
+                                         const float* __restrict__ lnw, const float* __restrict__ lnb, T* __restrict__ xn) {
+    constexpr int VN = Vec<T>::N;
+    const int wy = ty / sr, wx = tx / sr;
+    const size_t win = ((size_t)b * (g.Hr * RG / sr) + wy) * (g.W / sr) + wx;
+    T* dst = xn + ((win * sr + (ty - wy * sr)) * sr + (tx - wx * sr)) * g.C;
+#pragma unroll
+    for (int ch = 0; ch < CPL; ++ch) {
+        const int c0 = (sub + G * ch) * VN;
+        float o[VN];
+#pragma unroll
+        for (int i4 = 0; i4 < VN / 4; ++i4) {
+            const float4 w4 = __ldg(reinterpret_cast<const float4*>(lnw + c0) + i4);
+            const float4 b4 = __ldg(reinterpret_cast<const float4*>(lnb + c0) + i4);
+            const float gw[4] = {w4.x, w4.y, w4.z, w4.w}, gb[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) o[4 * i4 + i] = (f[ch][4 * i4 + i] - st.x) * st.y * gw[i] + gb[i];
+        }
+        Vec<T> ov;
+        ov.from_float(o);
+        ov.store(dst + c0);
+    }
+}
+// the e-th extra (cls) token, copied, by a group
+template <typename T, int G, int CPL, int MODE>
+__device__ __forceinline__ void pool_extra(int e, int sub, const T* __restrict__ x, const RegionGeom& g, const int32_t* __restrict__ region_first,
+                                           const int32_t* __restrict__ offsets, const int32_t* __restrict__ counts,
+                                           int32_t* __restrict__ counts_next, T* __restrict__ comp, float2* __restrict__ stats_x,
+                                           float2* __restrict__ stats_q, float2* __restrict__ stats_acc, int write_stats_x,
+                                           const float* __restrict__ lnw, const float* __restrict__ lnb, float eps, T* __restrict__ xn,
+                                           T* __restrict__ qn, int* status, int terms) {
+    constexpr bool STATS = MODE == POOL_STATS || MODE == POOL_COLS, EXPLICIT_LN = MODE == POOL_LN;
+    constexpr int VN = Vec<T>::N;
+    if (e >= g.B * g.num_extra) return;
+    const int b = e / g.num_extra, t = e % g.num_extra;
+    const size_t src_row = (size_t)b * g.N + t;
+    int dst_row;
+    if (region_first) {
+        dst_row = offsets[b] + t;
+        if (VTP_INDEX_GUARDS && g.l_max > 0 && (dst_row < 0 || dst_row >= g.l_max)) {   // caller's offsets
+            if (sub == 0 && status) atomicOr(status, STATUS_BAD_INDEX);
+            return;
+        }
+    } else {
+        int base = 0;
+        for (int j = sub; j < b; j += G) base += counts[j];
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) base += __shfl_xor_sync(0xffffffffu, base, o);
+        dst_row = base + t;
+    }
+    // start the next block's per-image count at the extra tokens; its gate adds the rest
+    if (t == 0 && sub == 0 && counts_next) counts_next[b] = g.num_extra;
+    Vec<T> row[CPL];
+    load_row<T, CPL>(row, x + src_row * g.C, sub, G);
+    store_row<T, CPL>(row, comp + (size_t)dst_row * g.C, sub, G);
+    float f[CPL][VN];
+    to_f<T, CPL>(f, row);
+    if (STATS) {
+        float2 st;
+        if (write_stats_x) {
+            st = mean_rstd(row_sums<T, G, CPL>(f), g.C, eps);
+            if (sub == 0) stats_x[src_row] = st;
+        } else {
+            st = stats_x[src_row];
+        }
+        if (sub == 0) { stats_q[dst_row] = st; if (stats_acc) stats_acc[dst_row] = make_float2(0.f, 0.f); }
+    } else if (EXPLICIT_LN) {
+        ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, xn, src_row, terms & 1);
+        ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, qn, (size_t)dst_row, terms & 2);
+    }
+}
 // (terms: POOL_LN of fp32 rows only; 1: xn, 2: qn as terms)
 template <typename T, int G, int CPL, int MODE>
 __device__ __forceinline__ void
@@ -257,45 +330,8 @@ pool_region(const int rid, const T* __restrict__ x, RegionGeom g, const int32_t*
     const int R = g.Hr * g.Wr;
 
     if (rid >= g.B * R) {
-        // ---- extra (cls) tokens: one per group, copied
-        const int e = (rid - g.B * R) * (RG * RG / TPG) + gi;
-        if (e >= g.B * g.num_extra) return;
-        const int b = e / g.num_extra, t = e % g.num_extra;
-        const size_t src_row = (size_t)b * g.N + t;
-        int dst_row;
-        if (region_first) {
-            dst_row = offsets[b] + t;
-            if (VTP_INDEX_GUARDS && g.l_max > 0 && (dst_row < 0 || dst_row >= g.l_max)) {   // caller's offsets
-                if (sub == 0 && status) atomicOr(status, STATUS_BAD_INDEX);
-                return;
-            }
-        } else {
-            int base = 0;
-            for (int j = sub; j < b; j += G) base += counts[j];
-#pragma unroll
-            for (int o = G / 2; o > 0; o >>= 1) base += __shfl_xor_sync(0xffffffffu, base, o);
-            dst_row = base + t;
-        }
-        // start the next block's per-image count at the extra tokens; its gate adds the rest
-        if (t == 0 && sub == 0 && counts_next) counts_next[b] = g.num_extra;
-        Vec<T> row[CPL];
-        load_row<T, CPL>(row, x + src_row * g.C, sub, G);
-        store_row<T, CPL>(row, comp + (size_t)dst_row * g.C, sub, G);
-        float f[CPL][VN];
-        to_f<T, CPL>(f, row);
-        if (STATS) {
-            float2 st;
-            if (write_stats_x) {
-                st = mean_rstd(row_sums<T, G, CPL>(f), g.C, eps);
-                if (sub == 0) stats_x[src_row] = st;
-            } else {
-                st = stats_x[src_row];
-            }
-            if (sub == 0) { stats_q[dst_row] = st; if (stats_acc) stats_acc[dst_row] = make_float2(0.f, 0.f); }
-        } else if (EXPLICIT_LN) {
-            ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, xn, src_row, terms & 1);
-            ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, qn, (size_t)dst_row, terms & 2);
-        }
+        pool_extra<T, G, CPL, MODE>((rid - g.B * R) * (RG * RG / TPG) + gi, sub, x, g, region_first, offsets, counts, counts_next, comp, stats_x, stats_q,
+                                    stats_acc, write_stats_x, lnw, lnb, eps, xn, qn, status, terms);
         return;
     }
 
@@ -363,26 +399,7 @@ pool_region(const int rid, const T* __restrict__ x, RegionGeom g, const int32_t*
             }
             if (step == 1 && sub == 0) { stats_q[prow] = st; if (stats_acc) stats_acc[prow] = make_float2(0.f, 0.f); }
             if (COLS) {
-                // (xn: the convolution's rows)
-                const int ty = ry * RG + w, tx = rx * RG + col, wy = ty / sr, wx = tx / sr;
-                const size_t win = ((size_t)b * (g.Hr * RG / sr) + wy) * (g.W / sr) + wx;
-                T* dst = xn + ((win * sr + (ty - wy * sr)) * sr + (tx - wx * sr)) * g.C;
-#pragma unroll
-                for (int ch = 0; ch < CPL; ++ch) {
-                    const int c0 = (sub + G * ch) * VN;
-                    float o[VN];
-#pragma unroll
-                    for (int i4 = 0; i4 < VN / 4; ++i4) {
-                        const float4 w4 = __ldg(reinterpret_cast<const float4*>(lnw + c0) + i4);
-                        const float4 b4 = __ldg(reinterpret_cast<const float4*>(lnb + c0) + i4);
-                        const float gw[4] = {w4.x, w4.y, w4.z, w4.w}, gb[4] = {b4.x, b4.y, b4.z, b4.w};
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) o[4 * i4 + i] = (f[ch][4 * i4 + i] - st.x) * st.y * gw[i] + gb[i];
-                    }
-                    Vec<T> ov;
-                    ov.from_float(o);
-                    ov.store(dst + c0);
-                }
+                cols_row<T, G, CPL>(f, st, b, ry * RG + w, rx * RG + col, g, sr, sub, lnw, lnb, xn);
             }
         } else if (EXPLICIT_LN) {
             ln_store<T, G, CPL>(f, sub, g.C, lnw, lnb, eps, xn, tok0 + j, terms & 1, step == 1 ? qn : nullptr, (size_t)prow, terms & 2);
@@ -452,6 +469,139 @@ pool_region_kernel(const T* __restrict__ x, RegionGeom g, const int32_t* __restr
     pdl_begin();
     pool_region<T, G, CPL, MODE>((int)blockIdx.x, x, g, idx, region_first, offsets, counts, offsets_out, region_first_out, counts_next, sp, comp,
                                  stats_x, stats_q, stats_acc, write_stats_x, lnw, lnb, eps, xn, qn, sum_only, sr, status, 0);
+}
+// The same with a warp per region, for many bf16 regions (POOL_STATS and POOL_COLS), bit for bit: see unpool_warp_kernel, whose reasons are the same
+// (a block per region, C = 384, 256 images: 30 % of DRAM's rate, half of the issue slots).  us of a launch, block -> warp: POOL_STATS C = 384, 4096 regions
+// 17.1 -> 13.6, 1536 regions 8.9 -> 7.1, C = 192, 4096 regions 14.7 -> 10.9; POOL_COLS (PVT-small, 96 images) C = 64, 24576 regions 58.2 -> 45.5,
+// C = 128, 6144 21.8 -> 19.0, C = 320, 1536 16.2 -> 13.3.
+constexpr int PW_WARPS = 4;
+template <int G, int CPL, int MODE>
+constexpr int pool_warp_ctas() { return G * CPL >= 40 ? (MODE == POOL_COLS ? 3 : 4) : G * CPL > 16 ? 4 : G * CPL == 16 ? 6 : 8; }
+
+template <int G, int CPL, bool COLS, int STEP>
+__device__ __forceinline__ void pool_rows(const bf16* __restrict__ x, const RegionGeom& g, int b, int ry, int rx, int first, bf16* __restrict__ comp,
+                                          float2* __restrict__ stats_x, float2* __restrict__ stats_q, float2* __restrict__ stats_acc,
+                                          bool write_stats_x, const float* __restrict__ lnw, const float* __restrict__ lnb, float eps,
+                                          bf16* __restrict__ xn, int sr, int sub, int grp) {
+    constexpr int VN = 8, GROUPS = 32 / G, TPG = RG / GROUPS, S = RG / STEP;
+    const size_t tok0 = (size_t)b * g.N + g.num_extra + (size_t)ry * RG * g.W + rx * RG + grp * TPG;
+    auto leave_stats = [&](int row, float2 st) {         // of a packed row
+        if (sub == 0) { stats_q[row] = st; if (stats_acc) stats_acc[row] = make_float2(0.f, 0.f); }
+    };
+    Vec<bf16> cur[TPG][CPL], next[TPG][CPL];
+#pragma unroll
+    for (int j = 0; j < TPG; ++j) load_row<bf16, CPL>(cur[j], x + (tok0 + j) * g.C, sub, G);
+    float acc[CPL][VN];                                  // of a patch
+    zero_f<bf16, CPL>(acc);
+#pragma unroll 1
+    for (int w = 0; w < RG; ++w) {
+        const size_t tok = tok0 + (size_t)w * g.W;
+        if (w + 1 < RG)
+#pragma unroll
+            for (int j = 0; j < TPG; ++j) load_row<bf16, CPL>(next[j], x + (tok + g.W + j) * g.C, sub, G);
+        float half[CPL][VN];                             // sum of this group's tokens of the row
+#pragma unroll
+        for (int j = 0; j < TPG; ++j) {
+            const int col = grp * TPG + j;
+            float f[CPL][VN];
+            to_f<bf16, CPL>(f, cur[j]);
+            float2 st = make_float2(0.f, 1.f);
+            if (write_stats_x) {
+                st = mean_rstd(row_sums<bf16, G, CPL>(f), g.C, eps);
+                if (sub == 0) stats_x[tok + j] = st;
+            } else if (COLS || STEP == 1) {
+                st = stats_x[tok + j];
+            }
+            if (COLS) cols_row<bf16, G, CPL>(f, st, b, ry * RG + w, rx * RG + col, g, sr, sub, lnw, lnb, xn);
+            if (STEP == 1) {
+                const int row = first + w * RG + col;
+                leave_stats(row, st);
+                store_row<bf16, CPL>(cur[j], comp + (size_t)row * g.C, sub, G);
+            }
+#pragma unroll
+            for (int ch = 0; ch < CPL; ++ch)
+#pragma unroll
+                for (int i = 0; i < VN; ++i) half[ch][i] = j == 0 ? f[ch][i] : half[ch][i] + f[ch][i];
+        }
+        if (STEP > 1) {
+#pragma unroll
+            for (int ch = 0; ch < CPL; ++ch)
+#pragma unroll
+                for (int i = 0; i < VN; ++i) {
+                    float v = half[ch][i];
+                    if (GROUPS == 4) v += __shfl_xor_sync(0xffffffffu, v, G);      // two neighbours
+                    acc[ch][i] += v;
+                    if (STEP == 4) acc[ch][i] += __shfl_xor_sync(0xffffffffu, v, 16);     // (right for the left half only, which stores)
+                }
+            if (w % STEP == STEP - 1) {
+                const bool mine = STEP == 4 ? grp == 0 : grp % (GROUPS / 2) == 0;
+                const int row = first + (w / STEP) * S + (STEP == 2 ? grp / (GROUPS / 2) : 0);
+#pragma unroll
+                for (int ch = 0; ch < CPL; ++ch) {
+#pragma unroll
+                    for (int i = 0; i < VN; ++i) acc[ch][i] *= 1.0f / (float)(STEP * STEP);
+                    Vec<bf16> o;
+                    o.from_float(acc[ch]);
+                    if (mine) o.store(comp + (size_t)row * g.C + (sub + G * ch) * VN);
+                    o.to_float(acc[ch]);
+                }
+                const float2 st = mean_rstd(row_sums<bf16, G, CPL>(acc), g.C, eps);
+                if (mine) leave_stats(row, st);
+                zero_f<bf16, CPL>(acc);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < TPG; ++j)
+#pragma unroll
+            for (int ch = 0; ch < CPL; ++ch) cur[j][ch] = next[j][ch];
+    }
+}
+
+template <int G, int CPL, int MODE>
+__global__ void __launch_bounds__(PW_WARPS * 32, (pool_warp_ctas<G, CPL, MODE>()))
+pool_warp_kernel(const bf16* __restrict__ x, RegionGeom g, const int32_t* __restrict__ idx, const int32_t* __restrict__ region_first,
+                 const int32_t* __restrict__ offsets, const int32_t* __restrict__ counts, int32_t* __restrict__ offsets_out,
+                 int32_t* __restrict__ region_first_out, int32_t* __restrict__ counts_next, Splits sp, bf16* __restrict__ comp,
+                 float2* __restrict__ stats_x, float2* __restrict__ stats_q, float2* __restrict__ stats_acc, int write_stats_x,
+                 const float* __restrict__ lnw, const float* __restrict__ lnb, float eps, bf16* __restrict__ xn, int sr) {
+    pdl_begin();
+    constexpr int GROUPS = 32 / G;
+    const int lane = threadIdx.x & 31, sub = lane % G, grp = lane / G, warp = threadIdx.x >> 5;
+    const int R = g.Hr * g.Wr, regions = g.B * R, blocks = (regions + PW_WARPS - 1) / PW_WARPS;
+    if ((int)blockIdx.x >= blocks) {
+        const int e = (((int)blockIdx.x - blocks) * PW_WARPS + warp) * GROUPS + grp;
+        if (e - grp < g.B * g.num_extra)                 // (a group past the end does the last one again: sums are the whole warp's)
+            pool_extra<bf16, G, CPL, MODE>(min(e, g.B * g.num_extra - 1), sub, x, g, region_first, offsets, counts, counts_next, comp, stats_x,
+                                           stats_q, stats_acc, write_stats_x, lnw, lnb, eps, xn, nullptr, nullptr, 0);
+        return;
+    }
+    const int rid = (int)blockIdx.x * PW_WARPS + warp;
+    if (rid >= regions) return;
+    const int b = rid / R, rr = rid % R;
+    const int ry = rr / g.Wr, rx = rr % g.Wr;
+    const int step = RG / sp.v[min(max(idx[rid], 0), sp.n - 1)];
+    int first;
+    if (region_first) {
+        first = region_first[rid];
+    } else {
+        int img_base;
+        first = derive_first(counts, idx, b, rr, R, sp, g.num_extra, lane, &img_base);
+        if (lane == 0) {
+            region_first_out[rid] = first;
+            if (rr == 0) {
+                offsets_out[b] = img_base;
+                if (b == g.B - 1) offsets_out[g.B] = img_base + counts[b];
+            }
+        }
+    }
+    // a grid without extra tokens has none to start the next block's count
+    if (rr == 0 && lane == 0 && counts_next && g.num_extra == 0) counts_next[b] = 0;
+#define VTP_POOL_ROWS(STEP) \
+    pool_rows<G, CPL, MODE == POOL_COLS, STEP>(x, g, b, ry, rx, first, comp, stats_x, stats_q, stats_acc, write_stats_x != 0, lnw, lnb, eps, xn, sr, sub, grp)
+    if (step == 1) VTP_POOL_ROWS(1);
+    else if (step == 2) VTP_POOL_ROWS(2);
+    else VTP_POOL_ROWS(4);
+#undef VTP_POOL_ROWS
 }
 // The pool of an fp32 block whose Linears take terms.  The CTAs in front of the pool's split the block's matrices, and do not wait
 // for the kernel in front: that is always one of the same call (the gate, or the unpool of the block before), which let this one start
@@ -1075,6 +1225,17 @@ static void launch_pool_t(const RegionPoolArgs& a, cudaStream_t st) {
             launch_kernel(pool_region_terms_kernel<G, CPL>, true, 1, dim3(split_grid + grid), block, smem, st, (const float*)a.x, a.g,
                 a.idx, a.region_first, a.offsets, a.counts, a.offsets_out, a.region_first_out, a.counts_next, a.sp, (float*)a.comp,
                 a.lnw, a.lnb, a.eps, (float*)a.xn, (float*)a.qn, a.xn_terms ? 3 : 2, split_grid, a.split);
+            return;
+        }
+    }
+    if constexpr (sizeof(T) == 2 && G <= 16 && G * CPL <= 48) {
+        // (eight regions a SM: the line of the unpool, which see; both forms write the same)
+        if (a.stats_q && a.g.l_max == 0 && a.g.B * R >= 8 * sm_count()) {
+            const int blocks = ceil_div(a.g.B * R, PW_WARPS) + ceil_div(a.g.B * a.g.num_extra, PW_WARPS * L::GROUPS);
+            auto kern = a.sr > 1 ? pool_warp_kernel<G, CPL, POOL_COLS> : pool_warp_kernel<G, CPL, POOL_STATS>;
+            launch_chain(kern, dim3(blocks), dim3(PW_WARPS * 32), 0, st, (const T*)a.x, a.g, a.idx, a.region_first, a.offsets, a.counts,
+                a.offsets_out, a.region_first_out, a.counts_next, a.sp, (T*)a.comp, a.stats_x, a.stats_q, a.stats_acc,
+                a.stats_x_ready ? 0 : 1, a.lnw, a.lnb, a.eps, (T*)a.cols, a.sr);
             return;
         }
     }
