@@ -1,7 +1,7 @@
 // Region-parallel token movers used by the fused block forward: router gate, multi-grain
 // pooling (with LayerNorm statistics or explicit LayerNorm rows) and replicate-unpool with
-// residual.  One CTA owns one 4x4 region of the token grid, whatever grain the gate picked
-// for it.  A token row is spread over a GROUP of G lanes, each lane holding CPL chunks of 16
+// residual.  One CTA (one warp, where there are many: pool_warp_kernel, unpool_warp_kernel) owns one 4x4 region of the token grid, whatever grain
+// the gate picked for it.  A token row is spread over a GROUP of G lanes, each lane holding CPL chunks of 16
 // bytes (C = G * CPL * 16 bytes exactly, e.g. 16 lanes x 3 chunks at C=384 bf16), so no lane
 // idles and no access needs a bounds check; a group owns TPG neighbouring tokens of a grid
 // row.  All 16 rows of a region are requested before any arithmetic, every region costs the
