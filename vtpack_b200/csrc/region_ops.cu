@@ -816,7 +816,8 @@ unpool_region_kernel(const T* __restrict__ q, const T* __restrict__ comp, const 
 // of channels and the code is the grain's own; a warp walks down the four grid rows, the next one's values on their way.
 // us of a launch, block -> warp: C = 384, 4096 regions (256 images) 37.7 -> 25.8, 1536 regions 17.0 -> 11.1; C = 64, 24576 regions (PVT-small, 96
 // images) 50.6 -> 33; C = 128, 6144 22.0 -> 15.3; C = 320, 1536 15.2 -> 11.0.  Without the next row's loads 24.0 / 12.2 (C = 384); with a row's vectors
-// loaded one chunk after the other, 24 warps a SM, 31.1 / 16.5.  Bound by HBM and L2 at 60 % (C = 384: 112 MB).
+// loaded one chunk after the other, 24 warps a SM, 31.1 / 16.5.  112 MB in 25.8 us are
+// 66 % of the copy rate, a third of them from L2; what is left is a warp's chain (159 registers, 12 warps a SM).
 constexpr int UW_WARPS = 4;
 template <int G, int CPL>
 constexpr int unpool_warp_ctas() { return G * CPL >= 40 ? 3 : G * CPL > 16 ? 4 : G * CPL == 16 ? 6 : 8; }
