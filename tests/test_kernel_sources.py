@@ -108,6 +108,21 @@ def test_lanes_that_wait_together_go_on_together(kernel):
         assert name in (("wait", "wait_a") if one or runs_out else ("wait_warp", "wait_cluster_warp")), (name, text[at:at + 80])
 
 
+def test_no_mma_is_issued_in_front_of_the_fence_behind_a_wait():
+    """What a wait on an mbarrier says about tensor memory (an accumulator was read, an operand is there) holds for an MMA only behind
+    tcgen05.fence::after_thread_sync.  The one-launch MLP has it in ``ready``, which stands in front of every MMA: on every way through
+    that goes on, and with no further wait between.  (No MMA and no wait can be made late enough on purpose to show the order.)"""
+    text = source("mlp_tc.cu")
+    ready = body("ready", text)
+    ways = [m.start() for m in re.finditer(r"return true;", ready)]
+    assert ways and all("tc_fence_after_sync()" in ready[:at] for at in ways)
+    kernel = body("mlp_tc_kernel", text)
+    mmas = [m.start() for m in re.finditer(r"\bw[12]\.mma\(", kernel)]
+    assert len(mmas) >= 4
+    for at in mmas:
+        assert kernel.rfind(".ready(", 0, at) > max(kernel.rfind("mbar_wait", 0, at), kernel.rfind(".done(", 0, at))
+
+
 def test_shared_memory_is_reserved_for_the_largest_launch():
     """A kernel's limit of shared memory is set once per device.  Set to what a launch takes that depends on the call, a thread could
     lower what another has just raised for a larger batch and is about to launch with."""

@@ -60,9 +60,10 @@ struct WRing {
     }
     // The next stage is looked at in front of a stage's MMAs: a wait that is issued behind them returns when the tensor core has taken them.
     __device__ __forceinline__ bool ready(const WaitCtx& c) {
+        const bool here = peeked || (RESIDENT && n >= (uint32_t)STAGES);
+        if (!here && !mbar_wait_a(full + 8 * s, ph, c.abort_flag, c.status, STATUS_GEMM_MMA)) return false;
+        tc_fence_after_sync();               // (also for the waits in front: accumulators that have been read, operands)
         if (RESIDENT && n >= (uint32_t)STAGES) return true;
-        if (!peeked && !mbar_wait_a(full + 8 * s, ph, c.abort_flag, c.status, STATUS_GEMM_MMA)) return false;
-        tc_fence_after_sync();
         const bool wrap = s + 1 == STAGES;
         peeked = mbar_passed_a(wrap ? full : full + 8 * (s + 1), wrap ? ph ^ 1 : ph);
         return true;
