@@ -182,3 +182,40 @@ def test_a_plan_that_no_longer_fits_is_made_again_at_once(no_capture):
     assert q is not p and plans.get("a", lambda p: True, _Plan) is q
     plans.clear()
     assert plans.get("a", lambda p: True, _Plan) is None and copy.deepcopy(plans).earn == 2
+
+
+class _OnDevice:
+    """What the training path looks at of a tensor before it picks a kernel, as if on a GPU."""
+
+    def __init__(self, shape, index=0, dtype=torch.float32):
+        self.shape, self.device, self.dtype, self.is_cuda = torch.Size(shape), torch.device("cuda", index), dtype, True
+
+    def dim(self):
+        return len(self.shape)
+
+    def element_size(self):
+        return self.dtype.itemsize
+
+    def data_ptr(self):
+        return 256
+
+
+@pytest.mark.parametrize("other", [None, "x", "comp", "gate", "ref", "patches"])
+def test_gated_decompress_in_one_launch_takes_operands_of_one_device(monkeypatch, other):
+    """Operands of two GPUs are refused by the operations that the launch stands for; the launch would read the other GPU's addresses."""
+    from vtpack_b200.layers import grained_sample as gs
+    monkeypatch.setattr(gs._GatedDecompress, "apply", lambda *a: "launched")
+    monkeypatch.setattr(gs, "_by_region", lambda *a: True)
+    t = {n: _OnDevice(shape, 1 if n == other else 0) for n, shape in
+         dict(x=(9, 64), comp=(9, 64), gate=(1, 2, 2, 3), ref=(1, 65, 64), patches=(9, 4)).items()}
+    t["patches"]._vtp_regions, t["patches"]._vtp_offsets = (None, None, [4, 2, 1], 4, 2, 2, 1), None
+    got = gs.gated_decompress(t["x"], t["comp"], t["gate"], t["ref"], t["patches"], 8, 1)
+    assert got == ("launched" if other is None else None)
+
+
+@pytest.mark.parametrize("index", [0, 1])
+def test_ragged_attention_as_one_node_takes_operands_of_one_device(monkeypatch, index):
+    from vtpack_b200.layers import sparse_ops
+    monkeypatch.setattr(sparse_ops._RaggedAttention, "apply", lambda *a: "launched")
+    got = sparse_ops.ragged_attention(_OnDevice((9, 64)), _OnDevice((2, 5, 128), index), torch.tensor([4, 5]), 1, 0.125, torch.nn.Dropout(0.0))
+    assert got == ("launched" if index == 0 else None)

@@ -190,6 +190,7 @@ def gated_decompress(x, comp, gate, ref, patches, width, num_extra_tokens):
     if (x.dim() != 2 or x.shape != comp.shape or x.shape[0] != patches.shape[0] or x.shape[1] != ref.shape[2]
             or not (x.dtype is comp.dtype is gate.dtype is ref.dtype) or x.dtype not in (torch.float32, torch.bfloat16)
             or not (x.is_cuda and comp.is_cuda and gate.is_cuda and ref.is_cuda)
+            or not x.device == comp.device == gate.device == ref.device == patches.device
             or not _by_region(regions, offsets, ref.shape, width, num_extra_tokens, x.dtype)
             or gate.shape != (ref.shape[0], regions[4], regions[5], len(regions[2]))
             or (x.data_ptr() | comp.data_ptr() | ref.data_ptr()) % 16 != 0

@@ -155,10 +155,11 @@ class _RaggedAttention(Function):
 
 def ragged_attention(q, kv, q_lengths, heads, scale, drop):
     """``_RaggedAttention`` where it is what the separate operations are: no dropout of its weights (`drop`, the module for it), rows of one
-    supported type on a GPU and lengths that add up; None elsewhere."""
+    supported type on one GPU and lengths that add up; None elsewhere."""
     if (type(drop) is not torch.nn.Dropout or drop.p != 0.0 or drop._forward_hooks or drop._forward_pre_hooks
-            or drop._backward_hooks or drop._backward_pre_hooks or not isinstance(scale, (int, float)) or q.dim() != 2 or kv.dim() != 3 or q.dtype is not kv.dtype
-            or q.dtype not in (torch.float32, torch.bfloat16) or not (q.is_cuda and kv.is_cuda) or kv.shape[2] != 2 * q.shape[1]
+            or drop._backward_hooks or drop._backward_pre_hooks or not isinstance(scale, (int, float))
+            or q.dim() != 2 or kv.dim() != 3 or q.dtype is not kv.dtype or q.dtype not in (torch.float32, torch.bfloat16)
+            or not (q.is_cuda and kv.is_cuda) or q.device != kv.device or kv.shape[2] != 2 * q.shape[1]
             or q.shape[1] % heads != 0 or q_lengths.shape != kv.shape[:1] or kv.shape[1] == 0
             or int(q_lengths.sum()) != q.shape[0]):
         return None
