@@ -45,10 +45,12 @@ scaled_softmax_kernel(const T* p, const T* x, T* y, long long rows, int n, float
             }
         };
         if constexpr (GRAD) {
+            // ds = scale * (p dp - p sum): with the products rounded alike inside the sum and in front of it, a probability near one cancels
+            // them (fp32, 16 scores of spread 64: relative error 1.57e-7, of p (dp - sum) 1.76e-7)
             float dot = 0.f;
-            each([&](int i, int c) { dot = fmaf(prob(i, c), val(i, c), dot); });
+            each([&](int i, int c) { dot += __fmul_rn(prob(i, c), val(i, c)); });
             dot = warp_sum(dot);
-            each([&](int i, int c) { yr[c] = from_f32<T>(scale * (prob(i, c) * (val(i, c) - dot))); });
+            each([&](int i, int c) { yr[c] = from_f32<T>(scale * fmaf(-prob(i, c), dot, __fmul_rn(prob(i, c), val(i, c)))); });
         } else {
             // (a scale below zero turns the order of the scores round, so the largest scaled one is looked for)
             float most = -INFINITY, sum = 0.f;
@@ -60,8 +62,8 @@ scaled_softmax_kernel(const T* p, const T* x, T* y, long long rows, int n, float
                 sum += e;
             });
             sum = warp_sum(sum);
-            const float inv = 1.f / sum;
-            each([&](int i, int c) { yr[c] = from_f32<T>((PER > 0 ? v[i] : expf(scale * to_f32(xr[c]) - most)) * inv); });
+            // (a quotient each: times the reciprocal of the sum is a rounding more, relative error 6.6e-8 -> 7.0e-8 in fp32 at 257 keys)
+            each([&](int i, int c) { yr[c] = from_f32<T>(__fdiv_rn(PER > 0 ? v[i] : expf(scale * to_f32(xr[c]) - most), sum)); });
         }
     }
 }
