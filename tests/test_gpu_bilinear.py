@@ -240,7 +240,7 @@ def test_bilinear_attention_of_many_queries_is_that_of_the_general_kernel(op, dt
     """Enough queries for several vectors a lane (one to three, whole or part-filled), as tiles of pixels with ragged edges, narrow maps and
     queries that are not the pixels, against the kernel for single channels (operands one element behind a 16-byte boundary), on maps with
     infinities and NaN off the way of all but a few queries.  Both sum the same terms in other orders: apart by two times n 2^-24 of the sum of
-    the terms' magnitudes (n terms), and a rounding of the result in bf16 (of every term of grad_input)."""
+    the terms' magnitudes (n terms), and a rounding of the result in bf16 (of every term that reaches a pixel of grad_input)."""
     P, lanes = 3, 2
     B = -(-16 * 32 * 148 // (lanes * G))
     g = torch.Generator(DEV).manual_seed(C + G)
@@ -270,12 +270,75 @@ def test_bilinear_attention_of_many_queries_is_that_of_the_general_kernel(op, dt
             ok = (x >= 0) & (x < W) & (y >= 0) & (y < H)
             at = (torch.arange(B, device=DEV)[:, None, None] * H + y) * W + x
             hits.index_add_(0, at[ok], torch.ones_like(at[ok], dtype=torch.float32))
-    most = float(hits.max())
+    hits = hits.view(B, H, W, 1)
     # two results on either side of a rounding boundary are a unit of the last place apart, 2^-7 of a bf16 number at most
     eps = 2.0 ** -7 if dtype is torch.bfloat16 else 0.0
-    for name, a, b, of, n in zip(("out", "grad_input", "grad_grid", "grad_weight"), got, want, size, (C + 4 * P + 8, most, C + 8, C + 4 * P + 8)):
-        bound = (2 * n * 2.0 ** -24 + (eps * (most + 1) if name == "grad_input" else 0)) * of + eps * torch.maximum(a.abs(), b.abs())
+    for name, a, b, of, n in zip(("out", "grad_input", "grad_grid", "grad_weight"), got, want, size, (C + 4 * P + 8, hits + 4, C + 8, C + 4 * P + 8)):
+        bound = (2 * n * 2.0 ** -24 + (eps * (hits + 1) if name == "grad_input" else 0)) * of + eps * torch.maximum(a.abs(), b.abs())
         assert bool(((a - b).abs() <= bound + 1e-30).all()), name
     t[0][0, 1, 1, 0], t[0][0, 2, 2, C - 1] = float("inf"), float("nan")
     for name, a, b in zip(("out", "grad_input", "grad_grid", "grad_weight"), run(t, 0), run(t, 1)):
         assert torch.equal(torch.isfinite(a), torch.isfinite(b)), name
+
+
+@pytest.mark.parametrize("mode", ["point", "channel"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,H,W,G,C", [(36, 29, 37, 29 * 37, 64), (2, 29, 37, 29 * 37, 64), (36, 29, 37, 1000, 136), (60, 40, 3, 120, 88),
+                                       (2, 7, 9, 60, 48)])
+def test_bilinear_attention_is_exact_where_its_sums_are(op, dtype, mode, B, H, W, G, C):
+    """Small whole numbers, and points half a pixel from the pixels: every product and sum is a multiple of 1/8 below 2^21, exact in fp32, and
+    every sum at a pixel below 32 (at most 100 terms of a quarter), exact in bf16 too.  So all four results are the float64 ones,
+    rounded once: a corner left out or weighted wrongly anywhere shows."""
+    P = 3
+    g = torch.Generator(DEV).manual_seed(C + G)
+
+    def whole(n, *shape):
+        return torch.randint(-n, n + 1, shape, device=DEV, generator=g).double()
+    ys, xs = torch.arange(G, device=DEV) // W % H, torch.arange(G, device=DEV) % W
+    point = mode == "point"
+    a = whole(3, B, H, W, C)
+    grid = torch.stack([xs, ys], -1)[None, :, None].double() + whole(3, B, G, P, 2) + 0.5
+    w, go = whole(1, B, G, P if point else C), whole(1, B, G, C if point else P)
+    a64, grid64, w64 = (t.clone().requires_grad_(True) for t in (a, grid, w))
+    base = grid64.detach().floor()
+    t = grid64 - base
+    val = 0.0
+    for dx in (0, 1):
+        for dy in (0, 1):
+            x, y = base[..., 0].long() + dx, base[..., 1].long() + dy
+            ok = (x >= 0) & (x < W) & (y >= 0) & (y < H)
+            at = (torch.arange(B, device=DEV)[:, None, None] * H + y.clamp(0, H - 1)) * W + x.clamp(0, W - 1)
+            share = (t[..., 0] if dx else 1 - t[..., 0]) * (t[..., 1] if dy else 1 - t[..., 1])
+            val = val + (a64.view(-1, C)[at] * ok[..., None]) * share[..., None]
+    y64 = (val * w64[..., None]).sum(2) if point else (val * w64[:, :, None]).sum(3)
+    want = (y64.detach(),) + torch.autograd.grad(y64, (a64, grid64, w64), go)
+    assert float(want[1].abs().max()) < 32
+    got = _run(op, a, grid, w, go, mode, dtype)
+    for name, x, y in zip(("out", "grad_input", "grad_grid", "grad_weight"), got, want):
+        assert torch.equal(x, y.to(dtype)), name
+
+
+@pytest.mark.parametrize("mode", ["point", "channel"])
+@pytest.mark.parametrize("dtype,C", [(torch.float32, 256), (torch.float32, 260), (torch.float32, 400), (torch.bfloat16, 512), (torch.bfloat16, 520),
+                                     (torch.bfloat16, 776)])
+def test_bilinear_attention_of_the_widest_rows(op, dtype, mode, C):
+    """The forward of rows of 64 and of more 16-byte vectors, which a warp walks through, against the kernel for single channels (operands one
+    element behind a 16-byte boundary): the same terms in other orders, apart by two times n 2^-24 of the sum of their magnitudes
+    and a rounding of the result in bf16."""
+    B, H, W, P = 3, 9, 11, 4
+    g = torch.Generator(DEV).manual_seed(C)
+    G = H * W
+    t = [torch.randn(B, H, W, C, device=DEV, generator=g), 12 * torch.rand(B, G, P, 2, device=DEV, generator=g) - 1,
+         torch.randn(B, G, P if mode == "point" else C, device=DEV, generator=g)]
+    t = [v.to(dtype) for v in t]
+
+    def run(t, shift):
+        moved = []
+        for v in t:
+            buf = torch.zeros(v.numel() + shift, dtype=dtype, device=DEV)
+            buf[shift:] = v.flatten()
+            moved.append(buf[shift:].view(v.shape))
+        return op(*moved, mode).double()
+    got, want, size = run(t, 0), run(t, 1), run([t[0].abs(), t[1], t[2].abs()], 1)
+    n, eps = C + 4 * P + 8, 2.0 ** -7 if dtype is torch.bfloat16 else 0.0
+    assert bool(((got - want).abs() <= 2 * n * 2.0 ** -24 * size + eps * torch.maximum(got.abs(), want.abs())).all())
