@@ -23,8 +23,10 @@ sys.path.insert(0, ROOT)
 import torch  # noqa: E402
 
 FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0}
-STAGES = ["router_gate", "patch_list", "pool_ln1", "q_proj", "kv_proj", "attention", "out_proj", "ln2", "fc1_gelu",
-          "fc2", "unpool_add"]
+# stages of a timed block and the event behind each; no event between q and kv or between fc1 and fc2, which would keep apart what the
+# forward runs as one launch
+STAGES = {"router_gate": 1, "patch_list": 2, "pool_ln1": 3, "q_kv_proj": 5, "attention": 6, "out_proj": 7, "ln2": 8, "mlp": 10,
+          "unpool_add": 11}
 # DRAM bytes (read + written) of one launch of the dominant kernel on the roofline's workload (the kv
 # projection at batch 256: M=65792, N=768, K=384), from the ncu capture summarised in
 # profiles/linear_tc_kv_projection_m65792_n768_k384.md, over the launch's operand and output bytes (below 1: part of the
@@ -193,7 +195,7 @@ def stage_profile(model, batch, device, iters, pk, ms_per_step, tokens=None, for
     between its launches.  Every stage then sits between two event records, which keeps a launch from
     queueing behind the one in front of it: these are upper bounds of what a kernel costs inside the replayed
     graph.  `ms_in_step_est` scales them so that depth x block + the front/back launches equals the measured
-    step.  Returns (rows, the five Linear launches together, block summary)."""
+    step.  Returns (rows, the Linear launches together, block summary)."""
     import ctypes
     from vtpack_b200 import _lib
     from vtpack_b200.models.dge.deit_dge import _pack_block
@@ -214,14 +216,15 @@ def stage_profile(model, batch, device, iters, pk, ms_per_step, tokens=None, for
     nbytes = lib.vtp_block_workspace_bytes(ctypes.byref(s))
     ws = scratch(device, nbytes)
     counts = torch.empty(batch, dtype=torch.int32, device=device)
-    n_ev = len(STAGES) + 1
+    n_ev = 12
+    ends = list(STAGES.values())
     evs = [[torch.cuda.Event(enable_timing=True) for _ in range(n_ev)] for _ in range(iters)]
     stream = torch.cuda.current_stream(device)
     for it in range(iters + 2):
         row = evs[max(it - 2, 0)]
         for ev in row:
             ev.record(stream)            # creates the underlying cudaEvent_t
-        arr = (ctypes.c_void_p * n_ev)(*[ev.cuda_event for ev in row])
+        arr = (ctypes.c_void_p * n_ev)(*[ev.cuda_event if i in (0, *ends) else None for i, ev in enumerate(row)])
         _lib.check(lib.vtp_dge_block_forward_timed(ctypes.byref(s), ctypes.byref(w), x.data_ptr(), out.data_ptr(),
                                                    forced.data_ptr() if forced is not None else None,
                                                    counts.data_ptr(), ws.data_ptr(), nbytes, arr, n_ev,
@@ -233,16 +236,16 @@ def stage_profile(model, batch, device, iters, pk, ms_per_step, tokens=None, for
     else:
         grains = region_grains(x, blk._pack.tensors["gate_w"], blk._pack.tensors["gate_b"], G, device)
         fine = float((grains == 0).float().mean().item())
-    ms = [sum(evs[i][j].elapsed_time(evs[i][j + 1]) for i in range(iters)) / iters for j in range(len(STAGES))]
+    ms = [sum(evs[i][a].elapsed_time(evs[i][b]) for i in range(iters)) / iters for a, b in zip([0, *ends], ends)]
     BN, H, HW = batch * N, 4 * C, G * G
     work = {   # (kind, algorithmic bytes or flops)
         # LayerNorm is folded into the GEMM epilogues on the bf16 path: the pool writes comp rows
         # and 8 bytes of statistics per row; there is no LN2 kernel (its slot measures ~0)
         "router_gate": ("hbm", batch * (N - 1) * C * e), "patch_list": ("hbm", batch * 16 * 12),
-        "pool_ln1": ("hbm", (BN + L) * C * e + (BN + 2 * L) * 8), "q_proj": ("tensor", 2 * L * C * C),
-        "kv_proj": ("tensor", 4 * BN * C * C), "attention": ("tensor", 4 * L * N * C),
+        "pool_ln1": ("hbm", (BN + L) * C * e + (BN + 2 * L) * 8),
+        "q_kv_proj": ("tensor", 2 * L * C * C + 4 * BN * C * C), "attention": ("tensor", 4 * L * N * C),
         "out_proj": ("tensor", 2 * L * C * C), "ln2": ("hbm", 0),
-        "fc1_gelu": ("tensor", 2 * L * C * H), "fc2": ("tensor", 2 * L * C * H),
+        "mlp": ("tensor", 4 * L * C * H),
         "unpool_add": ("hbm", unpool_rows(batch, HW, L, fine) * C * e),
     }
     depth = len(model.blocks)
@@ -265,12 +268,12 @@ def stage_profile(model, batch, device, iters, pk, ms_per_step, tokens=None, for
         if name in ("router_gate", "patch_list"):
             row["note"] = "first block of a forward only"
         rows.append(row)
-    gemm = [r for r in rows if r["kernel"] in ("q_proj", "kv_proj", "out_proj", "fc1_gelu", "fc2")]
+    gemm = [r for r in rows if r["kernel"] in ("q_kv_proj", "out_proj", "mlp")]
     gemm_ms = sum(r["ms_event_bracketed"] for r in gemm)
     gemm_flops = sum(work[r["kernel"]][1] for r in gemm)
     tf_bracketed = gemm_flops / (gemm_ms * 1e-3) / 1e12
     tf_step = gemm_flops / (gemm_ms * scale * 1e-3) / 1e12
-    all_linear = {"launches": "q, kv, out, fc1, fc2 projections of one block", "gflop": round(gemm_flops / 1e9, 1),
+    all_linear = {"launches": "q + kv, out projection, fc1 + fc2 of one block", "gflop": round(gemm_flops / 1e9, 1),
                   "achieved_event_bracketed": round(tf_bracketed, 1),
                   "frac_event_bracketed": round(tf_bracketed / pk["bf16_tflops_sustained"], 3),
                   "achieved_in_step_est": round(tf_step, 1),
@@ -992,10 +995,11 @@ def main():
             line["roofline"]["frac_all_launches"] = all_linear["frac_in_step_est"]
             line["kernels"] = rows
             line["kernels_note"] = ("one block (the middle one's weights and the tokens it received in this forward), "
-                                    "q and kv projections, and fc1 and fc2, as separate launches (the forward has one for each two); "
+                                    "launches as in the forward but for the unpool, which leaves no next block's gate here; "
                                     "ms_event_bracketed: every stage sits between two event records, which keeps the "
                                     "next launch from queueing behind the running one: an upper bound. ms_in_step_est "
-                                    "= that share scaled so that depth x block + front/back equals ms_per_step")
+                                    "= that share scaled so that depth x block + front/back equals ms_per_step (the blocks differ in queries: "
+                                    "where this one has more than the mean, its estimates are too short by as much)")
             line["block"] = extra
         if world == 1 and not args.no_cpu_baseline:
             rate, ms, cores = cpu_reference_rate(args.model, args.cpu_batch, 3, 1, S, args.gate_skew)

@@ -445,6 +445,8 @@ int vtp_dge_blocks_forward(const vtp_dge_shape* s, const vtp_block_weights* w, i
  * null entries skipped) on the stream after stage i:
  *   0 start, 1 router gate, 2 patch list, 3 pool+LN1, 4 q proj, 5 kv proj, 6 attention,
  *   7 out proj+residual, 8 LN2, 9 fc1+GELU, 10 fc2+residual, 11 unpool+residual.
+ * vtp_dge_block_forward may run 4 and 5, and 9 and 10, as one launch each; an event between the two keeps them
+ * apart, and without one (events[4], events[9] null) the launches are those of vtp_dge_block_forward.
  * For per-kernel timing; the reference has no counterpart (it logs wall-clock time per
  * iteration only, vtpack/engine/utils.py:128-172).
  */

@@ -28,4 +28,13 @@ def random_indices(B, Hr, Wr, n_splits, seed):
     return torch.randint(0, n_splits, (B, Hr, Wr), generator=g)
 
 
-__all__ = ["O", "rel_err", "load_block", "strip_col2_of_extra", "random_indices"]
+def kernels_of(fn):
+    """Names of the GPU kernels that fn() launches, in order."""
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        fn()
+        torch.cuda.synchronize()
+    events = [e for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA and not e.name.startswith(("Mem", "mem"))]
+    return [e.name for e in sorted(events, key=lambda e: e.time_range.start)]
+
+
+__all__ = ["O", "rel_err", "load_block", "strip_col2_of_extra", "random_indices", "kernels_of"]

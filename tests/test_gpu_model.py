@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 import torch
 
-from tests.gpu_util import O, rel_err
+from tests.gpu_util import O, kernels_of, rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -985,8 +985,6 @@ def test_mlp_in_one_launch(C, B, grid, sr, ratio, fine):
     """fc1 and fc2 as one launch, which large batches take, and as two, which is how a block with events between its stages runs: the
     same bits.  Few rows, some rounds of 256 rows for every pair of CTAs, a last round whose rows are two pairs' each (384: 2125 and
     33410 rows), rows that end inside a warp's, and a wider hidden layer."""
-    import ctypes
-
     from vtpack_b200 import _lib
     from vtpack_b200.models.dge import deit_dge, pvt_dge
     torch.manual_seed(C + B)
@@ -1005,24 +1003,75 @@ def test_mlp_in_one_launch(C, B, grid, sr, ratio, fine):
     gate[..., 0] = torch.where(torch.rand(gate.shape[:3], device=DEV) < fine, 9.0, -9.0)
     if fine == 0.0:
         gate[..., 2] = 9.0
-    got = blk(x, grid, grid, forced_gate=gate) if sr > 1 else blk(x, forced_gate=gate)
+
+    def plain():
+        return blk(x, grid, grid, forced_gate=gate) if sr > 1 else blk(x, forced_gate=gate)
+    got = plain()
     s = deit_dge._shape_struct(torch.bfloat16, B, grid, grid, extra, C, C // 64, ratio * C, [4, 2, 1], blk.norm1.eps, 0, blk.attn.scale)
     if sr > 1:
         s.sr_ratio, s.sr_eps = sr, float(blk.attn.norm.eps)
-    w, lib = (pvt_dge if sr > 1 else deit_dge)._pack_block(blk, torch.bfloat16), _lib.lib()
-    n = lib.vtp_block_workspace_bytes(ctypes.byref(s))
-    ws, out = torch.empty(n, dtype=torch.uint8, device=DEV), torch.empty_like(x)
-    counts = torch.empty(B, dtype=torch.int32, device=DEV)
-    events = [torch.cuda.Event(enable_timing=True) for _ in range(12)]
-    for e in events:
-        e.record()
-    arr = (ctypes.c_void_p * 12)(*[e.cuda_event for e in events])
-    _lib.check(lib.vtp_dge_block_forward_timed(ctypes.byref(s), ctypes.byref(w), x.data_ptr(), out.data_ptr(), gate.data_ptr(),
-                                               counts.data_ptr(), ws.data_ptr(), n, arr, 12,
-                                               torch.cuda.current_stream().cuda_stream))
+    run, out = _timed_block(s, (pvt_dge if sr > 1 else deit_dge)._pack_block(blk, torch.bfloat16), x, gate)
+    apart = range(12)
+    run(apart)
     torch.cuda.synchronize()
     assert _lib.device_status() == 0
     assert bool(got.isfinite().all()) and torch.equal(got, out)
+    # each side is what it is taken for
+    assert sum("mlp_tc_kernel" in n for n in kernels_of(plain)) == 1
+    assert not any("mlp_tc_kernel" in n for n in kernels_of(lambda: run(apart)))
+
+
+def _timed_block(s, w, x, gate):
+    """A block with events behind the stages of a list: (a function of that list, its output)."""
+    import ctypes
+
+    from vtpack_b200 import _lib
+    lib = _lib.lib()
+    n = lib.vtp_block_workspace_bytes(ctypes.byref(s))
+    ws, out = torch.empty(n, dtype=torch.uint8, device=DEV), torch.empty_like(x)
+    counts = torch.empty(x.shape[0], dtype=torch.int32, device=DEV)
+    events = [torch.cuda.Event(enable_timing=True) for _ in range(12)]
+    for e in events:
+        e.record()
+
+    def run(stages):
+        arr = (ctypes.c_void_p * 12)(*[e.cuda_event if i in stages else None for i, e in enumerate(events)])
+        _lib.check(lib.vtp_dge_block_forward_timed(ctypes.byref(s), ctypes.byref(w), x.data_ptr(), out.data_ptr(), gate.data_ptr(),
+                                                   counts.data_ptr(), ws.data_ptr(), n, arr, 12,
+                                                   torch.cuda.current_stream().cuda_stream))
+    return run, out
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("C,B,sr", [(384, 125, 1), (192, 3, 1), (64, 5, 8), (64, 8, 8)])
+def test_timed_block_without_events_inside_a_pair_runs_what_the_block_runs(dtype, C, B, sr):
+    """Stages 4 and 5 (q and kv) and 9 and 10 (fc1 and fc2) share launches in a block's forward; timed with no event between the two the
+    block launches the same kernels and gives the same bits, and the events behind the pairs are recorded."""
+    from vtpack_b200 import _lib
+    from vtpack_b200.models.dge import deit_dge, pvt_dge
+    torch.manual_seed(C + B)
+    grid, extra = (64, 0) if sr > 1 else (16, 1)
+    module = pvt_dge if sr > 1 else deit_dge
+    kw = dict(sr_ratio=sr) if sr > 1 else {}
+    blk = module.Block(C, C // 64, mlp_ratio=8 if sr > 1 else 4, qkv_bias=True, split_sizes=[4, 2, 1], **kw).eval().to(device=DEV, dtype=dtype)
+    x = torch.randn(B, grid * grid + extra, C, device=DEV).to(dtype)
+    gate = torch.randn(B, grid // 4, grid // 4, 3, device=DEV)
+
+    def plain():
+        return blk(x, grid, grid, forced_gate=gate) if sr > 1 else blk(x, forced_gate=gate)
+    s = deit_dge._shape_struct(dtype, B, grid, grid, extra, C, C // 64, (8 if sr > 1 else 4) * C, [4, 2, 1], blk.norm1.eps, 0, blk.attn.scale)
+    if sr > 1:
+        s.sr_ratio, s.sr_eps = sr, float(blk.attn.norm.eps)
+    run, out = _timed_block(s, module._pack_block(blk, dtype), x, gate)
+    together = [i for i in range(12) if i not in (4, 9)]
+    got = plain()
+    run(together)
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0 and torch.equal(got, out)
+    names = kernels_of(plain)
+    assert kernels_of(lambda: run(together)) == names
+    apart = kernels_of(lambda: run(range(12)))
+    assert len(apart) == len(names) + 1 + any("mlp_tc_kernel" in n for n in names)
 
 
 @pytest.mark.parametrize("C,G,B,extra,sr", [(64, 20, 49, 0, 1), (128, 12, 133, 1, 1), (192, 20, 49, 1, 1), (320, 20, 49, 1, 1), (384, 28, 25, 1, 1), (384, 4, 1187, 0, 1),

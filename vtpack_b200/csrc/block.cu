@@ -143,6 +143,8 @@ struct StageMarks {
     void* const* events = nullptr;
     int n = 0;
     cudaStream_t st = nullptr;
+    // An event is wanted behind stage i alone, so it cannot share a launch with stage i + 1.
+    bool apart(int i) const { return events && i < n && events[i]; }
     int mark(int i) const {
         if (!events || i >= n || !events[i]) return VTP_OK;
         const cudaError_t e = cudaEventRecord(static_cast<cudaEvent_t>(events[i]), st);
@@ -322,7 +324,7 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
     // The two projections do not depend on each other: one launch, the q tiles fill the kv tail.  Behind a reduction as well, where q
     // waits for the keys although it need not (apart / together: PVT-tiny, 3 / 33 / 96 images, 460 / 803 / 1493 us and 440 / 791 / 1470;
     // PVT-small, 1 and 96 images, 783 / 2704 and 751 / 2657; in fp32, 1 image, 1228 and 1149).
-    const bool pair_bf16 = fold_q && !marks.events && linear_pair_supported(lkv, lq), pair_f32 = terms && !marks.events;
+    const bool pair_bf16 = fold_q && !marks.apart(4) && linear_pair_supported(lkv, lq), pair_f32 = terms && !marks.apart(4);
     if (!pair_bf16 && !pair_f32 && ((rc = run_linear(lq, b.q_wt, terms_attn)) || (rc = marks.mark(4)))) return rc;
 
     if (reduce) {
@@ -347,9 +349,8 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
         rc = linear_f32_terms_pair(lkv, lq, st);
     } else {
         rc = run_linear(lkv, b.kv_wt, terms_attn);
-        if (!rc) rc = marks.mark(5);
     }
-    if (rc) return rc;
+    if (rc || (rc = marks.mark(5))) return rc;
 
     AttnArgs at;
     const long long e = (long long)elem_size(s.dtype);
@@ -384,12 +385,13 @@ static int block_forward(const vtp_dge_shape& s, const vtp_block_weights& w, con
     LinearArgs l2;   // q2 = q1 + hid W2^T + b   (into the q-projection buffer, dead by now)
     l2.a = b.hid; l2.lda = s.hidden; l2.w = w.fc2_w; l2.bias = w.fc2_b; l2.res = b.q1; l2.ldr = C; l2.y = b.qp;
     l2.ldy = C; l2.dtype = s.dtype; l2.m_max = rows; l2.m_dev = L_dev; l2.N = C; l2.K = s.hidden; l2.flags = kflag;
-    if (!marks.events && mlp_tcgen05_supported(l1, l2) && mlp_tcgen05_pays(l1)) {
-        if ((rc = mlp_tcgen05(l1, l2, st))) return rc;
-    } else if ((rc = run_linear(l1, b.fc1_wt, true)) || (rc = marks.mark(9)) || (rc = run_linear(l2, b.fc2_wt, false)) ||
-               (rc = marks.mark(10))) {
-        return rc;
+    if (!marks.apart(9) && mlp_tcgen05_supported(l1, l2) && mlp_tcgen05_pays(l1)) {
+        rc = mlp_tcgen05(l1, l2, st);
+    } else {
+        if ((rc = run_linear(l1, b.fc1_wt, true)) || (rc = marks.mark(9))) return rc;
+        rc = run_linear(l2, b.fc2_wt, false);
     }
+    if (rc || (rc = marks.mark(10))) return rc;
 
     if (by_region) {
         RegionUnpoolArgs ua;
