@@ -87,25 +87,73 @@ def test_pair_producers_wait_for_every_last_commit(stages):
         assert waited == set(last)
 
 
-@pytest.mark.parametrize("kernel", sorted(WAITING))
-def test_lanes_that_wait_together_go_on_together(kernel):
-    """A wait gives up after about a second, lane by lane.  Where a whole warp waits, warp-wide instructions follow, which a lane
-    that went to unwind never reaches: such waits are decided by a vote, or no lane leaves.  Others are those of one elected thread."""
-    text = body(kernel, source(WAITING[kernel]))
-    elected = []
+def elected_spans(text):
+    """What one elected thread runs of a kernel."""
+    spans = []
     for m in re.finditer(r"if \((rank == 0 && )?elect_one\(\)\) \{", text):
         depth, i = 1, m.end()
         while depth:
             depth += {"{": 1, "}": -1}.get(text[i], 0)
             i += 1
-        elected.append((m.end(), i))
+        spans.append((m.end(), i))
+    return spans
+
+
+def test_the_rings_of_the_mlp_are_one_thread_s():
+    """The waits of the rings of W stand in their methods: each is a thread's own, and every call of those methods is one elected thread's."""
+    text = source("mlp_tc.cu")
+    methods = body("WRing", text[:text.index("struct MlpConf")].replace("struct WRing {", "struct WRing( {"))
+    waits = re.findall(r"\bmbar_(\w*wait\w*)\(", methods)
+    assert len(waits) >= 4 and set(waits) == {"wait_a", "try_wait_a"}
+    kernel = body("mlp_tc_kernel", text)
+    spans = elected_spans(kernel)
+    calls = [m.start() for m in re.finditer(r"\bw[12]?\.(load|drain|ready|mma|done)\(", kernel)]
+    assert len(calls) >= 10 and all(any(a <= at < b for a, b in spans) for at in calls)
+
+
+@pytest.mark.parametrize("stages", range(1, 9))
+def test_ring_loader_waits_for_every_last_commit(stages):
+    """The same for the rings of the one-launch MLP: one loader, which has seen the commits of all but the last fill of every stage."""
+    drain = body("drain", source("mlp_tc.cu"))
+    assert "d = n > (uint32_t)STAGES ? n - STAGES : 0; d < n; ++d" in drain
+    wait = re.search(r"mbar_wait_a\(empty \+ 8 \* \((.*?)\), (.*?), c\.abort_flag", drain)
+    stage, parity = (e.replace("/", "//") for e in wait.groups())
+    for n in range(1, 6 * stages):
+        seen = max(0, n - stages)                              # commits of the fills in front of these
+        for d in range(max(0, n - stages), n):
+            names = dict(d=d, STAGES=stages)
+            assert eval(stage, {}, names) == d % stages
+            phases = len(range(d % stages, seen, stages))
+            assert (phases - 1) & 1 != eval(parity, {}, names)          # passes on no older commit
+            assert phases & 1 == eval(parity, {}, names)                # and on this fill's
+            seen = d + 1
+
+
+@pytest.mark.parametrize("stages", [6, 8])
+def test_shared_tile_commits_only_what_a_producer_waits_for(stages):
+    """linear_tc_pair_kernel has no drain: a stage is committed only where a later fill waits for it, in both CTAs."""
+    text = body("linear_tc_pair_kernel", source("linear_tc.cu"))
+    commits = re.findall(r"if \((.*?)\) umma_commit_a<2>\(empty_a", text)
+    waits = re.findall(r"if \((.*?) && !mbar_wait_a\(empty_a \+ 8 \* s, \(\(i / STAGES\) & 1\) \^ 1", text)
+    assert commits == ["i + STAGES < n_stages"] and waits == ["i >= STAGES"]
+    for n in range(1, 6 * stages):
+        committed = {i for i in range(n) if i + stages < n}
+        assert committed == {i - stages for i in range(n) if i >= stages}
+
+
+@pytest.mark.parametrize("kernel", sorted(WAITING))
+def test_lanes_that_wait_together_go_on_together(kernel):
+    """A wait gives up after about a second, lane by lane.  Where a whole warp waits, warp-wide instructions follow, which a lane
+    that went to unwind never reaches: such waits are decided by a vote, or no lane leaves.  Others are those of one elected thread."""
+    text = body(kernel, source(WAITING[kernel]))
+    elected = elected_spans(text)
     waits = [(m.start(), m.group(1)) for m in re.finditer(r"\bmbar_(\w*wait\w*)\(", text)]
     assert len(waits) >= 3
     for at, name in waits:
         one = any(a <= at < b for a, b in elected)
         # (the warps that split fp32 operands have only __syncwarp behind it, which a lane that leaves still runs as often)
         runs_out = "num_kb - kb; n > 0; --n) __syncwarp();" in text[at:at + 400]
-        assert name in (("wait", "wait_a") if one or runs_out else ("wait_warp", "wait_cluster_warp")), (name, text[at:at + 80])
+        assert name in (("wait", "wait_a", "try_wait_a") if one or runs_out else ("wait_warp", "wait_cluster_warp")), (name, text[at:at + 80])
 
 
 def test_no_mma_is_issued_in_front_of_the_fence_behind_a_wait():

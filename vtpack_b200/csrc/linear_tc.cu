@@ -826,10 +826,8 @@ linear_tc_pair_kernel(const __grid_constant__ SmallLaunch L, int K, int* status)
     const uint32_t tmem_base = *tmem_slot;
     const bool known_void = lead_word<2>(void_s) != 0;
     pdl_begin();
-    // a pair that starts when others have ended looks first whether its rows exist
-    const bool none = (int)blockIdx.x >= L.at_once && P.m_dev && m0 >= *reinterpret_cast<const volatile int32_t*>(P.m_dev);
 
-    if (known_void || none) {
+    if (known_void) {
     } else if (warp < PRODUCERS) {
         if (elect_one()) {
             for (int i = warp; i < n_stages; i += PRODUCERS) {
@@ -859,7 +857,7 @@ linear_tc_pair_kernel(const __grid_constant__ SmallLaunch L, int K, int* status)
                 tc_fence_after_sync();
                 const bool wrap = s + 1 == STAGES;
                 // (a look behind the MMAs would wait until the tensor core has taken them)
-                peeked = mbar_passed_a(wrap ? full_a : full_a + 8 * (s + 1), wrap ? ph ^ 1 : ph);
+                peeked = mbar_try_wait_a(wrap ? full_a : full_a + 8 * (s + 1), wrap ? ph ^ 1 : ph);
                 const uint32_t a = desc0 + s * (S::STAGE >> 4), b = a + (2 * S::A_BYTES >> 4);
 #pragma unroll
                 for (int k = 0; k < 2 * TBK / 16; ++k) {
@@ -1196,8 +1194,7 @@ static int launch_pair(const LinearArgs& p, cudaStream_t st) {
     fill_scalars(L.p[0], p, false, BN);
     L.ta[1] = L.ta[0]; L.tw[1] = L.tw[0]; L.p[1] = L.p[0];
     const int grid = 2 * (int)small_tiles(p, BN);
-    L.grid0 = grid;
-    L.at_once = sm_count() / 2 * 2;
+    L.grid0 = L.at_once = grid;          // (all of them run at once: long_reduction_pairs)
     auto kern = linear_tc_pair_kernel<BN, EPI>;
     static bool reserved[64] = {};   // per instantiation and device
     if (int rc = reserve_smem(kern, S::TOTAL, reserved)) return rc;

@@ -65,7 +65,7 @@ struct WRing {
         tc_fence_after_sync();               // (also for the waits in front: accumulators that have been read, operands)
         if (RESIDENT && n >= (uint32_t)STAGES) return true;
         const bool wrap = s + 1 == STAGES;
-        peeked = mbar_passed_a(wrap ? full : full + 8 * (s + 1), wrap ? ph ^ 1 : ph);
+        peeked = mbar_try_wait_a(wrap ? full : full + 8 * (s + 1), wrap ? ph ^ 1 : ph);
         return true;
     }
     // One box against 64 columns of A

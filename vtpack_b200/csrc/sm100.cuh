@@ -45,9 +45,6 @@ __device__ __forceinline__ bool mbar_try_wait_a(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
-// Whether the phase has completed, as far as one look tells (false: wait).
-__device__ __forceinline__ bool mbar_passed_a(uint32_t bar, uint32_t parity) { return mbar_try_wait_a(bar, parity); }
-
 // True in one lane of a converged warp.  Unlike with `lane == 0` the compiler then knows that one thread runs what
 // follows: a TMA load issues in about 10 cycles behind another one instead of 65, a tcgen05.commit in 45 fewer.
 __device__ __forceinline__ bool elect_one() {
@@ -407,7 +404,7 @@ __device__ __forceinline__ void tmem_ld_16x256b_x8(uint32_t taddr, uint32_t (&r)
         : "r"(taddr)
         : "memory");
 }
-// ... x 32 columns, x 16 columns.
+// ... x 32 columns.
 __device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
@@ -416,12 +413,6 @@ __device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, uint32_t (&r)
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr)
         : "memory");
-}
-__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr)
-                 : "memory");
 }
 // Four 8 x 8 matrices of 16-bit elements between shared memory and that layout: thread t gives the address of row t % 8 of
 // matrix t / 8 and holds columns 2 (t % 4), + 1 of row t / 4 of matrix i in r[i].
