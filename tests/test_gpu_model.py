@@ -1102,3 +1102,31 @@ def test_pool_and_unpool_of_many_regions_are_those_of_few(C, G, B, extra, sr):
         assert torch.equal(few, many[part]) and all(torch.equal(p, q[part]) for p, q in zip(c, counts))
     R = (G // 4) ** 2
     assert B * extra + B * R < int(counts[1].sum()) < B * extra + 16 * B * R and _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("C,G,B,extra,sr", [(64, 20, 49, 0, 1), (128, 12, 133, 1, 1), (192, 20, 49, 1, 1), (320, 20, 49, 1, 1), (384, 28, 25, 1, 1),
+                                            (64, 20, 49, 0, 4), (320, 20, 49, 0, 2)])
+def test_pool_of_many_regions_leaves_the_statistics_itself(C, G, B, extra, sr):
+    """With the gate given nothing has left the tokens' statistics, so the pool does: a warp a region for many regions, a block a region
+    for few, the same bits of a whole block."""
+    from functools import partial
+
+    from vtpack_b200 import _lib
+    from vtpack_b200.models.dge import deit_dge, pvt_dge
+    torch.manual_seed(C + G)
+    kw = dict(mlp_ratio=2, qkv_bias=True, norm_layer=partial(torch.nn.LayerNorm, eps=1e-6), split_sizes=[4, 2, 1])
+    blk = pvt_dge.Block(C, C // 64, sr_ratio=sr, **kw) if extra == 0 else deit_dge.Block(C, C // 64, **kw)
+    blk = blk.eval().to(device=DEV, dtype=torch.bfloat16)
+    x = (torch.randn(B, G * G + extra, C, device=DEV) * torch.rand(B, G * G + extra, 1, device=DEV) + 0.5).bfloat16()
+    gate = torch.randn(B, G // 4, G // 4, 3, device=DEV)
+    assert B * (G // 4) ** 2 >= 8 * torch.cuda.get_device_properties(0).multi_processor_count
+
+    def run(part):
+        args = (x[part].contiguous(), G, G) if extra == 0 else (x[part].contiguous(),)
+        return blk(*args, forced_gate=gate[part].contiguous())
+    many = run(slice(0, B))
+    for part in (slice(0, 1), slice(1, 12), slice(B - 5, B)):
+        assert torch.equal(run(part), many[part])
+    names = kernels_of(lambda: run(slice(0, B)))
+    assert any("pool_warp_kernel" in n and "unpool" not in n for n in names) and any("unpool_warp_kernel" in n for n in names)
+    assert not any("warp_kernel" in n for n in kernels_of(lambda: run(slice(0, 1)))) and _lib.device_status() == 0
