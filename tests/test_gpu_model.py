@@ -1075,11 +1075,12 @@ def test_timed_block_without_events_inside_a_pair_runs_what_the_block_runs(dtype
 
 
 @pytest.mark.parametrize("C,G,B,extra,sr", [(64, 20, 49, 0, 1), (128, 12, 133, 1, 1), (192, 20, 49, 1, 1), (320, 20, 49, 1, 1), (384, 28, 25, 1, 1), (384, 4, 1187, 0, 1),
-                                            (64, 20, 49, 0, 4), (128, 20, 49, 0, 4), (320, 20, 49, 0, 2)])
+                                            (64, 20, 49, 0, 4), (128, 20, 49, 0, 4), (320, 20, 49, 0, 2), (320, 12, 215, 0, 2),
+                                            (320, 12, 301, 0, 2)])
 def test_pool_and_unpool_of_many_regions_are_those_of_few(C, G, B, extra, sr):
     """From eight regions a SM on a warp pools and unpools a region, with fewer a block: the same tokens, statistics, rows of a spatial reduction and
     next decisions, so the same bits after two blocks that chain, at every grain; region counts that leave warps of the last block idle, with and
-    without extra tokens."""
+    without extra tokens, and (C = 320) one, one and a bit and one and a half rounds of the pool's blocks, of which the second has a block pool a region."""
     from functools import partial
 
     from vtpack_b200 import _lib
@@ -1101,6 +1102,9 @@ def test_pool_and_unpool_of_many_regions_are_those_of_few(C, G, B, extra, sr):
         few, c = run(x[part])
         assert torch.equal(few, many[part]) and all(torch.equal(p, q[part]) for p, q in zip(c, counts))
     R = (G // 4) ** 2
+    names = kernels_of(lambda: pvt_dge.stage_forward(blocks, x, G, G))
+    assert sum("unpool_warp_kernel" in n for n in names) == 2
+    assert sum("pool_warp_kernel" in n and "unpool" not in n for n in names) == (0 if B == 215 else 2)
     assert B * extra + B * R < int(counts[1].sum()) < B * extra + 16 * B * R and _lib.device_status() == 0
 
 

@@ -1235,9 +1235,15 @@ static void launch_pool_t(const RegionPoolArgs& a, cudaStream_t st) {
         }
     }
     if constexpr (sizeof(T) == 2 && G <= 16 && G * CPL <= 48) {
-        // (eight regions a SM: the line of the unpool, which see; both forms write the same)
-        if (a.stats_q && a.g.l_max == 0 && a.g.B * R >= 8 * sm_count()) {
-            const int blocks = ceil_div(a.g.B * R, PW_WARPS) + ceil_div(a.g.B * a.g.num_extra, PW_WARPS * L::GROUPS);
+        // Eight regions a SM: the line of the unpool, which see; both forms write the same.  But for the rows of a convolution where channels are
+        // many (three blocks a SM, each as long as a round of all) not while a second round is less than two fifths full.  Four blocks in a
+        // chain, C = 320, sr = 2, us a block at three grain mixes, block | warp: 96 images (0.9 rounds) 101 106 133 | 96 103 132, 112 (1.01) 111 117
+        // 151 | 111 117 151, 128 (1.2) 117 123 159 | 120 126 161, 144 (1.3) 125 131 169 | 125 132 169, 160 (1.4) 131 139 180 | 131 139 180, 192
+        // (1.7) 142 161 212 | 138 159 213; a block with its gate given, 128 images, 109 116 154 | 114 121 157.
+        const int blocks = ceil_div(a.g.B * R, PW_WARPS) + ceil_div(a.g.B * a.g.num_extra, PW_WARPS * L::GROUPS);
+        const int round = pool_warp_ctas<G, CPL, POOL_COLS>() * sm_count();
+        const bool short_round = a.sr > 1 && G * CPL >= 40 && blocks > round && 5 * blocks < 7 * round;
+        if (a.stats_q && a.g.l_max == 0 && a.g.B * R >= 8 * sm_count() && !short_round) {
             auto kern = a.sr > 1 ? pool_warp_kernel<G, CPL, POOL_COLS> : pool_warp_kernel<G, CPL, POOL_STATS>;
             launch_chain(kern, dim3(blocks), dim3(PW_WARPS * 32), 0, st, (const T*)a.x, a.g, a.idx, a.region_first, a.offsets, a.counts,
                 a.offsets_out, a.region_first_out, a.counts_next, a.sp, (T*)a.comp, a.stats_x, a.stats_q, a.stats_acc,
