@@ -534,7 +534,9 @@ mlp_tc_kernel(const __grid_constant__ MlpLaunch L, int* status) {
 
 // ------------------------------------------------------------------------------ host
 
-// fc1 (GELU; from C = 192 on with its LayerNorm folded) and fc2 back onto rows of fc1's width, as one launch.
+// fc1 (GELU; from C = 192 on with its LayerNorm folded) and fc2 back onto rows of fc1's width, as one launch.  The widths are those of this
+// framework's models: 256 would fit and no model has it; 512 and 768 do not, as the output's columns (512 at most, and fc1's beside them: C <= 384)
+// stand in tensor memory.
 bool mlp_tcgen05_supported(const LinearArgs& f, const LinearArgs& p) {
     const bool fold = f.K == 192 || f.K == 320 || f.K == 384, rows = f.K == 64 || f.K == 128;
     return f.dtype == VTP_BF16 && p.dtype == VTP_BF16 && f.flags == VTP_FLAG_GELU && p.flags == 0 && p.N == f.K && p.K == f.N &&
@@ -544,8 +546,11 @@ bool mlp_tcgen05_supported(const LinearArgs& f, const LinearArgs& p) {
 }
 
 // From how many rows on (those the host has to allow for; a third to a half of them are valid where a router picks) one launch is shorter
-// than two: it takes its time by rounds of 256 rows a pair, 18,944 at a time, however few are valid.  Blocks, us, two launches / one, at a
-// tenth / quarter / two fifths / all of the regions on the finest grain:
+// than two: it takes its time by rounds of 256 rows a pair, 18,944 at a time, however few are valid.  The lines are for a quarter of the regions on the
+// finest grain and more (random weights give a quarter, and a budget of half of the operations two fifths); that mixes without any lose up to 5 % of a block
+// up to about twice a line, and those with a tenth up to 3 %, is accepted, as only the device knows the mix.  Blocks, us, two launches / one, at a
+// tenth / quarter / two fifths / all of the regions on the finest grain (without any: C = 128, 32,768 rows 58/61, C = 192, 20,560 54/56,
+// C = 320, 24,576 87/91, 49,152 131/133, C = 384, 32,125 105/110, 49,344 137/139, 65,792 180/176):
 //   C = 64    16,384 rows 55/55 56/56 56/56 58/56, 32,768 62/61 65/63 65/62 73/71, 393,216 203/195 241/228 280/264 422/388
 //   C = 128   24,576 61/63 63/64 66/65 80/81, 32,768 67/68 70/67 74/70 92/88, 98,304 108/110 124/118 142/133 209/191
 //   C = 192   16,448 52/54 55/56 58/57 71/64, 20,560 59/60 62/61 69/66 92/87, 51,400 100/96 106/98 119/115 176/161
