@@ -1176,11 +1176,17 @@ static int launch_small(const LinearArgs& p, const LinearArgs* p1, cudaStream_t 
 //   384 x 384, 92 of 257                                     3.3  4.2    /  3.6      1536 x 384, 92 of 257 (72)    4.3  4.4  /  4.2
 //   384 x 384, 644 of 1799 (90)                              6.2  4.6    /  4.5      3072 x 768, 92 of 257 (144)   7.8  5.9  /  6.0
 // (In brackets the 128 x 64 tiles, where they come near the 74 pairs or exceed them.)
+// Rows that a router picks (m_dev) are a third to a half of those allowed for, and a pair without any has ended early.  Where all rows are
+// valid every pair stores a tile, and the forms above win earlier.  Time of this form over theirs, no router, by K and number of tiles:
+//   64 columns   K = 384   45 tiles 0.97   48 0.99..1.03   56 1.05     K = 512   56 0.99   60 1.00   64 1.02   72 1.00..1.07   K = 640   72 0.98..1.02
+//   128 columns  K = 768   40 0.98..1.05   54 1.08   72 1.14           K = 1024  45 0.99..1.01   51 1.00   57 1.01..1.03   72 1.06   K = 1280   72 1.02
 static int long_reduction_pairs(const LinearArgs& p) {
     if (p.K % (2 * TBK) != 0) return 0;
     const long long pairs = sm_count() / 2;
-    if (small_tiles(p, 64) <= (p.K >= 512 ? pairs : pairs * 4 / 5)) return p.K >= 384 ? 64 : 0;
-    return p.K >= 768 && p.N > 64 && small_tiles(p, 128) <= pairs ? 128 : 0;
+    const bool routed = p.m_dev != nullptr;
+    if (small_tiles(p, 64) <= (p.K >= (routed ? 512 : 640) ? pairs : routed || p.K >= 512 ? pairs * 4 / 5 : pairs * 2 / 3)) return p.K >= 384 ? 64 : 0;
+    const long long most = p.K >= (routed ? 768 : 1280) ? pairs : p.K >= 1024 ? pairs * 2 / 3 : 0;
+    return p.N > 64 && small_tiles(p, 128) <= most ? 128 : 0;
 }
 
 template <int BN, int EPI>
