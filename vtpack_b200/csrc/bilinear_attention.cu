@@ -301,21 +301,34 @@ static int channels_of_a_load(int dtype, int C, const void* grid, std::initializ
 // Lanes of a group and vectors of a lane; lanes == 0: not for bilinear_vectors_*_kernel.
 // One vector where queries are few (a lane's chain is shorter, and there are more warps: below 16 a SM).  Else the fewest slots, as a
 // slot without channels costs like any other, and of these two vectors a lane, in the backward only where a group still covers 128 bytes: its reds of
-// 64 bytes are slower than its arithmetic is quicker.  us, forward / backward of 32 maps of 64 x 64, 9 points, point mode, one | two vectors:
-// bf16 C = 64 56 / 124 | 45 / 134, C = 32 31 / 75 | 27 / 105, fp32 C = 64 86 / 224 | 74 / 209; 16 maps, C = 96 bf16, 5 points 35 / 74 | three vectors
-// 23 / 61; 4 maps of 28 x 28, C = 64 bf16 6.4 / 13.4 | 8.5 / 15.2, 16 maps in fp32 12.6 / 29.9 | 11.5 / 29.5.
+// 64 bytes are slower than its arithmetic is quicker.  In fp32, where a vector is half as much arithmetic, the backward never takes groups of four lanes,
+// two vectors for more than 12 of them only and groups of eight lanes from a hundred warps a SM on; a forward of four vectors keeps one a lane.
+// us, forward / backward, point mode, of 32 maps of 64 x 64, 9 points (in brackets backward of 24 of 22 x 48, 5 points):
+//   bf16   4 vectors   2 x 2   25.7 /             4 x 1   29.0 /  72 (13)
+//          8           4 x 2   43.9 / 131 (22)    8 x 1   54.6 / 120 (18)
+//         12           4 x 3   63.3 / 194 (30)    8 x 2   83.5 / 210 (29)   16 x 1  106.4 / 240 (30)
+//         24           8 x 3  133   / 339 (42)   16 x 2  174   / 426 (50)   32 x 1  210   / 478 (55)
+//   fp32   4 vectors   2 x 2   27.3 /             4 x 1   23.8 /  73 (12)
+//         12           4 x 3   57.0 / 194 (35)    8 x 2   70.3 / 184 (25)   16 x 1   84.4 / 189 (24)
+//         16           8 x 2   74.3 / 208 (27)   16 x 1   85.6 / 222 (26)
+//         24           8 x 3  111   / 304 (42)   16 x 2  133   / 331 (39)   32 x 1  169   / 362 (42)
+// 4 maps of 28 x 28, 8 vectors in bf16, 5 points 8 x 1 3.9 / 7.0, 4 x 2 4.8 / 8.5; 64 of 14 x 14, 16 vectors in fp32, 4 points, channel mode
+// 16 x 1 6.6 / 13.3, 8 x 2 5.7 / 14.1.
 static BvShape bv_shape(int v, int dtype, int C, int H, int W, long long n_inst, bool grads, int sms) {
     const int n = C / v;
     if (v * elem_size(dtype) != 16 || n > BV_MAXVEC || n_inst > (1ll << 30) || (long long)H * W > (1ll << 30)) return {0, 0};
     BvShape best{4, 1};
     while (best.lanes < n && best.lanes < 32) best.lanes *= 2;
     if (best.lanes < n) return {32, 2};
+    const bool f32 = dtype == VTP_F32;
     for (int j = 2; j <= 3; ++j) {
-        int lanes = grads ? 4 : 2;
+        int lanes = !grads ? 2 : f32 ? 8 : 4;
         while (lanes * j < n) lanes *= 2;
-        if (n < 3 || lanes > 16 || n_inst * lanes < 16ll * 32 * sms) continue;
+        const long long warps = n_inst * lanes / 32;
+        if (n < 3 || lanes > 16 || warps < 16ll * sms) continue;
         const int slots = lanes * j, least = best.lanes * best.vecs;
-        if (slots < least || (slots == least && best.vecs == 1 && (!grads || lanes >= 8))) best = {lanes, j};
+        const bool pays = !grads ? !f32 || n > 4 : !f32 ? lanes >= 8 : n > 12 && (lanes > 8 || warps >= 100ll * sms);
+        if (slots < least || (slots == least && best.vecs == 1 && pays)) best = {lanes, j};
     }
     return best;
 }

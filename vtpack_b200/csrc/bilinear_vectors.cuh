@@ -41,13 +41,12 @@ struct BvPlace {
         if (a.tile_rows.d) {
             const uint32_t img = fast_div((uint32_t)unit, a.tiles), t = unit - img * a.tiles.d;
             const uint32_t ty = fast_div(t, a.tile_rows), tx = t - ty * a.tile_rows.d;
-            const int x = (int)tx * PW + sub, y = (int)ty * BV_WARPS + warp;
-            own = x < a.W && y < a.H;               // a group past the end goes along for the shuffles
+            own = true;
             b = img;
-            inst = (int)img * a.G + (own ? y * a.W + x : 0);
+            inst = (int)img * a.G + ((int)ty * BV_WARPS + warp) * a.W + (int)tx * PW + sub;
         } else {
             const int i = (unit * BV_WARPS + warp) * PW + sub;
-            own = i < a.n_inst;
+            own = i < a.n_inst;                     // a group past the end goes along for the shuffles
             inst = own ? i : 0;
             b = a.batch_of ? a.batch_of[inst] : (long long)fast_div((uint32_t)inst, a.per_image);
         }
@@ -235,8 +234,9 @@ template <typename T, bool POINT, bool GRAD>
 static void bv_launch(BvArgs a, const BvShape& s, cudaStream_t st) {
     const int pw = 32 / s.lanes;
     const long long tx = (a.W + pw - 1) / pw, ty = (a.H + BV_WARPS - 1) / BV_WARPS, in_tiles = tx * pw * ty * BV_WARPS;
-    // (a tile's lanes beyond the map are idle: not where they would be more than a fifth)
-    if (!a.batch_of && a.G == (long long)a.H * a.W && in_tiles * 4 <= a.G * 5ll) {
+    // Whole tiles only: idle lanes beyond the map cost more than the tiles save.  260 maps of 5 to 64 pixels a side, mean time over that without tiles'
+    // lanes beyond the map allowed: up to a quarter of them 1.03 (forward) and 1.02 (backward), a twentieth 1.005 and 1.004.
+    if (!a.batch_of && a.G == (long long)a.H * a.W && in_tiles == a.G) {
         a.tile_rows = make_fast_div((uint32_t)tx);
         a.tiles = make_fast_div((uint32_t)(tx * ty));
         a.units = (int)(a.B * tx * ty);
