@@ -391,6 +391,15 @@ def profile_case(which):
         for _ in range(3):
             _lib.check(lib.vtp_linear(x.data_ptr(), K, w.data_ptr(), b.data_ptr(), None, 0, y.data_ptr(), N,
                                       1 if dt == torch.bfloat16 else 0, M, None, N, K, 0, None))
+    elif which == "linear_few":         # few rows, long reductions: PVT's first reduction (3 images) and DeiT-S fc2 (one image, 92 of 257 rows)
+        for M, valid, N, K in ((192, 192, 64, 4096), (257, 92, 384, 1536)):
+            x = torch.randn(M, K, device=dev).bfloat16()
+            w = (torch.randn(N, K, device=dev) * 0.05).bfloat16()
+            b, y = torch.randn(N, device=dev), torch.empty(M, N, device=dev, dtype=torch.bfloat16)
+            rows = torch.tensor([valid], dtype=torch.int32, device=dev)
+            for _ in range(3):
+                _lib.check(lib.vtp_linear(x.data_ptr(), K, w.data_ptr(), b.data_ptr(), None, 0, y.data_ptr(), N, 1, M,
+                                          rows.data_ptr() if valid < M else None, N, K, 0, None))
     elif which in ("attention", "attention_f32"):    # 256 images x 6 heads, 114 queries per image, 257 keys
         B, N, h, Li, d = 256, 257, 6, 114, 64
         C, L = h * d, B * Li
@@ -821,7 +830,7 @@ def main():
                          "data loader hands over)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-stage-profile", action="store_true")
-    ap.add_argument("--profile", default=None, choices=["linear_kv", "linear_f32", "attention", "attention_f32", "block", "train_ops", "pvt_stage1", "pvt_model"],
+    ap.add_argument("--profile", default=None, choices=["linear_kv", "linear_f32", "linear_few", "attention", "attention_f32", "block", "train_ops", "pvt_stage1", "pvt_model"],
                     help="run a small case of one kernel family (for ncu) and exit")
     ap.add_argument("--layer-sweep", action="store_true",
                     help="time one DGE layer over gate skew against the dense block and exit")

@@ -666,7 +666,7 @@ extern "C" int vtp_unpool_grad(const void* grad_out, int dtype, int B, int N, in
 }
 
 // The same gradient for a patch list that was made from grain indices: one CTA per region, every token
-// row of the region requested before any arithmetic, no walk over the list (region_ops.cu).
+// row of the region requested before any arithmetic, no walk over the list (region_ops.cuh).
 extern "C" int vtp_region_layout_supported(int dtype, int C) {
     RegionGeom g{};
     g.B = g.Hr = g.Wr = 1; g.C = C; g.region = 4;
