@@ -301,8 +301,9 @@ static int channels_of_a_load(int dtype, int C, const void* grid, std::initializ
 // Lanes of a group and vectors of a lane; lanes == 0: not for bilinear_vectors_*_kernel.
 // One vector where queries are few (a lane's chain is shorter, and there are more warps: below 16 a SM).  Else the fewest slots, as a
 // slot without channels costs like any other, and of these two vectors a lane, in the backward only where a group still covers 128 bytes: its reds of
-// 64 bytes are slower than its arithmetic is quicker.  In fp32, where a vector is half as much arithmetic, the backward never takes groups of four lanes,
-// two vectors for more than 12 of them only and groups of eight lanes from a hundred warps a SM on; a forward of four vectors keeps one a lane.
+// 64 bytes are slower than its arithmetic is quicker.  In fp32, where a vector is half as much arithmetic, the backward takes several
+// a lane in groups of eight lanes and more only, two a lane for rows of more than 12 (in groups of eight from a hundred warps a SM on); a forward of
+// rows of four keeps one a lane.
 // us, forward / backward, point mode, of 32 maps of 64 x 64, 9 points (in brackets backward of 24 of 22 x 48, 5 points):
 //   bf16   4 vectors   2 x 2   25.7 /             4 x 1   29.0 /  72 (13)
 //          8           4 x 2   43.9 / 131 (22)    8 x 1   54.6 / 120 (18)
